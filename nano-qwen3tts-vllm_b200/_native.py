@@ -95,6 +95,8 @@ def _load():
         "b2tts_window_sigmoid_attn": (I, [P, P, P, P, P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, I, P]),
         "b2tts_moe_route": (I, [P, P, P, P, P, P, I, I, I, I, F, P, I, I, I, I, P]),
         "b2tts_grouped_gemm_gated": (I, [P, L, P, P, L, P, P, I, I, I, I, I, F, F, P]),
+        "b2tts_grouped_gemm_silu": (I, [P, L, P, P, L, P, P, I, I, I, I, I, P]),
+        "b2tts_grouped_gemm_timeouts": (I, []),
         "b2tts_tanh_residual": (I, [P, P, P, I, P, P, P, I, P, P, P, F, P, P, P, P, P, I, I, I, I, P]),
         "b2tts_tanh_gather": (I, [P, P, P, P, P, P, I, I, I, P]),
         "b2tts_clamped_gate_mul": (I, [P, P, L, I, F, F, I, P]),
@@ -893,6 +895,27 @@ def grouped_gemm_gated(a, w, c, offsets, sorted_pair, n_pairs, top, limit, alpha
     gu = torch.empty(n_pairs, n, dtype=a.dtype, device=a.device)
     grouped_gemm(a, w, gu, offsets, sorted_pair, n_pairs, top, in_by_token=True, out_by_pair=False, act=0)
     return clamped_gate_mul(gu, limit, alpha, out=c)
+
+
+def grouped_gemm_silu(a, w, c, offsets, sorted_pair, n_pairs, top):
+    """c [n_pairs, ff] <- silu(gate) * up of every sorted pair's expert: w [E, 2 ff, K] = [gate; up] per expert.  bf16 with ff and K
+    multiples of 8 runs as one launch, the product taken from the float sums; anything else is the grouped product followed by
+    the activation kernel."""
+    _act(a, "a")
+    e, n, k = w.shape
+    ff = n // 2
+    if a.dtype == BF16 and ff % 8 == 0 and k % 8 == 0 and a.stride(0) % 8 == 0 and (a.data_ptr() | w.data_ptr() | c.data_ptr()) % 16 == 0:
+        assert w.dtype == BF16 and c.dtype == BF16 and w.is_contiguous() and c.is_contiguous()
+        _check(_load().b2tts_grouped_gemm_silu(a.data_ptr(), a.stride(0), w.data_ptr(), c.data_ptr(), c.stride(0), offsets.data_ptr(),
+                                               sorted_pair.data_ptr(), n_pairs, e, ff, k, top, _stream()), "grouped_gemm_silu")
+        return c
+    gu = torch.empty(n_pairs, n, dtype=a.dtype, device=a.device)
+    grouped_gemm(a, w, gu, offsets, sorted_pair, n_pairs, top, in_by_token=True, out_by_pair=False, act=0)
+    return silu_mul(gu, out=c)
+
+
+def grouped_gemm_timeouts() -> int:
+    return int(_load().b2tts_grouped_gemm_timeouts())
 
 
 # ------------------------------------------------------------------------------------------ latent-attention decoders

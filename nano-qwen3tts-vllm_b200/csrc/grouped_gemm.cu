@@ -8,10 +8,13 @@
 // them in a fixed order.  Inputs are bf16 or float, products accumulate in float.  A tile never mixes two experts:
 // tile y of the grid is mapped to (expert, row block) by walking the group sizes, and tiles beyond the last group exit.
 //
-// Gated experts (grouped_gemm_gated): W[e] is [gate; up], 2 ff rows.  A tile's 128 rows of W are 8 gate rows and the 8 matching
+// bf16 groups of more than a few rows run on the tcgen05 kernel of grouped_gemm_tc.cu; the kernels here take decode-sized groups,
+// float and odd sizes.
+//
+// Gated experts (grouped_gemm_gated, grouped_gemm_silu): W[e] is [gate; up], 2 ff rows.  A tile's 128 rows of W are 8 gate rows and the 8 matching
 // up rows in turn, so a thread's accumulators hold the gate and the up value of the same columns and the clamped gated product
 // is taken in the epilogue: C has ff columns and the [pairs, 2 ff] product never reaches memory.
-#include "clamped_gate.cuh"
+#include "grouped_gemm.cuh"
 
 namespace b2 {
 
@@ -122,8 +125,6 @@ template <int BM> struct GmShape {
   static constexpr size_t SMEM = sizeof(__nv_bfloat16) * STAGES * (BM + GM_BN) * GM_LD + sizeof(int) * 2 * BM;
 };
 
-constexpr int ACT_GATED = 2;
-
 template <int GM_BM, int ACT>
 __global__ void __launch_bounds__(GM_THREADS, 2)
 grouped_gemm_mma_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv_bfloat16* __restrict__ W,
@@ -168,7 +169,7 @@ grouped_gemm_mma_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const 
   for (int i = 0; i < GM_PASSES; ++i) {
     const int r = GM_RPP * i + tid / GM_CPR;
     a_row[i] = r < GM_BM ? in_rows[r] : -1;
-    if constexpr (ACT == ACT_GATED) {
+    if constexpr (ACT >= GG_CLAMPED) {
       const int f = n0 / 2 + (r >> 4) * 8 + (r & 7);      // 8 gate rows, 8 up rows, ..
       w_row[i] = f < N / 2 ? f + ((r >> 3) & 1) * (N / 2) : -1;
     } else {
@@ -234,12 +235,12 @@ grouped_gemm_mma_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const 
       const int orow = out_rows[r];
       if (orow < 0) continue;
       __nv_bfloat16* crow = C + static_cast<int64_t>(orow) * ldc;
-      if constexpr (ACT == ACT_GATED) {
+      if constexpr (ACT >= GG_CLAMPED) {
 #pragma unroll
         for (int np = 0; np < NT / 2; ++np) {
           const int n = n0 / 2 + (wn * (NT / 2) + np) * 8 + 2 * (lane & 3);
-          const float v0 = clamped_gate(acc[mt][2 * np][2 * half], acc[mt][2 * np + 1][2 * half], limit, alpha);
-          const float v1 = clamped_gate(acc[mt][2 * np][2 * half + 1], acc[mt][2 * np + 1][2 * half + 1], limit, alpha);
+          const float v0 = gated_value<ACT>(acc[mt][2 * np][2 * half], acc[mt][2 * np + 1][2 * half], limit, alpha);
+          const float v1 = gated_value<ACT>(acc[mt][2 * np][2 * half + 1], acc[mt][2 * np + 1][2 * half + 1], limit, alpha);
           if (n < N / 2) *reinterpret_cast<uint32_t*>(crow + n) = pack_bf16(v0, v1);      // ff is a multiple of 8
         }
         continue;
@@ -288,8 +289,11 @@ extern "C" int b2tts_grouped_gemm(const void* a, int64_t lda, const void* w, voi
   if (n_pairs == 0) return B2TTS_OK;
   B2_REQUIRE(a && w && c && offsets && sorted_pair, B2TTS_EINVAL, "grouped_gemm: null pointer");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // bf16 with 16-byte rows: the tensor-core kernel; float (true 32-bit products) and odd sizes: the plain one
+  // bf16 with 16-byte rows: the tensor-core kernels; float (true 32-bit products) and odd sizes: the plain one
   if (dtype == B2TTS_DTYPE_BF16 && k % 8 == 0 && lda % 8 == 0 && aligned16(a) && aligned16(w)) {
+    if (grouped_tc_applies(n_pairs, experts, n, ldc, c))
+      return launch_grouped_tc("grouped_gemm", a, lda, w, c, ldc, offsets, sorted_pair, n_pairs, experts, n, k, top, in_by_token, out_by_pair,
+                               act, 0.f, 0.f, st);
     // groups of a decode step (16 rows per expert on average, or fewer): the 32-row shape
     const bool small = n_pairs <= 16 * experts;
 #define GM_GO(BM, ACT) launch_grouped_mma<BM, ACT>(n_pairs, st, a, lda, w, c, ldc, offsets, sorted_pair, experts, n, k, top, in_by_token, out_by_pair)
@@ -320,10 +324,33 @@ extern "C" int b2tts_grouped_gemm_gated(const void* a, int64_t lda, const void* 
   B2_REQUIRE(a && w && c && offsets && sorted_pair, B2TTS_EINVAL, "grouped_gemm_gated: null pointer");
   B2_REQUIRE(aligned16(a) && aligned16(w) && aligned16(c), B2TTS_EALIGN, "grouped_gemm_gated: pointers must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (grouped_tc_applies(n_pairs, experts, ff, ldc, c))
+    return launch_grouped_tc("grouped_gemm_gated", a, lda, w, c, ldc, offsets, sorted_pair, n_pairs, experts, 2 * ff, k, top, 1, 0, GG_CLAMPED, limit,
+                             alpha, st);
   const bool small = n_pairs <= 16 * experts;
-  const cudaError_t e = small ? launch_grouped_mma<32, ACT_GATED>(n_pairs, st, a, lda, w, c, ldc, offsets, sorted_pair, experts, 2 * ff, k, top, 1, 0, limit, alpha)
-                              : launch_grouped_mma<128, ACT_GATED>(n_pairs, st, a, lda, w, c, ldc, offsets, sorted_pair, experts, 2 * ff, k, top, 1, 0, limit, alpha);
+  const cudaError_t e = small ? launch_grouped_mma<32, GG_CLAMPED>(n_pairs, st, a, lda, w, c, ldc, offsets, sorted_pair, experts, 2 * ff, k, top, 1, 0, limit, alpha)
+                              : launch_grouped_mma<128, GG_CLAMPED>(n_pairs, st, a, lda, w, c, ldc, offsets, sorted_pair, experts, 2 * ff, k, top, 1, 0, limit, alpha);
   if (e != cudaSuccess) return cuda_fail(e, "grouped_gemm_gated");
   B2_CHECK_LAUNCH("grouped_gemm_gated");
+  return B2TTS_OK;
+}
+
+extern "C" int b2tts_grouped_gemm_silu(const void* a, int64_t lda, const void* w, void* c, int64_t ldc, const int32_t* offsets,
+                                       const int32_t* sorted_pair, int n_pairs, int experts, int ff, int k, int top, void* stream) {
+  using namespace b2;
+  B2_REQUIRE(n_pairs >= 0 && experts > 0 && ff > 0 && k > 0 && top > 0, B2TTS_EINVAL, "grouped_gemm_silu: bad sizes");
+  B2_REQUIRE(ff % 8 == 0 && k % 8 == 0 && lda % 8 == 0 && ldc % 2 == 0, B2TTS_EUNSUPPORTED, "grouped_gemm_silu: ff=%d k=%d must be multiples of 8",
+             ff, k);
+  if (n_pairs == 0) return B2TTS_OK;
+  B2_REQUIRE(a && w && c && offsets && sorted_pair, B2TTS_EINVAL, "grouped_gemm_silu: null pointer");
+  B2_REQUIRE(aligned16(a) && aligned16(w) && aligned16(c), B2TTS_EALIGN, "grouped_gemm_silu: pointers must be 16-byte aligned");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (grouped_tc_applies(n_pairs, experts, ff, ldc, c))
+    return launch_grouped_tc("grouped_gemm_silu", a, lda, w, c, ldc, offsets, sorted_pair, n_pairs, experts, 2 * ff, k, top, 1, 0, GG_SILU, 0.f, 0.f, st);
+  const bool small = n_pairs <= 16 * experts;
+  const cudaError_t e = small ? launch_grouped_mma<32, GG_SILU>(n_pairs, st, a, lda, w, c, ldc, offsets, sorted_pair, experts, 2 * ff, k, top, 1, 0)
+                              : launch_grouped_mma<128, GG_SILU>(n_pairs, st, a, lda, w, c, ldc, offsets, sorted_pair, experts, 2 * ff, k, top, 1, 0);
+  if (e != cudaSuccess) return cuda_fail(e, "grouped_gemm_silu");
+  B2_CHECK_LAUNCH("grouped_gemm_silu");
   return B2TTS_OK;
 }

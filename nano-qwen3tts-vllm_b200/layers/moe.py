@@ -65,9 +65,8 @@ class TopKMoE(nn.Module):
             y = torch.empty(pairs, self.ff, dtype=h.dtype, device=h.device)
             nat.grouped_gemm_gated(h, self.up, y, offsets, sorted_pair, pairs, self.top, self.clamp)
         elif self.gated:
-            gu = torch.empty(pairs, 2 * self.ff, dtype=h.dtype, device=h.device)
-            nat.grouped_gemm(h, self.up, gu, offsets, sorted_pair, pairs, self.top, in_by_token=True, out_by_pair=False, act=0)
-            y = nat.silu_mul(gu)
+            y = torch.empty(pairs, self.ff, dtype=h.dtype, device=h.device)
+            nat.grouped_gemm_silu(h, self.up, y, offsets, sorted_pair, pairs, self.top)
         else:
             y = torch.empty(pairs, self.ff, dtype=h.dtype, device=h.device)
             nat.grouped_gemm(h, self.up, y, offsets, sorted_pair, pairs, self.top, in_by_token=True, out_by_pair=False, act=1)

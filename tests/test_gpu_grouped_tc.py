@@ -1,0 +1,91 @@
+"""Grouped products on the tensor cores against 64-bit sums: group sizes, columns and inner sizes around the edges of the tiles,
+scattered rows, every activation."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.fixture(scope="module")
+def nat():
+    import nano_qwen3tts_vllm_b200._native as n
+    n.lib()
+    return n
+
+
+def _groups(sizes, top, seed):
+    """offsets and a random assignment of (token, choice) pairs to groups of these sizes."""
+    n = sum(sizes)
+    g = torch.Generator().manual_seed(seed)
+    pair = torch.randperm(n, generator=g).to(torch.int32)
+    off = torch.tensor([sum(sizes[:i]) for i in range(len(sizes) + 1)], dtype=torch.int32)
+    return off.to(DEV), pair.to(DEV), n
+
+
+def _close(got, ref, inner):
+    """bf16 storage rounds to 2^-9 of the value (2^-8 allowed); the float sums of ``inner`` products err by at most inner * 2^-24 of
+    their absolute sum, which is below sqrt(inner) * 6 here (operands of unit size, six sigma), and the activations used have
+    slopes of at most about 2 |z| + 2."""
+    err = (got.double() - ref).abs()
+    assert bool((err <= ref.abs() * 2.0 ** -8 + inner * 2.0 ** -24 * 6 * inner ** 0.5 * (2 * ref.abs().sqrt() + 2)).all()), err.max().item()
+
+
+@pytest.mark.parametrize("sizes", [(129, 0, 1, 127, 128), (600, 33), (1, 1, 1, 700), (40, 40, 40)])
+@pytest.mark.parametrize("n,k", [(8, 8), (264, 200), (512, 64), (136, 72), (1032, 328)])
+def test_group_column_and_inner_edges(nat, sizes, n, k):
+    top, E = 2, len(sizes)
+    off, pair, pairs = _groups(sizes, top, n + k)
+    if pairs % top:
+        sizes = sizes[:-1] + (sizes[-1] + 1,)
+        off, pair, pairs = _groups(sizes, top, n + k)
+    g = torch.Generator(device=DEV).manual_seed(k)
+    r = lambda *s: torch.randn(s, generator=g, device=DEV).to(torch.bfloat16)
+    tok, w = r(pairs // top, k), r(E, n, k)
+    for act in (0, 1):
+        c = torch.full((pairs, n), 7.0, device=DEV, dtype=torch.bfloat16)
+        nat.grouped_gemm(tok, w, c, off, pair, pairs, top, in_by_token=True, out_by_pair=False, act=act)
+        for e in range(E):
+            rows = slice(off[e].item(), off[e + 1].item())
+            ref = tok[(pair[rows] // top).long()].double() @ w[e].double().T
+            _close(c[rows], ref.clamp(min=0) ** 2 if act else ref, k)
+    y = r(pairs, k)
+    c = torch.full((pairs, n), 7.0, device=DEV, dtype=torch.bfloat16)
+    nat.grouped_gemm(y, w, c, off, pair, pairs, top, in_by_token=False, out_by_pair=True, act=0)
+    for e in range(E):
+        rows = slice(off[e].item(), off[e + 1].item())
+        _close(c[pair[rows].long()], y[rows].double() @ w[e].double().T, k)
+    assert nat.grouped_gemm_timeouts() == 0
+
+
+@pytest.mark.parametrize("sizes", [(129, 0, 1, 128), (5, 3, 2), (400, 77)])         # the middle one: the decode-sized kernel
+@pytest.mark.parametrize("ff,k", [(8, 64), (136, 200), (128, 8), (264, 136)])
+def test_gated_activations(nat, sizes, ff, k):
+    top, E = 1, len(sizes)
+    off, pair, pairs = _groups(sizes, top, ff + k)
+    g = torch.Generator(device=DEV).manual_seed(ff)
+    r = lambda *s: torch.randn(s, generator=g, device=DEV).to(torch.bfloat16)
+    h, w = r(pairs, k), (r(E, 2 * ff, k) * k ** -0.5).to(torch.bfloat16)
+    got = {"silu": torch.empty(pairs, ff, device=DEV, dtype=torch.bfloat16), "clamped": torch.empty(pairs, ff, device=DEV, dtype=torch.bfloat16)}
+    nat.grouped_gemm_silu(h, w, got["silu"], off, pair, pairs, top)
+    nat.grouped_gemm_gated(h, w, got["clamped"], off, pair, pairs, top, 1.5)
+    for e in range(E):
+        rows = slice(off[e].item(), off[e + 1].item())
+        gu = h[pair[rows].long()].double() @ w[e].double().T
+        gate, up = gu[:, :ff], gu[:, ff:]
+        _close(got["silu"][rows], torch.nn.functional.silu(gate) * up, k)
+        gate, up = gate.clamp(max=1.5), up.clamp(-1.5, 1.5)
+        _close(got["clamped"][rows], gate * torch.sigmoid(1.702 * gate) * (up + 1), k)
+
+
+def test_not_finite_values_stay_in_their_rows(nat):
+    """A NaN in one row of the input reaches that row's outputs only, activation included."""
+    off, pair, pairs = _groups((150, 90), 1, 3)
+    g = torch.Generator(device=DEV).manual_seed(1)
+    h = torch.randn(pairs, 64, generator=g, device=DEV).to(torch.bfloat16)
+    w = torch.randn(2, 32, 64, generator=g, device=DEV).to(torch.bfloat16)
+    h[11, 5] = float("nan")
+    c = torch.empty(pairs, 16, device=DEV, dtype=torch.bfloat16)
+    nat.grouped_gemm_silu(h, w, c, off, pair, pairs, 1)
+    bad = torch.isnan(c).all(1)
+    assert bad.sum() == 1 and pair[bad.nonzero()[0, 0]] == 11 and torch.isfinite(c[~bad]).all()
