@@ -8,6 +8,9 @@
 //   retention        S <- decay_h S + k v^T                                o = S^T q      (a fixed decay per head; retention.cu
 //                                                                                         has its tensor-core and one-token kernels)
 //
+// Prompt portions of the state space in bf16 run in chunks on the tensor cores (recurrent_chunk.cu); what follows is about the
+// token-by-token kernel, which takes everything else.
+//
 // All of them update every value column of S independently.  A column is shared by RS = ceil(key size / 32) lanes of one
 // warp, each keeping 32 rows of it in registers for the whole portion; sums over the rows (the read-out, the delta rule's
 // S^T k, the unit norms) are butterfly shuffles over those lanes.  The per-token vectors (k, q or B, C) are staged in
@@ -22,7 +25,7 @@
 // CTAs which share a head share no state.
 #include <algorithm>
 
-#include "row_ops.cuh"
+#include "scan.cuh"
 
 namespace b2 {
 namespace row {
@@ -33,23 +36,6 @@ constexpr int SCAN_PER = 8;               // key elements per lane of the one-wa
 constexpr int SCAN_DEPTH = 4;             // tokens whose inputs are in flight in registers
 
 enum { SCAN_LINEAR = 0, SCAN_DELTA = 1, SCAN_GATED = 2 };
-
-struct ScanArgs {
-  const void* k; int64_t ldk;             // key-like vectors: (row, group g, i) at k[row * ldk + g * d + i]
-  const void* q; int64_t ldq;             // query-like vectors, same layout
-  const void* v; int64_t ldv;             // values: (row, head h, c) at v[row * ldv + h * dv + c]
-  const float* coef;                      // [rows, H, 3] per-token scalars, see scan_kernel (SCAN_GATED: unused)
-  const float* head_decay;                // [H] or null: coef = (head_decay[h], 1, 1) for every token (coef itself is then unused)
-  int rows;                               // 0: every sequence, 1: only those with more than one new token, 2: only one-token ones
-  const float* decay; int64_t ldd;        // SCAN_GATED: per key channel, (row, head h, i) at decay[row * ldd + h * d + i]
-  const float* skip;                      // [H] or null: out += skip[h] * value
-  float* state;                           // [slots, H, d, dv]
-  float* out;                             // [rows, H * dv]
-  const int32_t* seq_start; const int32_t* seq_pos0; const int32_t* seq_len; const int32_t* seq_slot;
-  int H, G, d, dv;
-  float qscale;
-  int divide;                             // linear: out = S^T q * qscale / coef[2] instead of S^T q * qscale
-};
 
 // sum over the RS lanes that share a column (lane = slice * (32 / RS) + column): every one of them gets the total
 template <int RS>
@@ -214,9 +200,12 @@ scan_kernel(const ScanArgs a) {
 }
 
 // ------------------------------------------------------------------ per-token scalars of the state space and the delta rule
-// kind 0: dt = softplus(s1 + f1[h]); coef = (exp(-exp(f2[h]) dt), dt, 1)                       (f1 = dt_bias, f2 = A_log)
-// kind 1: coef = (exp(-exp(f1[h]) softplus(s2 + f2[h])), sigmoid(s1), 1)                      (f1 = A_log, f2 = dt_bias)
+// kind 0: dt = softplus(s1 + f1[h]), l = -exp(f2[h]) dt; coef = (exp(l), dt, l)               (f1 = dt_bias, f2 = A_log)
+// kind 1: l = -exp(f1[h]) softplus(s2 + f2[h]); coef = (exp(l), sigmoid(s1), l)               (f1 = A_log, f2 = dt_bias)
 // kind 2: coef = (log input gate, log forget gate, 1) of the matrix memory                   (f1, f2 = the gates' biases)
+// The decays are formed in double: an error of a decay's logarithm grows with every token that the state is carried over.
+__device__ __forceinline__ double softplus_d(double x) { return fmax(x, 0.0) + log1p(exp(-fabs(x))); }
+
 template <typename T>
 __global__ void scan_coef_kernel(const T* __restrict__ s1, const T* __restrict__ s2, int64_t lds, const float* __restrict__ f1,
                                  const float* __restrict__ f2, float* __restrict__ coef, int n_tokens, int H, int kind, float cap) {
@@ -224,20 +213,23 @@ __global__ void scan_coef_kernel(const T* __restrict__ s1, const T* __restrict__
   if (idx >= n_tokens * H) return;
   const size_t t = idx / H;
   const int h = idx % H;
-  float c0, c1;
+  float c0, c1, log_decay = 1.f;
   if (kind == 2) {                                       // log gates: cap tanh((s1 + f1) / cap), logsigmoid(cap tanh((s2 + f2) / cap))
     c0 = cap * tanhf((to_f(s1[t * lds + h]) + f1[h]) / cap);
     c1 = logsigmoid_f(cap * tanhf((to_f(s2[t * lds + h]) + f2[h]) / cap));
   } else if (kind == 0) {
-    const float dt = softplus_f(to_f(s1[t * lds + h]) + f1[h]);
-    c0 = expf(-expf(f2[h]) * dt);
-    c1 = dt;
+    const double dt = softplus_d(to_f(s1[t * lds + h]) + f1[h]), l = -exp(static_cast<double>(f2[h])) * dt;
+    log_decay = static_cast<float>(l);
+    c0 = static_cast<float>(exp(l));
+    c1 = static_cast<float>(dt);
   } else {
-    c0 = expf(-expf(f1[h]) * softplus_f(to_f(s2[t * lds + h]) + f2[h]));
+    const double l = -exp(static_cast<double>(f1[h])) * softplus_d(to_f(s2[t * lds + h]) + f2[h]);
+    log_decay = static_cast<float>(l);
+    c0 = static_cast<float>(exp(l));
     c1 = sigmoid_f(to_f(s1[t * lds + h]));
   }
   float* c = coef + static_cast<size_t>(idx) * 3;
-  c[0] = c0; c[1] = c1; c[2] = 1.f;
+  c[0] = c0; c[1] = c1; c[2] = log_decay;
 }
 
 // ------------------------------------------------------------------ scalar part of the matrix memory
@@ -374,6 +366,11 @@ extern "C" int b2tts_ssm_scan(const void* xbc, int64_t ldx, const void* dt, int6
   a.state = state; a.out = out;
   a.seq_start = seq_start; a.seq_pos0 = seq_pos0; a.seq_len = seq_len; a.seq_slot = seq_slot;
   a.H = heads; a.G = groups; a.d = dim; a.dv = vdim; a.qscale = 1.f; a.divide = 0;
+  if (dtype == B2TTS_DTYPE_BF16 && n_tokens > n_seqs && scan_chunk_applies(a)) {
+    const int rc = launch_linear_chunk("ssm_scan (portions)", a, n_seqs, st);
+    if (rc != B2TTS_OK) return rc;
+    a.rows = 2;                                            // one-token rows beside the portions
+  }
   const int rc = dtype == B2TTS_DTYPE_BF16 ? launch_scan<__nv_bfloat16, SCAN_LINEAR>(a, n_seqs, st, "ssm_scan")
                                            : launch_scan<float, SCAN_LINEAR>(a, n_seqs, st, "ssm_scan");
   if (rc != B2TTS_OK) return rc;
