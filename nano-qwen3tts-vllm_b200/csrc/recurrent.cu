@@ -8,7 +8,7 @@
 //   retention        S <- decay_h S + k v^T                                o = S^T q      (a fixed decay per head; retention.cu
 //                                                                                         has its tensor-core and one-token kernels)
 //
-// Prompt portions of the state space in bf16 run in chunks on the tensor cores (recurrent_chunk.cu); what follows is about the
+// Prompt portions of the state space and the delta rule in bf16 run in chunks on the tensor cores (recurrent_chunk.cu); what follows is about the
 // token-by-token kernel, which takes everything else.
 //
 // All of them update every value column of S independently.  A column is shared by RS = ceil(key size / 32) lanes of one
@@ -402,6 +402,11 @@ extern "C" int b2tts_delta_rule_scan(const void* qkv, int64_t ldq, const void* b
   a.state = state; a.out = out;
   a.seq_start = seq_start; a.seq_pos0 = seq_pos0; a.seq_len = seq_len; a.seq_slot = seq_slot;
   a.H = heads; a.G = kv_heads; a.d = dim; a.dv = vdim; a.qscale = 1.0f / sqrtf(static_cast<float>(dim)); a.divide = 0;
+  if (dtype == B2TTS_DTYPE_BF16 && n_tokens > n_seqs && scan_chunk_applies(a)) {
+    const int rc = launch_delta_chunk("delta_rule_scan (portions)", a, n_seqs, st);
+    if (rc != B2TTS_OK) return rc;
+    a.rows = 2;                                            // one-token rows beside the portions
+  }
   const int rc = dtype == B2TTS_DTYPE_BF16 ? launch_scan<__nv_bfloat16, SCAN_DELTA>(a, n_seqs, st, "delta_rule_scan")
                                            : launch_scan<float, SCAN_DELTA>(a, n_seqs, st, "delta_rule_scan");
   if (rc != B2TTS_OK) return rc;

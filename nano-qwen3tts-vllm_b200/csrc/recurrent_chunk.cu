@@ -368,6 +368,413 @@ linear_chunk_kernel(const ScanArgs a) {
     for (int e = 0; e < 4; ++e) Sg[static_cast<size_t>(nt * 8 + c2 + (e & 1)) * dv + pr + 8 * (e >> 1)] = S[nt][e];
 }
 
+// ------------------------------------------------------------------ delta rule
+// S <- e^l S; u = beta (v - S^T k^); S <- S + k^ u^T; o = S^T q^ * scale with unit vectors k^ = kn k, q^ = qn q.  Inside a chunk
+//
+//   u_i + sum_(j < i) A_ij u_j = beta_i (v_i - e^(c_i) S^T k^_i),   A_ij = beta_i e^(c_i - c_j) (k^_i . k^_j)
+//   o_i = e^(c_i) S^T q^_i + sum_(j <= i) e^(c_i - c_j) (q^_i . k^_j) u_j          S <- e^(c_L) S + sum_j e^(c_L - c_j) k^_j u_j^T
+//
+// so that a chunk is two 64 x 64 tables of dot products (exact bf16 products, the norms multiplied in afterwards), the state against
+// keys and queries, a triangular solve per value column in float, and two products with the solution.
+//
+// One CTA of eight warps per (sequence, head, 64 value columns).  Warp (wp, wh) owns value columns 16 wp .. + 15 and the wh-th half of
+// the key channels of the state, transposed in its accumulators as above; what the halves sum meets in shared memory.  The solve
+// gives four lanes to a column (row i belongs to lane i mod 4): four rows at a time are exchanged, solved by all four lanes and
+// subtracted from the rows behind.  Floats enter products as three bf16 parts, two floats as the six part products down to 2^-16.
+template <int D> struct DeltaTiles {
+  static constexpr int FS = CK_L + 4;       // padded float rows: a warp's quads fall into distinct banks
+  __nv_bfloat16 q[2][CK_L * D], k[2][CK_L * D], v[2][CK_L * CK_P];
+  __nv_bfloat16 m[3][CK_L * CK_L];          // e^(c_i - c_j) (q^_i . k^_j) in three parts
+  float A[CK_L * FS];
+  float f[2][CK_P * FS];                    // [value column][token]: S^T k of the two halves, then u | the exchanged half of o
+  double cum[CK_L];
+  float ecum[CK_L], beta[CK_L], wl[CK_L], kn[CK_L], qn[CK_L];
+  float red[2][2][2][CK_P];                 // token by token: [parity][k or q][half][value column]
+  int wild;
+};
+
+template <int D>
+__global__ void __launch_bounds__(256, 1)
+delta_chunk_kernel(const ScanArgs a) {
+  using Sm = DeltaTiles<D>;
+  constexpr int RB = D * 2, VB = CK_P * 2, MB = CK_L * 2, FS = Sm::FS, THREADS = 256, CH = D / 2, NT = CH / 8;
+  extern __shared__ __align__(128) unsigned char ck_smem[];
+  Sm& sm = *reinterpret_cast<Sm*>(ck_smem);
+  const int b = blockIdx.z, h = blockIdx.y, p0 = blockIdx.x * CK_P;
+  const int len = a.seq_len[b];
+  if (len <= 1) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wp = warp & 3, wh = warp >> 2, g4 = lane >> 2, c2 = 2 * (lane & 3);
+  const int H = a.H, dv = a.dv, g = h / (H / a.G);
+  const size_t start = a.seq_start[b];
+  using B = __nv_bfloat16;
+  const B* qg = static_cast<const B*>(a.q) + start * a.ldq + static_cast<size_t>(g) * D;
+  const B* kg = static_cast<const B*>(a.k) + start * a.ldk + static_cast<size_t>(g) * D;
+  const B* vg = static_cast<const B*>(a.v) + start * a.ldv + static_cast<size_t>(h) * dv + p0;
+  const float* cp = a.coef + (start * H + h) * 3;
+  float* Sg = a.state + (static_cast<size_t>(a.seq_slot[b]) * H + h) * D * dv + p0;
+  float* og = a.out + start * H * dv + static_cast<size_t>(h) * dv + p0;
+  auto load_chunk = [&](int t0, int s) {
+    for (int idx = tid; idx < CK_L * (D / 8); idx += THREADS) {
+      const int j = idx / (D / 8), ch = idx % (D / 8);
+      const bool ok = t0 + j < len;
+      const size_t row = ok ? t0 + j : 0;
+      cp_async_16(reinterpret_cast<unsigned char*>(sm.q[s]) + tile_off(j, ch, RB), qg + row * a.ldq + ch * 8, ok);
+      cp_async_16(reinterpret_cast<unsigned char*>(sm.k[s]) + tile_off(j, ch, RB), kg + row * a.ldk + ch * 8, ok);
+    }
+    for (int idx = tid; idx < CK_L * (CK_P / 8); idx += THREADS) {
+      const int j = idx / (CK_P / 8), ch = idx % (CK_P / 8);
+      const bool ok = t0 + j < len;
+      cp_async_16(reinterpret_cast<unsigned char*>(sm.v[s]) + tile_off(j, ch, VB), vg + (ok ? t0 + j : 0) * a.ldv + ch * 8, ok);
+    }
+  };
+  load_chunk(0, 0);
+  cp_async_commit();
+  const int pr = wp * 16 + g4, n0 = wh * CH;               // S^T fragments: value columns pr (+ 8), key channels n0 + nt * 8 + c2 (+ 1)
+  float S[NT][4];
+  const bool carried = a.seq_pos0[b] > 0;
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) S[nt][e] = carried ? Sg[static_cast<size_t>(n0 + nt * 8 + c2 + (e & 1)) * dv + pr + 8 * (e >> 1)] : 0.f;
+  // scalars of a chunk (warp 0: lane l holds tokens 2 l, 2 l + 1), fetched a chunk ahead
+  float cl[2], cb_[2];
+  auto fetch_coef = [&](int t0) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int t = t0 + 2 * lane + e;
+      cl[e] = cb_[e] = 0.f;
+      if (warp == 0 && t < len) { cb_[e] = cp[static_cast<size_t>(t) * H * 3 + 1]; cl[e] = cp[static_cast<size_t>(t) * H * 3 + 2]; }
+    }
+  };
+  fetch_coef(0);
+  const uint32_t m_u = smem_u32(sm.m);
+  const int ra = lane & 15, ca = lane >> 4;
+  const int rb = (lane >> 4) * 8 + (lane & 7), cb = (lane >> 3) & 1;
+  const int rt = ((lane >> 3) & 1) * 8 + (lane & 7), ct = lane >> 4;
+  for (int t0 = 0, s = 0; t0 < len; t0 += CK_L, s ^= 1) {
+    const int L = min(CK_L, len - t0);
+    cp_async_wait<0>();
+    __syncthreads();                                       // the chunk has landed; the previous one is consumed
+    // ---- norms of k and q rows (two threads a row) and the range of everything that will be split
+    bool wild = false;
+    {
+      const int r = tid >> 1;
+      const unsigned char* row = reinterpret_cast<const unsigned char*>(r < CK_L ? sm.k[s] : sm.q[s]);
+      uint32_t m = 0;
+      float ss = 0.f;
+#pragma unroll
+      for (int c = 0; c < D / 16; ++c) {
+        const uint4 x = *reinterpret_cast<const uint4*>(row + tile_off(r & (CK_L - 1), c * 2 + (tid & 1), RB));
+        m = mag2(mag2(mag2(mag2(m, x.x), x.y), x.z), x.w);
+        ss += bf16lo(x.x) * bf16lo(x.x) + bf16hi(x.x) * bf16hi(x.x) + bf16lo(x.y) * bf16lo(x.y) + bf16hi(x.y) * bf16hi(x.y);
+        ss += bf16lo(x.z) * bf16lo(x.z) + bf16hi(x.z) * bf16hi(x.z) + bf16lo(x.w) * bf16lo(x.w) + bf16hi(x.w) * bf16hi(x.w);
+      }
+      ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+      if ((tid & 1) == 0) (r < CK_L ? sm.kn[r] : sm.qn[r - CK_L]) = (r < CK_L ? 1.0f : a.qscale) / sqrtf(ss + 1e-6f);
+      const uint4* v4 = reinterpret_cast<const uint4*>(sm.v[s]);
+      for (int i = tid; i < CK_L * CK_P / 8; i += THREADS) { const uint4 x = v4[i]; m = mag2(mag2(mag2(mag2(m, x.x), x.y), x.z), x.w); }
+      wild = (m & 0xffffu) >= CK_BIG_IN || (m >> 16) >= CK_BIG_IN;
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) wild = wild || !(fabsf(S[nt][e]) < CK_BIG_STATE);
+    }
+    if (warp == 0) {                                       // sums of the log decays
+      const bool fine = fabsf(cl[0]) < 1e30f && fabsf(cl[1]) < 1e30f && fabsf(cb_[0]) < 1e6f && fabsf(cb_[1]) < 1e6f;
+      double c1 = static_cast<double>(cl[0]) + cl[1], x;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        x = __shfl_up_sync(0xffffffffu, c1, o);
+        if (lane >= o) c1 += x;
+      }
+      double c0 = __shfl_up_sync(0xffffffffu, c1, 1);
+      c0 = (lane == 0 ? 0.0 : c0) + cl[0];
+      const double ce = __shfl_sync(0xffffffffu, c1, 31);
+      sm.cum[2 * lane] = c0; sm.cum[2 * lane + 1] = c1;
+      sm.ecum[2 * lane] = exp_sum(c0); sm.ecum[2 * lane + 1] = exp_sum(c1);
+      sm.beta[2 * lane] = cb_[0]; sm.beta[2 * lane + 1] = cb_[1];
+      sm.wl[2 * lane] = exp_sum(ce - c0); sm.wl[2 * lane + 1] = exp_sum(ce - c1);
+      wild = wild || !fine;
+    }
+    if (t0 + CK_L < len) { load_chunk(t0 + CK_L, s ^ 1); fetch_coef(t0 + CK_L); }
+    cp_async_commit();
+    if (__syncthreads_or(wild)) {
+      // ---- token by token: the same sums, every product in float
+      for (int i = 0; i < L; ++i) {
+        const float* c = cp + static_cast<size_t>(t0 + i) * H * 3;
+        const float c0 = c[0], c1 = c[1], kn = sm.kn[i];
+        float (*red)[2][CK_P] = sm.red[i & 1];
+        float x0 = 0.f, x1 = 0.f;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float kk = to_f(sm.k[s][tile_off(i, n0 / 8 + nt, RB) / 2 + c2 + e]);
+            S[nt][e] *= c0;     x0 += S[nt][e] * kk;
+            S[nt][e + 2] *= c0; x1 += S[nt][e + 2] * kk;
+          }
+#pragma unroll
+        for (int x = 1; x < 4; x <<= 1) { x0 += __shfl_xor_sync(0xffffffffu, x0, x); x1 += __shfl_xor_sync(0xffffffffu, x1, x); }
+        if ((lane & 3) == 0) { red[0][wh][pr] = x0; red[0][wh][pr + 8] = x1; }
+        __syncthreads();
+        const float v0 = to_f(sm.v[s][tile_off(i, pr >> 3, VB) / 2 + (pr & 7)]), v1 = to_f(sm.v[s][tile_off(i, (pr + 8) >> 3, VB) / 2 + (pr & 7)]);
+        const float w0 = c1 * (v0 - (red[0][0][pr] + red[0][1][pr]) * kn) * kn, w1 = c1 * (v1 - (red[0][0][pr + 8] + red[0][1][pr + 8]) * kn) * kn;
+        x0 = x1 = 0.f;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const uint32_t off = tile_off(i, n0 / 8 + nt, RB) / 2 + c2 + e;
+            const float kk = to_f(sm.k[s][off]), qq = to_f(sm.q[s][off]);
+            S[nt][e] += kk * w0;     x0 += S[nt][e] * qq;
+            S[nt][e + 2] += kk * w1; x1 += S[nt][e + 2] * qq;
+          }
+#pragma unroll
+        for (int x = 1; x < 4; x <<= 1) { x0 += __shfl_xor_sync(0xffffffffu, x0, x); x1 += __shfl_xor_sync(0xffffffffu, x1, x); }
+        if ((lane & 3) == 0) { red[1][wh][pr] = x0; red[1][wh][pr + 8] = x1; }
+        __syncthreads();
+        if (tid < CK_P) og[static_cast<size_t>(t0 + i) * H * dv + tid] = (red[1][0][tid] + red[1][1][tid]) * sm.qn[i];
+      }
+      continue;
+    }
+    const uint32_t q_u = smem_u32(sm.q[s]), k_u = smem_u32(sm.k[s]);
+    // ---- dot products of rows 16 wp .. + 15 with the keys up to the diagonal: of keys (wh 0) or of queries (wh 1)
+    if (wp * 16 < L) {
+      float sc[8][4];
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sc[nt][e] = 0.f;
+      const uint32_t x_u = wh ? q_u : k_u;
+#pragma unroll
+      for (int ks = 0; ks < D / 16; ++ks) {
+        uint32_t af[4];
+        ldsm4(af, x_u + tile_off(wp * 16 + ra, ks * 2 + ca, RB));
+#pragma unroll
+        for (int np = 0; np < 4; ++np) {
+          if (np <= wp) {
+            uint32_t bf[4];
+            ldsm4(bf, k_u + tile_off(np * 16 + rb, ks * 2 + cb, RB));
+            mma_add(sc[2 * np], af, bf[0], bf[1]);
+            mma_add(sc[2 * np + 1], af, bf[2], bf[3]);
+          }
+        }
+      }
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int i = wp * 16 + g4 + 8 * half;
+        const double ci = sm.cum[i];
+        const float fi = wh ? sm.qn[i] : sm.beta[i] * sm.kn[i];
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt) {
+          if (nt <= 2 * wp + 1) {
+            const int j = nt * 8 + c2;
+            const bool in0 = wh ? j <= i : j < i, in1 = wh ? j + 1 <= i : j + 1 < i;
+            const float x = in0 ? sc[nt][2 * half] * (exp_sum(ci - sm.cum[j]) * (fi * sm.kn[j])) : 0.f;
+            const float y = in1 ? sc[nt][2 * half + 1] * (exp_sum(ci - sm.cum[j + 1]) * (fi * sm.kn[j + 1])) : 0.f;
+            if (wh) {
+              uint32_t hi, mid, lo;
+              split3(x, y, hi, mid, lo);
+              const uint32_t off = (tile_off(i, nt, MB) + c2 * 2) / 4;
+              reinterpret_cast<uint32_t*>(sm.m[0])[off] = hi;
+              reinterpret_cast<uint32_t*>(sm.m[1])[off] = mid;
+              reinterpret_cast<uint32_t*>(sm.m[2])[off] = lo;
+            } else {
+              *reinterpret_cast<float2*>(sm.A + i * FS + j) = make_float2(x, y);
+            }
+          }
+        }
+      }
+    }
+    // ---- S^T k and S^T q over this half of the channels
+    float oq[8][4];
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) oq[nt][e] = 0.f;
+    const bool front = carried || t0 > 0;
+    {
+      float ok[8][4];
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) ok[nt][e] = 0.f;
+      if (front) {
+#pragma unroll
+        for (int pass = 0; pass < 2; ++pass)               // the small parts first
+#pragma unroll
+          for (int ks = 0; ks < CH / 16; ++ks) {
+            uint32_t hi[4], mid[4], lo[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) split3(S[2 * ks + (e >> 1)][2 * (e & 1)], S[2 * ks + (e >> 1)][2 * (e & 1) + 1], hi[e], mid[e], lo[e]);
+#pragma unroll
+            for (int np = 0; np < 4; ++np) {
+              if (np * 16 < L) {
+                uint32_t bk[4], bq[4];
+                ldsm4(bk, k_u + tile_off(np * 16 + rb, n0 / 8 + ks * 2 + cb, RB));
+                ldsm4(bq, q_u + tile_off(np * 16 + rb, n0 / 8 + ks * 2 + cb, RB));
+                if (pass == 0) {
+                  mma_bf16_16816(ok[2 * np], lo, bk[0], bk[1]);
+                  mma_bf16_16816(ok[2 * np + 1], lo, bk[2], bk[3]);
+                  mma_bf16_16816(oq[2 * np], lo, bq[0], bq[1]);
+                  mma_bf16_16816(oq[2 * np + 1], lo, bq[2], bq[3]);
+                  mma_bf16_16816(ok[2 * np], mid, bk[0], bk[1]);
+                  mma_bf16_16816(ok[2 * np + 1], mid, bk[2], bk[3]);
+                  mma_bf16_16816(oq[2 * np], mid, bq[0], bq[1]);
+                  mma_bf16_16816(oq[2 * np + 1], mid, bq[2], bq[3]);
+                } else {
+                  mma_add(ok[2 * np], hi, bk[0], bk[1]);
+                  mma_add(ok[2 * np + 1], hi, bk[2], bk[3]);
+                  mma_add(oq[2 * np], hi, bq[0], bq[1]);
+                  mma_add(oq[2 * np + 1], hi, bq[2], bq[3]);
+                }
+              }
+            }
+          }
+      }
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt) {
+        *reinterpret_cast<float2*>(sm.f[wh] + pr * FS + nt * 8 + c2) = make_float2(ok[nt][0], ok[nt][1]);
+        *reinterpret_cast<float2*>(sm.f[wh] + (pr + 8) * FS + nt * 8 + c2) = make_float2(ok[nt][2], ok[nt][3]);
+      }
+    }
+    __syncthreads();
+    // ---- the solve: four lanes per value column
+    {
+      const int col = warp * 8 + (lane >> 2), sub = lane & 3;
+      float r[CK_L / 4];
+#pragma unroll
+      for (int m = 0; m < CK_L / 4; ++m) {
+        const int i = 4 * m + sub;
+        const float v = to_f(sm.v[s][tile_off(i, col >> 3, VB) / 2 + (col & 7)]);
+        r[m] = i < L ? sm.beta[i] * (v - sm.ecum[i] * sm.kn[i] * (sm.f[0][col * FS + i] + sm.f[1][col * FS + i])) : 0.f;
+      }
+#pragma unroll
+      for (int m0 = 0; m0 < CK_L / 4; ++m0) {
+        if (4 * m0 < L) {
+          const float* d = sm.A + 4 * m0 * FS + 4 * m0;    // the 4 x 4 block on the diagonal
+          float u0 = __shfl_sync(0xffffffffu, r[m0], lane & ~3), u1 = __shfl_sync(0xffffffffu, r[m0], (lane & ~3) + 1);
+          float u2 = __shfl_sync(0xffffffffu, r[m0], (lane & ~3) + 2), u3 = __shfl_sync(0xffffffffu, r[m0], (lane & ~3) + 3);
+          u1 -= d[FS] * u0;
+          u2 -= d[2 * FS] * u0 + d[2 * FS + 1] * u1;
+          u3 -= d[3 * FS] * u0 + d[3 * FS + 1] * u1 + d[3 * FS + 2] * u2;
+          r[m0] = sub == 0 ? u0 : sub == 1 ? u1 : sub == 2 ? u2 : u3;
+#pragma unroll
+          for (int m = m0 + 1; m < CK_L / 4; ++m) {
+            const float4 x = *reinterpret_cast<const float4*>(sm.A + (4 * m + sub) * FS + 4 * m0);
+            if (4 * m < L) r[m] = r[m] - x.x * u0 - x.y * u1 - x.z * u2 - x.w * u3;
+          }
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < CK_L / 4; ++m) sm.f[0][col * FS + 4 * m + sub] = r[m];
+    }
+    __syncthreads();
+    // ---- the solution's part of the outputs (token blocks 0, 3 or 1, 2), beside this half's S^T q
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+      const int i = nt * 8 + c2;
+      const float e0 = sm.ecum[i] * sm.qn[i], e1 = sm.ecum[i + 1] * sm.qn[i + 1];
+      oq[nt][0] *= e0; oq[nt][1] *= e1; oq[nt][2] *= e0; oq[nt][3] *= e1;
+    }
+#pragma unroll
+    for (int jj = 0; jj < 2; ++jj) {
+      const int js = wh ? 1 + jj : 3 * jj;
+      if (js * 16 < L) {
+        uint32_t uf[3][4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 x = *reinterpret_cast<const float2*>(sm.f[0] + (pr + 8 * (e & 1)) * FS + js * 16 + (e >> 1) * 8 + c2);
+          split3(x.x, x.y, uf[0][e], uf[1][e], uf[2][e]);
+        }
+#pragma unroll
+        for (int np = 0; np < 4; ++np) {
+          if (np >= js && np * 16 < L) {
+            uint32_t b0[4], b1[4], b2[4];
+            const uint32_t off = tile_off(np * 16 + rb, js * 2 + cb, MB);
+            ldsm4(b0, m_u + off);
+            ldsm4(b1, m_u + CK_L * MB + off);
+            ldsm4(b2, m_u + 2 * CK_L * MB + off);
+#pragma unroll
+            for (int w = 0; w < 2; ++w) {
+              float t[4] = {0.f, 0.f, 0.f, 0.f};
+              mma_bf16_16816(t, uf[2], b0[2 * w], b0[2 * w + 1]);
+              mma_bf16_16816(t, uf[0], b2[2 * w], b2[2 * w + 1]);
+              mma_bf16_16816(t, uf[1], b1[2 * w], b1[2 * w + 1]);
+              mma_bf16_16816(t, uf[1], b0[2 * w], b0[2 * w + 1]);
+              mma_bf16_16816(t, uf[0], b1[2 * w], b1[2 * w + 1]);
+              mma_add(t, uf[0], b0[2 * w], b0[2 * w + 1]);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) oq[2 * np + w][e] += t[e];
+            }
+          }
+        }
+      }
+    }
+    // ---- the halves exchange: wh 0 finishes tokens 0 .. 31, wh 1 the others
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const float* y0 = wh ? oq[x] : oq[4 + x];
+      const int i = (wh ? x : 4 + x) * 8 + c2;
+      *reinterpret_cast<float2*>(sm.f[1] + pr * FS + i) = make_float2(y0[0], y0[1]);
+      *reinterpret_cast<float2*>(sm.f[1] + (pr + 8) * FS + i) = make_float2(y0[2], y0[3]);
+    }
+    // ---- the state behind the chunk, this half of the channels
+    {
+      uint32_t af[4][3][4];
+#pragma unroll
+      for (int js = 0; js < 4; ++js)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int j = js * 16 + (e >> 1) * 8 + c2;
+          const float2 x = *reinterpret_cast<const float2*>(sm.f[0] + (pr + 8 * (e & 1)) * FS + j);
+          split3(x.x * (sm.wl[j] * sm.kn[j]), x.y * (sm.wl[j + 1] * sm.kn[j + 1]), af[js][0][e], af[js][1][e], af[js][2][e]);
+        }
+      const float gl = sm.ecum[CK_L - 1];
+#pragma unroll
+      for (int np = 0; np < CH / 16; ++np) {
+        float t[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        uint32_t bf[4][4];
+#pragma unroll
+        for (int js = 0; js < 4; ++js)
+          if (js * 16 < L) ldsm4t(bf[js], k_u + tile_off(js * 16 + rt, n0 / 8 + np * 2 + ct, RB));
+#pragma unroll
+        for (int part = 2; part >= 0; --part)
+#pragma unroll
+          for (int js = 0; js < 4; ++js)
+            if (js * 16 < L) {
+              if (part > 0) {
+                mma_bf16_16816(t[0], af[js][part], bf[js][0], bf[js][1]);
+                mma_bf16_16816(t[1], af[js][part], bf[js][2], bf[js][3]);
+              } else {
+                mma_add(t[0], af[js][part], bf[js][0], bf[js][1]);
+                mma_add(t[1], af[js][part], bf[js][2], bf[js][3]);
+              }
+            }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          S[2 * np][e] = fmaf(gl, S[2 * np][e], t[0][e]);
+          S[2 * np + 1][e] = fmaf(gl, S[2 * np + 1][e], t[1][e]);
+        }
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const float* y0 = wh ? oq[4 + x] : oq[x];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = (wh ? 4 + x : x) * 8 + c2 + (e & 1), p = pr + 8 * (e >> 1);
+        if (i < L) og[static_cast<size_t>(t0 + i) * H * dv + p] = y0[e] + sm.f[1][p * FS + i];
+      }
+    }
+  }
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) Sg[static_cast<size_t>(n0 + nt * 8 + c2 + (e & 1)) * dv + pr + 8 * (e >> 1)] = S[nt][e];
+}
+
 bool scan_chunk_applies(const ScanArgs& a) {
   return (a.d == 64 || a.d == 128) && a.dv % CK_P == 0 && a.ldq % 8 == 0 && a.ldk % 8 == 0 && a.ldv % 8 == 0 && aligned16(a.q) &&
          aligned16(a.k) && aligned16(a.v) && a.head_decay == nullptr && !a.divide;
@@ -385,6 +792,20 @@ static int go_linear(const char* what, const ScanArgs& a, int n_seqs, cudaStream
 
 int launch_linear_chunk(const char* what, const ScanArgs& a, int n_seqs, cudaStream_t st) {
   return a.d == 64 ? go_linear<64>(what, a, n_seqs, st) : go_linear<128>(what, a, n_seqs, st);
+}
+
+template <int D>
+static int go_delta(const char* what, const ScanArgs& a, int n_seqs, cudaStream_t st) {
+  constexpr int smem = static_cast<int>(sizeof(DeltaTiles<D>));
+  const cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return cuda_fail(e, what);
+  delta_chunk_kernel<D><<<dim3(a.dv / CK_P, a.H, n_seqs), 256, smem, st>>>(a);
+  B2_CHECK_LAUNCH(what);
+  return B2TTS_OK;
+}
+
+int launch_delta_chunk(const char* what, const ScanArgs& a, int n_seqs, cudaStream_t st) {
+  return a.d == 64 ? go_delta<64>(what, a, n_seqs, st) : go_delta<128>(what, a, n_seqs, st);
 }
 
 }  // namespace row

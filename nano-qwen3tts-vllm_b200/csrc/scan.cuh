@@ -27,6 +27,7 @@ struct ScanArgs {
 // bf16 portions in chunks on the tensor cores: which sizes and layouts, and the launches (sequences with more than one token)
 bool scan_chunk_applies(const ScanArgs& a);
 int launch_linear_chunk(const char* what, const ScanArgs& a, int n_seqs, cudaStream_t st);
+int launch_delta_chunk(const char* what, const ScanArgs& a, int n_seqs, cudaStream_t st);
 
 }  // namespace row
 }  // namespace b2

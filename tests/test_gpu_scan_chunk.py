@@ -119,3 +119,92 @@ def test_state_space_numbers_outside_the_split(nat, value):
             assert not torch.isfinite(got[70:, 1, 5]).any() and not torch.isfinite(state[1, :, 5]).any()
         else:
             assert bool(((got - y).abs()[70:, 1, 5] <= 1e-4 * ya[70:, 1, 5]).all())
+
+
+# ------------------------------------------------------------------------------------------------ delta rule
+def _delta_reference(q, k, v, beta, la, S):
+    unit = lambda t: t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6)
+    n, H, P = v.shape
+    rep = H // q.shape[1]
+    q, k = unit(q) * q.shape[-1] ** -0.5, unit(k)
+    ys = []
+    for t in range(n):
+        kt, qt = k[t].repeat_interleave(rep, 0), q[t].repeat_interleave(rep, 0)
+        S = torch.exp(la[t])[:, None, None] * S
+        u = beta[t][:, None] * (v[t] - torch.einsum("hdp,hd->hp", S, kt))
+        S = S + kt[:, :, None] * u[:, None, :]
+        ys.append(torch.einsum("hdp,hd->hp", S, qt))
+    return torch.stack(ys), S
+
+
+def _delta_case(nat, seqs, H, G, D, P, seed=0, a_log=None, alike=0.0, big=None):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    r = lambda *s: torch.randn(s, generator=g, device=DEV)
+    lay = Lay(seqs)
+    n = lay.n_tokens
+    qkv = r(n, 2 * G * D + H * P)
+    qkv[:, G * D:2 * G * D] += alike * r(1, G * D)             # keys that point the same way: the solve's off-diagonal is dense
+    qkv, ba = qkv.to(torch.bfloat16), r(n, 2 * H).to(torch.bfloat16)
+    if big is not None:
+        row, col, value = big
+        qkv[row, col] = value
+    a_log = 0.5 * r(H) - 0.5 if a_log is None else torch.full((H,), a_log, device=DEV)
+    dt_bias = 0.5 * r(H)
+    slots = max(s[2] for s in seqs) + 2
+    state = r(slots, H, D, P)
+    before, out = state.clone(), torch.full((n, H * P), 3.0, device=DEV)
+    nat.delta_rule_scan(qkv, ba[:, :H], ba[:, H:], a_log, dt_bias, state, out, lay, H, G, D, P)
+    beta = torch.sigmoid(ba[:, :H].to(F64))
+    la = -torch.exp(a_log.to(F64)) * torch.nn.functional.softplus(ba[:, H:].float() + dt_bias).to(F64)
+    for (pos0, m, slot), o in zip(seqs, lay.starts):
+        if m == 0:
+            continue
+        e = slice(o, o + m)
+        X = qkv[e].to(F64)
+        S0 = before[slot].to(F64) if pos0 else torch.zeros(H, D, P, dtype=F64, device=DEV)
+        y, S = _delta_reference(X[:, :G * D].view(m, G, D), X[:, G * D:2 * G * D].view(m, G, D), X[:, 2 * G * D:].view(m, H, P), beta[e], la[e], S0)
+        yield out[e].view(m, H, P).to(F64), state[slot].to(F64), y, S
+    used = {s[2] for s in seqs if s[1]}
+    for slot in range(slots):
+        if slot not in used:
+            assert torch.equal(state[slot], before[slot])
+
+
+def _check_delta(got, state, y, S, m):
+    """A write moves the state by a contraction, so roundings add up: a few hundred per token's sums at first (128 terms, three of
+    them), a few per token afterwards, relative to the largest numbers of the state; an output adds 128 of them, scaled by 128^-0.5."""
+    u = 2.0 ** -24 * (512 + 8 * m) * max(S.abs().max().item(), 1.0)
+    assert (got - y).abs().max().item() <= u and (state - S).abs().max().item() <= u, ((got - y).abs().max().item(), (state - S).abs().max().item(), u)
+
+
+@pytest.mark.parametrize("D,P,H,G", [(128, 64, 2, 1), (64, 128, 4, 2)])
+@pytest.mark.parametrize("n", [2, 3, 15, 16, 17, 63, 64, 65, 128, 131, 200])
+def test_delta_rule_portion_lengths(nat, D, P, H, G, n):
+    for case in _delta_case(nat, [(0, n, 1), (9, n, 0)], H, G, D, P, seed=n):
+        _check_delta(*case, n)
+
+
+def test_delta_rule_portions_beside_single_tokens_and_padding(nat):
+    seqs = [(5, 1, 3), (0, 70, 0), (0, 0, 1), (0, 1, 4), (800, 3, 2)]
+    for case, (_, m, _) in zip(_delta_case(nat, seqs, 2, 2, 128, 128, seed=5), [s for s in seqs if s[1]]):
+        _check_delta(*case, m)
+
+
+@pytest.mark.parametrize("a_log,alike", [(-30.0, 0.0), (6.0, 0.0), (-30.0, 4.0), (-30.0, 100.0)])
+def test_delta_rule_extreme_decays_and_keys_that_point_the_same_way(nat, a_log, alike):
+    for case in _delta_case(nat, [(7, 150, 0)], 2, 1, 128, 64, seed=1, a_log=a_log, alike=alike):
+        _check_delta(*case, 150)
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), 1e30])
+def test_delta_rule_values_outside_the_split(nat, value):
+    """A value's column of its head is lost from its token on; everything else keeps its numbers."""
+    col = 2 * 128 + 64 + 5                                     # value column 5 of head 1
+    for got, state, y, S in _delta_case(nat, [(3, 100, 0)], 2, 1, 128, 64, seed=2, big=(70, col, value)):
+        hit, lost = torch.zeros_like(y, dtype=torch.bool), torch.zeros_like(S, dtype=torch.bool)
+        hit[70:, 1, 5] = lost[1, :, 5] = True
+        _check_delta(got.masked_fill(hit, 0.0), state.masked_fill(lost, 0.0), y.masked_fill(hit, 0.0), S.masked_fill(lost, 0.0), 100)
+        if value != 1e30:
+            assert not torch.isfinite(got[70:, 1, 5]).any()
+        else:
+            assert bool(((got - y)[70:, 1, 5].abs() <= 1e-4 * y[70:, 1, 5].abs().max()).all())
