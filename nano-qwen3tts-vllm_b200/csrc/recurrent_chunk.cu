@@ -385,12 +385,12 @@ template <int D> struct DeltaTiles {
   static constexpr int FS = CK_L + 4;       // padded float rows: a warp's quads fall into distinct banks
   __nv_bfloat16 q[2][CK_L * D], k[2][CK_L * D], v[2][CK_L * CK_P];
   __nv_bfloat16 m[3][CK_L * CK_L];          // e^(c_i - c_j) (q^_i . k^_j) in three parts
-  float A[CK_L * FS];
+  float A[CK_L * FS], E[CK_L * FS];         // E: e^(c_i - c_j), j <= i
   float f[2][CK_P * FS];                    // [value column][token]: S^T k of the two halves, then u | the exchanged half of o
-  double cum[CK_L];
-  float ecum[CK_L], beta[CK_L], wl[CK_L], kn[CK_L], qn[CK_L];
+  double cum[2][CK_L];
+  float ecum[2][CK_L], beta[2][CK_L], wl[2][CK_L], kn[CK_L], qn[CK_L];
   float red[2][2][2][CK_P];                 // token by token: [parity][k or q][half][value column]
-  int wild;
+  int wild[2];
 };
 
 template <int D>
@@ -436,17 +436,39 @@ delta_chunk_kernel(const ScanArgs a) {
   for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
     for (int e = 0; e < 4; ++e) S[nt][e] = carried ? Sg[static_cast<size_t>(n0 + nt * 8 + c2 + (e & 1)) * dv + pr + 8 * (e >> 1)] : 0.f;
-  // scalars of a chunk (warp 0: lane l holds tokens 2 l, 2 l + 1), fetched a chunk ahead
+  // scalars of a chunk (warp 1: lane l holds tokens 2 l, 2 l + 1), fetched two chunks ahead and summed one ahead
   float cl[2], cb_[2];
   auto fetch_coef = [&](int t0) {
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int t = t0 + 2 * lane + e;
       cl[e] = cb_[e] = 0.f;
-      if (warp == 0 && t < len) { cb_[e] = cp[static_cast<size_t>(t) * H * 3 + 1]; cl[e] = cp[static_cast<size_t>(t) * H * 3 + 2]; }
+      if (t < len) { cb_[e] = cp[static_cast<size_t>(t) * H * 3 + 1]; cl[e] = cp[static_cast<size_t>(t) * H * 3 + 2]; }
     }
   };
-  fetch_coef(0);
+  auto sum_coef = [&](int s) {
+    const bool fine = fabsf(cl[0]) < 1e30f && fabsf(cl[1]) < 1e30f && fabsf(cb_[0]) < 1e6f && fabsf(cb_[1]) < 1e6f;
+    double c1 = static_cast<double>(cl[0]) + cl[1], x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      x = __shfl_up_sync(0xffffffffu, c1, o);
+      if (lane >= o) c1 += x;
+    }
+    double c0 = __shfl_up_sync(0xffffffffu, c1, 1);
+    c0 = (lane == 0 ? 0.0 : c0) + cl[0];
+    const double ce = __shfl_sync(0xffffffffu, c1, 31);
+    sm.cum[s][2 * lane] = c0; sm.cum[s][2 * lane + 1] = c1;
+    sm.ecum[s][2 * lane] = exp_sum(c0); sm.ecum[s][2 * lane + 1] = exp_sum(c1);
+    sm.beta[s][2 * lane] = cb_[0]; sm.beta[s][2 * lane + 1] = cb_[1];
+    sm.wl[s][2 * lane] = exp_sum(ce - c0); sm.wl[s][2 * lane + 1] = exp_sum(ce - c1);
+    const bool all = __all_sync(0xffffffffu, fine);
+    if (lane == 0) sm.wild[s] = !all;
+  };
+  if (warp == 1) {
+    fetch_coef(0);
+    sum_coef(0);
+    fetch_coef(CK_L);
+  }
   const uint32_t m_u = smem_u32(sm.m);
   const int ra = lane & 15, ca = lane >> 4;
   const int rb = (lane >> 4) * 8 + (lane & 7), cb = (lane >> 3) & 1;
@@ -479,24 +501,18 @@ delta_chunk_kernel(const ScanArgs a) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) wild = wild || !(fabsf(S[nt][e]) < CK_BIG_STATE);
     }
-    if (warp == 0) {                                       // sums of the log decays
-      const bool fine = fabsf(cl[0]) < 1e30f && fabsf(cl[1]) < 1e30f && fabsf(cb_[0]) < 1e6f && fabsf(cb_[1]) < 1e6f;
-      double c1 = static_cast<double>(cl[0]) + cl[1], x;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        x = __shfl_up_sync(0xffffffffu, c1, o);
-        if (lane >= o) c1 += x;
+    // ---- decays between the chunk's tokens: rows x and 63 - x together have as many for every x
+    {
+      const int x = tid >> 3, sub = tid & 7;
+#pragma unroll 2
+      for (int n = 0; n < 2; ++n) {
+        const int i = n ? CK_L - 1 - x : x;
+        const double ci = sm.cum[s][i];
+        for (int j = sub; j <= i; j += 8) sm.E[i * FS + j] = exp_sum(ci - sm.cum[s][j]);
       }
-      double c0 = __shfl_up_sync(0xffffffffu, c1, 1);
-      c0 = (lane == 0 ? 0.0 : c0) + cl[0];
-      const double ce = __shfl_sync(0xffffffffu, c1, 31);
-      sm.cum[2 * lane] = c0; sm.cum[2 * lane + 1] = c1;
-      sm.ecum[2 * lane] = exp_sum(c0); sm.ecum[2 * lane + 1] = exp_sum(c1);
-      sm.beta[2 * lane] = cb_[0]; sm.beta[2 * lane + 1] = cb_[1];
-      sm.wl[2 * lane] = exp_sum(ce - c0); sm.wl[2 * lane + 1] = exp_sum(ce - c1);
-      wild = wild || !fine;
+      wild = wild || sm.wild[s];
     }
-    if (t0 + CK_L < len) { load_chunk(t0 + CK_L, s ^ 1); fetch_coef(t0 + CK_L); }
+    if (t0 + CK_L < len) load_chunk(t0 + CK_L, s ^ 1);
     cp_async_commit();
     if (__syncthreads_or(wild)) {
       // ---- token by token: the same sums, every product in float
@@ -535,47 +551,53 @@ delta_chunk_kernel(const ScanArgs a) {
         __syncthreads();
         if (tid < CK_P) og[static_cast<size_t>(t0 + i) * H * dv + tid] = (red[1][0][tid] + red[1][1][tid]) * sm.qn[i];
       }
+      if (warp == 1) {
+        sum_coef(s ^ 1);
+        fetch_coef(t0 + 2 * CK_L);
+      }
       continue;
     }
     const uint32_t q_u = smem_u32(sm.q[s]), k_u = smem_u32(sm.k[s]);
-    // ---- dot products of rows 16 wp .. + 15 with the keys up to the diagonal: of keys (wh 0) or of queries (wh 1)
-    if (wp * 16 < L) {
-      float sc[8][4];
-#pragma unroll
-      for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) sc[nt][e] = 0.f;
+    // ---- dot products of the keys (wh 0) or the queries (wh 1) with the keys up to the diagonal, in 16 x 16 blocks: rows and first
+    // column block of this warp's two or three
+    if (warp == 1) {
+      sum_coef(s ^ 1);                                     // warps 1, 3, 5, 7 have two blocks
+      fetch_coef(t0 + 2 * CK_L);
+    }
+    {
+      const int br = wp == 0 ? 3 : wp == 1 ? 3 : wp == 2 ? 2 : 1, b0 = wp == 1 ? 2 : 0;
       const uint32_t x_u = wh ? q_u : k_u;
 #pragma unroll
-      for (int ks = 0; ks < D / 16; ++ks) {
-        uint32_t af[4];
-        ldsm4(af, x_u + tile_off(wp * 16 + ra, ks * 2 + ca, RB));
+      for (int n = 0; n < 3; ++n) {
+        const bool extra = wp == 0 && n == 2;              // warp 0's third block is the first one on the diagonal
+        if (n == 2 && (wp & 1)) break;
+        const int rblk = extra ? 0 : br, cblk = extra ? 0 : b0 + n;
+        float sc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        uint32_t af[D / 16][4], bf[D / 16][4];
 #pragma unroll
-        for (int np = 0; np < 4; ++np) {
-          if (np <= wp) {
-            uint32_t bf[4];
-            ldsm4(bf, k_u + tile_off(np * 16 + rb, ks * 2 + cb, RB));
-            mma_add(sc[2 * np], af, bf[0], bf[1]);
-            mma_add(sc[2 * np + 1], af, bf[2], bf[3]);
-          }
+        for (int ks = 0; ks < D / 16; ++ks) {
+          ldsm4(af[ks], x_u + tile_off(rblk * 16 + ra, ks * 2 + ca, RB));
+          ldsm4(bf[ks], k_u + tile_off(cblk * 16 + rb, ks * 2 + cb, RB));
         }
-      }
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int i = wp * 16 + g4 + 8 * half;
-        const double ci = sm.cum[i];
-        const float fi = wh ? sm.qn[i] : sm.beta[i] * sm.kn[i];
+        for (int ks = 0; ks < D / 16; ++ks) {
+          mma_add(sc[0], af[ks], bf[ks][0], bf[ks][1]);
+          mma_add(sc[1], af[ks], bf[ks][2], bf[ks][3]);
+        }
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-          if (nt <= 2 * wp + 1) {
-            const int j = nt * 8 + c2;
+        for (int half = 0; half < 2; ++half) {
+          const int i = rblk * 16 + g4 + 8 * half;
+          const float fi = wh ? sm.qn[i] : sm.beta[s][i] * sm.kn[i];
+#pragma unroll
+          for (int w = 0; w < 2; ++w) {
+            const int j = cblk * 16 + w * 8 + c2;
+            const float2 e2 = *reinterpret_cast<const float2*>(sm.E + i * FS + j), k2 = *reinterpret_cast<const float2*>(sm.kn + j);
             const bool in0 = wh ? j <= i : j < i, in1 = wh ? j + 1 <= i : j + 1 < i;
-            const float x = in0 ? sc[nt][2 * half] * (exp_sum(ci - sm.cum[j]) * (fi * sm.kn[j])) : 0.f;
-            const float y = in1 ? sc[nt][2 * half + 1] * (exp_sum(ci - sm.cum[j + 1]) * (fi * sm.kn[j + 1])) : 0.f;
+            const float x = in0 ? sc[w][2 * half] * (e2.x * (fi * k2.x)) : 0.f, y = in1 ? sc[w][2 * half + 1] * (e2.y * (fi * k2.y)) : 0.f;
             if (wh) {
               uint32_t hi, mid, lo;
               split3(x, y, hi, mid, lo);
-              const uint32_t off = (tile_off(i, nt, MB) + c2 * 2) / 4;
+              const uint32_t off = (tile_off(i, cblk * 2 + w, MB) + c2 * 2) / 4;
               reinterpret_cast<uint32_t*>(sm.m[0])[off] = hi;
               reinterpret_cast<uint32_t*>(sm.m[1])[off] = mid;
               reinterpret_cast<uint32_t*>(sm.m[2])[off] = lo;
@@ -647,23 +669,24 @@ delta_chunk_kernel(const ScanArgs a) {
       for (int m = 0; m < CK_L / 4; ++m) {
         const int i = 4 * m + sub;
         const float v = to_f(sm.v[s][tile_off(i, col >> 3, VB) / 2 + (col & 7)]);
-        r[m] = i < L ? sm.beta[i] * (v - sm.ecum[i] * sm.kn[i] * (sm.f[0][col * FS + i] + sm.f[1][col * FS + i])) : 0.f;
+        r[m] = sm.beta[s][i] * (v - sm.ecum[s][i] * sm.kn[i] * (sm.f[0][col * FS + i] + sm.f[1][col * FS + i]));   // 0 behind the portion's end
       }
 #pragma unroll
       for (int m0 = 0; m0 < CK_L / 4; ++m0) {
-        if (4 * m0 < L) {
-          const float* d = sm.A + 4 * m0 * FS + 4 * m0;    // the 4 x 4 block on the diagonal
-          float u0 = __shfl_sync(0xffffffffu, r[m0], lane & ~3), u1 = __shfl_sync(0xffffffffu, r[m0], (lane & ~3) + 1);
-          float u2 = __shfl_sync(0xffffffffu, r[m0], (lane & ~3) + 2), u3 = __shfl_sync(0xffffffffu, r[m0], (lane & ~3) + 3);
-          u1 -= d[FS] * u0;
-          u2 -= d[2 * FS] * u0 + d[2 * FS + 1] * u1;
-          u3 -= d[3 * FS] * u0 + d[3 * FS + 1] * u1 + d[3 * FS + 2] * u2;
-          r[m0] = sub == 0 ? u0 : sub == 1 ? u1 : sub == 2 ? u2 : u3;
+        const float* d = sm.A + 4 * m0 * FS + 4 * m0;      // the 4 x 4 block on the diagonal
+        const float d10 = d[FS], d20 = d[2 * FS], d21 = d[2 * FS + 1], d30 = d[3 * FS], d31 = d[3 * FS + 1], d32 = d[3 * FS + 2];
+        const float u0 = __shfl_sync(0xffffffffu, r[m0], lane & ~3);
+        float u1 = __shfl_sync(0xffffffffu, r[m0], (lane & ~3) + 1), u2 = __shfl_sync(0xffffffffu, r[m0], (lane & ~3) + 2);
+        float u3 = __shfl_sync(0xffffffffu, r[m0], (lane & ~3) + 3);
+        u1 -= d10 * u0;
+        u2 -= d20 * u0; u3 -= d30 * u0;
+        u2 -= d21 * u1; u3 -= d31 * u1;
+        u3 -= d32 * u2;
+        r[m0] = sub == 0 ? u0 : sub == 1 ? u1 : sub == 2 ? u2 : u3;
 #pragma unroll
-          for (int m = m0 + 1; m < CK_L / 4; ++m) {
-            const float4 x = *reinterpret_cast<const float4*>(sm.A + (4 * m + sub) * FS + 4 * m0);
-            if (4 * m < L) r[m] = r[m] - x.x * u0 - x.y * u1 - x.z * u2 - x.w * u3;
-          }
+        for (int m = m0 + 1; m < CK_L / 4; ++m) {
+          const float4 x = *reinterpret_cast<const float4*>(sm.A + (4 * m + sub) * FS + 4 * m0);
+          r[m] = r[m] - x.x * u0 - x.y * u1 - x.z * u2 - x.w * u3;
         }
       }
 #pragma unroll
@@ -674,7 +697,7 @@ delta_chunk_kernel(const ScanArgs a) {
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt) {
       const int i = nt * 8 + c2;
-      const float e0 = sm.ecum[i] * sm.qn[i], e1 = sm.ecum[i + 1] * sm.qn[i + 1];
+      const float e0 = sm.ecum[s][i] * sm.qn[i], e1 = sm.ecum[s][i + 1] * sm.qn[i + 1];
       oq[nt][0] *= e0; oq[nt][1] *= e1; oq[nt][2] *= e0; oq[nt][3] *= e1;
     }
 #pragma unroll
@@ -728,9 +751,9 @@ delta_chunk_kernel(const ScanArgs a) {
         for (int e = 0; e < 4; ++e) {
           const int j = js * 16 + (e >> 1) * 8 + c2;
           const float2 x = *reinterpret_cast<const float2*>(sm.f[0] + (pr + 8 * (e & 1)) * FS + j);
-          split3(x.x * (sm.wl[j] * sm.kn[j]), x.y * (sm.wl[j + 1] * sm.kn[j + 1]), af[js][0][e], af[js][1][e], af[js][2][e]);
+          split3(x.x * (sm.wl[s][j] * sm.kn[j]), x.y * (sm.wl[s][j + 1] * sm.kn[j + 1]), af[js][0][e], af[js][1][e], af[js][2][e]);
         }
-      const float gl = sm.ecum[CK_L - 1];
+      const float gl = sm.ecum[s][CK_L - 1];
 #pragma unroll
       for (int np = 0; np < CH / 16; ++np) {
         float t[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
