@@ -1,6 +1,5 @@
 """The streaming row kernels at the edges of their runs and vectors: the causal convolution against a 64-bit one (runs of eight tokens, carried rows,
-filters off a 16-byte boundary) and the gated group norm around the vectors a thread
-keeps."""
+filters off a 16-byte boundary), the gated group norm around the vectors a thread keeps, the squared ReLU around its vectors."""
 import pytest
 import torch
 
@@ -56,3 +55,14 @@ def test_gated_group_norm(nat, dtype, cols, groups, act, first, gate):
     v = (y.to(F64) * (gg if first else 1.0)).view(5, groups, -1)
     ref = (v * (v.square().mean(-1, keepdim=True) + 1e-5).rsqrt()).view(5, cols) * w.to(F64) * (1.0 if first else gg)
     assert ((out.to(F64) - ref).abs() <= 1e-5 + ref.abs() * (2 ** -8 if dtype == BF else 1e-5)).all()
+
+
+@pytest.mark.parametrize("dtype", [BF, torch.float32])
+@pytest.mark.parametrize("n", [1, 4, 7, 8, 2047, 2048, 2056, 8192, 8200, 100008])
+@pytest.mark.parametrize("off", [0, 1])
+def test_squared_relu(nat, dtype, n, off):
+    y = torch.randn(n + off + 8, device=DEV).to(dtype)
+    ref = y.clone()
+    ref[off:off + n] = y[off:off + n].float().clamp_min(0).square().to(dtype)
+    nat.relu_sq_(y[off:off + n])
+    assert torch.equal(y, ref)
