@@ -274,26 +274,54 @@ static void launch_sink_plain_rep(int rep, cudaStream_t st, const void* q, const
 }
 
 // ------------------------------------------------------------------ one-token rows: the lanes split a cached row
-// One CTA of eight warps per (sequence with ONE new token, REP query heads of a key/value group).  LPK lanes read one key
+// One CTA of WARPS warps per (sequence with ONE new token, REP query heads of a key/value group).  LPK lanes read one key
 // row, 16 bytes each (N elements; d = dv = LPK * N), so a warp-wide load is contiguous and covers 32 / LPK keys; a lane
 // keeps its slice of the REP queries (times scale * log2 e) and of the REP accumulators in registers.  Four key steps
-// (K and V pieces of four keys per lane group) are in flight before the first is used.  A score is the slice's dot product
-// summed over the LPK lanes by shuffles; every lane group keeps a running maximum and denominator per head (base 2), the
-// groups of a warp are merged by shuffles and the warps through shared memory, where the sink joins the denominator.
+// (K and V pieces of four keys per lane group) are in flight before the first is used, and the block-table entries of the next
+// four are asked for meanwhile.
+//
+// The 4 REP partial scores of a lane are summed over the LPK lanes by halves: at each shuffle distance a lane keeps one half of
+// them and sends the other, so a lane ends with ONE score (4 REP / LPK of them where there are more scores than lanes), and the
+// cap, the running maximum and the exponential are formed once a score, not once a score and lane; the weights then go back to
+// all lanes.  The lanes of a head keep its running maximum and their part of its denominator (base 2).  The lane groups of a warp
+// are merged by shuffles and the warps through shared memory, where the sink joins the denominator.
+// What bounds it: instructions (about 300 a lane for four keys and two heads) above the traffic of the rows.  64 sequences of 1100 keys, 8
+// key heads of 128, 2 heads each, capped: 133 -> 80 us (44 at the copy rate); with a score's cap and exponential on every lane it ran twice
+// the instructions, and eight-warp CTAs made 1.7 waves of that grid.
 // Values may be VR = 1 or 2 times as wide as keys (dv = VR * d): a lane then takes VR 16-byte pieces of a value row, LPK
 // pieces apart, so that the warp's loads stay contiguous.
-constexpr int SD_WARPS = 8, SD_AHEAD = 4;
+constexpr int SD_AHEAD = 4;
 
-template <typename T, int LPK, int REP, int VR>
-__global__ void __launch_bounds__(SD_WARPS * 32)
+// v[0 .. L) summed over the lanes that differ in the bits below 2 * O; a lane is left with its own share of them in front
+template <int L, int O>
+__device__ __forceinline__ void scatter_sum(float* v, int lane) {
+  if constexpr (O > 0) {
+    if constexpr (L > 1) {
+      const bool hi = lane & O;
+#pragma unroll
+      for (int k = 0; k < L / 2; ++k) {
+        const float send = hi ? v[k] : v[k + L / 2], keep = hi ? v[k + L / 2] : v[k];
+        v[k] = keep + __shfl_xor_sync(0xffffffffu, send, O);
+      }
+      scatter_sum<L / 2, O / 2>(v, lane);
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], O);
+      scatter_sum<1, O / 2>(v, lane);
+    }
+  }
+}
+
+template <typename T, int LPK, int REP, int VR, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, (REP * VR > 2 ? 8 : 16) / WARPS)
 sink_attn_decode_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache, T* __restrict__ out,
                         const int32_t* __restrict__ seq_start, const int32_t* __restrict__ seq_pos0,
                         const int32_t* __restrict__ seq_len, const int32_t* __restrict__ block_tables, int64_t bt_stride,
                         const float* __restrict__ sink, const T* __restrict__ gate, int64_t ldg, int gate_el, int H, int G, int Gv, int page,
                         int mask_kind, int mask, int keep_first, float softcap, float scale, int out_f32) {
   constexpr int N = Vec16<T>::N, D = LPK * N, DV = D * VR, KPW = 32 / LPK;
+  constexpr int S = SD_AHEAD * REP, OWN = S < LPK ? 1 : S / LPK, DUP = S < LPK ? LPK / S : 1;   // score r * SD_AHEAD + u: lane (. / OWN) * DUP
   constexpr float LOG2E = 1.4426950408889634f;
-  __shared__ float part[SD_WARPS][REP][DV + 2];
+  __shared__ float part[WARPS][REP][DV + 2];
   // the head groups of a sequence are neighbours in launch order: key heads that share a value head (v_heads < kv_heads)
   // run at the same time and the second reader finds the value rows in L2
   const int b = blockIdx.y;
@@ -311,7 +339,7 @@ sink_attn_decode_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, 
   const int gv = g % Gv;
   const int npre = min(keep_first, lo), n_keys = npre + i - lo + 1;    // kept first keys the mask hides, then [lo, i]
   const float cap2 = softcap * LOG2E;                      // the cap in the base-2 domain the scores live in
-  float qv[REP][N], acc[REP][VR * N], m[REP], l[REP];
+  float qv[REP][N], acc[REP][VR * N], m_own = -1e30f, l_own = 0.f;
 #pragma unroll
   for (int r = 0; r < REP; ++r) {
     const T* qr = q + (t * H + h0 + r) * D + sub * N;
@@ -319,7 +347,6 @@ sink_attn_decode_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, 
     for (int e = 0; e < N; ++e) qv[r][e] = to_f(qr[e]) * (scale * LOG2E);
 #pragma unroll
     for (int e = 0; e < VR * N; ++e) acc[r][e] = 0.f;
-    m[r] = -1e30f; l[r] = 0.f;
   }
   auto unpack = [](const uint4& raw, float* f) {
     if constexpr (N == 8) {
@@ -329,27 +356,42 @@ sink_attn_decode_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, 
       f[0] = __uint_as_float(raw.x); f[1] = __uint_as_float(raw.y); f[2] = __uint_as_float(raw.z); f[3] = __uint_as_float(raw.w);
     }
   };
-  constexpr int STEP = SD_WARPS * KPW;                     // keys the CTA takes per step
-  for (int j0 = 0; j0 < n_keys; j0 += STEP * SD_AHEAD) {
-    uint4 kraw[SD_AHEAD], vraw[SD_AHEAD][VR];
-    bool ok[SD_AHEAD];
+  constexpr int STEP = WARPS * KPW;                        // keys the CTA takes per step
+  const int shift = (page & (page - 1)) == 0 ? __ffs(page) - 1 : -1;
+  const int first = warp * KPW + kg;
+  auto split = [&](int vi, int& pg, int& off) {            // the page of the vi-th visible key and its row there
+    const int j = vi < npre ? vi : lo + vi - npre;
+    pg = shift >= 0 ? j >> shift : j / page;
+    off = j - pg * page;
+  };
+  int blk[SD_AHEAD], off[SD_AHEAD];
+  auto lookup = [&](int j0) {
 #pragma unroll
     for (int u = 0; u < SD_AHEAD; ++u) {
-      const int vi = j0 + u * STEP + warp * KPW + kg;
-      const int j = vi < npre ? vi : lo + vi - npre;
-      ok[u] = vi < n_keys;
-      kraw[u] = make_uint4(0, 0, 0, 0);
-#pragma unroll
-      for (int p = 0; p < VR; ++p) vraw[u][p] = make_uint4(0, 0, 0, 0);
-      if (ok[u]) {
-        const int pg = j / page;
-        const size_t slot = static_cast<size_t>(bt[pg]) * page + (j - pg * page);
-        kraw[u] = ldg_v4(k_cache + slot * row + g * D + sub * N);
-#pragma unroll
-        for (int p = 0; p < VR; ++p) vraw[u][p] = ldg_v4(v_cache + slot * vrow + gv * DV + (p * LPK + sub) * N);
+      const int vi = j0 + u * STEP + first;
+      blk[u] = 0; off[u] = 0;
+      if (vi < n_keys) {
+        int pg;
+        split(vi, pg, off[u]);
+        blk[u] = bt[pg];
       }
     }
-    float sc[SD_AHEAD][REP];
+  };
+  lookup(0);
+  const int own = sub / DUP * OWN;                          // the lane's first score: head own / SD_AHEAD, step own % SD_AHEAD
+  for (int j0 = 0; j0 < n_keys; j0 += STEP * SD_AHEAD) {
+    uint4 kraw[SD_AHEAD], vraw[SD_AHEAD][VR];
+#pragma unroll
+    for (int u = 0; u < SD_AHEAD; ++u) {
+      const bool ok = j0 + u * STEP + first < n_keys;
+      const size_t slot = static_cast<size_t>(blk[u]) * page + off[u];
+      kraw[u] = ok ? ldg_v4(k_cache + slot * row + g * D + sub * N) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int p = 0; p < VR; ++p)
+        vraw[u][p] = ok ? ldg_v4(v_cache + slot * vrow + gv * DV + (p * LPK + sub) * N) : make_uint4(0, 0, 0, 0);
+    }
+    lookup(j0 + STEP * SD_AHEAD);
+    float sc[S];
 #pragma unroll
     for (int u = 0; u < SD_AHEAD; ++u) {
       float f[N];
@@ -359,30 +401,39 @@ sink_attn_decode_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, 
         float s = 0.f;
 #pragma unroll
         for (int e = 0; e < N; ++e) s += f[e] * qv[r][e];
-#pragma unroll
-        for (int o = LPK / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (softcap > 0.f) s = cap2 * tanhf(s / cap2);
-        sc[u][r] = ok[u] ? s : -INFINITY;
+        sc[r * SD_AHEAD + u] = s;
       }
     }
+    scatter_sum<S, LPK / 2>(sc, lane);
+    float mx = -INFINITY;
+#pragma unroll
+    for (int k = 0; k < OWN; ++k) {
+      if (softcap > 0.f) sc[k] = cap2 * tanhf(sc[k] / cap2);
+      if (j0 + ((own + k) % SD_AHEAD) * STEP + first >= n_keys) sc[k] = -INFINITY;
+      mx = fmaxf(mx, sc[k]);
+    }
+#pragma unroll
+    for (int o = DUP; o < DUP * SD_AHEAD / OWN; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    const float m_new = fmaxf(m_own, mx);                  // finite: m starts finite
+    const float corr_own = exp2f(m_own - m_new);
+    m_own = m_new;
+    l_own *= corr_own;
+#pragma unroll
+    for (int k = 0; k < OWN; ++k) {
+      sc[k] = exp2f(sc[k] - m_new);
+      l_own += sc[k];
+    }
+    float w[S];
+#pragma unroll
+    for (int n = 0; n < S; ++n) w[n] = __shfl_sync(0xffffffffu, sc[n % OWN], n / OWN * DUP, LPK);
 #pragma unroll
     for (int r = 0; r < REP; ++r) {
-      float mx = sc[0][r];
-#pragma unroll
-      for (int u = 1; u < SD_AHEAD; ++u) mx = fmaxf(mx, sc[u][r]);
-      const float m_new = fmaxf(m[r], mx);                 // finite: m starts finite
-      const float corr = exp2f(m[r] - m_new);
-      m[r] = m_new;
-      l[r] *= corr;
+      const float corr = __shfl_sync(0xffffffffu, corr_own, r * SD_AHEAD / OWN * DUP, LPK);
 #pragma unroll
       for (int e = 0; e < VR * N; ++e) acc[r][e] *= corr;
-#pragma unroll
-      for (int u = 0; u < SD_AHEAD; ++u) sc[u][r] = exp2f(sc[u][r] - m_new);
     }
 #pragma unroll
     for (int u = 0; u < SD_AHEAD; ++u) {
-#pragma unroll
-      for (int r = 0; r < REP; ++r) l[r] += sc[u][r];
 #pragma unroll
       for (int p = 0; p < VR; ++p) {
         float f[N];
@@ -390,9 +441,18 @@ sink_attn_decode_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, 
 #pragma unroll
         for (int r = 0; r < REP; ++r)
 #pragma unroll
-          for (int e = 0; e < N; ++e) acc[r][p * N + e] += sc[u][r] * f[e];
+          for (int e = 0; e < N; ++e) acc[r][p * N + e] += w[r * SD_AHEAD + u] * f[e];
       }
     }
+  }
+  // a head's denominator over its lanes, then every lane with every head's maximum and denominator
+#pragma unroll
+  for (int o = DUP; o < DUP * SD_AHEAD / OWN; o <<= 1) l_own += __shfl_xor_sync(0xffffffffu, l_own, o);
+  float m[REP], l[REP];
+#pragma unroll
+  for (int r = 0; r < REP; ++r) {
+    m[r] = __shfl_sync(0xffffffffu, m_own, r * SD_AHEAD / OWN * DUP, LPK);
+    l[r] = __shfl_sync(0xffffffffu, l_own, r * SD_AHEAD / OWN * DUP, LPK);
   }
   // the lane groups of the warp
 #pragma unroll
@@ -425,11 +485,11 @@ sink_attn_decode_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, 
     float mm = sink != nullptr ? sink[h] * LOG2E : -1e30f;
     const float sk = mm;
 #pragma unroll
-    for (int w = 0; w < SD_WARPS; ++w) mm = fmaxf(mm, part[w][r][DV]);
+    for (int w = 0; w < WARPS; ++w) mm = fmaxf(mm, part[w][r][DV]);
     float den = sink != nullptr ? exp2f(sk - mm) : 0.f;
-    float cw[SD_WARPS];
+    float cw[WARPS];
 #pragma unroll
-    for (int w = 0; w < SD_WARPS; ++w) {
+    for (int w = 0; w < WARPS; ++w) {
       cw[w] = exp2f(part[w][r][DV] - mm);
       den += cw[w] * part[w][r][DV + 1];
     }
@@ -440,7 +500,7 @@ sink_attn_decode_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, 
     for (int c = threadIdx.x; c < DV; c += blockDim.x) {
       float o = 0.f;
 #pragma unroll
-      for (int w = 0; w < SD_WARPS; ++w) o += cw[w] * part[w][r][c];
+      for (int w = 0; w < WARPS; ++w) o += cw[w] * part[w][r][c];
       if (gate != nullptr && gate_el) o *= sigmoid_f(to_f(gate[t * ldg + static_cast<int64_t>(h) * DV + c]));
       put_out(out, obase + c, o * inv, out_f32);
     }
@@ -452,15 +512,17 @@ static void launch_sink_decode(int rep, cudaStream_t st, const void* q, const vo
                                const int32_t* seq_start, const int32_t* seq_pos0, const int32_t* seq_len, const int32_t* bt,
                                int64_t bt_stride, const float* sink, const void* gate, int64_t ldg, int gate_el, int n_seqs, int H, int G, int Gv,
                                int page, int mask_kind, int mask, int keep_first, float softcap, float scale, int out_f32) {
-#define SD_GO(REP) sink_attn_decode_kernel<T, LPK, REP, VR><<<dim3(H / REP, n_seqs), SD_WARPS * 32, 0, st>>>(static_cast<const T*>(q), \
-      static_cast<const T*>(kc), static_cast<const T*>(vc), static_cast<T*>(out), seq_start, seq_pos0, seq_len, bt, bt_stride, sink, \
-      static_cast<const T*>(gate), ldg, gate_el, H, G, Gv, page, mask_kind, mask, keep_first, softcap, scale, out_f32)
+#define SD_RUN(REP, WARPS) sink_attn_decode_kernel<T, LPK, REP, VR, WARPS><<<dim3(H / REP, n_seqs), WARPS * 32, 0, st>>>( \
+      static_cast<const T*>(q), static_cast<const T*>(kc), static_cast<const T*>(vc), static_cast<T*>(out), seq_start, seq_pos0, seq_len, \
+      bt, bt_stride, sink, static_cast<const T*>(gate), ldg, gate_el, H, G, Gv, page, mask_kind, mask, keep_first, softcap, scale, out_f32)
+#define SD_GO(REP) do { if (static_cast<int64_t>(H / REP) * n_seqs <= 2 * sm_count()) SD_RUN(REP, 8); else SD_RUN(REP, 4); } while (0)
   if constexpr (LPK * Vec16<T>::N * VR <= 128) {          // four heads' accumulators fit registers and shared memory
     if (rep % 4 == 0) { SD_GO(4); return; }
   }
   if (rep % 2 == 0) SD_GO(2);
   else SD_GO(1);
 #undef SD_GO
+#undef SD_RUN
 }
 
 // the row-splitting kernel takes d = LPK * (16 / sizeof(T)) with LPK in {4, 8, 16, 32} and dv = d or 2 d
