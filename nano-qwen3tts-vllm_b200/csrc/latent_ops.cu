@@ -300,38 +300,6 @@ __global__ void silu_mul_kernel(const T* __restrict__ gu, T* __restrict__ y, siz
   }
 }
 
-// Rows of the latent cache that portions attend to, side by side: sequence b's keys from lo(b) on, lo(b) = its window's lower bound
-// rounded down to whole boxes of the attention kernel, sequence after sequence.  Row of key j: key_start[b] + j.  Bound: HBM (rows
-// read and written once); a warp copies one row of `width` numbers (a multiple of 8) in 16-byte pieces.
-__device__ __forceinline__ int first_key(int pos0, int window) { return window > 0 ? max(0, pos0 - window + 1) & ~63 : 0; }
-__global__ void __launch_bounds__(256)
-latent_gather_kernel(const __nv_bfloat16* __restrict__ cache, __nv_bfloat16* __restrict__ out, int32_t* __restrict__ key_start,
-                     const int32_t* __restrict__ block_tables, int64_t bt_stride, const int32_t* __restrict__ seq_pos0,
-                     const int32_t* __restrict__ seq_len, int window, int width, int page, int max_rows) {
-  __shared__ int sum[8];
-  const int b = blockIdx.y, tid = threadIdx.x;
-  int before = 0;                                          // rows of the sequences in front
-  for (int i = tid; i < b; i += 256)
-    if (seq_len[i] > 0) before += seq_pos0[i] + seq_len[i] - first_key(seq_pos0[i], window);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
-  if ((tid & 31) == 0) sum[tid >> 5] = before;
-  __syncthreads();
-  before = 0;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) before += sum[i];
-  const int lo = first_key(seq_pos0[b], window), n = seq_len[b] > 0 ? seq_pos0[b] + seq_len[b] - lo : 0;
-  if (blockIdx.x == 0 && tid == 0) key_start[b] = before - lo;
-  const int32_t* bt = block_tables + b * bt_stride;
-  for (int r = blockIdx.x * 8 + (tid >> 5); r < n; r += gridDim.x * 8) {
-    const int j = lo + r;
-    if (before + r >= max_rows) return;                    // never: the caller made room for all of them
-    const uint4* src = reinterpret_cast<const uint4*>(cache + (static_cast<size_t>(bt[j / page]) * page + j % page) * width);
-    uint4* dst = reinterpret_cast<uint4*>(out + static_cast<size_t>(before + r) * width);
-    for (int c = tid & 31; c < width / 8; c += 32) dst[c] = src[c];
-  }
-}
-
 static int flat_grid(size_t n) { return static_cast<int>(std::min<size_t>((n + 255) / 256, 148 * 16)); }
 
 }  // namespace lat
@@ -460,24 +428,5 @@ extern "C" int b2tts_silu_mul(const void* gu, void* y, int64_t rows, int ff, int
   LAT_DISPATCH(dtype, (silu_mul_kernel<T><<<flat_grid(static_cast<size_t>(rows) * ff), 256, 0, st>>>(static_cast<const T*>(gu), static_cast<T*>(y),
                                                                                                   static_cast<size_t>(rows), ff)));
   B2_CHECK_LAUNCH("silu_mul");
-  return B2TTS_OK;
-}
-
-extern "C" int b2tts_latent_gather(const void* cache, void* out, int32_t* key_start, const int32_t* block_tables, int64_t bt_stride,
-                                   const int32_t* seq_pos0, const int32_t* seq_len, int n_seqs, int max_keys, int max_rows, int window,
-                                   int width, int page, void* stream) {
-  using namespace b2;
-  using namespace b2::lat;
-  B2_REQUIRE(n_seqs >= 0 && max_keys >= 0 && max_rows >= 0 && window >= 0 && page > 0 && width > 0 && width % 8 == 0, B2TTS_EINVAL,
-             "latent_gather: bad sizes (width=%d page=%d)", width, page);
-  B2_REQUIRE(n_seqs <= 65535, B2TTS_EUNSUPPORTED, "latent_gather: %d sequences", n_seqs);
-  if (n_seqs == 0) return B2TTS_OK;
-  B2_REQUIRE(cache && out && key_start && block_tables && seq_pos0 && seq_len, B2TTS_EINVAL, "latent_gather: null pointer");
-  B2_REQUIRE(aligned16(cache) && aligned16(out), B2TTS_EALIGN, "latent_gather: rows must start on 16-byte boundaries");
-  const int gx = std::max(1, std::min((max_keys + 7) / 8, 512));
-  latent_gather_kernel<<<dim3(gx, n_seqs), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(cache), static_cast<__nv_bfloat16*>(out), key_start, block_tables, bt_stride, seq_pos0, seq_len, window,
-      width, page, max_rows);
-  B2_CHECK_LAUNCH("latent_gather");
   return B2TTS_OK;
 }

@@ -559,37 +559,6 @@ int launch_prompt_attn(const char* what, const PromptAttnArgs& a, cudaStream_t s
 }  // namespace row
 }  // namespace b2
 
-extern "C" int b2tts_latent_portions_attn(const void* q, int64_t q_tok, int64_t q_head, const void* k, int64_t k_row, const void* kr,
-                                          int64_t kr_row, const void* v, int64_t v_row, const int32_t* key_start, void* out, const float* sink,
-                                          const void* gate, int64_t ldg, int gate_el, const float* freq, float rot_mult, int rot_dims,
-                                          const int32_t* seq_start, const int32_t* seq_pos0, const int32_t* seq_len, int n_seqs, int max_new,
-                                          int heads, int dim, int rot_dim, int vdim, int window, float scale, void* stream) {
-  using namespace b2;
-  using namespace b2::row;
-  B2_REQUIRE(n_seqs >= 0 && max_new >= 0 && heads > 0 && dim > 0 && rot_dim >= 0 && vdim > 0 && window >= 0 && rot_dims >= 0 && rot_dims <= rot_dim &&
-                 rot_dims % 2 == 0, B2TTS_EINVAL, "latent_portions_attn: bad sizes");
-  B2_REQUIRE(heads <= 65535 && n_seqs <= 65535, B2TTS_EUNSUPPORTED, "latent_portions_attn: %d heads, %d sequences", heads, n_seqs);
-  if (n_seqs == 0 || max_new <= 1) return B2TTS_OK;
-  B2_REQUIRE(q && k && v && key_start && out && seq_start && seq_pos0 && seq_len && (rot_dim == 0 || kr) && (rot_dims == 0 || freq), B2TTS_EINVAL,
-             "latent_portions_attn: null pointer");
-  using B = __nv_bfloat16;
-  PromptAttnArgs p{};
-  p.q = static_cast<const B*>(q); p.q_tok = q_tok; p.q_head = q_head;
-  p.k = static_cast<const B*>(k); p.k_row = k_row; p.k_head = dim; p.d1 = dim;
-  p.k2 = rot_dim > 0 ? static_cast<const B*>(kr) : nullptr; p.k2_row = rot_dim > 0 ? kr_row : 0;
-  p.v = static_cast<const B*>(v); p.v_row = v_row; p.v_head = vdim;
-  p.key_start = key_start; p.page = 1;
-  p.seq_start = seq_start; p.seq_pos0 = seq_pos0; p.seq_len = seq_len;
-  p.sink = sink; p.gate = static_cast<const B*>(gate); p.ldg = ldg; p.gate_el = gate_el;
-  p.freq = freq; p.rot_mult = rot_mult; p.rot_dims = rot_dims;
-  p.out = out;
-  p.H = heads; p.G = heads; p.Gv = heads; p.d = dim + rot_dim; p.dv = vdim;
-  p.mask = window; p.scale = scale;
-  p.n_seqs = n_seqs; p.max_new = max_new;
-  B2_REQUIRE(prompt_attn_applies(p), B2TTS_EUNSUPPORTED, "latent_portions_attn: dim=%d rot_dim=%d vdim=%d or a row alignment", dim, rot_dim, vdim);
-  return launch_prompt_attn("latent_portions_attn", p, static_cast<cudaStream_t>(stream));
-}
-
 extern "C" int b2tts_prompt_attn_timeouts(void) {
   int v = 0;
   if (cudaMemcpyFromSymbol(&v, b2::row::g_prompt_attn_timeouts, sizeof(int)) != cudaSuccess) return -1;

@@ -37,7 +37,6 @@ class MixedStepLayout:
             self.hosts.append(h)
             self.events.append(None)
         self.n_tokens = self.n_seqs = self.max_new = self.n_want = 0
-        self.portions = None
 
     def _view(self, buf, name):
         o, n = self.offsets[name]
@@ -97,8 +96,6 @@ class MixedStepLayout:
             self.events[self.cur] = ev
         self.n_tokens, self.n_seqs, self.n_want = o, n_seqs, len(want_rows)
         self.max_new = max((n for _, n in items), default=0)
-        # (tokens cached, tokens new) per live row on the host: what sizes a launch or a buffer of the step
-        self.portions = [(seq.num_cached_tokens, n) for seq, n in items]
         self._bind()
 
     def _bind(self):
@@ -114,5 +111,4 @@ class MixedStepLayout:
         """Views for a captured decode step of ``rows`` one-token sequences (contents come from ``fill``)."""
         self.n_tokens = self.n_seqs = rows
         self.max_new, self.n_want = 1, 0
-        self.portions = None
         self._bind()
