@@ -604,8 +604,6 @@ B2TTS_API int b2tts_sink_attn(const void* q, const void* k_cache, const void* v_
                               int n_tokens, int n_seqs, int max_new, int heads, int kv_heads, int v_heads, int dim, int vdim,
                               int page, int mask_kind, int mask, int keep_first, float softcap, float scale, int dtype, int path,
                               int out_f32, void* stream);
-/* How often a wait inside the tensor-core kernel of prompt attention ran out since the library was loaded (expected: 0). */
-B2TTS_API int b2tts_prompt_attn_timeouts(void);
 /* out[t, c] = act(bias[c] + sum_j w[c, j] * u(position(t) - taps + 1 + j)[c_off + c]) for c < channels (act 0: none, 1: SiLU;
  * bias may be null).  Earlier positions come from this step's rows, from state [slots, taps-1, channels] (the sequence's last
  * rows, oldest first, advanced by this call) or are zero before position 0.  max_new >= every seq_len[b] (0: unknown). */

@@ -97,7 +97,6 @@ def _load():
         "b2tts_grouped_gemm_gated": (I, [P, L, P, P, L, P, P, I, I, I, I, I, F, F, P]),
         "b2tts_grouped_gemm_silu": (I, [P, L, P, P, L, P, P, I, I, I, I, I, P]),
         "b2tts_grouped_gemm_timeouts": (I, []),
-        "b2tts_prompt_attn_timeouts": (I, []),
         "b2tts_tanh_residual": (I, [P, P, P, I, P, P, P, I, P, P, P, F, P, P, P, P, P, I, I, I, I, P]),
         "b2tts_tanh_gather": (I, [P, P, P, P, P, P, I, I, I, P]),
         "b2tts_clamped_gate_mul": (I, [P, P, L, I, F, F, I, P]),
@@ -1112,10 +1111,6 @@ def sink_attn(q, k_cache, v_cache, out, lay, sink, gate, heads, kv_heads, dim, v
                                    0 if gate is None else gate.stride(0), int(gate_el), lay.n_tokens, lay.n_seqs, lay.max_new, heads, kv_heads,
                                    kv_heads if v_heads is None else v_heads, dim, vdim, page, mask_kind, mask, keep_first, softcap,
                                    scale, dt, path, int(out.dtype == F32 and q.dtype != F32), _stream()), "sink_attn")
-
-
-def prompt_attn_timeouts() -> int:
-    return int(_load().b2tts_prompt_attn_timeouts())
 
 
 def short_conv_act(u, c_off, channels, w, bias, state, lay, out, taps, act=1):

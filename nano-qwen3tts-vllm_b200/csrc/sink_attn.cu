@@ -13,7 +13,7 @@
 // maps over one set of values).
 //
 // Three kernels share a launch: prompt portions in bf16 with head sizes 32..128 x 64, 128 run on the tensor cores
-// (prompt_attn_tc.cu), rows with ONE new token and a head size of 4, 8, 16 or 32 16-byte pieces (dv = d or 2 d) in a kernel whose
+// (sink_attn_mma_kernel), rows with ONE new token and a head size of 4, 8, 16 or 32 16-byte pieces (dv = d or 2 d) in a kernel whose
 // lanes split a cached row (sink_attn_decode_kernel), everything else in the plain kernel; each skips the rows of the others.
 //
 // Plain kernel (bf16 or float, any head size up to 256): one CTA of four warps per token and 1, 2 or 4 query heads of one
@@ -23,7 +23,7 @@
 // through shared memory.  Scores, weights and sums are float in both modes.
 #include <math.h>
 
-#include "prompt_attn.cuh"
+#include "row_ops.cuh"
 
 namespace b2 {
 namespace row {
@@ -545,9 +545,261 @@ static bool launch_sink_decode_any(int d, int dv, int rep, cudaStream_t st, cons
 #undef SD_ARGS
 }
 
+// ------------------------------------------------------------------ prompt portions on the tensor cores (bf16)
+// 64 query tokens of one head per CTA (4 warps x 16 rows); key tiles of 64 are gathered through the block table into
+// padded shared-memory rows by 16-byte asynchronous copies, two stages deep.  S = Q K^T and O += P V run as m16n8k16 bf16
+// MMAs with float accumulators in registers.  The softmax is the running one: a row keeps its maximum m and denominator
+// l (both in the base-2 domain), rescales O when m grows, and the sink enters as the initial state m = sink, l = 1 with
+// no value.  Weights are computed in float from the float scores and enter the second product as a bf16 pair hi + lo
+// (lo = bf16(w - hi)), i.e. with 16 mantissa bits.  Both masks are a per-row lower bound lo(i) <= j <= i; tiles a warp
+// cannot see are skipped, tiles it sees whole take a path without per-element tests.  With kept first keys, tiles over
+// [0, min(F, lowest bound of the CTA)) run in front of the regular ones, and a regular tile that reaches below F is never
+// skipped.
+__device__ __forceinline__ float ex2_approx(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ void split_bf16(float x, float y, uint32_t& hi, uint32_t& lo) {
+  hi = pack_bf16(x, y);
+  lo = pack_bf16(x - bf16lo(hi), y - bf16hi(hi));
+}
+
+constexpr int SM_BM = 64, SM_BN = 64;
+
+__device__ __forceinline__ int mask_lo(int i, int mask_kind, int mask) {
+  if (mask <= 0) return 0;
+  return mask_kind == 0 ? max(0, i - mask + 1) : (i / mask) * mask;
+}
+
+template <int D, int DV>
+__global__ void __launch_bounds__(128)
+sink_attn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k_cache,
+                     const __nv_bfloat16* __restrict__ v_cache, __nv_bfloat16* __restrict__ out,
+                     const int32_t* __restrict__ seq_start, const int32_t* __restrict__ seq_pos0,
+                     const int32_t* __restrict__ seq_len, const int32_t* __restrict__ block_tables, int64_t bt_stride,
+                     const float* __restrict__ sink, const __nv_bfloat16* __restrict__ gate, int64_t ldg, int gate_el, int H, int G, int Gv,
+                     int page, int mask_kind, int mask, int keep_first, float softcap, float scale, int out_f32) {
+  constexpr int QS = D + 8, VS = DV + 8;             // padded rows: 16-byte aligned, ldmatrix rows land in distinct banks
+  constexpr float LOG2E = 1.4426950408889634f;
+  extern __shared__ __align__(16) unsigned char sm_raw[];
+  __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(sm_raw);        // [BM][QS]
+  __nv_bfloat16* Ks = Qs + SM_BM * QS;                                 // [2][BN][QS]
+  __nv_bfloat16* Vs = Ks + 2 * SM_BN * QS;                             // [2][BN][VS]
+  const int b = blockIdx.z, h = blockIdx.y, g = h / (H / G), gv = g % Gv;
+  const int len = seq_len[b];
+  const int t0 = blockIdx.x * SM_BM;
+  if (len <= 1 || t0 >= len) return;                 // one-token and padding rows belong to the plain kernel
+  const int tid = threadIdx.x, lane = tid & 31, wr = tid >> 5;
+  const int start = seq_start[b], pos0 = seq_pos0[b];
+  const int32_t* bt = block_tables + static_cast<int64_t>(b) * bt_stride;
+  for (int idx = tid; idx < SM_BM * (D / 8); idx += 128) {
+    const int r = idx / (D / 8), ch = idx % (D / 8);
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (t0 + r < len) v = ldg_v4(q + (static_cast<size_t>(start + t0 + r) * H + h) * D + ch * 8);
+    *reinterpret_cast<uint4*>(Qs + r * QS + ch * 8) = v;
+  }
+  const float scale2 = scale * LOG2E, cap2 = softcap * LOG2E;
+  const int t_hi = min(len - 1, t0 + SM_BM - 1);
+  const int j_lo = mask_lo(pos0 + t0, mask_kind, mask), j_hi = pos0 + t_hi;
+  const int row_lo = wr * 16 + (lane >> 2);
+  const int p_lo = pos0 + t0 + row_lo, p_hi = p_lo + 8;
+  const bool ok_lo = t0 + row_lo < len, ok_hi = t0 + row_lo + 8 < len;
+  const int lo_lo = mask_lo(p_lo, mask_kind, mask), lo_hi = mask_lo(p_hi, mask_kind, mask);
+  const int wp_lo = pos0 + t0 + wr * 16, wp_hi = wp_lo + 15;
+  const int w_first = mask_lo(wp_lo, mask_kind, mask), w_last = mask_lo(wp_hi, mask_kind, mask);
+  float oacc[DV / 8][4];
+#pragma unroll
+  for (int i = 0; i < DV / 8; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) oacc[i][e] = 0.f;
+  // running maximum and (this thread's share of the) denominator of its two rows; the sink is counted by one lane of four
+  float m0 = -1e30f, m1 = -1e30f, l0 = 0.f, l1 = 0.f;
+  if (sink != nullptr) {
+    m0 = m1 = sink[h] * LOG2E;
+    if ((lane & 3) == 0) l0 = l1 = 1.f;
+  }
+
+  // two threads per key: the slot once, then the thread's 16-byte chunks lch, lch + 2, ... of the key's K and V rows
+  const int lkey = tid >> 1, lch = tid & 1;
+  // kept first keys that the lowest bound of the CTA hides: tiles of their own, in front of the regular ones
+  const int pre_end = min(keep_first, j_lo), n_pre = (pre_end + SM_BN - 1) / SM_BN;
+  auto tile_j0 = [&](int t) { return t < n_pre ? t * SM_BN : j_lo + (t - n_pre) * SM_BN; };
+  auto load_tile = [&](int stage, int t) {
+    const int j = tile_j0(t) + lkey;
+    const bool ok = j <= (t < n_pre ? pre_end - 1 : j_hi);
+    size_t slot = 0;
+    if (ok) {
+      const int pg = j / page;
+      slot = static_cast<size_t>(bt[pg]) * page + (j - pg * page);
+    }
+    const __nv_bfloat16* ksrc = k_cache + (slot * G + g) * D + lch * 8;
+    const __nv_bfloat16* vsrc = v_cache + (slot * Gv + gv) * DV + lch * 8;
+    __nv_bfloat16* kd = Ks + (stage * SM_BN + lkey) * QS + lch * 8;
+    __nv_bfloat16* vd = Vs + (stage * SM_BN + lkey) * VS + lch * 8;
+#pragma unroll
+    for (int i = 0; i < D / 16; ++i) cp_async_16(kd + i * 16, ksrc + i * 16, ok);
+#pragma unroll
+    for (int i = 0; i < DV / 16; ++i) cp_async_16(vd + i * 16, vsrc + i * 16, ok);
+  };
+  const int n_tiles = n_pre + (j_hi - j_lo) / SM_BN + 1;
+  load_tile(0, 0);
+  cp_async_commit();
+  for (int t = 0; t < n_tiles; ++t) {
+    const int j0 = tile_j0(t);
+    const bool pre = t < n_pre;
+    cp_async_wait<0>();
+    __syncthreads();                                 // tile t has landed (Q too); tile t - 1 is consumed
+    if (t + 1 < n_tiles) load_tile((t + 1) & 1, t + 1);
+    cp_async_commit();
+    const __nv_bfloat16* Kt = Ks + (t & 1) * SM_BN * QS;
+    const __nv_bfloat16* Vt = Vs + (t & 1) * SM_BN * VS;
+    if (t0 + wr * 16 >= len) continue;
+    if (!pre && (j0 > wp_hi || (j0 + SM_BN - 1 < w_first && j0 >= keep_first))) continue;   // none of the warp's rows sees the tile
+    float sacc[SM_BN / 8][4];
+#pragma unroll
+    for (int i = 0; i < SM_BN / 8; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) sacc[i][e] = 0.f;
+#pragma unroll
+    for (int ks = 0; ks < D / 16; ++ks) {
+      uint32_t a[4];
+      ldsm_x4(a[0], a[1], a[2], a[3], Qs + (wr * 16 + (lane & 15)) * QS + ks * 16 + (lane >> 4) * 8);
+#pragma unroll
+      for (int np = 0; np < SM_BN / 16; ++np) {
+        uint32_t b0, b1, b2, b3;
+        ldsm_x4(b0, b1, b2, b3, Kt + (np * 16 + (lane >> 4) * 8 + (lane & 7)) * QS + ks * 16 + ((lane >> 3) & 1) * 8);
+        mma_bf16_16816(sacc[2 * np], a, b0, b1);
+        mma_bf16_16816(sacc[2 * np + 1], a, b2, b3);
+      }
+    }
+    const bool inner = !pre && j0 + SM_BN - 1 <= wp_lo && j0 >= w_last;
+    float mx0 = -INFINITY, mx1 = -INFINITY;
+#pragma unroll
+    for (int nt = 0; nt < SM_BN / 8; ++nt) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        float s = sacc[nt][e] * scale2;
+        if (softcap > 0.f) s = cap2 * tanhf(s / cap2);
+        if (!inner) {
+          const int j = j0 + nt * 8 + 2 * (lane & 3) + (e & 1);
+          bool ok;
+          if (pre) ok = j < pre_end;                 // below every row's bound and position: seen by all, counted here only
+          else ok = e < 2 ? (j <= p_lo && (j >= lo_lo || j < keep_first)) : (j <= p_hi && (j >= lo_hi || j < keep_first));
+          if (!ok) s = -INFINITY;
+        }
+        sacc[nt][e] = s;
+        if (e < 2) mx0 = fmaxf(mx0, s); else mx1 = fmaxf(mx1, s);
+      }
+    }
+    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
+    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
+    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
+    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
+    const float n0 = fmaxf(m0, mx0), n1 = fmaxf(m1, mx1);      // finite: m starts finite
+    const float c0 = ex2_approx(m0 - n0), c1 = ex2_approx(m1 - n1);
+    m0 = n0; m1 = n1;
+    float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+    for (int nt = 0; nt < SM_BN / 8; ++nt) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float w = ex2_approx(sacc[nt][e] - (e < 2 ? n0 : n1));
+        sacc[nt][e] = w;
+        if (e < 2) s0 += w; else s1 += w;
+      }
+    }
+    l0 = l0 * c0 + s0;
+    l1 = l1 * c1 + s1;
+#pragma unroll
+    for (int i = 0; i < DV / 8; ++i) { oacc[i][0] *= c0; oacc[i][1] *= c0; oacc[i][2] *= c1; oacc[i][3] *= c1; }
+#pragma unroll
+    for (int kk = 0; kk < SM_BN / 16; ++kk) {
+      uint32_t ah[4], al[4];
+      split_bf16(sacc[2 * kk][0], sacc[2 * kk][1], ah[0], al[0]);
+      split_bf16(sacc[2 * kk][2], sacc[2 * kk][3], ah[1], al[1]);
+      split_bf16(sacc[2 * kk + 1][0], sacc[2 * kk + 1][1], ah[2], al[2]);
+      split_bf16(sacc[2 * kk + 1][2], sacc[2 * kk + 1][3], ah[3], al[3]);
+#pragma unroll
+      for (int np = 0; np < DV / 16; ++np) {
+        uint32_t b0, b1, b2, b3;
+        ldsm_x4_t(b0, b1, b2, b3, Vt + (kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * VS + np * 16 + (lane >> 4) * 8);
+        mma_bf16_16816(oacc[2 * np], ah, b0, b1);
+        mma_bf16_16816(oacc[2 * np], al, b0, b1);
+        mma_bf16_16816(oacc[2 * np + 1], ah, b2, b3);
+        mma_bf16_16816(oacc[2 * np + 1], al, b2, b3);
+      }
+    }
+  }
+  cp_async_wait<0>();
+  l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
+  l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
+  l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
+  l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    if (!(half ? ok_hi : ok_lo)) continue;
+    const size_t row = static_cast<size_t>(start + t0 + row_lo + 8 * half);
+    float inv = 1.0f / (half ? l1 : l0);
+    if (gate != nullptr && !gate_el) inv *= sigmoid_f(__bfloat162float(gate[row * ldg + h]));
+    const size_t obase = (row * H + h) * DV + 2 * (lane & 3);
+    if (gate != nullptr && gate_el) {                // a pair of columns per load: the caller checked the alignment
+      const __nv_bfloat16* gr = gate + row * ldg + h * DV + 2 * (lane & 3);
+#pragma unroll
+      for (int nt = 0; nt < DV / 8; ++nt) {
+        const uint32_t gw = *reinterpret_cast<const uint32_t*>(gr + nt * 8);
+        oacc[nt][2 * half] *= sigmoid_f(bf16lo(gw));
+        oacc[nt][2 * half + 1] *= sigmoid_f(bf16hi(gw));
+      }
+    }
+    if (out_f32) {
+      float* o = reinterpret_cast<float*>(out) + obase;
+#pragma unroll
+      for (int nt = 0; nt < DV / 8; ++nt)
+        *reinterpret_cast<float2*>(o + nt * 8) = make_float2(oacc[nt][2 * half] * inv, oacc[nt][2 * half + 1] * inv);
+    } else {
+      __nv_bfloat16* o = out + obase;
+#pragma unroll
+      for (int nt = 0; nt < DV / 8; ++nt)
+        *reinterpret_cast<uint32_t*>(o + nt * 8) = pack_bf16(oacc[nt][2 * half] * inv, oacc[nt][2 * half + 1] * inv);
+    }
+  }
+}
+
+template <int D, int DV>
+static cudaError_t launch_sink_mma(int max_new, int n_seqs, cudaStream_t st, const void* q, const void* kc, const void* vc, void* out,
+                                   const int32_t* seq_start, const int32_t* seq_pos0, const int32_t* seq_len, const int32_t* bt,
+                                   int64_t bt_stride, const float* sink, const void* gate, int64_t ldg, int gate_el, int H, int G, int Gv, int page,
+                                   int mask_kind, int mask, int keep_first, float softcap, float scale, int out_f32) {
+  auto kern = sink_attn_mma_kernel<D, DV>;
+  const size_t smem = sizeof(__nv_bfloat16) * ((SM_BM + 2 * SM_BN) * (D + 8) + 2 * SM_BN * (DV + 8));
+  static bool opted = false;
+  if (!opted) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
+    opted = true;
+  }
+  using B = __nv_bfloat16;
+  const dim3 grid((max_new + SM_BM - 1) / SM_BM, H, n_seqs);
+  kern<<<grid, 128, smem, st>>>(static_cast<const B*>(q), static_cast<const B*>(kc), static_cast<const B*>(vc), static_cast<B*>(out),
+                                seq_start, seq_pos0, seq_len, bt, bt_stride, sink, static_cast<const B*>(gate), ldg, gate_el, H, G, Gv, page,
+                                mask_kind, mask, keep_first, softcap, scale, out_f32);
+  return cudaSuccess;
+}
+
 // head sizes the tensor-core kernel is built for
 static bool sink_mma_shape(int d, int dv) {
   return (d == 32 || d == 48 || d == 64 || d == 96 || d == 128) && (dv == 64 || dv == 128);
+}
+
+#define SINK_MMA_ARGS max_new, n_seqs, st, q, kc, vc, out, seq_start, seq_pos0, seq_len, bt, bt_stride, sink, gate, ldg, gate_el, H, G, Gv, page, mask_kind, mask, keep_first, softcap, scale, out_f32
+template <int D>
+static cudaError_t launch_sink_mma_dv(int dv, int max_new, int n_seqs, cudaStream_t st, const void* q, const void* kc, const void* vc,
+                                      void* out, const int32_t* seq_start, const int32_t* seq_pos0, const int32_t* seq_len,
+                                      const int32_t* bt, int64_t bt_stride, const float* sink, const void* gate, int64_t ldg, int gate_el, int H,
+                                      int G, int Gv, int page, int mask_kind, int mask, int keep_first, float softcap, float scale,
+                                      int out_f32) {
+  return dv == 64 ? launch_sink_mma<D, 64>(SINK_MMA_ARGS) : launch_sink_mma<D, 128>(SINK_MMA_ARGS);
 }
 
 }  // namespace row
@@ -583,21 +835,18 @@ extern "C" int b2tts_sink_attn(const void* q, const void* k_cache, const void* v
   B2_REQUIRE(path != 2 || mma_ok, B2TTS_EUNSUPPORTED, "sink_attn: the tensor-core kernel takes bf16 with head sizes 32..128 / 64, 128");
   const bool use_mma = mma_ok && path != 1 && max_new > 1;
   if (use_mma) {
-    using B = __nv_bfloat16;
-    PromptAttnArgs p{};
-    p.q = static_cast<const B*>(q); p.q_tok = static_cast<int64_t>(heads) * dim; p.q_head = dim;
-    p.k = static_cast<const B*>(k_cache); p.k_row = static_cast<int64_t>(kv_heads) * dim; p.k_head = dim; p.d1 = dim;
-    p.v = static_cast<const B*>(v_cache); p.v_row = static_cast<int64_t>(v_heads) * vdim; p.v_head = vdim;
-    p.block_tables = block_tables; p.bt_stride = bt_stride; p.page = page;
-    p.seq_start = seq_start; p.seq_pos0 = seq_pos0; p.seq_len = seq_len;
-    p.sink = sink; p.gate = static_cast<const B*>(gate); p.ldg = ldg; p.gate_el = gate_el;
-    p.out = out; p.out_f32 = out_f32;
-    p.H = heads; p.G = kv_heads; p.Gv = v_heads; p.d = dim; p.dv = vdim;
-    p.mask_kind = mask_kind; p.mask = mask; p.keep_first = keep_first; p.softcap = softcap; p.scale = scale;
-    p.split_weights = 1;
-    p.n_seqs = n_seqs; p.max_new = max_new;
-    const int rc = launch_prompt_attn("sink_attn (tensor cores)", p, st);
-    if (rc != B2TTS_OK) return rc;
+    const int H = heads, G = kv_heads, Gv = v_heads;
+    const void* kc = k_cache; const void* vc = v_cache; const int32_t* bt = block_tables;
+    cudaError_t e;
+    switch (dim) {
+      case 32: e = launch_sink_mma_dv<32>(vdim, SINK_MMA_ARGS); break;
+      case 48: e = launch_sink_mma_dv<48>(vdim, SINK_MMA_ARGS); break;
+      case 64: e = launch_sink_mma_dv<64>(vdim, SINK_MMA_ARGS); break;
+      case 96: e = launch_sink_mma_dv<96>(vdim, SINK_MMA_ARGS); break;
+      default: e = launch_sink_mma_dv<128>(vdim, SINK_MMA_ARGS); break;
+    }
+    if (e != cudaSuccess) return cuda_fail(e, "sink_attn (tensor cores)");
+    B2_CHECK_LAUNCH("sink_attn (tensor cores)");
   }
   // one-token rows: the row-splitting kernel where the head size fits it (path 1 keeps everything in the plain kernel)
   bool split = false;
