@@ -275,12 +275,12 @@ def test_gemm_prefetch_next_weights_changes_nothing(native):
         native.gemm_bf16(x, pk, n, prefetch=nxt.view(-1)[8:8 + 16384])        # not 16-byte aligned
 
 
-# ------------------------------------------------------------------ batch split (splits < 0): W multicast, no K split
+# ------------------------------------------------------------------ batch split (splits < 0): row chunks, no K split
 @pytest.mark.parametrize("m,bs", [(64, 4), (50, 4), (32, 2), (17, 2), (128, 4), (96, 2), (64, 2)])
 @pytest.mark.parametrize("n,k", [(4096, 1024), (2048, 1024), (1024, 2048), (256, 128), (128, 64)])
 def test_gemm_batch_split_plain_bias_residual(native, m, bs, n, k):
-    """The cluster splits the batch (each CTA: 16 - 48 rows x the whole K, weight tiles multicast): one fp32 accumulator
-    over K in order, so against fp64 it obeys the same bound as the K-split kernel; run-to-run identical."""
+    """The batch is cut into chunks (each CTA: 16 - 48 rows x the whole K): one fp32 accumulator over K in order, so
+    against fp64 it obeys the same bound as the K-split kernel; run-to-run identical."""
     g = torch.Generator(device="cuda").manual_seed(m * 13 + n + k + bs)
     x = torch.randn(m, k, device="cuda", generator=g).to(BF16)
     w = (torch.randn(n, k, device="cuda", generator=g) * 0.05).to(BF16)
