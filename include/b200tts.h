@@ -496,8 +496,12 @@ B2TTS_API int b2tts_grouped_gemm_gated(const void* a, int64_t lda, const void* w
 /* The same with c[s, ff] = silu(g) * u. */
 B2TTS_API int b2tts_grouped_gemm_silu(const void* a, int64_t lda, const void* w, void* c, int64_t ldc, const int32_t* offsets,
                                       const int32_t* sorted_pair, int n_pairs, int experts, int ff, int k, int top, void* stream);
-/* How often a wait inside the grouped tensor-core kernel ran out since the library was loaded (expected: 0). */
+/* How often a wait inside the grouped tensor-core kernel ran out since the library was loaded (expected: 0).  A launch whose wait runs
+ * out leaves no result; the next grouped_gemm* call answers with B2TTS_ECUDA, and so does _check(), once: call it behind a
+ * synchronisation (it makes none itself) before results are used.  _lose_wait() launches a kernel whose wait runs out, for tests. */
 B2TTS_API int b2tts_grouped_gemm_timeouts(void);
+B2TTS_API int b2tts_grouped_gemm_check(void);
+B2TTS_API int b2tts_grouped_gemm_lose_wait(void* stream);
 
 /* ---- decoders with latent attention, token shift and a norm on each sublayer's output (csrc/latent_ops.cu, latent_attn.cu).
  * `dtype` is the activation / cache type (B2TTS_DTYPE_*); x is the float residual stream [rows, cols]. */

@@ -97,6 +97,8 @@ def _load():
         "b2tts_grouped_gemm_gated": (I, [P, L, P, P, L, P, P, I, I, I, I, I, F, F, P]),
         "b2tts_grouped_gemm_silu": (I, [P, L, P, P, L, P, P, I, I, I, I, I, P]),
         "b2tts_grouped_gemm_timeouts": (I, []),
+        "b2tts_grouped_gemm_check": (I, []),
+        "b2tts_grouped_gemm_lose_wait": (I, [P]),
         "b2tts_tanh_residual": (I, [P, P, P, I, P, P, P, I, P, P, P, F, P, P, P, P, P, I, I, I, I, P]),
         "b2tts_tanh_gather": (I, [P, P, P, P, P, P, I, I, I, P]),
         "b2tts_clamped_gate_mul": (I, [P, P, L, I, F, F, I, P]),
@@ -916,6 +918,12 @@ def grouped_gemm_silu(a, w, c, offsets, sorted_pair, n_pairs, top):
 
 def grouped_gemm_timeouts() -> int:
     return int(_load().b2tts_grouped_gemm_timeouts())
+
+
+def check_waits():
+    """Raises when a wait inside a launched kernel has run out, so that results read since the last call are not valid.  Reads a word of
+    host memory: call it behind the synchronisation that the results need anyway."""
+    _check(_load().b2tts_grouped_gemm_check(), "check_waits")
 
 
 # ------------------------------------------------------------------------------------------ latent-attention decoders

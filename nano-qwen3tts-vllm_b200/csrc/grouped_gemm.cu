@@ -288,6 +288,7 @@ extern "C" int b2tts_grouped_gemm(const void* a, int64_t lda, const void* w, voi
   B2_REQUIRE(act == 0 || act == 1, B2TTS_EINVAL, "grouped_gemm: act %d", act);
   if (n_pairs == 0) return B2TTS_OK;
   B2_REQUIRE(a && w && c && offsets && sorted_pair, B2TTS_EINVAL, "grouped_gemm: null pointer");
+  if (const int rc = grouped_tc_check("grouped_gemm")) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // bf16 with 16-byte rows: the tensor-core kernels; float (true 32-bit products) and odd sizes: the plain one
   if (dtype == B2TTS_DTYPE_BF16 && k % 8 == 0 && lda % 8 == 0 && aligned16(a) && aligned16(w)) {
@@ -322,6 +323,7 @@ extern "C" int b2tts_grouped_gemm_gated(const void* a, int64_t lda, const void* 
              ff, k);
   if (n_pairs == 0) return B2TTS_OK;
   B2_REQUIRE(a && w && c && offsets && sorted_pair, B2TTS_EINVAL, "grouped_gemm_gated: null pointer");
+  if (const int rc = grouped_tc_check("grouped_gemm_gated")) return rc;
   B2_REQUIRE(aligned16(a) && aligned16(w) && aligned16(c), B2TTS_EALIGN, "grouped_gemm_gated: pointers must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (grouped_tc_applies(n_pairs, experts, ff, ldc, c))
@@ -343,6 +345,7 @@ extern "C" int b2tts_grouped_gemm_silu(const void* a, int64_t lda, const void* w
              ff, k);
   if (n_pairs == 0) return B2TTS_OK;
   B2_REQUIRE(a && w && c && offsets && sorted_pair, B2TTS_EINVAL, "grouped_gemm_silu: null pointer");
+  if (const int rc = grouped_tc_check("grouped_gemm_silu")) return rc;
   B2_REQUIRE(aligned16(a) && aligned16(w) && aligned16(c), B2TTS_EALIGN, "grouped_gemm_silu: pointers must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (grouped_tc_applies(n_pairs, experts, ff, ldc, c))

@@ -16,6 +16,8 @@ __device__ __forceinline__ float gated_value(float gate, float up, float limit, 
 
 // the tcgen05 kernel's range: n = output columns, see grouped_gemm_tc.cu
 bool grouped_tc_applies(int n_pairs, int experts, int n, int64_t ldc, const void* c);
+// an error, once, when a wait inside an earlier launch has run out
+int grouped_tc_check(const char* what);
 // `n` = rows of W per expert (twice the output columns from GG_CLAMPED on)
 int launch_grouped_tc(const char* what, const void* a, int64_t lda, const void* w, void* c, int64_t ldc, const int32_t* offsets,
                       const int32_t* sorted_pair, int n_pairs, int experts, int n, int k, int top, int in_by_token, int out_by_pair,

@@ -25,8 +25,14 @@ constexpr int TC_GATHER_WARPS = 4, TC_LAG = 2;     // slices a gather warp issue
 constexpr int TC_A_BYTES = TC_BM * G_BK * 2, TC_B_BYTES = TC_BN * G_BK * 2, TC_STAGE_BYTES = TC_A_BYTES + TC_B_BYTES;
 constexpr size_t TC_SMEM = 1024 + static_cast<size_t>(TC_STAGES) * TC_STAGE_BYTES + 256;
 
-// How often a wait inside the kernel ran out (it never should); read by b2tts_grouped_gemm_timeouts().
+// How often a wait inside the kernel ran out (it never should).  The count goes to a word of host memory as well, which the host reads
+// without a copy or a synchronisation: the entry points, and the engine behind each step's own synchronisation, answer with an error
+// when it has moved, since what the launch left behind is not a result.
 __device__ int g_grouped_tc_timeouts = 0;
+__device__ __forceinline__ void report_timeout(int* word) {
+  *reinterpret_cast<volatile int*>(word) = atomicAdd(&g_grouped_tc_timeouts, 1) + 1;
+  __threadfence_system();
+}
 
 struct GroupedTcArgs {
   const int32_t* offsets;
@@ -36,6 +42,7 @@ struct GroupedTcArgs {
   int E, N, K, top, out_by_pair;
   int nk, nb;                              // slices of K, column blocks per expert
   float limit, alpha;
+  int* timeouts;                           // host memory, see report_timeout
 };
 
 // tile -> (expert, row block, column block), for tile numbers that only grow
@@ -129,6 +136,8 @@ grouped_gemm_tc_kernel(const GroupedTcArgs p, const __grid_constant__ CUtensorMa
         __syncwarp();
       }
     }
+    // every commit of this warp has arrived (and with it every product) before the CTA gives up its TMEM and shared memory
+    for (int i = max(0, it - TC_STAGES); i < it; ++i) ok = mbar_wait_limit(empty + i % TC_STAGES, (i / TC_STAGES) & 1) && ok;
   } else if (GATHER && warp >= TC_THREADS / 32) {
     // =========================== gather: warp w copies rows 32 w .. + 31 of the tile, four rows of 128 bytes per instruction
     const int w = warp - TC_THREADS / 32, ch = lane & 7;
@@ -207,7 +216,7 @@ grouped_gemm_tc_kernel(const GroupedTcArgs p, const __grid_constant__ CUtensorMa
       if (lane == 0) mbar_arrive(acc_empty + b);
     }
   }
-  if (!ok && lane == 0) atomicAdd(&g_grouped_tc_timeouts, 1);
+  if (!ok && lane == 0) report_timeout(p.timeouts);
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -226,6 +235,29 @@ bool grouped_tc_applies(int n_pairs, int experts, int n, int64_t ldc, const void
   return n_pairs > TC_MIN_ROWS * static_cast<int64_t>(experts) && n % 8 == 0 && ldc % 8 == 0 && aligned16(c);
 }
 
+static int* timeouts_word() {
+  static int* const word = [] {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;             // the first launch may be a captured one
+    void* p = nullptr;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) p = nullptr;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (p != nullptr) *static_cast<volatile int*>(p) = 0;
+    return static_cast<int*>(p);
+  }();
+  return word;
+}
+static int* g_word = nullptr;              // timeouts_word() once a launch has asked for it: reading the count allocates nothing
+static int g_told = 0;                     // the count that has been answered with an error
+
+int grouped_tc_check(const char* what) {
+  int* word = __atomic_load_n(&g_word, __ATOMIC_ACQUIRE);
+  const int n = word != nullptr ? *static_cast<volatile int*>(word) : 0;
+  if (__atomic_exchange_n(&g_told, n, __ATOMIC_RELAXED) == n) return B2TTS_OK;
+  set_error("%s: a wait inside an earlier grouped product ran out, its results are not valid", what);
+  return B2TTS_ECUDA;
+}
+
 template <int ACT, bool GATHER>
 static int go(const char* what, const GroupedTcArgs& p, const CUtensorMap& ma, const CUtensorMap& mw, int tiles, cudaStream_t st) {
   auto kern = grouped_gemm_tc_kernel<ACT, GATHER>;
@@ -239,6 +271,9 @@ static int go(const char* what, const GroupedTcArgs& p, const CUtensorMap& ma, c
 int launch_grouped_tc(const char* what, const void* a, int64_t lda, const void* w, void* c, int64_t ldc, const int32_t* offsets,
                       const int32_t* sorted_pair, int n_pairs, int experts, int n, int k, int top, int in_by_token, int out_by_pair,
                       int act, float limit, float alpha, cudaStream_t st) {
+  int* word = timeouts_word();
+  B2_REQUIRE(word != nullptr, B2TTS_ECUDA, "%s: no host memory for the kernel's status", what);
+  __atomic_store_n(&g_word, word, __ATOMIC_RELEASE);
   B2_REQUIRE(static_cast<int64_t>(experts) * n < (1ll << 31), B2TTS_EUNSUPPORTED, "%s: %d experts of %d rows", what, experts, n);
   const bool gated = act >= GG_CLAMPED;
   CUtensorMap ma{}, mw;
@@ -254,6 +289,7 @@ int launch_grouped_tc(const char* what, const void* a, int64_t lda, const void* 
   const int cols = gated ? n / 2 : n, bf = gated ? TC_BN / 2 : TC_BN;
   p.nb = (cols + bf - 1) / bf;
   p.limit = limit; p.alpha = alpha;
+  p.timeouts = word;
   const int64_t tiles = (static_cast<int64_t>(n_pairs + TC_BM - 1) / TC_BM + experts) * p.nb;
   const int most = static_cast<int>(std::min<int64_t>(tiles, 1 << 20));
 #define GT_GO(ACT) return in_by_token ? go<ACT, true>(what, p, ma, mw, most, st) : go<ACT, false>(what, p, ma, mw, most, st)
@@ -269,7 +305,27 @@ int launch_grouped_tc(const char* what, const void* a, int64_t lda, const void* 
 }  // namespace b2
 
 extern "C" int b2tts_grouped_gemm_timeouts(void) {
-  int v = 0;
-  if (cudaMemcpyFromSymbol(&v, b2::g_grouped_tc_timeouts, sizeof(int)) != cudaSuccess) return -1;
-  return v;
+  const int* word = __atomic_load_n(&b2::g_word, __ATOMIC_ACQUIRE);
+  return word != nullptr ? *static_cast<const volatile int*>(word) : 0;
+}
+extern "C" int b2tts_grouped_gemm_check(void) { return b2::grouped_tc_check("grouped_gemm"); }
+
+namespace b2 {
+// One wait of the kind that the kernel has, on a barrier that nothing arrives at, with a short limit.
+__global__ void grouped_tc_lost_wait_kernel(int* word) {
+  __shared__ uint64_t bar;
+  if (threadIdx.x == 0) { mbar_init(&bar, 1); mbar_fence_init(); }
+  __syncwarp();
+  if (!mbar_wait_limit(&bar, 0, 64) && threadIdx.x == 0) report_timeout(word);
+}
+}  // namespace b2
+
+extern "C" int b2tts_grouped_gemm_lose_wait(void* stream) {
+  using namespace b2;
+  int* word = timeouts_word();
+  B2_REQUIRE(word != nullptr, B2TTS_ECUDA, "grouped_gemm_lose_wait: no host memory");
+  __atomic_store_n(&g_word, word, __ATOMIC_RELEASE);
+  grouped_tc_lost_wait_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(word);
+  B2_CHECK_LAUNCH("grouped_gemm_lose_wait");
+  return B2TTS_OK;
 }

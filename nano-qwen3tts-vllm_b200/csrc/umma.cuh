@@ -168,9 +168,9 @@ __device__ __forceinline__ uint4 norm8(uint4 x, uint4 w, float rs, bool eager) {
 }
 
 // Wait for phase `parity` of an mbarrier, giving up after a bounded number of polls.
-__device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity, int polls = 1 << 20) {
   const uint32_t addr = smem_u32(bar);
-  for (int i = 0; i < (1 << 20); ++i) {
+  for (int i = 0; i < polls; ++i) {
     uint32_t ok;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(ok) : "r"(addr), "r"(parity) : "memory");

@@ -16,6 +16,7 @@ from dataclasses import dataclass, field
 
 import torch
 
+from ... import _native as nat
 from ...sampling_params import SamplingParams
 from ..model_runner.lm_model_runner import LMModelRunner
 from ..scheduler import ChunkScheduler
@@ -97,6 +98,7 @@ class CausalLMEngine(LLMEngine):
                 ids = self.model_runner.call("sample", sel, [sampling[i][0].temperature for i in idx], top_k).tolist()
                 for i, t in zip(idx, ids):
                     tokens[i] = t
+            nat.check_waits()                            # the tokens are on the host: everything that made them has run
             seqs = [s for s, _ in sampling]
             self.scheduler.postprocess(seqs, tokens)
             for s in seqs:

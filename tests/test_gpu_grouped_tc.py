@@ -76,6 +76,7 @@ def test_gated_activations(nat, sizes, ff, k):
         _close(got["silu"][rows], torch.nn.functional.silu(gate) * up, k)
         gate, up = gate.clamp(max=1.5), up.clamp(-1.5, 1.5)
         _close(got["clamped"][rows], gate * torch.sigmoid(1.702 * gate) * (up + 1), k)
+    nat.check_waits()
 
 
 def test_not_finite_values_stay_in_their_rows(nat):
@@ -88,4 +89,23 @@ def test_not_finite_values_stay_in_their_rows(nat):
     c = torch.empty(pairs, 16, device=DEV, dtype=torch.bfloat16)
     nat.grouped_gemm_silu(h, w, c, off, pair, pairs, 1)
     bad = torch.isnan(c).all(1)
+    nat.check_waits()
     assert bad.sum() == 1 and pair[bad.nonzero()[0, 0]] == 11 and torch.isfinite(c[~bad]).all()
+
+
+def test_a_wait_that_ran_out_is_an_error(nat):
+    """The next grouped product refuses once, and so does the check that an engine makes; the next call after that runs again."""
+    off, pair, pairs = _groups((40, 20), 1, 3)
+    h, w = torch.ones(pairs, 64, device=DEV, dtype=torch.bfloat16), torch.ones(2, 32, 64, device=DEV, dtype=torch.bfloat16)
+    c = torch.empty(pairs, 32, device=DEV, dtype=torch.bfloat16)
+    product = lambda: nat.grouped_gemm(h, w, c, off, pair, pairs, 1, in_by_token=True, out_by_pair=False, act=0)
+    before = nat.grouped_gemm_timeouts()
+    for consumer in (product, nat.check_waits):
+        assert nat.lib().b2tts_grouped_gemm_lose_wait(None) == 0
+        torch.cuda.synchronize()
+        with pytest.raises(RuntimeError, match="ran out"):
+            consumer()
+        nat.check_waits()
+        product()
+        assert bool((c == 64).all())
+    assert nat.grouped_gemm_timeouts() == before + 2
