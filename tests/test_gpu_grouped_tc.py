@@ -79,6 +79,41 @@ def test_gated_activations(nat, sizes, ff, k):
     nat.check_waits()
 
 
+@pytest.mark.parametrize("k", [64, 72, 192, 256, 320])               # slices of K: 1, 2, 3, 4, 5, so the ring stands elsewhere at each tile
+def test_several_tiles_per_cta(nat, k):
+    """More than five tiles for every CTA of the persistent kernel: both accumulators in turn, the ring carried over tile borders, empty
+    groups between full ones; scattered rows, consecutive rows and gated products."""
+    sizes, top = (2600, 0, 1, 4100, 129, 0, 9000, 4170), 2
+    E, n, ff = len(sizes), 1032, 520
+    off, pair, pairs = _groups(sizes, top, k)
+    blocks = sum((s + 127) // 128 for s in sizes)
+    assert blocks * ((n + 255) // 256) > 5 * 148 and blocks * ((ff + 127) // 128) > 5 * 148
+    g = torch.Generator(device=DEV).manual_seed(k)
+    r = lambda *s: torch.randn(s, generator=g, device=DEV).to(torch.bfloat16)
+    tok, w, y = r(pairs // top, k), r(E, n, k), r(pairs, k)
+    wg = (r(E, 2 * ff, k) * k ** -0.5).to(torch.bfloat16)
+    new = lambda cols: torch.full((pairs, cols), 7.0, device=DEV, dtype=torch.bfloat16)
+    gathered, boxed, silu, clamped = new(n), new(n), new(ff), new(ff)
+    nat.grouped_gemm(tok, w, gathered, off, pair, pairs, top, in_by_token=True, out_by_pair=False, act=1)
+    nat.grouped_gemm(y, w, boxed, off, pair, pairs, top, in_by_token=False, out_by_pair=True, act=0)
+    nat.grouped_gemm_silu(tok, wg, silu, off, pair, pairs, top)
+    nat.grouped_gemm_gated(tok, wg, clamped, off, pair, pairs, top, 1.5)
+    for e in range(E):
+        rows = slice(off[e].item(), off[e + 1].item())
+        if rows.start == rows.stop:
+            continue
+        x = tok[(pair[rows] // top).long()].double()
+        _close(gathered[rows], (x @ w[e].double().T).clamp(min=0) ** 2, k)
+        _close(boxed[pair[rows].long()], y[rows].double() @ w[e].double().T, k)
+        gu = x @ wg[e].double().T
+        gate, up = gu[:, :ff], gu[:, ff:]
+        _close(silu[rows], torch.nn.functional.silu(gate) * up, k)
+        gate, up = gate.clamp(max=1.5), up.clamp(-1.5, 1.5)
+        _close(clamped[rows], gate * torch.sigmoid(1.702 * gate) * (up + 1), k)
+    nat.check_waits()
+    assert nat.grouped_gemm_timeouts() == 0
+
+
 def test_not_finite_values_stay_in_their_rows(nat):
     """A NaN in one row of the input reaches that row's outputs only, activation included."""
     off, pair, pairs = _groups((150, 90), 1, 3)
