@@ -123,8 +123,8 @@ __global__ void relu_sq_kernel(T* __restrict__ y, size_t n) {
 
 // The same for a 16-byte aligned y of whole 16-byte vectors, RS_AHEAD of them in flight a thread: bound by the traffic to where the
 // product left y, which is L2 for a large part (a prompt step's [7.3 k, 8192] in bf16: 60 -> 18 us; 2-byte accesses did not keep up).
-constexpr int RS_AHEAD = 4;
-template <typename T>
+// One vector a thread as long as that does not fill the multiprocessors: a few rows are one chain of load, square and store.
+template <typename T, int RS_AHEAD>
 __global__ void __launch_bounds__(256) relu_sq_vec_kernel(uint4* __restrict__ y, size_t n) {
   const size_t i0 = blockIdx.x * static_cast<size_t>(256 * RS_AHEAD) + threadIdx.x;
   uint4 raw[RS_AHEAD];
@@ -890,9 +890,16 @@ extern "C" int b2tts_relu_sq(void* y, int64_t n, int dtype, void* stream) {
   const int64_t per = dtype == B2TTS_DTYPE_BF16 ? 8 : 4;
   if (n % per == 0 && aligned16(y) && n / per <= (int64_t{1} << 40)) {
     const size_t nv = static_cast<size_t>(n / per);
-    const unsigned grid = static_cast<unsigned>((nv + 256 * RS_AHEAD - 1) / (256 * RS_AHEAD));
-    if (dtype == B2TTS_DTYPE_BF16) relu_sq_vec_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(static_cast<uint4*>(y), nv);
-    else relu_sq_vec_kernel<float><<<grid, 256, 0, st>>>(static_cast<uint4*>(y), nv);
+    const bool few = nv <= static_cast<size_t>(256) * 4 * sm_count();
+    const unsigned grid = static_cast<unsigned>((nv + (few ? 255 : 1023)) / (few ? 256 : 1024));
+    uint4* v = static_cast<uint4*>(y);
+    if (dtype == B2TTS_DTYPE_BF16) {
+      if (few) relu_sq_vec_kernel<__nv_bfloat16, 1><<<grid, 256, 0, st>>>(v, nv);
+      else relu_sq_vec_kernel<__nv_bfloat16, 4><<<grid, 256, 0, st>>>(v, nv);
+    } else {
+      if (few) relu_sq_vec_kernel<float, 1><<<grid, 256, 0, st>>>(v, nv);
+      else relu_sq_vec_kernel<float, 4><<<grid, 256, 0, st>>>(v, nv);
+    }
   } else {
     const int grid = static_cast<int>(std::min<int64_t>((n + 255) / 256, 148 * 16));
     if (dtype == B2TTS_DTYPE_BF16) relu_sq_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(static_cast<__nv_bfloat16*>(y), static_cast<size_t>(n));
