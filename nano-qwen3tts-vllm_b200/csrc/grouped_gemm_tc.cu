@@ -231,8 +231,9 @@ grouped_gemm_tc_kernel(const GroupedTcArgs p, const __grid_constant__ CUtensorMa
 // fill 16-byte output vectors stay there.
 constexpr int TC_MIN_ROWS = 12;
 
-bool grouped_tc_applies(int n_pairs, int experts, int n, int64_t ldc, const void* c) {
-  return n_pairs > TC_MIN_ROWS * static_cast<int64_t>(experts) && n % 8 == 0 && ldc % 8 == 0 && aligned16(c);
+bool grouped_tc_applies(int n_pairs, int experts, int n, int w_rows, int64_t ldc, const void* c) {
+  return n_pairs > TC_MIN_ROWS * static_cast<int64_t>(experts) && n % 8 == 0 && ldc % 8 == 0 && aligned16(c) &&
+         static_cast<int64_t>(experts) * w_rows < (1ll << 31);             // rows of W are 32-bit coordinates
 }
 
 static int* timeouts_word() {
@@ -274,7 +275,6 @@ int launch_grouped_tc(const char* what, const void* a, int64_t lda, const void* 
   int* word = timeouts_word();
   B2_REQUIRE(word != nullptr, B2TTS_ECUDA, "%s: no host memory for the kernel's status", what);
   __atomic_store_n(&g_word, word, __ATOMIC_RELEASE);
-  B2_REQUIRE(static_cast<int64_t>(experts) * n < (1ll << 31), B2TTS_EUNSUPPORTED, "%s: %d experts of %d rows", what, experts, n);
   const bool gated = act >= GG_CLAMPED;
   CUtensorMap ma{}, mw;
   int rc = make_x_tensor_map(&mw, w, k, experts * n, k, gated ? TC_BN / 2 : TC_BN, what);

@@ -144,3 +144,25 @@ def test_a_wait_that_ran_out_is_an_error(nat):
         product()
         assert bool((c == 64).all())
     assert nat.grouped_gemm_timeouts() == before + 2
+
+
+def test_more_rows_of_weights_than_a_copy_can_name(nat):
+    """2^31 rows of W and more are beyond a tensor map's coordinates and stay on the general kernel.  Two experts of 2^30 rows of which
+    the second is not used (and not there); rows of W repeat every 2^20, so do the outputs, and gate and up rows are the same."""
+    free, _ = torch.cuda.mem_get_info()
+    rows, k, pairs, period = 1 << 30, 8, 25, 1 << 20
+    if free < 60 << 30:
+        pytest.skip("needs 45 GB")
+    g = torch.Generator(device=DEV).manual_seed(1)
+    block = torch.randn(period, k, generator=g, device=DEV).to(torch.bfloat16)
+    w = torch.empty(rows, k, device=DEV, dtype=torch.bfloat16)
+    w.view(-1, period, k).copy_(block)
+    h = torch.randn(pairs, k, generator=g, device=DEV).to(torch.bfloat16)
+    off, pair = torch.tensor([0, pairs, pairs], dtype=torch.int32, device=DEV), torch.arange(pairs, dtype=torch.int32, device=DEV)
+    c = torch.empty(pairs, rows // 2, device=DEV, dtype=torch.bfloat16)
+    rc = nat.lib().b2tts_grouped_gemm_silu(h.data_ptr(), k, w.data_ptr(), c.data_ptr(), rows // 2, off.data_ptr(), pair.data_ptr(), pairs, 2,
+                                           rows // 2, k, 1, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    x = h.double() @ block.double().T
+    _close(c[:, :period], torch.nn.functional.silu(x) * x, k)
+    assert all(torch.equal(c[i].view(-1, period), c[i, :period].expand(rows // 2 // period, period)) for i in range(pairs))
