@@ -200,36 +200,34 @@ scan_kernel(const ScanArgs a) {
 }
 
 // ------------------------------------------------------------------ per-token scalars of the state space and the delta rule
-// kind 0: dt = softplus(s1 + f1[h]), l = -exp(f2[h]) dt; coef = (exp(l), dt, l)               (f1 = dt_bias, f2 = A_log)
-// kind 1: l = -exp(f1[h]) softplus(s2 + f2[h]); coef = (exp(l), sigmoid(s1), l)               (f1 = A_log, f2 = dt_bias)
+// kind 0: dt = softplus(s1 + f1[h]); coef = (exp(-exp(f2[h]) dt), dt, l)                      (f1 = dt_bias, f2 = A_log)
+// kind 1: coef = (exp(-exp(f1[h]) softplus(s2 + f2[h])), sigmoid(s1), l)                      (f1 = A_log, f2 = dt_bias)
 // kind 2: coef = (log input gate, log forget gate, 1) of the matrix memory                   (f1, f2 = the gates' biases)
-// The decays are formed in double: an error of a decay's logarithm grows with every token that the state is carried over.
+// l = 1 unless LOGS: then the logarithm of the decay, formed in double, because the chunk kernels sum it over their tokens and an error
+// of it grows with every token that the state is carried over.  What the token-by-token kernel reads is formed in float either way, so
+// that a token's results do not depend on what runs beside it.
 __device__ __forceinline__ double softplus_d(double x) { return fmax(x, 0.0) + log1p(exp(-fabs(x))); }
 
-template <typename T>
+template <typename T, bool LOGS>
 __global__ void scan_coef_kernel(const T* __restrict__ s1, const T* __restrict__ s2, int64_t lds, const float* __restrict__ f1,
                                  const float* __restrict__ f2, float* __restrict__ coef, int n_tokens, int H, int kind, float cap) {
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n_tokens * H) return;
   const size_t t = idx / H;
   const int h = idx % H;
-  float c0, c1, log_decay = 1.f;
+  float c0, c1, l = 1.f;
   if (kind == 2) {                                       // log gates: cap tanh((s1 + f1) / cap), logsigmoid(cap tanh((s2 + f2) / cap))
     c0 = cap * tanhf((to_f(s1[t * lds + h]) + f1[h]) / cap);
     c1 = logsigmoid_f(cap * tanhf((to_f(s2[t * lds + h]) + f2[h]) / cap));
-  } else if (kind == 0) {
-    const double dt = softplus_d(to_f(s1[t * lds + h]) + f1[h]), l = -exp(static_cast<double>(f2[h])) * dt;
-    log_decay = static_cast<float>(l);
-    c0 = static_cast<float>(exp(l));
-    c1 = static_cast<float>(dt);
   } else {
-    const double l = -exp(static_cast<double>(f1[h])) * softplus_d(to_f(s2[t * lds + h]) + f2[h]);
-    log_decay = static_cast<float>(l);
-    c0 = static_cast<float>(exp(l));
-    c1 = sigmoid_f(to_f(s1[t * lds + h]));
+    const float x = kind == 0 ? to_f(s1[t * lds + h]) + f1[h] : to_f(s2[t * lds + h]) + f2[h], a_log = kind == 0 ? f2[h] : f1[h];
+    const float dt = softplus_f(x);
+    c0 = expf(-expf(a_log) * dt);
+    c1 = kind == 0 ? dt : sigmoid_f(to_f(s1[t * lds + h]));
+    if constexpr (LOGS) l = static_cast<float>(-exp(static_cast<double>(a_log)) * softplus_d(x));
   }
   float* c = coef + static_cast<size_t>(idx) * 3;
-  c[0] = c0; c[1] = c1; c[2] = log_decay;
+  c[0] = c0; c[1] = c1; c[2] = l;
 }
 
 // ------------------------------------------------------------------ scalar part of the matrix memory
@@ -324,10 +322,11 @@ static int launch_scan(const ScanArgs& a, int n_seqs, cudaStream_t st, const cha
 
 template <typename T>
 static void launch_coef(const void* s1, const void* s2, int64_t lds, const float* f1, const float* f2, float* coef, int n_tokens, int H,
-                        int kind, cudaStream_t st, float cap = 1.f) {
-  const int total = n_tokens * H;
-  scan_coef_kernel<T><<<(total + 255) / 256, 256, 0, st>>>(static_cast<const T*>(s1), static_cast<const T*>(s2), lds, f1, f2, coef,
-                                                          n_tokens, H, kind, cap);
+                        int kind, cudaStream_t st, float cap = 1.f, bool logs = false) {
+  const int total = n_tokens * H, blocks = (total + 255) / 256;
+  const T *a = static_cast<const T*>(s1), *b = static_cast<const T*>(s2);
+  if (logs) scan_coef_kernel<T, true><<<blocks, 256, 0, st>>>(a, b, lds, f1, f2, coef, n_tokens, H, kind, cap);
+  else scan_coef_kernel<T, false><<<blocks, 256, 0, st>>>(a, b, lds, f1, f2, coef, n_tokens, H, kind, cap);
 }
 
 }  // namespace row
@@ -354,9 +353,6 @@ extern "C" int b2tts_ssm_scan(const void* xbc, int64_t ldx, const void* dt, int6
   const size_t el = dtype == B2TTS_DTYPE_BF16 ? 2 : 4;
   const int inner = heads * vdim;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (dtype == B2TTS_DTYPE_BF16) launch_coef<__nv_bfloat16>(dt, nullptr, lddt, dt_bias, a_log, coef, n_tokens, heads, 0, st);
-  else launch_coef<float>(dt, nullptr, lddt, dt_bias, a_log, coef, n_tokens, heads, 0, st);
-  B2_CHECK_LAUNCH("ssm_scan (scalars)");
   ScanArgs a{};
   const char* base = static_cast<const char*>(xbc);
   a.v = base; a.ldv = ldx;
@@ -366,7 +362,11 @@ extern "C" int b2tts_ssm_scan(const void* xbc, int64_t ldx, const void* dt, int6
   a.state = state; a.out = out;
   a.seq_start = seq_start; a.seq_pos0 = seq_pos0; a.seq_len = seq_len; a.seq_slot = seq_slot;
   a.H = heads; a.G = groups; a.d = dim; a.dv = vdim; a.qscale = 1.f; a.divide = 0;
-  if (dtype == B2TTS_DTYPE_BF16 && n_tokens > n_seqs && scan_chunk_applies(a)) {
+  const bool chunks = dtype == B2TTS_DTYPE_BF16 && n_tokens > n_seqs && scan_chunk_applies(a);
+  if (dtype == B2TTS_DTYPE_BF16) launch_coef<__nv_bfloat16>(dt, nullptr, lddt, dt_bias, a_log, coef, n_tokens, heads, 0, st, 1.f, chunks);
+  else launch_coef<float>(dt, nullptr, lddt, dt_bias, a_log, coef, n_tokens, heads, 0, st);
+  B2_CHECK_LAUNCH("ssm_scan (scalars)");
+  if (chunks) {
     const int rc = launch_linear_chunk("ssm_scan (portions)", a, n_seqs, st);
     if (rc != B2TTS_OK) return rc;
     a.rows = 2;                                            // one-token rows beside the portions
@@ -389,9 +389,6 @@ extern "C" int b2tts_delta_rule_scan(const void* qkv, int64_t ldq, const void* b
   if (n_tokens == 0) return B2TTS_OK;
   const size_t el = dtype == B2TTS_DTYPE_BF16 ? 2 : 4;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (dtype == B2TTS_DTYPE_BF16) launch_coef<__nv_bfloat16>(beta, a_in, ldu, a_log, dt_bias, coef, n_tokens, heads, 1, st);
-  else launch_coef<float>(beta, a_in, ldu, a_log, dt_bias, coef, n_tokens, heads, 1, st);
-  B2_CHECK_LAUNCH("delta_rule_scan (scalars)");
   ScanArgs a{};
   const char* base = static_cast<const char*>(qkv);
   const size_t gd = static_cast<size_t>(kv_heads) * dim;
@@ -402,7 +399,11 @@ extern "C" int b2tts_delta_rule_scan(const void* qkv, int64_t ldq, const void* b
   a.state = state; a.out = out;
   a.seq_start = seq_start; a.seq_pos0 = seq_pos0; a.seq_len = seq_len; a.seq_slot = seq_slot;
   a.H = heads; a.G = kv_heads; a.d = dim; a.dv = vdim; a.qscale = 1.0f / sqrtf(static_cast<float>(dim)); a.divide = 0;
-  if (dtype == B2TTS_DTYPE_BF16 && n_tokens > n_seqs && scan_chunk_applies(a)) {
+  const bool chunks = dtype == B2TTS_DTYPE_BF16 && n_tokens > n_seqs && scan_chunk_applies(a);
+  if (dtype == B2TTS_DTYPE_BF16) launch_coef<__nv_bfloat16>(beta, a_in, ldu, a_log, dt_bias, coef, n_tokens, heads, 1, st, 1.f, chunks);
+  else launch_coef<float>(beta, a_in, ldu, a_log, dt_bias, coef, n_tokens, heads, 1, st);
+  B2_CHECK_LAUNCH("delta_rule_scan (scalars)");
+  if (chunks) {
     const int rc = launch_delta_chunk("delta_rule_scan (portions)", a, n_seqs, st);
     if (rc != B2TTS_OK) return rc;
     a.rows = 2;                                            // one-token rows beside the portions

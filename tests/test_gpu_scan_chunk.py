@@ -208,3 +208,39 @@ def test_delta_rule_values_outside_the_split(nat, value):
             assert not torch.isfinite(got[70:, 1, 5]).any()
         else:
             assert bool(((got - y)[70:, 1, 5].abs() <= 1e-4 * y[70:, 1, 5].abs().max()).all())
+
+
+# ------------------------------------------------------------------------------------------------ beside the token-by-token kernel
+def _inputs(kind, tokens, seed, scale=1.0, D=128, P=64):
+    """[sequences x tokens] inputs of 8 heads as a model has them, and what runs rows of them (as they are packed) on states."""
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    r = lambda *s: torch.randn(s, generator=g, device=DEV)
+    H, G, silu = 8, (1 if kind == "ssm" else 4), torch.nn.functional.silu
+    x = (silu(r(*tokens, (H * P + 2 * G * D))) * scale).to(torch.bfloat16)
+    gates = r(*tokens, H if kind == "ssm" else 2 * H).to(torch.bfloat16)
+    a_log, bias, skip = 0.5 * r(H) - 0.5, 0.5 * r(H), 0.5 * r(H)
+
+    def run(nat, seqs, rows_x, rows_g, state):
+        lay = Lay(seqs)
+        out = torch.empty(lay.n_tokens, H * P, device=DEV)
+        if kind == "ssm":
+            nat.ssm_scan(rows_x, rows_g, bias, a_log, skip, state, out, lay, H, G, P, D)
+        else:
+            nat.delta_rule_scan(rows_x, rows_g[:, :H], rows_g[:, H:], a_log, bias, state, out, lay, H, G, D, P)
+        return out
+    return x, gates, (a_log, bias, skip), run, H, G
+
+
+@pytest.mark.parametrize("kind", ["ssm", "delta"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_scalars_of_one_token_steps_are_float(nat, kind, dtype):
+    """The step of a decoding sequence forms its decay with float functions, whatever runs beside it: with nothing written (keys and values
+    zero) the state is the old one times that decay, bit for bit."""
+    x, gates, (a_log, bias, skip), run, H, G = _inputs(kind, (64, 1), 4)
+    gates = gates[:, 0].to(dtype).contiguous()
+    state = torch.randn(64, H, 128, 64, device=DEV)
+    z = gates[:, -H:].float() + bias
+    decay = torch.exp(-(torch.exp(a_log) * (z.clamp(min=0) + torch.log1p(torch.exp(-z.abs())))))
+    want = state * decay[:, :, None, None]
+    run(nat, [(9, 1, i) for i in range(64)], torch.zeros_like(x[:, 0]).to(dtype), gates, state)
+    assert torch.equal(state, want)
