@@ -123,7 +123,8 @@ __global__ void relu_sq_kernel(T* __restrict__ y, size_t n) {
 
 // The same for a 16-byte aligned y of whole 16-byte vectors, RS_AHEAD of them in flight a thread: bound by the traffic to where the
 // product left y, which is L2 for a large part (a prompt step's [7.3 k, 8192] in bf16: 60 -> 18 us; 2-byte accesses did not keep up).
-// One vector a thread as long as that does not fill the multiprocessors: a few rows are one chain of load, square and store.
+// One vector a thread as long as that does not fill the multiprocessors: a few rows are one chain of load, square and store (4096 floats
+// 2.1 -> 1.8 us).
 template <typename T, int RS_AHEAD>
 __global__ void __launch_bounds__(256) relu_sq_vec_kernel(uint4* __restrict__ y, size_t n) {
   const size_t i0 = blockIdx.x * static_cast<size_t>(256 * RS_AHEAD) + threadIdx.x;

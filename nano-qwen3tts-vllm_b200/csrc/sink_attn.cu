@@ -312,8 +312,8 @@ __device__ __forceinline__ void scatter_sum(float* v, int lane) {
 }
 
 // Registers are bounded for 16 warps a multiprocessor, 8 for the wide accumulators, and 24 where float rows leave a lane the least to have
-// in flight (float, one head of 128 per key head, 128 sequences of 600 keys: 112 -> 103 us; 16 warps with an own score per lane were
-// slower than 32 with a score on every lane).
+// in flight (float, 8 heads of 128, one per key head, 128 sequences of 600 keys: 112 -> 95 us; with the few warps of a small grid the tighter bound
+// costs 6 %, so it holds for the CTAs of four warps).
 template <typename T, int LPK, int REP, int VR, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, (REP * VR > 2 ? 8 : sizeof(T) == 4 && REP * VR == 1 && WARPS == 4 ? 24 : 16) / WARPS)
 sink_attn_decode_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache, T* __restrict__ out,
@@ -520,7 +520,7 @@ static void launch_sink_decode(int rep, cudaStream_t st, const void* q, const vo
       bt, bt_stride, sink, static_cast<const T*>(gate), ldg, gate_el, H, G, Gv, page, mask_kind, mask, keep_first, softcap, scale, out_f32)
   // Eight warps a CTA as long as all CTAs are resident at once - two per multiprocessor, or one where the accumulators (REP * VR * N
   // floats a lane) take more than 128 registers - and four otherwise.  Float, 4 heads a group, d 64, dv 128, 64 sequences (256 CTAs of 168
-  // registers), 1 / 200 keys: 11.3 / 17.7 us with eight warps in two waves, 8.6 / 15.9 with four.
+  // registers), 1 / 200 / 600 keys: 11.3 / 17.8 / 38.9 us with eight warps in two waves, 6.8 / 13.1 / 33.5 with four.
 #define SD_GO(REP) do { if (static_cast<int64_t>(H / REP) * n_seqs <= (REP * VR * Vec16<T>::N > 16 ? 1 : 2) * sm_count()) SD_RUN(REP, 8); \
                          else SD_RUN(REP, 4); } while (0)
   if constexpr (LPK * Vec16<T>::N * VR <= 128) {          // four heads' accumulators fit registers and shared memory
