@@ -634,6 +634,17 @@ B2TTS_API int b2tts_delta_rule_scan(const void* qkv, int64_t ldq, const void* be
                                     const float* dt_bias, float* state, float* coef, float* out, const int32_t* seq_start,
                                     const int32_t* seq_pos0, const int32_t* seq_len, const int32_t* seq_slot, int n_tokens, int n_seqs,
                                     int heads, int kv_heads, int dim, int vdim, int dtype, void* stream);
+/* The same two for callers that know the longest portion of the step: max_new >= every seq_len (0: not known, as above).  Portions
+ * above a size run in chunks by a kernel of their own, which is then not launched for steps without one. */
+B2TTS_API int b2tts_ssm_scan_portions(const void* xbc, int64_t ldx, const void* dt, int64_t lddt, const float* dt_bias, const float* a_log,
+                                      const float* d_skip, float* state, float* coef, float* out, const int32_t* seq_start,
+                                      const int32_t* seq_pos0, const int32_t* seq_len, const int32_t* seq_slot, int n_tokens, int n_seqs,
+                                      int max_new, int heads, int groups, int vdim, int dim, int dtype, void* stream);
+B2TTS_API int b2tts_delta_rule_scan_portions(const void* qkv, int64_t ldq, const void* beta, const void* a_in, int64_t ldu,
+                                             const float* a_log, const float* dt_bias, float* state, float* coef, float* out,
+                                             const int32_t* seq_start, const int32_t* seq_pos0, const int32_t* seq_len,
+                                             const int32_t* seq_slot, int n_tokens, int n_seqs, int max_new, int heads, int kv_heads, int dim,
+                                             int vdim, int dtype, void* stream);
 /* Matrix memory with exponential gates per head: i = cap tanh((ig[t, h] + i_bias[h]) / cap), f = logsigmoid(cap tanh((fg[t, h] +
  * f_bias[h]) / cap)); m' = max(f + m, i) (m starts at 0); S <- exp(f + m - m') S + exp(i - m') k v^T, n likewise with k alone;
  * out[t, h] = S^T q / (max(|n . q|, exp(-m')) + 1e-6) with q times dim^(-1/2).  q, k [rows, heads*dim] and v [rows, heads*vdim]

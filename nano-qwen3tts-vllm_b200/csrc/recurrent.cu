@@ -62,7 +62,8 @@ scan_kernel(const ScanArgs a) {
   __shared__ __align__(16) float vec[2][SCAN_DEPTH][NV][DP];  // [buffer][token of the group][k | q | decay][row]
   const int b = blockIdx.z, h = blockIdx.y;
   const int len = a.seq_len[b];
-  if (len <= 0 || (a.rows == 1 && len == 1) || (a.rows == 2 && len > 1)) return;
+  if (len <= 0) return;
+  if (len < a.min_len || len > a.max_len) return;
   const int d = a.d, dv = a.dv, H = a.H;
   const int g = h / (H / a.G);
   const int start = a.seq_start[b], pos0 = a.seq_pos0[b];
@@ -342,9 +343,9 @@ using namespace b2::row;
   if (n_seqs == 0) return B2TTS_OK;                                                                                     \
   B2_REQUIRE(state && out && seq_start && seq_pos0 && seq_len && seq_slot, B2TTS_EINVAL, name ": null pointer")
 
-extern "C" int b2tts_ssm_scan(const void* xbc, int64_t ldx, const void* dt, int64_t lddt, const float* dt_bias,
+extern "C" int b2tts_ssm_scan_portions(const void* xbc, int64_t ldx, const void* dt, int64_t lddt, const float* dt_bias,
                               const float* a_log, const float* d_skip, float* state, float* coef, float* out, const int32_t* seq_start,
-                              const int32_t* seq_pos0, const int32_t* seq_len, const int32_t* seq_slot, int n_tokens, int n_seqs,
+                              const int32_t* seq_pos0, const int32_t* seq_len, const int32_t* seq_slot, int n_tokens, int n_seqs, int max_new,
                               int heads, int groups, int vdim, int dim, int dtype, void* stream) {
   SCAN_COMMON_CHECKS("ssm_scan");
   B2_REQUIRE(groups > 0 && heads % groups == 0 && n_tokens >= 0, B2TTS_EINVAL, "ssm_scan: %d heads over %d groups", heads, groups);
@@ -362,14 +363,16 @@ extern "C" int b2tts_ssm_scan(const void* xbc, int64_t ldx, const void* dt, int6
   a.state = state; a.out = out;
   a.seq_start = seq_start; a.seq_pos0 = seq_pos0; a.seq_len = seq_len; a.seq_slot = seq_slot;
   a.H = heads; a.G = groups; a.d = dim; a.dv = vdim; a.qscale = 1.f; a.divide = 0;
-  const bool chunks = dtype == B2TTS_DTYPE_BF16 && n_tokens > n_seqs && scan_chunk_applies(a);
+  const int walk = linear_walk_len(a, n_seqs), longest = max_new > 0 ? max_new : n_tokens - n_seqs + 1;
+  const bool chunks = dtype == B2TTS_DTYPE_BF16 && longest > walk && scan_chunk_applies(a);
   if (dtype == B2TTS_DTYPE_BF16) launch_coef<__nv_bfloat16>(dt, nullptr, lddt, dt_bias, a_log, coef, n_tokens, heads, 0, st, 1.f, chunks);
   else launch_coef<float>(dt, nullptr, lddt, dt_bias, a_log, coef, n_tokens, heads, 0, st);
   B2_CHECK_LAUNCH("ssm_scan (scalars)");
   if (chunks) {
+    a.min_len = walk + 1;
     const int rc = launch_linear_chunk("ssm_scan (portions)", a, n_seqs, st);
-    if (rc != B2TTS_OK) return rc;
-    a.rows = 2;                                            // one-token rows beside the portions
+    if (rc != B2TTS_OK || (n_seqs == 1 && max_new > 0)) return rc;
+    a.min_len = 1; a.max_len = walk;                       // single tokens and short portions beside them
   }
   const int rc = dtype == B2TTS_DTYPE_BF16 ? launch_scan<__nv_bfloat16, SCAN_LINEAR>(a, n_seqs, st, "ssm_scan")
                                            : launch_scan<float, SCAN_LINEAR>(a, n_seqs, st, "ssm_scan");
@@ -378,10 +381,18 @@ extern "C" int b2tts_ssm_scan(const void* xbc, int64_t ldx, const void* dt, int6
   return B2TTS_OK;
 }
 
-extern "C" int b2tts_delta_rule_scan(const void* qkv, int64_t ldq, const void* beta, const void* a_in, int64_t ldu,
+extern "C" int b2tts_ssm_scan(const void* xbc, int64_t ldx, const void* dt, int64_t lddt, const float* dt_bias,
+                              const float* a_log, const float* d_skip, float* state, float* coef, float* out, const int32_t* seq_start,
+                              const int32_t* seq_pos0, const int32_t* seq_len, const int32_t* seq_slot, int n_tokens, int n_seqs,
+                              int heads, int groups, int vdim, int dim, int dtype, void* stream) {
+  return b2tts_ssm_scan_portions(xbc, ldx, dt, lddt, dt_bias, a_log, d_skip, state, coef, out, seq_start, seq_pos0, seq_len, seq_slot,
+                                 n_tokens, n_seqs, 0, heads, groups, vdim, dim, dtype, stream);
+}
+
+extern "C" int b2tts_delta_rule_scan_portions(const void* qkv, int64_t ldq, const void* beta, const void* a_in, int64_t ldu,
                                      const float* a_log, const float* dt_bias, float* state, float* coef, float* out,
                                      const int32_t* seq_start, const int32_t* seq_pos0, const int32_t* seq_len,
-                                     const int32_t* seq_slot, int n_tokens, int n_seqs, int heads, int kv_heads, int dim, int vdim,
+                                     const int32_t* seq_slot, int n_tokens, int n_seqs, int max_new, int heads, int kv_heads, int dim, int vdim,
                                      int dtype, void* stream) {
   SCAN_COMMON_CHECKS("delta_rule_scan");
   B2_REQUIRE(kv_heads > 0 && heads % kv_heads == 0 && n_tokens >= 0, B2TTS_EINVAL, "delta_rule_scan: %d heads over %d key heads", heads, kv_heads);
@@ -399,20 +410,31 @@ extern "C" int b2tts_delta_rule_scan(const void* qkv, int64_t ldq, const void* b
   a.state = state; a.out = out;
   a.seq_start = seq_start; a.seq_pos0 = seq_pos0; a.seq_len = seq_len; a.seq_slot = seq_slot;
   a.H = heads; a.G = kv_heads; a.d = dim; a.dv = vdim; a.qscale = 1.0f / sqrtf(static_cast<float>(dim)); a.divide = 0;
-  const bool chunks = dtype == B2TTS_DTYPE_BF16 && n_tokens > n_seqs && scan_chunk_applies(a);
+  const int walk = delta_walk_len(a, n_seqs), longest = max_new > 0 ? max_new : n_tokens - n_seqs + 1;
+  const bool chunks = dtype == B2TTS_DTYPE_BF16 && longest > walk && scan_chunk_applies(a);
   if (dtype == B2TTS_DTYPE_BF16) launch_coef<__nv_bfloat16>(beta, a_in, ldu, a_log, dt_bias, coef, n_tokens, heads, 1, st, 1.f, chunks);
   else launch_coef<float>(beta, a_in, ldu, a_log, dt_bias, coef, n_tokens, heads, 1, st);
   B2_CHECK_LAUNCH("delta_rule_scan (scalars)");
   if (chunks) {
+    a.min_len = walk + 1;
     const int rc = launch_delta_chunk("delta_rule_scan (portions)", a, n_seqs, st);
-    if (rc != B2TTS_OK) return rc;
-    a.rows = 2;                                            // one-token rows beside the portions
+    if (rc != B2TTS_OK || (n_seqs == 1 && max_new > 0)) return rc;
+    a.min_len = 1; a.max_len = walk;                       // single tokens and short portions beside them
   }
   const int rc = dtype == B2TTS_DTYPE_BF16 ? launch_scan<__nv_bfloat16, SCAN_DELTA>(a, n_seqs, st, "delta_rule_scan")
                                            : launch_scan<float, SCAN_DELTA>(a, n_seqs, st, "delta_rule_scan");
   if (rc != B2TTS_OK) return rc;
   B2_CHECK_LAUNCH("delta_rule_scan");
   return B2TTS_OK;
+}
+
+extern "C" int b2tts_delta_rule_scan(const void* qkv, int64_t ldq, const void* beta, const void* a_in, int64_t ldu,
+                                     const float* a_log, const float* dt_bias, float* state, float* coef, float* out,
+                                     const int32_t* seq_start, const int32_t* seq_pos0, const int32_t* seq_len,
+                                     const int32_t* seq_slot, int n_tokens, int n_seqs, int heads, int kv_heads, int dim, int vdim,
+                                     int dtype, void* stream) {
+  return b2tts_delta_rule_scan_portions(qkv, ldq, beta, a_in, ldu, a_log, dt_bias, state, coef, out, seq_start, seq_pos0, seq_len, seq_slot,
+                                        n_tokens, n_seqs, 0, heads, kv_heads, dim, vdim, dtype, stream);
 }
 
 extern "C" int b2tts_matrix_memory_scan(const void* q, const void* k, const void* v, const void* ig, const void* fg, int64_t ldu,
@@ -493,7 +515,9 @@ extern "C" int b2tts_fixed_decay_scan(const float* q, int64_t ldq, const float* 
   B2_REQUIRE(q && k && v && head_decay && rows >= 0 && rows <= 2, B2TTS_EINVAL, "fixed_decay_scan: null pointer or rows %d", rows);
   ScanArgs a{};
   a.q = q; a.ldq = ldq; a.k = k; a.ldk = ldk; a.v = v; a.ldv = ldv;
-  a.head_decay = head_decay; a.rows = rows;
+  a.head_decay = head_decay;
+  if (rows == 1) a.min_len = 2;
+  if (rows == 2) a.max_len = 1;
   a.state = state; a.out = out;
   a.seq_start = seq_start; a.seq_pos0 = seq_pos0; a.seq_len = seq_len; a.seq_slot = seq_slot;
   a.H = heads; a.G = heads; a.d = dim; a.dv = vdim; a.qscale = 1.f; a.divide = 0;

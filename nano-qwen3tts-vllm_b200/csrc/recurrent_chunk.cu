@@ -19,7 +19,7 @@
 //
 // Bound: the chain of chunks (about 510 m16n8k16 per warp and chunk, each waiting for its fragments; the tensor pipe is 19 % busy).
 // 4 sequences x 2048 tokens, 64 heads of 64 values x 128 channels: 527 us, token by token 3392 us; one sequence of 300 tokens with
-// convolution and norm 100 / 229 us, of 24 tokens 70 / 73 us, of 2 tokens 93 / 95 us (launches), so every portion takes this path.
+// convolution and norm 100 / 229 us; short portions stay with the token-by-token kernel, see linear_walk_len().
 // Error of the outputs against 64 bits over 1024 tokens 8.8e-8 of their norm, token by token 8.4e-8 (plain chains of MMAs
 // and scalars formed in float: 2.0e-7).
 #include "scan.cuh"
@@ -109,7 +109,7 @@ linear_chunk_kernel(const ScanArgs a) {
   ChunkTiles<D>& sm = *reinterpret_cast<ChunkTiles<D>*>(ck_smem);
   const int b = blockIdx.z, h = blockIdx.y, p0 = blockIdx.x * CK_P;
   const int len = a.seq_len[b];
-  if (len <= 1) return;
+  if (len < a.min_len) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g4 = lane >> 2, c2 = 2 * (lane & 3);
   const int H = a.H, dv = a.dv, g = h / (H / a.G);
   const size_t start = a.seq_start[b];
@@ -402,7 +402,7 @@ delta_chunk_kernel(const ScanArgs a) {
   Sm& sm = *reinterpret_cast<Sm*>(ck_smem);
   const int b = blockIdx.z, h = blockIdx.y, p0 = blockIdx.x * CK_P;
   const int len = a.seq_len[b];
-  if (len <= 1) return;
+  if (len < a.min_len) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wp = warp & 3, wh = warp >> 2, g4 = lane >> 2, c2 = 2 * (lane & 3);
   const int H = a.H, dv = a.dv, g = h / (H / a.G);
   const size_t start = a.seq_start[b];
@@ -801,6 +801,26 @@ delta_chunk_kernel(const ScanArgs a) {
 bool scan_chunk_applies(const ScanArgs& a) {
   return (a.d == 64 || a.d == 128) && a.dv % CK_P == 0 && a.ldq % 8 == 0 && a.ldk % 8 == 0 && a.ldv % 8 == 0 && aligned16(a.q) &&
          aligned16(a.k) && aligned16(a.v) && a.head_decay == nullptr && !a.divide;
+}
+
+// The longest portion that is left to the token-by-token kernel.  A chunk costs the same whatever the portion's length, a token of the
+// other kernel the same whatever its place, so each size has one crossing; it lies elsewhere while the CTAs are fewer than the
+// multiprocessors (both kernels wait for their own chain) than above (both wait for their turn).  Token by token / in chunks, us, behind
+// and in front of the lines (portions x tokens):
+//   state space   128 channels, 64 heads    4 x 14 26 / 23    16 x 14 67 / 67    64 x 14 269 / 234    64 x 10 208 / 227
+//                 64 channels, 32 heads     64 x 24 90 / 79   64 x 18 72 / 79
+//   delta rule    128 channels, 16 heads    8 x 24 48 / 38    16 x 24 74 / 69    64 x 24 258 / 243    64 x 20 217 / 240
+//                 64 channels, 32 heads     16 x 48 67 / 61   64 x 48 228 / 207  64 x 32 156 / 202
+static int64_t chunk_ctas(const ScanArgs& a, int n_seqs) { return static_cast<int64_t>(n_seqs) * a.H * (a.dv / CK_P); }
+int linear_walk_len(const ScanArgs& a, int n_seqs) {
+  const int64_t ctas = chunk_ctas(a, n_seqs), sms = sm_count();
+  if (a.d == 128) return ctas <= sms ? 24 : ctas <= 2 * sms ? 10 : 12;
+  return ctas <= sms ? 26 : 20;
+}
+int delta_walk_len(const ScanArgs& a, int n_seqs) {
+  const int64_t ctas = chunk_ctas(a, n_seqs), sms = sm_count();
+  if (a.d == 128) return ctas <= sms ? 19 : ctas <= 2 * sms ? 16 : 21;
+  return ctas <= sms ? 28 : 40;
 }
 
 template <int D>

@@ -1,6 +1,8 @@
 // scan.cuh - the arguments of the recurrent scans (recurrent.cu token by token, recurrent_chunk.cu in chunks).
 #pragma once
 
+#include <climits>
+
 #include "row_ops.cuh"
 
 namespace b2 {
@@ -13,7 +15,7 @@ struct ScanArgs {
   const float* coef;                      // [rows, H, 3] per-token scalars, see scan_kernel (SCAN_GATED: unused); the chunk kernels
                                           // read (decay, write scale, log of the decay)
   const float* head_decay;                // [H] or null: coef = (head_decay[h], 1, 1) for every token (coef itself is then unused)
-  int rows;                               // 0: every sequence, 1: only those with more than one new token, 2: only one-token ones
+  int min_len = 1, max_len = INT_MAX;     // only sequences with so many new tokens
   const float* decay; int64_t ldd;        // SCAN_GATED: per key channel, (row, head h, i) at decay[row * ldd + h * d + i]
   const float* skip;                      // [H] or null: out += skip[h] * value
   float* state;                           // [slots, H, d, dv]
@@ -24,8 +26,11 @@ struct ScanArgs {
   int divide;                             // linear: out = S^T q * qscale / coef[2] instead of S^T q * qscale
 };
 
-// bf16 portions in chunks on the tensor cores: which sizes and layouts, and the launches (sequences with more than one token)
+// bf16 portions in chunks on the tensor cores: which sizes and layouts, the longest portion that is faster token by token, and the
+// launches (sequences of min_len tokens and more)
 bool scan_chunk_applies(const ScanArgs& a);
+int linear_walk_len(const ScanArgs& a, int n_seqs);
+int delta_walk_len(const ScanArgs& a, int n_seqs);
 int launch_linear_chunk(const char* what, const ScanArgs& a, int n_seqs, cudaStream_t st);
 int launch_delta_chunk(const char* what, const ScanArgs& a, int n_seqs, cudaStream_t st);
 

@@ -244,3 +244,28 @@ def test_scalars_of_one_token_steps_are_float(nat, kind, dtype):
     want = state * decay[:, :, None, None]
     run(nat, [(9, 1, i) for i in range(64)], torch.zeros_like(x[:, 0]).to(dtype), gates, state)
     assert torch.equal(state, want)
+
+
+@pytest.mark.parametrize("kind", ["ssm", "delta"])
+def test_short_portions_are_walked_token_by_token(nat, kind):
+    """A portion of a few tokens gives the bits of as many one-token steps, alone, beside others and beside a portion that runs in chunks."""
+    x, gates, _, run, H, G = _inputs(kind, (6, 300), 1)
+    for n in (2, 6, 12):
+        long = 300
+        state = torch.zeros(7, H, 128, 64, device=DEV)
+        steps = torch.stack([run(nat, [(t, 1, i) for i in range(5)], x[:5, t].contiguous(), gates[:5, t].contiguous(), state) for t in range(n)], 1)
+        for seqs in ([(0, n, i) for i in range(5)], [(0, n, i) for i in range(5)] + [(0, long, 5)]):
+            rows = lambda v: torch.cat([v[i, :m] for i, (_, m, _) in enumerate(seqs)])
+            whole = torch.zeros_like(state)
+            out = run(nat, seqs, rows(x), rows(gates), whole)
+            assert torch.equal(out[:5 * n].view(5, n, -1), steps) and torch.equal(whole[:5], state[:5])
+
+
+@pytest.mark.parametrize("D,P", [(128, 64), (64, 128)])
+@pytest.mark.parametrize("n", [25, 33, 41, 49, 79, 80, 81, 95, 112, 127])
+def test_last_chunks_of_every_number_of_blocks(nat, n, D, P):
+    """Portions just above what is walked, and last chunks on either side of each block of 16 tokens."""
+    for case in _ssm_case(nat, [(0, n, 1), (9, n, 0)], 2, 1, P, D, seed=n):
+        _check(*case, n)
+    for case in _delta_case(nat, [(0, n, 1), (9, n, 0)], 2, 1, D, P, seed=n):
+        _check_delta(*case, n)
