@@ -69,6 +69,10 @@ __device__ __forceinline__ float exp_sum(double x) {
   return fmaf(e, static_cast<float>(x - hi), e);
 }
 
+// A log decay as it enters the sums.  e^l is 0 in float below -104; taken as it comes, a very large l would leave the running sum of
+// doubles no bits for the decays behind it (from |l| = 1e12 on), so it is cut at a value that gives the same products.
+__device__ __forceinline__ float cut_log(float l) { return fmaxf(l, -200.f); }
+
 // Scalars of the chunk that starts at token t0, by one warp: lane l holds tokens 2 l, 2 l + 1.
 template <int D>
 __device__ __forceinline__ void chunk_scalars(ChunkTiles<D>& sm, int s, const float* cp, int H, int t0, int len, int lane) {
@@ -79,6 +83,7 @@ __device__ __forceinline__ void chunk_scalars(ChunkTiles<D>& sm, int s, const fl
     if (t < len) { w[e] = cp[static_cast<size_t>(t) * H * 3 + 1]; l[e] = cp[static_cast<size_t>(t) * H * 3 + 2]; }
   }
   const bool fine = fabsf(l[0]) < 1e30f && fabsf(l[1]) < 1e30f && fabsf(w[0]) < 1e6f && fabsf(w[1]) < 1e6f;
+  l[0] = cut_log(l[0]); l[1] = cut_log(l[1]);
   double c1 = static_cast<double>(l[0]) + l[1], x;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -448,6 +453,7 @@ delta_chunk_kernel(const ScanArgs a) {
   };
   auto sum_coef = [&](int s) {
     const bool fine = fabsf(cl[0]) < 1e30f && fabsf(cl[1]) < 1e30f && fabsf(cb_[0]) < 1e6f && fabsf(cb_[1]) < 1e6f;
+    cl[0] = cut_log(cl[0]); cl[1] = cut_log(cl[1]);
     double c1 = static_cast<double>(cl[0]) + cl[1], x;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {

@@ -1,6 +1,8 @@
 """Recurrences of prompt portions in chunks on the tensor cores against the 64-bit recurrence token by token: portions around the
 chunk's edges, carried state, one-token and padding rows beside them, decays from none to total, numbers outside the range of the
 three-part split."""
+import math
+
 import pytest
 import torch
 
@@ -45,12 +47,21 @@ def _ssm_reference(x, B, C, dt, la, D, S):
     return torch.stack(ys), S, torch.stack(ya), A
 
 
-def _ssm_case(nat, seqs, H, G, P, N, seed=0, a_log=None, big=None):
+def _strong_gates(x, a_log, rows):
+    """Gate pre-activations whose decays are e^-1 or so, but for a token in 23 with about e^(-0.7 e^a_log)."""
+    x = 0.5 * x - a_log
+    x[5 % rows::23] = 0.0
+    return x
+
+
+def _ssm_case(nat, seqs, H, G, P, N, seed=0, a_log=None, big=None, strong=False):
     g = torch.Generator(device=DEV).manual_seed(seed)
     r = lambda *s: torch.randn(s, generator=g, device=DEV)
     lay = Lay(seqs)
     n = lay.n_tokens
     xbc, dt_in = r(n, H * P + 2 * G * N).to(torch.bfloat16), r(n, H).to(torch.bfloat16)
+    if strong:
+        dt_in = _strong_gates(dt_in.float(), a_log, n).to(torch.bfloat16)
     if big is not None:
         row, col, value = big
         xbc[row, col] = value
@@ -103,6 +114,13 @@ def test_state_space_extreme_decays(nat, a_log):
         _check(*case, 150)
 
 
+@pytest.mark.parametrize("magnitude", [1e6, 1e9, 1e12, 1e16, 1e20, 1e30])
+def test_state_space_gates_far_beyond_a_total_decay(nat, magnitude):
+    """The token forgets everything; what the tokens behind it forget is as little as ever."""
+    for case in _ssm_case(nat, [(7, 150, 0)], 2, 1, 64, 128, seed=3, a_log=math.log(magnitude), strong=True):
+        _check(*case, 150)
+
+
 @pytest.mark.parametrize("value", [float("inf"), float("nan"), 1e30])
 def test_state_space_numbers_outside_the_split(nat, value):
     """They reach the outputs that the recurrence carries them to - the head and value column, from their token on - and the rest of
@@ -137,7 +155,7 @@ def _delta_reference(q, k, v, beta, la, S):
     return torch.stack(ys), S
 
 
-def _delta_case(nat, seqs, H, G, D, P, seed=0, a_log=None, alike=0.0, big=None):
+def _delta_case(nat, seqs, H, G, D, P, seed=0, a_log=None, alike=0.0, big=None, strong=False):
     g = torch.Generator(device=DEV).manual_seed(seed)
     r = lambda *s: torch.randn(s, generator=g, device=DEV)
     lay = Lay(seqs)
@@ -145,6 +163,8 @@ def _delta_case(nat, seqs, H, G, D, P, seed=0, a_log=None, alike=0.0, big=None):
     qkv = r(n, 2 * G * D + H * P)
     qkv[:, G * D:2 * G * D] += alike * r(1, G * D)             # keys that point the same way: the solve's off-diagonal is dense
     qkv, ba = qkv.to(torch.bfloat16), r(n, 2 * H).to(torch.bfloat16)
+    if strong:
+        ba[:, H:] = _strong_gates(ba[:, H:].float(), a_log, n).to(torch.bfloat16)
     if big is not None:
         row, col, value = big
         qkv[row, col] = value
@@ -193,6 +213,12 @@ def test_delta_rule_portions_beside_single_tokens_and_padding(nat):
 @pytest.mark.parametrize("a_log,alike", [(-30.0, 0.0), (6.0, 0.0), (-30.0, 4.0), (-30.0, 100.0)])
 def test_delta_rule_extreme_decays_and_keys_that_point_the_same_way(nat, a_log, alike):
     for case in _delta_case(nat, [(7, 150, 0)], 2, 1, 128, 64, seed=1, a_log=a_log, alike=alike):
+        _check_delta(*case, 150)
+
+
+@pytest.mark.parametrize("magnitude", [1e6, 1e9, 1e12, 1e16, 1e20, 1e30])
+def test_delta_rule_gates_far_beyond_a_total_decay(nat, magnitude):
+    for case in _delta_case(nat, [(7, 150, 0)], 2, 1, 128, 64, seed=3, a_log=math.log(magnitude), strong=True):
         _check_delta(*case, 150)
 
 
