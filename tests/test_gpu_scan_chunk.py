@@ -295,3 +295,38 @@ def test_last_chunks_of_every_number_of_blocks(nat, n, D, P):
         _check(*case, n)
     for case in _delta_case(nat, [(0, n, 1), (9, n, 0)], 2, 1, D, P, seed=n):
         _check_delta(*case, n)
+
+
+@pytest.mark.parametrize("kind", ["delta"])
+@pytest.mark.parametrize("D,P", [(128, 64), (64, 64)])
+def test_no_precision_is_given_up_in_chunks(nat, kind, D, P):
+    """The norms of the errors against 64 bits over 512 tokens, outputs and state, are on average over eight inputs of three sizes not above
+    the token-by-token kernel's (the same inputs in portions of 10), which are about 1e-7.  Without the third part of a split it is 1.4 times
+    that (state against queries and keys) to 2e-6 (weights, update)."""
+    B, n, totals = 2, 512, torch.zeros(4, dtype=F64)
+    for seed in range(1, 9):
+        x, gates, (a_log, bias, skip), run, H, G = _inputs(kind, (B, n), seed, (1.0, 0.3, 3.0)[seed % 3], D, P)
+        state = torch.zeros(B, H, D, P, device=DEV)
+        out = run(nat, [(0, n, i) for i in range(B)], x.view(B * n, -1), gates.view(B * n, -1), state).view(B, n, H, P)
+        walked_state, walked = torch.zeros_like(state), []
+        for t in range(0, n, 10):
+            m = min(10, n - t)
+            walked.append(run(nat, [(t, m, i) for i in range(B)], x[:, t:t + m].reshape(B * m, -1), gates[:, t:t + m].reshape(B * m, -1),
+                              walked_state).view(B, m, H, P))
+        # both sequences at once, as heads of one
+        X, u = x.to(F64).transpose(0, 1), gates.to(F64).transpose(0, 1)
+        heads = lambda t, h: t.reshape(n, B * h, -1)
+        S0 = torch.zeros(B * H, D, P, dtype=F64, device=DEV)
+        if kind == "ssm":
+            dt = torch.nn.functional.softplus(u + bias.to(F64))
+            y, S, _, _ = _ssm_reference(heads(X[..., :H * P], H), heads(X[..., H * P:H * P + D], 1), heads(X[..., H * P + D:], 1), dt.reshape(n, -1),
+                                        (-torch.exp(a_log.to(F64)) * dt).reshape(n, -1), skip.to(F64).repeat(B), S0)
+        else:
+            la = -torch.exp(a_log.to(F64)) * torch.nn.functional.softplus(u[..., H:] + bias.to(F64))
+            y, S = _delta_reference(heads(X[..., :G * D], G), heads(X[..., G * D:2 * G * D], G), heads(X[..., 2 * G * D:], H),
+                                    torch.sigmoid(u[..., :H]).reshape(n, -1), la.reshape(n, -1), S0)
+        y, S = y.view(n, B, H, P).transpose(0, 1), S.view(B, H, D, P)
+        err = lambda a, b: ((a.to(F64) - b).norm() / b.norm()).item()
+        totals += torch.tensor([err(out, y), err(torch.cat(walked, 1), y), err(state, S), err(walked_state, S)], dtype=F64)
+    chunk, walk, chunk_state, walk_state = (totals / 8).tolist()
+    assert chunk <= walk and chunk_state <= walk_state and max(chunk, chunk_state) < 1.5e-7, (chunk, walk, chunk_state, walk_state)
