@@ -10,18 +10,17 @@
 // TRANSPOSED in its accumulators (columns of S x key channels) across the chunks, where it is at once the A operand of S^T q and the
 // accumulator of the update, so that the state never crosses shared memory and warps only meet over the chunk's weights.
 //
-// No precision is given up against the token-by-token kernel: q, k and v are bf16 and enter their products exactly; the state, the
-// weights and the weighted values are floats and enter as THREE bf16 parts (24 bits), one MMA each, the small parts first (the
-// tensor core truncates its sums: what is added while they are small costs nothing), the large ones summed outside; c is summed in
-// double.
+// No precision is given up against the token-by-token kernel (outputs 7.9e-8 of their norm from 64 bits and the state 7.0e-8, that
+// one's 8.5e-8 and 8.1e-8: means over 512 tokens of eight inputs of three sizes; plain chains of MMAs 2.0e-7).  q, k and v are bf16
+// and enter their products exactly; the state, the weights and the weighted values are floats and enter as THREE bf16 parts (24
+// bits), one MMA each, the small parts first (the tensor core truncates its sums: what is added while they are small costs
+// nothing), the large ones summed outside; c is summed in double.
 // Numbers that the split could not represent (not finite, or so large that a product might overflow) send their chunk through a
 // token-by-token walk over the same registers, so that an infinity reaches the outputs it reaches there and no others.
 //
-// Bound: the chain of chunks (about 510 m16n8k16 per warp and chunk, each waiting for its fragments; the tensor pipe is 19 % busy).
-// 4 sequences x 2048 tokens, 64 heads of 64 values x 128 channels: 527 us, token by token 3392 us; one sequence of 300 tokens with
-// convolution and norm 100 / 229 us; short portions stay with the token-by-token kernel, see linear_walk_len().
-// Error of the outputs against 64 bits over 1024 tokens 8.8e-8 of their norm, token by token 8.4e-8 (plain chains of MMAs
-// and scalars formed in float: 2.0e-7).
+// Bound: the chain of chunks (about 620 m16n8k16 per warp and chunk, each waiting for its fragments; most of a chunk's work does not
+// depend on the state in front of it, but sits in the chain).  4 sequences x 2048 tokens, 64 heads of 64 values x 128 channels: 574 us,
+// token by token 3371 us; one sequence of 300 tokens 79 / 186 us.  Short portions stay with that kernel, see linear_walk_len().
 #include "scan.cuh"
 
 namespace b2 {
@@ -53,6 +52,13 @@ __device__ __forceinline__ void mma_add(float* c, const uint32_t* a, uint32_t b0
   mma_bf16_16816(t, a, b0, b1);
 #pragma unroll
   for (int e = 0; e < 4; ++e) c[e] += t[e];
+}
+
+// two bf16 in two pairs: the upper four of their significant bits, and the rest (exact)
+__device__ __forceinline__ void halves(uint32_t x, uint32_t& head, uint32_t& tail) {
+  head = x & 0xfff0fff0u;
+  const __nv_bfloat162 r = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&x), *reinterpret_cast<const __nv_bfloat162*>(&head));
+  tail = *reinterpret_cast<const uint32_t*>(&r);
 }
 
 template <int D> struct ChunkTiles {
@@ -208,25 +214,35 @@ linear_chunk_kernel(const ScanArgs a) {
     const uint32_t q_u = smem_u32(sm.q[s]), k_u = smem_u32(sm.k[s]), v_u = smem_u32(sm.v[s]);
     // ---- weights of rows 16 warp .. + 15: scores against the keys up to the diagonal, decay and write scale, in three parts
     if (warp * 16 < L) {
-      float sc[8][4];
+      // the upper halves of q's significant bits give sums of 16 products that a float nearly always holds, the lower ones small sums:
+      // what the tensor core cuts off is a sixteenth (outputs 8.8e-8 -> 7.9e-8 from 64 bits, 12 of 574 us)
+      float sc[8][4], st[8][4];
 #pragma unroll
       for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) sc[nt][e] = 0.f;
+        for (int e = 0; e < 4; ++e) sc[nt][e] = st[nt][e] = 0.f;
 #pragma unroll
       for (int ks = 0; ks < D / 16; ++ks) {
-        uint32_t af[4];
+        uint32_t af[4], hf[4], tf[4];
         ldsm4(af, q_u + tile_off(warp * 16 + ra, ks * 2 + ca, RB));
+#pragma unroll
+        for (int e = 0; e < 4; ++e) halves(af[e], hf[e], tf[e]);
 #pragma unroll
         for (int np = 0; np < 4; ++np) {
           if (np <= warp) {
             uint32_t bf[4];
             ldsm4(bf, k_u + tile_off(np * 16 + rb, ks * 2 + cb, RB));
-            mma_add(sc[2 * np], af, bf[0], bf[1]);
-            mma_add(sc[2 * np + 1], af, bf[2], bf[3]);
+            mma_bf16_16816(st[2 * np], tf, bf[0], bf[1]);
+            mma_bf16_16816(st[2 * np + 1], tf, bf[2], bf[3]);
+            mma_add(sc[2 * np], hf, bf[0], bf[1]);
+            mma_add(sc[2 * np + 1], hf, bf[2], bf[3]);
           }
         }
       }
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sc[nt][e] += st[nt][e];
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         const int i = warp * 16 + g4 + 8 * half;
@@ -331,13 +347,15 @@ linear_chunk_kernel(const ScanArgs a) {
         }
     }
     // ---- the state behind the chunk: what the chunk adds is summed by itself, then S <- e^(c_L) S + sum with one rounding
-    uint32_t af[4][3][4];
+    uint32_t af[4][4][4];
 #pragma unroll
     for (int js = 0; js < 4; ++js)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {                                                 // registers 0, 1: tokens c2, c2 + 1; 2, 3: eight further on
         const int j = js * 16 + (e >> 1) * 8 + c2;
-        split3(bf16lo(vf[js][e]) * sm.wl[s][j], bf16hi(vf[js][e]) * sm.wl[s][j + 1], af[js][0][e], af[js][1][e], af[js][2][e]);
+        uint32_t hi;
+        split3(bf16lo(vf[js][e]) * sm.wl[s][j], bf16hi(vf[js][e]) * sm.wl[s][j + 1], hi, af[js][2][e], af[js][3][e]);
+        halves(hi, af[js][0][e], af[js][1][e]);                                     // as above: state 7.4e-8 -> 7.0e-8, 28 us
       }
     const float gl = sm.ecum[s][CK_L - 1];                                          // log decays behind the portion's end are zero
 #pragma unroll
@@ -348,7 +366,7 @@ linear_chunk_kernel(const ScanArgs a) {
       for (int js = 0; js < 4; ++js)
         if (js * 16 < L) ldsm4t(bf[js], k_u + tile_off(js * 16 + rt, np * 2 + ct, RB));
 #pragma unroll
-      for (int part = 2; part >= 0; --part)
+      for (int part = 3; part >= 0; --part)
 #pragma unroll
         for (int js = 0; js < 4; ++js)
           if (js * 16 < L) {

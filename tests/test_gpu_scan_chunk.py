@@ -297,7 +297,7 @@ def test_last_chunks_of_every_number_of_blocks(nat, n, D, P):
         _check_delta(*case, n)
 
 
-@pytest.mark.parametrize("kind", ["delta"])
+@pytest.mark.parametrize("kind", ["ssm", "delta"])
 @pytest.mark.parametrize("D,P", [(128, 64), (64, 64)])
 def test_no_precision_is_given_up_in_chunks(nat, kind, D, P):
     """The norms of the errors against 64 bits over 512 tokens, outputs and state, are on average over eight inputs of three sizes not above
