@@ -8,8 +8,8 @@
 // them in a fixed order.  Inputs are bf16 or float, products accumulate in float.  A tile never mixes two experts:
 // tile y of the grid is mapped to (expert, row block) by walking the group sizes, and tiles beyond the last group exit.
 //
-// bf16 groups of more than a few rows run on the tcgen05 kernel of grouped_gemm_tc.cu; the kernels here take decode-sized groups,
-// float and odd sizes.
+// bf16 groups of more than a few rows run on the tcgen05 kernel of grouped_gemm_tc.cu; the kernels here take decode-sized groups, small
+// products, float and odd sizes.
 //
 // Gated experts (grouped_gemm_gated, grouped_gemm_silu): W[e] is [gate; up], 2 ff rows.  A tile's 128 rows of W are 8 gate rows and the 8 matching
 // up rows in turn, so a thread's accumulators hold the gate and the up value of the same columns and the clamped gated product
@@ -292,7 +292,7 @@ extern "C" int b2tts_grouped_gemm(const void* a, int64_t lda, const void* w, voi
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // bf16 with 16-byte rows: the tensor-core kernels; float (true 32-bit products) and odd sizes: the plain one
   if (dtype == B2TTS_DTYPE_BF16 && k % 8 == 0 && lda % 8 == 0 && aligned16(a) && aligned16(w)) {
-    if (grouped_tc_applies(n_pairs, experts, n, n, ldc, c))
+    if (grouped_tc_applies(n_pairs, experts, n, k, false, in_by_token, ldc, c))
       return launch_grouped_tc("grouped_gemm", a, lda, w, c, ldc, offsets, sorted_pair, n_pairs, experts, n, k, top, in_by_token, out_by_pair,
                                act, 0.f, 0.f, st);
     // groups of a decode step (16 rows per expert on average, or fewer): the 32-row shape
@@ -326,7 +326,7 @@ extern "C" int b2tts_grouped_gemm_gated(const void* a, int64_t lda, const void* 
   if (const int rc = grouped_tc_check("grouped_gemm_gated")) return rc;
   B2_REQUIRE(aligned16(a) && aligned16(w) && aligned16(c), B2TTS_EALIGN, "grouped_gemm_gated: pointers must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (grouped_tc_applies(n_pairs, experts, ff, 2 * ff, ldc, c))
+  if (grouped_tc_applies(n_pairs, experts, 2 * ff, k, true, true, ldc, c))
     return launch_grouped_tc("grouped_gemm_gated", a, lda, w, c, ldc, offsets, sorted_pair, n_pairs, experts, 2 * ff, k, top, 1, 0, GG_CLAMPED, limit,
                              alpha, st);
   const bool small = n_pairs <= 16 * experts;
@@ -348,7 +348,7 @@ extern "C" int b2tts_grouped_gemm_silu(const void* a, int64_t lda, const void* w
   if (const int rc = grouped_tc_check("grouped_gemm_silu")) return rc;
   B2_REQUIRE(aligned16(a) && aligned16(w) && aligned16(c), B2TTS_EALIGN, "grouped_gemm_silu: pointers must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (grouped_tc_applies(n_pairs, experts, ff, 2 * ff, ldc, c))
+  if (grouped_tc_applies(n_pairs, experts, 2 * ff, k, true, true, ldc, c))
     return launch_grouped_tc("grouped_gemm_silu", a, lda, w, c, ldc, offsets, sorted_pair, n_pairs, experts, 2 * ff, k, top, 1, 0, GG_SILU, 0.f, 0.f, st);
   const bool small = n_pairs <= 16 * experts;
   const cudaError_t e = small ? launch_grouped_mma<32, GG_SILU>(n_pairs, st, a, lda, w, c, ldc, offsets, sorted_pair, experts, 2 * ff, k, top, 1, 0)

@@ -14,8 +14,8 @@ __device__ __forceinline__ float gated_value(float gate, float up, float limit, 
   return clamped_gate(gate, up, limit, alpha);
 }
 
-// the tcgen05 kernel's range: n = output columns, w_rows = rows of W per expert, see grouped_gemm_tc.cu
-bool grouped_tc_applies(int n_pairs, int experts, int n, int w_rows, int64_t ldc, const void* c);
+// the tcgen05 kernel's range (w_rows = rows of W per expert), see grouped_gemm_tc.cu
+bool grouped_tc_applies(int n_pairs, int experts, int w_rows, int k, bool gated, bool in_by_token, int64_t ldc, const void* c);
 // an error, once, when a wait inside an earlier launch has run out
 int grouped_tc_check(const char* what);
 // `n` = rows of W per expert (twice the output columns from GG_CLAMPED on)

@@ -225,15 +225,32 @@ grouped_gemm_tc_kernel(const GroupedTcArgs p, const __grid_constant__ CUtensorMa
   }
 }
 
-// Rows per expert, on average, from which this kernel is the faster one.  Whole feed-forward, 16 experts of 3072 x 2048, the
-// decode-sized kernel of grouped_gemm.cu against this one: 2 rows 144 / 159 us, 8 rows 149 / 151, 16 rows 156 / 149; above, that
-// file's 128-row tiles: 276 / 151 us at 16.1 rows, 302 / 149 at 50, 474 / 182 at 125, 2410 / 709 at 1024.  Sizes that do not
-// fill 16-byte output vectors stay there.
-constexpr int TC_MIN_ROWS = 12;
-
-bool grouped_tc_applies(int n_pairs, int experts, int n, int w_rows, int64_t ldc, const void* c) {
-  return n_pairs > TC_MIN_ROWS * static_cast<int64_t>(experts) && n % 8 == 0 && ldc % 8 == 0 && aligned16(c) &&
-         static_cast<int64_t>(experts) * w_rows < (1ll << 31);             // rows of W are 32-bit coordinates
+// Where this kernel is the faster one.  A tile costs it about 4 us of start and end (gathered rows 5, gated sums 10: one warp a
+// scheduler forms 128 columns of them) and then little per slice of K; the kernels of grouped_gemm.cu start in 3 us and pay more per
+// slice, and more when their 128-row tiles are mostly empty.  So what decides is K, and with a short K how many of their 128-column
+// tiles there are to spread over the GPU.  Measured over 4 to 256 experts, K 64 to 4096, 64 to 6144 rows of W and 13 to 1024 rows an
+// expert (4566 shapes, weights cold): always this kernel is 10 % from the faster of the two on average, this rule 0.7 %.  Some of the
+// lines, here / there in us:
+//   more than 16 rows an expert   gated     16 experts, 256 rows of W, 32 rows     K 256 14 / 9      K 1024 20 / 22    K 2048 34 / 41
+//                                           64 experts, 1024 rows of W, 128 rows   K 64 36 / 27      K 256 37 / 40     K 1024 53 / 107
+//                                 gathered  64 experts, 512 rows of W, 17 rows     K 64 13 / 9       K 256 14 / 13     K 1024 22 / 33
+//   13 to 16 rows (32-row tiles)  gated     16 experts, 6144 rows of W             K 2048 102 / 84   (128 experts, 1536 rows of W, K 768: 80 / 98)
+//                                 gathered  16 experts, 2048 rows of W             K 1024 21 / 18    K 2048 32 / 31
+//                                 in order  16 experts, 6144 rows of W             K 1024 39 / 45    K 2048 70 / 82
+// Sizes that do not fill 16-byte output vectors, rows of W that a copy's 32-bit coordinates cannot name and rows shorter than one
+// slice stay there too.
+bool grouped_tc_applies(int n_pairs, int experts, int w_rows, int k, bool gated, bool in_by_token, int64_t ldc, const void* c) {
+  const int64_t e = experts, col_tiles = (w_rows + 127) / 128;
+  if (n_pairs <= 12 * e || k < G_BK || (gated ? w_rows / 2 : w_rows) % 8 != 0 || ldc % 8 != 0 || !aligned16(c) || e * w_rows >= (1ll << 31))
+    return false;
+  if (n_pairs <= 16 * e) {
+    const int64_t tiles = (e + n_pairs / 32) * col_tiles;
+    if (gated) return e >= 128 && tiles >= 1200;
+    return in_by_token ? (e >= 64 && tiles >= 700) || (k >= 1536 && tiles <= 70) : k > 640 || tiles >= 600;
+  }
+  const int64_t tiles = (e + n_pairs / 128) * col_tiles;
+  if (gated) return k >= 768 || (k >= 128 && tiles * k >= 280000) || (w_rows <= 64 && n_pairs > 24 * e);
+  return k >= 192 || tiles * k >= 40000;
 }
 
 static int* timeouts_word() {

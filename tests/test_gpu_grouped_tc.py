@@ -114,6 +114,60 @@ def test_several_tiles_per_cta(nat, k):
     assert nat.grouped_gemm_timeouts() == 0
 
 
+@pytest.mark.parametrize("sizes", [(129, 0, 1, 127, 128), (600, 33), (1, 1, 1, 700)])
+@pytest.mark.parametrize("n,k", [(8, 192), (264, 200), (136, 712)])
+@pytest.mark.parametrize("ff,kg", [(8, 768), (136, 776), (264, 840), (32, 72)])
+def test_edges_at_the_inner_sizes_of_the_tensor_core_kernel(nat, sizes, n, k, ff, kg):
+    """The same edges of rows and columns with K long enough (and gated rows of W few enough) for that kernel to be chosen."""
+    top, E = 2, len(sizes)
+    if sum(sizes) % top:
+        sizes = sizes[:-1] + (sizes[-1] + 1,)
+    off, pair, pairs = _groups(sizes, top, n + k)
+    g = torch.Generator(device=DEV).manual_seed(k)
+    r = lambda *s: torch.randn(s, generator=g, device=DEV).to(torch.bfloat16)
+    tok, w, y, tg = r(pairs // top, k), r(E, n, k), r(pairs, k), r(pairs // top, kg)
+    wg = (r(E, 2 * ff, kg) * kg ** -0.5).to(torch.bfloat16)
+    new = lambda cols: torch.full((pairs, cols), 7.0, device=DEV, dtype=torch.bfloat16)
+    gathered, boxed, silu, clamped = new(n), new(n), new(ff), new(ff)
+    nat.grouped_gemm(tok, w, gathered, off, pair, pairs, top, in_by_token=True, out_by_pair=False, act=1)
+    nat.grouped_gemm(y, w, boxed, off, pair, pairs, top, in_by_token=False, out_by_pair=True, act=0)
+    nat.grouped_gemm_silu(tg, wg, silu, off, pair, pairs, top)
+    nat.grouped_gemm_gated(tg, wg, clamped, off, pair, pairs, top, 1.5)
+    for e in range(E):
+        rows = slice(off[e].item(), off[e + 1].item())
+        token = (pair[rows] // top).long()
+        _close(gathered[rows], (tok[token].double() @ w[e].double().T).clamp(min=0) ** 2, k)
+        _close(boxed[pair[rows].long()], y[rows].double() @ w[e].double().T, k)
+        gu = tg[token].double() @ wg[e].double().T
+        gate, up = gu[:, :ff], gu[:, ff:]
+        _close(silu[rows], torch.nn.functional.silu(gate) * up, kg)
+        gate, up = gate.clamp(max=1.5), up.clamp(-1.5, 1.5)
+        _close(clamped[rows], gate * torch.sigmoid(1.702 * gate) * (up + 1), kg)
+    nat.check_waits()
+
+
+@pytest.mark.parametrize("rows", [12, 13, 16, 17, 24, 25])
+@pytest.mark.parametrize("n,k", [(64, 64), (64, 184), (64, 192), (256, 648), (1032, 640), (520, 768)])
+def test_both_sides_of_the_choice_of_kernel(nat, rows, n, k):
+    """Rows an expert and inner sizes on either side of each line of the rule, gathered, in order and gated."""
+    E, top, pairs = 6, 2, 6 * rows
+    off, pair, _ = _groups((rows,) * E, top, rows)
+    g = torch.Generator(device=DEV).manual_seed(n + k)
+    r = lambda *s: torch.randn(s, generator=g, device=DEV).to(torch.bfloat16)
+    tok, w, y = r(pairs // top, k), (r(E, n, k) * k ** -0.5).to(torch.bfloat16), r(pairs, k)
+    a, b, c = (torch.empty(pairs, m, device=DEV, dtype=torch.bfloat16) for m in (n, n, n // 2))
+    nat.grouped_gemm(tok, w, a, off, pair, pairs, top, in_by_token=True, out_by_pair=False, act=0)
+    nat.grouped_gemm(y, w, b, off, pair, pairs, top, in_by_token=False, out_by_pair=True, act=0)
+    nat.grouped_gemm_silu(tok, w, c, off, pair, pairs, top) if n % 16 == 0 else None
+    for e in range(E):
+        s = slice(e * rows, (e + 1) * rows)
+        x = tok[(pair[s] // top).long()].double() @ w[e].double().T
+        _close(a[s], x, k)
+        _close(b[pair[s].long()], y[s].double() @ w[e].double().T, k)
+        if n % 16 == 0:
+            _close(c[s], torch.nn.functional.silu(x[:, :n // 2]) * x[:, n // 2:], k)
+
+
 def test_not_finite_values_stay_in_their_rows(nat):
     """A NaN in one row of the input reaches that row's outputs only, activation included."""
     off, pair, pairs = _groups((150, 90), 1, 3)
