@@ -369,9 +369,10 @@ extern "C" int b2tts_ssm_scan_portions(const void* xbc, int64_t ldx, const void*
   else launch_coef<float>(dt, nullptr, lddt, dt_bias, a_log, coef, n_tokens, heads, 0, st);
   B2_CHECK_LAUNCH("ssm_scan (scalars)");
   if (chunks) {
-    a.min_len = walk + 1;
+    const bool alone = n_seqs == 1 && max_new > 0;         // no second launch: max_new may be above its length, which is then taken too
+    a.min_len = alone ? 1 : walk + 1;
     const int rc = launch_linear_chunk("ssm_scan (portions)", a, n_seqs, st);
-    if (rc != B2TTS_OK || (n_seqs == 1 && max_new > 0)) return rc;
+    if (rc != B2TTS_OK || alone) return rc;
     a.min_len = 1; a.max_len = walk;                       // single tokens and short portions beside them
   }
   const int rc = dtype == B2TTS_DTYPE_BF16 ? launch_scan<__nv_bfloat16, SCAN_LINEAR>(a, n_seqs, st, "ssm_scan")
@@ -416,9 +417,10 @@ extern "C" int b2tts_delta_rule_scan_portions(const void* qkv, int64_t ldq, cons
   else launch_coef<float>(beta, a_in, ldu, a_log, dt_bias, coef, n_tokens, heads, 1, st);
   B2_CHECK_LAUNCH("delta_rule_scan (scalars)");
   if (chunks) {
-    a.min_len = walk + 1;
+    const bool alone = n_seqs == 1 && max_new > 0;         // no second launch: max_new may be above its length, which is then taken too
+    a.min_len = alone ? 1 : walk + 1;
     const int rc = launch_delta_chunk("delta_rule_scan (portions)", a, n_seqs, st);
-    if (rc != B2TTS_OK || (n_seqs == 1 && max_new > 0)) return rc;
+    if (rc != B2TTS_OK || alone) return rc;
     a.min_len = 1; a.max_len = walk;                       // single tokens and short portions beside them
   }
   const int rc = dtype == B2TTS_DTYPE_BF16 ? launch_scan<__nv_bfloat16, SCAN_DELTA>(a, n_seqs, st, "delta_rule_scan")

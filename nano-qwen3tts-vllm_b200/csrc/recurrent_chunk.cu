@@ -855,22 +855,23 @@ bool scan_chunk_applies(const ScanArgs& a) {
 
 // The longest portion that is left to the token-by-token kernel.  A chunk costs the same whatever the portion's length, a token of the
 // other kernel the same whatever its place, so each size has one crossing; it lies elsewhere while the CTAs are fewer than the
-// multiprocessors (both kernels wait for their own chain) than above (both wait for their turn).  Token by token / in chunks, us, behind
-// and in front of the lines (portions x tokens):
-//   state space   128 channels, 64 heads    4 x 14 26 / 23    16 x 14 67 / 67    64 x 14 269 / 234    64 x 10 208 / 227
-//                 64 channels, 32 heads     64 x 24 90 / 79   64 x 18 72 / 79
-//   delta rule    128 channels, 16 heads    8 x 24 48 / 38    16 x 24 74 / 69    64 x 24 258 / 243    64 x 20 217 / 240
-//                 64 channels, 32 heads     16 x 48 67 / 61   64 x 48 228 / 207  64 x 32 156 / 202
+// multiprocessors (both kernels wait for their own chain) than above (both wait for their turn), and a little earlier for a portion
+// that is alone in its step, where no second kernel looks for short ones.  Token by token / in chunks, us, behind and in front of the
+// lines (portions x tokens); over 588 such steps the choice is within 5 % of the better kernel:
+//   state space   128 channels, 64 heads    1 x 24 20 / 17    4 x 14 28 / 22    16 x 14 67 / 68    64 x 14 269 / 235    64 x 10 208 / 233
+//                 64 channels, 32 heads     64 x 24 90 / 80   64 x 18 73 / 80
+//   delta rule    128 channels, 16 heads    8 x 24 50 / 38    16 x 24 76 / 69    64 x 24 258 / 244    64 x 20 217 / 241
+//                 64 channels, 32 heads     16 x 48 67 / 61   64 x 48 228 / 208  64 x 32 156 / 192
 static int64_t chunk_ctas(const ScanArgs& a, int n_seqs) { return static_cast<int64_t>(n_seqs) * a.H * (a.dv / CK_P); }
 int linear_walk_len(const ScanArgs& a, int n_seqs) {
   const int64_t ctas = chunk_ctas(a, n_seqs), sms = sm_count();
-  if (a.d == 128) return ctas <= sms ? 24 : ctas <= 2 * sms ? 10 : 12;
-  return ctas <= sms ? 26 : 20;
+  if (a.d == 128) return ctas <= sms ? (n_seqs == 1 ? 20 : 24) : ctas <= 2 * sms ? 10 : 12;
+  return ctas <= sms ? (n_seqs == 1 ? 22 : 26) : 20;
 }
 int delta_walk_len(const ScanArgs& a, int n_seqs) {
   const int64_t ctas = chunk_ctas(a, n_seqs), sms = sm_count();
   if (a.d == 128) return ctas <= sms ? 19 : ctas <= 2 * sms ? 16 : 21;
-  return ctas <= sms ? 28 : 40;
+  return ctas <= sms ? (n_seqs == 1 ? 24 : 28) : 40;
 }
 
 template <int D>

@@ -246,8 +246,9 @@ def _inputs(kind, tokens, seed, scale=1.0, D=128, P=64):
     gates = r(*tokens, H if kind == "ssm" else 2 * H).to(torch.bfloat16)
     a_log, bias, skip = 0.5 * r(H) - 0.5, 0.5 * r(H), 0.5 * r(H)
 
-    def run(nat, seqs, rows_x, rows_g, state):
+    def run(nat, seqs, rows_x, rows_g, state, max_new=0):
         lay = Lay(seqs)
+        lay.max_new = max_new
         out = torch.empty(lay.n_tokens, H * P, device=DEV)
         if kind == "ssm":
             nat.ssm_scan(rows_x, rows_g, bias, a_log, skip, state, out, lay, H, G, P, D)
@@ -285,6 +286,21 @@ def test_short_portions_are_walked_token_by_token(nat, kind):
             whole = torch.zeros_like(state)
             out = run(nat, seqs, rows(x), rows(gates), whole)
             assert torch.equal(out[:5 * n].view(5, n, -1), steps) and torch.equal(whole[:5], state[:5])
+
+
+@pytest.mark.parametrize("kind", ["ssm", "delta"])
+def test_the_longest_portion_may_be_given_too_long(nat, kind):
+    """``max_new`` is a bound: portions below it, alone or beside others, come out the same (float roundings apart)."""
+    x, gates, _, run, H, G = _inputs(kind, (3, 70), 5)
+    for lens in ([1], [5], [70], [5, 1], [70, 5, 1]):
+        seqs = [(0, m, i) for i, m in enumerate(lens)]
+        rows = lambda v: torch.cat([v[i, :m] for i, m in enumerate(lens)])
+        outs, states = [], []
+        for max_new in (0, max(lens), 200):
+            states.append(torch.zeros(4, H, 128, 64, device=DEV))
+            outs.append(run(nat, seqs, rows(x), rows(gates), states[-1], max_new))
+        for o, S in zip(outs[1:], states[1:]):
+            assert (o - outs[0]).norm() <= 1e-6 * outs[0].norm() and (S - states[0]).norm() <= 1e-6 * states[0].norm()
 
 
 @pytest.mark.parametrize("D,P", [(128, 64), (64, 128)])
