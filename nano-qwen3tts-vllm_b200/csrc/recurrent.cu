@@ -8,8 +8,8 @@
 //   retention        S <- decay_h S + k v^T                                o = S^T q      (a fixed decay per head; retention.cu
 //                                                                                         has its tensor-core and one-token kernels)
 //
-// Prompt portions of the state space and the delta rule in bf16 run in chunks on the tensor cores (recurrent_chunk.cu); what follows is about the
-// token-by-token kernel, which takes everything else.
+// Prompt portions of the state space and the delta rule in bf16 that are longer than 10 to 40 tokens run in chunks on the tensor cores
+// (recurrent_chunk.cu has the lines); what follows is about the token-by-token kernel, which takes everything else.
 //
 // All of them update every value column of S independently.  A column is shared by RS = ceil(key size / 32) lanes of one
 // warp, each keeping 32 rows of it in registers for the whole portion; sums over the rows (the read-out, the delta rule's
