@@ -498,10 +498,13 @@ B2TTS_API int b2tts_grouped_gemm_silu(const void* a, int64_t lda, const void* w,
                                       const int32_t* sorted_pair, int n_pairs, int experts, int ff, int k, int top, void* stream);
 /* How often a wait inside the grouped tensor-core kernel ran out since the library was loaded (expected: 0).  A launch whose wait runs
  * out leaves no result; the next grouped_gemm* call answers with B2TTS_ECUDA, and so does _check(), once: call it behind a
- * synchronisation (it makes none itself) before results are used.  _lose_wait() launches a kernel whose wait runs out, for tests. */
+ * synchronisation (it makes none itself) before results are used; it answers for the waits of portion_attn.cu as well.  _lose_wait()
+ * launches a kernel whose wait runs out, for tests. */
 B2TTS_API int b2tts_grouped_gemm_timeouts(void);
 B2TTS_API int b2tts_grouped_gemm_check(void);
 B2TTS_API int b2tts_grouped_gemm_lose_wait(void* stream);
+/* How often a wait inside the tcgen05 kernel of prompt attention ran out since the library was loaded (expected: 0). */
+B2TTS_API int b2tts_portion_attn_timeouts(void);
 
 /* ---- decoders with latent attention, token shift and a norm on each sublayer's output (csrc/latent_ops.cu, latent_attn.cu).
  * `dtype` is the activation / cache type (B2TTS_DTYPE_*); x is the float residual stream [rows, cols]. */
@@ -607,6 +610,15 @@ B2TTS_API int b2tts_sink_attn(const void* q, const void* k_cache, const void* v_
                               int n_tokens, int n_seqs, int max_new, int heads, int kv_heads, int v_heads, int dim, int vdim,
                               int page, int mask_kind, int mask, int keep_first, float softcap, float scale, int dtype, int path,
                               int out_f32, void* stream);
+/* The same, told how many rows (pages times page) both caches have and how many keys the longest sequence has (0: not known).  Prompt
+ * portions with head sizes of 64 or 128 and pages of a multiple of 16 then run on the tcgen05 kernel (csrc/portion_attn.cu), whose copies
+ * are bounded by the rows; steps whose longest sequence is known to be short stay with the other one. */
+B2TTS_API int b2tts_sink_attn_rows(const void* q, const void* k_cache, const void* v_cache, void* out, const int32_t* tok_seq,
+                              const int32_t* positions, const int32_t* seq_start, const int32_t* seq_pos0, const int32_t* seq_len,
+                              const int32_t* block_tables, int64_t bt_stride, const float* sink, const void* gate, int64_t ldg, int gate_el,
+                              int n_tokens, int n_seqs, int max_new, int heads, int kv_heads, int v_heads, int dim, int vdim,
+                              int page, int mask_kind, int mask, int keep_first, float softcap, float scale, int dtype, int path,
+                              int out_f32, int64_t cache_rows, int max_keys, void* stream);
 /* out[t, c] = act(bias[c] + sum_j w[c, j] * u(position(t) - taps + 1 + j)[c_off + c]) for c < channels (act 0: none, 1: SiLU;
  * bias may be null).  Earlier positions come from this step's rows, from state [slots, taps-1, channels] (the sequence's last
  * rows, oldest first, advanced by this call) or are zero before position 0.  max_new >= every seq_len[b] (0: unknown). */

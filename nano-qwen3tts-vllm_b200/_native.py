@@ -120,6 +120,8 @@ def _load():
         "b2tts_stream_gather_norm": (I, [P, P, P, P, P, I, I, I, F, I, P]),
         "b2tts_attn_prep": (I, [P, L, I, I, I, P, P, P, P, P, P, I, P, P, P, P, P, I, I, I, I, I, F, I, I, I, P]),
         "b2tts_sink_attn": (I, [P, P, P, P, P, P, P, P, P, P, L, P, P, L, I, I, I, I, I, I, I, I, I, I, I, I, I, F, F, I, I, I, P]),
+        "b2tts_sink_attn_rows": (I, [P, P, P, P, P, P, P, P, P, P, L, P, P, L, I, I, I, I, I, I, I, I, I, I, I, I, I, F, F, I, I, I, L, I, P]),
+        "b2tts_portion_attn_timeouts": (I, []),
         "b2tts_gated_linear_scan": (I, [P, L, P, L, P, L, P, L, P, F, P, P, P, P, P, P, P, I, I, I, I, I, I, P]),
         "b2tts_sandwich_residual": (I, [P, P, P, I, P, P, P, F, P, P, P, I, I, P, P, P, P, I, I, I, F, I, P]),
         "b2tts_polynorm": (I, [P, P, I, I, F, I, P]),
@@ -1115,12 +1117,20 @@ def sink_attn(q, k_cache, v_cache, out, lay, sink, gate, heads, kv_heads, dim, v
     dt = _act(q, "q")
     assert k_cache.dtype == q.dtype and v_cache.dtype == q.dtype and out.dtype in (q.dtype, F32) and out.is_contiguous()
     assert gate is None or (gate.dtype == q.dtype and gate.stride(1) == 1)
-    _check(_load().b2tts_sink_attn(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), lay.tok_seq.data_ptr(),
-                                   lay.positions.data_ptr(), lay.seq_start.data_ptr(), lay.seq_pos0.data_ptr(), lay.seq_len.data_ptr(),
-                                   lay.block_tables.data_ptr(), lay.block_tables.stride(0), _ptr(sink), _ptr(gate),
-                                   0 if gate is None else gate.stride(0), int(gate_el), lay.n_tokens, lay.n_seqs, lay.max_new, heads, kv_heads,
-                                   kv_heads if v_heads is None else v_heads, dim, vdim, page, mask_kind, mask, keep_first, softcap,
-                                   scale, dt, path, int(out.dtype == F32 and q.dtype != F32), _stream()), "sink_attn")
+    vh = kv_heads if v_heads is None else v_heads
+    # how many rows the caches have bounds the copies of the prompt kernel; a view that skips memory has no such number
+    rows = min(k_cache.numel() // (kv_heads * dim), v_cache.numel() // (vh * vdim)) if k_cache.is_contiguous() and v_cache.is_contiguous() else 0
+    _check(_load().b2tts_sink_attn_rows(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), lay.tok_seq.data_ptr(),
+                                        lay.positions.data_ptr(), lay.seq_start.data_ptr(), lay.seq_pos0.data_ptr(), lay.seq_len.data_ptr(),
+                                        lay.block_tables.data_ptr(), lay.block_tables.stride(0), _ptr(sink), _ptr(gate),
+                                        0 if gate is None else gate.stride(0), int(gate_el), lay.n_tokens, lay.n_seqs, lay.max_new, heads,
+                                        kv_heads, vh, dim, vdim, page, mask_kind, mask, keep_first, softcap, scale, dt, path,
+                                        int(out.dtype == F32 and q.dtype != F32), rows, getattr(lay, "max_keys", 0), _stream()), "sink_attn")
+
+
+def portion_attn_timeouts() -> int:
+    """Bounded waits of the prompt attention kernel that ran out since the library was loaded (0 when healthy)."""
+    return int(_load().b2tts_portion_attn_timeouts())
 
 
 def short_conv_act(u, c_off, channels, w, bias, state, lay, out, taps, act=1):

@@ -3,6 +3,7 @@
 #include <string.h>
 
 #include "common.cuh"
+#include "waits.cuh"
 
 namespace b2 {
 
@@ -34,6 +35,42 @@ int sm_count() {
     cached[dev] = n;
   }
   return cached[dev];
+}
+
+// ---------------------------------------------------------------- waits that ran out (waits.cuh)
+static int* wait_words() {
+  static int* const words = [] {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;             // the first launch may be a captured one
+    void* p = nullptr;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (cudaHostAlloc(&p, WAITS_KINDS * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) p = nullptr;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    for (int i = 0; p != nullptr && i < WAITS_KINDS; ++i) static_cast<volatile int*>(p)[i] = 0;
+    return static_cast<int*>(p);
+  }();
+  return words;
+}
+static int* g_words = nullptr;             // wait_words() once a launch has asked for one: reading a count allocates nothing
+static int g_told[WAITS_KINDS];            // the counts that have been answered with an error
+
+int* wait_word(int kind) {
+  int* words = wait_words();
+  if (words == nullptr) return nullptr;
+  __atomic_store_n(&g_words, words, __ATOMIC_RELEASE);
+  return words + kind;
+}
+
+int wait_count(int kind) {
+  const int* words = __atomic_load_n(&g_words, __ATOMIC_ACQUIRE);
+  return words != nullptr ? static_cast<const volatile int*>(words)[kind] : 0;
+}
+
+int wait_check(int kind, const char* what) {
+  const int n = wait_count(kind);
+  if (__atomic_exchange_n(&g_told[kind], n, __ATOMIC_RELAXED) == n) return B2TTS_OK;
+  set_error("%s: a wait inside an earlier %s ran out, its results are not valid", what,
+            kind == WAITS_GROUPED ? "grouped product" : "attention over prompt portions");
+  return B2TTS_ECUDA;
 }
 
 }  // namespace b2

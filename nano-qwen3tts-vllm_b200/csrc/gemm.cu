@@ -647,7 +647,7 @@ namespace b2 {
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-int make_x_tensor_map(CUtensorMap* tm, const void* x, int64_t row_stride, int m, int k, int mpad, const char* what) {
+int make_tensor_map(CUtensorMap* tm, const void* x, int rank, const int64_t* dims, const int64_t* strides, const int* box, const char* what) {
   static EncodeTiledFn fn = nullptr;
   if (!fn) {
     void* sym = nullptr;
@@ -659,18 +659,29 @@ int make_x_tensor_map(CUtensorMap* tm, const void* x, int64_t row_stride, int m,
     }
     fn = reinterpret_cast<EncodeTiledFn>(sym);
   }
-  const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)m};
-  const cuuint64_t strides[1] = {(cuuint64_t)row_stride * 2};
-  const cuuint32_t box[2] = {(cuuint32_t)G_BK, (cuuint32_t)mpad};
-  const cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(x), dims, strides, box, estr,
+  cuuint64_t d[3], st[2];
+  cuuint32_t bx[3];
+  const cuuint32_t estr[3] = {1, 1, 1};
+  for (int i = 0; i < rank; ++i) {
+    d[i] = static_cast<cuuint64_t>(dims[i]);
+    bx[i] = static_cast<cuuint32_t>(box[i]);
+    if (i > 0) st[i - 1] = static_cast<cuuint64_t>(strides[i - 1]) * 2;
+  }
+  CUresult r = fn(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(x), d, st, bx, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
-    set_error("%s: cuTensorMapEncodeTiled failed (%d) for x [%d, %d] stride %lld", what, (int)r, m, k, (long long)row_stride);
+    set_error("%s: cuTensorMapEncodeTiled failed (%d) for [%lld, %lld] stride %lld", what, (int)r, (long long)dims[1], (long long)dims[0],
+              (long long)strides[0]);
     return B2TTS_ECUDA;
   }
   return B2TTS_OK;
+}
+
+int make_x_tensor_map(CUtensorMap* tm, const void* x, int64_t row_stride, int m, int k, int mpad, const char* what) {
+  const int64_t dims[2] = {k, m};
+  const int box[2] = {G_BK, mpad};
+  return make_tensor_map(tm, x, 2, dims, &row_stride, box, what);
 }
 
 static unsigned long long* g_trace_base = nullptr;   // debug only (b2tts_debug_gemm_trace)

@@ -17,6 +17,7 @@
 
 #include "grouped_gemm.cuh"
 #include "umma.cuh"
+#include "waits.cuh"
 
 namespace b2 {
 
@@ -25,9 +26,7 @@ constexpr int TC_GATHER_WARPS = 4, TC_LAG = 2;     // slices a gather warp issue
 constexpr int TC_A_BYTES = TC_BM * G_BK * 2, TC_B_BYTES = TC_BN * G_BK * 2, TC_STAGE_BYTES = TC_A_BYTES + TC_B_BYTES;
 constexpr size_t TC_SMEM = 1024 + static_cast<size_t>(TC_STAGES) * TC_STAGE_BYTES + 256;
 
-// How often a wait inside the kernel ran out (it never should).  The count goes to a word of host memory as well, which the host reads
-// without a copy or a synchronisation: the entry points, and the engine behind each step's own synchronisation, answer with an error
-// when it has moved, since what the launch left behind is not a result.
+// How often a wait inside the kernel ran out, see waits.cuh.
 __device__ int g_grouped_tc_timeouts = 0;
 __device__ __forceinline__ void report_timeout(int* word) {
   *reinterpret_cast<volatile int*>(word) = atomicAdd(&g_grouped_tc_timeouts, 1) + 1;
@@ -253,28 +252,7 @@ bool grouped_tc_applies(int n_pairs, int experts, int w_rows, int k, bool gated,
   return k >= 192 || tiles * k >= 40000;
 }
 
-static int* timeouts_word() {
-  static int* const word = [] {
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;             // the first launch may be a captured one
-    void* p = nullptr;
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    if (cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) p = nullptr;
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    if (p != nullptr) *static_cast<volatile int*>(p) = 0;
-    return static_cast<int*>(p);
-  }();
-  return word;
-}
-static int* g_word = nullptr;              // timeouts_word() once a launch has asked for it: reading the count allocates nothing
-static int g_told = 0;                     // the count that has been answered with an error
-
-int grouped_tc_check(const char* what) {
-  int* word = __atomic_load_n(&g_word, __ATOMIC_ACQUIRE);
-  const int n = word != nullptr ? *static_cast<volatile int*>(word) : 0;
-  if (__atomic_exchange_n(&g_told, n, __ATOMIC_RELAXED) == n) return B2TTS_OK;
-  set_error("%s: a wait inside an earlier grouped product ran out, its results are not valid", what);
-  return B2TTS_ECUDA;
-}
+int grouped_tc_check(const char* what) { return wait_check(WAITS_GROUPED, what); }
 
 template <int ACT, bool GATHER>
 static int go(const char* what, const GroupedTcArgs& p, const CUtensorMap& ma, const CUtensorMap& mw, int tiles, cudaStream_t st) {
@@ -289,9 +267,8 @@ static int go(const char* what, const GroupedTcArgs& p, const CUtensorMap& ma, c
 int launch_grouped_tc(const char* what, const void* a, int64_t lda, const void* w, void* c, int64_t ldc, const int32_t* offsets,
                       const int32_t* sorted_pair, int n_pairs, int experts, int n, int k, int top, int in_by_token, int out_by_pair,
                       int act, float limit, float alpha, cudaStream_t st) {
-  int* word = timeouts_word();
+  int* word = wait_word(WAITS_GROUPED);
   B2_REQUIRE(word != nullptr, B2TTS_ECUDA, "%s: no host memory for the kernel's status", what);
-  __atomic_store_n(&g_word, word, __ATOMIC_RELEASE);
   const bool gated = act >= GG_CLAMPED;
   CUtensorMap ma{}, mw;
   int rc = make_x_tensor_map(&mw, w, k, experts * n, k, gated ? TC_BN / 2 : TC_BN, what);
@@ -322,10 +299,15 @@ int launch_grouped_tc(const char* what, const void* a, int64_t lda, const void* 
 }  // namespace b2
 
 extern "C" int b2tts_grouped_gemm_timeouts(void) {
-  const int* word = __atomic_load_n(&b2::g_word, __ATOMIC_ACQUIRE);
-  return word != nullptr ? *static_cast<const volatile int*>(word) : 0;
+  return b2::wait_count(b2::WAITS_GROUPED);
 }
-extern "C" int b2tts_grouped_gemm_check(void) { return b2::grouped_tc_check("grouped_gemm"); }
+extern "C" int b2tts_grouped_gemm_check(void) {
+  for (int k = 0; k < b2::WAITS_KINDS; ++k) {
+    const int rc = b2::wait_check(k, "check_waits");
+    if (rc != B2TTS_OK) return rc;
+  }
+  return B2TTS_OK;
+}
 
 namespace b2 {
 // One wait of the kind that the kernel has, on a barrier that nothing arrives at, with a short limit.
@@ -339,9 +321,8 @@ __global__ void grouped_tc_lost_wait_kernel(int* word) {
 
 extern "C" int b2tts_grouped_gemm_lose_wait(void* stream) {
   using namespace b2;
-  int* word = timeouts_word();
+  int* word = wait_word(WAITS_GROUPED);
   B2_REQUIRE(word != nullptr, B2TTS_ECUDA, "grouped_gemm_lose_wait: no host memory");
-  __atomic_store_n(&g_word, word, __ATOMIC_RELEASE);
   grouped_tc_lost_wait_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(word);
   B2_CHECK_LAUNCH("grouped_gemm_lose_wait");
   return B2TTS_OK;

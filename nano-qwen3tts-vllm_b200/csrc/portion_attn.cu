@@ -1,0 +1,719 @@
+// portion_attn.cu - softmax attention of prompt portions (more than one new token of a sequence) on the 5th-generation tensor cores:
+// keys and values through block tables or in rows of their own, sliding-window, chunk or causal masks with kept first keys, sinks, score
+// caps, gates.  bf16 operands; scores, weights, sums and the outputs' accumulators are float.
+//
+// A persistent CTA per SM takes items of one or two row tiles.  A row tile is 128 query rows: 128 / HPC tokens times HPC heads that share
+// a key head; the two tiles of an item are neighbouring tokens and share the key tiles (128 keys) that pass through one ring of
+// 16 KiB slots (128 rows x 64 columns).  Twenty warps:
+//   softmax   two groups of eight, a group per row tile, two threads of a warp per row: each takes 64 scores from TMEM, and gives the weights
+//             back in the same columns as the A operand of the second product, a bf16 pair hi + lo each (16 bits);
+//   MMA       S = Q K^T (128 x 128 x d), O += P V (128 x dv x 128, twice: hi and lo) for the tiles in turn, so that one tile's products run
+//             while the other tile's weights are formed.  A tile's next S overwrites its weights: the products of one thread
+//             run in the order of their issue;
+//   loader    queries (one box of 64 columns x HPC heads x tokens per slice), keys and values as boxes of R rows inside pages;
+//   cleaner   zeros the value rows of a tile that no query of the item sees (behind the last key, before the window): their weights are
+//             zero, but what a page holds there may be infinite.
+// The running maximum is lazy: O and the sum are rescaled only when a row's maximum has grown by more than 2^8; weights are then up to
+// 2^8, which floats and bf16 pairs hold as well as 1.
+//
+// Bound: the issue of the tensor core's products.  A key tile of a row tile is 24 of them of 64 cycles (1536); the issuer's own instructions and
+// barriers between two tiles make that about 2300, and the weights (64 exponents, splits and sums a thread) are ready before that.  An item
+// starts and ends in about 12000 cycles (first key tile under a mask, last products, division and gates).  Two threads a row and 64 scores
+// each in two passes over TMEM keep everything in 96 registers: spilled ones went through L2, since shared memory leaves L1 next to nothing
+// (one thread a row with 40 spilled registers: 143 us for the case below; one barrier per slot of the ring instead of per tile: 20 us more).
+// 4 prompts of 2048 tokens, 16 heads over 8 of 128, window 1024 + 4 kept, element gates: 118 us (mma.sync, 64 queries per CTA: 547 us; 31 at
+// the tensor core's rate); causal with a score cap, 4448 tokens: 141 us (579 us).
+//
+// Every copy is bounded: maps have the true extents of their tensors, so a row that a block table should not name reads zeros.  Every
+// commit of the last products is waited for before the CTA leaves.
+#include <algorithm>
+
+#include "portion_attn.cuh"
+#include "umma.cuh"
+#include "waits.cuh"
+
+namespace b2 {
+namespace row {
+
+constexpr int PO_N = 128, PO_SLOT = 128 * 128;         // keys per tile; bytes of a slot: 128 rows of 64 bf16 columns
+constexpr int PO_SOFT = 16, PO_THREADS = 640, PO_ITEMS = 64;           // softmax warps; items a CTA takes at most
+constexpr int PO_MMA = 16, PO_LOADER = 17, PO_CLEANER = 18, PO_LISTER = 19;
+__device__ int g_portion_timeouts = 0;                 // see waits.cuh
+
+// Low word of an MN-major SWIZZLE_128B operand: a K index (key) is a 128-byte row of 64 columns; LBO: the next 64 columns (the next slot),
+// SBO: 8 keys.  The high word is that of the K-major operands.
+__device__ __forceinline__ uint32_t po_desc_mn_lo(uint32_t addr) { return ((addr & 0x3ffffu) >> 4) | (static_cast<uint32_t>(PO_SLOT >> 4) << 16); }
+// D [128 x n] (+)= A (TMEM: two bf16 per column, lane = row) B (shared memory)
+__device__ __forceinline__ void po_umma_ts(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      ".reg .b64 db;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "mov.b64 db, {%2, %5};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t"
+      "}"
+      :: "r"(d), "r"(a), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(UMMA_DESC_HI_SW128) : "memory");
+}
+// pairs of floats
+__device__ __forceinline__ uint64_t po_pair(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void po_split(uint64_t x, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x)); }
+__device__ __forceinline__ uint64_t po_fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t po_add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t po_mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// 32 columns of 16 lanes for lanes 0 .. 15 of the warp and 32 columns of the same lanes, SPLIT columns further, for the others
+template <int SPLIT>
+__device__ __forceinline__ void po_ld32(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x32bx2.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32], %33;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+        "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
+        "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]),
+        "=r"(r[31])
+      : "r"(taddr), "n"(SPLIT));
+}
+template <int SPLIT>
+__device__ __forceinline__ void po_ld16(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x32bx2.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16], %17;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr), "n"(SPLIT));
+}
+template <int SPLIT>
+__device__ __forceinline__ void po_st16(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.16x32bx2.x16.b32 [%0], %17, {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+      :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+         "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "n"(SPLIT) : "memory");
+}
+template <int SPLIT>
+__device__ __forceinline__ void po_st32(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.16x32bx2.x32.b32 [%0], %33, {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+      :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+        "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]),
+        "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]),
+        "n"(SPLIT) : "memory");
+}
+__device__ __forceinline__ void po_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ float po_ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ int po_mask_lo(int i, int kind, int mask) {
+  if (mask <= 0) return 0;
+  return kind == 0 ? max(0, i - mask + 1) : (i / mask) * mask;
+}
+// the n lowest of 32 bits (none for n <= 0, all from 32 on)
+__device__ __forceinline__ uint32_t po_below(int n) { return n <= 0 ? 0u : n >= 32 ? 0xffffffffu : (1u << n) - 1u; }
+
+// Columns of a row tile's weights of 16 keys: step s < 8 the rounded weights of keys 16 s .., s >= 8 the remainders of keys 16 (s - 8) ..  32 keys
+// have the 32 columns where their scores were: 16 of rounded weights, 16 of remainders.
+__device__ __forceinline__ constexpr int po_weights_at(int s) { return (s >> 1 & 3) * 32 + (s >> 3) * 16 + (s & 1) * 8; }
+
+struct PortionPlan { int hpc, hpc_shift, tiles, box_rows, page_shift, gate_vec; int* timeouts; };    // set by the launch
+struct PortionMaps { CUtensorMap q, k, k2, v; };
+struct PortionEntry { int tile, b, hg, len, start, pos0; };
+
+// What every role knows of an item.  The key list: kept first keys that the lowest bound of the item hides, in whole boxes, then
+// [jl, j_hi] from a multiple of R on; where the boxes of the kept keys reach that bound, one run from key 0.
+struct PortionItem {
+  int b, t0, end, start, pos0, h0, j_lo, j_hi, jl, pre_r, n_pre, keep_in, n_keys, n_tiles, per;
+  __device__ __forceinline__ PortionItem(const PortionArgs& a, const PortionPlan& p, const PortionEntry& e) {
+    per = 128 >> p.hpc_shift;
+    b = e.b;
+    t0 = e.tile * p.tiles * per;
+    end = min(e.len, t0 + p.tiles * per);              // behind the item's last token
+    start = e.start; pos0 = e.pos0;
+    h0 = e.hg << p.hpc_shift;
+    const int R = p.box_rows, keep_r = (a.keep_first + R - 1) & ~(R - 1);
+    j_lo = po_mask_lo(pos0 + t0, a.mask_kind, a.mask);
+    j_hi = pos0 + end - 1;
+    const bool pre = a.keep_first > 0 && keep_r <= j_lo;
+    n_pre = pre ? a.keep_first : 0;
+    pre_r = pre ? keep_r : 0;
+    jl = pre || a.keep_first == 0 ? j_lo & ~(R - 1) : 0;
+    keep_in = pre ? 0 : a.keep_first;                  // kept keys that are part of the run
+    n_keys = pre_r + j_hi - jl + 1;
+    n_tiles = (n_keys + PO_N - 1) / PO_N;
+  }
+  __device__ __forceinline__ bool has(int g) const { return t0 + g * per < end; }
+};
+
+// The key tiles of which some row of row tile g sees a key: those of the kept keys, [0, front), and [first, last]
+struct PortionSpan {
+  int front = 0, first = 0, last = -1;
+  PortionSpan() = default;
+  __device__ __forceinline__ PortionSpan(const PortionArgs& a, const PortionItem& m, int g) {
+    if (!m.has(g)) return;
+    const int t = m.t0 + g * m.per, lo = po_mask_lo(m.pos0 + t, a.mask_kind, a.mask);
+    first = (max(lo - m.jl, 0) + m.pre_r) / PO_N;
+    last = (m.pos0 + min(m.end, t + m.per) - 1 - m.jl + m.pre_r) / PO_N;
+    front = min((m.n_pre + m.keep_in + PO_N - 1) / PO_N, last + 1);
+  }
+  __device__ __forceinline__ bool has(int j) const { return j < front || (j >= first && j <= last); }
+};
+
+template <int NS> constexpr int po_slots() { return NS == 1 ? 12 : NS == 2 ? 10 : 8; }      // of the ring
+constexpr int PO_DEEP = 8, PO_BAR_BYTES = 512, PO_TAIL = PO_BAR_BYTES + PO_ITEMS * 24;
+template <int NS> constexpr int po_smem() { return 1024 + (2 * NS + po_slots<NS>()) * PO_SLOT + PO_TAIL; }
+static_assert(po_smem<1>() <= 232448 && po_smem<2>() <= 232448 && po_smem<3>() <= 232448, "shared memory of a CTA");
+
+// NS: 64-column slices of q and k; NV: of v
+template <int NS, int NV>
+__global__ void __launch_bounds__(PO_THREADS, 1)
+portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_constant__ PortionMaps maps) {
+  constexpr int SLOTS = po_slots<NS>(), PER_TILE = NS + NV;
+  static_assert(2 * NS + NV <= SLOTS, "a tile's values beside two tiles of keys");
+  static_assert(SLOTS / PER_TILE + 1 < PO_DEEP, "tiles in the ring at once");
+  extern __shared__ uint8_t po_smem_dyn[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(po_smem_dyn) + 1023) & ~uintptr_t(1023));
+  uint8_t* q_s = smem;                                 // [2 tiles][NS]
+  uint8_t* ring = q_s + 2 * NS * PO_SLOT;              // keys of tile 0, values of tile 0, keys of tile 1, ..
+  // key tile t of the CTA, counted over its items, at t % PO_DEEP: keys there, values there, values cleaned; its
+  // keys and the values of the tile before given back
+  uint64_t* k_full = reinterpret_cast<uint64_t*>(ring + SLOTS * PO_SLOT);
+  uint64_t *v_full = k_full + PO_DEEP, *clean = v_full + PO_DEEP, *empty = clean + PO_DEEP;
+  uint64_t *q_full = empty + PO_DEEP, *q_empty = q_full + 2, *s_full = q_empty + 2, *p_full = s_full + 2;
+  uint64_t* o_full = p_full + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
+  int* n_items_s = reinterpret_cast<int*>(tmem_slot + 1);
+  PortionEntry* list = reinterpret_cast<PortionEntry*>(reinterpret_cast<uint8_t*>(k_full) + PO_BAR_BYTES);
+
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  if (warp == PO_LISTER) {
+    // The CTA's items: number i of the valid (tile, sequence, heads), late tiles first (they are the longest under a causal mask), for
+    // i = c, 2 G - 1 - c, 2 G + c, ..
+    const int span = p.tiles * (128 >> p.hpc_shift), groups = a.H >> p.hpc_shift, c = blockIdx.x, G = gridDim.x;
+    int k = 0, cum = 0, want = c;
+    const int len0 = lane < a.n_seqs ? a.seq_len[lane] : 0;
+    for (int tile = (a.max_new + span - 1) / span - 1; tile >= 0 && k < PO_ITEMS; --tile) {
+      for (int base = 0; base < a.n_seqs && k < PO_ITEMS; base += 32) {
+        const int len = base == 0 ? len0 : base + lane < a.n_seqs ? a.seq_len[base + lane] : 0;
+        const unsigned live = __ballot_sync(0xffffffffu, len > 1 && tile * span < len);
+        const int cnt = __popc(live) * groups;
+        while (k < PO_ITEMS && want < cum + cnt) {
+          const int at = want - cum, rank = at / groups;
+          const int at_b = static_cast<int>(__fns(live, 0, rank + 1));
+          if (lane == at_b) list[k] = PortionEntry{tile, base + lane, at - rank * groups, len, a.seq_start[base + lane], a.seq_pos0[base + lane]};
+          ++k;
+          want = k * G + (k & 1 ? G - 1 - c : c);
+        }
+        cum += cnt;
+      }
+    }
+    if (lane == 0) *n_items_s = k;
+  }
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < PO_DEEP; ++s) {
+      mbar_init(k_full + s, 1); mbar_init(v_full + s, 1); mbar_init(clean + s, 1); mbar_init(empty + s, 1);
+    }
+    for (int g = 0; g < 2; ++g) {
+      mbar_init(q_full + g, 1); mbar_init(q_empty + g, 1); mbar_init(s_full + g, 1); mbar_init(p_full + g, PO_SOFT / 2); mbar_init(o_full + g, 1);
+    }
+    mbar_fence_init();
+  }
+  if (warp == PO_MMA) tmem_alloc(tmem_slot, 512);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;                    // S and weights of tile g: columns 128 g; O: 256 + 128 g
+  const int n_items = *n_items_s;
+  bool ok = true;
+
+  if (warp >= PO_SOFT) {
+    if (warp == PO_LOADER) {
+      // =========================== loader
+      int t = 0, slot = 0, q_uses[2] = {0, 0};         // the tile, the next slot, query tiles loaded so far
+      for (int x = 0; ok && x < n_items; ++x) {
+        const PortionItem m(a, p, list[x]);
+        const int g = m.h0 / (a.H / a.G), gv = g % a.Gv, R = p.box_rows;
+        const int32_t* bt = a.block_tables != nullptr ? a.block_tables + static_cast<int64_t>(m.b) * a.bt_stride : nullptr;
+        const int row0 = bt == nullptr ? a.key_start[m.b] : 0;
+        const int n1 = min(NS, (a.d1 + 63) / 64);
+        // lane = box * 4 + slice; row of the lane's box of tile j, a tile ahead: nothing waits for the load of the page's number here
+        const int box = lane >> 2, sl = lane & 3, boxes = PO_N / R;
+        struct Row { int pg, off; };
+        auto row_of = [&](int j) {
+          const int vi = j * PO_N + box * R;
+          if (box >= boxes || vi >= m.n_keys) return Row{0, 0};
+          const int key = vi < m.pre_r ? vi : m.jl + vi - m.pre_r;
+          if (bt == nullptr) return Row{0, row0 + key};
+          const int pg = p.page_shift >= 0 ? key >> p.page_shift : key / a.page;
+          return Row{bt[pg], key - pg * a.page};
+        };
+        // the next n slots: keys or values of tile t, columns x0 ..
+        auto fill = [&](int j, Row r, int n, bool keys, int x0) {
+          // what lay there: the ring holds SLOTS slots, given back in order, values with the keys of the tile behind them
+          const int old = t * PER_TILE + (keys ? 0 : NS) + n - 1 - SLOTS, ot = (old + NV) / PER_TILE;
+          if (old >= 0) ok = mbar_wait_limit(empty + (ot & (PO_DEEP - 1)), (ot / PO_DEEP) & 1);
+          if (!ok) return;
+          const int nb = (min(m.n_keys - j * PO_N, PO_N) + R - 1) / R;
+          uint64_t* bar = (keys ? k_full : v_full) + (t & (PO_DEEP - 1));
+          if (lane == 0) mbar_expect_tx(bar, n * nb * R * 128);
+          __syncwarp();
+          if (box < nb && sl < n) {
+            const int at = slot + sl < SLOTS ? slot + sl : slot + sl - SLOTS, row = r.pg * a.page + r.off;
+            uint8_t* dst = ring + at * PO_SLOT + box * R * 128;
+            if (keys && sl >= n1) tma_load_2d(dst, &maps.k2, (sl - n1) * 64, row, bar);
+            else tma_load_2d(dst, keys ? &maps.k : &maps.v, x0 + sl * 64, row, bar);
+          }
+          __syncwarp();
+          slot = slot + n < SLOTS ? slot + n : slot + n - SLOTS;
+        };
+        Row cur = row_of(0);
+        for (int j = 0; ok && j < m.n_tiles; ++j, ++t) {
+          fill(j, cur, NS, true, g * a.d1);
+          for (int tg = 0; ok && j == 0 && tg < 2; ++tg) {
+            if (!m.has(tg)) continue;
+            if (!(ok = mbar_wait_limit(q_empty + tg, (q_uses[tg] & 1) ^ 1))) break;
+            if (lane == 0) mbar_expect_tx(q_full + tg, NS * PO_SLOT);
+            __syncwarp();
+            if (lane < NS) tma_load_3d(q_s + (tg * NS + lane) * PO_SLOT, &maps.q, lane * 64, m.h0, m.start + m.t0 + tg * m.per, q_full + tg);
+            __syncwarp();
+            ++q_uses[tg];
+          }
+          const Row mine = cur;
+          if (j + 1 < m.n_tiles) cur = row_of(j + 1);
+          if (ok) fill(j, mine, NV, false, gv * a.dv);
+        }
+      }
+      // every copy has landed before the CTA leaves
+      for (int i = max(0, t - PO_DEEP); i < t; ++i)
+        ok = mbar_wait_limit(k_full + (i & (PO_DEEP - 1)), (i / PO_DEEP) & 1) && mbar_wait_limit(v_full + (i & (PO_DEEP - 1)), (i / PO_DEEP) & 1) && ok;
+      for (int tg = 0; tg < 2; ++tg)
+        if (q_uses[tg] > 0) ok = mbar_wait_limit(q_full + tg, (q_uses[tg] - 1) & 1) && ok;
+    } else if (warp == PO_CLEANER) {
+      // =========================== cleaner: value rows that nothing sees
+      int t = 0, slot = 0;                             // of the tile's keys
+      for (int x = 0; ok && x < n_items; ++x) {
+        const PortionItem m(a, p, list[x]);
+        for (int j = 0; ok && j < m.n_tiles; ++j, ++t) {
+          const int v0 = slot + NS < SLOTS ? slot + NS : slot + NS - SLOTS;
+          slot = slot + PER_TILE < SLOTS ? slot + PER_TILE : slot + PER_TILE - SLOTS;
+          if (!(ok = mbar_wait_limit(v_full + (t & (PO_DEEP - 1)), (t / PO_DEEP) & 1))) break;
+          bool wrote = false;
+#pragma unroll
+          for (int i = 0; i < PO_N / 32; ++i) {
+            const int r = i * 32 + lane, vi = j * PO_N + r, key = m.jl + vi - m.pre_r;
+            const bool keep = vi < m.n_pre || (vi >= m.pre_r && vi < m.n_keys && (key >= m.j_lo || key < m.keep_in));
+            if (!keep) {
+              wrote = true;
+#pragma unroll
+              for (int s = 0; s < NV; ++s) {
+                uint4* row = reinterpret_cast<uint4*>(ring + (v0 + s < SLOTS ? v0 + s : v0 + s - SLOTS) * PO_SLOT + r * 128);
+#pragma unroll
+                for (int c = 0; c < 8; ++c) row[(c + lane) & 7] = make_uint4(0u, 0u, 0u, 0u);
+              }
+            }
+          }
+          if (wrote) fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(clean + (t & (PO_DEEP - 1)));
+        }
+      }
+    } else if (warp == PO_MMA) {
+      // =========================== MMA issuer: per key tile j and row tile g: O_g += P_g(j - 1) V(j - 1), then S_g(j)
+      const uint32_t idesc_s = umma_idesc_bf16(PO_N), idesc_half = umma_idesc_bf16(64) | (1u << 16),
+                     idesc_o = umma_idesc_bf16(NV * 64) | (1u << 16);                   // the value operand is MN-major
+      const uint32_t ring_k = umma_desc_lo_sw128(smem_u32(ring)), ring_v = po_desc_mn_lo(smem_u32(ring)), q_lo = umma_desc_lo_sw128(smem_u32(q_s));
+      constexpr uint32_t SLOT_LO = PO_SLOT >> 4;
+      int t = 0, slot = 0, q_uses[2] = {0, 0}, p_uses[2] = {0, 0}, o_uses[2] = {0, 0};
+      for (int x = 0; ok && x < n_items; ++x) {
+        const PortionItem m(a, p, list[x]);
+        const PortionSpan span[2] = {PortionSpan(a, m, 0), PortionSpan(a, m, 1)};
+        int v_slot = 0;                                // of the tile before
+        bool was[2] = {false, false}, begun[2] = {false, false};
+        for (int j = 0; ok && j <= m.n_tiles; ++j) {
+          // everything but the weights is waited for in front: what the issuer does between two products leaves the tensor core idle
+          const int at = t & (PO_DEEP - 1), before = (t - 1) & (PO_DEEP - 1);
+          if (j > 0) ok = mbar_wait_limit(clean + before, ((t - 1) / PO_DEEP) & 1);
+          if (ok && j < m.n_tiles) ok = mbar_wait_limit(k_full + at, (t / PO_DEEP) & 1);
+          const uint32_t v_lo = ring_v + v_slot * SLOT_LO;
+          // values in the ring's last and first slot (only a ring of 8 slots with 5 a tile comes to that): 64 columns at a time
+          const bool apart = NS == 3 && NV == 2 && v_slot == SLOTS - 1;
+          uint32_t k_lo[NS];
+#pragma unroll
+          for (int sl = 0; sl < NS; ++sl) k_lo[sl] = ring_k + (slot + sl < SLOTS ? slot + sl : slot + sl - SLOTS) * SLOT_LO;
+#pragma unroll
+          for (int g = 0; g < 2; ++g) {
+            const uint32_t tm_o = tmem + 256 + g * 128, tm_p = tmem + g * 128;
+            const bool now = j < m.n_tiles && span[g].has(j), last_s = j == span[g].last, last_o = j - 1 == span[g].last;
+            if (ok && was[g]) {
+              ok = mbar_wait_limit(p_full + g, p_uses[g] & 1);
+              ++p_uses[g];
+            }
+            if (ok && now && !begun[g]) ok = mbar_wait_limit(q_full + g, q_uses[g] & 1);
+            if (ok && (was[g] || now)) {
+              tc_fence_after();
+              if (elect_one()) {
+                if (was[g]) {
+                  if (!apart) {
+                    po_umma_ts(tm_o, tm_p, v_lo, idesc_o, begun[g]);
+#pragma unroll
+                    for (int s = 1; s < PO_N / 8; ++s) po_umma_ts(tm_o, tm_p + po_weights_at(s), v_lo + (s & 7) * 128, idesc_o, 1);
+                  } else {
+#pragma unroll 1
+                    for (int half = 0; half < 2; ++half)
+#pragma unroll
+                      for (int s = 0; s < PO_N / 8; ++s)
+                        po_umma_ts(tm_o + half * 64, tm_p + po_weights_at(s), (half ? ring_v : v_lo) + (s & 7) * 128, idesc_half, begun[g] || s);
+                  }
+                  if (last_o) umma_commit(o_full + g);
+                }
+                if (now) {
+#pragma unroll
+                  for (int sl = 0; sl < NS; ++sl)
+#pragma unroll
+                    for (int s = 0; s < 4; ++s) umma_bf16_lo(tm_p, q_lo + (g * NS + sl) * SLOT_LO + 2 * s, k_lo[sl] + 2 * s, idesc_s, sl | s);
+                  umma_commit(s_full + g);
+                  if (last_s) umma_commit(q_empty + g);
+                }
+                if (g == 1 && j < m.n_tiles) umma_commit(empty + at);
+              }
+              __syncwarp();
+              begun[g] = begun[g] || was[g];
+              o_uses[g] += was[g] && last_o;
+              q_uses[g] += now && last_s;
+            } else if (g == 1 && j < m.n_tiles) {
+              if (ok && elect_one()) umma_commit(empty + at);
+              __syncwarp();
+            }
+            was[g] = now;
+          }
+          if (j < m.n_tiles) {
+            v_slot = slot + NS < SLOTS ? slot + NS : slot + NS - SLOTS;
+            slot = slot + PER_TILE < SLOTS ? slot + PER_TILE : slot + PER_TILE - SLOTS;
+            ++t;
+          }
+        }
+      }
+      // every commit of this warp has arrived (and with it every product) before the CTA gives up its TMEM and shared memory
+      for (int i = max(0, t - PO_DEEP); i < t; ++i)
+        ok = mbar_wait_limit(empty + (i & (PO_DEEP - 1)), (i / PO_DEEP) & 1) && ok;
+      for (int g = 0; g < 2; ++g) {
+        if (q_uses[g] > 0) ok = mbar_wait_limit(q_empty + g, (q_uses[g] - 1) & 1) && ok;
+        if (o_uses[g] > 0) ok = mbar_wait_limit(o_full + g, (o_uses[g] - 1) & 1) && ok;
+      }
+    }
+  } else {
+    // =========================== softmax: lanes i and i + 16 of a warp share row r (TMEM lane r), 64 keys of a tile each
+    const int tg = warp >> 3, r0 = (warp & 3) * 32 + (warp & 4) * 4, half = lane >> 4, r = r0 + (lane & 15);
+    const uint32_t tm_s = tmem + (static_cast<uint32_t>(r0) << 16) + tg * 128, tm_o = tm_s + 256;
+    constexpr int HK = PO_N / 2, OC = NV * 32;         // keys and output columns of a thread
+    constexpr float LOG2E = 1.4426950408889634f;
+    const float scale2 = a.scale * LOG2E, cap2 = a.softcap * LOG2E;
+    // scores in the base-2 domain are f * v: the factor rides in the exponent's fma unless a cap or a sign needs it before
+    const bool early = a.softcap > 0.f || !(scale2 > 0.f);
+    const float f = early ? 1.f : scale2;
+    const bool gated = a.gate != nullptr && a.gate_el;
+    int s_uses = 0, o_uses = 0;
+    for (int x = 0; ok && x < n_items; ++x) {
+      // What an item needs in its masked tiles and in the end is formed there again: the loop over whole tiles has no registers for it
+      float m = -1e30f, l = 0.f;
+      PortionSpan span;
+      int whole0, whole1;                              // key tiles that all rows of the warp see whole
+      {
+        const PortionItem it(a, p, list[x]);
+        if (!it.has(tg)) continue;
+        span = PortionSpan(a, it, tg);
+        if (a.sink != nullptr) { m = a.sink[it.h0 + (r & (p.hpc - 1))] * LOG2E; l = half == 0 ? 1.f : 0.f; }
+        const int t_first = it.t0 + tg * it.per, t_last = min(it.end, t_first + it.per) - 1;
+        const int lo = po_mask_lo(it.pos0 + min(t_first + ((r0 + 15) >> p.hpc_shift), t_last), a.mask_kind, a.mask);    // the highest of its rows
+        whole0 = (max(lo - it.jl, 0) + it.pre_r + PO_N - 1) / PO_N;
+        whole1 = (it.pos0 + min(t_first + (r0 >> p.hpc_shift), t_last) + 1 - it.jl + it.pre_r) / PO_N;
+        if (gated)                                     // read in the end, far from any cache by then
+          asm volatile("prefetch.global.L2 [%0];" :: "l"(a.gate + static_cast<int64_t>(it.start + min(t_first + (r >> p.hpc_shift), t_last)) * a.ldg +
+                                                         static_cast<int64_t>(it.h0 + (r & (p.hpc - 1))) * a.dv + half * OC));
+      }
+      bool first = true;
+      for (int j = 0; ok && j <= span.last; ++j) {
+        if (!span.has(j)) continue;
+        if (!(ok = mbar_wait_limit(s_full + tg, s_uses & 1))) break;
+        ++s_uses;
+        tc_fence_after();
+        const bool masked = j < whole0 || j >= whole1;
+        if (early || masked) {                         // scores are put right where they lie
+          // visible columns, counted from the thread's first: of the list's front those below fr_vis, behind it from `from` (or below `keep`) to `to`
+          const PortionItem it(a, p, list[x]);
+          const int t_first = it.t0 + tg * it.per, pos = it.pos0 + min(t_first + (r >> p.hpc_shift), min(it.end, t_first + it.per) - 1);
+          const int c0 = j * PO_N + half * HK, j0 = c0 - it.pre_r + it.jl;
+          int to = pos - j0, from = po_mask_lo(pos, a.mask_kind, a.mask) - j0, keep = it.keep_in - j0, fr_end = it.pre_r - c0, fr_vis = it.n_pre - c0;
+#pragma unroll 1
+          for (int c = 0; c < HK; c += 32) {
+            uint32_t v[32];
+            po_ld32<HK>(tm_s + c, v);
+            tmem_ld_wait();
+            if (early) {
+              const float fx = a.softcap > 0.f ? a.scale / a.softcap : scale2;
+              float big = 0.f;
+#pragma unroll
+              for (int e = 0; e < 32; ++e) {
+                const float y = __uint_as_float(v[e]) * fx;
+                v[e] = __float_as_uint(y);
+                big = fmaxf(big, fabsf(y));
+              }
+              if (a.softcap > 0.f) {
+                // cap tanh(s / cap); while all of the warp's |s / cap| are at most 0.4 by its series (the next term is below 2e-9 of it)
+                if (__all_sync(0xffffffffu, big <= 0.4f)) {
+#pragma unroll
+                  for (int e = 0; e < 32; ++e) {
+                    const float z = __uint_as_float(v[e]), y = z * z;
+                    float t = fmaf(y, 21844.f / 6081075.f, -1382.f / 155925.f);
+                    t = fmaf(y, t, 62.f / 2835.f);
+                    t = fmaf(y, t, -17.f / 315.f);
+                    t = fmaf(y, t, 2.f / 15.f);
+                    t = fmaf(y, t, -1.f / 3.f);
+                    v[e] = __float_as_uint(cap2 * fmaf(z * y, t, z));
+                  }
+                } else {
+#pragma unroll
+                  for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(cap2 * tanhf(__uint_as_float(v[e])));
+                }
+              }
+            }
+            if (masked) {
+              const uint32_t see = (po_below(fr_vis) & po_below(fr_end)) | (~po_below(fr_end) & po_below(to + 1) & (~po_below(from) | po_below(keep)));
+#pragma unroll
+              for (int e = 0; e < 32; ++e)
+                if (!(see & (1u << e))) v[e] = __float_as_uint(-INFINITY);
+              to -= 32; from -= 32; keep -= 32; fr_end -= 32; fr_vis -= 32;
+            }
+            po_st32<HK>(tm_s + c, v);
+          }
+          po_st_wait();
+        }
+        // two passes over the scores, which stay in TMEM meanwhile: a thread has no registers for all of them beside the weights' parts
+        float mx;
+        {
+          uint32_t v[HK];
+          po_ld32<HK>(tm_s, v);
+          po_ld32<HK>(tm_s + 32, v + 32);
+          tmem_ld_wait();
+          float x0 = -INFINITY, x1 = -INFINITY, x2 = -INFINITY, x3 = -INFINITY;
+#pragma unroll
+          for (int c = 0; c < HK; c += 8) {
+            x0 = fmaxf(x0, fmaxf(__uint_as_float(v[c]), __uint_as_float(v[c + 1])));
+            x1 = fmaxf(x1, fmaxf(__uint_as_float(v[c + 2]), __uint_as_float(v[c + 3])));
+            x2 = fmaxf(x2, fmaxf(__uint_as_float(v[c + 4]), __uint_as_float(v[c + 5])));
+            x3 = fmaxf(x3, fmaxf(__uint_as_float(v[c + 6]), __uint_as_float(v[c + 7])));
+          }
+          mx = fmaxf(fmaxf(x0, x1), fmaxf(x2, x3));
+        }
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16)) * f;
+        // ---- the running maximum moves in steps of more than 2^8.  These scores were issued behind the last weight products, so O is at rest
+        const bool grow = mx > m + (first ? 0.f : 8.f);
+        if (__any_sync(0xffffffffu, grow)) {
+          const float n = grow ? mx : m, alpha = po_ex2(m - n);
+          m = n;
+          l *= alpha;
+          if (!first) {
+#pragma unroll 1
+            for (int c = 0; c < OC; c += 32) {
+              uint32_t o[32];
+              po_ld32<OC>(tm_o + c, o);
+              tmem_ld_wait();
+#pragma unroll
+              for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
+              po_st32<OC>(tm_o + c, o);
+            }
+          }
+        }
+        first = false;
+        // ---- weights, their sum, and their bf16 parts, in place of the scores
+        const uint64_t f2 = po_pair(f, f), m2 = po_pair(-m, -m);
+        uint64_t sa = 0, sb = 0;
+#pragma unroll 1
+        for (int part = 0; part < HK; part += 32) {
+          uint32_t v[32], hi[16], rest[16];
+          po_ld32<HK>(tm_s + part, v);
+          tmem_ld_wait();
+#pragma unroll
+          for (int c = 0; c < 32; c += 4) {
+            const uint32_t* vv = v + c;
+            float w0, w1, w2, w3, r0, r1, r2, r3;
+            po_split(po_fma2(po_pair(__uint_as_float(vv[0]), __uint_as_float(vv[1])), f2, m2), w0, w1);
+            po_split(po_fma2(po_pair(__uint_as_float(vv[2]), __uint_as_float(vv[3])), f2, m2), w2, w3);
+            w0 = po_ex2(w0); w1 = po_ex2(w1); w2 = po_ex2(w2); w3 = po_ex2(w3);
+            const uint64_t wa = po_pair(w0, w1), wb = po_pair(w2, w3);
+            sa = po_add2(sa, wa);
+            sb = po_add2(sb, wb);
+            const uint32_t p0 = pack_bf16(w0, w1), p1 = pack_bf16(w2, w3), n0 = p0 ^ 0x80008000u, n1 = p1 ^ 0x80008000u;
+            po_split(po_add2(wa, po_pair(bf16lo(n0), bf16hi(n0))), r0, r1);
+            po_split(po_add2(wb, po_pair(bf16lo(n1), bf16hi(n1))), r2, r3);
+            rest[c / 2] = pack_bf16(r0, r1);
+            rest[c / 2 + 1] = pack_bf16(r2, r3);
+            hi[c / 2] = p0;
+            hi[c / 2 + 1] = p1;
+          }
+          po_st16<HK>(tm_s + part, hi);
+          po_st16<HK>(tm_s + part + 16, rest);
+        }
+        float s0, s1;
+        po_split(po_add2(sa, sb), s0, s1);
+        l += s0 + s1;
+        po_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_full + tg);
+      }
+      if (!ok) break;
+      const PortionItem it(a, p, list[x]);
+      const int t_first = it.t0 + tg * it.per, t_last = min(it.end, t_first + it.per) - 1, tk = t_first + (r >> p.hpc_shift), h = it.h0 + (r & (p.hpc - 1));
+      const int64_t row = it.start + min(tk, t_last), obase = (row * a.H + h) * a.dv + half * OC;
+      // 16 columns at a time, their gates a step ahead
+      const __nv_bfloat16* gr = gated ? a.gate + row * a.ldg + static_cast<int64_t>(h) * a.dv + half * OC : nullptr;
+      uint4 g0 = make_uint4(0u, 0u, 0u, 0u), g1 = g0;
+      auto gates = [&](int c) {
+        if (p.gate_vec) { g0 = ldg_v4(gr + c); g1 = ldg_v4(gr + c + 8); return; }
+        const uint32_t* gw = reinterpret_cast<const uint32_t*>(gr + c);                    // pairs: the caller checked the alignment
+        g0 = make_uint4(gw[0], gw[1], gw[2], gw[3]);
+        g1 = make_uint4(gw[4], gw[5], gw[6], gw[7]);
+      };
+      if (gated) gates(0);
+      l += __shfl_xor_sync(0xffffffffu, l, 16);
+      float inv = 1.0f / l;
+      if (a.gate != nullptr && !a.gate_el) inv *= sigmoid_f(__bfloat162float(a.gate[row * a.ldg + h]));
+      if (!(ok = mbar_wait_limit(o_full + tg, o_uses & 1))) break;
+      ++o_uses;
+      tc_fence_after();
+#pragma unroll 1
+      for (int c = 0; c < OC; c += 16) {
+        uint32_t o[16];
+        po_ld16<OC>(tm_o + c, o);
+        tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * inv);
+        if (gated) {
+          const uint32_t w[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+          if (c + 16 < OC) gates(c + 16);
+#pragma unroll
+          for (int e = 0; e < 16; ++e) {
+            const float u = e & 1 ? bf16hi(w[e >> 1]) : bf16lo(w[e >> 1]);
+            o[e] = __float_as_uint(__fdividef(__uint_as_float(o[e]), 1.0f + expf(-u)));
+          }
+        }
+        if (tk <= t_last && a.out_f32) {
+          float* op = static_cast<float*>(a.out) + obase + c;
+#pragma unroll
+          for (int e = 0; e < 16; e += 4) *reinterpret_cast<uint4*>(op + e) = make_uint4(o[e], o[e + 1], o[e + 2], o[e + 3]);
+        } else if (tk <= t_last) {
+          __nv_bfloat16* op = static_cast<__nv_bfloat16*>(a.out) + obase + c;
+#pragma unroll
+          for (int e = 0; e < 16; e += 8) {
+            const float* y = reinterpret_cast<const float*>(o + e);
+            stg_v4(op + e, make_uint4(pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]), pack_bf16(y[4], y[5]), pack_bf16(y[6], y[7])));
+          }
+        }
+        __syncwarp();
+      }
+      tc_fence_before();                               // the next item's first weights tell the issuer that O may be overwritten
+    }
+  }
+  if (!ok && lane == 0) {
+    *reinterpret_cast<volatile int*>(p.timeouts) = atomicAdd(&g_portion_timeouts, 1) + 1;
+    __threadfence_system();
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == PO_MMA) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 512);
+  }
+}
+
+// Whole slices of 64 columns (a box is never wider than a row), rows that copies can name and pages in whole boxes of 16 rows.
+bool portion_attn_applies(const PortionArgs& a) {
+  const bool rows8 = a.q_tok % 8 == 0 && a.q_head % 8 == 0 && a.k_row % 8 == 0 && a.k2_row % 8 == 0 && a.v_row % 8 == 0;
+  return rows8 && a.d % 64 == 0 && a.d <= 192 && a.d1 % 64 == 0 && a.d1 <= a.d && (a.dv == 64 || a.dv == 128) && aligned16(a.q) &&
+         aligned16(a.k) && (a.k2 == nullptr || aligned16(a.k2)) && aligned16(a.v) && aligned16(a.out) && a.n_rows > 0 &&
+         a.n_rows < (1ll << 31) && (a.block_tables == nullptr || a.page % 16 == 0) && a.k_row >= static_cast<int64_t>(a.G) * a.d1 &&
+         a.v_row >= static_cast<int64_t>(a.Gv) * a.dv &&
+         (a.gate == nullptr || !a.gate_el || (reinterpret_cast<uintptr_t>(a.gate) % 4 == 0 && a.ldg % 2 == 0));
+}
+
+template <int NS, int NV>
+static int go_portion(const char* what, const PortionArgs& a, const PortionPlan& p, const PortionMaps& maps, int grid, cudaStream_t st) {
+  auto kern = portion_attn_kernel<NS, NV>;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, po_smem<NS>());
+  if (e != cudaSuccess) return cuda_fail(e, what);
+  kern<<<grid, PO_THREADS, po_smem<NS>(), st>>>(a, p, maps);
+  B2_CHECK_LAUNCH(what);
+  return B2TTS_OK;
+}
+
+int launch_portion_attn(const char* what, const PortionArgs& a, cudaStream_t st) {
+  int rc = wait_check(WAITS_PORTIONS, what);
+  if (rc != B2TTS_OK) return rc;
+  PortionPlan p{};
+  p.timeouts = wait_word(WAITS_PORTIONS);
+  B2_REQUIRE(p.timeouts != nullptr, B2TTS_ECUDA, "%s: no host memory for the kernel's status", what);
+  p.hpc = 1;                                           // heads of a key head that share a row tile: a power of two up to 8
+  while (p.hpc < 8 && (a.H / a.G) % (2 * p.hpc) == 0) { p.hpc *= 2; ++p.hpc_shift; }
+  p.page_shift = -1;
+  for (int x = 0; x < 30; ++x)
+    if (a.page == 1 << x) p.page_shift = x;
+  p.box_rows = 64;
+  while (a.block_tables != nullptr && a.page % p.box_rows) p.box_rows /= 2;
+  p.gate_vec = a.gate != nullptr && aligned16(a.gate) && a.ldg % 8 == 0;
+  // two row tiles an item share its key tiles; one, where two would leave multiprocessors without an item
+  const int per = 128 >> p.hpc_shift;
+  auto items = [&](int tiles) { return static_cast<int64_t>((a.max_new + tiles * per - 1) / (tiles * per)) * (a.H / p.hpc) * a.n_seqs; };
+  p.tiles = items(2) >= sm_count() ? 2 : 1;
+  const int64_t most = items(p.tiles);
+  const int grid = static_cast<int>(std::max<int64_t>(std::min<int64_t>(most, sm_count()), (most + PO_ITEMS - 1) / PO_ITEMS));
+  PortionMaps maps{};
+  {
+    const int64_t dims[3] = {a.d, a.H, a.n_tokens}, strides[2] = {a.q_head, a.q_tok};
+    const int box[3] = {64, p.hpc, per};
+    rc = make_tensor_map(&maps.q, a.q, 3, dims, strides, box, what);
+  }
+  const int box[2] = {64, p.box_rows};
+  {
+    const int64_t dims[2] = {static_cast<int64_t>(a.G) * a.d1, a.n_rows};
+    if (rc == B2TTS_OK) rc = make_tensor_map(&maps.k, a.k, 2, dims, &a.k_row, box, what);
+  }
+  if (a.d1 < a.d) {
+    const int64_t dims[2] = {a.d - a.d1, a.n_rows};
+    if (rc == B2TTS_OK) rc = make_tensor_map(&maps.k2, a.k2, 2, dims, &a.k2_row, box, what);
+  }
+  {
+    const int64_t dims[2] = {static_cast<int64_t>(a.Gv) * a.dv, a.n_rows};
+    if (rc == B2TTS_OK) rc = make_tensor_map(&maps.v, a.v, 2, dims, &a.v_row, box, what);
+  }
+  if (rc != B2TTS_OK) return rc;
+  const int ns = a.d / 64;
+#define PO_GO(NS, NV) return go_portion<NS, NV>(what, a, p, maps, grid, st)
+  if (a.dv == 64) {
+    if (ns == 1) PO_GO(1, 1);
+    if (ns == 2) PO_GO(2, 1);
+    PO_GO(3, 1);
+  }
+  if (ns == 1) PO_GO(1, 2);
+  if (ns == 2) PO_GO(2, 2);
+  PO_GO(3, 2);
+#undef PO_GO
+}
+
+}  // namespace row
+}  // namespace b2
+
+extern "C" int b2tts_portion_attn_timeouts(void) { return b2::wait_count(b2::WAITS_PORTIONS); }

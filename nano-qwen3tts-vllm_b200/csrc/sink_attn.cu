@@ -12,8 +12,8 @@
 // s into c tanh(s / c) before the softmax; v_heads < kv_heads makes key head g read value head g mod v_heads (several key
 // maps over one set of values).
 //
-// Three kernels share a launch: prompt portions in bf16 with head sizes 32..128 x 64, 128 run on the tensor cores
-// (sink_attn_mma_kernel), rows with ONE new token and a head size of 4, 8, 16 or 32 16-byte pieces (dv = d or 2 d) in a kernel whose
+// Four kernels share a launch: prompt portions in bf16 with head sizes 64, 128 x 64, 128 run on tcgen05 (portion_attn.cu), those with
+// other head sizes from 32 on or odd pages, and very short sequences, on mma.sync (sink_attn_mma_kernel), rows with ONE new token and a head size of 4, 8, 16 or 32 16-byte pieces (dv = d or 2 d) in a kernel whose
 // lanes split a cached row (sink_attn_decode_kernel), everything else in the plain kernel; each skips the rows of the others.
 //
 // Plain kernel (bf16 or float, any head size up to 256): one CTA of four warps per token and 1, 2 or 4 query heads of one
@@ -23,6 +23,7 @@
 // through shared memory.  Scores, weights and sums are float in both modes.
 #include <math.h>
 
+#include "portion_attn.cuh"
 #include "row_ops.cuh"
 
 namespace b2 {
@@ -821,6 +822,17 @@ extern "C" int b2tts_sink_attn(const void* q, const void* k_cache, const void* v
                                int n_tokens, int n_seqs, int max_new, int heads, int kv_heads, int v_heads, int dim, int vdim, int page,
                                int mask_kind, int mask, int keep_first, float softcap, float scale, int dtype, int path, int out_f32,
                                void* stream) {
+  return b2tts_sink_attn_rows(q, k_cache, v_cache, out, tok_seq, positions, seq_start, seq_pos0, seq_len, block_tables, bt_stride, sink, gate, ldg, gate_el,
+                              n_tokens, n_seqs, max_new, heads, kv_heads, v_heads, dim, vdim, page, mask_kind, mask, keep_first, softcap, scale, dtype, path,
+                              out_f32, 0, 0, stream);
+}
+
+extern "C" int b2tts_sink_attn_rows(const void* q, const void* k_cache, const void* v_cache, void* out, const int32_t* tok_seq,
+                                    const int32_t* positions, const int32_t* seq_start, const int32_t* seq_pos0, const int32_t* seq_len,
+                                    const int32_t* block_tables, int64_t bt_stride, const float* sink, const void* gate, int64_t ldg, int gate_el,
+                                    int n_tokens, int n_seqs, int max_new, int heads, int kv_heads, int v_heads, int dim, int vdim, int page,
+                                    int mask_kind, int mask, int keep_first, float softcap, float scale, int dtype, int path, int out_f32,
+                                    int64_t cache_rows, int max_keys, void* stream) {
   if (dtype == B2TTS_DTYPE_F32) out_f32 = 0;         // the outputs are floats already
   B2_REQUIRE(v_heads > 0 && kv_heads % v_heads == 0 && keep_first >= 0 && softcap >= 0.f, B2TTS_EINVAL,
              "sink_attn: bad switches (v_heads=%d of kv_heads=%d, keep_first=%d, softcap=%g)", v_heads, kv_heads, keep_first, softcap);
@@ -844,16 +856,38 @@ extern "C" int b2tts_sink_attn(const void* q, const void* k_cache, const void* v
   if (use_mma) {
     const int H = heads, G = kv_heads, Gv = v_heads;
     const void* kc = k_cache; const void* vc = v_cache; const int32_t* bt = block_tables;
-    cudaError_t e;
-    switch (dim) {
-      case 32: e = launch_sink_mma_dv<32>(vdim, SINK_MMA_ARGS); break;
-      case 48: e = launch_sink_mma_dv<48>(vdim, SINK_MMA_ARGS); break;
-      case 64: e = launch_sink_mma_dv<64>(vdim, SINK_MMA_ARGS); break;
-      case 96: e = launch_sink_mma_dv<96>(vdim, SINK_MMA_ARGS); break;
-      default: e = launch_sink_mma_dv<128>(vdim, SINK_MMA_ARGS); break;
+    using B = __nv_bfloat16;
+    PortionArgs p{};
+    p.q = static_cast<const B*>(q); p.q_tok = static_cast<int64_t>(H) * dim; p.q_head = dim; p.n_tokens = n_tokens;
+    p.k = static_cast<const B*>(kc); p.k_row = static_cast<int64_t>(G) * dim; p.d1 = dim;
+    p.v = static_cast<const B*>(vc); p.v_row = static_cast<int64_t>(Gv) * vdim;
+    p.n_rows = cache_rows;
+    p.block_tables = bt; p.bt_stride = bt_stride; p.page = page;
+    p.seq_start = seq_start; p.seq_pos0 = seq_pos0; p.seq_len = seq_len;
+    p.sink = sink; p.gate = static_cast<const B*>(gate); p.ldg = ldg; p.gate_el = gate_el;
+    p.out = out; p.out_f32 = out_f32;
+    p.H = H; p.G = G; p.Gv = Gv; p.d = dim; p.dv = vdim;
+    p.mask_kind = mask_kind; p.mask = mask; p.keep_first = keep_first; p.softcap = softcap; p.scale = scale;
+    p.n_seqs = n_seqs; p.max_new = max_new;
+    // The tcgen05 kernel takes 9 us to start and end where the other one takes 7; a tile of keys later it is the faster one.  16 heads over 8 of 128,
+    // graphs of ten layers, other / tcgen05 in us: 2 new tokens 15.6 / 17.8 (chunks) and 13.3 / 14.3 (window), 33 new 17.9 / 18.2 and 19.0 / 15.1,
+    // 2 x 64 20.1 / 19.3 and 21.9 / 16.8, 40 behind 1400 36.7 / 25.4 and 72.8 / 37.7, 2 x 2048 227 / 103 and 325 / 104.
+    const bool few = max_keys > 0 && max_keys <= 40;
+    if (!few && portion_attn_applies(p)) {
+      const int rc = launch_portion_attn("sink_attn (portions)", p, st);
+      if (rc != B2TTS_OK) return rc;
+    } else {
+      cudaError_t e;
+      switch (dim) {
+        case 32: e = launch_sink_mma_dv<32>(vdim, SINK_MMA_ARGS); break;
+        case 48: e = launch_sink_mma_dv<48>(vdim, SINK_MMA_ARGS); break;
+        case 64: e = launch_sink_mma_dv<64>(vdim, SINK_MMA_ARGS); break;
+        case 96: e = launch_sink_mma_dv<96>(vdim, SINK_MMA_ARGS); break;
+        default: e = launch_sink_mma_dv<128>(vdim, SINK_MMA_ARGS); break;
+      }
+      if (e != cudaSuccess) return cuda_fail(e, "sink_attn (tensor cores)");
+      B2_CHECK_LAUNCH("sink_attn (tensor cores)");
     }
-    if (e != cudaSuccess) return cuda_fail(e, "sink_attn (tensor cores)");
-    B2_CHECK_LAUNCH("sink_attn (tensor cores)");
   }
   // one-token rows: the row-splitting kernel where the head size fits it (path 1 keeps everything in the plain kernel)
   bool split = false;

@@ -36,7 +36,7 @@ class MixedStepLayout:
                 h = h.pin_memory()
             self.hosts.append(h)
             self.events.append(None)
-        self.n_tokens = self.n_seqs = self.max_new = self.n_want = 0
+        self.n_tokens = self.n_seqs = self.max_new = self.n_want = self.max_keys = 0
 
     def _view(self, buf, name):
         o, n = self.offsets[name]
@@ -96,6 +96,7 @@ class MixedStepLayout:
             self.events[self.cur] = ev
         self.n_tokens, self.n_seqs, self.n_want = o, n_seqs, len(want_rows)
         self.max_new = max((n for _, n in items), default=0)
+        self.max_keys = max((seq.num_cached_tokens + n for seq, n in items), default=0)    # 0: not known on the host
         self._bind()
 
     def _bind(self):
@@ -110,5 +111,5 @@ class MixedStepLayout:
     def set_decode_shape(self, rows: int):
         """Views for a captured decode step of ``rows`` one-token sequences (contents come from ``fill``)."""
         self.n_tokens = self.n_seqs = rows
-        self.max_new, self.n_want = 1, 0
+        self.max_new, self.n_want, self.max_keys = 1, 0, 0
         self._bind()

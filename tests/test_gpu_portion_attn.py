@@ -1,0 +1,124 @@
+"""Prompt attention on tcgen05 against 64-bit softmax attention: page sizes (the boxes that fetch keys shrink with them), kept first keys
+around box and tile edges, portions around the query and key tiles, several items per CTA, caches whose unused rows hold NaN, heads per
+key head, value heads, float outputs, gates and caps."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+BF = torch.bfloat16
+F64 = torch.float64
+
+
+@pytest.fixture(scope="module")
+def nat():
+    import nano_qwen3tts_vllm_b200._native as n
+    n.lib()
+    return n
+
+
+def _case(nat, seqs, *, H=4, G=2, Gv=None, d=64, dv=64, page=16, kind="window", mask=0, keep=0, cap=0.0, sink=True, gate="head", scale=None,
+          f32=False, seed=0, poison=False, known=False):
+    """``seqs`` = [(cached, new)].  Everything in the caches that no sequence owns is NaN."""
+    from tests.lm_util import Lay
+    Gv = Gv or G
+    g = torch.Generator().manual_seed(seed)
+    need = [-(-(c + n) // page) for c, n in seqs]
+    perm = (torch.randperm(sum(need), generator=g) + 1).tolist()
+    tabs = [perm[sum(need[:i]):sum(need[:i + 1])] for i in range(len(need))]
+    lay = Lay([(c, n, t) for (c, n), t in zip(seqs, tabs)], page, max(need))
+    if known:
+        lay.max_keys = max(c + n for c, n in seqs)
+    r = lambda *s: torch.randn(s, generator=g)
+    kc, vc = torch.full((sum(need) + 2, page, G * d), math.nan), torch.full((sum(need) + 2, page, Gv * dv), math.nan)
+    n_tok = lay.n_tokens
+    q, scale = r(n_tok, H * d).to(BF), scale if scale is not None else d ** -0.5
+    sk, gt = r(H), r(n_tok, H * dv if gate == "element" else H).to(BF)
+    ref, o = [], 0
+    for (c, n), t in zip(seqs, tabs):
+        k, v = r(c + n, G, d).to(BF), r(c + n, Gv, dv).to(BF)
+        for p in range(c + n):
+            kc[t[p // page], p % page], vc[t[p // page], p % page] = k[p].reshape(-1).float(), v[p].reshape(-1).float()
+        i, j = torch.arange(c, c + n)[:, None], torch.arange(c + n)[None]
+        ok = j <= i
+        if mask:
+            ok = ok & (((i - j < mask) if kind == "window" else (i // mask == j // mask)) | (j < keep))
+        if poison:                                                   # values that no new token of the sequence sees
+            for p in (~ok.any(0)).nonzero().flatten().tolist():
+                vc[t[p // page], p % page], v[p] = math.inf, 0
+        qq, out = q[o:o + n].view(n, H, d).to(F64), []
+        for h in range(H):
+            kg = h // (H // G)
+            s = qq[:, h] @ k[:, kg].to(F64).T * scale
+            if cap:
+                s = cap * torch.tanh(s / cap)
+            s = s.masked_fill(~ok, -math.inf)
+            if sink:
+                s = torch.cat([s, sk[h].to(F64).expand(n, 1)], 1)
+            p = s.softmax(-1)[:, :c + n]
+            out.append(p @ v[:, kg % Gv].to(F64))
+        y = torch.stack(out, 1)
+        gg = torch.sigmoid(gt[o:o + n].to(F64))
+        y = y * (gg.view(n, H, dv) if gate == "element" else gg[:, :, None] if gate == "head" else 1.0)
+        ref.append(y.reshape(n, -1))
+        o += n
+    ref = torch.cat(ref)
+    out = torch.empty(n_tok, H * dv, dtype=torch.float32 if f32 else BF, device=DEV)
+    nat.sink_attn(q.to(DEV), kc.to(BF).to(DEV), vc.to(BF).to(DEV), out, lay, sk.to(DEV) if sink else None, gt.to(DEV) if gate else None, H, G, d, dv,
+                  page, nat.MASK_WINDOW if kind == "window" else nat.MASK_CHUNK, mask, scale, nat.SINK_ATTN_TENSOR, v_heads=Gv, keep_first=keep,
+                  softcap=cap, gate_el=gate == "element")
+    err = (out.double().cpu() - ref).abs().max() / ref.abs().max()
+    # weights carry 16 bits and scores float sums (a few 1e-5 together); bf16 outputs round to 2^-9
+    assert err.item() < (5e-5 if f32 else 4e-3), err.item()
+    assert nat.portion_attn_timeouts() == 0
+
+
+@pytest.mark.parametrize("page", [16, 32, 48, 80, 256])
+def test_page_sizes(nat, page):
+    _case(nat, [(0, 150), (37, 141), (260, 5)], page=page, mask=70, seed=page, f32=True)
+
+
+@pytest.mark.parametrize("keep", [1, 4, 15, 16, 17, 40, 127, 128, 129, 300])
+@pytest.mark.parametrize("mask", [9, 130])
+def test_kept_first_keys(nat, keep, mask):
+    _case(nat, [(0, 200), (150, 90), (keep + mask - 1, 40), (keep + 20, 33)], mask=mask, keep=keep, seed=keep + mask, f32=True, sink=False, gate=None)
+
+
+@pytest.mark.parametrize("H,G", [(2, 2), (4, 2), (6, 2), (8, 2), (16, 1), (5, 1)])
+@pytest.mark.parametrize("d,dv", [(64, 64), (64, 128), (128, 64), (128, 128)])
+def test_heads_per_key_head_and_sizes(nat, H, G, d, dv):
+    _case(nat, [(0, 63), (3, 64), (0, 65), (500, 130), (8, 2), (11, 1)], H=H, G=G, d=d, dv=dv, mask=200, kind="chunk", gate="element", seed=H * d)
+
+
+@pytest.mark.parametrize("n", [2, 127, 128, 129, 255, 257, 513])
+@pytest.mark.parametrize("cached", [0, 1, 127, 128, 1000])
+def test_portions_around_the_tiles(nat, n, cached):
+    _case(nat, [(cached, n)], H=2, G=2, d=64, dv=64, page=64, seed=n + cached, cap=20.0 if n % 2 else 0.0, f32=n % 3 == 0)
+
+
+def test_value_heads_shared_by_key_heads_and_negative_scale(nat):
+    _case(nat, [(0, 140), (77, 60)], H=8, G=4, Gv=2, d=64, dv=128, mask=50, keep=3, sink=False, gate=None, f32=True)
+    _case(nat, [(0, 140), (77, 60)], H=4, G=2, scale=-0.2, f32=True)
+
+
+def test_scores_that_grow_along_the_keys(nat):
+    """The running maximum moves in every tile: weights are rescaled again and again."""
+    _case(nat, [(0, 700)], H=2, G=1, d=64, dv=64, scale=9.0, f32=True)
+
+
+@pytest.mark.parametrize("n", [1500, 3001])
+def test_several_items_for_every_cta(nat, n):
+    """Two row tiles an item and more items than multiprocessors; the ring and its barriers go on from item to item."""
+    _case(nat, [(0, n), (300, n - 700), (0, 1), (5, 33)], H=16, G=8, d=128, dv=128, page=64, mask=200, keep=4, gate="element", seed=n)
+
+
+def test_values_nobody_sees_may_be_infinite(nat):
+    """Rows in front of the window, behind the last key and beyond the kept ones share tiles with visible rows."""
+    _case(nat, [(700, 150), (90, 60)], H=4, G=2, d=64, dv=64, page=64, mask=100, keep=5, poison=True, f32=True)
+
+
+@pytest.mark.parametrize("keys", [2, 39, 40, 41, 64])
+def test_short_sequences_that_the_host_knows_of(nat, keys):
+    _case(nat, [(keys - 2, 2), (0, min(keys, 33)), (0, 1)], H=8, G=4, d=128, dv=128, page=64, mask=30, keep=2, gate="element", known=True, seed=keys)
