@@ -619,6 +619,25 @@ B2TTS_API int b2tts_sink_attn_rows(const void* q, const void* k_cache, const voi
                               int n_tokens, int n_seqs, int max_new, int heads, int kv_heads, int v_heads, int dim, int vdim,
                               int page, int mask_kind, int mask, int keep_first, float softcap, float scale, int dtype, int path,
                               int out_f32, int64_t cache_rows, int max_keys, void* stream);
+/* Rows of a paged latent cache that the step's sequences attend to (all keys, or from the window's bound of their first new token on,
+ * rounded down to a multiple of 64), sequence after sequence, into out [max_rows, width]; row of key j: key_start[b] + j.  max_keys: the
+ * longest sequence's.  cache_rows bounds what is read: rows that a table should not name come out as zeros.  bf16, width a multiple of 8. */
+B2TTS_API int b2tts_latent_gather(const void* cache, int64_t cache_rows, void* out, int32_t* key_start, const int32_t* block_tables,
+                                  int64_t bt_stride, const int32_t* seq_pos0, const int32_t* seq_len, int n_seqs, int max_keys, int max_rows,
+                                  int window, int width, int page, void* stream);
+/* Turns the last rot_dims coordinates' pairs (2 i, 2 i + 1) from `off` on of every head of q, in place: angle positions[t] * freq[i], lengths
+ * times rot_mult.  bf16; off, rot_dims, q_tok and q_head multiples of 8. */
+B2TTS_API int b2tts_latent_turn(void* q, int64_t q_tok, int64_t q_head, int off, const int32_t* positions, const float* freq, float rot_mult,
+                                int rot_dims, int n_tokens, int heads, void* stream);
+/* Latent attention of sequences with more than one new token over keys and values expanded per head: key j of head h is
+ * [k[row, h * dim ..] | kr[row, ..rot_dim]] with row = key_start[b] + j < n_rows, its value v[row, h * vdim ..]; queries (token, head,
+ * dim + rot_dim), turned, at q + token * q_tok + head * q_head; out [tokens, heads * vdim].  Optional sink per head and sigmoid gate per
+ * head or (gate_el) per output element.  bf16; dim and rot_dim multiples of 64, together up to 192, vdim 64 or 128. */
+B2TTS_API int b2tts_latent_portions_attn(const void* q, int64_t q_tok, int64_t q_head, const void* k, int64_t k_row, const void* kr,
+                                         int64_t kr_row, const void* v, int64_t v_row, int64_t n_rows, const int32_t* key_start, void* out,
+                                         const float* sink, const void* gate, int64_t ldg, int gate_el, const int32_t* seq_start,
+                                         const int32_t* seq_pos0, const int32_t* seq_len, int n_tokens, int n_seqs, int max_new, int heads,
+                                         int dim, int rot_dim, int vdim, int window, float scale, void* stream);
 /* out[t, c] = act(bias[c] + sum_j w[c, j] * u(position(t) - taps + 1 + j)[c_off + c]) for c < channels (act 0: none, 1: SiLU;
  * bias may be null).  Earlier positions come from this step's rows, from state [slots, taps-1, channels] (the sequence's last
  * rows, oldest first, advanced by this call) or are zero before position 0.  max_new >= every seq_len[b] (0: unknown). */

@@ -122,6 +122,9 @@ def _load():
         "b2tts_sink_attn": (I, [P, P, P, P, P, P, P, P, P, P, L, P, P, L, I, I, I, I, I, I, I, I, I, I, I, I, I, F, F, I, I, I, P]),
         "b2tts_sink_attn_rows": (I, [P, P, P, P, P, P, P, P, P, P, L, P, P, L, I, I, I, I, I, I, I, I, I, I, I, I, I, F, F, I, I, I, L, I, P]),
         "b2tts_portion_attn_timeouts": (I, []),
+        "b2tts_latent_gather": (I, [P, L, P, P, P, L, P, P, I, I, I, I, I, I, P]),
+        "b2tts_latent_turn": (I, [P, L, L, I, P, P, F, I, I, I, P]),
+        "b2tts_latent_portions_attn": (I, [P, L, L, P, L, P, L, P, L, L, P, P, P, P, L, I, P, P, P, I, I, I, I, I, I, I, I, F, P]),
         "b2tts_gated_linear_scan": (I, [P, L, P, L, P, L, P, L, P, F, P, P, P, P, P, P, P, I, I, I, I, I, I, P]),
         "b2tts_sandwich_residual": (I, [P, P, P, I, P, P, P, F, P, P, P, I, I, P, P, P, P, I, I, I, F, I, P]),
         "b2tts_polynorm": (I, [P, P, I, I, F, I, P]),
@@ -977,6 +980,39 @@ def latent_attn(ql, ql_strides, qr, qr_strides, cache, out, out_strides, sink, f
                                   rot_mult, rot_dims, lay.seq_start.data_ptr(), lay.seq_pos0.data_ptr(), lay.seq_len.data_ptr(),
                                   lay.block_tables.data_ptr(), lay.block_tables.stride(0), lay.n_seqs, lay.max_new, heads,
                                   kv_rank, rot_dim, page, window, scale, dt, path, splits, _ptr(ws), _stream()), "latent_attn")
+
+
+def latent_gather(cache, lay, window, rows, max_keys):
+    """The cached latents that the step's sequences attend to, side by side: ([rows, width], key_start [n_seqs]); see b2tts_latent_gather."""
+    _cuda(cache, BF16, "cache")
+    assert cache.is_contiguous()
+    width = cache.shape[-1]
+    out = torch.empty(rows, width, dtype=BF16, device=cache.device)
+    key_start = torch.empty(lay.n_seqs, dtype=torch.int32, device=cache.device)
+    _check(_load().b2tts_latent_gather(cache.data_ptr(), cache.numel() // width, out.data_ptr(), key_start.data_ptr(), lay.block_tables.data_ptr(),
+                                       lay.block_tables.stride(0), lay.seq_pos0.data_ptr(), lay.seq_len.data_ptr(), lay.n_seqs, max_keys, rows,
+                                       window, width, cache.shape[1], _stream()), "latent_gather")
+    return out, key_start
+
+
+def latent_turn(q, q_strides, off, lay, freq, rot_mult, rot_dims, heads):
+    """The rotated parts of the queries, in place."""
+    _cuda(q, BF16, "q")
+    _check(_load().b2tts_latent_turn(q.data_ptr(), q_strides[0], q_strides[1], off, lay.positions.data_ptr(), freq.data_ptr(), rot_mult, rot_dims,
+                                     q.shape[0], heads, _stream()), "latent_turn")
+
+
+def latent_portions_attn(q, q_strides, k, kr, v, key_start, out, lay, sink, gate, gate_el, heads, dim, rot_dim, vdim, window, scale):
+    """Latent attention of prompt portions over expanded keys and values (row strides of ``k``, ``kr`` and ``v`` are theirs)."""
+    for t in (q, k, v, out):
+        _cuda(t, BF16, "latent_portions_attn operand")
+    assert k.stride(1) == 1 and v.stride(1) == 1 and (kr is None or kr.stride(1) == 1) and out.is_contiguous()
+    _check(_load().b2tts_latent_portions_attn(q.data_ptr(), q_strides[0], q_strides[1], k.data_ptr(), k.stride(0), _ptr(kr),
+                                              0 if kr is None else kr.stride(0), v.data_ptr(), v.stride(0), min(k.shape[0], v.shape[0]),
+                                              key_start.data_ptr(), out.data_ptr(), _ptr(sink), _ptr(gate), 0 if gate is None else gate.stride(0),
+                                              int(gate_el), lay.seq_start.data_ptr(), lay.seq_pos0.data_ptr(), lay.seq_len.data_ptr(), q.shape[0],
+                                              lay.n_seqs, lay.max_new, heads, dim, rot_dim, vdim, window, scale, _stream()), "latent_portions_attn")
+    return out
 
 
 def latent_attn_timeouts() -> int:

@@ -300,6 +300,67 @@ __global__ void silu_mul_kernel(const T* __restrict__ gu, T* __restrict__ y, siz
   }
 }
 
+// Rows of the latent cache that portions attend to, side by side: sequence b's keys from lo(b) on, lo(b) = its window's lower bound
+// rounded down to whole boxes of the attention kernel, sequence after sequence.  Row of key j: key_start[b] + j.  Bound: HBM (rows
+// read and written once); a warp copies one row of `width` numbers (a multiple of 8) in 16-byte pieces.
+__device__ __forceinline__ int first_key(int pos0, int window) { return window > 0 ? max(0, pos0 - window + 1) & ~63 : 0; }
+__global__ void __launch_bounds__(256)
+latent_gather_kernel(const __nv_bfloat16* __restrict__ cache, int64_t cache_rows, __nv_bfloat16* __restrict__ out, int32_t* __restrict__ key_start,
+                     const int32_t* __restrict__ block_tables, int64_t bt_stride, const int32_t* __restrict__ seq_pos0,
+                     const int32_t* __restrict__ seq_len, int window, int width, int page, int max_rows) {
+  __shared__ int sum[8];
+  const int b = blockIdx.y, tid = threadIdx.x;
+  int before = 0;                                          // rows of the sequences in front
+  for (int i = tid; i < b; i += 256)
+    if (seq_len[i] > 0) before += seq_pos0[i] + seq_len[i] - first_key(seq_pos0[i], window);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+  if ((tid & 31) == 0) sum[tid >> 5] = before;
+  __syncthreads();
+  before = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) before += sum[i];
+  const int lo = first_key(seq_pos0[b], window), n = seq_len[b] > 0 ? seq_pos0[b] + seq_len[b] - lo : 0;
+  if (blockIdx.x == 0 && tid == 0) key_start[b] = before - lo;
+  const int32_t* bt = block_tables + b * bt_stride;
+  for (int r = blockIdx.x * 8 + (tid >> 5); r < n && before + r < max_rows; r += gridDim.x * 8) {
+    const int j = lo + r;
+    const int64_t slot = static_cast<int64_t>(bt[j / page]) * page + j % page;
+    const bool there = slot >= 0 && slot < cache_rows;
+    const uint4* src = reinterpret_cast<const uint4*>(cache + (there ? slot : 0) * width);
+    uint4* dst = reinterpret_cast<uint4*>(out + static_cast<size_t>(before + r) * width);
+    for (int c = tid & 31; c < width / 8; c += 32) dst[c] = there ? src[c] : make_uint4(0u, 0u, 0u, 0u);
+  }
+}
+
+// Queries' rotated parts in place: a CTA takes one token, forms its angles once and turns eight coordinates of a head per thread.
+__global__ void __launch_bounds__(128)
+latent_turn_kernel(__nv_bfloat16* __restrict__ q, int64_t q_tok, int64_t q_head, int off, const int32_t* __restrict__ positions,
+                   const float* __restrict__ freq, float rot_mult, int rot_dims, int heads) {
+  extern __shared__ float2 turn[];
+  const float p = static_cast<float>(positions[blockIdx.x]);
+  for (int i = threadIdx.x; i < rot_dims / 2; i += 128) {
+    float sn, cs;
+    sincosf(p * freq[i], &sn, &cs);
+    turn[i] = make_float2(cs * rot_mult, sn * rot_mult);
+  }
+  __syncthreads();
+  const int per = rot_dims / 8;
+  for (int i = threadIdx.x; i < heads * per; i += 128) {
+    const int h = i / per, c = i - h * per;
+    __nv_bfloat16* at = q + blockIdx.x * q_tok + h * q_head + off + c * 8;
+    uint4 x = ldg_v4(at);
+    uint32_t* w = &x.x;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 t = turn[c * 4 + e];
+      const float a = bf16lo(w[e]), b = bf16hi(w[e]);
+      w[e] = pack_bf16(a * t.x - b * t.y, b * t.x + a * t.y);
+    }
+    stg_v4(at, x);
+  }
+}
+
 static int flat_grid(size_t n) { return static_cast<int>(std::min<size_t>((n + 255) / 256, 148 * 16)); }
 
 }  // namespace lat
@@ -428,5 +489,39 @@ extern "C" int b2tts_silu_mul(const void* gu, void* y, int64_t rows, int ff, int
   LAT_DISPATCH(dtype, (silu_mul_kernel<T><<<flat_grid(static_cast<size_t>(rows) * ff), 256, 0, st>>>(static_cast<const T*>(gu), static_cast<T*>(y),
                                                                                                   static_cast<size_t>(rows), ff)));
   B2_CHECK_LAUNCH("silu_mul");
+  return B2TTS_OK;
+}
+
+extern "C" int b2tts_latent_gather(const void* cache, int64_t cache_rows, void* out, int32_t* key_start, const int32_t* block_tables,
+                                   int64_t bt_stride, const int32_t* seq_pos0, const int32_t* seq_len, int n_seqs, int max_keys, int max_rows,
+                                   int window, int width, int page, void* stream) {
+  using namespace b2;
+  using namespace b2::lat;
+  B2_REQUIRE(n_seqs >= 0 && max_keys >= 0 && max_rows >= 0 && window >= 0 && page > 0 && width > 0 && width % 8 == 0 && cache_rows > 0, B2TTS_EINVAL,
+             "latent_gather: bad sizes (width=%d page=%d)", width, page);
+  B2_REQUIRE(n_seqs <= 65535, B2TTS_EUNSUPPORTED, "latent_gather: %d sequences", n_seqs);
+  if (n_seqs == 0) return B2TTS_OK;
+  B2_REQUIRE(cache && out && key_start && block_tables && seq_pos0 && seq_len, B2TTS_EINVAL, "latent_gather: null pointer");
+  B2_REQUIRE(aligned16(cache) && aligned16(out), B2TTS_EALIGN, "latent_gather: rows must start on 16-byte boundaries");
+  const int gx = std::max(1, std::min((max_keys + 7) / 8, 512));
+  latent_gather_kernel<<<dim3(gx, n_seqs), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const __nv_bfloat16*>(cache), cache_rows, static_cast<__nv_bfloat16*>(out), key_start, block_tables, bt_stride, seq_pos0, seq_len,
+      window, width, page, max_rows);
+  B2_CHECK_LAUNCH("latent_gather");
+  return B2TTS_OK;
+}
+
+extern "C" int b2tts_latent_turn(void* q, int64_t q_tok, int64_t q_head, int off, const int32_t* positions, const float* freq, float rot_mult,
+                                 int rot_dims, int n_tokens, int heads, void* stream) {
+  using namespace b2;
+  using namespace b2::lat;
+  B2_REQUIRE(n_tokens >= 0 && heads > 0 && off >= 0 && off % 8 == 0 && rot_dims >= 0 && rot_dims % 8 == 0 && rot_dims <= 4096 && q_tok % 8 == 0 && q_head % 8 == 0,
+             B2TTS_EINVAL, "latent_turn: bad sizes (off=%d rot_dims=%d)", off, rot_dims);
+  if (n_tokens == 0 || rot_dims == 0) return B2TTS_OK;
+  B2_REQUIRE(q && positions && freq, B2TTS_EINVAL, "latent_turn: null pointer");
+  B2_REQUIRE(aligned16(q), B2TTS_EALIGN, "latent_turn: rows must start on 16-byte boundaries");
+  latent_turn_kernel<<<n_tokens, 128, rot_dims / 2 * sizeof(float2), static_cast<cudaStream_t>(stream)>>>(
+      static_cast<__nv_bfloat16*>(q), q_tok, q_head, off, positions, freq, rot_mult, rot_dims, heads);
+  B2_CHECK_LAUNCH("latent_turn");
   return B2TTS_OK;
 }

@@ -22,7 +22,8 @@
 // each in two passes over TMEM keep everything in 96 registers: spilled ones went through L2, since shared memory leaves L1 next to nothing
 // (one thread a row with 40 spilled registers: 143 us for the case below; one barrier per slot of the ring instead of per tile: 20 us more).
 // 4 prompts of 2048 tokens, 16 heads over 8 of 128, window 1024 + 4 kept, element gates: 118 us (mma.sync, 64 queries per CTA: 547 us; 31 at
-// the tensor core's rate); causal with a score cap, 4448 tokens: 141 us (579 us).
+// the tensor core's rate); causal with a score cap, 4448 tokens: 141 us (579 us); latent
+// heads of 192 over expanded keys, 4 x 2048 causal: 152 us.
 //
 // Every copy is bounded: maps have the true extents of their tensors, so a row that a block table should not name reads zeros.  Every
 // commit of the last products is waited for before the CTA leaves.
@@ -715,5 +716,36 @@ int launch_portion_attn(const char* what, const PortionArgs& a, cudaStream_t st)
 
 }  // namespace row
 }  // namespace b2
+
+extern "C" int b2tts_latent_portions_attn(const void* q, int64_t q_tok, int64_t q_head, const void* k, int64_t k_row, const void* kr,
+                                          int64_t kr_row, const void* v, int64_t v_row, int64_t n_rows, const int32_t* key_start, void* out,
+                                          const float* sink, const void* gate, int64_t ldg, int gate_el, const int32_t* seq_start,
+                                          const int32_t* seq_pos0, const int32_t* seq_len, int n_tokens, int n_seqs, int max_new, int heads,
+                                          int dim, int rot_dim, int vdim, int window, float scale, void* stream) {
+  using namespace b2;
+  using namespace b2::row;
+  B2_REQUIRE(n_tokens >= 0 && n_seqs >= 0 && max_new >= 0 && heads > 0 && dim > 0 && rot_dim >= 0 && vdim > 0 && window >= 0, B2TTS_EINVAL,
+             "latent_portions_attn: bad sizes");
+  B2_REQUIRE(heads <= 65535 && n_seqs <= 65535, B2TTS_EUNSUPPORTED, "latent_portions_attn: %d heads, %d sequences", heads, n_seqs);
+  if (n_tokens == 0 || n_seqs == 0 || max_new <= 1) return B2TTS_OK;
+  B2_REQUIRE(q && k && v && key_start && out && seq_start && seq_pos0 && seq_len && (rot_dim == 0 || kr), B2TTS_EINVAL,
+             "latent_portions_attn: null pointer");
+  using B = __nv_bfloat16;
+  PortionArgs p{};
+  p.q = static_cast<const B*>(q); p.q_tok = q_tok; p.q_head = q_head; p.n_tokens = n_tokens;
+  p.k = static_cast<const B*>(k); p.k_row = k_row; p.d1 = dim;
+  p.k2 = rot_dim > 0 ? static_cast<const B*>(kr) : nullptr; p.k2_row = rot_dim > 0 ? kr_row : 0;
+  p.v = static_cast<const B*>(v); p.v_row = v_row;
+  p.n_rows = n_rows;
+  p.key_start = key_start; p.page = 1;
+  p.seq_start = seq_start; p.seq_pos0 = seq_pos0; p.seq_len = seq_len;
+  p.sink = sink; p.gate = static_cast<const B*>(gate); p.ldg = ldg; p.gate_el = gate_el;
+  p.out = out;
+  p.H = heads; p.G = heads; p.Gv = heads; p.d = dim + rot_dim; p.dv = vdim;
+  p.mask = window; p.scale = scale;
+  p.n_seqs = n_seqs; p.max_new = max_new;
+  B2_REQUIRE(portion_attn_applies(p), B2TTS_EUNSUPPORTED, "latent_portions_attn: dim=%d rot_dim=%d vdim=%d or a row alignment", dim, rot_dim, vdim);
+  return launch_portion_attn("latent_portions_attn", p, static_cast<cudaStream_t>(stream));
+}
 
 extern "C" int b2tts_portion_attn_timeouts(void) { return b2::wait_count(b2::WAITS_PORTIONS); }

@@ -37,6 +37,7 @@ class MixedStepLayout:
             self.hosts.append(h)
             self.events.append(None)
         self.n_tokens = self.n_seqs = self.max_new = self.n_want = self.max_keys = 0
+        self.portions = None
 
     def _view(self, buf, name):
         o, n = self.offsets[name]
@@ -97,6 +98,8 @@ class MixedStepLayout:
         self.n_tokens, self.n_seqs, self.n_want = o, n_seqs, len(want_rows)
         self.max_new = max((n for _, n in items), default=0)
         self.max_keys = max((seq.num_cached_tokens + n for seq, n in items), default=0)    # 0: not known on the host
+        # (tokens cached, tokens new) per live row on the host: what sizes a launch or a buffer of the step
+        self.portions = [(seq.num_cached_tokens, n) for seq, n in items]
         self._bind()
 
     def _bind(self):
@@ -112,4 +115,5 @@ class MixedStepLayout:
         """Views for a captured decode step of ``rows`` one-token sequences (contents come from ``fill``)."""
         self.n_tokens = self.n_seqs = rows
         self.max_new, self.n_want, self.max_keys = 1, 0, 0
+        self.portions = None
         self._bind()

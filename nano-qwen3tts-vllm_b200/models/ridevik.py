@@ -13,7 +13,8 @@ Every layer carries its own sizes (``config.RidevikLayerSpec``); a layer with ``
 over a cache and state of its own.  One forward runs a whole engine step: prompt portions and single decoded tokens side
 by side, described by the step layout in the global Context.  Launches per layer: token shift, merged input GEMM,
 latent preparation (norms, key rotation, cache write), [query up-projection], per-head W_uk^T (batched GEMM), attention,
-per-head W_uv (batched GEMM), gate + re-layout, output GEMM, residual + group norm, the feed-forward, residual + group norm.
+per-head W_uv (batched GEMM), gate + re-layout, output GEMM, residual + group norm, the feed-forward, residual + group norm.  Steps of
+long prompt portions expand the latents to per-head keys and values instead (``LatentAttentionMixer.expanded_rows``).
 """
 from __future__ import annotations
 
@@ -72,14 +73,57 @@ class LatentAttentionMixer(nn.Module):
                         m.q_rank, m.kv_rank, m.rot_dim, m.rot.dims, self.eps)
         q = self.uq(cq) if m.q_rank else u                                       # heads laid out [dim | rot_dim] each
         hd = m.dim + m.rot_dim
+        gate = u[:, self.q_in + m.kv_rank + m.rot_dim:] if m.gate else None
+        rows = self.expanded_rows(q, gate, cache, lay)
+        if rows is not None:
+            return self.o_proj(self.attend_expanded(q, gate, cache, lay, *rows))
         qn = torch.as_strided(q, (m.heads, n, m.dim), (hd, q.stride(0), 1))     # un-rotated parts, head-major view
         ql = per_head_linear(qn, self.uk)                                        # [heads, n, kv_rank] = W_uk,h^T q
         o = self.attn(ql, q[:, m.dim:], (q.stride(0), hd), cache)                # [heads, n, kv_rank]
         v = per_head_linear(o, self.uv, transpose_weight=True)                   # [heads, n, vdim]
         heads_out = torch.empty(n, m.heads * m.vdim, dtype=hs.dtype, device=hs.device)
-        gate = u[:, self.q_in + m.kv_rank + m.rot_dim:] if m.gate else None
         nat.gate_heads(v, (m.vdim, n * m.vdim), gate, heads_out, m.heads, m.vdim, per_head=m.head_gate)
         return self.o_proj(heads_out)
+
+    # Portions over expanded keys and values.  Absorbed queries make a (query, key) pair of a head cost 2 r + dr products where per-head
+    # keys and values cost dim + rot_dim + vdim (1088 against 320 at a latent of 512 + 64 and heads of 128), and the plain layout is what the
+    # tcgen05 kernel takes.  16 heads, width 2048, a mixer in us, absorbed / expanded: 4 x 2048 causal 1967 / 365; 2048 610 / 152; 800 169 /
+    # 150; 200 new behind 1400 145 / 158; 500 138 / 163.  The small ones are bound by the host, which has two launches more to make (on the
+    # device alone, from a graph, the lines cross at 100 tokens), so the least number of pairs, over all heads, lies where the absorbed
+    # form's own time passes that.  Decode steps, steps with a portion of a few tokens and float32 stay with the absorbed form.
+    EXPAND_MIN_NEW, EXPAND_MIN_PAIRS = 32, 1 << 23
+    EXPAND_MAX_BYTES = 1 << 30                 # of expanded keys and values
+
+    def expanded_rows(self, q, gate, cache, lay):
+        """(rows, longest sequence's rows) of the expanded form, or None where the step does not take it."""
+        m, portions = self.spec, getattr(lay, "portions", None)
+        if not portions or q.dtype != torch.bfloat16 or min(n for _, n in portions) < self.EXPAND_MIN_NEW:
+            return None
+        if m.vdim not in (64, 128) or m.dim % 64 or m.rot_dim % 64 or m.dim + m.rot_dim > 192 or m.kv_rank % 8 or m.rot.dims % 8:
+            return None
+        if q.stride(0) % 8 or q.data_ptr() % 16 or cache.data_ptr() % 16 or not cache.is_contiguous():
+            return None
+        if gate is not None and not m.head_gate and (gate.data_ptr() % 4 or gate.stride(0) % 2):
+            return None
+        low = lambda c: (max(0, c - m.window + 1) & ~63) if m.window else 0      # as latent_gather
+        rows = [c + n - low(c) for c, n in portions]
+        if m.heads * sum(n * r for (_, n), r in zip(portions, rows)) < self.EXPAND_MIN_PAIRS:
+            return None
+        total = sum(rows)
+        return (total, max(rows)) if 2 * total * m.heads * (m.dim + m.vdim) <= self.EXPAND_MAX_BYTES else None
+
+    def attend_expanded(self, q, gate, cache, lay, rows, longest):
+        """``q`` is this forward's own: its rotated parts are turned where they are."""
+        m = self.spec
+        strides = (q.stride(0), m.dim + m.rot_dim)
+        lat, key_start = nat.latent_gather(cache, lay, m.window, rows, longest)
+        nat.latent_turn(q, strides, m.dim, lay, self.rotary.freq, self.rotary.mult, self.rotary.dims, m.heads)
+        c = lat[:, :m.kv_rank]
+        k = torch.nn.functional.linear(c, self.uk.view(-1, m.kv_rank))
+        v = torch.nn.functional.linear(c, self.uv.view(-1, m.kv_rank))
+        out = torch.empty(q.shape[0], m.heads * m.vdim, dtype=q.dtype, device=q.device)
+        return nat.latent_portions_attn(q, strides, k, lat[:, m.kv_rank:] if m.rot_dim else None, v, key_start, out, lay, self.attn.sink, gate,
+                                        not m.head_gate, m.heads, m.dim, m.rot_dim, m.vdim, m.window, m.scale)
 
 
 class XieluFF(nn.Module):
