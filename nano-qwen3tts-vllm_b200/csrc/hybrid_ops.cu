@@ -462,6 +462,190 @@ static void launch_head_prep(const HeadPrepArgs& p, cudaStream_t st) {
 #undef HP_GO_T
 }
 
+// Both preparations for bf16 rows in 16-byte pieces: a CTA takes TOK tokens, forms (or copies) their angles once for all heads, and a thread
+// takes eight coordinates of one head of all of them, with bias and norm weight in registers and the TOK pieces asked for before the first
+// is used.  d / 8 neighbouring lanes hold a head: they sum its squares, and hand each other the partners i, i + rot_dims / 2.
+// Bound: HBM (u read, queries and cache rows written once) where nothing is normed, issue and latency of the norms else.  16 + 8 + 8 heads of
+// 128, 8192 tokens (20 us at the copy rate), kernels above / this one in us: plain 93 / 31, 64 coordinates turned 116 / 37, whole norms and
+// turns 131 / 74, head norms and a table 65 / 45 (pairs) and 122 / 58 (halves); 64 tokens 6.9 / 2.5, 9.1 / 3.0, 12.9 / 5.4.  One number a
+// thread and step, and angles formed again for every head, were what the first three cost.  Two tokens a CTA: four take 124 registers
+// and are slower where norms are formed (head norms 51, whole norms 106 us), as fast where not.
+struct PrepArgs {
+  const __nv_bfloat16* u; int64_t ldu; int q_off, k_off, v_off;              // v_off < 0: the values are the keys before norm and rotation
+  const float *q_bias, *k_bias, *v_bias, *q_norm_w, *k_norm_w;
+  int norm;                                                                  // 0: none, 1: over the whole projection, 2: head by head
+  const float *rot, *freq; const int32_t* positions; int rot_dims, interleaved;   // a table [n, rot_dims] or frequencies
+  const int32_t* slot_mapping;
+  __nv_bfloat16 *q_out, *k_cache, *v_cache;
+  int n_tokens, H, G, Gv, d, dv;
+  float eps;
+};
+constexpr int PREP_MAX_ROT = 512;
+
+__device__ __forceinline__ void unpack8(const uint4& x, float* f) {
+  f[0] = bf16lo(x.x); f[1] = bf16hi(x.x); f[2] = bf16lo(x.y); f[3] = bf16hi(x.y);
+  f[4] = bf16lo(x.z); f[5] = bf16hi(x.z); f[6] = bf16lo(x.w); f[7] = bf16hi(x.w);
+}
+__device__ __forceinline__ void load8_f(const float* p, float* f) {
+  const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+  f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+}
+
+template <int TOK, int LPH>
+__global__ void __launch_bounds__(ROW_THREADS)
+prep_vec8_kernel(const PrepArgs p) {
+  extern __shared__ __align__(16) float2 turn[];                        // [TOK][rot_dims / 2]: cosine, sine
+  __shared__ float red[33], inv_s[2][TOK];
+  const int t0 = blockIdx.x * TOK, tid = threadIdx.x, half = p.rot_dims / 2;
+  const int nq = p.H * p.d, nk = p.G * p.d, nv = p.Gv * p.dv;
+  int slot[TOK];
+#pragma unroll
+  for (int t = 0; t < TOK; ++t) slot[t] = t0 + t < p.n_tokens ? p.slot_mapping[t0 + t] : -1;      // -1: padding row, or behind the last token
+  const int q8 = nq / 8, k8 = p.k_cache != nullptr ? nk / 8 : 0, v8 = p.v_cache != nullptr ? nv / 8 : 0, items = q8 + k8 + v8;
+  const int lane = tid & 31;                              // LPH = d / 8 lanes have a head
+  uint4 x[TOK], ahead[TOK];                               // a thread's pieces, and those of its next turn
+  auto load = [&](int i) {
+    const bool is_q = i < q8, is_k = !is_q && i < q8 + k8;
+    const int c = (is_q ? i : is_k ? i - q8 : i - q8 - k8) * 8, off = is_q ? p.q_off : is_k || p.v_off < 0 ? p.k_off : p.v_off;
+#pragma unroll
+    for (int t = 0; t < TOK; ++t) {
+      ahead[t] = make_uint4(0u, 0u, 0u, 0u);
+      if (i < items && slot[t] >= 0) ahead[t] = ldg_v4(p.u + static_cast<int64_t>(t0 + t) * p.ldu + off + c);
+    }
+  };
+  load(tid);
+  for (int i = tid; i < TOK * half; i += ROW_THREADS) {
+    const int t = i / half, c = i - t * half;
+    if (t0 + t >= p.n_tokens) break;
+    float2 cs;
+    if (p.rot != nullptr) {
+      const float* row = p.rot + static_cast<int64_t>(t0 + t) * p.rot_dims;
+      cs = make_float2(row[c], row[half + c]);
+    } else {
+      sincosf(static_cast<float>(p.positions[t0 + t]) * p.freq[c], &cs.y, &cs.x);
+    }
+    turn[i] = cs;
+  }
+  if (p.norm == 1) {
+    for (int t = 0; t < TOK; ++t) {
+      if (slot[t] < 0) continue;                          // uniform over the block
+      const __nv_bfloat16* ur = p.u + static_cast<int64_t>(t0 + t) * p.ldu;
+      for (int side = 0; side < 2; ++side) {
+        const int n = side ? nk : nq;
+        const float* bias = side ? p.k_bias : p.q_bias;
+        float ss = 0.f;
+        for (int c = tid * 8; c < n; c += ROW_THREADS * 8) {
+          float f[8], b[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+          unpack8(ldg_v4(ur + (side ? p.k_off : p.q_off) + c), f);
+          if (bias != nullptr) load8_f(bias + c, b);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) { const float v = f[e] + b[e]; ss += v * v; }
+        }
+        const float sum = block_sum(ss, red);
+        if (tid == 0) inv_s[side][t] = 1.0f / sqrtf(sum / static_cast<float>(n) + p.eps);
+      }
+    }
+  }
+  __syncthreads();
+  for (int base = tid & ~31; base < items; base += ROW_THREADS) {              // a warp stays together for the shuffles
+    const int i = base + lane;
+    const bool live = i < items, is_q = i < q8, is_k = !is_q && i < q8 + k8;
+    const int c = (is_q ? i : is_k ? i - q8 : i - q8 - k8) * 8;
+    const float* bias = is_q ? p.q_bias : is_k || p.v_off < 0 ? p.k_bias : p.v_bias;
+#pragma unroll
+    for (int t = 0; t < TOK; ++t) x[t] = ahead[t];
+    load(i + ROW_THREADS);
+    float b[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, w[8] = {1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f};
+    if (live && bias != nullptr) load8_f(bias + c, b);
+    const bool qk = live && (is_q || is_k);
+    const int ci = qk ? c % p.d : p.d;                    // the piece's first coordinate in its head
+    if (qk && p.norm != 0) load8_f((is_q ? p.q_norm_w : p.k_norm_w) + (p.norm == 2 ? ci : c), w);
+    const bool turned = qk && ci < p.rot_dims;
+    float inv[TOK];
+#pragma unroll
+    for (int t = 0; t < TOK; ++t) inv[t] = 1.f;
+    if (p.norm == 2) {
+#pragma unroll
+      for (int t = 0; t < TOK; ++t) {
+        float f[8];
+        unpack8(x[t], f);
+        inv[t] = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) { const float v = f[e] + b[e]; inv[t] += v * v; }
+      }
+#pragma unroll
+      for (int o = LPH / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int t = 0; t < TOK; ++t) inv[t] += __shfl_xor_sync(0xffffffffu, inv[t], o);
+#pragma unroll
+      for (int t = 0; t < TOK; ++t) inv[t] = qk ? 1.0f / sqrtf(inv[t] / static_cast<float>(p.d) + p.eps) : 1.f;
+    } else if (p.norm == 1 && qk) {
+#pragma unroll
+      for (int t = 0; t < TOK; ++t) inv[t] = inv_s[is_k][t];
+    }
+#pragma unroll
+    for (int t = 0; t < TOK; ++t) {
+      float f[8];
+      unpack8(x[t], f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) f[e] = (f[e] + b[e]) * inv[t] * w[e];
+      if (p.rot_dims > 0 && p.interleaved) {
+        if (turned) {
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float4 cs = reinterpret_cast<const float4*>(turn + t * half + ci / 2)[e];
+            const float a0 = f[4 * e], a1 = f[4 * e + 2];
+            f[4 * e] = a0 * cs.x - f[4 * e + 1] * cs.y;     f[4 * e + 1] = f[4 * e + 1] * cs.x + a0 * cs.y;
+            f[4 * e + 2] = a1 * cs.z - f[4 * e + 3] * cs.w; f[4 * e + 3] = f[4 * e + 3] * cs.z + a1 * cs.w;
+          }
+        }
+      } else if (p.rot_dims > 0) {
+        const bool second = ci >= half;
+        const int from = turned ? lane + (second ? -half / 8 : half / 8) : lane;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float other = __shfl_sync(0xffffffffu, f[e], from);
+          if (turned) {
+            const float2 cs = turn[t * half + (second ? ci - half : ci) + e];
+            f[e] = second ? f[e] * cs.x + other * cs.y : f[e] * cs.x - other * cs.y;
+          }
+        }
+      }
+      if (live && slot[t] >= 0) {
+        __nv_bfloat16* dst = is_q ? p.q_out + static_cast<int64_t>(t0 + t) * nq : is_k ? p.k_cache + static_cast<int64_t>(slot[t]) * nk
+                                                                                       : p.v_cache + static_cast<int64_t>(slot[t]) * nv;
+        stg_v4(dst + c, make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7])));
+      }
+    }
+  }
+}
+
+// Whole 16-byte pieces everywhere, and a head's lanes a power of two, so that heads never straddle warps; the kernels above take the rest.
+static bool prep_vec8_applies(const PrepArgs& p) {
+  const int lanes = p.d / 8;
+  auto ok = [](const void* x) { return x == nullptr || aligned16(x); };
+  return p.d % 8 == 0 && (lanes == 4 || lanes == 8 || lanes == 16 || lanes == 32) && p.dv % 8 == 0 && p.ldu % 8 == 0 && p.q_off % 8 == 0 && p.k_off % 8 == 0 &&
+         (p.v_off < 0 || p.v_off % 8 == 0) && p.rot_dims % 8 == 0 && (p.interleaved || p.rot_dims % 16 == 0) && p.rot_dims <= PREP_MAX_ROT &&
+         // few tokens with head norms: a warp per head has more of them in flight (64 tokens 2.8 / 3.5 us, 300 tokens 4.4 / 4.3)
+         (p.norm != 2 || p.n_tokens >= 2 * sm_count()) &&
+         ok(p.u) && ok(p.q_bias) && ok(p.k_bias) && ok(p.v_bias) && ok(p.q_norm_w) && ok(p.k_norm_w) && ok(p.q_out) && ok(p.k_cache) && ok(p.v_cache);
+}
+
+template <int LPH>
+static void go_prep_vec8(const PrepArgs& p, cudaStream_t st) {
+  const size_t turn = static_cast<size_t>(p.rot_dims / 2) * sizeof(float2);
+  if (p.n_tokens >= 8 * sm_count()) prep_vec8_kernel<2, LPH><<<(p.n_tokens + 1) / 2, ROW_THREADS, 2 * turn, st>>>(p);
+  else prep_vec8_kernel<1, LPH><<<p.n_tokens, ROW_THREADS, turn, st>>>(p);
+}
+static void launch_prep_vec8(const PrepArgs& p, cudaStream_t st) {
+  switch (p.d / 8) {
+    case 4: return go_prep_vec8<4>(p, st);
+    case 8: return go_prep_vec8<8>(p, st);
+    case 16: return go_prep_vec8<16>(p, st);
+    default: return go_prep_vec8<32>(p, st);
+  }
+}
+
 // ------------------------------------------------------------------ short causal convolution + activation
 // y[t, c] = act(bias[c] + sum_j w[c, j] * u(position(t) - taps + 1 + j)[c]) over the C columns of u from c_off on.  An
 // earlier position comes from this step's rows when it lies in the step's portion, from the sequence's carried state
@@ -852,7 +1036,13 @@ extern "C" int b2tts_attn_prep(const void* u, int64_t ldu, int q_off, int k_off,
   if (n_tokens == 0) return B2TTS_OK;
   B2_REQUIRE(u && positions && slot_mapping && q_out && (rot_dims == 0 || freq), B2TTS_EINVAL, "attn_prep: null pointer");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (dtype == B2TTS_DTYPE_BF16)
+  using B = __nv_bfloat16;
+  const PrepArgs p{static_cast<const B*>(u), ldu, q_off, k_off, v_off, q_bias, k_bias, v_bias, q_norm_w, k_norm_w, q_norm_w != nullptr ? 1 : 0,
+                   nullptr, freq, positions, rot_dims, interleaved, slot_mapping, static_cast<B*>(q_out), static_cast<B*>(k_cache),
+                   static_cast<B*>(v_cache), n_tokens, heads, kv_heads, v_heads, dim, vdim, eps};
+  if (dtype == B2TTS_DTYPE_BF16 && prep_vec8_applies(p))
+    launch_prep_vec8(p, st);
+  else if (dtype == B2TTS_DTYPE_BF16)
     attn_prep_kernel<__nv_bfloat16><<<n_tokens, ROW_THREADS, 0, st>>>(static_cast<const __nv_bfloat16*>(u), ldu, q_off, k_off, v_off,
         q_bias, k_bias, v_bias, q_norm_w, k_norm_w, freq, rot_dims, positions, slot_mapping, static_cast<__nv_bfloat16*>(q_out),
         static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache), heads, kv_heads, v_heads, dim, vdim, eps, interleaved);
@@ -875,9 +1065,14 @@ extern "C" int b2tts_attn_head_prep(const void* u, int64_t ldu, int q_off, int k
   B2_REQUIRE(B2_ROW_DTYPE_OK(dtype), B2TTS_EINVAL, "attn_head_prep: dtype %d", dtype);
   if (n_tokens == 0) return B2TTS_OK;
   B2_REQUIRE(u && slot_mapping && q_out && k_cache && v_cache && (rot_dims == 0 || rot), B2TTS_EINVAL, "attn_head_prep: null pointer");
+  using B = __nv_bfloat16;
+  const PrepArgs v{static_cast<const B*>(u), ldu, q_off, k_off, v_off, q_bias, k_bias, v_bias, q_norm_w, k_norm_w, q_norm_w != nullptr ? 2 : 0,
+                   rot, nullptr, nullptr, rot_dims, interleaved, slot_mapping, static_cast<B*>(q_out), static_cast<B*>(k_cache),
+                   static_cast<B*>(v_cache), n_tokens, heads, kv_heads, kv_heads, dim, vdim, eps};
   const HeadPrepArgs p{u, ldu, q_off, k_off, v_off, q_bias, k_bias, v_bias, q_norm_w, k_norm_w, rot, rot_dims, interleaved, slot_mapping,
                        q_out, k_cache, v_cache, n_tokens, heads, kv_heads, dim, vdim, eps};
-  if (dtype == B2TTS_DTYPE_BF16) launch_head_prep<__nv_bfloat16>(p, static_cast<cudaStream_t>(stream));
+  if (dtype == B2TTS_DTYPE_BF16 && prep_vec8_applies(v)) launch_prep_vec8(v, static_cast<cudaStream_t>(stream));
+  else if (dtype == B2TTS_DTYPE_BF16) launch_head_prep<__nv_bfloat16>(p, static_cast<cudaStream_t>(stream));
   else launch_head_prep<float>(p, static_cast<cudaStream_t>(stream));
   B2_CHECK_LAUNCH("attn_head_prep");
   return B2TTS_OK;
