@@ -473,6 +473,13 @@ B2TTS_API int b2tts_window_sigmoid_attn(const void* q, const void* k_cache, cons
                                         const int32_t* block_tables, int bt_stride, const float* r1, const float* r2,
                                         const float* pb, int n_seqs, int max_new, int heads, int kv_heads, int dim, int vdim,
                                         int page, int window, float scale, int dtype, void* stream);
+/* The same, told how many rows q has, how many rows (pages times page) both caches have, and how many keys the longest sequence has (0: not
+ * known); see b2tts_sink_attn_rows. */
+B2TTS_API int b2tts_window_sigmoid_attn_rows(const void* q, const void* k_cache, const void* v_cache, void* out,
+                                        const int32_t* seq_start, const int32_t* seq_pos0, const int32_t* seq_len,
+                                        const int32_t* block_tables, int bt_stride, const float* r1, const float* r2,
+                                        const float* pb, int n_seqs, int max_new, int heads, int kv_heads, int dim, int vdim,
+                                        int page, int window, float scale, int dtype, int n_tokens, int64_t cache_rows, int max_keys, void* stream);
 /* Top-k router, in float.  mode 0: scores = sigmoid(h router^T), top_w = score / (sum of the chosen + 1e-20) * scale.
  * mode 1: scores = h router^T + bias (bias may be null), top_w = softmax over the chosen scores only, * scale.
  * mode 2: scores = softmax(h router^T) over all experts, the choice is made on score + bias, top_w = the chosen scores

@@ -93,6 +93,7 @@ def _load():
         "b2tts_retention": (I, [P, L, P, L, P, L, P, I, P, F, P, P, L, P, P, P, P, P, P, P, I, I, I, I, I, I, F, I, I, P]),
         "b2tts_retention_scratch": (I, [I, I, I, I, I, I, I]),
         "b2tts_window_sigmoid_attn": (I, [P, P, P, P, P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, I, P]),
+        "b2tts_window_sigmoid_attn_rows": (I, [P, P, P, P, P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, I, I, L, I, P]),
         "b2tts_moe_route": (I, [P, P, P, P, P, P, I, I, I, I, F, P, I, I, I, I, P]),
         "b2tts_grouped_gemm_gated": (I, [P, L, P, P, L, P, P, I, I, I, I, I, F, F, P]),
         "b2tts_grouped_gemm_silu": (I, [P, L, P, P, L, P, P, I, I, I, I, I, P]),
@@ -839,11 +840,12 @@ def conv_headnorm_kvwrite(u, conv_w, state, lay, q_norm_w, k_norm_w, q_out, k_ca
 def window_sigmoid_attn(q, k_cache, v_cache, out, lay, r1, r2, pb, heads, kv_heads, dim, vdim, page, window, scale):
     dt = _act(q, "q")
     assert k_cache.dtype == q.dtype and v_cache.dtype == q.dtype and out.dtype == q.dtype
-    _check(_load().b2tts_window_sigmoid_attn(
+    rows = min(k_cache.numel() // (kv_heads * dim), v_cache.numel() // (kv_heads * vdim)) if k_cache.is_contiguous() and v_cache.is_contiguous() else 0
+    _check(_load().b2tts_window_sigmoid_attn_rows(
         q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), lay.seq_start.data_ptr(),
         lay.seq_pos0.data_ptr(), lay.seq_len.data_ptr(), lay.block_tables.data_ptr(), lay.block_tables.stride(0),
         r1.data_ptr(), r2.data_ptr(), pb.data_ptr(), lay.n_seqs, lay.max_new, heads, kv_heads, dim, vdim, page, window,
-        scale, dt, _stream()), "window_sigmoid_attn")
+        scale, dt, lay.n_tokens, rows, getattr(lay, "max_keys", 0), _stream()), "window_sigmoid_attn")
 
 
 ROUTE_SIGMOID, ROUTE_SOFTMAX_CHOSEN, ROUTE_SOFTMAX_ALL = 0, 1, 2

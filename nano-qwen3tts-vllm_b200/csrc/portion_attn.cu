@@ -1,6 +1,7 @@
-// portion_attn.cu - softmax attention of prompt portions (more than one new token of a sequence) on the 5th-generation tensor cores:
+// portion_attn.cu - attention of prompt portions (more than one new token of a sequence) on the 5th-generation tensor cores:
 // keys and values through block tables or in rows of their own, sliding-window, chunk or causal masks with kept first keys, sinks, score
-// caps, gates.  bf16 operands; scores, weights, sums and the outputs' accumulators are float.
+// caps, gates; or sigmoid weights with a logarithmic distance bias in a window.  bf16 operands; scores, weights, sums and the outputs'
+// accumulators are float.
 //
 // A persistent CTA per SM takes items of one or two row tiles.  A row tile is 128 query rows: 128 / HPC tokens times HPC heads that share
 // a key head; the two tiles of an item are neighbouring tokens and share the key tiles (128 keys) that pass through one ring of
@@ -23,7 +24,8 @@
 // (one thread a row with 40 spilled registers: 143 us for the case below; one barrier per slot of the ring instead of per tile: 20 us more).
 // 4 prompts of 2048 tokens, 16 heads over 8 of 128, window 1024 + 4 kept, element gates: 118 us (mma.sync, 64 queries per CTA: 547 us; 31 at
 // the tensor core's rate); causal with a score cap, 4448 tokens: 141 us (579 us); latent
-// heads of 192 over expanded keys, 4 x 2048 causal: 152 us.
+// heads of 192 over expanded keys, 4 x 2048 causal: 152 us.  Sigmoid weights (two special-function results and a table's number a pair), window
+// 1024, 4138 tokens: 79 us (143 us).
 //
 // Every copy is bounded: maps have the true extents of their tensors, so a row that a block table should not name reads zeros.  Every
 // commit of the last products is waited for before the CTA leaves.
@@ -37,7 +39,7 @@ namespace b2 {
 namespace row {
 
 constexpr int PO_N = 128, PO_SLOT = 128 * 128;         // keys per tile; bytes of a slot: 128 rows of 64 bf16 columns
-constexpr int PO_SOFT = 16, PO_THREADS = 640, PO_ITEMS = 64;           // softmax warps; items a CTA takes at most
+constexpr int PO_SOFT = 16, PO_THREADS = 640, PO_ITEMS = 48;           // softmax warps; items a CTA takes at most
 constexpr int PO_MMA = 16, PO_LOADER = 17, PO_CLEANER = 18, PO_LISTER = 19;
 __device__ int g_portion_timeouts = 0;                 // see waits.cuh
 
@@ -119,6 +121,12 @@ __device__ __forceinline__ float po_ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// 1 / (1 + 2^x): about 2 ulp; 2^big = inf and 1 / inf = 0
+__device__ __forceinline__ float po_sigmoid(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(1.0f + po_ex2(x)));
+  return y;
+}
 __device__ __forceinline__ int po_mask_lo(int i, int kind, int mask) {
   if (mask <= 0) return 0;
   return kind == 0 ? max(0, i - mask + 1) : (i / mask) * mask;
@@ -130,7 +138,7 @@ __device__ __forceinline__ uint32_t po_below(int n) { return n <= 0 ? 0u : n >= 
 // have the 32 columns where their scores were: 16 of rounded weights, 16 of remainders.
 __device__ __forceinline__ constexpr int po_weights_at(int s) { return (s >> 1 & 3) * 32 + (s >> 3) * 16 + (s & 1) * 8; }
 
-struct PortionPlan { int hpc, hpc_shift, tiles, box_rows, page_shift, gate_vec; int* timeouts; };    // set by the launch
+struct PortionPlan { int hpc, hpc_shift, tiles, box_rows, page_shift, gate_vec, tab_row; int* timeouts; };    // set by the launch
 struct PortionMaps { CUtensorMap q, k, k2, v; };
 struct PortionEntry { int tile, b, hg, len, start, pos0; };
 
@@ -173,16 +181,17 @@ struct PortionSpan {
   __device__ __forceinline__ bool has(int j) const { return j < front || (j >= first && j <= last); }
 };
 
-template <int NS> constexpr int po_slots() { return NS == 1 ? 12 : NS == 2 ? 10 : 8; }      // of the ring
-constexpr int PO_DEEP = 8, PO_BAR_BYTES = 512, PO_TAIL = PO_BAR_BYTES + PO_ITEMS * 24;
-template <int NS> constexpr int po_smem() { return 1024 + (2 * NS + po_slots<NS>()) * PO_SLOT + PO_TAIL; }
-static_assert(po_smem<1>() <= 232448 && po_smem<2>() <= 232448 && po_smem<3>() <= 232448, "shared memory of a CTA");
+// slots of the ring; sigmoid weights need room for their tables beside it
+template <int NS, bool SIG> constexpr int po_slots() { return SIG ? 8 : NS == 1 ? 12 : NS == 2 ? 10 : 8; }
+constexpr int PO_DEEP = 8, PO_BAR_BYTES = 512, PO_TAIL = PO_BAR_BYTES + PO_ITEMS * 24, PO_SMEM = 232448;
+template <int NS, bool SIG> constexpr int po_smem() { return 1024 + (2 * NS + po_slots<NS, SIG>()) * PO_SLOT + PO_TAIL; }
+static_assert(po_smem<1, false>() <= PO_SMEM && po_smem<2, false>() <= PO_SMEM && po_smem<3, false>() <= PO_SMEM, "shared memory of a CTA");
 
-// NS: 64-column slices of q and k; NV: of v
-template <int NS, int NV>
+// NS: 64-column slices of q and k; NV: of v; SIG: sigmoid weights
+template <int NS, int NV, bool SIG>
 __global__ void __launch_bounds__(PO_THREADS, 1)
 portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_constant__ PortionMaps maps) {
-  constexpr int SLOTS = po_slots<NS>(), PER_TILE = NS + NV;
+  constexpr int SLOTS = po_slots<NS, SIG>(), PER_TILE = NS + NV;
   static_assert(2 * NS + NV <= SLOTS, "a tile's values beside two tiles of keys");
   static_assert(SLOTS / PER_TILE + 1 < PO_DEEP, "tiles in the ring at once");
   extern __shared__ uint8_t po_smem_dyn[];
@@ -194,8 +203,8 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
   uint64_t* k_full = reinterpret_cast<uint64_t*>(ring + SLOTS * PO_SLOT);
   uint64_t *v_full = k_full + PO_DEEP, *clean = v_full + PO_DEEP, *empty = clean + PO_DEEP;
   uint64_t *q_full = empty + PO_DEEP, *q_empty = q_full + 2, *s_full = q_empty + 2, *p_full = s_full + 2;
-  uint64_t* o_full = p_full + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
+  uint64_t *o_full = p_full + 2, *t_full = o_full + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(t_full + 2);
   int* n_items_s = reinterpret_cast<int*>(tmem_slot + 1);
   PortionEntry* list = reinterpret_cast<PortionEntry*>(reinterpret_cast<uint8_t*>(k_full) + PO_BAR_BYTES);
 
@@ -229,6 +238,7 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
     }
     for (int g = 0; g < 2; ++g) {
       mbar_init(q_full + g, 1); mbar_init(q_empty + g, 1); mbar_init(s_full + g, 1); mbar_init(p_full + g, PO_SOFT / 2); mbar_init(o_full + g, 1);
+      mbar_init(t_full + g, PO_SOFT / 2);
     }
     mbar_fence_init();
   }
@@ -349,8 +359,8 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
           if (j > 0) ok = mbar_wait_limit(clean + before, ((t - 1) / PO_DEEP) & 1);
           if (ok && j < m.n_tiles) ok = mbar_wait_limit(k_full + at, (t / PO_DEEP) & 1);
           const uint32_t v_lo = ring_v + v_slot * SLOT_LO;
-          // values in the ring's last and first slot (only a ring of 8 slots with 5 a tile comes to that): 64 columns at a time
-          const bool apart = NS == 3 && NV == 2 && v_slot == SLOTS - 1;
+          // values in the ring's last and first slot (rings whose length no whole tiles make up come to that): 64 columns at a time
+          const bool apart = NV == 2 && SLOTS % PER_TILE != 0 && (NS + NV) % 2 != 0 && v_slot == SLOTS - 1;
           uint32_t k_lo[NS];
 #pragma unroll
           for (int sl = 0; sl < NS; ++sl) k_lo[sl] = ring_k + (slot + sl < SLOTS ? slot + sl : slot + sl - SLOTS) * SLOT_LO;
@@ -426,7 +436,11 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
     const bool early = a.softcap > 0.f || !(scale2 > 0.f);
     const float f = early ? 1.f : scale2;
     const bool gated = a.gate != nullptr && a.gate_el;
-    int s_uses = 0, o_uses = 0;
+    // SIG: log2(e) (r1 ln(1 + r2 x) - pb) of the distances x, a table per head, for each half of the lanes its own copy (rows of p.tab_row floats, which
+    // puts the 32 numbers that a warp reads at once into different banks)
+    float* tab = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(k_full) + PO_TAIL) + tg * 2 * p.hpc * p.tab_row;
+    const float* my_tab = tab + (half * p.hpc + (r & (p.hpc - 1))) * p.tab_row;
+    int s_uses = 0, o_uses = 0, t_uses = 0;
     for (int x = 0; ok && x < n_items; ++x) {
       // What an item needs in its masked tiles and in the end is formed there again: the loop over whole tiles has no registers for it
       float m = -1e30f, l = 0.f;
@@ -436,7 +450,7 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
         const PortionItem it(a, p, list[x]);
         if (!it.has(tg)) continue;
         span = PortionSpan(a, it, tg);
-        if (a.sink != nullptr) { m = a.sink[it.h0 + (r & (p.hpc - 1))] * LOG2E; l = half == 0 ? 1.f : 0.f; }
+        if (!SIG && a.sink != nullptr) { m = a.sink[it.h0 + (r & (p.hpc - 1))] * LOG2E; l = half == 0 ? 1.f : 0.f; }
         const int t_first = it.t0 + tg * it.per, t_last = min(it.end, t_first + it.per) - 1;
         const int lo = po_mask_lo(it.pos0 + min(t_first + ((r0 + 15) >> p.hpc_shift), t_last), a.mask_kind, a.mask);    // the highest of its rows
         whole0 = (max(lo - it.jl, 0) + it.pre_r + PO_N - 1) / PO_N;
@@ -444,6 +458,19 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
         if (gated)                                     // read in the end, far from any cache by then
           asm volatile("prefetch.global.L2 [%0];" :: "l"(a.gate + static_cast<int64_t>(it.start + min(t_first + (r >> p.hpc_shift), t_last)) * a.ldg +
                                                          static_cast<int64_t>(it.h0 + (r & (p.hpc - 1))) * a.dv + half * OC));
+      }
+      if constexpr (SIG) {                             // nobody reads the last item's table any more: its last weights are all there
+        const int h0 = list[x].hg << p.hpc_shift;
+        for (int i = threadIdx.x & 255; i < p.hpc * a.mask; i += 256) {
+          const int h = i / a.mask, dist = i - h * a.mask;
+          const float y = LOG2E * (a.r1[h0 + h] * log1pf(a.r2[h0 + h] * static_cast<float>(dist)) - a.pb[h0 + h]);
+          tab[h * p.tab_row + dist] = y;
+          tab[(p.hpc + h) * p.tab_row + dist] = y;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(t_full + tg);
+        if (!(ok = mbar_wait_limit(t_full + tg, t_uses & 1))) break;
+        ++t_uses;
       }
       bool first = true;
       for (int j = 0; ok && j <= span.last; ++j) {
@@ -491,6 +518,12 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
                 }
               }
             }
+            if (SIG && masked) {                       // the exponent's argument, from the other side, while the distance is at hand
+              const int dist = pos - j0 - c;
+#pragma unroll
+              for (int e = 0; e < 32; ++e)
+                v[e] = __float_as_uint(fmaf(__uint_as_float(v[e]), f, -my_tab[min(max(dist - e, 0), a.mask - 1)]));
+            }
             if (masked) {
               const uint32_t see = (po_below(fr_vis) & po_below(fr_end)) | (~po_below(fr_end) & po_below(to + 1) & (~po_below(from) | po_below(keep)));
 #pragma unroll
@@ -502,43 +535,45 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
           }
           po_st_wait();
         }
-        // two passes over the scores, which stay in TMEM meanwhile: a thread has no registers for all of them beside the weights' parts
-        float mx;
-        {
-          uint32_t v[HK];
-          po_ld32<HK>(tm_s, v);
-          po_ld32<HK>(tm_s + 32, v + 32);
-          tmem_ld_wait();
-          float x0 = -INFINITY, x1 = -INFINITY, x2 = -INFINITY, x3 = -INFINITY;
+        if constexpr (!SIG) {
+          // two passes over the scores, which stay in TMEM meanwhile: a thread has no registers for all of them beside the weights' parts
+          float mx;
+          {
+            uint32_t v[HK];
+            po_ld32<HK>(tm_s, v);
+            po_ld32<HK>(tm_s + 32, v + 32);
+            tmem_ld_wait();
+            float x0 = -INFINITY, x1 = -INFINITY, x2 = -INFINITY, x3 = -INFINITY;
 #pragma unroll
-          for (int c = 0; c < HK; c += 8) {
-            x0 = fmaxf(x0, fmaxf(__uint_as_float(v[c]), __uint_as_float(v[c + 1])));
-            x1 = fmaxf(x1, fmaxf(__uint_as_float(v[c + 2]), __uint_as_float(v[c + 3])));
-            x2 = fmaxf(x2, fmaxf(__uint_as_float(v[c + 4]), __uint_as_float(v[c + 5])));
-            x3 = fmaxf(x3, fmaxf(__uint_as_float(v[c + 6]), __uint_as_float(v[c + 7])));
+            for (int c = 0; c < HK; c += 8) {
+              x0 = fmaxf(x0, fmaxf(__uint_as_float(v[c]), __uint_as_float(v[c + 1])));
+              x1 = fmaxf(x1, fmaxf(__uint_as_float(v[c + 2]), __uint_as_float(v[c + 3])));
+              x2 = fmaxf(x2, fmaxf(__uint_as_float(v[c + 4]), __uint_as_float(v[c + 5])));
+              x3 = fmaxf(x3, fmaxf(__uint_as_float(v[c + 6]), __uint_as_float(v[c + 7])));
+            }
+            mx = fmaxf(fmaxf(x0, x1), fmaxf(x2, x3));
           }
-          mx = fmaxf(fmaxf(x0, x1), fmaxf(x2, x3));
-        }
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16)) * f;
-        // ---- the running maximum moves in steps of more than 2^8.  These scores were issued behind the last weight products, so O is at rest
-        const bool grow = mx > m + (first ? 0.f : 8.f);
-        if (__any_sync(0xffffffffu, grow)) {
-          const float n = grow ? mx : m, alpha = po_ex2(m - n);
-          m = n;
-          l *= alpha;
-          if (!first) {
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16)) * f;
+          // ---- the running maximum moves in steps of more than 2^8.  These scores were issued behind the last weight products, so O is at rest
+          const bool grow = mx > m + (first ? 0.f : 8.f);
+          if (__any_sync(0xffffffffu, grow)) {
+            const float n = grow ? mx : m, alpha = po_ex2(m - n);
+            m = n;
+            l *= alpha;
+            if (!first) {
 #pragma unroll 1
-            for (int c = 0; c < OC; c += 32) {
-              uint32_t o[32];
-              po_ld32<OC>(tm_o + c, o);
-              tmem_ld_wait();
+              for (int c = 0; c < OC; c += 32) {
+                uint32_t o[32];
+                po_ld32<OC>(tm_o + c, o);
+                tmem_ld_wait();
 #pragma unroll
-              for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
-              po_st32<OC>(tm_o + c, o);
+                for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
+                po_st32<OC>(tm_o + c, o);
+              }
             }
           }
+          first = false;
         }
-        first = false;
         // ---- weights, their sum, and their bf16 parts, in place of the scores
         const uint64_t f2 = po_pair(f, f), m2 = po_pair(-m, -m);
         uint64_t sa = 0, sb = 0;
@@ -547,16 +582,36 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
           uint32_t v[32], hi[16], rest[16];
           po_ld32<HK>(tm_s + part, v);
           tmem_ld_wait();
+          if constexpr (SIG) {
+            if (masked) {
+#pragma unroll
+              for (int c = 0; c < 32; ++c) v[c] = __float_as_uint(-__uint_as_float(v[c]));
+            } else {
+              const PortionEntry& e = list[x];
+              const int tk = (e.tile * p.tiles + tg) * (128 >> p.hpc_shift) + (r >> p.hpc_shift), pos = e.pos0 + min(tk, e.len - 1);
+              const PortionItem it(a, p, e);
+              const float* at = my_tab + (pos - (j * PO_N + half * HK + it.jl) - part);
+#pragma unroll
+              for (int c = 0; c < 32; ++c) v[c] = __float_as_uint(fmaf(__uint_as_float(v[c]), -f, at[-c]));
+            }
+          }
 #pragma unroll
           for (int c = 0; c < 32; c += 4) {
             const uint32_t* vv = v + c;
             float w0, w1, w2, w3, r0, r1, r2, r3;
-            po_split(po_fma2(po_pair(__uint_as_float(vv[0]), __uint_as_float(vv[1])), f2, m2), w0, w1);
-            po_split(po_fma2(po_pair(__uint_as_float(vv[2]), __uint_as_float(vv[3])), f2, m2), w2, w3);
-            w0 = po_ex2(w0); w1 = po_ex2(w1); w2 = po_ex2(w2); w3 = po_ex2(w3);
+            if constexpr (SIG) {
+              w0 = po_sigmoid(__uint_as_float(vv[0])); w1 = po_sigmoid(__uint_as_float(vv[1]));
+              w2 = po_sigmoid(__uint_as_float(vv[2])); w3 = po_sigmoid(__uint_as_float(vv[3]));
+            } else {
+              po_split(po_fma2(po_pair(__uint_as_float(vv[0]), __uint_as_float(vv[1])), f2, m2), w0, w1);
+              po_split(po_fma2(po_pair(__uint_as_float(vv[2]), __uint_as_float(vv[3])), f2, m2), w2, w3);
+              w0 = po_ex2(w0); w1 = po_ex2(w1); w2 = po_ex2(w2); w3 = po_ex2(w3);
+            }
             const uint64_t wa = po_pair(w0, w1), wb = po_pair(w2, w3);
-            sa = po_add2(sa, wa);
-            sb = po_add2(sb, wb);
+            if constexpr (!SIG) {
+              sa = po_add2(sa, wa);
+              sb = po_add2(sb, wb);
+            }
             const uint32_t p0 = pack_bf16(w0, w1), p1 = pack_bf16(w2, w3), n0 = p0 ^ 0x80008000u, n1 = p1 ^ 0x80008000u;
             po_split(po_add2(wa, po_pair(bf16lo(n0), bf16hi(n0))), r0, r1);
             po_split(po_add2(wb, po_pair(bf16lo(n1), bf16hi(n1))), r2, r3);
@@ -591,7 +646,7 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
       };
       if (gated) gates(0);
       l += __shfl_xor_sync(0xffffffffu, l, 16);
-      float inv = 1.0f / l;
+      float inv = SIG ? 1.f : 1.0f / l;
       if (a.gate != nullptr && !a.gate_el) inv *= sigmoid_f(__bfloat162float(a.gate[row * a.ldg + h]));
       if (!(ok = mbar_wait_limit(o_full + tg, o_uses & 1))) break;
       ++o_uses;
@@ -641,6 +696,18 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
   }
 }
 
+// floats of a row of the distance tables: the rows' tokens, heads and halves of a warp fall into different banks
+static int po_tab_row(int window, int hpc) { return (window + 31) / 32 * 32 + 16 / hpc; }
+// heads of a key head that share a row tile: a power of two up to 8; for sigmoid weights as many as have room for their tables (0: none)
+static int po_heads(const PortionArgs& a) {
+  int hpc = 1;
+  while (hpc < 8 && (a.H / a.G) % (2 * hpc) == 0) hpc *= 2;
+  if (a.r1 == nullptr) return hpc;
+  const int room = PO_SMEM - (a.d == 64 ? po_smem<1, true>() : po_smem<2, true>());
+  while (hpc > 0 && static_cast<int64_t>(4) * hpc * po_tab_row(a.mask, hpc) * 4 > room) hpc /= 2;
+  return hpc;
+}
+
 // Whole slices of 64 columns (a box is never wider than a row), rows that copies can name and pages in whole boxes of 16 rows.
 bool portion_attn_applies(const PortionArgs& a) {
   const bool rows8 = a.q_tok % 8 == 0 && a.q_head % 8 == 0 && a.k_row % 8 == 0 && a.k2_row % 8 == 0 && a.v_row % 8 == 0;
@@ -648,15 +715,17 @@ bool portion_attn_applies(const PortionArgs& a) {
          aligned16(a.k) && (a.k2 == nullptr || aligned16(a.k2)) && aligned16(a.v) && aligned16(a.out) && a.n_rows > 0 &&
          a.n_rows < (1ll << 31) && (a.block_tables == nullptr || a.page % 16 == 0) && a.k_row >= static_cast<int64_t>(a.G) * a.d1 &&
          a.v_row >= static_cast<int64_t>(a.Gv) * a.dv &&
+         (a.r1 == nullptr || (a.d == a.dv && a.d <= 128 && a.mask > 0 && a.mask_kind == 0 && a.keep_first == 0 && a.softcap == 0.f && po_heads(a) > 0)) &&
          (a.gate == nullptr || !a.gate_el || (reinterpret_cast<uintptr_t>(a.gate) % 4 == 0 && a.ldg % 2 == 0));
 }
 
-template <int NS, int NV>
+template <int NS, int NV, bool SIG>
 static int go_portion(const char* what, const PortionArgs& a, const PortionPlan& p, const PortionMaps& maps, int grid, cudaStream_t st) {
-  auto kern = portion_attn_kernel<NS, NV>;
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, po_smem<NS>());
+  auto kern = portion_attn_kernel<NS, NV, SIG>;
+  const int smem = po_smem<NS, SIG>() + (SIG ? 4 * p.hpc * p.tab_row * 4 : 0);
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return cuda_fail(e, what);
-  kern<<<grid, PO_THREADS, po_smem<NS>(), st>>>(a, p, maps);
+  kern<<<grid, PO_THREADS, smem, st>>>(a, p, maps);
   B2_CHECK_LAUNCH(what);
   return B2TTS_OK;
 }
@@ -667,8 +736,9 @@ int launch_portion_attn(const char* what, const PortionArgs& a, cudaStream_t st)
   PortionPlan p{};
   p.timeouts = wait_word(WAITS_PORTIONS);
   B2_REQUIRE(p.timeouts != nullptr, B2TTS_ECUDA, "%s: no host memory for the kernel's status", what);
-  p.hpc = 1;                                           // heads of a key head that share a row tile: a power of two up to 8
-  while (p.hpc < 8 && (a.H / a.G) % (2 * p.hpc) == 0) { p.hpc *= 2; ++p.hpc_shift; }
+  p.hpc = po_heads(a);
+  while (1 << p.hpc_shift < p.hpc) ++p.hpc_shift;
+  if (a.r1 != nullptr) p.tab_row = po_tab_row(a.mask, p.hpc);
   p.page_shift = -1;
   for (int x = 0; x < 30; ++x)
     if (a.page == 1 << x) p.page_shift = x;
@@ -702,7 +772,8 @@ int launch_portion_attn(const char* what, const PortionArgs& a, cudaStream_t st)
   }
   if (rc != B2TTS_OK) return rc;
   const int ns = a.d / 64;
-#define PO_GO(NS, NV) return go_portion<NS, NV>(what, a, p, maps, grid, st)
+  if (a.r1 != nullptr) return ns == 1 ? go_portion<1, 1, true>(what, a, p, maps, grid, st) : go_portion<2, 2, true>(what, a, p, maps, grid, st);
+#define PO_GO(NS, NV) return go_portion<NS, NV, false>(what, a, p, maps, grid, st)
   if (a.dv == 64) {
     if (ns == 1) PO_GO(1, 1);
     if (ns == 2) PO_GO(2, 1);

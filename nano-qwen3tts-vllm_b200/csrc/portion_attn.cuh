@@ -23,6 +23,8 @@ struct PortionArgs {
   int H, G, Gv, d, dv;
   int mask_kind, mask, keep_first;                    // as sink_attn
   float softcap, scale;
+  // not null: no softmax, the weight of distance x = position - key is 1 / (1 + exp(r1[h] ln(1 + r2[h] x) - pb[h] - scale score)); a window, nothing kept
+  const float *r1, *r2, *pb;
   int n_seqs, max_new;
 };
 

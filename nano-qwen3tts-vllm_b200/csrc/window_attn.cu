@@ -11,7 +11,7 @@
 // written to the cache by the preceding kernel, so a portion in the middle of a prompt and a decoded token look the same.
 #include <math.h>
 
-#include "common.cuh"
+#include "portion_attn.cuh"
 
 namespace b2 {
 
@@ -777,6 +777,16 @@ extern "C" int b2tts_window_sigmoid_attn(const void* q, const void* k_cache, con
                                          const int32_t* block_tables, int bt_stride, const float* r1, const float* r2,
                                          const float* pb, int n_seqs, int max_new, int heads, int kv_heads, int dim, int vdim,
                                          int page, int window, float scale, int dtype, void* stream) {
+  return b2tts_window_sigmoid_attn_rows(q, k_cache, v_cache, out, seq_start, seq_pos0, seq_len, block_tables, bt_stride, r1, r2, pb, n_seqs, max_new, heads,
+                                        kv_heads, dim, vdim, page, window, scale, dtype, 0, 0, 0, stream);
+}
+
+extern "C" int b2tts_window_sigmoid_attn_rows(const void* q, const void* k_cache, const void* v_cache, void* out,
+                                              const int32_t* seq_start, const int32_t* seq_pos0, const int32_t* seq_len,
+                                              const int32_t* block_tables, int bt_stride, const float* r1, const float* r2,
+                                              const float* pb, int n_seqs, int max_new, int heads, int kv_heads, int dim, int vdim,
+                                              int page, int window, float scale, int dtype, int n_tokens, int64_t cache_rows,
+                                              int max_keys, void* stream) {
   using namespace b2;
   B2_REQUIRE(n_seqs >= 0 && max_new >= 0 && heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && dim > 0 && vdim > 0 &&
              page > 0 && window > 0 && bt_stride > 0, B2TTS_EINVAL, "window_sigmoid_attn: bad sizes");
@@ -826,6 +836,23 @@ extern "C" int b2tts_window_sigmoid_attn(const void* q, const void* k_cache, con
   }
   // prompt portions in bf16 with a supported head size: the tensor-core kernel
   if (stream_ok && dtype == B2TTS_DTYPE_BF16 && dim == vdim && (dim == 32 || dim == 64 || dim == 96 || dim == 128) && window <= 8192) {
+    row::PortionArgs p{};
+    using B = __nv_bfloat16;
+    p.q = static_cast<const B*>(q); p.q_tok = static_cast<int64_t>(heads) * dim; p.q_head = dim; p.n_tokens = n_tokens;
+    p.k = static_cast<const B*>(k_cache); p.k_row = static_cast<int64_t>(kv_heads) * dim; p.d1 = dim;
+    p.v = static_cast<const B*>(v_cache); p.v_row = static_cast<int64_t>(kv_heads) * vdim;
+    p.n_rows = cache_rows;
+    p.block_tables = block_tables; p.bt_stride = bt_stride; p.page = page;
+    p.seq_start = seq_start; p.seq_pos0 = seq_pos0; p.seq_len = seq_len;
+    p.out = out;
+    p.H = heads; p.G = kv_heads; p.Gv = kv_heads; p.d = dim; p.dv = vdim;
+    p.mask = window; p.scale = scale; p.r1 = r1; p.r2 = r2; p.pb = pb;
+    p.n_seqs = n_seqs; p.max_new = max_new;
+    // The tcgen05 kernel (portion_attn.cu) where the longest sequence is not known to be short: its items start and end in 12 us, the kernel
+    // below in 6.  16 heads over 8 of 128, window 1024, below / tcgen05 in us: 64 new tokens 8.3 / 12.5, 400 20.7 / 21.9, 3 x 300 21.9 / 19.8,
+    // 700 41 / 30, 40 behind 1000 44 / 40, 4 x 100 behind 800 39 / 36, 2048 100 / 70; 2048 + 1333 + 700 + 57 143 / 79.
+    const bool few = max_keys > 0 && max_keys <= 420;
+    if (!few && row::portion_attn_applies(p)) return row::launch_portion_attn("window_sigmoid_attn (portions)", p, st);
     // One head and 32-key tiles per CTA, four CTAs per SM: independent CTAs overlap their MMA and weight phases better
     // than a wider CTA in which two heads share the K/V tiles (306 against 322 us at 4 x 2048 tokens, window 1024).
 #define WM_GO(DD) e = launch_window_mma<DD, 1, 32>(max_new, n_seqs, st, q, k_cache, v_cache, out, seq_start, seq_pos0, seq_len, \

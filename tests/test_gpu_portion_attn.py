@@ -122,3 +122,57 @@ def test_values_nobody_sees_may_be_infinite(nat):
 @pytest.mark.parametrize("keys", [2, 39, 40, 41, 64])
 def test_short_sequences_that_the_host_knows_of(nat, keys):
     _case(nat, [(keys - 2, 2), (0, min(keys, 33)), (0, 1)], H=8, G=4, d=128, dv=128, page=64, mask=30, keep=2, gate="element", known=True, seed=keys)
+
+
+@pytest.mark.parametrize("H,G", [(2, 2), (4, 2), (6, 2), (16, 1)])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("window", [1, 70, 128, 500, 1024])
+def test_sigmoid_weights(nat, H, G, d, window):
+    _sigmoid_case(nat, [(0, 63), (3, 64), (0, 65), (500, 130), (8, 2), (11, 1), (900, 300)], H, G, d, window, page=48 if d == 64 else 64)
+
+
+def test_sigmoid_weights_of_several_items_for_every_cta(nat):
+    _sigmoid_case(nat, [(0, 2000), (100, 1500)], 16, 8, 128, 300, page=256)
+
+
+def test_sigmoid_weights_with_a_negative_scale(nat):
+    _sigmoid_case(nat, [(0, 300)], 4, 2, 64, 90, page=16, scale=-0.2)
+
+
+@pytest.mark.parametrize("keys", [420, 421])
+def test_sigmoid_weights_of_sequences_that_the_host_knows_of(nat, keys):
+    _sigmoid_case(nat, [(keys - 40, 40), (0, 33)], 4, 2, 64, 90, page=16, known=True)
+
+
+def _sigmoid_case(nat, seqs, H, G, d, window, page, scale=None, known=False):
+    from tests.lm_util import Lay
+    g = torch.Generator().manual_seed(H * d + window)
+    need = [-(-(c + n) // page) for c, n in seqs]
+    perm = (torch.randperm(sum(need), generator=g) + 1).tolist()
+    tabs = [perm[sum(need[:i]):sum(need[:i + 1])] for i in range(len(need))]
+    lay = Lay([(c, n, t) for (c, n), t in zip(seqs, tabs)], page, max(need))
+    if known:
+        lay.max_keys = max(c + n for c, n in seqs)
+    r = lambda *s: torch.randn(s, generator=g, dtype=torch.float32)
+    kc, vc = (torch.full((sum(need) + 2, page, G * d), math.nan) for _ in range(2))
+    scale = scale if scale is not None else d ** -0.5
+    q, r1, r2, pb = r(lay.n_tokens, H * d).to(BF), r(H) * 0.3 + 0.5, r(H).abs(), r(H) - 1.0
+    ref, o = [], 0
+    for (c, n), t in zip(seqs, tabs):
+        k, v = r(c + n, G, d).to(BF), r(c + n, G, d).to(BF)
+        at = torch.arange(c + n)
+        slot = torch.tensor(t)[at // page] * page + at % page
+        kc.view(-1, G * d)[slot], vc.view(-1, G * d)[slot] = k.reshape(c + n, -1).float(), v.reshape(c + n, -1).float()
+        x = torch.arange(c, c + n)[:, None] - at[None]
+        bias = (r1.to(F64)[:, None, None] * torch.log1p(r2.to(F64)[:, None, None] * x.clamp_min(0)) - pb.to(F64)[:, None, None])
+        s = torch.einsum("ihd,jhd->hij", q[o:o + n].view(n, H, d).to(F64), k.to(F64).repeat_interleave(H // G, 1)) * scale - bias
+        w = torch.sigmoid(s) * ((x >= 0) & (x < window))
+        ref.append(torch.einsum("hij,jhd->ihd", w, v.to(F64).repeat_interleave(H // G, 1)).reshape(n, -1))
+        o += n
+    ref = torch.cat(ref)
+    out = torch.empty(lay.n_tokens, H * d, dtype=BF, device=DEV)
+    nat.window_sigmoid_attn(q.to(DEV), kc.to(BF).to(DEV), vc.to(BF).to(DEV), out, lay, r1.to(DEV), r2.to(DEV), pb.to(DEV), H, G, d, d, page, window, scale)
+    # weights carry 16 bits; the results round to 2^-9
+    err = (out.double().cpu() - ref).abs().max() / ref.abs().max()
+    assert err.item() < 4e-3, err.item()
+    assert nat.portion_attn_timeouts() == 0
