@@ -705,7 +705,8 @@ template <typename T> struct RowVec {
 
 // What bounds it is the rows' traffic once they are in flight early enough: every row of the run is asked for before the first is
 // used (the loads sat behind the previous token's activation before, one 16-byte load in flight a thread), and a thread's filters are
-// contiguous and come as 16-byte vectors (as scalars a warp's load touched 32 lines).  8192 tokens of 4352 channels: 129 -> 78 us.
+// contiguous and come as 16-byte vectors (as scalars a warp's load touched 32 lines).  8192 tokens of 4352 channels: 129 -> 78 us, with the
+// special-function forms of the activation 50.
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(128)
 short_conv_act_run_kernel(const T* __restrict__ u, int64_t ldu, const float* __restrict__ w, const float* __restrict__ bias,
@@ -753,7 +754,7 @@ short_conv_act_run_kernel(const T* __restrict__ u, int64_t ldu, const float* __r
       float a = bs[e];
 #pragma unroll
       for (int j = 0; j < TAPS; ++j) a += wt[e * TAPS + j] * win[j][e];
-      acc[e] = act == 1 ? silu_f(a) : a;
+      acc[e] = act == 1 ? silu_for<T>(a) : a;
     }
     V::store(out + static_cast<int64_t>(start + t0 + i) * ldo + c, acc);
 #pragma unroll
@@ -847,12 +848,13 @@ gated_group_norm_vec4_kernel(const float* __restrict__ y, const T* __restrict__ 
   };
   auto gated = [&](float4& v, float4& g) {                 // g comes in as the gate's argument
     if (gr == nullptr) g = make_float4(1.f, 1.f, 1.f, 1.f);
-    else if (act == 0) g = make_float4(sigmoid_f(g.x), sigmoid_f(g.y), sigmoid_f(g.z), sigmoid_f(g.w));
-    else g = make_float4(silu_f(g.x), silu_f(g.y), silu_f(g.z), silu_f(g.w));
+    else if (act == 0) g = make_float4(sigmoid_for<T>(g.x), sigmoid_for<T>(g.y), sigmoid_for<T>(g.z), sigmoid_for<T>(g.w));
+    else g = make_float4(silu_for<T>(g.x), silu_for<T>(g.y), silu_for<T>(g.z), silu_for<T>(g.w));
     if (gate_first) { v.x *= g.x; v.y *= g.y; v.z *= g.z; v.w *= g.w; }
   };
   // a group of up to GN_KEEP vectors per thread stays in registers between the sum of squares and the scaled write; all of them are
-  // asked for before the first gate is formed (8192 rows of 4096: 89 -> 71 us; behind each other's gates the loads came one at a time)
+  // asked for before the first gate is formed (8192 rows of 4096: 89 -> 71 us, with the
+  // special-function forms of the gates 53; behind each other's gates the loads came one at a time)
   constexpr int GN_KEEP = 4;
   const bool keep = gs <= 4 * GN_KEEP * static_cast<int>(blockDim.x);
   float4 kv[GN_KEEP], kg[GN_KEEP];
@@ -883,7 +885,7 @@ gated_group_norm_vec4_kernel(const float* __restrict__ y, const T* __restrict__ 
   const float inv = 1.0f / sqrtf(block_sum(ssq, red) / static_cast<float>(gs) + eps);
   T* o = out + r * cols + c0;
   auto emit = [&](int c, const float4& v, const float4& g) {
-    const int wc = (c0 + c) % w_len;                       // w_len is a multiple of four here
+    const int wc = w_len >= cols ? c0 + c : (c0 + c) % w_len;                              // w_len is a multiple of four here
     const float4 ww = w != nullptr ? *reinterpret_cast<const float4*>(w + wc) : make_float4(1.f, 1.f, 1.f, 1.f);
     float4 res = make_float4(v.x * inv * ww.x, v.y * inv * ww.y, v.z * inv * ww.z, v.w * inv * ww.w);
     if (!gate_first) { res.x *= g.x; res.y *= g.y; res.z *= g.z; res.w *= g.w; }
@@ -929,8 +931,8 @@ gated_group_norm_warp_kernel(const float* __restrict__ y, const T* __restrict__ 
         kv[it] = *reinterpret_cast<const float4*>(yr + c);
         if (gr != nullptr) {
           const float4 z = load4<T>(gr + c);
-          if (act == 0) kg[it] = make_float4(sigmoid_f(z.x), sigmoid_f(z.y), sigmoid_f(z.z), sigmoid_f(z.w));
-          else kg[it] = make_float4(silu_f(z.x), silu_f(z.y), silu_f(z.z), silu_f(z.w));
+          if (act == 0) kg[it] = make_float4(sigmoid_for<T>(z.x), sigmoid_for<T>(z.y), sigmoid_for<T>(z.z), sigmoid_for<T>(z.w));
+          else kg[it] = make_float4(silu_for<T>(z.x), silu_for<T>(z.y), silu_for<T>(z.z), silu_for<T>(z.w));
         }
         if (gate_first) { kv[it].x *= kg[it].x; kv[it].y *= kg[it].y; kv[it].z *= kg[it].z; kv[it].w *= kg[it].w; }
         ssq += kv[it].x * kv[it].x + kv[it].y * kv[it].y + kv[it].z * kv[it].z + kv[it].w * kv[it].w;

@@ -39,6 +39,19 @@ __device__ __forceinline__ float logsigmoid_f(float x) { return fminf(x, 0.f) - 
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
 __device__ __forceinline__ float silu_f(float x) { return x / (1.0f + expf(-x)); }
 
+// The same for results that are rounded to T: behind bf16's 2^-9 the special-function forms (within a few 2^-22 up to |x| = 20, 0 below -87)
+// take the place of the exponential's and the division's exact ones, which cost more than the rows they are formed for.
+template <typename T>
+__device__ __forceinline__ float sigmoid_for(float x) {
+  if constexpr (sizeof(T) == 2) return __fdividef(1.0f, 1.0f + __expf(-x));
+  else return sigmoid_f(x);
+}
+template <typename T>
+__device__ __forceinline__ float silu_for(float x) {
+  if constexpr (sizeof(T) == 2) return __fdividef(x, 1.0f + __expf(-x));
+  else return silu_f(x);
+}
+
 #define B2_ROW_DTYPE_OK(dt) ((dt) == B2TTS_DTYPE_BF16 || (dt) == B2TTS_DTYPE_F32)
 
 }  // namespace row
