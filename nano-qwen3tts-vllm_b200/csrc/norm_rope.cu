@@ -132,8 +132,10 @@ rmsnorm_narrow_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_stride, con
 
 // ------------------------------------------------------------------------------------------
 // Fused q/k head-norm + RoPE + KV write.  One CTA per token, 8 warps; a warp owns one head at a
-// time (lane l holds dims {2l, 2l+1, 64+2l, 64+2l+1} -> two fully coalesced 128-byte accesses),
-// computes cos/sin for its two frequencies once and walks heads warp, warp+8, ...
+// time (lane l holds dims {2l, 2l+1, 64+2l, 64+2l+1} -> two fully coalesced 128-byte accesses) and walks heads
+// warp, warp+8, ...  Cosines and sines are formed once a token, by 128 threads, while the rows of a warp's first four heads
+// and of the values are on their way.  Bound: HBM; 5627 tokens of 16 + 8 + 8 heads: 42 -> 37 us (14 at the copy rate; every warp
+// formed all of them for itself before, in front of its loads).
 struct QkRopeParams {
   const __nv_bfloat16 *q, *k, *v;
   int64_t q_stride, k_stride, v_stride;
@@ -159,75 +161,91 @@ qknorm_rope_kvwrite_kernel(const QkRopeParams p) {
   const int kv_dim = p.num_kv_heads * HD;
   const int slot = p.slot_mapping ? __ldg(p.slot_mapping + tok) : -1;
 
-  // cos/sin of this lane's columns {2l, 2l+1} (c1/s1) and {64+2l, 64+2l+1} (c2/s2): fp32 angle,
-  // fp32 cos/sin, bf16 result.  Columns f and 64+f share frequency f but - in the sectioned M-RoPE
-  // branch (rotary_embedding.py:73-80) - not necessarily the position row, so the two halves keep
-  // their own cos/sin; with 1-D positions (modality NULL) they are computed once.
+  const int total = p.num_heads + p.num_kv_heads;
+  constexpr int AHEAD = 4;                             // heads whose rows are asked for at once
+  uint32_t r1[AHEAD], r2[AHEAD];
+  auto fetch = [&](int h0) {
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) {
+      const int hh = h0 + 8 * i;
+      r1[i] = r2[i] = 0;
+      if (hh < total) {
+        const __nv_bfloat16* src = hh >= p.num_heads ? p.k + (int64_t)tok * p.k_stride + (hh - p.num_heads) * HD : p.q + (int64_t)tok * p.q_stride + hh * HD;
+        r1[i] = *reinterpret_cast<const uint32_t*>(src + 2 * lane);
+        r2[i] = *reinterpret_cast<const uint32_t*>(src + 64 + 2 * lane);
+      }
+    }
+  };
+  fetch(warp);
+  const bool put_v = slot >= 0 && p.v;                 // V goes to the cache untouched
+  uint4 v0 = make_uint4(0, 0, 0, 0);
+  if (put_v && threadIdx.x < (kv_dim >> 3)) v0 = ldg_nc_v4(p.v + (int64_t)tok * p.v_stride + 8 * threadIdx.x);
+  // cos/sin of columns f (turns[0]) and 64 + f (turns[1]): fp32 angle, fp32 cos/sin, bf16 result.  Both share frequency f but - in the
+  // sectioned M-RoPE branch (rotary_embedding.py:73-80) - not necessarily the position row.
+  __shared__ float2 turns[2][HD / 2];
+  if (threadIdx.x < HD) {
+    const int f = threadIdx.x & 63;
+    const int m = p.modality ? __ldg(p.modality + threadIdx.x) : 0;
+    const float ang = (float)__ldg(p.positions + (int64_t)m * p.pos_row_stride + tok) * __ldg(p.inv_freq + f);
+    turns[threadIdx.x >> 6][f] = make_float2(rbf(cosf(ang) * p.attention_scaling), rbf(sinf(ang) * p.attention_scaling));
+  }
+  __syncthreads();
   float c1[2], s1[2], c2[2], s2[2];
 #pragma unroll
   for (int e = 0; e < 2; ++e) {
-    const int fi = 2 * lane + e;
-    const float f = __ldg(p.inv_freq + fi);
-    const int m1 = p.modality ? __ldg(p.modality + fi) : 0;
-    const float a1 = (float)__ldg(p.positions + (int64_t)m1 * p.pos_row_stride + tok) * f;
-    c1[e] = rbf(cosf(a1) * p.attention_scaling);
-    s1[e] = rbf(sinf(a1) * p.attention_scaling);
-    const int m2 = p.modality ? __ldg(p.modality + HD / 2 + fi) : 0;
-    if (m2 != m1) {
-      const float a2 = (float)__ldg(p.positions + (int64_t)m2 * p.pos_row_stride + tok) * f;
-      c2[e] = rbf(cosf(a2) * p.attention_scaling);
-      s2[e] = rbf(sinf(a2) * p.attention_scaling);
-    } else {
-      c2[e] = c1[e]; s2[e] = s1[e];
-    }
+    const float2 a = turns[0][2 * lane + e], b = turns[1][2 * lane + e];
+    c1[e] = a.x; s1[e] = a.y; c2[e] = b.x; s2[e] = b.y;
   }
 
-  const int total = p.num_heads + p.num_kv_heads;
-  for (int hh = warp; hh < total; hh += 8) {
-    const bool is_k = hh >= p.num_heads;
-    const int h = is_k ? hh - p.num_heads : hh;
-    const __nv_bfloat16* src = is_k ? p.k + (int64_t)tok * p.k_stride + h * HD : p.q + (int64_t)tok * p.q_stride + h * HD;
-    const __nv_bfloat16* w = is_k ? p.k_w : p.q_w;
-    const uint32_t r1 = *reinterpret_cast<const uint32_t*>(src + 2 * lane);
-    const uint32_t r2 = *reinterpret_cast<const uint32_t*>(src + 64 + 2 * lane);
-    float x1[2] = {bf16lo(r1), bf16hi(r1)};
-    float x2[2] = {bf16lo(r2), bf16hi(r2)};
-    if (w) {
-      float ss = x1[0] * x1[0];
-      ss = fmaf(x1[1], x1[1], ss); ss = fmaf(x2[0], x2[0], ss); ss = fmaf(x2[1], x2[1], ss);
-      const float rstd = rstd_of<EAGER>(warp_sum(ss), HD, p.eps);
-      const uint32_t w1 = *reinterpret_cast<const uint32_t*>(w + 2 * lane);
-      const uint32_t w2 = *reinterpret_cast<const uint32_t*>(w + 64 + 2 * lane);
-      x1[0] = rbf(norm_out<EAGER>(x1[0], rstd, bf16lo(w1))); x1[1] = rbf(norm_out<EAGER>(x1[1], rstd, bf16hi(w1)));
-      x2[0] = rbf(norm_out<EAGER>(x2[0], rstd, bf16lo(w2))); x2[1] = rbf(norm_out<EAGER>(x2[1], rstd, bf16hi(w2)));
-    }
-    float o1[2], o2[2];
+  for (int h0 = warp; h0 < total; h0 += 8 * AHEAD) {
+    if (h0 != warp) fetch(h0);
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      o1[e] = rbf(x1[e] * c1[e]) + rbf(-x2[e] * s1[e]);   // rotate_half: first half pairs with -x2
-      o2[e] = rbf(x2[e] * c2[e]) + rbf(x1[e] * s2[e]);
-    }
-    const uint32_t y1 = pack_bf16(o1[0], o1[1]), y2 = pack_bf16(o2[0], o2[1]);
-    __nv_bfloat16* dst = nullptr;
-    if (is_k) {
-      if (p.k_out) dst = p.k_out + (int64_t)tok * kv_dim + h * HD;
-      if (slot >= 0) {
-        __nv_bfloat16* cd = p.k_cache + (int64_t)slot * kv_dim + h * HD;
-        *reinterpret_cast<uint32_t*>(cd + 2 * lane) = y1;
-        *reinterpret_cast<uint32_t*>(cd + 64 + 2 * lane) = y2;
+    for (int i = 0; i < AHEAD; ++i) {
+      const int hh = h0 + 8 * i;
+      if (hh >= total) break;
+      const bool is_k = hh >= p.num_heads;
+      const int h = is_k ? hh - p.num_heads : hh;
+      const __nv_bfloat16* w = is_k ? p.k_w : p.q_w;
+      float x1[2] = {bf16lo(r1[i]), bf16hi(r1[i])};
+      float x2[2] = {bf16lo(r2[i]), bf16hi(r2[i])};
+      if (w) {
+        float ss = x1[0] * x1[0];
+        ss = fmaf(x1[1], x1[1], ss); ss = fmaf(x2[0], x2[0], ss); ss = fmaf(x2[1], x2[1], ss);
+        const float rstd = rstd_of<EAGER>(warp_sum(ss), HD, p.eps);
+        const uint32_t w1 = *reinterpret_cast<const uint32_t*>(w + 2 * lane);
+        const uint32_t w2 = *reinterpret_cast<const uint32_t*>(w + 64 + 2 * lane);
+        x1[0] = rbf(norm_out<EAGER>(x1[0], rstd, bf16lo(w1))); x1[1] = rbf(norm_out<EAGER>(x1[1], rstd, bf16hi(w1)));
+        x2[0] = rbf(norm_out<EAGER>(x2[0], rstd, bf16lo(w2))); x2[1] = rbf(norm_out<EAGER>(x2[1], rstd, bf16hi(w2)));
       }
-    } else {
-      dst = p.q_out + ((int64_t)tok * p.num_heads + h) * HD;
-    }
-    if (dst) {
-      *reinterpret_cast<uint32_t*>(dst + 2 * lane) = y1;
-      *reinterpret_cast<uint32_t*>(dst + 64 + 2 * lane) = y2;
+      float o1[2], o2[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        o1[e] = rbf(x1[e] * c1[e]) + rbf(-x2[e] * s1[e]);   // rotate_half: first half pairs with -x2
+        o2[e] = rbf(x2[e] * c2[e]) + rbf(x1[e] * s2[e]);
+      }
+      const uint32_t y1 = pack_bf16(o1[0], o1[1]), y2 = pack_bf16(o2[0], o2[1]);
+      __nv_bfloat16* dst = nullptr;
+      if (is_k) {
+        if (p.k_out) dst = p.k_out + (int64_t)tok * kv_dim + h * HD;
+        if (slot >= 0) {
+          __nv_bfloat16* cd = p.k_cache + (int64_t)slot * kv_dim + h * HD;
+          *reinterpret_cast<uint32_t*>(cd + 2 * lane) = y1;
+          *reinterpret_cast<uint32_t*>(cd + 64 + 2 * lane) = y2;
+        }
+      } else {
+        dst = p.q_out + ((int64_t)tok * p.num_heads + h) * HD;
+      }
+      if (dst) {
+        *reinterpret_cast<uint32_t*>(dst + 2 * lane) = y1;
+        *reinterpret_cast<uint32_t*>(dst + 64 + 2 * lane) = y2;
+      }
     }
   }
-  if (slot >= 0 && p.v) {                                  // V goes to the cache untouched
+  if (put_v) {
     const __nv_bfloat16* vs = p.v + (int64_t)tok * p.v_stride;
     __nv_bfloat16* vd = p.v_cache + (int64_t)slot * kv_dim;
-    for (int i = threadIdx.x; i < (kv_dim >> 3); i += blockDim.x) stg_v4(vd + 8 * i, ldg_nc_v4(vs + 8 * i));
+    if (threadIdx.x < (kv_dim >> 3)) stg_v4(vd + 8 * threadIdx.x, v0);
+    for (int i = threadIdx.x + blockDim.x; i < (kv_dim >> 3); i += blockDim.x) stg_v4(vd + 8 * i, ldg_nc_v4(vs + 8 * i));
   }
 }
 
