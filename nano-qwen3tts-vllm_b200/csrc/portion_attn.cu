@@ -24,7 +24,8 @@
 // (one thread a row with 40 spilled registers: 143 us for the case below; one barrier per slot of the ring instead of per tile: 20 us more).
 // 4 prompts of 2048 tokens, 16 heads over 8 of 128, window 1024 + 4 kept, element gates: 118 us (mma.sync, 64 queries per CTA: 547 us; 31 at
 // the tensor core's rate); causal with a score cap, 4448 tokens: 141 us (579 us); latent
-// heads of 192 over expanded keys, 4 x 2048 causal: 152 us.  Sigmoid weights (two special-function results and a table's number a pair), window
+// heads of 192 over expanded keys, 4 x 2048 causal: 142 us; prompts that
+// are their own keys, weights rounded once, 4096 + 1531 causal: 100 us (152 us one query tile a CTA).  Sigmoid weights (two special-function results and a table's number a pair), window
 // 1024, 4138 tokens: 79 us (143 us).
 //
 // Every copy is bounded: maps have the true extents of their tensors, so a row that a block table should not name reads zeros.  Every
@@ -181,17 +182,21 @@ struct PortionSpan {
   __device__ __forceinline__ bool has(int j) const { return j < front || (j >= first && j <= last); }
 };
 
+// softmax weights as bf16 pairs, or rounded once; sigmoid weights as pairs
+enum { PO_PAIRS = 0, PO_ROUNDED = 1, PO_SIGMOID = 2 };
 // slots of the ring; sigmoid weights need room for their tables beside it
-template <int NS, bool SIG> constexpr int po_slots() { return SIG ? 8 : NS == 1 ? 12 : NS == 2 ? 10 : 8; }
+template <int NS, int MODE> constexpr int po_slots() { return MODE == PO_SIGMOID ? 8 : NS == 1 ? 12 : NS == 2 ? 10 : 8; }
 constexpr int PO_DEEP = 8, PO_BAR_BYTES = 512, PO_TAIL = PO_BAR_BYTES + PO_ITEMS * 24, PO_SMEM = 232448;
-template <int NS, bool SIG> constexpr int po_smem() { return 1024 + (2 * NS + po_slots<NS, SIG>()) * PO_SLOT + PO_TAIL; }
-static_assert(po_smem<1, false>() <= PO_SMEM && po_smem<2, false>() <= PO_SMEM && po_smem<3, false>() <= PO_SMEM, "shared memory of a CTA");
+template <int NS, int MODE> constexpr int po_smem() { return 1024 + (2 * NS + po_slots<NS, MODE>()) * PO_SLOT + PO_TAIL; }
+static_assert(po_smem<1, PO_PAIRS>() <= PO_SMEM && po_smem<2, PO_PAIRS>() <= PO_SMEM && po_smem<3, PO_PAIRS>() <= PO_SMEM, "shared memory of a CTA");
 
-// NS: 64-column slices of q and k; NV: of v; SIG: sigmoid weights
-template <int NS, int NV, bool SIG>
+// NS: 64-column slices of q and k; NV: of v
+template <int NS, int NV, int MODE>
 __global__ void __launch_bounds__(PO_THREADS, 1)
 portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_constant__ PortionMaps maps) {
-  constexpr int SLOTS = po_slots<NS, SIG>(), PER_TILE = NS + NV;
+  constexpr int SLOTS = po_slots<NS, MODE>(), PER_TILE = NS + NV;
+  constexpr bool SIG = MODE == PO_SIGMOID;
+  constexpr int STEPS = PO_N / 16 * (MODE == PO_ROUNDED ? 1 : 2);        // products of a tile's weights and values
   static_assert(2 * NS + NV <= SLOTS, "a tile's values beside two tiles of keys");
   static_assert(SLOTS / PER_TILE + 1 < PO_DEEP, "tiles in the ring at once");
   extern __shared__ uint8_t po_smem_dyn[];
@@ -211,21 +216,25 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   if (warp == PO_LISTER) {
     // The CTA's items: number i of the valid (tile, sequence, heads), late tiles first (they are the longest under a causal mask), for
-    // i = c, 2 G - 1 - c, 2 G + c, ..
+    // i = c, 2 G - 1 - c, 3 G - 1 - c, 3 G + c, 4 G + c, ..: who begins with a long one gets the short ones, and a round that is not full goes to
+    // those with the least so far
     const int span = p.tiles * (128 >> p.hpc_shift), groups = a.H >> p.hpc_shift, c = blockIdx.x, G = gridDim.x;
     int k = 0, cum = 0, want = c;
-    const int len0 = lane < a.n_seqs ? a.seq_len[lane] : 0;
+    auto len_of = [&](int b) { return a.cu != nullptr ? a.cu[b + 1] - a.cu[b] : a.seq_len[b]; };
+    const int len0 = lane < a.n_seqs ? len_of(lane) : 0, least = a.one_token ? 1 : 2;
     for (int tile = (a.max_new + span - 1) / span - 1; tile >= 0 && k < PO_ITEMS; --tile) {
       for (int base = 0; base < a.n_seqs && k < PO_ITEMS; base += 32) {
-        const int len = base == 0 ? len0 : base + lane < a.n_seqs ? a.seq_len[base + lane] : 0;
-        const unsigned live = __ballot_sync(0xffffffffu, len > 1 && tile * span < len);
+        const int len = base == 0 ? len0 : base + lane < a.n_seqs ? len_of(base + lane) : 0;
+        const unsigned live = __ballot_sync(0xffffffffu, len >= least && tile * span < len);
         const int cnt = __popc(live) * groups;
         while (k < PO_ITEMS && want < cum + cnt) {
           const int at = want - cum, rank = at / groups;
           const int at_b = static_cast<int>(__fns(live, 0, rank + 1));
-          if (lane == at_b) list[k] = PortionEntry{tile, base + lane, at - rank * groups, len, a.seq_start[base + lane], a.seq_pos0[base + lane]};
+          if (lane == at_b)
+            list[k] = PortionEntry{tile, base + lane, at - rank * groups, len, a.cu != nullptr ? a.cu[base + lane] : a.seq_start[base + lane],
+                                   a.cu != nullptr ? 0 : a.seq_pos0[base + lane]};
           ++k;
-          want = k * G + (k & 1 ? G - 1 - c : c);
+          want = k * G + ((k + 1) >> 1 & 1 ? G - 1 - c : c);
         }
         cum += cnt;
       }
@@ -258,7 +267,7 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
         const PortionItem m(a, p, list[x]);
         const int g = m.h0 / (a.H / a.G), gv = g % a.Gv, R = p.box_rows;
         const int32_t* bt = a.block_tables != nullptr ? a.block_tables + static_cast<int64_t>(m.b) * a.bt_stride : nullptr;
-        const int row0 = bt == nullptr ? a.key_start[m.b] : 0;
+        const int row0 = bt != nullptr ? 0 : a.cu != nullptr ? m.start : a.key_start[m.b];
         const int n1 = min(NS, (a.d1 + 63) / 64);
         // lane = box * 4 + slice; row of the lane's box of tile j, a tile ahead: nothing waits for the load of the page's number here
         const int box = lane >> 2, sl = lane & 3, boxes = PO_N / R;
@@ -380,12 +389,12 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
                   if (!apart) {
                     po_umma_ts(tm_o, tm_p, v_lo, idesc_o, begun[g]);
 #pragma unroll
-                    for (int s = 1; s < PO_N / 8; ++s) po_umma_ts(tm_o, tm_p + po_weights_at(s), v_lo + (s & 7) * 128, idesc_o, 1);
+                    for (int s = 1; s < STEPS; ++s) po_umma_ts(tm_o, tm_p + po_weights_at(s), v_lo + (s & 7) * 128, idesc_o, 1);
                   } else {
 #pragma unroll 1
                     for (int half = 0; half < 2; ++half)
 #pragma unroll
-                      for (int s = 0; s < PO_N / 8; ++s)
+                      for (int s = 0; s < STEPS; ++s)
                         po_umma_ts(tm_o + half * 64, tm_p + po_weights_at(s), (half ? ring_v : v_lo) + (s & 7) * 128, idesc_half, begun[g] || s);
                   }
                   if (last_o) umma_commit(o_full + g);
@@ -612,16 +621,19 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
               sa = po_add2(sa, wa);
               sb = po_add2(sb, wb);
             }
-            const uint32_t p0 = pack_bf16(w0, w1), p1 = pack_bf16(w2, w3), n0 = p0 ^ 0x80008000u, n1 = p1 ^ 0x80008000u;
-            po_split(po_add2(wa, po_pair(bf16lo(n0), bf16hi(n0))), r0, r1);
-            po_split(po_add2(wb, po_pair(bf16lo(n1), bf16hi(n1))), r2, r3);
-            rest[c / 2] = pack_bf16(r0, r1);
-            rest[c / 2 + 1] = pack_bf16(r2, r3);
+            const uint32_t p0 = pack_bf16(w0, w1), p1 = pack_bf16(w2, w3);
+            if constexpr (MODE != PO_ROUNDED) {
+              const uint32_t n0 = p0 ^ 0x80008000u, n1 = p1 ^ 0x80008000u;
+              po_split(po_add2(wa, po_pair(bf16lo(n0), bf16hi(n0))), r0, r1);
+              po_split(po_add2(wb, po_pair(bf16lo(n1), bf16hi(n1))), r2, r3);
+              rest[c / 2] = pack_bf16(r0, r1);
+              rest[c / 2 + 1] = pack_bf16(r2, r3);
+            }
             hi[c / 2] = p0;
             hi[c / 2 + 1] = p1;
           }
           po_st16<HK>(tm_s + part, hi);
-          po_st16<HK>(tm_s + part + 16, rest);
+          if constexpr (MODE != PO_ROUNDED) po_st16<HK>(tm_s + part + 16, rest);
         }
         float s0, s1;
         po_split(po_add2(sa, sb), s0, s1);
@@ -703,7 +715,7 @@ static int po_heads(const PortionArgs& a) {
   int hpc = 1;
   while (hpc < 8 && (a.H / a.G) % (2 * hpc) == 0) hpc *= 2;
   if (a.r1 == nullptr) return hpc;
-  const int room = PO_SMEM - (a.d == 64 ? po_smem<1, true>() : po_smem<2, true>());
+  const int room = PO_SMEM - (a.d == 64 ? po_smem<1, PO_SIGMOID>() : po_smem<2, PO_SIGMOID>());
   while (hpc > 0 && static_cast<int64_t>(4) * hpc * po_tab_row(a.mask, hpc) * 4 > room) hpc /= 2;
   return hpc;
 }
@@ -719,10 +731,10 @@ bool portion_attn_applies(const PortionArgs& a) {
          (a.gate == nullptr || !a.gate_el || (reinterpret_cast<uintptr_t>(a.gate) % 4 == 0 && a.ldg % 2 == 0));
 }
 
-template <int NS, int NV, bool SIG>
+template <int NS, int NV, int MODE>
 static int go_portion(const char* what, const PortionArgs& a, const PortionPlan& p, const PortionMaps& maps, int grid, cudaStream_t st) {
-  auto kern = portion_attn_kernel<NS, NV, SIG>;
-  const int smem = po_smem<NS, SIG>() + (SIG ? 4 * p.hpc * p.tab_row * 4 : 0);
+  auto kern = portion_attn_kernel<NS, NV, MODE>;
+  const int smem = po_smem<NS, MODE>() + (MODE == PO_SIGMOID ? 4 * p.hpc * p.tab_row * 4 : 0);
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return cuda_fail(e, what);
   kern<<<grid, PO_THREADS, smem, st>>>(a, p, maps);
@@ -772,8 +784,9 @@ int launch_portion_attn(const char* what, const PortionArgs& a, cudaStream_t st)
   }
   if (rc != B2TTS_OK) return rc;
   const int ns = a.d / 64;
-  if (a.r1 != nullptr) return ns == 1 ? go_portion<1, 1, true>(what, a, p, maps, grid, st) : go_portion<2, 2, true>(what, a, p, maps, grid, st);
-#define PO_GO(NS, NV) return go_portion<NS, NV, false>(what, a, p, maps, grid, st)
+  if (a.r1 != nullptr) return ns == 1 ? go_portion<1, 1, PO_SIGMOID>(what, a, p, maps, grid, st) : go_portion<2, 2, PO_SIGMOID>(what, a, p, maps, grid, st);
+  if (a.round_weights && ns == 2 && a.dv == 128) return go_portion<2, 2, PO_ROUNDED>(what, a, p, maps, grid, st);
+#define PO_GO(NS, NV) return go_portion<NS, NV, PO_PAIRS>(what, a, p, maps, grid, st)
   if (a.dv == 64) {
     if (ns == 1) PO_GO(1, 1);
     if (ns == 2) PO_GO(2, 1);

@@ -17,6 +17,9 @@ struct PortionArgs {
   const int32_t* block_tables; int64_t bt_stride; int page;
   const int32_t* key_start;
   const int32_t *seq_start, *seq_pos0, *seq_len;
+  const int32_t* cu;                                  // not null: sequence b is tokens cu[b] .. cu[b + 1] - 1 of q, k and v, from position 0 on
+  int one_token;                                      // sequences of one token are taken too
+  int round_weights;                                  // the weights enter the second product rounded to bf16 once, not as pairs
   const float* sink;                                  // [H] or null
   const __nv_bfloat16* gate; int64_t ldg; int gate_el;
   void* out; int out_f32;                             // [tokens, H * dv]

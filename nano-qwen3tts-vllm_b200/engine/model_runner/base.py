@@ -244,7 +244,7 @@ class ModelRunner:
         positions = dev[:total]
         slot_mapping = dev[total:2 * total].to(torch.int32)
         cuq = dev[2 * total:2 * total + len(seqs) + 1].to(torch.int32)
-        cuk = dev[2 * total + len(seqs) + 1:].to(torch.int32)
+        cuk = cuq if np.array_equal(cu_k, cu_q) else dev[2 * total + len(seqs) + 1:].to(torch.int32)       # one tensor: the prompts are their own keys
         block_tables = None
         if cu_k[-1] > cu_q[-1]:                                              # prefix cache hit (never, see block manager)
             block_tables = self.prepare_block_tables(seqs)

@@ -139,6 +139,33 @@ def test_sigmoid_weights_with_a_negative_scale(nat):
     _sigmoid_case(nat, [(0, 300)], 4, 2, 64, 90, page=16, scale=-0.2)
 
 
+@pytest.mark.parametrize("H,G", [(16, 8), (4, 4), (8, 1), (6, 2)])
+@pytest.mark.parametrize("lens", [(128,), (1, 300, 2, 129, 1), (257, 64, 127), (1000, 700)])
+def test_prompts_that_are_their_own_keys(nat, H, G, lens):
+    """Strided rows of a packed projection, causal; sequences of one token among them."""
+    d, n = 128, sum(lens)
+    g = torch.Generator().manual_seed(n + H)
+    u = torch.randn(n, (H + 2 * G) * d + 64, generator=g).to(BF)
+    cu = torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32, device=DEV)
+    ud = u.to(DEV)
+    q, k, v = ud[:, :H * d], ud[:, H * d:(H + G) * d], ud[:, (H + G) * d:(H + 2 * G) * d]
+    heads = lambda t, m: t.unflatten(1, (m, d))
+    out = nat.varlen_attn_prefill(heads(q, H), heads(k, G), heads(v, G), cu, cu, max(lens), max(lens), d ** -0.5)
+    ref, o = [], 0
+    for m in lens:
+        x = u[o:o + m].to(F64)
+        qq, kk, vv = x[:, :H * d].view(m, H, d), x[:, H * d:(H + G) * d].view(m, G, d), x[:, (H + G) * d:(H + 2 * G) * d].view(m, G, d)
+        s = torch.einsum("ihd,jhd->hij", qq, kk.repeat_interleave(H // G, 1)) * d ** -0.5
+        s = s.masked_fill(torch.ones(m, m).tril() == 0, -math.inf).softmax(-1)
+        ref.append(torch.einsum("hij,jhd->ihd", s, vv.repeat_interleave(H // G, 1)))
+        o += m
+    ref = torch.cat(ref).reshape(n, -1)
+    err = (out.reshape(n, -1).double().cpu() - ref).abs().max() / ref.abs().max()
+    # weights rounded once to 2^-9 and averaged, results rounded to 2^-9
+    assert err.item() < 6e-3, err.item()
+    assert nat.portion_attn_timeouts() == 0
+
+
 @pytest.mark.parametrize("keys", [420, 421])
 def test_sigmoid_weights_of_sequences_that_the_host_knows_of(nat, keys):
     _sigmoid_case(nat, [(keys - 40, 40), (0, 33)], 4, 2, 64, 90, page=16, known=True)
