@@ -134,8 +134,12 @@ def _load():
         "b2tts_short_conv_act": (I, [P, L, I, P, P, P, P, P, P, P, P, P, P, L, I, I, I, I, I, I, I, P]),
         "b2tts_gated_group_norm": (I, [P, P, L, P, I, I, I, I, F, P, I, I, I, P]),
         "b2tts_ssm_scan": (I, [P, L, P, L, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P]),
+        "b2tts_ssm_scan_ahead_floats": (Z, [I, I, I]),
+        "b2tts_ssm_scan_ahead": (I, [P, L, P, L, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, P, Z, P]),
         "b2tts_ssm_scan_portions": (I, [P, L, P, L, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, P]),
         "b2tts_delta_rule_scan": (I, [P, L, P, P, L, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P]),
+        "b2tts_delta_rule_scan_ahead_floats": (Z, [I, I, I]),
+        "b2tts_delta_rule_scan_ahead": (I, [P, L, P, P, L, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, P, Z, P]),
         "b2tts_delta_rule_scan_portions": (I, [P, L, P, P, L, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, P]),
         "b2tts_matrix_memory_scan": (I, [P, P, P, P, P, L, P, P, F, P, P, P, P, P, P, P, P, I, I, I, I, I, I, P]),
         "b2tts_grouped_gemm": (I, [P, L, P, P, L, P, P, I, I, I, I, I, I, I, I, I, P]),
@@ -1206,28 +1210,35 @@ def _coef(out, heads):
     return torch.empty(out.shape[0], heads, 3, dtype=F32, device=out.device)
 
 
-def ssm_scan(xbc, dt_in, dt_bias, a_log, d_skip, state, out, lay, heads, groups, vdim, nstate):
+def ssm_scan(xbc, dt_in, dt_bias, a_log, d_skip, state, out, lay, heads, groups, vdim, nstate, ahead=True):
     """xbc [n, heads*vdim + 2*groups*nstate] (convolved, activated); dt_in: a column slice [n, heads]; state float
-    [slots, heads, nstate, vdim]; out float [n, heads*vdim]."""
+    [slots, heads, nstate, vdim]; out float [n, heads*vdim].  ``ahead``: long portions' scores are formed once a group of heads."""
     dt = _act(xbc, "xbc")
     _cuda(state, F32, "state"); _cuda(out, F32, "out")
     assert dt_in.dtype == xbc.dtype and dt_in.stride(1) == 1 and state.is_contiguous() and out.is_contiguous()
-    _check(_load().b2tts_ssm_scan_portions(xbc.data_ptr(), xbc.stride(0), dt_in.data_ptr(), dt_in.stride(0), dt_bias.data_ptr(),
-                                           a_log.data_ptr(), d_skip.data_ptr(), state.data_ptr(), _coef(out, heads).data_ptr(),
-                                           out.data_ptr(), *_seq_args(lay, True), getattr(lay, "max_new", 0), heads, groups, vdim, nstate,
-                                           dt, _stream()), "ssm_scan")
+    max_new, scores = getattr(lay, "max_new", 0), None
+    if ahead and max_new > 64 and dt == DTYPE_CODE[BF16] and heads >= 4 * groups:
+        scores = torch.empty(_load().b2tts_ssm_scan_ahead_floats(lay.n_tokens, lay.n_seqs, groups), dtype=F32, device=xbc.device)
+    _check(_load().b2tts_ssm_scan_ahead(xbc.data_ptr(), xbc.stride(0), dt_in.data_ptr(), dt_in.stride(0), dt_bias.data_ptr(),
+                                        a_log.data_ptr(), d_skip.data_ptr(), state.data_ptr(), _coef(out, heads).data_ptr(),
+                                        out.data_ptr(), *_seq_args(lay, True), max_new, heads, groups, vdim, nstate,
+                                        dt, _ptr(scores), 0 if scores is None else scores.numel(), _stream()), "ssm_scan")
 
 
-def delta_rule_scan(qkv, beta_in, a_in, a_log, dt_bias, state, out, lay, heads, kv_heads, dim, vdim):
-    """qkv [n, 2*kv_heads*dim + heads*vdim] (convolved, activated); beta_in, a_in: column slices [n, heads] of one tensor."""
+def delta_rule_scan(qkv, beta_in, a_in, a_log, dt_bias, state, out, lay, heads, kv_heads, dim, vdim, ahead=True):
+    """qkv [n, 2*kv_heads*dim + heads*vdim] (convolved, activated); beta_in, a_in: column slices [n, heads] of one tensor.  ``ahead``: what long
+    portions' keys and queries alone say is formed once a key head."""
     dt = _act(qkv, "qkv")
     _cuda(state, F32, "state"); _cuda(out, F32, "out")
     assert beta_in.dtype == qkv.dtype and a_in.dtype == qkv.dtype and beta_in.stride(0) == a_in.stride(0)
     assert state.is_contiguous() and out.is_contiguous()
-    _check(_load().b2tts_delta_rule_scan_portions(qkv.data_ptr(), qkv.stride(0), beta_in.data_ptr(), a_in.data_ptr(), beta_in.stride(0),
-                                                  a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), _coef(out, heads).data_ptr(),
-                                                  out.data_ptr(), *_seq_args(lay, True), getattr(lay, "max_new", 0), heads, kv_heads, dim,
-                                                  vdim, dt, _stream()), "delta_rule_scan")
+    max_new, dots = getattr(lay, "max_new", 0), None
+    if ahead and max_new > 64 and dt == DTYPE_CODE[BF16] and heads * vdim >= 128 * kv_heads:
+        dots = torch.empty(_load().b2tts_delta_rule_scan_ahead_floats(lay.n_tokens, lay.n_seqs, kv_heads), dtype=F32, device=qkv.device)
+    _check(_load().b2tts_delta_rule_scan_ahead(qkv.data_ptr(), qkv.stride(0), beta_in.data_ptr(), a_in.data_ptr(), beta_in.stride(0),
+                                               a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), _coef(out, heads).data_ptr(),
+                                               out.data_ptr(), *_seq_args(lay, True), max_new, heads, kv_heads, dim, vdim, dt, _ptr(dots),
+                                               0 if dots is None else dots.numel(), _stream()), "delta_rule_scan")
 
 
 def gated_linear_scan(q, k, v, z, z_bias, tau, state, out, lay, heads, dim, vdim):

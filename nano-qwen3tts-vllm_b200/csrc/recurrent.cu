@@ -347,6 +347,16 @@ extern "C" int b2tts_ssm_scan_portions(const void* xbc, int64_t ldx, const void*
                               const float* a_log, const float* d_skip, float* state, float* coef, float* out, const int32_t* seq_start,
                               const int32_t* seq_pos0, const int32_t* seq_len, const int32_t* seq_slot, int n_tokens, int n_seqs, int max_new,
                               int heads, int groups, int vdim, int dim, int dtype, void* stream) {
+  return b2tts_ssm_scan_ahead(xbc, ldx, dt, lddt, dt_bias, a_log, d_skip, state, coef, out, seq_start, seq_pos0, seq_len, seq_slot, n_tokens, n_seqs,
+                              max_new, heads, groups, vdim, dim, dtype, nullptr, 0, stream);
+}
+extern "C" size_t b2tts_ssm_scan_ahead_floats(int n_tokens, int n_seqs, int groups) {
+  return n_tokens > 0 && n_seqs > 0 && groups > 0 ? static_cast<size_t>(chunk_scores_floats(n_tokens, n_seqs, groups)) : 0;
+}
+extern "C" int b2tts_ssm_scan_ahead(const void* xbc, int64_t ldx, const void* dt, int64_t lddt, const float* dt_bias,
+                              const float* a_log, const float* d_skip, float* state, float* coef, float* out, const int32_t* seq_start,
+                              const int32_t* seq_pos0, const int32_t* seq_len, const int32_t* seq_slot, int n_tokens, int n_seqs, int max_new,
+                              int heads, int groups, int vdim, int dim, int dtype, float* scores, size_t scores_floats, void* stream) {
   SCAN_COMMON_CHECKS("ssm_scan");
   B2_REQUIRE(groups > 0 && heads % groups == 0 && n_tokens >= 0, B2TTS_EINVAL, "ssm_scan: %d heads over %d groups", heads, groups);
   B2_REQUIRE(xbc && dt && dt_bias && a_log && d_skip && coef, B2TTS_EINVAL, "ssm_scan: null pointer");
@@ -371,7 +381,13 @@ extern "C" int b2tts_ssm_scan_portions(const void* xbc, int64_t ldx, const void*
   if (chunks) {
     const bool alone = n_seqs == 1 && max_new > 0;         // no second launch: max_new may be above its length, which is then taken too
     a.min_len = alone ? 1 : walk + 1;
-    const int rc = launch_linear_chunk("ssm_scan (portions)", a, n_seqs, st);
+    // a group's scores ahead of the chain where at least four heads share them: else their traffic is what their products cost
+    if (scores != nullptr && heads / groups >= 4) {
+      B2_REQUIRE(aligned16(scores) && scores_floats >= b2tts_ssm_scan_ahead_floats(n_tokens, n_seqs, groups), B2TTS_EWORKSPACE,
+                 "ssm_scan: %zu floats for scores (or unaligned)", scores_floats);
+      a.scores = scores;
+    }
+    const int rc = launch_linear_chunk("ssm_scan (portions)", a, n_seqs, longest, static_cast<int64_t>(n_tokens) / 64 + n_seqs + 1, st);
     if (rc != B2TTS_OK || alone) return rc;
     a.min_len = 1; a.max_len = walk;                       // single tokens and short portions beside them
   }
@@ -395,6 +411,17 @@ extern "C" int b2tts_delta_rule_scan_portions(const void* qkv, int64_t ldq, cons
                                      const int32_t* seq_start, const int32_t* seq_pos0, const int32_t* seq_len,
                                      const int32_t* seq_slot, int n_tokens, int n_seqs, int max_new, int heads, int kv_heads, int dim, int vdim,
                                      int dtype, void* stream) {
+  return b2tts_delta_rule_scan_ahead(qkv, ldq, beta, a_in, ldu, a_log, dt_bias, state, coef, out, seq_start, seq_pos0, seq_len, seq_slot, n_tokens,
+                                     n_seqs, max_new, heads, kv_heads, dim, vdim, dtype, nullptr, 0, stream);
+}
+extern "C" size_t b2tts_delta_rule_scan_ahead_floats(int n_tokens, int n_seqs, int kv_heads) {
+  return n_tokens > 0 && n_seqs > 0 && kv_heads > 0 ? static_cast<size_t>(delta_dots_floats(n_tokens, n_seqs, kv_heads)) : 0;
+}
+extern "C" int b2tts_delta_rule_scan_ahead(const void* qkv, int64_t ldq, const void* beta, const void* a_in, int64_t ldu,
+                                     const float* a_log, const float* dt_bias, float* state, float* coef, float* out,
+                                     const int32_t* seq_start, const int32_t* seq_pos0, const int32_t* seq_len,
+                                     const int32_t* seq_slot, int n_tokens, int n_seqs, int max_new, int heads, int kv_heads, int dim, int vdim,
+                                     int dtype, float* dots, size_t dots_floats, void* stream) {
   SCAN_COMMON_CHECKS("delta_rule_scan");
   B2_REQUIRE(kv_heads > 0 && heads % kv_heads == 0 && n_tokens >= 0, B2TTS_EINVAL, "delta_rule_scan: %d heads over %d key heads", heads, kv_heads);
   B2_REQUIRE(qkv && beta && a_in && a_log && dt_bias && coef, B2TTS_EINVAL, "delta_rule_scan: null pointer");
@@ -419,7 +446,12 @@ extern "C" int b2tts_delta_rule_scan_portions(const void* qkv, int64_t ldq, cons
   if (chunks) {
     const bool alone = n_seqs == 1 && max_new > 0;         // no second launch: max_new may be above its length, which is then taken too
     a.min_len = alone ? 1 : walk + 1;
-    const int rc = launch_delta_chunk("delta_rule_scan (portions)", a, n_seqs, st);
+    if (dots != nullptr && heads / kv_heads * (vdim / 64) >= 2) {          // somebody to share them
+      B2_REQUIRE(aligned16(dots) && dots_floats >= b2tts_delta_rule_scan_ahead_floats(n_tokens, n_seqs, kv_heads), B2TTS_EWORKSPACE,
+                 "delta_rule_scan: %zu floats for dot products (or unaligned)", dots_floats);
+      a.scores = dots;
+    }
+    const int rc = launch_delta_chunk("delta_rule_scan (portions)", a, n_seqs, longest, st);
     if (rc != B2TTS_OK || alone) return rc;
     a.min_len = 1; a.max_len = walk;                       // single tokens and short portions beside them
   }

@@ -18,8 +18,9 @@
 // Numbers that the split could not represent (not finite, or so large that a product might overflow) send their chunk through a
 // token-by-token walk over the same registers, so that an infinity reaches the outputs it reaches there and no others.
 //
-// Bound: the chain of chunks (about 620 m16n8k16 per warp and chunk, each waiting for its fragments; most of a chunk's work does not
-// depend on the state in front of it, but sits in the chain).  4 sequences x 2048 tokens, 64 heads of 64 values x 128 channels: 574 us,
+// Bound: the chain of chunks (about 500 m16n8k16 per warp and chunk, each waiting for its fragments).  Scores of queries and keys do not
+// depend on the state and are the same for all heads of a group, so a kernel in front forms them once (chunk_scores_kernel) where at least four
+// heads share them.  4 sequences x 2048 tokens, 64 heads of 64 values x 128 channels: 561 us with the scores in the chain, 492 + 5 ahead of it,
 // token by token 3371 us; one sequence of 300 tokens 79 / 186 us.  Short portions stay with that kernel, see linear_walk_len().
 #include "scan.cuh"
 
@@ -112,9 +113,89 @@ __device__ __forceinline__ uint32_t mag2(uint32_t m, uint32_t x) { return __vmax
 constexpr uint32_t CK_BIG_IN = (127 + 40) << 7;       // bf16 bits of 2^40
 constexpr float CK_BIG_STATE = 1.2089258e24f;         // 2^80: times 2^40 and 128 terms still finite
 
+// Scores of a chunk's queries 16 warp .. + 15 against its keys up to the diagonal, sc[nt]: keys 8 nt + c2 (+ 1), queries g4 (+ 8).
 template <int D>
+__device__ __forceinline__ void chunk_row_scores(uint32_t q_u, uint32_t k_u, int warp, int lane, float sc[8][4]) {
+  constexpr int RB = D * 2;
+  const int ra = lane & 15, ca = lane >> 4, rb = (lane >> 4) * 8 + (lane & 7), cb = (lane >> 3) & 1;
+  // the upper halves of q's significant bits give sums of 16 products that a float nearly always holds, the lower ones small sums:
+  // what the tensor core cuts off is a sixteenth (outputs 8.8e-8 -> 7.9e-8 from 64 bits, 12 of 574 us)
+  float st[8][4];
+#pragma unroll
+  for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) sc[nt][e] = st[nt][e] = 0.f;
+#pragma unroll
+  for (int ks = 0; ks < D / 16; ++ks) {
+    uint32_t af[4], hf[4], tf[4];
+    ldsm4(af, q_u + tile_off(warp * 16 + ra, ks * 2 + ca, RB));
+#pragma unroll
+    for (int e = 0; e < 4; ++e) halves(af[e], hf[e], tf[e]);
+#pragma unroll
+    for (int np = 0; np < 4; ++np) {
+      if (np <= warp) {
+        uint32_t bf[4];
+        ldsm4(bf, k_u + tile_off(np * 16 + rb, ks * 2 + cb, RB));
+        mma_bf16_16816(st[2 * np], tf, bf[0], bf[1]);
+        mma_bf16_16816(st[2 * np + 1], tf, bf[2], bf[3]);
+        mma_add(sc[2 * np], hf, bf[0], bf[1]);
+        mma_add(sc[2 * np + 1], hf, bf[2], bf[3]);
+      }
+    }
+  }
+#pragma unroll
+  for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) sc[nt][e] += st[nt][e];
+}
+
+// Which chunk of the step's: the chunks of sequence b, which starts at row `start`, have numbers of their own.
+__device__ __forceinline__ int64_t chunk_number(int64_t start, int t0, int b) { return (start + t0) / CK_L + b; }
+constexpr int CK_SCORES = CK_L * CK_L;     // floats of a chunk's scores, as the threads hold them: [warp][nt][lane] float4
+
+// The scores of every chunk and group of heads, formed once where many heads share their queries and keys: in the chain of chunks they
+// were a fifth of the products and were formed again for every head.  Behind them one word per chunk: something is out of the split's range.
+template <int D>
+__global__ void __launch_bounds__(CK_THREADS)
+chunk_scores_kernel(const ScanArgs a, int64_t chunks) {
+  constexpr int RB = D * 2;
+  __shared__ __align__(128) __nv_bfloat16 q_s[CK_L * D], k_s[CK_L * D];
+  const int b = blockIdx.z, g = blockIdx.y, t0 = blockIdx.x * CK_L, len = a.seq_len[b];
+  if (len < a.min_len || t0 >= len) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t start = a.seq_start[b], number = chunk_number(start, t0, b) * a.G + g;
+  const __nv_bfloat16* qg = static_cast<const __nv_bfloat16*>(a.q) + start * a.ldq + static_cast<size_t>(g) * D;
+  const __nv_bfloat16* kg = static_cast<const __nv_bfloat16*>(a.k) + start * a.ldk + static_cast<size_t>(g) * D;
+  for (int idx = tid; idx < CK_L * (D / 8); idx += CK_THREADS) {
+    const int j = idx / (D / 8), ch = idx % (D / 8);
+    const bool ok = t0 + j < len;
+    const size_t row = ok ? t0 + j : 0;
+    cp_async_16(reinterpret_cast<unsigned char*>(q_s) + tile_off(j, ch, RB), qg + row * a.ldq + ch * 8, ok);
+    cp_async_16(reinterpret_cast<unsigned char*>(k_s) + tile_off(j, ch, RB), kg + row * a.ldk + ch * 8, ok);
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  uint32_t m = 0;
+  for (int i = tid; i < CK_L * D / 8; i += CK_THREADS) {
+    const uint4 x = reinterpret_cast<const uint4*>(q_s)[i], y = reinterpret_cast<const uint4*>(k_s)[i];
+    m = mag2(mag2(mag2(mag2(m, x.x), x.y), x.z), x.w);
+    m = mag2(mag2(mag2(mag2(m, y.x), y.y), y.z), y.w);
+  }
+  const int wild = __syncthreads_or((m & 0xffffu) >= CK_BIG_IN || (m >> 16) >= CK_BIG_IN);
+  if (tid == 0) reinterpret_cast<int*>(a.scores + chunks * a.G * CK_SCORES)[number] = wild;
+  float sc[8][4];
+  chunk_row_scores<D>(smem_u32(q_s), smem_u32(k_s), warp, lane, sc);
+  float4* out = reinterpret_cast<float4*>(a.scores + number * CK_SCORES) + warp * 8 * 32 + lane;
+#pragma unroll
+  for (int nt = 0; nt < 8; ++nt)
+    if (nt <= 2 * warp + 1) out[nt * 32] = make_float4(sc[nt][0], sc[nt][1], sc[nt][2], sc[nt][3]);
+}
+
+// AHEAD: chunk_scores_kernel has run
+template <int D, bool AHEAD>
 __global__ void __launch_bounds__(CK_THREADS, 2)
-linear_chunk_kernel(const ScanArgs a) {
+linear_chunk_kernel(const ScanArgs a, int64_t chunks) {
   constexpr int RB = D * 2, VB = CK_P * 2, MB = CK_L * 2, NT = D / 8;
   extern __shared__ __align__(128) unsigned char ck_smem[];
   ChunkTiles<D>& sm = *reinterpret_cast<ChunkTiles<D>*>(ck_smem);
@@ -158,7 +239,6 @@ linear_chunk_kernel(const ScanArgs a) {
 #pragma unroll
     for (int e = 0; e < 4; ++e) S[nt][e] = carried ? Sg[static_cast<size_t>(nt * 8 + c2 + (e & 1)) * dv + pr + 8 * (e >> 1)] : 0.f;
   const uint32_t m_u = smem_u32(sm.m);
-  const int ra = lane & 15, ca = lane >> 4;                                         // A rows / B rows by [n][k] and [k][n] tiles
   const int rb = (lane >> 4) * 8 + (lane & 7), cb = (lane >> 3) & 1;
   const int rt = ((lane >> 3) & 1) * 8 + (lane & 7), ct = lane >> 4;
   for (int t0 = 0, s = 0; t0 < len; t0 += CK_L, s ^= 1) {
@@ -166,16 +246,26 @@ linear_chunk_kernel(const ScanArgs a) {
     cp_async_wait<0>();
     // ---- this thread's share of the tiles and of the state within the range of the split?
     bool wild = false;
+    float4 ahead[AHEAD ? 8 : 1];
     {
       __syncthreads();                                                              // the chunk has landed; the previous one is consumed
       uint32_t m = 0;
-      const uint4* t4 = reinterpret_cast<const uint4*>(sm.q[s]);
-      for (int i = tid; i < CK_L * D / 8; i += CK_THREADS) { const uint4 x = t4[i]; m = mag2(mag2(mag2(mag2(m, x.x), x.y), x.z), x.w); }
-      t4 = reinterpret_cast<const uint4*>(sm.k[s]);
-      for (int i = tid; i < CK_L * D / 8; i += CK_THREADS) { const uint4 x = t4[i]; m = mag2(mag2(mag2(mag2(m, x.x), x.y), x.z), x.w); }
+      const uint4* t4;
+      if constexpr (AHEAD) {
+        const int64_t number = chunk_number(start, t0, b) * a.G + g;
+        wild = reinterpret_cast<const int*>(a.scores + chunks * a.G * CK_SCORES)[number] != 0;
+        const float4* sc = reinterpret_cast<const float4*>(a.scores + number * CK_SCORES) + warp * 8 * 32 + lane;
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt) ahead[nt] = nt <= 2 * warp + 1 ? sc[nt * 32] : make_float4(0.f, 0.f, 0.f, 0.f);
+      } else {
+        t4 = reinterpret_cast<const uint4*>(sm.q[s]);
+        for (int i = tid; i < CK_L * D / 8; i += CK_THREADS) { const uint4 x = t4[i]; m = mag2(mag2(mag2(mag2(m, x.x), x.y), x.z), x.w); }
+        t4 = reinterpret_cast<const uint4*>(sm.k[s]);
+        for (int i = tid; i < CK_L * D / 8; i += CK_THREADS) { const uint4 x = t4[i]; m = mag2(mag2(mag2(mag2(m, x.x), x.y), x.z), x.w); }
+      }
       t4 = reinterpret_cast<const uint4*>(sm.v[s]);
       for (int i = tid; i < CK_L * CK_P / 8; i += CK_THREADS) { const uint4 x = t4[i]; m = mag2(mag2(mag2(mag2(m, x.x), x.y), x.z), x.w); }
-      wild = (m & 0xffffu) >= CK_BIG_IN || (m >> 16) >= CK_BIG_IN || sm.wild[s];
+      wild = wild || (m & 0xffffu) >= CK_BIG_IN || (m >> 16) >= CK_BIG_IN || sm.wild[s];
       bool small = true;
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
@@ -214,35 +304,13 @@ linear_chunk_kernel(const ScanArgs a) {
     const uint32_t q_u = smem_u32(sm.q[s]), k_u = smem_u32(sm.k[s]), v_u = smem_u32(sm.v[s]);
     // ---- weights of rows 16 warp .. + 15: scores against the keys up to the diagonal, decay and write scale, in three parts
     if (warp * 16 < L) {
-      // the upper halves of q's significant bits give sums of 16 products that a float nearly always holds, the lower ones small sums:
-      // what the tensor core cuts off is a sixteenth (outputs 8.8e-8 -> 7.9e-8 from 64 bits, 12 of 574 us)
-      float sc[8][4], st[8][4];
+      float sc[8][4];
+      if constexpr (AHEAD) {
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) sc[nt][e] = st[nt][e] = 0.f;
-#pragma unroll
-      for (int ks = 0; ks < D / 16; ++ks) {
-        uint32_t af[4], hf[4], tf[4];
-        ldsm4(af, q_u + tile_off(warp * 16 + ra, ks * 2 + ca, RB));
-#pragma unroll
-        for (int e = 0; e < 4; ++e) halves(af[e], hf[e], tf[e]);
-#pragma unroll
-        for (int np = 0; np < 4; ++np) {
-          if (np <= warp) {
-            uint32_t bf[4];
-            ldsm4(bf, k_u + tile_off(np * 16 + rb, ks * 2 + cb, RB));
-            mma_bf16_16816(st[2 * np], tf, bf[0], bf[1]);
-            mma_bf16_16816(st[2 * np + 1], tf, bf[2], bf[3]);
-            mma_add(sc[2 * np], hf, bf[0], bf[1]);
-            mma_add(sc[2 * np + 1], hf, bf[2], bf[3]);
-          }
-        }
+        for (int nt = 0; nt < 8; ++nt) { sc[nt][0] = ahead[nt].x; sc[nt][1] = ahead[nt].y; sc[nt][2] = ahead[nt].z; sc[nt][3] = ahead[nt].w; }
+      } else {
+        chunk_row_scores<D>(q_u, k_u, warp, lane, sc);
       }
-#pragma unroll
-      for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) sc[nt][e] += st[nt][e];
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         const int i = warp * 16 + g4 + 8 * half;
@@ -409,7 +477,7 @@ linear_chunk_kernel(const ScanArgs a) {
 // token 1.13e-7 and 1.05e-7.  That takes the solve's sums beside the rows instead of in them (a row is rounded once at its own size and
 // not up to 64 times: outputs 1.57e-7 -> 1.14e-7, state 1.8e-7 -> 0.9e-7 together with norms formed in double) and the rest that the
 // tensor core cuts off the solution's products (1.14e-7 -> 1.05e-7, 7 us).  4 ragged sequences (4856 tokens, 16 heads of 128 x 128):
-// 493 us, token by token 1641 us.
+// 492 us with dot products and norms in the chain, 450 + 11 formed ahead once a key head (delta_dots_kernel), token by token 1641 us.
 // mma_add with what the tensor core cut off its sum (it keeps two bits behind a float's): the same product on top of minus the sum
 __device__ __forceinline__ void mma_add_rest(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
   float t[4] = {0.f, 0.f, 0.f, 0.f};
@@ -432,7 +500,101 @@ template <int D> struct DeltaTiles {
   int wild[2];
 };
 
+// The 16 x 16 blocks of the dot products, rows rblk and columns cblk, that warp (wp, wh) has: three for even wp, two for odd ones
+__device__ __forceinline__ void delta_block(int wp, int n, int& rblk, int& cblk) {
+  const bool extra = wp == 0 && n == 2;                    // warp 0's third block is the first one on the diagonal
+  rblk = extra ? 0 : wp == 0 ? 3 : wp == 1 ? 3 : wp == 2 ? 2 : 1;
+  cblk = extra ? 0 : (wp == 1 ? 2 : 0) + n;
+}
 template <int D>
+__device__ __forceinline__ void delta_block_dots(uint32_t x_u, uint32_t k_u, int rblk, int cblk, int lane, float sc[2][4]) {
+  constexpr int RB = D * 2;
+  const int ra = lane & 15, ca = lane >> 4, rb = (lane >> 4) * 8 + (lane & 7), cb = (lane >> 3) & 1;
+#pragma unroll
+  for (int w = 0; w < 2; ++w)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) sc[w][e] = 0.f;
+  uint32_t af[D / 16][4], bf[D / 16][4];
+#pragma unroll
+  for (int ks = 0; ks < D / 16; ++ks) {
+    ldsm4(af[ks], x_u + tile_off(rblk * 16 + ra, ks * 2 + ca, RB));
+    ldsm4(bf[ks], k_u + tile_off(cblk * 16 + rb, ks * 2 + cb, RB));
+  }
+#pragma unroll
+  for (int ks = 0; ks < D / 16; ++ks) {
+    mma_add(sc[0], af[ks], bf[ks][0], bf[ks][1]);
+    mma_add(sc[1], af[ks], bf[ks][2], bf[ks][3]);
+  }
+}
+// 1 / |row| (times the scale for queries) of row tid / 2 of the keys, then of the queries, on the even one of two threads; the largest
+// magnitude of what the thread has seen
+template <int D>
+__device__ __forceinline__ float delta_row_norm(const __nv_bfloat16* k, const __nv_bfloat16* q, int tid, float qscale, uint32_t& m) {
+  constexpr int RB = D * 2;
+  const int r = tid >> 1;
+  const unsigned char* row = reinterpret_cast<const unsigned char*>(r < CK_L ? k : q);
+  double ss = 0.0;
+#pragma unroll
+  for (int c = 0; c < D / 16; ++c) {
+    const uint4 x = *reinterpret_cast<const uint4*>(row + tile_off(r & (CK_L - 1), c * 2 + (tid & 1), RB));
+    m = mag2(mag2(mag2(mag2(m, x.x), x.y), x.z), x.w);
+    const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float f0 = bf16lo(w[e]), f1 = bf16hi(w[e]);
+      ss += static_cast<double>(f0 * f0);                  // exact: 16 significant bits
+      ss += static_cast<double>(f1 * f1);
+    }
+  }
+  ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+  return static_cast<float>((r < CK_L ? 1.0 : static_cast<double>(qscale)) / sqrt(ss + 1e-6));
+}
+
+// What a chunk's keys and queries alone say, formed once a key head where value heads or blocks of their columns share it: the dot products
+// as the warps of delta_chunk_kernel hold them ([warp][block][half] float4 a lane), the norms, and whether something is out of the split's range.
+constexpr int CK_DOTS_NORMS = 8 * 3 * 2 * 32 * 4, CK_DOTS = CK_DOTS_NORMS + 2 * CK_L + 4;
+template <int D>
+__global__ void __launch_bounds__(256)
+delta_dots_kernel(const ScanArgs a) {
+  constexpr int RB = D * 2;
+  __shared__ __align__(128) __nv_bfloat16 q_s[CK_L * D], k_s[CK_L * D];
+  const int b = blockIdx.z, g = blockIdx.y, t0 = blockIdx.x * CK_L, len = a.seq_len[b];
+  if (len < a.min_len || t0 >= len) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wp = warp & 3, wh = warp >> 2;
+  const int64_t start = a.seq_start[b];
+  const __nv_bfloat16* qg = static_cast<const __nv_bfloat16*>(a.q) + start * a.ldq + static_cast<size_t>(g) * D;
+  const __nv_bfloat16* kg = static_cast<const __nv_bfloat16*>(a.k) + start * a.ldk + static_cast<size_t>(g) * D;
+  for (int idx = tid; idx < CK_L * (D / 8); idx += 256) {
+    const int j = idx / (D / 8), ch = idx % (D / 8);
+    const bool ok = t0 + j < len;
+    const size_t row = ok ? t0 + j : 0;
+    cp_async_16(reinterpret_cast<unsigned char*>(q_s) + tile_off(j, ch, RB), qg + row * a.ldq + ch * 8, ok);
+    cp_async_16(reinterpret_cast<unsigned char*>(k_s) + tile_off(j, ch, RB), kg + row * a.ldk + ch * 8, ok);
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  float* at = a.scores + (chunk_number(start, t0, b) * a.G + g) * CK_DOTS;
+  uint32_t m = 0;
+  const float n = delta_row_norm<D>(k_s, q_s, tid, a.qscale, m);
+  if ((tid & 1) == 0) at[CK_DOTS_NORMS + (tid >> 1)] = n;  // keys, then queries
+  const int wild = __syncthreads_or((m & 0xffffu) >= CK_BIG_IN || (m >> 16) >= CK_BIG_IN);
+  if (tid == 0) at[CK_DOTS_NORMS + 2 * CK_L] = wild ? 1.f : 0.f;
+  float4* out = reinterpret_cast<float4*>(at) + warp * 6 * 32 + lane;
+#pragma unroll
+  for (int x = 0; x < 3; ++x) {
+    if (x == 2 && (wp & 1)) break;
+    int rblk, cblk;
+    delta_block(wp, x, rblk, cblk);
+    float sc[2][4];
+    delta_block_dots<D>(smem_u32(wh ? q_s : k_s), smem_u32(k_s), rblk, cblk, lane, sc);
+#pragma unroll
+    for (int w = 0; w < 2; ++w) out[(x * 2 + w) * 32] = make_float4(sc[w][0], sc[w][1], sc[w][2], sc[w][3]);
+  }
+}
+
+// AHEAD: delta_dots_kernel has run
+template <int D, bool AHEAD>
 __global__ void __launch_bounds__(256, 1)
 delta_chunk_kernel(const ScanArgs a) {
   using Sm = DeltaTiles<D>;
@@ -510,7 +672,6 @@ delta_chunk_kernel(const ScanArgs a) {
     fetch_coef(CK_L);
   }
   const uint32_t m_u = smem_u32(sm.m);
-  const int ra = lane & 15, ca = lane >> 4;
   const int rb = (lane >> 4) * 8 + (lane & 7), cb = (lane >> 3) & 1;
   const int rt = ((lane >> 3) & 1) * 8 + (lane & 7), ct = lane >> 4;
   for (int t0 = 0, s = 0; t0 < len; t0 += CK_L, s ^= 1) {
@@ -519,29 +680,26 @@ delta_chunk_kernel(const ScanArgs a) {
     __syncthreads();                                       // the chunk has landed; the previous one is consumed
     // ---- norms of k and q rows (two threads a row) and the range of everything that will be split
     bool wild = false;
+    float4 ahead[AHEAD ? 3 : 1][2];
     {
-      const int r = tid >> 1;
-      const unsigned char* row = reinterpret_cast<const unsigned char*>(r < CK_L ? sm.k[s] : sm.q[s]);
       uint32_t m = 0;
-      double ss = 0.0;
+      if constexpr (AHEAD) {
+        const float* at = a.scores + (chunk_number(start, t0, b) * a.G + g) * CK_DOTS;
+        const float4* sc = reinterpret_cast<const float4*>(at) + warp * 6 * 32 + lane;
 #pragma unroll
-      for (int c = 0; c < D / 16; ++c) {
-        const uint4 x = *reinterpret_cast<const uint4*>(row + tile_off(r & (CK_L - 1), c * 2 + (tid & 1), RB));
-        m = mag2(mag2(mag2(mag2(m, x.x), x.y), x.z), x.w);
-        const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+        for (int n = 0; n < 3; ++n)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float f0 = bf16lo(w[e]), f1 = bf16hi(w[e]);
-          ss += static_cast<double>(f0 * f0);              // exact: 16 significant bits
-          ss += static_cast<double>(f1 * f1);
-        }
+          for (int w = 0; w < 2; ++w) ahead[n][w] = n == 2 && (wp & 1) ? make_float4(0.f, 0.f, 0.f, 0.f) : sc[(n * 2 + w) * 32];
+        if (tid < CK_L) sm.kn[tid] = at[CK_DOTS_NORMS + tid];
+        else if (tid < 2 * CK_L) sm.qn[tid - CK_L] = at[CK_DOTS_NORMS + tid];
+        wild = at[CK_DOTS_NORMS + 2 * CK_L] != 0.f;
+      } else {
+        const float n = delta_row_norm<D>(sm.k[s], sm.q[s], tid, a.qscale, m);
+        if ((tid & 1) == 0) (tid < 2 * CK_L ? sm.kn[tid >> 1] : sm.qn[(tid >> 1) - CK_L]) = n;
       }
-      ss += __shfl_xor_sync(0xffffffffu, ss, 1);
-      if ((tid & 1) == 0)
-        (r < CK_L ? sm.kn[r] : sm.qn[r - CK_L]) = static_cast<float>((r < CK_L ? 1.0 : static_cast<double>(a.qscale)) / sqrt(ss + 1e-6));
       const uint4* v4 = reinterpret_cast<const uint4*>(sm.v[s]);
       for (int i = tid; i < CK_L * CK_P / 8; i += THREADS) { const uint4 x = v4[i]; m = mag2(mag2(mag2(mag2(m, x.x), x.y), x.z), x.w); }
-      wild = (m & 0xffffu) >= CK_BIG_IN || (m >> 16) >= CK_BIG_IN;
+      wild = wild || (m & 0xffffu) >= CK_BIG_IN || (m >> 16) >= CK_BIG_IN;
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -611,24 +769,18 @@ delta_chunk_kernel(const ScanArgs a) {
       fetch_coef(t0 + 2 * CK_L);
     }
     {
-      const int br = wp == 0 ? 3 : wp == 1 ? 3 : wp == 2 ? 2 : 1, b0 = wp == 1 ? 2 : 0;
       const uint32_t x_u = wh ? q_u : k_u;
 #pragma unroll
       for (int n = 0; n < 3; ++n) {
-        const bool extra = wp == 0 && n == 2;              // warp 0's third block is the first one on the diagonal
         if (n == 2 && (wp & 1)) break;
-        const int rblk = extra ? 0 : br, cblk = extra ? 0 : b0 + n;
-        float sc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-        uint32_t af[D / 16][4], bf[D / 16][4];
+        int rblk, cblk;
+        delta_block(wp, n, rblk, cblk);
+        float sc[2][4];
+        if constexpr (AHEAD) {
 #pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks) {
-          ldsm4(af[ks], x_u + tile_off(rblk * 16 + ra, ks * 2 + ca, RB));
-          ldsm4(bf[ks], k_u + tile_off(cblk * 16 + rb, ks * 2 + cb, RB));
-        }
-#pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks) {
-          mma_add(sc[0], af[ks], bf[ks][0], bf[ks][1]);
-          mma_add(sc[1], af[ks], bf[ks][2], bf[ks][3]);
+          for (int w = 0; w < 2; ++w) { sc[w][0] = ahead[n][w].x; sc[w][1] = ahead[n][w].y; sc[w][2] = ahead[n][w].z; sc[w][3] = ahead[n][w].w; }
+        } else {
+          delta_block_dots<D>(x_u, k_u, rblk, cblk, lane, sc);
         }
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
@@ -874,32 +1026,48 @@ int delta_walk_len(const ScanArgs& a, int n_seqs) {
   return ctas <= sms ? (n_seqs == 1 ? 24 : 28) : 40;
 }
 
-template <int D>
-static int go_linear(const char* what, const ScanArgs& a, int n_seqs, cudaStream_t st) {
+int64_t chunk_scores_floats(int n_tokens, int n_seqs, int G) {
+  return (static_cast<int64_t>(n_tokens) / CK_L + n_seqs + 1) * G * (CK_SCORES + 1);
+}
+
+template <int D, bool AHEAD>
+static int go_linear(const char* what, const ScanArgs& a, int n_seqs, int longest, int64_t chunks, cudaStream_t st) {
   constexpr int smem = static_cast<int>(sizeof(ChunkTiles<D>));
-  const cudaError_t e = cudaFuncSetAttribute(linear_chunk_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const cudaError_t e = cudaFuncSetAttribute(linear_chunk_kernel<D, AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return cuda_fail(e, what);
-  linear_chunk_kernel<D><<<dim3(a.dv / CK_P, a.H, n_seqs), CK_THREADS, smem, st>>>(a);
+  if constexpr (AHEAD) {
+    chunk_scores_kernel<D><<<dim3((longest + CK_L - 1) / CK_L, a.G, n_seqs), CK_THREADS, 0, st>>>(a, chunks);
+    B2_CHECK_LAUNCH(what);
+  }
+  linear_chunk_kernel<D, AHEAD><<<dim3(a.dv / CK_P, a.H, n_seqs), CK_THREADS, smem, st>>>(a, chunks);
   B2_CHECK_LAUNCH(what);
   return B2TTS_OK;
 }
 
-int launch_linear_chunk(const char* what, const ScanArgs& a, int n_seqs, cudaStream_t st) {
-  return a.d == 64 ? go_linear<64>(what, a, n_seqs, st) : go_linear<128>(what, a, n_seqs, st);
+int launch_linear_chunk(const char* what, const ScanArgs& a, int n_seqs, int longest, int64_t chunks, cudaStream_t st) {
+  if (a.scores == nullptr) return a.d == 64 ? go_linear<64, false>(what, a, n_seqs, longest, 0, st) : go_linear<128, false>(what, a, n_seqs, longest, 0, st);
+  return a.d == 64 ? go_linear<64, true>(what, a, n_seqs, longest, chunks, st) : go_linear<128, true>(what, a, n_seqs, longest, chunks, st);
 }
 
-template <int D>
-static int go_delta(const char* what, const ScanArgs& a, int n_seqs, cudaStream_t st) {
+int64_t delta_dots_floats(int n_tokens, int n_seqs, int G) { return (static_cast<int64_t>(n_tokens) / CK_L + n_seqs + 1) * G * CK_DOTS; }
+
+template <int D, bool AHEAD>
+static int go_delta(const char* what, const ScanArgs& a, int n_seqs, int longest, cudaStream_t st) {
   constexpr int smem = static_cast<int>(sizeof(DeltaTiles<D>));
-  const cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel<D, AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return cuda_fail(e, what);
-  delta_chunk_kernel<D><<<dim3(a.dv / CK_P, a.H, n_seqs), 256, smem, st>>>(a);
+  if constexpr (AHEAD) {
+    delta_dots_kernel<D><<<dim3((longest + CK_L - 1) / CK_L, a.G, n_seqs), 256, 0, st>>>(a);
+    B2_CHECK_LAUNCH(what);
+  }
+  delta_chunk_kernel<D, AHEAD><<<dim3(a.dv / CK_P, a.H, n_seqs), 256, smem, st>>>(a);
   B2_CHECK_LAUNCH(what);
   return B2TTS_OK;
 }
 
-int launch_delta_chunk(const char* what, const ScanArgs& a, int n_seqs, cudaStream_t st) {
-  return a.d == 64 ? go_delta<64>(what, a, n_seqs, st) : go_delta<128>(what, a, n_seqs, st);
+int launch_delta_chunk(const char* what, const ScanArgs& a, int n_seqs, int longest, cudaStream_t st) {
+  if (a.scores == nullptr) return a.d == 64 ? go_delta<64, false>(what, a, n_seqs, longest, st) : go_delta<128, false>(what, a, n_seqs, longest, st);
+  return a.d == 64 ? go_delta<64, true>(what, a, n_seqs, longest, st) : go_delta<128, true>(what, a, n_seqs, longest, st);
 }
 
 }  // namespace row

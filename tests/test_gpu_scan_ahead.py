@@ -1,0 +1,59 @@
+"""Prompt portions of the recurrences with what their keys and queries alone say formed ahead of the chain of chunks: the same numbers, to the
+bit, as formed inside it - chunk edges, several portions that share a chunk of rows, carried states, groups, and values out of the split's range
+(whose chunks are walked token by token)."""
+import pytest
+import torch
+
+from tests.lm_util import Lay as StepLay
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+SEQS = [[(0, 130)], [(9, 65), (0, 64), (5, 1), (0, 200), (0, 0), (3, 7), (0, 66)], [(0, 63), (0, 63), (0, 63), (700, 321)]]
+
+
+def _layout(seqs):
+    return StepLay([(c, n, list(range(20))) for c, n in seqs], 64, 20)
+
+
+def _both(run, state):
+    got = []
+    for ahead in (True, False):
+        s = state.clone()
+        got.append((run(s, ahead), s))
+    (a, sa), (b, sb) = got
+    same = lambda x, y: torch.equal(torch.nan_to_num(x, 1.5), torch.nan_to_num(y, 1.5)) and torch.equal(x.isnan(), y.isnan())
+    assert same(a, b) and same(sa, sb)
+    assert not torch.equal(sa, state)
+
+
+@pytest.mark.parametrize("seqs", SEQS)
+@pytest.mark.parametrize("big", [None, "q", "k", "v"])
+@pytest.mark.parametrize("N,H,G", [(128, 8, 2), (64, 4, 1)])
+def test_state_space(seqs, big, N, H, G):
+    import nano_qwen3tts_vllm_b200._native as nat
+    g = torch.Generator(device=DEV).manual_seed(N + len(seqs))
+    r = lambda *s: torch.randn(s, generator=g, device=DEV)
+    lay, P = _layout(seqs), 64
+    n = lay.n_tokens
+    x, dt = r(n, H * P + 2 * G * N).bfloat16(), r(n, H).bfloat16()
+    if big:
+        x[n // 2, {"v": 3, "k": H * P + 5, "q": H * P + G * N + N // 2}[big]] = float("inf") if big == "v" else 1e30
+    args, out = (r(H), 0.5 * r(H) - 0.5, r(H)), torch.empty(n, H * P, device=DEV)
+    _both(lambda s, ahead: (nat.ssm_scan(x, dt, *args, s, out.fill_(7), lay, H, G, P, N, ahead=ahead), out.clone())[1], r(len(seqs), H, N, P))
+
+
+@pytest.mark.parametrize("seqs", SEQS)
+@pytest.mark.parametrize("big", [None, "q", "k", "v"])
+@pytest.mark.parametrize("d,dv,H,G", [(128, 64, 4, 2), (64, 128, 2, 2)])
+def test_delta_rule(seqs, big, d, dv, H, G):
+    import nano_qwen3tts_vllm_b200._native as nat
+    g = torch.Generator(device=DEV).manual_seed(d + len(seqs))
+    r = lambda *s: torch.randn(s, generator=g, device=DEV)
+    lay = _layout(seqs)
+    n = lay.n_tokens
+    x, ba = r(n, 2 * G * d + H * dv).bfloat16(), r(n, 2 * H).bfloat16()
+    if big:
+        x[n // 2, {"q": 5, "k": G * d + d, "v": 2 * G * d + 3}[big]] = 1e30
+    args, out = (0.5 * r(H) - 0.5, r(H)), torch.empty(n, H * dv, device=DEV)
+    _both(lambda s, ahead: (nat.delta_rule_scan(x, ba[:, :H], ba[:, H:], *args, s, out.fill_(7), lay, H, G, d, dv, ahead=ahead), out.clone())[1],
+          r(len(seqs), H, d, dv))
