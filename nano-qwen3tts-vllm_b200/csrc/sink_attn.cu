@@ -321,7 +321,7 @@ sink_attn_decode_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, 
                         const int32_t* __restrict__ seq_start, const int32_t* __restrict__ seq_pos0,
                         const int32_t* __restrict__ seq_len, const int32_t* __restrict__ block_tables, int64_t bt_stride,
                         const float* __restrict__ sink, const T* __restrict__ gate, int64_t ldg, int gate_el, int H, int G, int Gv, int page,
-                        int mask_kind, int mask, int keep_first, float softcap, float scale, int out_f32) {
+                        int mask_kind, int mask, int keep_first, float softcap, float scale, int pad_rows, int out_f32) {
   constexpr int N = Vec16<T>::N, D = LPK * N, DV = D * VR, KPW = 32 / LPK;
   constexpr int S = SD_AHEAD * REP, OWN = S < LPK ? 1 : S / LPK, DUP = S < LPK ? LPK / S : 1;   // score r * SD_AHEAD + u: lane (. / OWN) * DUP
   constexpr float LOG2E = 1.4426950408889634f;
@@ -329,8 +329,12 @@ sink_attn_decode_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, 
   // the head groups of a sequence are neighbours in launch order: key heads that share a value head (v_heads < kv_heads)
   // run at the same time and the second reader finds the value rows in L2
   const int b = blockIdx.y;
-  if (seq_len[b] != 1) return;
   const int h0 = blockIdx.x * REP, g = h0 / (H / G);
+  if (pad_rows && seq_len[b] <= 0) {                      // padding row
+    const size_t o = (static_cast<size_t>(seq_start[b]) * H + h0) * DV;
+    for (int c = threadIdx.x; c < REP * DV; c += WARPS * 32) put_out(out, o + c, 0.f, out_f32);
+  }
+  if (seq_len[b] != 1) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int sub = lane % LPK, kg = lane / LPK;
   const size_t t = seq_start[b];
@@ -515,10 +519,10 @@ template <typename T, int LPK, int VR>
 static void launch_sink_decode(int rep, cudaStream_t st, const void* q, const void* kc, const void* vc, void* out,
                                const int32_t* seq_start, const int32_t* seq_pos0, const int32_t* seq_len, const int32_t* bt,
                                int64_t bt_stride, const float* sink, const void* gate, int64_t ldg, int gate_el, int n_seqs, int H, int G, int Gv,
-                               int page, int mask_kind, int mask, int keep_first, float softcap, float scale, int out_f32) {
+                               int page, int mask_kind, int mask, int keep_first, float softcap, float scale, int pad_rows, int out_f32) {
 #define SD_RUN(REP, WARPS) sink_attn_decode_kernel<T, LPK, REP, VR, WARPS><<<dim3(H / REP, n_seqs), WARPS * 32, 0, st>>>( \
       static_cast<const T*>(q), static_cast<const T*>(kc), static_cast<const T*>(vc), static_cast<T*>(out), seq_start, seq_pos0, seq_len, \
-      bt, bt_stride, sink, static_cast<const T*>(gate), ldg, gate_el, H, G, Gv, page, mask_kind, mask, keep_first, softcap, scale, out_f32)
+      bt, bt_stride, sink, static_cast<const T*>(gate), ldg, gate_el, H, G, Gv, page, mask_kind, mask, keep_first, softcap, scale, pad_rows, out_f32)
   // Eight warps a CTA as long as all CTAs are resident at once - two per multiprocessor, or one where the accumulators (REP * VR * N
   // floats a lane) take more than 128 registers - and four otherwise.  Float, 4 heads a group, d 64, dv 128, 64 sequences (256 CTAs of 168
   // registers), 1 / 200 / 600 keys: 11.3 / 17.8 / 38.9 us with eight warps in two waves, 6.8 / 13.1 / 33.5 with four.
@@ -538,11 +542,11 @@ template <typename T>
 static bool launch_sink_decode_any(int d, int dv, int rep, cudaStream_t st, const void* q, const void* kc, const void* vc, void* out,
                                    const int32_t* seq_start, const int32_t* seq_pos0, const int32_t* seq_len, const int32_t* bt,
                                    int64_t bt_stride, const float* sink, const void* gate, int64_t ldg, int gate_el, int n_seqs, int H, int G, int Gv,
-                                   int page, int mask_kind, int mask, int keep_first, float softcap, float scale, int out_f32) {
+                                   int page, int mask_kind, int mask, int keep_first, float softcap, float scale, int pad_rows, int out_f32) {
   constexpr int N = Vec16<T>::N;
   if ((dv != d && dv != 2 * d) || d % N != 0) return false;
   const bool wide = dv == 2 * d;
-#define SD_ARGS rep, st, q, kc, vc, out, seq_start, seq_pos0, seq_len, bt, bt_stride, sink, gate, ldg, gate_el, n_seqs, H, G, Gv, page, mask_kind, mask, keep_first, softcap, scale, out_f32
+#define SD_ARGS rep, st, q, kc, vc, out, seq_start, seq_pos0, seq_len, bt, bt_stride, sink, gate, ldg, gate_el, n_seqs, H, G, Gv, page, mask_kind, mask, keep_first, softcap, scale, pad_rows, out_f32
   switch (d / N) {
     case 4: if (wide) launch_sink_decode<T, 4, 2>(SD_ARGS); else launch_sink_decode<T, 4, 1>(SD_ARGS); return true;
     case 8: if (wide) launch_sink_decode<T, 8, 2>(SD_ARGS); else launch_sink_decode<T, 8, 1>(SD_ARGS); return true;
@@ -890,19 +894,22 @@ extern "C" int b2tts_sink_attn_rows(const void* q, const void* k_cache, const vo
     }
   }
   // one-token rows: the row-splitting kernel where the head size fits it (path 1 keeps everything in the plain kernel)
+  // A step of one-token sequences, a row each, needs no more than that kernel, which then zeroes the padding rows as well (the plain kernel's
+  // launch, whose CTAs all had nothing else to do, took 2.4 us of 88 with 64 sequences).
+  const bool alone = max_new == 1 && n_tokens == n_seqs;
   bool split = false;
   if (path != 1 && aligned16(q) && n_seqs > 0) {
     if (dtype == B2TTS_DTYPE_BF16)
       split = launch_sink_decode_any<__nv_bfloat16>(dim, vdim, heads / kv_heads, st, q, k_cache, v_cache, out, seq_start, seq_pos0, seq_len,
                                                     block_tables, bt_stride, sink, gate, ldg, gate_el, n_seqs, heads, kv_heads, v_heads, page, mask_kind,
-                                                    mask, keep_first, softcap, scale, out_f32);
+                                                    mask, keep_first, softcap, scale, alone, out_f32);
     else
       split = launch_sink_decode_any<float>(dim, vdim, heads / kv_heads, st, q, k_cache, v_cache, out, seq_start, seq_pos0, seq_len,
                                             block_tables, bt_stride, sink, gate, ldg, gate_el, n_seqs, heads, kv_heads, v_heads, page, mask_kind, mask,
-                                            keep_first, softcap, scale, out_f32);
+                                            keep_first, softcap, scale, alone, out_f32);
     if (split) B2_CHECK_LAUNCH("sink_attn (one-token rows)");
   }
-  if (use_mma && split) return B2TTS_OK;             // every sequence has its kernel (padding rows come with one-token steps only)
+  if (split && (use_mma || alone)) return B2TTS_OK;  // every sequence has its kernel (padding rows come with one-token steps only)
   const int skip = (use_mma ? 1 : 0) | (split ? 2 : 0);
   if (dtype == B2TTS_DTYPE_BF16)
     launch_sink_plain_rep<__nv_bfloat16>(heads / kv_heads, st, q, k_cache, v_cache, out, tok_seq, positions, seq_len, block_tables,

@@ -66,3 +66,31 @@ def test_sizes(nat, dtype, lanes, rep, many):
 def test_masks_pages_and_caps(nat, page, mask, keep, cap, sink):
     for lens in ([0, 5, 200, 333], [0, 5, 200, 333, 70, 129] * 30):
         _check(nat, lens, BF, rep=2, G=2, d=128, wide=False, page=page, mask=mask, keep=keep, cap=cap, sink=sink, seed=page + mask)
+
+
+@pytest.mark.parametrize("dtype,out_dtype", [(BF, torch.float32), (BF, BF), (torch.float32, torch.float32)])
+@pytest.mark.parametrize("rep,wide", [(1, False), (2, False), (4, True)])
+def test_padding_rows_are_zeroed_and_empty_sequences_leave_the_others_alone(nat, dtype, out_dtype, rep, wide):
+    from tests.lm_util import Lay
+    G, d, page = 2, 64, 16
+    H, dv = rep * G, d * (2 if wide else 1)
+    gd = torch.Generator(device=DEV).manual_seed(rep)
+    r = lambda *s: torch.randn(s, generator=gd, device=DEV)
+    kc, vc = r(9, page, G * d).to(dtype), r(9, page, G * dv).to(dtype)
+    q, sk = r(5, H * d).to(dtype), r(H)
+
+    def run(lay, rows):
+        out = torch.full((len(rows), H * dv), math.nan, dtype=out_dtype, device=DEV)
+        nat.sink_attn(q[rows].contiguous(), kc, vc, out, lay, sk, None, H, G, d, dv, page, nat.MASK_WINDOW, 0, d ** -0.5)
+        return out
+
+    live = {1: (40, 1, [1, 2, 3]), 3: (3, 1, [4])}
+    ref = run(Lay([live[1], live[3]], page, 3), [1, 3])
+    padded = run(Lay([(0, 0, [0]), live[1], (0, 0, [0]), live[3], (0, 0, [0])], page, 3), [0, 1, 2, 3, 4])
+    assert torch.equal(padded[[1, 3]], ref) and (padded[[0, 2, 4]] == 0).all()
+    lay = Lay([live[1], live[3]], page, 3)                     # a sequence without tokens and without a row between them
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    lay.seq_start, lay.seq_pos0, lay.seq_len, lay.seq_slot = i32([0, 1, 1]), i32([40, 0, 3]), i32([1, 0, 1]), i32([0, 1, 2])
+    lay.tok_seq, lay.n_seqs = i32([0, 2]), 3
+    lay.block_tables = lay.block_tables[[0, 0, 1]].contiguous()
+    assert torch.equal(run(lay, [1, 3]), ref)
