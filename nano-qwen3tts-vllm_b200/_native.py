@@ -1160,8 +1160,10 @@ def sink_attn(q, k_cache, v_cache, out, lay, sink, gate, heads, kv_heads, dim, v
     assert k_cache.dtype == q.dtype and v_cache.dtype == q.dtype and out.dtype in (q.dtype, F32) and out.is_contiguous()
     assert gate is None or (gate.dtype == q.dtype and gate.stride(1) == 1)
     vh = kv_heads if v_heads is None else v_heads
-    # how many rows the caches have bounds the copies of the prompt kernel; a view that skips memory has no such number
-    rows = min(k_cache.numel() // (kv_heads * dim), v_cache.numel() // (vh * vdim)) if k_cache.is_contiguous() and v_cache.is_contiguous() else 0
+    # how many rows the caches have bounds the copies of the prompt kernel (one-token steps have none); a view that skips memory has no such number
+    rows = 0
+    if lay.max_new > 1 and k_cache.is_contiguous() and v_cache.is_contiguous():
+        rows = min(k_cache.numel() // (kv_heads * dim), v_cache.numel() // (vh * vdim))
     _check(_load().b2tts_sink_attn_rows(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), lay.tok_seq.data_ptr(),
                                         lay.positions.data_ptr(), lay.seq_start.data_ptr(), lay.seq_pos0.data_ptr(), lay.seq_len.data_ptr(),
                                         lay.block_tables.data_ptr(), lay.block_tables.stride(0), _ptr(sink), _ptr(gate),
@@ -1210,13 +1212,23 @@ def _coef(out, heads):
     return torch.empty(out.shape[0], heads, 3, dtype=F32, device=out.device)
 
 
-def ssm_scan(xbc, dt_in, dt_bias, a_log, d_skip, state, out, lay, heads, groups, vdim, nstate, ahead=True):
+# The longest portion from which what keys and queries alone say is formed by a launch of its own.  That launch and its scratch cost the host 6 to 8 us
+# and each 64 tokens of the chain give back 1 to 2; layers of 1, 2, 4 and 8 portions, in the chain / ahead of it in us.  State space: 192 tokens
+# 70 75 87 160 / 75 78 85 149, 256 tokens 85 90 108 200 / 82 88 103 185.  Delta rule: 128 tokens 69 72 71 94 / 76 91 79 95, 256 tokens
+# 85 91 94 172 / 85 90 95 169, 384 tokens 115 120 130 252 / 113 118 130 240.
+SSM_AHEAD_FROM, DELTA_AHEAD_FROM = 256, 384
+
+
+def ssm_scan(xbc, dt_in, dt_bias, a_log, d_skip, state, out, lay, heads, groups, vdim, nstate, ahead=None):
     """xbc [n, heads*vdim + 2*groups*nstate] (convolved, activated); dt_in: a column slice [n, heads]; state float
-    [slots, heads, nstate, vdim]; out float [n, heads*vdim].  ``ahead``: long portions' scores are formed once a group of heads."""
+    [slots, heads, nstate, vdim]; out float [n, heads*vdim].  ``ahead``: portions' scores are formed once a
+    group of heads (None: where that is faster)."""
     dt = _act(xbc, "xbc")
     _cuda(state, F32, "state"); _cuda(out, F32, "out")
     assert dt_in.dtype == xbc.dtype and dt_in.stride(1) == 1 and state.is_contiguous() and out.is_contiguous()
     max_new, scores = getattr(lay, "max_new", 0), None
+    if ahead is None:
+        ahead = max_new >= SSM_AHEAD_FROM
     if ahead and max_new > 64 and dt == DTYPE_CODE[BF16] and heads >= 4 * groups:
         scores = torch.empty(_load().b2tts_ssm_scan_ahead_floats(lay.n_tokens, lay.n_seqs, groups), dtype=F32, device=xbc.device)
     _check(_load().b2tts_ssm_scan_ahead(xbc.data_ptr(), xbc.stride(0), dt_in.data_ptr(), dt_in.stride(0), dt_bias.data_ptr(),
@@ -1225,14 +1237,16 @@ def ssm_scan(xbc, dt_in, dt_bias, a_log, d_skip, state, out, lay, heads, groups,
                                         dt, _ptr(scores), 0 if scores is None else scores.numel(), _stream()), "ssm_scan")
 
 
-def delta_rule_scan(qkv, beta_in, a_in, a_log, dt_bias, state, out, lay, heads, kv_heads, dim, vdim, ahead=True):
-    """qkv [n, 2*kv_heads*dim + heads*vdim] (convolved, activated); beta_in, a_in: column slices [n, heads] of one tensor.  ``ahead``: what long
-    portions' keys and queries alone say is formed once a key head."""
+def delta_rule_scan(qkv, beta_in, a_in, a_log, dt_bias, state, out, lay, heads, kv_heads, dim, vdim, ahead=None):
+    """qkv [n, 2*kv_heads*dim + heads*vdim] (convolved, activated); beta_in, a_in: column slices [n, heads] of one tensor.  ``ahead``: what
+    portions' keys and queries alone say is formed once a key head (None: where that is faster)."""
     dt = _act(qkv, "qkv")
     _cuda(state, F32, "state"); _cuda(out, F32, "out")
     assert beta_in.dtype == qkv.dtype and a_in.dtype == qkv.dtype and beta_in.stride(0) == a_in.stride(0)
     assert state.is_contiguous() and out.is_contiguous()
     max_new, dots = getattr(lay, "max_new", 0), None
+    if ahead is None:
+        ahead = max_new >= DELTA_AHEAD_FROM
     if ahead and max_new > 64 and dt == DTYPE_CODE[BF16] and heads * vdim >= 128 * kv_heads:
         dots = torch.empty(_load().b2tts_delta_rule_scan_ahead_floats(lay.n_tokens, lay.n_seqs, kv_heads), dtype=F32, device=qkv.device)
     _check(_load().b2tts_delta_rule_scan_ahead(qkv.data_ptr(), qkv.stride(0), beta_in.data_ptr(), a_in.data_ptr(), beta_in.stride(0),
