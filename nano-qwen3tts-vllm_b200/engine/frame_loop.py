@@ -292,11 +292,15 @@ class DeviceFrameLoop:
         """[frames, streams, 16] int64 on the host (synchronises).  Rows of a stream beyond its ``frame_counts()``
         entry (EOS) are padding."""
         n = int(self.frame_idx.item())
-        return self.frames[:n].cpu()
+        frames = self.frames[:n].cpu()
+        nat.check_waits()
+        return frames
 
     def frame_counts(self) -> list[int]:
         """Frames produced per stream (a stream stops at its codec EOS unless ``ignore_eos``)."""
-        return self.frames_done.tolist()
+        counts = self.frames_done.tolist()
+        nat.check_waits()
+        return counts
 
     def result_per_stream(self) -> list[torch.Tensor]:
         fr, counts = self.result(), self.frame_counts()

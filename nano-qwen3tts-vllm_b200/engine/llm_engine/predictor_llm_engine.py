@@ -3,6 +3,7 @@ from __future__ import annotations
 
 import torch
 
+from ... import _native as nat
 from ...sampling_params import SamplingParams
 from ..model_runner.predictor_model_runner import PredictorModelRunner
 from ..scheduler import PredictorScheduler
@@ -67,6 +68,7 @@ class PredictorLLMEngine(LLMEngine):
     def _burst_collect(self, launched):
         seqs, host, done = launched
         done.synchronize()                                                   # the one synchronisation of the burst
+        nat.check_waits()
         toks = host.tolist()
         for s, row in zip(seqs, toks):
             s.token_ids.extend(row)
@@ -106,6 +108,7 @@ class PredictorLLMEngine(LLMEngine):
             return
         sizes = [int(t.numel()) for t in steps]
         flat = torch.cat(steps).tolist()                                     # the one synchronisation of the burst
+        nat.check_waits()
         offs = [0]
         for n in sizes:
             offs.append(offs[-1] + n)

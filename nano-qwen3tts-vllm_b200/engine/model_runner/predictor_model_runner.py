@@ -168,6 +168,7 @@ class PredictorModelRunner(ModelRunner):
         temperatures = self.layout.d["temperatures"][:len(seqs)] if not is_prefill else self.prepare_sample(seqs)
         token_ids = self.sampler(logits, temperatures, top_k=self.top_k).tolist()
         reset_context()
+        nat.check_waits()
         return token_ids
 
     @torch.inference_mode()

@@ -8,6 +8,7 @@ from __future__ import annotations
 import numpy as np
 import torch
 
+from ... import _native as nat
 from ...models.qwen3_tts_talker import Qwen3TTSTalkerForCausalLM
 from ...utils.context import reset_context
 from ..sequence import Sequence
@@ -153,6 +154,7 @@ class TalkerModeModelRunner(ModelRunner):
     def run_collect(self, launched):
         host, done, hidden = launched
         done.synchronize()                                                                      # the step's one device sync
+        nat.check_waits()                              # behind replayed graphs too, which pass no launch's own check
         return host.tolist(), hidden
 
     def run(self, seqs: list[Sequence], is_prefill: bool):
