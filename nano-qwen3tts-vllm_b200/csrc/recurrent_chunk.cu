@@ -149,8 +149,13 @@ __device__ __forceinline__ void chunk_row_scores(uint32_t q_u, uint32_t k_u, int
     for (int e = 0; e < 4; ++e) sc[nt][e] += st[nt][e];
 }
 
-// Which chunk of the step's: the chunks of sequence b, which starts at row `start`, have numbers of their own.
-__device__ __forceinline__ int64_t chunk_number(int64_t start, int t0, int b) { return (start + t0) / CK_L + b; }
+// The chunks of the sequences in front of sequence b, which its own are numbered behind: wherever the sequences' rows lie, no two
+// chunks of a step share a number.  All 32 lanes of a warp call it.
+__device__ __forceinline__ int chunks_before(const int32_t* seq_len, int b, int lane) {
+  int n = 0;
+  for (int i = lane; i < b; i += 32) n += (max(seq_len[i], 0) + CK_L - 1) / CK_L;
+  return __reduce_add_sync(0xffffffffu, n);
+}
 constexpr int CK_SCORES = CK_L * CK_L;     // floats of a chunk's scores, as the threads hold them: [warp][nt][lane] float4
 
 // The scores of every chunk and group of heads, formed once where many heads share their queries and keys: in the chain of chunks they
@@ -163,7 +168,7 @@ chunk_scores_kernel(const ScanArgs a, int64_t chunks) {
   const int b = blockIdx.z, g = blockIdx.y, t0 = blockIdx.x * CK_L, len = a.seq_len[b];
   if (len < a.min_len || t0 >= len) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t start = a.seq_start[b], number = chunk_number(start, t0, b) * a.G + g;
+  const int64_t start = a.seq_start[b], number = static_cast<int64_t>(chunks_before(a.seq_len, b, lane) + t0 / CK_L) * a.G + g;
   const __nv_bfloat16* qg = static_cast<const __nv_bfloat16*>(a.q) + start * a.ldq + static_cast<size_t>(g) * D;
   const __nv_bfloat16* kg = static_cast<const __nv_bfloat16*>(a.k) + start * a.ldk + static_cast<size_t>(g) * D;
   for (int idx = tid; idx < CK_L * (D / 8); idx += CK_THREADS) {
@@ -229,6 +234,8 @@ linear_chunk_kernel(const ScanArgs a, int64_t chunks) {
   };
   load_chunk(0, 0);
   cp_async_commit();
+  int chunk0 = 0;                                          // number of the sequence's first chunk
+  if constexpr (AHEAD) chunk0 = chunks_before(a.seq_len, b, lane);
   if (warp == 3) chunk_scalars<D>(sm, 0, cp, H, 0, len, lane);
   // S^T fragments: value columns pr (+ 8), key channels nt * 8 + c2 (+ 1)
   const int pr = warp * 16 + g4;
@@ -252,7 +259,7 @@ linear_chunk_kernel(const ScanArgs a, int64_t chunks) {
       uint32_t m = 0;
       const uint4* t4;
       if constexpr (AHEAD) {
-        const int64_t number = chunk_number(start, t0, b) * a.G + g;
+        const int64_t number = static_cast<int64_t>(chunk0 + t0 / CK_L) * a.G + g;
         wild = reinterpret_cast<const int*>(a.scores + chunks * a.G * CK_SCORES)[number] != 0;
         const float4* sc = reinterpret_cast<const float4*>(a.scores + number * CK_SCORES) + warp * 8 * 32 + lane;
 #pragma unroll
@@ -574,7 +581,7 @@ delta_dots_kernel(const ScanArgs a) {
   cp_async_commit();
   cp_async_wait<0>();
   __syncthreads();
-  float* at = a.scores + (chunk_number(start, t0, b) * a.G + g) * CK_DOTS;
+  float* at = a.scores + (static_cast<int64_t>(chunks_before(a.seq_len, b, lane) + t0 / CK_L) * a.G + g) * CK_DOTS;
   uint32_t m = 0;
   const float n = delta_row_norm<D>(k_s, q_s, tid, a.qscale, m);
   if ((tid & 1) == 0) at[CK_DOTS_NORMS + (tid >> 1)] = n;  // keys, then queries
@@ -630,6 +637,8 @@ delta_chunk_kernel(const ScanArgs a) {
   };
   load_chunk(0, 0);
   cp_async_commit();
+  int chunk0 = 0;                                          // number of the sequence's first chunk
+  if constexpr (AHEAD) chunk0 = chunks_before(a.seq_len, b, lane);
   const int pr = wp * 16 + g4, n0 = wh * CH;               // S^T fragments: value columns pr (+ 8), key channels n0 + nt * 8 + c2 (+ 1)
   float S[NT][4];
   const bool carried = a.seq_pos0[b] > 0;
@@ -684,7 +693,7 @@ delta_chunk_kernel(const ScanArgs a) {
     {
       uint32_t m = 0;
       if constexpr (AHEAD) {
-        const float* at = a.scores + (chunk_number(start, t0, b) * a.G + g) * CK_DOTS;
+        const float* at = a.scores + (static_cast<int64_t>(chunk0 + t0 / CK_L) * a.G + g) * CK_DOTS;
         const float4* sc = reinterpret_cast<const float4*>(at) + warp * 6 * 32 + lane;
 #pragma unroll
         for (int n = 0; n < 3; ++n)

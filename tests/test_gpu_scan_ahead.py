@@ -57,3 +57,28 @@ def test_delta_rule(seqs, big, d, dv, H, G):
     args, out = (0.5 * r(H) - 0.5, r(H)), torch.empty(n, H * dv, device=DEV)
     _both(lambda s, ahead: (nat.delta_rule_scan(x, ba[:, :H], ba[:, H:], *args, s, out.fill_(7), lay, H, G, d, dv, ahead=ahead), out.clone())[1],
           r(len(seqs), H, d, dv))
+
+
+def _out_of_order(seqs, order):
+    """The same rows, described sequence by sequence in another order: starts no longer ascend."""
+    lay = _layout(seqs)
+    p = torch.tensor(order, device=DEV)
+    for name in ("seq_start", "seq_pos0", "seq_len", "seq_slot", "block_tables"):
+        setattr(lay, name, getattr(lay, name)[p].contiguous())
+    lay.tok_seq = torch.argsort(p)[lay.tok_seq.long()].to(torch.int32)
+    return lay
+
+
+@pytest.mark.parametrize("seqs,order", [([(0, 512), (0, 512)], [1, 0]), ([(9, 64), (0, 64), (0, 0), (5, 320), (0, 200)], [3, 2, 0, 4, 1])])
+def test_rows_that_do_not_lie_in_the_order_of_the_sequences(seqs, order):
+    """Chunks of two sequences must not share a place in the scratch (chunk 8 of one was the last of the other)."""
+    import nano_qwen3tts_vllm_b200._native as nat
+    g = torch.Generator(device=DEV).manual_seed(len(seqs))
+    r = lambda *s: torch.randn(s, generator=g, device=DEV)
+    lay, H, G, d = _out_of_order(seqs, order), 4, 1, 64
+    n = lay.n_tokens
+    x, dt, args, out = r(n, H * d + 2 * G * d).bfloat16(), r(n, H).bfloat16(), (r(H), 0.5 * r(H) - 0.5, r(H)), torch.empty(n, H * d, device=DEV)
+    _both(lambda s, ahead: (nat.ssm_scan(x, dt, *args, s, out.fill_(7), lay, H, G, d, d, ahead=ahead), out.clone())[1], r(len(seqs), H, d, d))
+    x, ba, args = r(n, 2 * G * d + H * d).bfloat16(), r(n, 2 * H).bfloat16(), (0.5 * r(H) - 0.5, r(H))
+    _both(lambda s, ahead: (nat.delta_rule_scan(x, ba[:, :H], ba[:, H:], *args, s, out.fill_(7), lay, H, G, d, d, ahead=ahead), out.clone())[1],
+          r(len(seqs), H, d, d))
