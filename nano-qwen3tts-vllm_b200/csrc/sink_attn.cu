@@ -321,7 +321,7 @@ sink_attn_decode_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, 
                         const int32_t* __restrict__ seq_start, const int32_t* __restrict__ seq_pos0,
                         const int32_t* __restrict__ seq_len, const int32_t* __restrict__ block_tables, int64_t bt_stride,
                         const float* __restrict__ sink, const T* __restrict__ gate, int64_t ldg, int gate_el, int H, int G, int Gv, int page,
-                        int mask_kind, int mask, int keep_first, float softcap, float scale, int pad_rows, int out_f32) {
+                        int mask_kind, int mask, int keep_first, float softcap, float scale, const int32_t* __restrict__ pad_seq, int out_f32) {
   constexpr int N = Vec16<T>::N, D = LPK * N, DV = D * VR, KPW = 32 / LPK;
   constexpr int S = SD_AHEAD * REP, OWN = S < LPK ? 1 : S / LPK, DUP = S < LPK ? LPK / S : 1;   // score r * SD_AHEAD + u: lane (. / OWN) * DUP
   constexpr float LOG2E = 1.4426950408889634f;
@@ -330,11 +330,16 @@ sink_attn_decode_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, 
   // run at the same time and the second reader finds the value rows in L2
   const int b = blockIdx.y;
   const int h0 = blockIdx.x * REP, g = h0 / (H / G);
-  if (pad_rows && seq_len[b] <= 0) {                      // padding row
-    const size_t o = (static_cast<size_t>(seq_start[b]) * H + h0) * DV;
+  // pad_seq: the sequence of every row, where the step's rows are as many as its sequences; this CTA also zeroes ROW b where the
+  // sequence of that row brings no token.  Where an empty sequence starts means nothing.
+  auto zero_row = [&] {
+    const size_t o = (static_cast<size_t>(b) * H + h0) * DV;
     for (int c = threadIdx.x; c < REP * DV; c += WARPS * 32) put_out(out, o + c, 0.f, out_f32);
+  };
+  if (seq_len[b] != 1) {
+    if (pad_seq != nullptr && seq_len[pad_seq[b]] <= 0) zero_row();
+    return;
   }
-  if (seq_len[b] != 1) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int sub = lane % LPK, kg = lane / LPK;
   const size_t t = seq_start[b];
@@ -462,6 +467,7 @@ sink_attn_decode_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, 
     m[r] = __shfl_sync(0xffffffffu, m_own, r * SD_AHEAD / OWN * DUP, LPK);
     l[r] = __shfl_sync(0xffffffffu, l_own, r * SD_AHEAD / OWN * DUP, LPK);
   }
+  const bool pad = pad_seq != nullptr && seq_len[pad_seq[b]] <= 0;
   // the lane groups of the warp
 #pragma unroll
   for (int o = LPK; o < 32; o <<= 1) {
@@ -513,16 +519,17 @@ sink_attn_decode_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, 
       put_out(out, obase + c, o * inv, out_f32);
     }
   }
+  if (pad) zero_row();
 }
 
 template <typename T, int LPK, int VR>
 static void launch_sink_decode(int rep, cudaStream_t st, const void* q, const void* kc, const void* vc, void* out,
                                const int32_t* seq_start, const int32_t* seq_pos0, const int32_t* seq_len, const int32_t* bt,
                                int64_t bt_stride, const float* sink, const void* gate, int64_t ldg, int gate_el, int n_seqs, int H, int G, int Gv,
-                               int page, int mask_kind, int mask, int keep_first, float softcap, float scale, int pad_rows, int out_f32) {
+                               int page, int mask_kind, int mask, int keep_first, float softcap, float scale, const int32_t* pad_seq, int out_f32) {
 #define SD_RUN(REP, WARPS) sink_attn_decode_kernel<T, LPK, REP, VR, WARPS><<<dim3(H / REP, n_seqs), WARPS * 32, 0, st>>>( \
       static_cast<const T*>(q), static_cast<const T*>(kc), static_cast<const T*>(vc), static_cast<T*>(out), seq_start, seq_pos0, seq_len, \
-      bt, bt_stride, sink, static_cast<const T*>(gate), ldg, gate_el, H, G, Gv, page, mask_kind, mask, keep_first, softcap, scale, pad_rows, out_f32)
+      bt, bt_stride, sink, static_cast<const T*>(gate), ldg, gate_el, H, G, Gv, page, mask_kind, mask, keep_first, softcap, scale, pad_seq, out_f32)
   // Eight warps a CTA as long as all CTAs are resident at once - two per multiprocessor, or one where the accumulators (REP * VR * N
   // floats a lane) take more than 128 registers - and four otherwise.  Float, 4 heads a group, d 64, dv 128, 64 sequences (256 CTAs of 168
   // registers), 1 / 200 / 600 keys: 11.3 / 17.8 / 38.9 us with eight warps in two waves, 6.8 / 13.1 / 33.5 with four.
@@ -542,11 +549,11 @@ template <typename T>
 static bool launch_sink_decode_any(int d, int dv, int rep, cudaStream_t st, const void* q, const void* kc, const void* vc, void* out,
                                    const int32_t* seq_start, const int32_t* seq_pos0, const int32_t* seq_len, const int32_t* bt,
                                    int64_t bt_stride, const float* sink, const void* gate, int64_t ldg, int gate_el, int n_seqs, int H, int G, int Gv,
-                                   int page, int mask_kind, int mask, int keep_first, float softcap, float scale, int pad_rows, int out_f32) {
+                                   int page, int mask_kind, int mask, int keep_first, float softcap, float scale, const int32_t* pad_seq, int out_f32) {
   constexpr int N = Vec16<T>::N;
   if ((dv != d && dv != 2 * d) || d % N != 0) return false;
   const bool wide = dv == 2 * d;
-#define SD_ARGS rep, st, q, kc, vc, out, seq_start, seq_pos0, seq_len, bt, bt_stride, sink, gate, ldg, gate_el, n_seqs, H, G, Gv, page, mask_kind, mask, keep_first, softcap, scale, pad_rows, out_f32
+#define SD_ARGS rep, st, q, kc, vc, out, seq_start, seq_pos0, seq_len, bt, bt_stride, sink, gate, ldg, gate_el, n_seqs, H, G, Gv, page, mask_kind, mask, keep_first, softcap, scale, pad_seq, out_f32
   switch (d / N) {
     case 4: if (wide) launch_sink_decode<T, 4, 2>(SD_ARGS); else launch_sink_decode<T, 4, 1>(SD_ARGS); return true;
     case 8: if (wide) launch_sink_decode<T, 8, 2>(SD_ARGS); else launch_sink_decode<T, 8, 1>(SD_ARGS); return true;
@@ -894,19 +901,20 @@ extern "C" int b2tts_sink_attn_rows(const void* q, const void* k_cache, const vo
     }
   }
   // one-token rows: the row-splitting kernel where the head size fits it (path 1 keeps everything in the plain kernel)
-  // A step of one-token sequences, a row each, needs no more than that kernel, which then zeroes the padding rows as well (the plain kernel's
+  // A step of one-token sequences with as many rows needs no more than that kernel, which then zeroes the padding rows as well (the plain kernel's
   // launch, whose CTAs all had nothing else to do, took 2.4 us of 88 with 64 sequences).
   const bool alone = max_new == 1 && n_tokens == n_seqs;
+  const int32_t* pad_seq = alone ? tok_seq : nullptr;
   bool split = false;
   if (path != 1 && aligned16(q) && n_seqs > 0) {
     if (dtype == B2TTS_DTYPE_BF16)
       split = launch_sink_decode_any<__nv_bfloat16>(dim, vdim, heads / kv_heads, st, q, k_cache, v_cache, out, seq_start, seq_pos0, seq_len,
                                                     block_tables, bt_stride, sink, gate, ldg, gate_el, n_seqs, heads, kv_heads, v_heads, page, mask_kind,
-                                                    mask, keep_first, softcap, scale, alone, out_f32);
+                                                    mask, keep_first, softcap, scale, pad_seq, out_f32);
     else
       split = launch_sink_decode_any<float>(dim, vdim, heads / kv_heads, st, q, k_cache, v_cache, out, seq_start, seq_pos0, seq_len,
                                             block_tables, bt_stride, sink, gate, ldg, gate_el, n_seqs, heads, kv_heads, v_heads, page, mask_kind, mask,
-                                            keep_first, softcap, scale, alone, out_f32);
+                                            keep_first, softcap, scale, pad_seq, out_f32);
     if (split) B2_CHECK_LAUNCH("sink_attn (one-token rows)");
   }
   if (split && (use_mma || alone)) return B2TTS_OK;  // every sequence has its kernel (padding rows come with one-token steps only)

@@ -94,3 +94,29 @@ def test_padding_rows_are_zeroed_and_empty_sequences_leave_the_others_alone(nat,
     lay.tok_seq, lay.n_seqs = i32([0, 2]), 3
     lay.block_tables = lay.block_tables[[0, 0, 1]].contiguous()
     assert torch.equal(run(lay, [1, 3]), ref)
+
+
+@pytest.mark.parametrize("dtype", [BF, torch.float32])
+@pytest.mark.parametrize("lens,tok_seq", [([1, 0, 1], [0, 2, 1]), ([0, 1, 1, 0], [1, 2, 0, 3]), ([1, 0, 0, 1], [1, 0, 3, 2])])
+def test_padding_rows_lie_where_their_tokens_say(nat, dtype, lens, tok_seq):
+    """A row is padding where its own sequence brings no token; where empty sequences start - here a running sum, which names other sequences'
+    rows, or a number beyond all rows - means nothing."""
+    from tests.lm_util import Lay
+    G, d, page, H, n = 2, 64, 16, 4, len(lens)
+    gd = torch.Generator(device=DEV).manual_seed(n)
+    r = lambda *s: torch.randn(s, generator=gd, device=DEV)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    kc, vc, q, sk = r(9, page, G * d).to(dtype), r(9, page, G * d).to(dtype), r(n, H * d).to(dtype), r(H)
+    cached = [40 - 9 * b for b in range(n)]
+    lay = Lay([(c, 1, [1 + b, 4 + b, 2]) for b, c in enumerate(cached)], page, 3)
+    run = lambda rows, lay: (nat.sink_attn(q[rows].contiguous(), kc, vc, o := torch.full((len(rows), H * d), math.nan, dtype=dtype, device=DEV), lay, sk, None,
+                                           H, G, d, d, page, nat.MASK_WINDOW, 0, d ** -0.5), o)[1]
+    row_of = {b: t for t, b in enumerate(tok_seq)}
+    ref = run([row_of[b] for b in range(n)], lay)                # every sequence with a token, in order
+    for starts in ([sum(lens[:b]) for b in range(n)], [1 << 20] * n):
+        lay.seq_len, lay.tok_seq = i32(lens), i32(tok_seq)
+        lay.seq_start = i32([row_of[b] if m else starts[b] for b, m in enumerate(lens)])
+        lay.positions = i32([cached[b] for b in tok_seq])
+        out = run(list(range(n)), lay)
+        for b, m in enumerate(lens):
+            assert torch.equal(out[row_of[b]], ref[b]) if m else bool((out[row_of[b]] == 0).all()), (b, starts)
