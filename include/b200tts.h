@@ -679,7 +679,7 @@ B2TTS_API int b2tts_ssm_scan_portions(const void* xbc, int64_t ldx, const void* 
                                       const int32_t* seq_pos0, const int32_t* seq_len, const int32_t* seq_slot, int n_tokens, int n_seqs,
                                       int max_new, int heads, int groups, int vdim, int dim, int dtype, void* stream);
 /* The same with room for the scores of long portions' queries and keys (_floats() of them, 16-byte aligned; null: none), which are then
- * formed once a group of heads instead of once a head.  The results are the same numbers. */
+ * formed once a group of heads instead of once a head.  The results are the same numbers; the sequences' rows may lie in any order. */
 B2TTS_API size_t b2tts_ssm_scan_ahead_floats(int n_tokens, int n_seqs, int groups);
 B2TTS_API int b2tts_ssm_scan_ahead(const void* xbc, int64_t ldx, const void* dt, int64_t lddt, const float* dt_bias, const float* a_log,
                                       const float* d_skip, float* state, float* coef, float* out, const int32_t* seq_start,
@@ -691,7 +691,7 @@ B2TTS_API int b2tts_delta_rule_scan_portions(const void* qkv, int64_t ldq, const
                                              const int32_t* seq_slot, int n_tokens, int n_seqs, int max_new, int heads, int kv_heads, int dim,
                                              int vdim, int dtype, void* stream);
 /* The same with room for what long portions' keys and queries alone say (_floats() of them, 16-byte aligned; null: none), formed once a key
- * head.  The results are the same numbers. */
+ * head.  The results are the same numbers; rows in any order. */
 B2TTS_API size_t b2tts_delta_rule_scan_ahead_floats(int n_tokens, int n_seqs, int kv_heads);
 B2TTS_API int b2tts_delta_rule_scan_ahead(const void* qkv, int64_t ldq, const void* beta, const void* a_in, int64_t ldu,
                                              const float* a_log, const float* dt_bias, float* state, float* coef, float* out,

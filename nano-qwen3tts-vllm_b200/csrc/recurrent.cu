@@ -387,7 +387,8 @@ extern "C" int b2tts_ssm_scan_ahead(const void* xbc, int64_t ldx, const void* dt
                  "ssm_scan: %zu floats for scores (or unaligned)", scores_floats);
       a.scores = scores;
     }
-    const int rc = launch_linear_chunk("ssm_scan (portions)", a, n_seqs, longest, static_cast<int64_t>(n_tokens) / 64 + n_seqs + 1, st);
+    // the ahead kernel's grid: without a bound on the portions one of them may have all rows (empty sequences have none)
+    const int rc = launch_linear_chunk("ssm_scan (portions)", a, n_seqs, max_new > 0 ? max_new : n_tokens, static_cast<int64_t>(n_tokens) / 64 + n_seqs + 1, st);
     if (rc != B2TTS_OK || alone) return rc;
     a.min_len = 1; a.max_len = walk;                       // single tokens and short portions beside them
   }
@@ -451,7 +452,7 @@ extern "C" int b2tts_delta_rule_scan_ahead(const void* qkv, int64_t ldq, const v
                  "delta_rule_scan: %zu floats for dot products (or unaligned)", dots_floats);
       a.scores = dots;
     }
-    const int rc = launch_delta_chunk("delta_rule_scan (portions)", a, n_seqs, longest, st);
+    const int rc = launch_delta_chunk("delta_rule_scan (portions)", a, n_seqs, max_new > 0 ? max_new : n_tokens, st);     // as above
     if (rc != B2TTS_OK || alone) return rc;
     a.min_len = 1; a.max_len = walk;                       // single tokens and short portions beside them
   }

@@ -82,3 +82,33 @@ def test_rows_that_do_not_lie_in_the_order_of_the_sequences(seqs, order):
     x, ba, args = r(n, 2 * G * d + H * d).bfloat16(), r(n, 2 * H).bfloat16(), (0.5 * r(H) - 0.5, r(H))
     _both(lambda s, ahead: (nat.delta_rule_scan(x, ba[:, :H], ba[:, H:], *args, s, out.fill_(7), lay, H, G, d, d, ahead=ahead), out.clone())[1],
           r(len(seqs), H, d, d))
+
+
+@pytest.mark.parametrize("lens", [[200] + [0] * 99, [0] * 40 + [130] + [0] * 30 + [70, 1]])
+def test_portions_of_unknown_length_beside_empty_sequences(lens):
+    """Without max_new the longest portion is not n_tokens - n_seqs + 1: empty sequences need no row."""
+    import nano_qwen3tts_vllm_b200._native as nat
+    g = torch.Generator(device=DEV).manual_seed(len(lens))
+    r = lambda *s: torch.randn(s, generator=g, device=DEV)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    n, b, H, d, L, st = sum(lens), len(lens), 4, 64, nat.lib(), torch.cuda.current_stream().cuda_stream
+    seq = [i32([sum(lens[:i]) for i in range(b)]), i32([0] * b), i32(lens), i32(list(range(b)))]
+    ptrs, out, coef = [t.data_ptr() for t in seq], torch.empty(n, H * d, device=DEV), torch.empty(n, H, 3, device=DEV)
+    x, dt, par = r(n, H * d + 2 * d).bfloat16(), r(n, H).bfloat16(), (r(H), 0.5 * r(H) - 0.5, r(H))
+    y, ba, par2 = r(n, 2 * d + H * d).bfloat16(), r(n, 2 * H).bfloat16(), (0.5 * r(H) - 0.5, r(H))
+
+    def ssm(s, ahead):
+        room = torch.full((L.b2tts_ssm_scan_ahead_floats(n, b, 1),), 3.0, device=DEV)
+        assert L.b2tts_ssm_scan_ahead(x.data_ptr(), x.stride(0), dt.data_ptr(), H, *[t.data_ptr() for t in par], s.data_ptr(), coef.data_ptr(),
+                                      out.fill_(7).data_ptr(), *ptrs, n, b, 0, H, 1, d, d, nat.DTYPE_CODE[torch.bfloat16],
+                                      room.data_ptr() if ahead else None, room.numel(), st) == 0
+        return out.clone()
+
+    def delta(s, ahead):
+        room = torch.full((L.b2tts_delta_rule_scan_ahead_floats(n, b, 1),), 3.0, device=DEV)
+        assert L.b2tts_delta_rule_scan_ahead(y.data_ptr(), y.stride(0), ba.data_ptr(), ba[:, H:].data_ptr(), 2 * H, *[t.data_ptr() for t in par2],
+                                             s.data_ptr(), coef.data_ptr(), out.fill_(7).data_ptr(), *ptrs, n, b, 0, H, 1, d, d,
+                                             nat.DTYPE_CODE[torch.bfloat16], room.data_ptr() if ahead else None, room.numel(), st) == 0
+        return out.clone()
+    _both(ssm, r(b, H, d, d))
+    _both(delta, r(b, H, d, d))
