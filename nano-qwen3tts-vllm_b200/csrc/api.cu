@@ -43,9 +43,9 @@ static int* wait_words() {
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;             // the first launch may be a captured one
     void* p = nullptr;
     cudaThreadExchangeStreamCaptureMode(&mode);
-    if (cudaHostAlloc(&p, WAITS_KINDS * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) p = nullptr;
+    if (cudaHostAlloc(&p, WAIT_DEVICES * WAITS_KINDS * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) p = nullptr;
     cudaThreadExchangeStreamCaptureMode(&mode);
-    for (int i = 0; p != nullptr && i < WAITS_KINDS; ++i) static_cast<volatile int*>(p)[i] = 0;
+    for (int i = 0; p != nullptr && i < WAIT_DEVICES * WAITS_KINDS; ++i) static_cast<volatile int*>(p)[i] = 0;
     return static_cast<int*>(p);
   }();
   return words;
@@ -57,17 +57,19 @@ int* wait_word(int kind) {
   int* words = wait_words();
   if (words == nullptr) return nullptr;
   __atomic_store_n(&g_words, words, __ATOMIC_RELEASE);
-  return words + kind;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  return words + wait_slot(dev, kind);
 }
 
 int wait_count(int kind) {
   const int* words = __atomic_load_n(&g_words, __ATOMIC_ACQUIRE);
-  return words != nullptr ? static_cast<const volatile int*>(words)[kind] : 0;
+  return words != nullptr ? wait_total(words, kind) : 0;
 }
 
 int wait_check(int kind, const char* what) {
-  const int n = wait_count(kind);
-  if (__atomic_exchange_n(&g_told[kind], n, __ATOMIC_RELAXED) == n) return B2TTS_OK;
+  const int* words = __atomic_load_n(&g_words, __ATOMIC_ACQUIRE);
+  if (words == nullptr || !wait_moved(words, kind, &g_told[kind])) return B2TTS_OK;
   set_error("%s: a wait inside an earlier %s ran out, its results are not valid", what,
             kind == WAITS_GROUPED ? "grouped product" : "attention over prompt portions");
   return B2TTS_ECUDA;
