@@ -14,8 +14,10 @@
 //   loader    queries (one box of 64 columns x HPC heads x tokens per slice), keys and values as boxes of R rows inside pages;
 //   cleaner   zeros the value rows of a tile that no query of the item sees (behind the last key, before the window): their weights are
 //             zero, but what a page holds there may be infinite.
-// The running maximum is lazy: O and the sum are rescaled only when a row's maximum has grown by more than 2^8; weights are then up to
-// 2^8, which floats and bf16 pairs hold as well as 1.
+// A row's maximum is the running one: where one key has most of the weight, its weight is then 1 and carries no rounding.  (A lazy one, moved in steps
+// of 2^8, left it a weight with a rounding of its own: outputs of 2000 peaked keys 1.21 times as far from 64 bits with weights
+// rounded once, 1.9 times with pairs in float.  O is scaled more often for it: layers 2 % longer.)  The sum is that of the weights as the
+// products see them, rounded, so that what rounding adds to all of them cancels.
 //
 // Bound: the issue of the tensor core's products.  A key tile of a row tile is 24 of them of 64 cycles (1536); the issuer's own instructions and
 // barriers between two tiles make that about 2300, and the weights (64 exponents, splits and sums a thread) are ready before that.  An item
@@ -563,8 +565,8 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
             mx = fmaxf(fmaxf(x0, x1), fmaxf(x2, x3));
           }
           mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16)) * f;
-          // ---- the running maximum moves in steps of more than 2^8.  These scores were issued behind the last weight products, so O is at rest
-          const bool grow = mx > m + (first ? 0.f : 8.f);
+          // ---- the running maximum.  These scores were issued behind the last weight products, so O is at rest
+          const bool grow = mx > m;
           if (__any_sync(0xffffffffu, grow)) {
             const float n = grow ? mx : m, alpha = po_ex2(m - n);
             m = n;
@@ -583,7 +585,7 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
           }
           first = false;
         }
-        // ---- weights, their sum, and their bf16 parts, in place of the scores
+        // ---- weights, their bf16 parts in place of the scores, and the sum of those: pairs' remainders in sb, minus the rounded weights in sa
         const uint64_t f2 = po_pair(f, f), m2 = po_pair(-m, -m);
         uint64_t sa = 0, sb = 0;
 #pragma unroll 1
@@ -617,17 +619,22 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
               w0 = po_ex2(w0); w1 = po_ex2(w1); w2 = po_ex2(w2); w3 = po_ex2(w3);
             }
             const uint64_t wa = po_pair(w0, w1), wb = po_pair(w2, w3);
-            if constexpr (!SIG) {
-              sa = po_add2(sa, wa);
-              sb = po_add2(sb, wb);
-            }
             const uint32_t p0 = pack_bf16(w0, w1), p1 = pack_bf16(w2, w3);
             if constexpr (MODE != PO_ROUNDED) {
               const uint32_t n0 = p0 ^ 0x80008000u, n1 = p1 ^ 0x80008000u;
-              po_split(po_add2(wa, po_pair(bf16lo(n0), bf16hi(n0))), r0, r1);
-              po_split(po_add2(wb, po_pair(bf16lo(n1), bf16hi(n1))), r2, r3);
-              rest[c / 2] = pack_bf16(r0, r1);
-              rest[c / 2 + 1] = pack_bf16(r2, r3);
+              const uint64_t h0 = po_pair(bf16lo(n0), bf16hi(n0)), h1 = po_pair(bf16lo(n1), bf16hi(n1));
+              po_split(po_add2(wa, h0), r0, r1);
+              po_split(po_add2(wb, h1), r2, r3);
+              const uint32_t q0 = pack_bf16(r0, r1), q1 = pack_bf16(r2, r3);
+              if constexpr (!SIG) {
+                sa = po_add2(po_add2(sa, h0), h1);
+                sb = po_add2(po_add2(sb, po_pair(bf16lo(q0), bf16hi(q0))), po_pair(bf16lo(q1), bf16hi(q1)));
+              }
+              rest[c / 2] = q0;
+              rest[c / 2 + 1] = q1;
+            } else {
+              sa = po_add2(sa, po_pair(bf16lo(p0), bf16hi(p0)));
+              sb = po_add2(sb, po_pair(bf16lo(p1), bf16hi(p1)));
             }
             hi[c / 2] = p0;
             hi[c / 2 + 1] = p1;
@@ -636,7 +643,7 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
           if constexpr (MODE != PO_ROUNDED) po_st16<HK>(tm_s + part + 16, rest);
         }
         float s0, s1;
-        po_split(po_add2(sa, sb), s0, s1);
+        po_split(po_add2(MODE == PO_PAIRS ? sa ^ 0x8000000080000000ull : sa, sb), s0, s1);
         l += s0 + s1;
         po_st_wait();
         tc_fence_before();

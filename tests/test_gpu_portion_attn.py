@@ -166,6 +166,47 @@ def test_prompts_that_are_their_own_keys(nat, H, G, lens):
     assert nat.portion_attn_timeouts() == 0
 
 
+@pytest.mark.parametrize("sharp", [0.3, 1, 3, 10])
+def test_prompts_are_no_further_from_64_bits_than_tile_by_tile(nat, sharp):
+    """Weights rounded once: as far from 64 bits as the kernel for starts of their own, whose largest weight of a row is exact.  (A maximum behind
+    the true one leaves that weight a rounding, and a sum of weights before rounding does not take it back: 1.2 times as far.)"""
+    n, H, G, d = 1500, 4, 2, 128
+    g = torch.Generator(device=DEV).manual_seed(int(sharp * 10))
+    r = lambda *s: torch.randn(s, generator=g, device=DEV)
+    q, k, v = (r(n, H, d) * sharp).to(BF), r(n, G, d).to(BF), r(n, G, d).to(BF)
+    cu = torch.tensor([0, n], dtype=torch.int32, device=DEV)
+    s = torch.einsum("ihd,jhd->hij", q.to(F64), k.to(F64).repeat_interleave(H // G, 1)) * d ** -0.5
+    ref = torch.einsum("hij,jhd->ihd", s.masked_fill(torch.ones(n, n, device=DEV).tril() == 0, -math.inf).softmax(-1), v.to(F64).repeat_interleave(H // G, 1))
+    err = [((nat.varlen_attn_prefill(q, k, v, cu, c, n, n, d ** -0.5).view(n, H, d).to(F64) - ref).norm() / ref.norm()).item() for c in (cu, cu.clone())]
+    assert err[0] < 1.01 * err[1], err
+
+
+@pytest.mark.parametrize("sharp", [0.3, 1, 4])
+@pytest.mark.parametrize("mask,cap", [(0, 0.0), (64, 0.0), (0, 5.0)])
+def test_float_outputs_are_no_further_from_64_bits_than_on_the_other_kernel(nat, sharp, mask, cap):
+    """Weights in pairs, outputs in float: the same roundings as the kernel for short sequences, so the same error (1 to 3e-6 here); a fifth
+    of it is left for sums in another order."""
+    from tests.lm_util import Lay
+    n, H, G, d, page = 1000, 4, 2, 128, 64
+    g = torch.Generator(device=DEV).manual_seed(mask + int(sharp * 10))
+    r = lambda *s: torch.randn(s, generator=g, device=DEV)
+    pages = -(-n // page)
+    q, kc, vc = (r(n, H * d) * sharp).to(BF), r(pages, page, G * d).to(BF), r(pages, page, G * d).to(BF)
+    k, v = (t.view(-1, G, d)[:n].to(F64).repeat_interleave(H // G, 1) for t in (kc, vc))
+    s = torch.einsum("ihd,jhd->hij", q.to(F64).view(n, H, d), k) * d ** -0.5
+    s = cap * torch.tanh(s / cap) if cap else s
+    dist = torch.arange(n, device=DEV)[:, None] - torch.arange(n, device=DEV)[None]
+    ok = (dist >= 0) & ((dist < mask) if mask else True)
+    ref, err = torch.einsum("hij,jhd->ihd", s.masked_fill(~ok, -math.inf).softmax(-1), v).reshape(n, -1), []
+    for known in (0, 1):                                             # 1: said to be short, which is the other kernel's
+        lay = Lay([(0, n, list(range(pages)))], page, pages)
+        lay.max_keys = known
+        out = torch.empty(n, H * d, device=DEV)
+        nat.sink_attn(q, kc, vc, out, lay, None, None, H, G, d, d, page, nat.MASK_WINDOW, mask, d ** -0.5, softcap=cap)
+        err.append(((out.to(F64) - ref).norm() / ref.norm()).item())
+    assert err[0] < 1.2 * err[1], err
+
+
 @pytest.mark.parametrize("keys", [420, 421])
 def test_sigmoid_weights_of_sequences_that_the_host_knows_of(nat, keys):
     _sigmoid_case(nat, [(keys - 40, 40), (0, 33)], 4, 2, 64, 90, page=16, known=True)
