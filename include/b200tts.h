@@ -473,8 +473,8 @@ B2TTS_API int b2tts_window_sigmoid_attn(const void* q, const void* k_cache, cons
                                         const int32_t* block_tables, int bt_stride, const float* r1, const float* r2,
                                         const float* pb, int n_seqs, int max_new, int heads, int kv_heads, int dim, int vdim,
                                         int page, int window, float scale, int dtype, void* stream);
-/* The same, told how many rows q has, how many rows (pages times page) both caches have, and how many keys the longest sequence has (0: not
- * known); see b2tts_sink_attn_rows. */
+/* The same, told how many rows q has, how many rows (pages times page) both caches have, and how many keys the longest sequence with more
+ * than one new token has (0: not known); see b2tts_sink_attn_rows. */
 B2TTS_API int b2tts_window_sigmoid_attn_rows(const void* q, const void* k_cache, const void* v_cache, void* out,
                                         const int32_t* seq_start, const int32_t* seq_pos0, const int32_t* seq_len,
                                         const int32_t* block_tables, int bt_stride, const float* r1, const float* r2,
@@ -617,8 +617,8 @@ B2TTS_API int b2tts_sink_attn(const void* q, const void* k_cache, const void* v_
                               int n_tokens, int n_seqs, int max_new, int heads, int kv_heads, int v_heads, int dim, int vdim,
                               int page, int mask_kind, int mask, int keep_first, float softcap, float scale, int dtype, int path,
                               int out_f32, void* stream);
-/* The same, told how many rows (pages times page) both caches have and how many keys the longest sequence has (0: not known).  Prompt
- * portions with head sizes of 64 or 128 and pages of a multiple of 16 then run on the tcgen05 kernel (csrc/portion_attn.cu), whose copies
+/* The same, told how many rows (pages times page) both caches have and how many keys the longest sequence with more than one new token
+ * has (0: not known).  Prompt portions with head sizes of 64 or 128 and pages of a multiple of 16 then run on the tcgen05 kernel (csrc/portion_attn.cu), whose copies
  * are bounded by the rows; steps whose longest sequence is known to be short stay with the other one. */
 B2TTS_API int b2tts_sink_attn_rows(const void* q, const void* k_cache, const void* v_cache, void* out, const int32_t* tok_seq,
                               const int32_t* positions, const int32_t* seq_start, const int32_t* seq_pos0, const int32_t* seq_len,

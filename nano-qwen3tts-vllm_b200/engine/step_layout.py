@@ -97,7 +97,8 @@ class MixedStepLayout:
             self.events[self.cur] = ev
         self.n_tokens, self.n_seqs, self.n_want = o, n_seqs, len(want_rows)
         self.max_new = max((n for _, n in items), default=0)
-        self.max_keys = max((seq.num_cached_tokens + n for seq, n in items), default=0)    # 0: not known on the host
+        # of the portions: one-token sequences have kernels of their own, and their contexts say nothing about these; 0: not known on the host
+        self.max_keys = max((seq.num_cached_tokens + n for seq, n in items if n > 1), default=0)
         # (tokens cached, tokens new) per live row on the host: what sizes a launch or a buffer of the step
         self.portions = [(seq.num_cached_tokens, n) for seq, n in items]
         self._bind()
