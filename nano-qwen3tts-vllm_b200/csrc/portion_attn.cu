@@ -683,7 +683,7 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
             const float u = e & 1 ? bf16hi(w[e >> 1]) : bf16lo(w[e >> 1]);
-            o[e] = __float_as_uint(__fdividef(__uint_as_float(o[e]), 1.0f + expf(-u)));
+            o[e] = __float_as_uint(__uint_as_float(o[e]) * sigmoid_f(u));
           }
         }
         if (tk <= t_last && a.out_f32) {

@@ -207,6 +207,21 @@ def test_float_outputs_are_no_further_from_64_bits_than_on_the_other_kernel(nat,
     assert err[0] < 1.2 * err[1], err
 
 
+def test_element_gates_in_float(nat):
+    """A token that sees itself alone: value times gate, also where the gate leaves next to nothing on (an approximate division answers 0 there).  A few
+    roundings of 2^-23, and of 2^-149 where results are that small."""
+    from tests.lm_util import Lay
+    n, H, G, d, page = 200, 4, 2, 64, 16
+    g = torch.Generator(device=DEV).manual_seed(1)
+    r = lambda *s: torch.randn(s, generator=g, device=DEV).to(BF)
+    pages = -(-n // page)
+    q, kc, vc = r(n, H * d), r(pages, page, G * d), r(pages, page, G * d)
+    gate, out = torch.linspace(-88.5, 88, n * H * d, device=DEV).to(BF).view(n, H * d), torch.empty(n, H * d, device=DEV)
+    nat.sink_attn(q, kc, vc, out, Lay([(0, n, list(range(pages)))], page, pages), None, gate, H, G, d, d, page, nat.MASK_WINDOW, 1, d ** -0.5, gate_el=True)
+    ref = vc.view(-1, G, d)[:n].repeat_interleave(H // G, 1).reshape(n, -1).to(F64) * torch.sigmoid(gate.to(F64))
+    assert bool(((out - ref).abs() <= ref.abs() * 2 ** -20 + 2 ** -146).all())
+
+
 @pytest.mark.parametrize("keys", [420, 421])
 def test_sigmoid_weights_of_sequences_that_the_host_knows_of(nat, keys):
     _sigmoid_case(nat, [(keys - 40, 40), (0, 33)], 4, 2, 64, 90, page=16, known=True)
