@@ -1,11 +1,11 @@
 #!/usr/bin/env python
-"""bench.py - codec frames/s of the Qwen3-TTS decode hot path (BASELINE.json metric).
+"""bench.py - codec frames/s of the Qwen3-TTS decode hot path.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--streams B] [--impl ours|reference]
 
 A STEP is one codec frame (16 codes) for every stream: 1 talker decode pass (28 layers) + 1 predictor
 prefill (2 tokens/stream) + 14 predictor decode passes (5 layers) + samplers + the 16-codebook embedding
-sum.  Workload: Qwen3-TTS-12Hz-1.7B shapes (SURVEY.md section 7.0), random-init bf16 weights, B concurrent
+sum.  Workload: Qwen3-TTS-12Hz-1.7B shapes, random-init bf16 weights, B concurrent
 synthetic streams with a 64-token prompt, top-k 50 sampling at T=1.0/0.9, EOS ignored.
 
   value     frames/s with everything resident in HBM: one CUDA-graph launch per frame (DeviceFrameLoop)
@@ -13,13 +13,13 @@ synthetic streams with a 64-token prompt, top-k 50 sampling at T=1.0/0.9, EOS ig
             with HOST buffers crossing both ways every frame (StepApiFrameLoop)
   roofline  the dominant kernel (weight-streaming tcgen05 GEMM) + roofline_kernels for every other kernel of the path
   reference_kernels   cuBLAS / flash-attn / Triton on the same shapes, timed the same way (bench_kernels.py)
-  other_workloads     1 / 8 / 128 / 256 / 512 streams;  icl_workload = BASELINE configs[3] (4k-token prompts)
+  other_workloads     1 / 8 / 128 / 256 / 512 streams;  icl_workload = voice-clone prompts of 4k tokens
   prompt_prep         f3: prompt assembly for a 64-request burst and for one 4096-frame ICL request
   cpu_baseline   the CPU oracle (port of the reference's torch path) on the host cores, bounded sample
 
 N > 1: independent per-GPU replicas (no collective on the data path); barrier + max-over-ranks timing.
 `--impl reference` times the oracle port on the host cores (the reference's own modules need
-/root/reference, which does not exist on the GPU box).
+its source tree).
 """
 from __future__ import annotations
 
@@ -51,8 +51,8 @@ def parse():
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--cpu-streams", type=int, default=0, help="streams of the CPU legs (0 = the same as --streams)")
     ap.add_argument("--also-streams", default="1,8,128,256,512",
-                    help="extra stream counts reported under other_workloads (BASELINE configs[1], [2], [4])")
-    ap.add_argument("--no-icl", action="store_true", help="skip the BASELINE configs[3] leg (4k-token prompts, 8 streams)")
+                    help="extra stream counts reported under other_workloads")
+    ap.add_argument("--no-icl", action="store_true", help="skip the voice-clone leg (4k-token prompts, 8 streams)")
     ap.add_argument("--no-reference-kernels", action="store_true")
     ap.add_argument("--lm", action="store_true",
                     help="instead of the frame benchmark: prefill / decode throughput of the Bokenex decoder beside the talker "
@@ -175,7 +175,7 @@ def synthetic_prompts(streams: int, hidden: int, pinned: bool, prompt_len: int =
 
 
 def frame_bytes(mc, lens_sum: float) -> float:
-    """Algorithmic HBM bytes of one frame for all streams (SURVEY.md section 8d): every weight matrix streamed
+    """Algorithmic HBM bytes of one frame for all streams: every weight matrix streamed
     once per pass + the talker's KV read."""
     t, p = mc.talker, mc.predictor
 
@@ -221,7 +221,7 @@ def _graph_ms(fn, launches: int, iters: int = 3):
 
 
 def time_attention_long(device, streams: int = 64, ctx_len: int = 4096, layers: int = 3):
-    """paged_attn_kernel at the north-star shape (~4k-token KV): `streams` sequences of `ctx_len`
+    """paged_attn_kernel at the voice-clone shape (~4k-token KV): `streams` sequences of `ctx_len`
     cached tokens, scattered pages, `layers` launches over different caches (each 2 x streams x ctx_len x 2 KiB)."""
     import torch
     import nano_qwen3tts_vllm_b200._native as nat
@@ -417,8 +417,8 @@ def reference_arm(a):
 
 
 def time_prompt_prep(device):
-    """Prompt assembly for (a) 64 simultaneous arrivals of ~20-word prompts (BASELINE configs[4]'s admission burst) and
-    (b) one voice-clone ICL request with a 4096-frame reference (configs[3]); random-init embeddings at the 1.7B widths
+    """Prompt assembly for (a) 64 simultaneous arrivals of ~20-word prompts (an admission burst) and
+    (b) one voice-clone ICL request with a 4096-frame reference; random-init embeddings at the 1.7B widths
     (text 151936 x 2048 -> hidden 2048).  CUDA events around the public call, host planning included."""
     import types
     import torch
@@ -471,7 +471,7 @@ def time_prompt_prep(device):
 
 def workload_config(a, streams):
     return {"workload": f"Qwen3-TTS-12Hz-{a.model} talker+code-predictor, {streams} concurrent streams per GPU "
-                        f"(BASELINE configs[4]; configs[1]/[2] = 1/8 streams under other_workloads), prompt {PROMPT_LEN} tokens, "
+                        f"(1/8 streams under other_workloads), prompt {PROMPT_LEN} tokens, "
                         f"random-init weights, top-k 50 sampling T=1.0/0.9, EOS ignored, paged KV block 256",
             "streams_per_gpu": streams, "prompt_len": PROMPT_LEN, "frame": "1 talker decode + predictor prefill + 14 predictor decodes",
             "l2": "no flush needed: each step streams >5 GB of weights + KV through the 126 MB L2",
@@ -564,7 +564,7 @@ def main():
                 "bytes = sum_b(4096*L_b + 8192)", mean_context=round(mean_ctx, 1)),
             hbm("fused_decode_attn_kernel, 64 sequences x 512 cached tokens", a512_ms, a512_alg, "graph of 6 launches, cold caches",
                 traffic=traffic.get("fused_decode_attn_kernel"), traffic_note=traffic.get("_fused_decode_attn_kernel")),
-            hbm("fused_decode_attn_kernel, 64 sequences x 4096 cached tokens (BASELINE configs[3] KV length)", a4k_ms, a4k_alg,
+            hbm("fused_decode_attn_kernel, 64 sequences x 4096 cached tokens (voice-clone KV length)", a4k_ms, a4k_alg,
                 "graph of 3 launches over different 1 GiB caches, scattered pages"),
             hbm("paged_attn_kernel<2,false> (stand-alone a2 entry point), 64 sequences x 4096 cached tokens", long_ms, long_alg,
                 "graph of 3 launches over different 1 GiB caches, scattered pages",
@@ -573,7 +573,7 @@ def main():
                 "graph of 8 launches; bytes = tokens * 1024 * 2 B * 2 (K, V) * 2 (read + write)"),
             hbm(f"topk_sample_row_kernel, [{a.streams}, {mc.predictor.vocab_size}] bf16 logits, top-k 50", sm_ms, sm_alg,
                 "graph of 16 launches; bytes = the logits (latency-bound: one CTA per row)"),
-            {"kernel": "prefill_attn_tc_kernel (tcgen05 128x128 tiles, TMEM), one 4096-token sequence (BASELINE configs[3])",
+            {"kernel": "portion_attn_kernel (tcgen05 128x128 tiles, TMEM), one 4096-token sequence (voice-clone prompt)",
              "bound": "tensor", "achieved": round(pf_flops / pf_ms / 1e9, 1), "peak": tpeak, "unit": "TFLOP/s",
              "frac": round(pf_flops / pf_ms / 1e9 / tpeak, 4), "traffic": None, "flops_per_launch": pf_flops,
              "launch_ms": round(pf_ms, 5), "peak_source": tpeak_src,
@@ -661,7 +661,7 @@ def main():
             line["e2e"] = {"value": round(e2e_fps, 1), "unit": "frames/s", "h2d_bytes_per_step": int(h2d),
                            "d2h_bytes_per_step": int(d2h), "steps": a.e2e_steps, "segments": "median of 3",
                            "api": "TalkerLLM.add_requests/step_launch/step_collect + PredictorLLM.add_requests/step_launch/step_collect (StepApiFrameLoop, pipelined), pinned host tensors"}
-    # ---- other stream counts ([2], [4]) on rank 0, short runs
+    # ---- other stream counts on rank 0, short runs
     if rank == 0 and world == 1 and a.also_streams:
         others = {}
         for b in [int(x) for x in a.also_streams.split(",") if x]:
@@ -681,7 +681,7 @@ def main():
                 mc, talker, predictor = build_engines(a.model, 1, 16, device)
                 loop = None
         line["other_workloads"] = others
-    # ---- BASELINE configs[3]: voice-clone ICL, ~4k-token prompts (varlen prefill + decode), 8 streams
+    # ---- voice-clone ICL, ~4k-token prompts (varlen prefill + decode), 8 streams
     if rank == 0 and world == 1 and not a.no_icl:
         talker.exit(); predictor.exit()
         del loop, talker, predictor
@@ -696,7 +696,7 @@ def main():
                                                           + 3 * t.hidden_size * t.intermediate_size)
             att = b * t.num_hidden_layers * 4.0 * t.num_attention_heads * t.head_dim * plen * (plen + 1) / 2
             line["icl_workload"] = {
-                "workload": f"BASELINE configs[3]: {b} streams x {plen}-token prompt (packed varlen prefill: tcgen05 prefill "
+                "workload": f"voice clone: {b} streams x {plen}-token prompt (packed varlen prefill: tcgen05 prefill "
                             f"attention + cuBLAS projections above {os.environ.get('B2TTS_GEMM_NATIVE_MAX_M', '512')} rows), "
                             f"then {frames} frames of decode at ~{plen + frames // 2}-token contexts",
                 "prefill_ms": round(pre[0], 3), "prefill_tokens_per_s": round(b * plen / (pre[0] / 1e3), 1),
@@ -715,7 +715,7 @@ def main():
     if rank == 0 and not a.no_cpu_baseline and world == 1:
         fps, cores, what, dt = cpu_oracle_frames(a.model, a.cpu_streams or a.streams, 2, 1, budget_s=25.0)
         line["cpu_baseline"] = {"value": round(fps, 3), "unit": "frames/s", "cores": cores, "kind": "port", "sample": what}
-        # BASELINE configs[0]: 0.6B, 1 stream, ~20-word (40-token) prompt - the reference's own CPU-runnable case
+        # 0.6B, 1 stream, ~20-word (40-token) prompt - the reference's own CPU-runnable case
         fps0, cores0, what0, _ = cpu_oracle_frames("0.6B", 1, 8, 2, budget_s=20.0, prompt_len=40)
         line["cpu_baseline_configs0"] = {"value": round(fps0, 3), "unit": "frames/s", "cores": cores0, "kind": "port",
                                          "rtf": round(FRAME_HZ / fps0, 4), "sample": what0}

@@ -5,7 +5,7 @@
  *
  * The reference (tsdocode/nano-qwen3tts-vllm) has no FFI: its "operator API" for this
  * path is a set of Python callables.  Each entry point below replaces the arithmetic
- * of one of them; citations are file:line under /root/reference/nano-qwen3tts-vllm/.
+ * of one of them; citations are file:line of the reference, nano-qwen3tts-vllm/.
  * The Python modules in nano-qwen3tts-vllm_b200/layers/ keep the reference's names and
  * signatures and call these through ctypes.
  *
@@ -44,7 +44,7 @@ extern "C" {
 #define B2TTS_ECUDA        -4   /* CUDA launch error (message carries cudaGetErrorString) */
 #define B2TTS_EWORKSPACE   -5   /* workspace too small                                   */
 
-/* rounding modes of the element-wise kernels (see DESIGN.md "rounding points") */
+/* rounding modes of the element-wise kernels */
 #define B2TTS_ROUND_EAGER 0   /* the reference's Python source evaluated op by op in bf16 */
 #define B2TTS_ROUND_FUSED 1   /* what torch-inductor emits for the same source on a GPU:
                                   fp32 throughout, one rounding at the store            */
@@ -381,7 +381,7 @@ B2TTS_API int b2tts_prompt_assemble(const void* a, int64_t a_row_stride, int a_r
 /* ---- f4 (tail): decoded waveform -> PCM16 ----------------------------------------------------------------------
  * replaces _float_to_pcm16 / _apply_volume_pcm16                                    examples/server.py:338-349
  *   out[i] = (int16) trunc(clip(wav[i], -1, 1) * 32767);  volume != 1: out[i] = clip(rint(out[i] * volume), -32768, 32767)
- * (the vocoder itself - qwen_tts 0.0.5, not part of the reference tree - is out of reach; DESIGN.md section 7). */
+ * (the vocoder itself - qwen_tts 0.0.5, not part of the reference tree - is out of reach). */
 B2TTS_API int b2tts_float_to_pcm16(const float* wav, int16_t* out, int64_t n, float volume, void* stream);
 
 /* ---- a10 in one launch: the decode pass of a whole (small) decoder stack ----------------------------------------

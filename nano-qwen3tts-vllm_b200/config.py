@@ -3,7 +3,7 @@
 ``Config`` keeps the field names of the reference's engine dataclass (config.py:41-66) so the
 ``TalkerLLM(model_path, enforce_eager=..., gpu_memory_utilization=...)`` call is unchanged; unlike the
 reference it does NOT overwrite ``max_model_len`` with 1024 (config.py:64): the decode block-table
-buffers are sized from the real value, so voice-clone prompts (~4k tokens, BASELINE config 4) run
+buffers are sized from the real value, so voice-clone prompts (~4k tokens) run
 on the graph path.  ``StackConfig`` is the subset of the HF ``config.json`` the decoder stacks read
 (``talker_config`` and its nested ``code_predictor_config``, config.py:171-360,362-560).
 """
@@ -77,7 +77,7 @@ class ModelConfig:
 
 
 def qwen3_tts_config(size: str = "1.7B") -> ModelConfig:
-    """The shipped model shapes; weights are random-init in every BASELINE
+    """The shipped model shapes; weights are random-init in every benchmark
     config, so these numbers define the workload."""
     mrope = {"mrope_section": [24, 20, 20], "interleaved": True}
     if size in ("1.7B", "1.7b"):
@@ -923,7 +923,7 @@ class Config:
     process_gpu_memory_fraction: float | None = None
     # additions (not in the reference)
     device: str = "cuda:0"
-    rounding: int = 0                          # _native.ROUND_EAGER | ROUND_FUSED, see DESIGN.md
+    rounding: int = 0                          # _native.ROUND_EAGER | ROUND_FUSED
     graph_batch_sizes: list = field(default_factory=list)   # [] = reference's schedule
 
     max_state_slots: int = 0                   # per-sequence recurrent / convolution state slots (0 = max_num_seqs)

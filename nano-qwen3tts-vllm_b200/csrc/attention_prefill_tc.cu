@@ -1,7 +1,7 @@
 // attention_prefill_tc.cu - a3 at its real size: varlen causal prefill attention on the 5th-gen tensor cores.
 // Replaces flash_attn_varlen_func(q, k, v, cu_seqlens_q/k, max_seqlen_q/k, softmax_scale, causal=True) as called from
 // Attention.forward's prefill branch (layers/attention.py:78-91) when the prompt is long enough for the work to be a
-// real contraction - the voice-clone ICL prompt of BASELINE configs[3] is ~4096 tokens: 2*T^2*128*16 / 2 = 69 GFLOP
+// real contraction - the voice-clone ICL prompt is ~4096 tokens: 2*T^2*128*16 / 2 = 69 GFLOP
 // per layer, tensor-bound.  (Short prompts and the paged prefix-cache variant stay on paged_attn_kernel<G,true>.)
 //
 // One CTA = 128 queries of one (sequence, q head); K/V are walked in 128-key tiles up to the causal diagonal:

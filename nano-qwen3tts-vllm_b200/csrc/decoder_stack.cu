@@ -22,7 +22,7 @@
 //     summation order of fused_decode_attn_kernel) runs on 4 worker warps of ALL CTAs, one (sequence, kv head) per
 //     warp, between the qkv and o phases; the cached K / V rows of the item (written by earlier launches) are staged
 //     in shared memory by cp.async while the QKV projection is still running.
-// Rounding points are those of the separate launches (DESIGN.md section 4); with the same K splits the result is
+// Rounding points are those of the separate launches; with the same K splits the result is
 // bit-identical to rmsnorm -> gemm -> fused_decode_attn -> gemm(residual) -> rmsnorm -> gemm(SiLU*mul) -> gemm(residual).
 //
 // Every wait is bounded: a dependency that does not resolve within DS_TIMEOUT_NS traps (launch failure) instead of
@@ -998,7 +998,7 @@ extern "C" B2TTS_API int b2tts_decoder_stack_decode(
   return B2TTS_OK;
 }
 
-// Debug aid (tools/stack_trace.py): following launches record 32 globaltimer stamps per (CTA, layer) into
+// Debug aid: following launches record 32 globaltimer stamps per (CTA, layer) into
 // buffer[(cta * 8 + layer) * 16 + slot] (uint64).  NULL switches tracing off.
 extern "C" B2TTS_API int b2tts_debug_stack_trace(void* buffer) {
   b2::g_ds_trace = static_cast<unsigned long long*>(buffer);

@@ -734,7 +734,7 @@ static int gemm_impl(const char* what, const void* x, int64_t x_row_stride, cons
   }
   p.chunk_rows = m > chunk_cfg ? chunk_cfg : G_MAX_M;
   // Plain x (no fused norm: above 64 rows the norms are separate launches) cut into chunks: a k-block costs ~0.2 us
-  // there (0.45 with the in-place norm transform), so (measured at 256 streams, tools/plan_sweep.py)
+  // there (0.45 with the in-place norm transform), so (measured at 256 streams)
   //   * K <= 1024 is not split at all: 16 k-blocks per CTA cost less than drain + DSMEM exchange of 64-row partials
   //     (predictor qkv: -0.16 ms per frame at 256 streams; 128 streams with separate norms 5.94 -> 5.70 ms);
   //   * an unsplit launch takes the chunk size that fills ONE wave of 2 CTAs per SM best (predictor gate_up: 48 tiles x
@@ -1474,7 +1474,7 @@ extern "C" B2TTS_API int b2tts_gemm_chain(const b2tts_gemm_op* ops, int nops, in
   return B2TTS_OK;
 }
 
-// Debug aid (tools/gemm_trace.py): every following GEMM launch records 8 globaltimer stamps per CTA into
+// Debug aid: every following GEMM launch records 8 globaltimer stamps per CTA into
 // buffer + launch_index * 4096 * 8 (uint64), for `launches` launches.  NULL switches tracing off.
 extern "C" B2TTS_API int b2tts_debug_gemm_trace(void* buffer, int launches) {
   b2::g_trace_base = static_cast<unsigned long long*>(buffer);

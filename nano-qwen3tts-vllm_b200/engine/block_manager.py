@@ -3,7 +3,7 @@
 
 A plain LIFO free list of page ids.  The reference additionally hashes full blocks of token ids for
 prefix caching; for this engine's embed-only sequences that cache can never hit (the prompt has no
-token ids, SURVEY.md section 2), so it is not built - ``num_cached_tokens`` stays 0.  LIFO hands a just-freed
+token ids), so it is not built - ``num_cached_tokens`` stays 0.  LIFO hands a just-freed
 page (still warm in the 126 MB L2) to the next request: the predictor frees and re-takes one page
 per stream every frame."""
 from __future__ import annotations

@@ -1,4 +1,4 @@
-"""The per-frame talker <-> predictor loop (SURVEY.md section 8f rows 1-2; reference interface.py:1207-1290,
+"""The per-frame talker <-> predictor loop (reference interface.py:1207-1290,
 zmq/engine_loop_mp.py, workers/*), two ways:
 
 ``DeviceFrameLoop``  B200-first: talker and predictor share one process and one GPU, every stream's
@@ -31,7 +31,7 @@ class DeviceFrameLoop:
 
     Protocol of the reference's ``generate_async`` (interface.py:1207-1290), per stream: the talker's code0 ==
     codec EOS (2150) ends the stream before the frame is produced (``ignore_eos`` keeps it running, the benchmark /
-    parity setting of SURVEY.md section 8d); the next talker input is the 16-codebook embedding sum plus
+    parity setting); the next talker input is the 16-codebook embedding sum plus
     ``trailing_text_hiddens[:, generation_step]`` while the trailing text lasts and ``tts_pad_embed`` after.
     Finished streams stay in the batch as padding rows (slot -1, context 0) until every stream is done.
 

@@ -1,4 +1,4 @@
-"""KV-pool memory policy (SURVEY.md section 8 row a11): how many 256-token pages each model gets.
+"""KV-pool memory policy: how many 256-token pages each model gets.
 
 Integer / float arithmetic only, no CUDA calls - the runner feeds it the live allocator numbers
 (``ModelRunner.allocate_kv_cache``), the CPU tests feed it tables.  Restates, with the same operand order so

@@ -1,5 +1,5 @@
 """Model runner: batch layout, paged KV pool, CUDA-graph capture/replay of the decode step and the
-sampler call (surface S2 of SURVEY.md section 8b; reference engine/model_runner/base.py:30-312).
+sampler call (reference engine/model_runner/base.py:30-312).
 
 B200-first differences from the reference, none visible through ``run(seqs, is_prefill)``:
   * the step's layout (positions, slot_mapping, context_lens, block_tables, temperatures, last tokens,
@@ -9,8 +9,8 @@ B200-first differences from the reference, none visible through ``run(seqs, is_p
   * the graph's static tensors are views of the device mirror of that buffer, so replay needs no
     per-field ``copy_/fill_/zero_`` staging kernels (talker_mode_runner.py:95-101);
   * block tables are sized from the real ``max_model_len`` (the reference pins it to 1024 and
-    overflows its 4-column table beyond that, SURVEY.md section 5);
-  * one process per GPU, no NCCL group: replicas only (DESIGN.md "multi-GPU").
+    overflows its 4-column table beyond that);
+  * one process per GPU, no NCCL group: replicas only.
 """
 from __future__ import annotations
 
@@ -155,7 +155,7 @@ class ModelRunner:
     # ------------------------------------------------------------------ init
     def post_init(self):
         self.sampler = Sampler()
-        self.top_k = 50        # the reference never forwards SamplingParams.top_k (SURVEY.md section 3.4); 1 = greedy
+        self.top_k = 50        # the reference never forwards SamplingParams.top_k; 1 = greedy
         self.layout = StepLayout(self.max_bs, self.max_blocks, self.device)
         self.allocate_kv_cache()
         self.graphs: dict[int, torch.cuda.CUDAGraph] = {}

@@ -1,7 +1,7 @@
 """Talker runner (reference engine/model_runner/talker_mode_runner.py:23-234): decode inputs are
 embeddings fed by the frame loop, ``run`` returns ``(token_ids, hidden_states)``.
 
-Quirk kept on purpose (SURVEY.md section 7.1-3): the decode RoPE position is ``len(seq)`` while the KV slot
+Quirk kept on purpose: the decode RoPE position is ``len(seq)`` while the KV slot
 index is ``len(seq) - 1`` (talker_mode_runner.py:126-128)."""
 from __future__ import annotations
 

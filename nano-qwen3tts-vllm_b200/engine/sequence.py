@@ -1,5 +1,5 @@
 """Per-request state read by the scheduler and the model runner; same field names as the
-reference's ``Sequence`` (engine/sequence.py:15-90) because the runner contract (SURVEY.md section 8b, S2)
+reference's ``Sequence`` (engine/sequence.py:15-90) because the runner contract
 is expressed in them.  Sequences are embed-only: the prompt arrives as ``input_embeds [1, T, H]``
 and ``token_ids`` holds generated codec ids only."""
 from __future__ import annotations

@@ -1,2 +1,2 @@
-"""Drop-in layer modules (surface S1 of SURVEY.md section 8b): the reference's class names, constructor
+"""Drop-in layer modules: the reference's class names, constructor
 signatures, parameter names and forward signatures, with the arithmetic in libb200tts.so."""

@@ -24,7 +24,7 @@ GEMM_NATIVE_MAX_M = int(os.environ.get("B2TTS_GEMM_NATIVE_MAX_M", "512"))
 PDL = os.environ.get("B2TTS_PDL_GEMM", "1") != "0"     # programmatic dependent launch of the native GEMM (weight stream starts early)
 # each GEMM pulls the NEXT projection's weights into L2 (b2tts_gemm_prefetch_bf16).  Off by default: measured at 64
 # streams it does not shorten the frame (5873 us against 5885 us; talker pass 2052 against 2018) - the launches are
-# bound by their dependent latencies, not by the weight stream (DESIGN.md section 8).
+# bound by their dependent latencies, not by the weight stream.
 PREFETCH = os.environ.get("B2TTS_GEMM_PREFETCH", "0") != "0"
 _packed: dict = {}
 

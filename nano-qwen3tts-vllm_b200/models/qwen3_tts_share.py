@@ -12,7 +12,7 @@
   gate_proj, up_proj, silu*mul                           one gate_up GEMM, one SiLU*mul
   down_proj                                              down GEMM
 
-Rounding points are the reference's (DESIGN.md "rounding points"); the state-dict keys of the
+Rounding points are the reference's; the state-dict keys of the
 reference (``self_attn.{q,k,v,o}_proj.weight`` ...) are accepted by ``load_reference_weights`` and
 merged at load time."""
 from __future__ import annotations
@@ -48,7 +48,7 @@ FUSED_NORM_MAX_ROWS = int(os.environ.get("B2TTS_FUSED_NORM_MAX_ROWS", "64"))
 FUSED_NORM_MIN_ROWS = int(os.environ.get("B2TTS_FUSED_NORM_MIN_ROWS", "9"))
 # decode of a small stack (the code predictor) as ONE persistent dataflow launch (csrc/decoder_stack.cu).  Opt-in:
 # bit-identical to the separate launches, but measured at 260 us per 5-layer pass against their 246 us at 64 rows
-# (DESIGN.md section 8: every hand-over between phases costs a gpu-scope release + an L2 poll, ~2.5 us, 7 per layer)
+# (every hand-over between phases costs a gpu-scope release + an L2 poll, ~2.5 us, 7 per layer)
 DATAFLOW_STACK = os.environ.get("B2TTS_DATAFLOW_STACK", "0") != "0"
 
 
@@ -386,9 +386,9 @@ def load_reference_weights(module: nn.Module, state_dict: dict, strict: bool = T
 
 @torch.no_grad()
 def random_init_(module: nn.Module, seed: int = 1234, std: float = 0.02) -> None:
-    """Random-init weights in place on the module's device (every BASELINE config uses random
+    """Random-init weights in place on the module's device (every benchmark uses random
     weights): matrices / embeddings N(0, std^2) (``initializer_range``, config.py:299,484), norm weights
-    1 + N(0, std^2), biases 0 - the distribution of SURVEY.md section 8d."""
+    1 + N(0, std^2), biases 0."""
     gen = torch.Generator(device=next(module.parameters()).device).manual_seed(seed)
     for name, p in module.named_parameters():
         if name.endswith("bias"):

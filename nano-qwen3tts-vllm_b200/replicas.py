@@ -1,4 +1,4 @@
-"""Per-GPU replicas (SURVEY.md section 8e): the path has no exchange step, so N GPUs are N independent
+"""Per-GPU replicas: the path has no exchange step, so N GPUs are N independent
 talker+predictor engines with the request streams partitioned across them.  The only cross-rank
 traffic is bookkeeping: the barrier around a timed region and the max-over-ranks of its duration.
 Works over any ``torch.distributed`` backend (nccl on the box, gloo in the CPU tests)."""

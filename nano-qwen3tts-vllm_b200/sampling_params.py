@@ -1,6 +1,6 @@
 """``SamplingParams`` with the reference's fields and its greedy-is-forbidden assertion
 (sampling_params.py:5-14).  ``top_k`` IS honoured here when a runner is built with
-``honor_top_k=True`` (the reference accepts and drops it, SURVEY.md section 3.4); the default keeps the
+``honor_top_k=True`` (the reference accepts and drops it); the default keeps the
 reference behaviour: every row is sampled with top_k=50."""
 from dataclasses import dataclass
 

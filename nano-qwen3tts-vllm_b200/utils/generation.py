@@ -1,4 +1,4 @@
-"""Prompt-prep embedding assembly on the GPU (SURVEY.md section 8f rank 3): the talker's input embeddings, the
+"""Prompt-prep embedding assembly on the GPU: the talker's input embeddings, the
 trailing text hiddens, the tts pad row and the attention mask, with the reference's call surface
 (``prepare_inputs`` / ``generate_icl_prompt`` / ``generate_speaker_prompt``, utils/generation.py:18-379, 412-515,
 380-409).

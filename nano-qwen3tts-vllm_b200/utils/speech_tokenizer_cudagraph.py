@@ -1,4 +1,4 @@
-"""Codec decode windows (SURVEY.md section 8f rank 4): the graph-per-length wrapper the reference puts around the
+"""Codec decode windows: the graph-per-length wrapper the reference puts around the
 speech tokenizer's decoder (utils/speech_tokenizer_cudagraph.py:18-56, 59-168) and the streaming window logic of its
 server (examples/server.py:196-222, 338-349) - WITHOUT the vocoder itself.
 

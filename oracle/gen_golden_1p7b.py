@@ -1,10 +1,10 @@
 """Golden greedy codec frames + logits of the CPU oracle at the NAMED model size (Qwen3-TTS-12Hz-1.7B
-shapes, SURVEY.md section 7.0 / 8d), for the GPU parity tests of tests/test_gpu_parity_1p7b.py.
+shapes), for the GPU parity tests of tests/test_gpu_parity_1p7b.py.
 
 TEST INFRASTRUCTURE ONLY - see ``oracle/__init__.py``.
 
-north_star: "greedy codec-token sequences are identical for the first 256 frames" (512 for BASELINE
-configs[1]); "attention outputs and logits match within 2e-2 relative in bf16".  The CPU oracle needs
+Wanted: "greedy codec-token sequences are identical for the first 256 frames" (512 for one
+stream); "attention outputs and logits match within 2e-2 relative in bf16".  The CPU oracle needs
 ~0.5 s (1 stream) to ~3.6 s (64 streams) per frame at this size, so the expected frames are generated ONCE
 here, in the build container, and committed under tests/golden/:
 
@@ -21,7 +21,7 @@ Per (streams, rounding mode) one file ``frames_1p7b_b{B}_{mode}.pt``:
 
 Weights: ``oracle.model.synthetic_weights(seed=1234)`` (CPU generator, machine independent); prompts
 ``N(0, 0.05^2)`` bf16 [64, H] from ``manual_seed(1000 + s)``; trailing-text term = one pad row, seed 999;
-EOS ignored (SURVEY.md section 8d).  ``mode`` = eager (the reference source op by op: what its CPU path
+EOS ignored.  ``mode`` = eager (the reference source op by op: what its CPU path
 computes) | fused (RMSNorm / SiLU*mul with inductor's single store rounding: what its GPU path computes).
 """
 from __future__ import annotations
@@ -41,7 +41,7 @@ from oracle import ops as O         # noqa: E402
 
 BF16 = torch.bfloat16
 PROMPT_LEN = 64
-CONFIGS = {"b1": (1, 512), "b8": (8, 256), "b64": (64, 256)}      # BASELINE configs[1], [2], [4]
+CONFIGS = {"b1": (1, 512), "b8": (8, 256), "b64": (64, 256)}
 
 
 def dims_1p7b():
@@ -103,7 +103,7 @@ def fp32_logits(b: int, gold: dict, tw, pw, td, pd, nframes: int = 4):
     """The same model evaluated WITHOUT bf16 rounding points: weights upcast to fp32, every op in fp32, fed the
     golden run's codes (teacher-forced), for the decisions whose bf16 logits the golden file keeps.  This is the
     yardstick for "how far may two correct bf16 pipelines be from each other": the CPU oracle itself (= the
-    reference's own CPU path, bit for bit) sits ~4 % of max|logit| away from it after 28 layers, so the north-star
+    reference's own CPU path, bit for bit) sits ~4 % of max|logit| away from it after 28 layers, so the
     2e-2 bound holds per op / per layer (tests/test_gpu_ops.py, test_gpu_models.py) but cannot hold for whole-stack
     logits, for ANY bf16 implementation including the reference's."""
     old = OM.BF16, O.BF16

@@ -3,7 +3,7 @@ per-frame talker<->predictor loop.
 
 TEST INFRASTRUCTURE ONLY - see ``oracle/__init__.py``.
 
-Restates (``file:line`` under ``/root/reference/nano-qwen3tts-vllm/``):
+Restates (``file:line`` of the reference, ``nano-qwen3tts-vllm/``):
   models/qwen3_tts_share.py:79-113,131-135,163-176   layer recipe
   models/qwen3_tts_talker.py:53-62,123-136           talker stack + codec_head
   models/qwen3_tts_predictor.py:87-124               predictor embed/head select
@@ -283,7 +283,7 @@ def run_frames(talker: Talker, predictor: Predictor, prompts, num_frames, tts_pa
 
 def synthetic_weights(talker: StackDims, predictor: StackDims, seed=1234, text_vocab=0, text_hidden=0,
                       num_code_groups=16, std=0.02):
-    """Random-init bf16 state dicts (SURVEY.md section 8d): matrices / embeddings
+    """Random-init bf16 state dicts: matrices / embeddings
     ``N(0, std^2)`` (``initializer_range``, config.py:299,484), norm weights
     ``1 + N(0, std^2)``, biases 0.  Keys are the reference's *converted* names
     (qwen3_tts_talker.py:81-109, qwen3_tts_predictor.py:63-85).  Drawn on the CPU

@@ -2,7 +2,7 @@
 
 TEST INFRASTRUCTURE ONLY - see ``oracle/__init__.py``.
 
-Citations are ``file:line`` under ``/root/reference/nano-qwen3tts-vllm/``.
+Citations are ``file:line`` of the reference, ``nano-qwen3tts-vllm/``.
 
 Pinned against the live reference (``oracle/pin_against_reference.py`` ->
 ``tests/golden/``): rmsnorm, add_rmsnorm, rope (1-D and M-RoPE), silu, silu*mul,
@@ -10,7 +10,7 @@ linear, sampler, lm heads, decoder layer, talker / predictor stacks.
 PARITY UNPINNED by a reference run (CUDA-only in the reference): store_kvcache
 (Triton kernel) and the two flash-attn calls; restated from
 ``layers/attention.py:10-30,73-96`` and cross-checked against the flash-attn
-wheel and the reference's Triton kernel on the GPU box
+wheel and the reference's Triton kernel on a GPU
 (tests/test_gpu_reference_kernels.py).
 """
 from __future__ import annotations

@@ -2,7 +2,7 @@
 
 TEST INFRASTRUCTURE ONLY - see ``oracle/__init__.py``.
 
-Runs only in the build container (needs ``/root/reference``); the GPU box never
+Runs only in the build container (needs ``/root/reference``); nothing with a GPU
 executes this file.  It imports the reference package through a symlink
 (``/tmp/refpkg/nano_qwen3tts_vllm`` -> ``/root/reference/nano-qwen3tts-vllm``),
 with ``TORCHDYNAMO_DISABLE=1`` (inductor's CPU build is broken in this image) and
@@ -14,7 +14,7 @@ outputs under ``tests/golden/*.pt`` for the CPU and GPU test-suites.
 Two reference ops are CUDA-only (Triton ``store_kvcache``, flash-attn): for the
 model-level vectors ``Attention.forward`` is replaced by the oracle restatement of
 ``layers/attention.py:73-96`` - those two ops stay "parity unpinned" here and are
-cross-checked against the flash-attn wheel on the GPU box instead.
+cross-checked against the flash-attn wheel on a GPU instead.
 
     TORCHDYNAMO_DISABLE=1 python oracle/pin_against_reference.py
 """

@@ -1,4 +1,4 @@
-"""CPU oracle of the prompt-prep embedding assembly (SURVEY.md section 8f rank 3).
+"""CPU oracle of the prompt-prep embedding assembly.
 
 TEST INFRASTRUCTURE ONLY - see ``oracle/__init__.py``.
 

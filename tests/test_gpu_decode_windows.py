@@ -1,6 +1,6 @@
 """f4 (what can be built of it): the graph-per-length wrapper and the streaming window logic of the reference's
 codec decode path (utils/speech_tokenizer_cudagraph.py:18-168, examples/server.py:196-222, 338-349) around a STAND-IN
-decoder - the real vocoder (qwen-tts 0.0.5) is not available (DESIGN.md section 7)."""
+decoder - the real vocoder (qwen-tts 0.0.5) is not available."""
 import types
 
 import numpy as np

@@ -1,6 +1,6 @@
-"""GPU parity of the device-resident frame loop (SURVEY.md section 8f rows 1-2): greedy (top_k = 1) codec
+"""GPU parity of the device-resident frame loop: greedy (top_k = 1) codec
 frames of DeviceFrameLoop / StepApiFrameLoop against the CPU oracle's run_frames on the
-same random-init weights and prompts (north_star: greedy codec-token sequences identical).
+same random-init weights and prompts (greedy codec-token sequences are identical).
 
 A greedy sequence can only be required to be identical while the oracle's own arg-max is decided by more
 than the arithmetic noise between two correct bf16 pipelines: where the oracle's top-2 logit margin is below

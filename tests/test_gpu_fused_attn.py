@@ -1,7 +1,7 @@
 """GPU parity of the fused decode attention (b2tts_fused_decode_attn) against the separate launches it
 replaces - b2tts_qknorm_rope_kvwrite then b2tts_paged_attn_decode (models/qwen3_tts_share.py:96-109 of the
 reference: q_norm, k_norm, rotary_emb, store_kvcache, flash_attn_with_kvcache).  KV-cache bytes must be
-identical; attention outputs within 2e-2 relative (north_star), in practice ~1e-3 (split-KV order only)."""
+identical; attention outputs within 2e-2 relative, in practice ~1e-3 (split-KV order only)."""
 import pytest
 import torch
 

@@ -1,9 +1,9 @@
-"""GPU parity of the weight-streaming tcgen05 GEMM (b2tts_gemm_bf16, SURVEY.md section 8a row a7) through the C ABI.
+"""GPU parity of the weight-streaming tcgen05 GEMM (b2tts_gemm_bf16) through the C ABI.
 
 Reference semantics: ``F.linear`` (layers/linear.py:72-73,149-153) in bf16 with fp32 accumulation; the
 fused epilogues restate ``residual + hidden`` (models/qwen3_tts_share.py:171,175) and
 ``act_fn(gate) * up`` (models/qwen3_tts_share.py:131-135).  Tolerance: logits/projections within 2e-2
-relative (north_star); in practice the only difference from an fp64 contraction is the fp32 summation
+relative; in practice the only difference from an fp64 contraction is the fp32 summation
 order, so the bound used here is one bf16 ulp on almost every element."""
 import pytest
 import torch
@@ -214,7 +214,7 @@ def test_gemm_bias_epilogue_ssq_out(native):
 # ------------------------------------------------------------------ more than 128 rows: grid chunks of 128 rows
 @pytest.mark.parametrize("m", [129, 256, 300, 1000, 4096])
 def test_gemm_row_chunks(native, m):
-    """Prefill-sized M (SURVEY.md section 8a row a7 "lift G_MAX_M"): every 128-row chunk is its own set of CTAs,
+    """Prefill-sized M: every 128-row chunk is its own set of CTAs,
     the last one ragged.  Same bound as the single-chunk case, every epilogue."""
     n, k = 2048, 1024
     g = torch.Generator(device="cuda").manual_seed(m)

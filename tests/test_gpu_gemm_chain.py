@@ -1,8 +1,8 @@
-"""GPU parity of the persistent GEMM chain (b2tts_gemm_chain, SURVEY.md section 8a rows a7 + a4 + a6) through
+"""GPU parity of the persistent GEMM chain (b2tts_gemm_chain) through
 the C ABI: the four dependent projections of a decoder layer in one launch must give what the four separate
 b2tts_gemm_norm_bf16 launches give (same packed weights, epilogues, fused norms and rounding points; the only
 difference allowed is the fp32 summation order of the K splits: one bf16 ulp on a few elements of each op's
-output, compounding along the chain, bounded here at 1e-2 of the output's magnitude - inside the north_star
+output, compounding along the chain, bounded here at 1e-2 of the output's magnitude - inside the
 tolerance of 2e-2; the separate launches are themselves checked against fp64 in tests/test_gpu_gemm.py)."""
 import pytest
 import torch

@@ -1,7 +1,7 @@
 """GPU parity of the model runners / step API against the committed outputs of the LIVE reference
 (tests/golden/models.pt, written by oracle/pin_against_reference.py) and against the CPU oracle.
 
-Tolerance (BASELINE.json north_star): logits / hidden within 2e-2 relative (max|a-b| / max|b|);
+Tolerance: logits / hidden within 2e-2 relative (max|a-b| / max|b|);
 KV slot contents compared at the same tolerance here because K depends on GEMM accumulation
 order upstream of the write (the write itself is bit-exact, tests/test_gpu_ops.py)."""
 import pytest

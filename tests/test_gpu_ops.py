@@ -1,7 +1,7 @@
 """GPU parity tests: every entry point of libb200tts (through the C ABI) against the CPU oracle
 and the committed golden vectors (outputs of the live reference, tests/golden/).
 
-Bars (BASELINE.json north_star): KV slots and sampled indices bit-exact; element-wise ops
+Bars: KV slots and sampled indices bit-exact; element-wise ops
 bit-exact up to a counted handful of 1-ulp bf16 flips caused by fp32 summation order / libm
 ulps (documented per test); attention within 2e-2 relative.
 """
@@ -264,7 +264,7 @@ def test_paged_attn_decode_vs_oracle(native, lens, max_ctx):
     scale = 128 ** -0.5
     want = O.paged_attn_decode(q, kc, vc, cl, bt, scale)
     got = native.paged_attn_decode(q.to(DEV), kc.to(DEV), vc.to(DEV), bt.to(DEV), cl.to(DEV), scale, max_ctx)
-    assert rel_err(got, want) <= 2e-2, rel_err(got, want)      # north_star tolerance
+    assert rel_err(got, want) <= 2e-2, rel_err(got, want)
     assert rel_err(got, want) <= 8e-3                           # and in practice one bf16 ulp
     for i, l in enumerate(lens):
         if l == 0:
@@ -272,7 +272,7 @@ def test_paged_attn_decode_vs_oracle(native, lens, max_ctx):
 
 
 def test_paged_attn_decode_full_size_properties(native):
-    """BASELINE C5 sizes (B=64 ragged contexts): size-independent properties instead of the
+    """64 ragged contexts: size-independent properties instead of the
     oracle - (i) V == const => output == const; (ii) softmax over identical keys == mean of V;
     (iii) result independent of the split-KV factor (max_ctx changes nsplit)."""
     g = torch.Generator().manual_seed(9)

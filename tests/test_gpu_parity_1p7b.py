@@ -1,6 +1,6 @@
-"""GPU parity at the NAMED model size (Qwen3-TTS-12Hz-1.7B shapes): north_star "logits match within 2e-2
-relative in bf16, greedy codec-token sequences are identical for the first 256 frames" (512 for BASELINE
-configs[1]), at 1 / 8 / 64 streams (configs[1], [2], [4]), in both rounding modes (EAGER = what the reference's
+"""GPU parity at the NAMED model size (Qwen3-TTS-12Hz-1.7B shapes): "logits match within 2e-2
+relative in bf16, greedy codec-token sequences are identical for the first 256 frames" (512 for one
+stream), at 1 / 8 / 64 streams, in both rounding modes (EAGER = what the reference's
 source computes op by op, FUSED = what its inductor-compiled RMSNorm / SiLU*mul compute on a GPU).
 
 Expected values: tests/golden/frames_1p7b_b{B}_{mode}.pt, generated once by oracle/gen_golden_1p7b.py from the
@@ -8,13 +8,13 @@ CPU oracle (which is pinned bit-exactly against the live reference modules, orac
 
 What "match" can mean after 28 layers of bf16.  The golden files also hold the SAME model evaluated in fp32 (no bf16
 rounding points, same weights, same inputs).  The reference's own bf16 path (= the CPU oracle, bit for bit) sits
-2.7 - 4.4 % of max|logit| away from that fp32 evaluation (oracle/gen_golden_1p7b.py prints it): the 2e-2 bound of
-north_star holds per op and per layer (tests/test_gpu_ops.py, test_gpu_models.py, test_gpu_reference_kernels.py),
+2.7 - 4.4 % of max|logit| away from that fp32 evaluation (oracle/gen_golden_1p7b.py prints it): the 2e-2 bound
+holds per op and per layer (tests/test_gpu_ops.py, test_gpu_models.py, test_gpu_reference_kernels.py),
 but no bf16 implementation - the reference included - can meet it on whole-stack logits.  The bar here is therefore
 "as accurate as the reference": for every kept decision
     err(GPU, fp32)  <=  1.5 * err(oracle bf16, fp32)        (the GPU path is no further from the exact result)
     err(GPU, oracle bf16)  <=  2 * err(oracle bf16, fp32)   (two pipelines, each within the floor of the truth)
-with err = max|a - b| / max|b| (north_star's measure).
+with err = max|a - b| / max|b|.
 
 How greedy sequences are compared.  With random-init weights the logits are nearly flat: the oracle's top-2 margin
 is <= 2 bf16 ulp on ~16 % of the decisions, and the per-logit noise floor above is ~8 ulp of the top logit.  A
@@ -26,7 +26,7 @@ exactly the oracle's history, all of them are compared, and the test demands tha
   * where the oracle's margin is larger than that the choice is 100 % identical,
   * the share of differing decisions stays under MAX_FLIP_FRAC,
 and writes first-divergence frame (= the identical prefix of a free-running comparison), flip count and worst
-flipped margin per stream to profiles/parity_1p7b.json (gpurun_out/ on the GPU box)."""
+flipped margin per stream to profiles/parity_1p7b.json."""
 import json
 import os
 

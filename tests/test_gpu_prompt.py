@@ -135,7 +135,7 @@ def test_prompt_assembly_is_bit_exact_given_the_same_projected_rows(golden):
 
 def test_prompt_assembly_at_model_width_and_4k_icl():
     """1.7B widths (text 2048 -> hidden 2048, native GEMM projection) and a 4096-frame voice-clone reference
-    shapes, mask, and the projection within 2e-2 of an fp32 evaluation."""
+    (a voice-clone prompt): shapes, mask, and the projection within 2e-2 of an fp32 evaluation."""
     from nano_qwen3tts_vllm_b200.models.qwen3_tts_talker import Qwen3TTSTalkerResizeMLP
     from nano_qwen3tts_vllm_b200.utils.generation import prepare_inputs
     cfg = _config()

@@ -1,4 +1,4 @@
-"""a1 / a2 / a3 / a5 against what the reference EXECUTES on a GPU (SURVEY.md section 8c: these ops are CUDA-only
+"""a1 / a2 / a3 / a5 against what the reference EXECUTES on a GPU (these ops are CUDA-only
 in the reference, so the CPU oracle's versions are restatements - this file pins them on the box):
 
   a1  store_kvcache         the reference launches a Triton kernel, one program per token, that copies the token's D
@@ -8,14 +8,14 @@ in the reference, so the CPU oracle's versions are restatements - this file pins
   a2  decode attention      flash_attn_with_kvcache(q.unsqueeze(1), k_cache, v_cache, cache_seqlens=, block_table=,
                             softmax_scale=, causal=True)                    layers/attention.py:92-95
   a3  prefill attention     flash_attn_varlen_func(q, k, v, cu_seqlens_q/k, max_seqlen_q/k, softmax_scale, causal=True)
-                            at the BASELINE shapes: [2] x 64 (predictor), [40], [64] x 64, ragged, [4096]
+                            at the served shapes: [2] x 64 (predictor), [40], [64] x 64, ragged, [4096] (voice clone)
                                                                                layers/attention.py:78-91
   a5  RoPE                  the reference's eager torch ops ON THE GPU (CUDA cos/sin, bf16 arithmetic):
                             layers/rotary_embedding.py:101-148, 172-212 via oracle.ops run on CUDA tensors - the plain
                             RoPE surface must be bit-identical, and so must the K rows the fused kernel writes to the
                             cache from already-normalised heads.
 
-Tolerances: bytes for a1 / a5; 2e-2 relative (north_star) for attention outputs, flash-attn being the reference."""
+Tolerances: bytes for a1 / a5; 2e-2 relative for attention outputs, flash-attn being the reference."""
 import pytest
 import torch
 
@@ -136,7 +136,7 @@ def test_paged_decode_vs_flash_attn_with_kvcache(native, b, max_len):
 # ---------------------------------------------------------------------------------------------------- a5
 @pytest.mark.parametrize("mrope", [None, "interleaved", "sectioned"])
 def test_rope_bit_exact_vs_reference_ops_on_cuda(native, mrope):
-    """The reference's RoPE is eager torch; on the GPU box its cos/sin are CUDA's.  oracle.ops.rope is that op
+    """The reference's RoPE is eager torch; on a GPU its cos/sin are CUDA's.  oracle.ops.rope is that op
     sequence (pinned bit-exactly against rotary_embedding.py on CPU): run on CUDA tensors it IS the reference's GPU
     arithmetic, and the kernel must reproduce it to the bit - q, k and the K rows written to the cache."""
     g = torch.Generator(device="cuda").manual_seed(11)

@@ -1,4 +1,4 @@
-"""a11: the KV-pool memory policy restated in engine/memory.py against the numbers the
+"""The KV-pool memory policy restated in engine/memory.py against the numbers the
 reference's OWN code produced for the same inputs (tests/golden/memory_policy.json, written by
 oracle/pin_against_reference.py from interface.py:57-197 and engine/model_runner/base.py:131-164)."""
 import json
@@ -42,7 +42,7 @@ def test_block_bytes_of_the_named_models():
     from nano_qwen3tts_vllm_b200.config import qwen3_tts_config
     from nano_qwen3tts_vllm_b200.engine import memory as mem
     mc = qwen3_tts_config("1.7B")
-    assert mem.kv_block_bytes(mc.talker) == 28 << 20              # SURVEY.md section 8 a11: 28 MiB / 5 MiB
+    assert mem.kv_block_bytes(mc.talker) == 28 << 20              # 28 MiB / 5 MiB
     assert mem.kv_block_bytes(mc.predictor) == 5 << 20
     split = mem.compute_memory_split(mc, 0.9, 191_514_542_080)
     assert split["blocks_each"] > 4000 and 0.05 <= split["talker_util"] <= 0.95

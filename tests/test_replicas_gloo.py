@@ -1,4 +1,4 @@
-"""N > 1 host logic (SURVEY.md section 8e: replicas only, no data-path collective) over world-size-2
+"""N > 1 host logic (replicas only, no data-path collective) over world-size-2
 gloo on CPU: stream partition, least-loaded routing, sum/max aggregation of a timed region."""
 import os
 import socket
