@@ -141,9 +141,9 @@ __device__ __forceinline__ uint32_t po_below(int n) { return n <= 0 ? 0u : n >= 
 // have the 32 columns where their scores were: 16 of rounded weights, 16 of remainders.
 __device__ __forceinline__ constexpr int po_weights_at(int s) { return (s >> 1 & 3) * 32 + (s >> 3) * 16 + (s & 1) * 8; }
 
-struct PortionPlan { int hpc, hpc_shift, tiles, box_rows, page_shift, gate_vec, tab_row; int* timeouts; };    // set by the launch
+struct PortionPlan { int hpc, hpc_shift, sms, few, box_rows, page_shift, gate_vec, tab_row; int* timeouts; };    // set by the launch
 struct PortionMaps { CUtensorMap q, k, k2, v; };
-struct PortionEntry { int tile, b, hg, len, start, pos0; };
+struct PortionEntry { int t0, end, b, hg, start, pos0; };       // tokens t0 .. end - 1 of sequence b, heads of group hg
 
 // What every role knows of an item.  The key list: kept first keys that the lowest bound of the item hides, in whole boxes, then
 // [jl, j_hi] from a multiple of R on; where the boxes of the kept keys reach that bound, one run from key 0.
@@ -152,8 +152,7 @@ struct PortionItem {
   __device__ __forceinline__ PortionItem(const PortionArgs& a, const PortionPlan& p, const PortionEntry& e) {
     per = 128 >> p.hpc_shift;
     b = e.b;
-    t0 = e.tile * p.tiles * per;
-    end = min(e.len, t0 + p.tiles * per);              // behind the item's last token
+    t0 = e.t0; end = e.end;
     start = e.start; pos0 = e.pos0;
     h0 = e.hg << p.hpc_shift;
     const int R = p.box_rows, keep_r = (a.keep_first + R - 1) & ~(R - 1);
@@ -220,10 +219,44 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
     // The CTA's items: number i of the valid (tile, sequence, heads), late tiles first (they are the longest under a causal mask), for
     // i = c, 2 G - 1 - c, 3 G - 1 - c, 3 G + c, 4 G + c, ..: who begins with a long one gets the short ones, and a round that is not full goes to
     // those with the least so far
-    const int span = p.tiles * (128 >> p.hpc_shift), groups = a.H >> p.hpc_shift, c = blockIdx.x, G = gridDim.x;
-    int k = 0, cum = 0, want = c;
+    const int per_shift = 7 - p.hpc_shift, per = 1 << per_shift, groups = a.H >> p.hpc_shift, c = blockIdx.x;
     auto len_of = [&](int b) { return a.cu != nullptr ? a.cu[b + 1] - a.cu[b] : a.seq_len[b]; };
-    const int len0 = lane < a.n_seqs ? len_of(lane) : 0, least = a.one_token ? 1 : 2;
+    auto pos_of = [&](int b) { return a.cu != nullptr ? 0 : a.seq_pos0[b]; };
+    const int len0 = lane < a.n_seqs ? len_of(lane) : 0, pos00 = lane < a.n_seqs ? pos_of(lane) : 0, least = a.one_token ? 1 : 2;
+    // f(tokens, position of the first) of each sequence, summed over the step's
+    auto over_sequences = [&](auto f) {
+      int n = 0;
+      for (int b = lane; b < a.n_seqs; b += 32) {
+        const int len = b < 32 ? len0 : len_of(b);
+        if (len >= least) n += f(len, b < 32 ? pos00 : pos_of(b));
+      }
+      return __reduce_add_sync(0xffffffffu, n);
+    };
+    // One row tile an item, or two.  An item of two takes a third longer than one of one, so it is the better one once some multiprocessor gets two single
+    // tiles of two thirds of the longest's keys: two where they fill the chip, or where there are more such long single tiles than
+    // multiprocessors.  The host knows the longest portion only, and beside decoded tokens that says little: every CTA counts, with the
+    // same result.  16 heads over 8 of 128, window of 1024, one / two in us: 1500 tokens 34 / 43, 2048 52 / 43, 6 x 200 behind 800 50 / 38.
+    int span = per, G = gridDim.x;
+    if (!p.few) {
+      int keys = 0;
+      int64_t items = static_cast<int64_t>(groups) * over_sequences([&](int len, int pos0) {
+        keys = max(keys, pos0 + len);
+        return (len + 2 * per - 1) >> (per_shift + 1);
+      });
+      span = 2 * per;
+      if (items < p.sms) {
+        keys = __reduce_max_sync(0xffffffffu, keys);
+        const int far = (a.mask > 0 ? min(keys, a.mask) : keys) / 3 * 2;
+        const int n_long = over_sequences([&](int len, int pos0) { return max(((len + per - 1) >> per_shift) - (max(far - pos0, 0) >> per_shift), 0); });
+        if (static_cast<int64_t>(groups) * n_long <= p.sms) {
+          span = per;
+          items = static_cast<int64_t>(groups) * over_sequences([&](int len, int) { return (len + per - 1) >> per_shift; });
+        }
+      }
+      // the CTAs that have a part in it: the others were launched for portions that are not there
+      G = static_cast<int>(max(min(items, static_cast<int64_t>(p.sms)), (items + PO_ITEMS - 1) / PO_ITEMS));
+    }
+    int k = 0, cum = 0, want = c < G ? c : 0x7fffffff;
     for (int tile = (a.max_new + span - 1) / span - 1; tile >= 0 && k < PO_ITEMS; --tile) {
       for (int base = 0; base < a.n_seqs && k < PO_ITEMS; base += 32) {
         const int len = base == 0 ? len0 : base + lane < a.n_seqs ? len_of(base + lane) : 0;
@@ -233,8 +266,8 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
           const int at = want - cum, rank = at / groups;
           const int at_b = static_cast<int>(__fns(live, 0, rank + 1));
           if (lane == at_b)
-            list[k] = PortionEntry{tile, base + lane, at - rank * groups, len, a.cu != nullptr ? a.cu[base + lane] : a.seq_start[base + lane],
-                                   a.cu != nullptr ? 0 : a.seq_pos0[base + lane]};
+            list[k] = PortionEntry{tile * span, min(len, (tile + 1) * span), base + lane, at - rank * groups, a.cu != nullptr ? a.cu[base + lane] : a.seq_start[base + lane],
+                                   base == 0 ? pos00 : pos_of(base + lane)};
           ++k;
           want = k * G + ((k + 1) >> 1 & 1 ? G - 1 - c : c);
         }
@@ -599,7 +632,7 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
               for (int c = 0; c < 32; ++c) v[c] = __float_as_uint(-__uint_as_float(v[c]));
             } else {
               const PortionEntry& e = list[x];
-              const int tk = (e.tile * p.tiles + tg) * (128 >> p.hpc_shift) + (r >> p.hpc_shift), pos = e.pos0 + min(tk, e.len - 1);
+              const int tk = e.t0 + tg * (128 >> p.hpc_shift) + (r >> p.hpc_shift), pos = e.pos0 + min(tk, e.end - 1);
               const PortionItem it(a, p, e);
               const float* at = my_tab + (pos - (j * PO_N + half * HK + it.jl) - part);
 #pragma unroll
@@ -764,12 +797,12 @@ int launch_portion_attn(const char* what, const PortionArgs& a, cudaStream_t st)
   p.box_rows = 64;
   while (a.block_tables != nullptr && a.page % p.box_rows) p.box_rows /= 2;
   p.gate_vec = a.gate != nullptr && aligned16(a.gate) && a.ldg % 8 == 0;
-  // two row tiles an item share its key tiles; one, where two would leave multiprocessors without an item
+  // A CTA per multiprocessor, or as many as their lists have room for; the kernel counts the items that there are
   const int per = 128 >> p.hpc_shift;
   auto items = [&](int tiles) { return static_cast<int64_t>((a.max_new + tiles * per - 1) / (tiles * per)) * (a.H / p.hpc) * a.n_seqs; };
-  p.tiles = items(2) >= sm_count() ? 2 : 1;
-  const int64_t most = items(p.tiles);
-  const int grid = static_cast<int>(std::max<int64_t>(std::min<int64_t>(most, sm_count()), (most + PO_ITEMS - 1) / PO_ITEMS));
+  p.sms = sm_count();
+  p.few = items(1) <= p.sms;                           // single tiles with a multiprocessor each, as long as the portions may be
+  const int grid = static_cast<int>(std::max<int64_t>(std::min<int64_t>(items(1), p.sms), (items(2) + PO_ITEMS - 1) / PO_ITEMS));
   PortionMaps maps{};
   {
     const int64_t dims[3] = {a.d, a.H, a.n_tokens}, strides[2] = {a.q_head, a.q_tok};

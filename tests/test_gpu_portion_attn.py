@@ -114,6 +114,16 @@ def test_several_items_for_every_cta(nat, n):
     _case(nat, [(0, n), (300, n - 700), (0, 1), (5, 33)], H=16, G=8, d=128, dv=128, page=64, mask=200, keep=4, gate="element", seed=n)
 
 
+@pytest.mark.parametrize("seqs", [[(0, 300)] + [(50, 1)] * 40, [(30, 1)] * 33 + [(100, 257), (0, 65)], [(5, 33)] * 40, [(0, 128)] * 8 + [(9, 65), (0, 65)],
+                                  [(300, 200)] * 6, [(50, 1)] * 240 + [(0, 130), (70, 400)]])
+def test_portions_beside_decoded_tokens(nat, seqs):
+    """One or two row tiles an item, by how many single ones (64 tokens of 2 of 16 heads) the portions really have: 40, 56, 160 and 80 take one, 320 and
+    192 long ones two, where there are 148 multiprocessors.  Their longest portion, taken for all, says two everywhere, and
+    more CTAs than multiprocessors in the last step."""
+    _case(nat, seqs, H=16, G=8, d=128, dv=128, page=64, mask=100, keep=3, gate="head", seed=len(seqs))
+    _sigmoid_case(nat, seqs, 16, 8, 128, 120, page=64)
+
+
 def test_values_nobody_sees_may_be_infinite(nat):
     """Rows in front of the window, behind the last key and beyond the kept ones share tiles with visible rows."""
     _case(nat, [(700, 150), (90, 60)], H=4, G=2, d=64, dv=64, page=64, mask=100, keep=5, poison=True, f32=True)
