@@ -480,8 +480,9 @@ extern "C" int b2tts_varlen_attn_prefill(const void* q, int64_t q_row_stride,
                "%s: page_size %d must be a positive multiple of %d", what, page_size, ATT_TILE);
   // long prompts: tcgen05 kernels; short ones: one CTA per query token below
   static const bool tc_enabled = [] { const char* e = getenv("B2TTS_PREFILL_TC"); return !(e && e[0] == '0'); }();
-  // prompts that are their own keys (the same sequence starts for both): portion_attn.cu, two query tiles over a ring of key tiles;
-  // keys of their own starts: attention_prefill_tc.cu.  4096 + 1531 tokens, 16 heads over 8: 152 us there, 100 here
+  // prompts that are their own keys, which the host sees where both starts are one tensor (as the runners pass them): portion_attn.cu, two query
+  // tiles over a ring of key tiles; two tensors, whose values it does not see, may differ: attention_prefill_tc.cu.  Both round at the same places;
+  // sums are in another order.  4096 + 1531 tokens, 16 heads over 8: 152 us there, 114 here
   if (tc_enabled && !block_table && cu_seqlens_q == cu_seqlens_k && total_q == total_k && head_dim == 128 && max_seqlen_q >= 128) {
     using B = __nv_bfloat16;
     row::PortionArgs a{};

@@ -1,7 +1,8 @@
 // attention_prefill_tc.cu - a3 at its real size: varlen causal prefill attention on the 5th-gen tensor cores.
 // Replaces flash_attn_varlen_func(q, k, v, cu_seqlens_q/k, max_seqlen_q/k, softmax_scale, causal=True) as called from
 // Attention.forward's prefill branch (layers/attention.py:78-91) when the prompt is long enough for the work to be a
-// real contraction - the voice-clone ICL prompt is ~4096 tokens: 2*T^2*128*16 / 2 = 69 GFLOP
+// real contraction, with sequence starts of their own for queries and keys (the runners pass the same starts for both, which portion_attn.cu
+// takes, or a block table) - the voice-clone ICL prompt is ~4096 tokens: 2*T^2*128*16 / 2 = 69 GFLOP
 // per layer, tensor-bound.  (Short prompts and the paged prefix-cache variant stay on paged_attn_kernel<G,true>.)
 //
 // One CTA = 128 queries of one (sequence, q head); K/V are walked in 128-key tiles up to the causal diagonal:
@@ -143,12 +144,19 @@ prefill_attn_tc_kernel(const PrefillTcParams p, const __grid_constant__ CUtensor
 
   const int q0 = __ldg(p.cu_q + seq), lq = __ldg(p.cu_q + seq + 1) - q0;
   const int k0 = __ldg(p.cu_k + seq), lk = __ldg(p.cu_k + seq + 1) - k0;
-  if (tile * PF_BM >= lq || lk <= 0) return;                        // uniform over the CTA
+  if (tile * PF_BM >= lq) return;                                   // uniform over the CTA
   const int offset = lk - lq;                                       // bottom-right aligned causal mask
   const int rows_valid = min(PF_BM, lq - tile * PF_BM);
   // last key any valid row of this tile may see
   int last_key = tile * PF_BM + rows_valid - 1 + offset;
   if (last_key > lk - 1) last_key = lk - 1;
+  if (last_key < 0) {                                               // fewer keys than queries: none of these sees one.  Zeros, before any wait
+    for (int i = threadIdx.x; i < rows_valid * (PF_HD / 8); i += PF_THREADS) {
+      const int64_t row = q0 + tile * PF_BM + i / (PF_HD / 8);
+      stg_v4(p.out + (row * p.num_heads + head) * PF_HD + i % (PF_HD / 8) * 8, make_uint4(0u, 0u, 0u, 0u));
+    }
+    return;
+  }
   const int n_tiles = last_key / PF_BN + 1;
 
   if (threadIdx.x == 0) {

@@ -176,6 +176,26 @@ def test_prompts_that_are_their_own_keys(nat, H, G, lens):
     assert nat.portion_attn_timeouts() == 0
 
 
+@pytest.mark.parametrize("lens_q,lens_k", [((300, 130), (300, 130)), ((300, 64, 130), (1000, 64, 131)), ((200, 500, 40, 130), (300, 100, 0, 20))])
+def test_prompts_with_key_starts_of_their_own(nat, lens_q, lens_k):
+    """Queries are the last of their sequence's tokens; those that would lie in front of its first key see nothing and get zeros."""
+    H, G, d = 4, 2, 128
+    g = torch.Generator(device=DEV).manual_seed(sum(lens_k))
+    r = lambda *s: torch.randn(s, generator=g, device=DEV).to(BF)
+    cu = lambda lens: torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32, device=DEV)
+    q, k, v = r(sum(lens_q), H, d), r(sum(lens_k), G, d), r(sum(lens_k), G, d)
+    out = nat.varlen_attn_prefill(q, k, v, cu(lens_q), cu(lens_k), max(lens_q), max(lens_k), d ** -0.5).view(-1, H, d).to(F64)
+    a = b = 0
+    for n, m in zip(lens_q, lens_k):
+        kk, vv = (t[b:b + m].to(F64).repeat_interleave(H // G, 1) for t in (k, v))
+        s = torch.einsum("ihd,jhd->hij", q[a:a + n].to(F64), kk) * d ** -0.5
+        seen = torch.arange(m, device=DEV)[None] <= torch.arange(m - n, m, device=DEV)[:, None]
+        ref = torch.einsum("hij,jhd->ihd", s.masked_fill(~seen, -math.inf).softmax(-1).nan_to_num(0.0), vv)
+        # weights rounded once to 2^-9 and averaged, results rounded to 2^-9
+        assert ((out[a:a + n] - ref).abs().max() <= 6e-3 * ref.abs().max()), (n, m)
+        a, b = a + n, b + m
+
+
 @pytest.mark.parametrize("sharp", [0.3, 1, 3, 10])
 def test_prompts_are_no_further_from_64_bits_than_tile_by_tile(nat, sharp):
     """Weights rounded once: as far from 64 bits as the kernel for starts of their own, whose largest weight of a row is exact.  (A maximum behind
