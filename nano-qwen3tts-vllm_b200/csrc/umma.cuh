@@ -173,14 +173,15 @@ __device__ __forceinline__ uint4 norm8(uint4 x, uint4 w, float rs, bool eager) {
   return o;
 }
 
-// Wait for phase `parity` of an mbarrier, giving up after a bounded number of polls.
+// Wait for phase `parity` of an mbarrier, giving up after a bounded number of polls.  A whole warp calls it and gets one answer: lanes that gave up on
+// their own would part from the others in front of instructions that need all of them.
 __device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity, int polls = 1 << 20) {
   const uint32_t addr = smem_u32(bar);
   for (int i = 0; i < polls; ++i) {
     uint32_t ok;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(ok) : "r"(addr), "r"(parity) : "memory");
-    if (ok) return true;
+    if (__all_sync(0xffffffffu, ok)) return true;
   }
   return false;
 }
