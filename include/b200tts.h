@@ -510,8 +510,11 @@ B2TTS_API int b2tts_grouped_gemm_silu(const void* a, int64_t lda, const void* w,
 B2TTS_API int b2tts_grouped_gemm_timeouts(void);
 B2TTS_API int b2tts_grouped_gemm_check(void);
 B2TTS_API int b2tts_grouped_gemm_lose_wait(void* stream);
-/* How often a wait inside the tcgen05 kernel of prompt attention ran out since the library was loaded (expected: 0). */
+/* The same for the tcgen05 kernel of prompt attention: how often a wait inside it ran out since the library was loaded (expected: 0), how often the
+ * kernel was launched (or captured), and a kernel whose wait runs out, for tests. */
 B2TTS_API int b2tts_portion_attn_timeouts(void);
+B2TTS_API unsigned long long b2tts_portion_attn_launches(void);
+B2TTS_API int b2tts_portion_attn_lose_wait(void* stream);
 
 /* ---- decoders with latent attention, token shift and a norm on each sublayer's output (csrc/latent_ops.cu, latent_attn.cu).
  * `dtype` is the activation / cache type (B2TTS_DTYPE_*); x is the float residual stream [rows, cols]. */

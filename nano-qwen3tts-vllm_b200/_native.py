@@ -123,6 +123,8 @@ def _load():
         "b2tts_sink_attn": (I, [P, P, P, P, P, P, P, P, P, P, L, P, P, L, I, I, I, I, I, I, I, I, I, I, I, I, I, F, F, I, I, I, P]),
         "b2tts_sink_attn_rows": (I, [P, P, P, P, P, P, P, P, P, P, L, P, P, L, I, I, I, I, I, I, I, I, I, I, I, I, I, F, F, I, I, I, L, I, P]),
         "b2tts_portion_attn_timeouts": (I, []),
+        "b2tts_portion_attn_launches": (ctypes.c_ulonglong, []),
+        "b2tts_portion_attn_lose_wait": (I, [P]),
         "b2tts_latent_gather": (I, [P, L, P, P, P, L, P, P, I, I, I, I, I, I, P]),
         "b2tts_latent_turn": (I, [P, L, L, I, P, P, F, I, I, I, P]),
         "b2tts_latent_portions_attn": (I, [P, L, L, P, L, P, L, P, L, L, P, P, P, P, L, I, P, P, P, I, I, I, I, I, I, I, I, F, P]),
@@ -1175,6 +1177,11 @@ def sink_attn(q, k_cache, v_cache, out, lay, sink, gate, heads, kv_heads, dim, v
 def portion_attn_timeouts() -> int:
     """Bounded waits of the prompt attention kernel that ran out since the library was loaded (0 when healthy)."""
     return int(_load().b2tts_portion_attn_timeouts())
+
+
+def portion_attn_launches() -> int:
+    """Launches of the prompt attention kernel since the library was loaded: tells which kernel a call has taken."""
+    return int(_load().b2tts_portion_attn_launches())
 
 
 def short_conv_act(u, c_off, channels, w, bias, state, lay, out, taps, act=1):

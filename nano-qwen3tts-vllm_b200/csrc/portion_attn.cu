@@ -45,6 +45,10 @@ constexpr int PO_N = 128, PO_SLOT = 128 * 128;         // keys per tile; bytes o
 constexpr int PO_SOFT = 16, PO_THREADS = 640, PO_ITEMS = 48;           // softmax warps; items a CTA takes at most
 constexpr int PO_MMA = 16, PO_LOADER = 17, PO_CLEANER = 18, PO_LISTER = 19;
 __device__ int g_portion_timeouts = 0;                 // see waits.cuh
+__device__ __forceinline__ void po_report(int* word) {
+  *reinterpret_cast<volatile int*>(word) = atomicAdd(&g_portion_timeouts, 1) + 1;
+  __threadfence_system();
+}
 
 // Low word of an MN-major SWIZZLE_128B operand: a K index (key) is a 128-byte row of 64 columns; LBO: the next 64 columns (the next slot),
 // SBO: 8 keys.  The high word is that of the K-major operands.
@@ -736,16 +740,21 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
       tc_fence_before();                               // the next item's first weights tell the issuer that O may be overwritten
     }
   }
-  if (!ok && lane == 0) {
-    *reinterpret_cast<volatile int*>(p.timeouts) = atomicAdd(&g_portion_timeouts, 1) + 1;
-    __threadfence_system();
-  }
+  if (!ok && lane == 0) po_report(p.timeouts);
   tc_fence_before();
   __syncthreads();
   if (warp == PO_MMA) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
   }
+}
+
+// One wait of the kernel's kind, on a barrier that nothing arrives at, with a short limit, and its report.
+__global__ void portion_lost_wait_kernel(int* word) {
+  __shared__ uint64_t bar;
+  if (threadIdx.x == 0) { mbar_init(&bar, 1); mbar_fence_init(); }
+  __syncwarp();
+  if (!mbar_wait_limit(&bar, 0, 64) && threadIdx.x == 0) po_report(word);
 }
 
 // floats of a row of the distance tables: the rows' tokens, heads and halves of a warp fall into different banks
@@ -771,6 +780,8 @@ bool portion_attn_applies(const PortionArgs& a) {
          (a.gate == nullptr || !a.gate_el || (reinterpret_cast<uintptr_t>(a.gate) % 4 == 0 && a.ldg % 2 == 0));
 }
 
+static unsigned long long g_portion_launches = 0;
+
 template <int NS, int NV, int MODE>
 static int go_portion(const char* what, const PortionArgs& a, const PortionPlan& p, const PortionMaps& maps, int grid, cudaStream_t st) {
   auto kern = portion_attn_kernel<NS, NV, MODE>;
@@ -779,6 +790,7 @@ static int go_portion(const char* what, const PortionArgs& a, const PortionPlan&
   if (e != cudaSuccess) return cuda_fail(e, what);
   kern<<<grid, PO_THREADS, smem, st>>>(a, p, maps);
   B2_CHECK_LAUNCH(what);
+  __atomic_add_fetch(&g_portion_launches, 1ull, __ATOMIC_RELAXED);
   return B2TTS_OK;
 }
 
@@ -873,3 +885,12 @@ extern "C" int b2tts_latent_portions_attn(const void* q, int64_t q_tok, int64_t 
 }
 
 extern "C" int b2tts_portion_attn_timeouts(void) { return b2::wait_count(b2::WAITS_PORTIONS); }
+extern "C" unsigned long long b2tts_portion_attn_launches(void) { return __atomic_load_n(&b2::row::g_portion_launches, __ATOMIC_RELAXED); }
+extern "C" int b2tts_portion_attn_lose_wait(void* stream) {
+  using namespace b2;
+  int* word = wait_word(WAITS_PORTIONS);
+  B2_REQUIRE(word != nullptr, B2TTS_ECUDA, "portion_attn_lose_wait: no host memory");
+  row::portion_lost_wait_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(word);
+  B2_CHECK_LAUNCH("portion_attn_lose_wait");
+  return B2TTS_OK;
+}

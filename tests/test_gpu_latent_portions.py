@@ -108,12 +108,15 @@ def test_portions_over_expanded_keys(nat, monkeypatch, dim, rot, vdim, rank, q_r
         cache = start.clone()
         set_context(False, step_layout=lay)
         with torch.inference_mode():
+            launches = nat.portion_attn_launches()
             got[least] = m(h, cache).to(F64)
+            assert nat.portion_attn_launches() - launches == (least == 32)
     assert taken[0] is not None and taken[1] is None
     err = {k: ((v - ref).norm() / ref.norm()).item() for k, v in got.items()}
     # both forms round their operands to bf16 at as many places (2^-9 each); the expanded one must not be the worse one
     assert err[32] < 1e-2 and err[32] < 1.15 * err[1 << 30], err
-    assert nat.portion_attn_timeouts() == 0
+    torch.cuda.synchronize()
+    nat.check_waits()
 
 
 def test_small_portions_and_decoded_tokens_stay_absorbed(nat):
