@@ -880,10 +880,12 @@ extern "C" int b2tts_sink_attn_rows(const void* q, const void* k_cache, const vo
     p.H = H; p.G = G; p.Gv = Gv; p.d = dim; p.dv = vdim;
     p.mask_kind = mask_kind; p.mask = mask; p.keep_first = keep_first; p.softcap = softcap; p.scale = scale;
     p.n_seqs = n_seqs; p.max_new = max_new;
-    // The tcgen05 kernel takes 9 us to start and end where the other one takes 7; a tile of keys later it is the faster one.  16 heads over 8 of 128,
-    // graphs of ten layers, other / tcgen05 in us: 2 new tokens 15.6 / 17.8 (chunks) and 13.3 / 14.3 (window), 33 new 17.9 / 18.2 and 19.0 / 15.1,
-    // 2 x 64 20.1 / 19.3 and 21.9 / 16.8, 40 behind 1400 36.7 / 25.4 and 72.8 / 37.7, 2 x 2048 227 / 103 and 325 / 104.
-    const bool few = max_keys > 0 && max_keys <= 40;
+    // The tcgen05 kernel takes 3 us more to start and end; a tile of keys later it is the faster one, and sooner where the other one is slow at
+    // element gates or caps, or has more CTAs than fit at once.  16 heads over 8 of 128, other / tcgen05 in us: 41 keys 9.4 / 11.7 (window), 16.6 / 16.2 (element
+    // gates), 13.8 / 12.7 (capped); 64 keys 10.5 / 12.3, 17.6 / 16.4, 12.9 / 13.3; 80 keys 11.7 / 12.5, 18.9 / 16.6, 18.9 / 13.6; 16 x 64 keys 12.5 / 13.7; 16 x 80
+    // 23.1 / 16.6; 64 x 41 33.4 / 28.9; 40 behind 2000 101 / 50; 2048 227 / 52.
+    const bool plain = softcap == 0.f && !(gate != nullptr && gate_el) && static_cast<int64_t>(heads) * n_seqs <= 2 * sm_count();
+    const bool few = max_keys > 0 && max_keys <= (plain ? 64 : 40);
     if (!few && portion_attn_applies(p)) {
       const int rc = launch_portion_attn("sink_attn (portions)", p, st);
       if (rc != B2TTS_OK) return rc;

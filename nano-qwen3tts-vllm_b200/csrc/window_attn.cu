@@ -851,7 +851,9 @@ extern "C" int b2tts_window_sigmoid_attn_rows(const void* q, const void* k_cache
     // The tcgen05 kernel (portion_attn.cu) where the longest sequence is not known to be short: its items start and end in 12 us, the kernel
     // below in 6.  16 heads over 8 of 128, window 1024, below / tcgen05 in us: 64 new tokens 8.3 / 12.5, 400 20.7 / 21.9, 3 x 300 21.9 / 19.8,
     // 700 41 / 30, 40 behind 1000 44 / 40, 4 x 100 behind 800 39 / 36, 2048 100 / 70; 2048 + 1333 + 700 + 57 143 / 79.
-    const bool few = max_keys > 0 && max_keys <= 420;
+    // Portions shorter than a row tile of 128 (token, head) rows leave most of it empty: more of them than multiprocessors stay below too (64 x 16 behind
+    // 500 73 / 104, 64 x 2 behind 1500 129 / 153, 32 x 64 behind 600 72 / 65; 16 x 2 behind 1500 50 / 41).
+    const bool few = max_keys > 0 && (max_keys <= 420 || (max_new <= 32 && static_cast<int64_t>(kv_heads) * n_seqs > sm_count()));
     if (!few && row::portion_attn_applies(p)) return row::launch_portion_attn("window_sigmoid_attn (portions)", p, st);
     // One head and 32-key tiles per CTA, four CTAs per SM: independent CTAs overlap their MMA and weight phases better
     // than a wider CTA in which two heads share the K/V tiles (306 against 322 us at 4 x 2048 tokens, window 1024).

@@ -11,7 +11,6 @@ DEV = "cuda:0"
 BF = torch.bfloat16
 F64 = torch.float64
 LOST = [0]                                            # waits that ran out on purpose
-SHORT = 40                                            # keys up to which softmax attention whose longest portion is known stays with the other kernel
 
 
 @pytest.fixture(scope="module")
@@ -85,7 +84,9 @@ def _case(nat, seqs, *, H=4, G=2, Gv=None, d=64, dv=64, page=16, kind="window", 
         o += n
     ref = torch.cat(ref)
     out = torch.empty(n_tok, H * dv, dtype=torch.float32 if f32 else BF, device=DEV)
-    with _Takes(nat, not known or lay.max_keys > SHORT):
+    # the longest portion's keys up to which the other kernel is the faster one, where they are known
+    short = 64 if cap == 0 and gate != "element" and H * lay.n_seqs <= 296 else 40
+    with _Takes(nat, not known or lay.max_keys > short):
         nat.sink_attn(q.to(DEV), kc.to(BF).to(DEV), vc.to(BF).to(DEV), out, lay, sk.to(DEV) if sink else None, gt.to(DEV) if gate else None, H, G, d, dv,
                       page, nat.MASK_WINDOW if kind == "window" else nat.MASK_CHUNK, mask, scale, nat.SINK_ATTN_TENSOR, v_heads=Gv, keep_first=keep,
                       softcap=cap, gate_el=gate == "element")
@@ -148,9 +149,11 @@ def test_values_nobody_sees_may_be_infinite(nat):
     _case(nat, [(700, 150), (90, 60)], H=4, G=2, d=64, dv=64, page=64, mask=100, keep=5, poison=True, f32=True)
 
 
-@pytest.mark.parametrize("keys", [2, 39, 40, 41, 64])
-def test_short_sequences_that_the_host_knows_of(nat, keys):
-    _case(nat, [(keys - 2, 2), (0, min(keys, 33)), (0, 1)], H=8, G=4, d=128, dv=128, page=64, mask=30, keep=2, gate="element", known=True, seed=keys)
+@pytest.mark.parametrize("keys", [2, 39, 40, 41, 64, 65])
+@pytest.mark.parametrize("gate,cap,more", [("element", 0.0, 0), ("head", 0.0, 0), (None, 20.0, 0), (None, 0.0, 40)])
+def test_short_sequences_that_the_host_knows_of(nat, keys, gate, cap, more):
+    _case(nat, [(keys - 2, 2), (0, min(keys, 33)), (0, 1)] + [(1, 3)] * more, H=8, G=4, d=128, dv=128, page=64, mask=30, keep=2, gate=gate, cap=cap,
+          known=True, seed=keys)
 
 
 @pytest.mark.parametrize("H,G", [(2, 2), (4, 2), (6, 2), (16, 1)])
@@ -282,6 +285,12 @@ def test_sigmoid_weights_of_sequences_that_the_host_knows_of(nat, keys):
     _sigmoid_case(nat, [(keys - 40, 40), (0, 33)], 4, 2, 64, 90, page=16, known=True)
 
 
+@pytest.mark.parametrize("new,more", [(32, 17), (33, 17), (32, 18), (33, 18)])
+def test_sigmoid_weights_of_many_short_portions(nat, new, more):
+    """Of 148 multiprocessors: 18 sequences of 8 key heads, and 19, which leave portions of up to 32 tokens to the other kernel."""
+    _sigmoid_case(nat, [(500, new)] + [(9, 5)] * more, 16, 8, 64, 90, page=64, known=True)
+
+
 def _sigmoid_case(nat, seqs, H, G, d, window, page, scale=None, known=False):
     from tests.lm_util import Lay
     g = torch.Generator().manual_seed(H * d + window)
@@ -309,7 +318,8 @@ def _sigmoid_case(nat, seqs, H, G, d, window, page, scale=None, known=False):
         o += n
     ref = torch.cat(ref)
     out = torch.empty(lay.n_tokens, H * d, dtype=BF, device=DEV)
-    with _Takes(nat, (not known or lay.max_keys > 420) and H // G <= 8):               # more heads a key head stay with the plain kernel
+    few = known and (lay.max_keys <= 420 or (lay.max_new <= 32 and G * lay.n_seqs > 148))
+    with _Takes(nat, not few and H // G <= 8):               # more heads a key head stay with the plain kernel
         nat.window_sigmoid_attn(q.to(DEV), kc.to(BF).to(DEV), vc.to(BF).to(DEV), out, lay, r1.to(DEV), r2.to(DEV), pb.to(DEV), H, G, d, d, page, window, scale)
     # weights carry 16 bits; the results round to 2^-9
     err = (out.double().cpu() - ref).abs().max() / ref.abs().max()
