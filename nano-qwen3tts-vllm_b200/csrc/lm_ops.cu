@@ -700,7 +700,7 @@ moe_route_kernel(const T* __restrict__ h, const RouteArgs p) {
       for (int t = 0; t < TOK; ++t) acc[t][x] = 0.f;
     }
     if constexpr (V == 4) {
-#pragma unroll 2
+#pragma unroll (EXP == 1 ? 4 : 2)
       for (int c = lane * 4; c < cols; c += 128) {
         float4 w[EXP];
 #pragma unroll
@@ -797,8 +797,18 @@ static cudaError_t launch_route(const void* h, const RouteArgs& p, cudaStream_t 
   const int tok = many ? ROUTE_TOKENS : 1;
   const bool vec = p.cols % 4 == 0 && aligned16(h) && aligned16(p.router);
   const int grid = (p.n_tokens + tok - 1) / tok;
+  // Experts a warp takes at a time.  One token a CTA waits for its loads: up to four, as even over the warp's turns as can be (64 tokens of 17 experts 14
+  // -> 10 us, of 64 30 -> 18).  Eight tokens are bound by their sums, which a place without an expert costs as well: two at a time take 0.93, four 0.84 of one's time
+  // a place (4096 tokens of 64 experts 117 -> 100 us; of 17, four at a time 39, one 34).
+  const int per_warp = (p.E + ROUTE_WARPS - 1) / ROUTE_WARPS, turns = (per_warp + 3) / 4;
+  int exp = (per_warp + turns - 1) / turns;
+  if (many) {
+    const int one = per_warp * 100, two = (per_warp + 1) / 2 * 2 * 93, four = turns * 4 * 84;
+    exp = four < one && four <= two ? 4 : two < one ? 2 : 1;
+  }
 #define ROUTE_GO(TOK, V) do { \
-    auto kern = p.E > 2 * ROUTE_WARPS ? moe_route_kernel<T, TOK, V, 4> : p.E > ROUTE_WARPS ? moe_route_kernel<T, TOK, V, 2> : moe_route_kernel<T, TOK, V, 1>; \
+    auto kern = exp == 4 ? moe_route_kernel<T, TOK, V, 4> : exp == 3 ? moe_route_kernel<T, 1, V, 3> : \
+                exp == 2 ? moe_route_kernel<T, TOK, V, 2> : moe_route_kernel<T, TOK, V, 1>; \
     if (smem(TOK) > 48 * 1024) { \
       const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); \
       if (e != cudaSuccess) return e; \
