@@ -484,7 +484,7 @@ extern "C" int b2tts_varlen_attn_prefill(const void* q, int64_t q_row_stride,
   // tiles over a ring of key tiles; two tensors, whose values it does not see, may differ: attention_prefill_tc.cu.  Both round at the same places;
   // sums are in another order.  That kernel's CTAs, a head's 128 queries each, start and end in 4 us and this one's items in 9, so it needs
   // about one and a half rounds of them over the chip to be the faster one, and up to three of short ones.  16 heads over 8, there / here in us:
-  // 200 tokens 7.6 / 11.4, 1000 18 / 26, 1500 33 / 35, 1800 46 / 41, 4096 + 1531 144 / 108; 8 x 200 15 / 20, 16 x 200 26 / 23; 24 x 128 18 / 22, 32 x 128
+  // 200 tokens 7.6 / 11.4, 1000 18 / 26, 1500 33 / 35, 1800 46 / 41, 4096 + 1531 144 / 107; 8 x 200 15 / 20, 16 x 200 26 / 23; 24 x 128 18 / 22, 32 x 128
   // 24 / 22; 4 x 400 20 / 22, 6 x 400 27 / 24; 2 x 700 21.6 / 22.4, 3 x 700 27 / 26; 32 heads: 200 7.9 / 12.1, 1000 31 / 32, 2048 81 / 57.
   const int64_t tile_ctas = (total_q + 64ll * num_seqs) / 128 * num_heads, key_tiles = (max_seqlen_q + 127) / 128;
   const bool many = tile_ctas * key_tiles * 10 > (14 * key_tiles + 18) * sm_count();

@@ -706,7 +706,7 @@ template <typename T> struct RowVec {
 // What bounds it is the rows' traffic once they are in flight early enough: every row of the run is asked for before the first is
 // used (the loads sat behind the previous token's activation before, one 16-byte load in flight a thread), and a thread's filters are
 // contiguous and come as 16-byte vectors (as scalars a warp's load touched 32 lines).  8192 tokens of 4352 channels: 129 -> 78 us, with the
-// special-function forms of the activation 50.
+// approximate quotient of the activation 58.
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(128)
 short_conv_act_run_kernel(const T* __restrict__ u, int64_t ldu, const float* __restrict__ w, const float* __restrict__ bias,
@@ -854,7 +854,7 @@ gated_group_norm_vec4_kernel(const float* __restrict__ y, const T* __restrict__ 
   };
   // a group of up to GN_KEEP vectors per thread stays in registers between the sum of squares and the scaled write; all of them are
   // asked for before the first gate is formed (8192 rows of 4096: 89 -> 71 us, with the
-  // special-function forms of the gates 53; behind each other's gates the loads came one at a time)
+  // approximate quotient of the gates 59; behind each other's gates the loads came one at a time)
   constexpr int GN_KEEP = 4;
   const bool keep = gs <= 4 * GN_KEEP * static_cast<int>(blockDim.x);
   float4 kv[GN_KEEP], kg[GN_KEEP];

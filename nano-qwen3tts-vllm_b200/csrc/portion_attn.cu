@@ -16,7 +16,7 @@
 //             zero, but what a page holds there may be infinite.
 // A row's maximum is the running one: where one key has most of the weight, its weight is then 1 and carries no rounding.  (A lazy one, moved in steps
 // of 2^8, left it a weight with a rounding of its own: outputs of 2000 peaked keys 1.21 times as far from 64 bits with weights
-// rounded once, 1.9 times with pairs in float.  O is scaled more often for it: layers 2 % longer.)  The sum is that of the weights as the
+// rounded once, 1.9 times with pairs in float.  O is scaled more often for it: layers 2 % longer, single tiles 10 %.)  The sum is that of the weights as the
 // products see them, rounded, so that what rounding adds to all of them cancels.
 //
 // Bound: the issue of the tensor core's products.  A key tile of a row tile is 24 of them of 64 cycles (1536); the issuer's own instructions and
@@ -24,14 +24,16 @@
 // starts and ends in about 12000 cycles (first key tile under a mask, last products, division and gates).  Two threads a row and 64 scores
 // each in two passes over TMEM keep everything in 96 registers: spilled ones went through L2, since shared memory leaves L1 next to nothing
 // (one thread a row with 40 spilled registers: 143 us for the case below; one barrier per slot of the ring instead of per tile: 20 us more).
-// 4 prompts of 2048 tokens, 16 heads over 8 of 128, window 1024 + 4 kept, element gates: 118 us (mma.sync, 64 queries per CTA: 547 us; 31 at
-// the tensor core's rate); causal with a score cap, 4448 tokens: 141 us (579 us); latent
-// heads of 192 over expanded keys, 4 x 2048 causal: 142 us; prompts that
-// are their own keys, weights rounded once, 4096 + 1531 causal: 100 us (152 us one query tile a CTA).  Sigmoid weights (two special-function results and a table's number a pair), window
-// 1024, 4138 tokens: 79 us (143 us).
+// 4 prompts of 2048 tokens, 16 heads over 8 of 128, window 1024 + 4 kept, element gates: 131 us (mma.sync, 64 queries per CTA: 547 us; 31 at
+// the tensor core's rate; 123 with the lazy maximum); causal with a score cap, 4448 tokens: 133 us (579 us); latent
+// heads of 192 over expanded keys, 4 x 2048 causal: 150 us; prompts that are their own keys, weights rounded once, 4096 + 1531 causal: 114 us (152 us
+// one query tile a CTA).  Sigmoid weights (two special-function results and a table's number a pair), window 1024, 4138 tokens: 77 us (143 us).
+//
+// Values that a query does not see have a weight of zero, and zero times infinity is not a number: an infinite value that some query of an item sees
+// reaches the others that share its key tile, up to two row tiles of tokens (256 / HPC) in front of it.  On mma.sync that is up to 78 tokens.
 //
 // Every copy is bounded: maps have the true extents of their tensors, so a row that a block table should not name reads zeros.  Every
-// commit of the last products is waited for before the CTA leaves.
+// commit of the last products is waited for before the CTA leaves.  tests/test_portion_bookkeeping.py plays the items, ring and barriers on the CPU.
 #include <algorithm>
 
 #include "portion_attn.cuh"
@@ -226,7 +228,9 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
     const int per_shift = 7 - p.hpc_shift, per = 1 << per_shift, groups = a.H >> p.hpc_shift, c = blockIdx.x;
     auto len_of = [&](int b) { return a.cu != nullptr ? a.cu[b + 1] - a.cu[b] : a.seq_len[b]; };
     auto pos_of = [&](int b) { return a.cu != nullptr ? 0 : a.seq_pos0[b]; };
-    const int len0 = lane < a.n_seqs ? len_of(lane) : 0, pos00 = lane < a.n_seqs ? pos_of(lane) : 0, least = a.one_token ? 1 : 2;
+    auto start_of = [&](int b) { return a.cu != nullptr ? a.cu[b] : a.seq_start[b]; };
+    const bool here = lane < a.n_seqs;                 // the first 32 sequences' numbers stay in registers
+    const int len0 = here ? len_of(lane) : 0, pos00 = here ? pos_of(lane) : 0, start0 = here ? start_of(lane) : 0, least = a.one_token ? 1 : 2;
     // f(tokens, position of the first) of each sequence, summed over the step's
     auto over_sequences = [&](auto f) {
       int n = 0;
@@ -270,7 +274,7 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
           const int at = want - cum, rank = at / groups;
           const int at_b = static_cast<int>(__fns(live, 0, rank + 1));
           if (lane == at_b)
-            list[k] = PortionEntry{tile * span, min(len, (tile + 1) * span), base + lane, at - rank * groups, a.cu != nullptr ? a.cu[base + lane] : a.seq_start[base + lane],
+            list[k] = PortionEntry{tile * span, min(len, (tile + 1) * span), base + lane, at - rank * groups, base == 0 ? start0 : start_of(base + lane),
                                    base == 0 ? pos00 : pos_of(base + lane)};
           ++k;
           want = k * G + ((k + 1) >> 1 & 1 ? G - 1 - c : c);
@@ -717,10 +721,13 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
         if (gated) {
           const uint32_t w[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
           if (c + 16 < OC) gates(c + 16);
+          if (a.out_f32) {
 #pragma unroll
-          for (int e = 0; e < 16; ++e) {
-            const float u = e & 1 ? bf16hi(w[e >> 1]) : bf16lo(w[e >> 1]);
-            o[e] = __float_as_uint(__uint_as_float(o[e]) * sigmoid_f(u));
+            for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * sigmoid_f(e & 1 ? bf16hi(w[e >> 1]) : bf16lo(w[e >> 1])));
+          } else {                                     // rounded to bf16 behind it: 203 us the window layer below, 208 with exact divisions
+#pragma unroll
+            for (int e = 0; e < 16; ++e)
+              o[e] = __float_as_uint(__uint_as_float(o[e]) * sigmoid_for<__nv_bfloat16>(e & 1 ? bf16hi(w[e >> 1]) : bf16lo(w[e >> 1])));
           }
         }
         if (tk <= t_last && a.out_f32) {

@@ -13,8 +13,9 @@
 // maps over one set of values).
 //
 // Four kernels share a launch: prompt portions in bf16 with head sizes 64, 128 x 64, 128 run on tcgen05 (portion_attn.cu), those with
-// other head sizes from 32 on or odd pages, and very short sequences, on mma.sync (sink_attn_mma_kernel), rows with ONE new token and a head size of 4, 8, 16 or 32 16-byte pieces (dv = d or 2 d) in a kernel whose
-// lanes split a cached row (sink_attn_decode_kernel), everything else in the plain kernel; each skips the rows of the others.
+// other head sizes from 32 on or odd pages, and steps whose longest portion is known to be short, on mma.sync (sink_attn_mma_kernel), rows with ONE
+// new token and a head size of 4, 8, 16 or 32 16-byte pieces (dv = d or 2 d) in a kernel whose lanes split a cached row
+// (sink_attn_decode_kernel), everything else in the plain kernel; each skips the rows of the others.
 //
 // Plain kernel (bf16 or float, any head size up to 256): one CTA of four warps per token and 1, 2 or 4 query heads of one
 // key/value group, so a cached row is loaded once for all of them.  A warp takes 32-key tiles: each lane scores one key

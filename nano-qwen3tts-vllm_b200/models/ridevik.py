@@ -90,7 +90,8 @@ class LatentAttentionMixer(nn.Module):
     # tcgen05 kernel takes.  16 heads, width 2048, a mixer in us, absorbed / expanded: 4 x 2048 causal 1967 / 365; 2048 610 / 152; 800 169 /
     # 150; 200 new behind 1400 145 / 158; 500 138 / 163.  The small ones are bound by the host, which has two launches more to make (on the
     # device alone, from a graph, the lines cross at 100 tokens), so the least number of pairs, over all heads, lies where the absorbed
-    # form's own time passes that.  Decode steps, steps with a portion of a few tokens and float32 stay with the absorbed form.
+    # form's own time passes that.  Few queries behind many keys do not turn it over, since the expansion runs at the rate of the library's products:
+    # 32 new behind 4000 287 / 263, behind 17000 857 / 555, 8 x 32 behind 8000 631 / 562, 64 x 32 behind 300 337 / 301.  Decode steps, steps with a portion of a few tokens and float32 stay with the absorbed form.
     EXPAND_MIN_NEW, EXPAND_MIN_PAIRS = 32, 1 << 23
     EXPAND_MAX_BYTES = 1 << 30                 # of expanded keys and values
 
