@@ -1,5 +1,5 @@
 """Summarise an ncu `--metrics gpu__time_duration.sum --csv` launch list by kernel name.
-    python tools/summarize_launches.py gpurun_out/launches.csv > profiles/<round>_launches_summary.txt"""
+    python tools/summarize_launches.py launches.csv > summary.txt"""
 import collections
 import csv
 import re
