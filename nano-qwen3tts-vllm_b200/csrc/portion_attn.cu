@@ -502,7 +502,11 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
         const PortionItem it(a, p, list[x]);
         if (!it.has(tg)) continue;
         span = PortionSpan(a, it, tg);
-        if (!SIG && a.sink != nullptr) { m = a.sink[it.h0 + (r & (p.hpc - 1))] * LOG2E; l = half == 0 ? 1.f : 0.f; }
+        if (!SIG && a.sink != nullptr) {
+          const float s = a.sink[it.h0 + (r & (p.hpc - 1))] * LOG2E;
+          m = s < m ? m : s;                           // a sink that is off (-inf, the lowest float) leaves the maximum finite: its weight is 0 behind the first key
+          l = half == 0 ? 1.f : 0.f;
+        }
         const int t_first = it.t0 + tg * it.per, t_last = min(it.end, t_first + it.per) - 1;
         const int lo = po_mask_lo(it.pos0 + min(t_first + ((r0 + 15) >> p.hpc_shift), t_last), a.mask_kind, a.mask);    // the highest of its rows
         whole0 = (max(lo - it.jl, 0) + it.pre_r + PO_N - 1) / PO_N;

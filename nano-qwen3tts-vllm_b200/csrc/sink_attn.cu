@@ -636,7 +636,8 @@ sink_attn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* _
   // running maximum and (this thread's share of the) denominator of its two rows; the sink is counted by one lane of four
   float m0 = -1e30f, m1 = -1e30f, l0 = 0.f, l1 = 0.f;
   if (sink != nullptr) {
-    m0 = m1 = sink[h] * LOG2E;
+    const float s = sink[h] * LOG2E;
+    m0 = m1 = s < m0 ? m0 : s;                         // a sink that is off leaves the maximum finite
     if ((lane & 3) == 0) l0 = l1 = 1.f;
   }
 

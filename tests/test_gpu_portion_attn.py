@@ -326,6 +326,27 @@ def _sigmoid_case(nat, seqs, H, G, d, window, page, scale=None, known=False):
     assert err.item() < 4e-3, err.item()
 
 
+@pytest.mark.parametrize("known", [0, 1])                             # 1: said to be short, which is the other kernel's
+@pytest.mark.parametrize("off", [-math.inf, torch.finfo(torch.float32).min, -1e31])
+@pytest.mark.parametrize("kind,mask", [("window", 50), ("chunk", 100)])
+def test_sinks_that_are_off(nat, known, off, kind, mask):
+    """A sink of the lowest value is no sink, also for rows that see nothing of their tile's first keys (128 tokens a row tile here)."""
+    from tests.lm_util import Lay
+    n, H, G, d, page = 400, 2, 2, 64, 16
+    g = torch.Generator(device=DEV).manual_seed(5)
+    r = lambda *s: torch.randn(s, generator=g, device=DEV).to(BF)
+    pages = -(-n // page)
+    q, kc, vc, got = r(n, H * d), r(pages, page, G * d), r(pages, page, G * d), []
+    for sink in (None, torch.full((H,), off, device=DEV)):
+        lay, out = Lay([(0, n, list(range(pages)))], page, pages), torch.empty(n, H * d, device=DEV)
+        lay.max_keys = known
+        with _Takes(nat, known == 0):
+            nat.sink_attn(q, kc, vc, out, lay, sink, None, H, G, d, d, page, nat.MASK_WINDOW if kind == "window" else nat.MASK_CHUNK,
+                          mask, d ** -0.5)
+        got.append(out)
+    assert torch.equal(*got)
+
+
 @pytest.mark.parametrize("path", ["softmax", "sigmoid"])
 def test_a_wait_that_ran_out_is_an_error(nat, path):
     """The next launch refuses once, and so does the check that the engines make; the next call after that runs again."""
