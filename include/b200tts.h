@@ -693,9 +693,10 @@ B2TTS_API int b2tts_delta_rule_scan_portions(const void* qkv, int64_t ldq, const
                                              const int32_t* seq_start, const int32_t* seq_pos0, const int32_t* seq_len,
                                              const int32_t* seq_slot, int n_tokens, int n_seqs, int max_new, int heads, int kv_heads, int dim,
                                              int vdim, int dtype, void* stream);
-/* The same with room for what long portions' keys and queries alone say (_floats() of them, 16-byte aligned; null: none), formed once a key
- * head.  The results are the same numbers; rows in any order. */
-B2TTS_API size_t b2tts_delta_rule_scan_ahead_floats(int n_tokens, int n_seqs, int kv_heads);
+/* The same with room for what the chunks of long portions say without the state (16-byte aligned; null: none): _floats() of them for ``heads`` let
+ * it be formed for all chunks at once; less than that, down to _floats() for ``kv_heads``, is accepted and leaves it to the chain of chunks.
+ * The results are the same numbers; rows in any order. */
+B2TTS_API size_t b2tts_delta_rule_scan_ahead_floats(int n_tokens, int n_seqs, int heads);
 B2TTS_API int b2tts_delta_rule_scan_ahead(const void* qkv, int64_t ldq, const void* beta, const void* a_in, int64_t ldu,
                                              const float* a_log, const float* dt_bias, float* state, float* coef, float* out,
                                              const int32_t* seq_start, const int32_t* seq_pos0, const int32_t* seq_len,

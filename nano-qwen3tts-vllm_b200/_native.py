@@ -1219,11 +1219,11 @@ def _coef(out, heads):
     return torch.empty(out.shape[0], heads, 3, dtype=F32, device=out.device)
 
 
-# The longest portion from which what keys and queries alone say is formed by a launch of its own.  That launch and its scratch cost the host 6 to 8 us
-# and each 64 tokens of the chain give back 1 to 2; layers of 1, 2, 4 and 8 portions, in the chain / ahead of it in us.  State space: 192 tokens
-# 70 75 87 160 / 75 78 85 149, 256 tokens 85 90 108 200 / 82 88 103 185.  Delta rule: 128 tokens 69 72 71 94 / 76 91 79 95, 256 tokens
-# 85 91 94 172 / 85 90 95 169, 384 tokens 115 120 130 252 / 113 118 130 240.
-SSM_AHEAD_FROM, DELTA_AHEAD_FROM = 256, 384
+# The longest portion from which what chunks say without the state is formed by a launch of its own.  That launch and its scratch cost the host 4 to 8 us; each
+# 64 tokens of the state space's chain give back 1 to 2, those of the delta rule 8, so that there two chunks are enough.  State space, layers of 1, 2, 4 and 8
+# portions, in the chain / ahead of it in us: 192 tokens 70 75 87 160 / 75 78 85 149, 256 tokens 85 90 108 200 / 82 88 103 185.  Delta rule, the scan
+# of 1, 4 and 8 portions alone on the GPU: 100 tokens 34 38 70 / 29 31 54 (called one by one, host and all, 37.6 before and 37.7), 200 tokens 64 68 / 45 51.
+SSM_AHEAD_FROM, DELTA_AHEAD_FROM = 256, 65
 
 
 def ssm_scan(xbc, dt_in, dt_bias, a_log, d_skip, state, out, lay, heads, groups, vdim, nstate, ahead=None):
@@ -1244,22 +1244,32 @@ def ssm_scan(xbc, dt_in, dt_bias, a_log, d_skip, state, out, lay, heads, groups,
                                         dt, _ptr(scores), 0 if scores is None else scores.numel(), _stream()), "ssm_scan")
 
 
+_delta_chunk_floats = None
+
+
 def delta_rule_scan(qkv, beta_in, a_in, a_log, dt_bias, state, out, lay, heads, kv_heads, dim, vdim, ahead=None):
     """qkv [n, 2*kv_heads*dim + heads*vdim] (convolved, activated); beta_in, a_in: column slices [n, heads] of one tensor.  ``ahead``: what
-    portions' keys and queries alone say is formed once a key head (None: where that is faster)."""
+    portions' chunks say without the state is formed for all of them at once (None: where that is faster)."""
+    global _delta_chunk_floats
     dt = _act(qkv, "qkv")
     _cuda(state, F32, "state"); _cuda(out, F32, "out")
     assert beta_in.dtype == qkv.dtype and a_in.dtype == qkv.dtype and beta_in.stride(0) == a_in.stride(0)
     assert state.is_contiguous() and out.is_contiguous()
-    max_new, dots = getattr(lay, "max_new", 0), None
+    max_new, room, n = getattr(lay, "max_new", 0), 0, lay.n_tokens
     if ahead is None:
         ahead = max_new >= DELTA_AHEAD_FROM
-    if ahead and max_new > 64 and dt == DTYPE_CODE[BF16] and heads * vdim >= 128 * kv_heads:
-        dots = torch.empty(_load().b2tts_delta_rule_scan_ahead_floats(lay.n_tokens, lay.n_seqs, kv_heads), dtype=F32, device=qkv.device)
+    if ahead and max_new > 64 and dt == DTYPE_CODE[BF16]:
+        if _delta_chunk_floats is None:                                          # of a head and chunk; a call for its number costs as much as a launch
+            _delta_chunk_floats = _load().b2tts_delta_rule_scan_ahead_floats(64, 1, 1) // 3
+        room = (n // 64 + lay.n_seqs + 1) * heads * _delta_chunk_floats
+        if room > 1 << 28:                                                       # not more than 1 GB of scratch
+            room = 0
+    work = torch.empty(room + 3 * out.shape[0] * heads, dtype=F32, device=out.device)        # the chunks, then the scalars, in one piece
+    at = work.data_ptr()
     _check(_load().b2tts_delta_rule_scan_ahead(qkv.data_ptr(), qkv.stride(0), beta_in.data_ptr(), a_in.data_ptr(), beta_in.stride(0),
-                                               a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), _coef(out, heads).data_ptr(),
-                                               out.data_ptr(), *_seq_args(lay, True), max_new, heads, kv_heads, dim, vdim, dt, _ptr(dots),
-                                               0 if dots is None else dots.numel(), _stream()), "delta_rule_scan")
+                                               a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), at + 4 * room,
+                                               out.data_ptr(), *_seq_args(lay, True), max_new, heads, kv_heads, dim, vdim, dt, at if room else None,
+                                               room, _stream()), "delta_rule_scan")
 
 
 def gated_linear_scan(q, k, v, z, z_bias, tau, state, out, lay, heads, dim, vdim):

@@ -415,8 +415,8 @@ extern "C" int b2tts_delta_rule_scan_portions(const void* qkv, int64_t ldq, cons
   return b2tts_delta_rule_scan_ahead(qkv, ldq, beta, a_in, ldu, a_log, dt_bias, state, coef, out, seq_start, seq_pos0, seq_len, seq_slot, n_tokens,
                                      n_seqs, max_new, heads, kv_heads, dim, vdim, dtype, nullptr, 0, stream);
 }
-extern "C" size_t b2tts_delta_rule_scan_ahead_floats(int n_tokens, int n_seqs, int kv_heads) {
-  return n_tokens > 0 && n_seqs > 0 && kv_heads > 0 ? static_cast<size_t>(delta_dots_floats(n_tokens, n_seqs, kv_heads)) : 0;
+extern "C" size_t b2tts_delta_rule_scan_ahead_floats(int n_tokens, int n_seqs, int heads) {
+  return n_tokens > 0 && n_seqs > 0 && heads > 0 ? static_cast<size_t>(delta_prep_floats(n_tokens, n_seqs, heads)) : 0;
 }
 extern "C" int b2tts_delta_rule_scan_ahead(const void* qkv, int64_t ldq, const void* beta, const void* a_in, int64_t ldu,
                                      const float* a_log, const float* dt_bias, float* state, float* coef, float* out,
@@ -447,10 +447,10 @@ extern "C" int b2tts_delta_rule_scan_ahead(const void* qkv, int64_t ldq, const v
   if (chunks) {
     const bool alone = n_seqs == 1 && max_new > 0;         // no second launch: max_new may be above its length, which is then taken too
     a.min_len = alone ? 1 : walk + 1;
-    if (dots != nullptr && heads / kv_heads * (vdim / 64) >= 2) {          // somebody to share them
+    if (dots != nullptr) {
       B2_REQUIRE(aligned16(dots) && dots_floats >= b2tts_delta_rule_scan_ahead_floats(n_tokens, n_seqs, kv_heads), B2TTS_EWORKSPACE,
-                 "delta_rule_scan: %zu floats for dot products (or unaligned)", dots_floats);
-      a.scores = dots;
+                 "delta_rule_scan: %zu floats for the chunks (or unaligned)", dots_floats);
+      if (dots_floats >= b2tts_delta_rule_scan_ahead_floats(n_tokens, n_seqs, heads)) a.scores = dots;      // every head's, or in the chain
     }
     const int rc = launch_delta_chunk("delta_rule_scan (portions)", a, n_seqs, max_new > 0 ? max_new : n_tokens, st);     // as above
     if (rc != B2TTS_OK || alone) return rc;

@@ -22,6 +22,8 @@
 // depend on the state and are the same for all heads of a group, so a kernel in front forms them once (chunk_scores_kernel) where at least four
 // heads share them.  4 sequences x 2048 tokens, 64 heads of 64 values x 128 channels: 561 us with the scores in the chain, 492 + 5 ahead of it,
 // token by token 3371 us; one sequence of 300 tokens 79 / 186 us.  Short portions stay with that kernel, see linear_walk_len().
+#include <type_traits>
+
 #include "scan.cuh"
 
 namespace b2 {
@@ -469,22 +471,28 @@ linear_chunk_kernel(const ScanArgs a, int64_t chunks) {
 // ------------------------------------------------------------------ delta rule
 // S <- e^l S; u = beta (v - S^T k^); S <- S + k^ u^T; o = S^T q^ * scale with unit vectors k^ = kn k, q^ = qn q.  Inside a chunk
 //
-//   u_i + sum_(j < i) A_ij u_j = beta_i (v_i - e^(c_i) S^T k^_i),   A_ij = beta_i e^(c_i - c_j) (k^_i . k^_j)
-//   o_i = e^(c_i) S^T q^_i + sum_(j <= i) e^(c_i - c_j) (q^_i . k^_j) u_j          S <- e^(c_L) S + sum_j e^(c_L - c_j) k^_j u_j^T
+//   u_i + sum_(j < i) A_ij u_j = r_i = beta_i (v_i - e^(c_i) S^T k^_i),   A_ij = beta_i e^(c_i - c_j) (k^_i . k^_j)
+//   o_i = e^(c_i) S^T q^_i + sum_(j <= i) M_ij u_j,  M_ij = e^(c_i - c_j) (q^_i . k^_j)          S <- e^(c_L) S + sum_j e^(c_L - c_j) k^_j u_j^T
 //
-// so that a chunk is two 64 x 64 tables of dot products (exact bf16 products, the norms multiplied in afterwards), the state against
-// keys and queries, a triangular solve per value column in float, and two products with the solution.
+// Everything but r, u, o and S says nothing about the state: decays, norms, M and the solved system u = r - N r with N = 1 - (1 + A)^-1 are
+// formed per chunk and head by delta_prepare() - by delta_prepare_kernel for all chunks at once where there is room for them, by the chain itself
+// else, to the same bits.  What is left of the chain: S^T k, N r, the state's update (and, beside them, the outputs).
 //
 // One CTA of eight warps per (sequence, head, 64 value columns).  Warp (wp, wh) owns value columns 16 wp .. + 15 and the wh-th half of
-// the key channels of the state, transposed in its accumulators as above; what the halves sum meets in shared memory.  The solve
-// gives four lanes to a column (row i belongs to lane i mod 4): four rows at a time are exchanged, solved by all four lanes and
-// subtracted from the rows behind.  Floats enter products as three bf16 parts, two floats as the six part products down to 2^-16.
+// the key channels of the state, transposed in its accumulators as above.  A pair of warps meets twice a chunk over a barrier of its own: what the
+// halves sum of S^T k, then the token blocks of u (wh 0 forms and finishes blocks 0 and 3, wh 1 blocks 1 and 2: five blocks of N and M each).
+// Accumulators turn into operands in registers; N and M arrive as the fragments that the lanes need.  Floats enter products as three bf16 parts,
+// two floats as the six part products down to 2^-16.
 //
-// Errors against 64 bits over 512 tokens (means of eight inputs of three sizes): outputs 1.05e-7 of their norm, state 8.9e-8; token by
-// token 1.13e-7 and 1.05e-7.  That takes the solve's sums beside the rows instead of in them (a row is rounded once at its own size and
-// not up to 64 times: outputs 1.57e-7 -> 1.14e-7, state 1.8e-7 -> 0.9e-7 together with norms formed in double) and the rest that the
-// tensor core cuts off the solution's products (1.14e-7 -> 1.05e-7, 7 us).  4 ragged sequences (4856 tokens, 16 heads of 128 x 128):
-// 492 us with dot products and norms in the chain, 450 + 11 formed ahead once a key head (delta_dots_kernel), token by token 1641 us.
+// Bound: the chain of chunks, of which a chunk takes about 17000 cycles: its 430 m16n8k16 a warp are 40 % of that, the rest is what they wait for
+// (two warps a scheduler; a CTA has the shared memory to itself).  With the tables and a triangular solve per value column in the chain it was 28000.
+// 4 ragged sequences (4856 tokens, 16 heads of 128 x 128): 302 us a chain and 50 ahead of it, the form before (dot products alone ahead) 444 + 11; all
+// launches 467 -> 366 us, one sequence of 300 tokens 83 -> 66, of 100 tokens 38 -> 38 (GPU 32 -> 29).  Where there is no room for what is formed ahead, the
+// chain forms it at 15500 cycles a chunk: 4 x 2048 tokens 492 -> 530 us, 16 x 40 63 -> 65.
+//
+// Errors against 64 bits over 512 tokens (means of 24 inputs of three sizes, outputs / state, before -> now): 128 channels 1.054e-7 / 9.15e-8 -> 1.052e-7 /
+// 9.19e-8, 64 channels 0.998e-7 / 9.35e-8 -> 0.995e-7 / 9.37e-8, keys that point half the same way 1.166e-7 / 9.18e-8 -> 1.175e-7 / 9.37e-8; token by token
+// 1.14e-7 / 1.05e-7.
 // mma_add with what the tensor core cut off its sum (it keeps two bits behind a float's): the same product on top of minus the sum
 __device__ __forceinline__ void mma_add_rest(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
   float t[4] = {0.f, 0.f, 0.f, 0.f};
@@ -495,16 +503,26 @@ __device__ __forceinline__ void mma_add_rest(float* c, const uint32_t* a, uint32
   for (int e = 0; e < 4; ++e) c[e] = (c[e] + r[e]) + t[e];
 }
 
-template <int D> struct DeltaTiles {
-  static constexpr int FS = CK_L + 4;       // padded float rows: a warp's quads fall into distinct banks
-  __nv_bfloat16 q[2][CK_L * D], k[2][CK_L * D], v[2][CK_L * CK_P];
-  __nv_bfloat16 m[3][CK_L * CK_L];          // e^(c_i - c_j) (q^_i . k^_j) in three parts
-  float A[CK_L * FS], E[CK_L * FS];         // E: e^(c_i - c_j), j <= i
-  float f[2][CK_P * FS];                    // [value column][token]: S^T k of the two halves, then u | the exchanged half of o
-  double cum[2][CK_L];
-  float ecum[2][CK_L], beta[2][CK_L], wl[2][CK_L], kn[CK_L], qn[CK_L];
-  float red[2][2][2][CK_P];                 // token by token: [parity][k or q][half][value column]
-  int wild[2];
+constexpr int CK_FS = CK_L + 4;             // padded float rows: a warp's quads fall into distinct banks
+constexpr int CK_DELTA_THREADS = 256;
+
+// What a chunk says without the state.  m, n: 16 x 16 blocks (row block i, column block j <= i at i (i + 1) / 2 + j) in three bf16 parts, as the B
+// fragments of a lane: rows 8 h + lane / 4, columns 8 w + 2 (lane % 4) at word 2 h + w.
+struct DeltaPrep {
+  uint4 m[10][3][32], n[10][3][32];
+  float ecum[CK_L], beta[CK_L];             // e^(c_i); beta
+  float ek[CK_L], eq[CK_L], wk[CK_L];       // e^(c_i) kn; e^(c_i) qn; e^(c_L - c_j) kn
+  float kn[CK_L], qn[CK_L];                 // 1 / |k|; scale / |q|
+  float wild, pad[3];                       // a key, a query or a scalar of the chunk is out of the split's range
+};
+static_assert(sizeof(DeltaPrep) % 16 == 0, "copied in 16-byte pieces");
+constexpr int CK_DELTA_PREP = sizeof(DeltaPrep) / 4;
+
+struct DeltaWork {                          // scratch of delta_prepare()
+  float A[CK_L * CK_FS], E[CK_L * CK_FS];   // E: e^(c_i - c_j), j <= i; then N
+  double cum[CK_L];
+  float beta[CK_L], kn[CK_L], qn[CK_L];
+  int wild;
 };
 
 // The 16 x 16 blocks of the dot products, rows rblk and columns cblk, that warp (wp, wh) has: three for even wp, two for odd ones
@@ -540,7 +558,7 @@ __device__ __forceinline__ float delta_row_norm(const __nv_bfloat16* k, const __
   constexpr int RB = D * 2;
   const int r = tid >> 1;
   const unsigned char* row = reinterpret_cast<const unsigned char*>(r < CK_L ? k : q);
-  double ss = 0.0;
+  double part[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
   for (int c = 0; c < D / 16; ++c) {
     const uint4 x = *reinterpret_cast<const uint4*>(row + tile_off(r & (CK_L - 1), c * 2 + (tid & 1), RB));
@@ -549,63 +567,265 @@ __device__ __forceinline__ float delta_row_norm(const __nv_bfloat16* k, const __
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const float f0 = bf16lo(w[e]), f1 = bf16hi(w[e]);
-      ss += static_cast<double>(f0 * f0);                  // exact: 16 significant bits
-      ss += static_cast<double>(f1 * f1);
+      part[e] += static_cast<double>(f0 * f0);             // exact: 16 significant bits
+      part[e] += static_cast<double>(f1 * f1);
     }
   }
+  double ss = (part[0] + part[1]) + (part[2] + part[3]);
   ss += __shfl_xor_sync(0xffffffffu, ss, 1);
   return static_cast<float>((r < CK_L ? 1.0 : static_cast<double>(qscale)) / sqrt(ss + 1e-6));
 }
 
-// What a chunk's keys and queries alone say, formed once a key head where value heads or blocks of their columns share it: the dot products
-// as the warps of delta_chunk_kernel hold them ([warp][block][half] float4 a lane), the norms, and whether something is out of the split's range.
-constexpr int CK_DOTS_NORMS = 8 * 3 * 2 * 32 * 4, CK_DOTS = CK_DOTS_NORMS + 2 * CK_L + 4;
+// All 256 threads; keys and queries of the chunk that starts at token t0 in shared memory.  Ends without a barrier.
+//
+// N in blocks of 16: those on the diagonal by substitution (column c of (1 + A)^-1 solves the system for the unit vector c; four lanes have a column, four
+// rows at a time are exchanged, solved by all four lanes and subtracted from the rows behind), those below from them by products.  64 rows of substitution in a row
+// took 7500 cycles of a chunk, this 3000.  Sums are formed beside the rows: a row is rounded once at its own size and not up to 64 times.
 template <int D>
-__global__ void __launch_bounds__(256)
-delta_dots_kernel(const ScanArgs a) {
-  constexpr int RB = D * 2;
-  __shared__ __align__(128) __nv_bfloat16 q_s[CK_L * D], k_s[CK_L * D];
-  const int b = blockIdx.z, g = blockIdx.y, t0 = blockIdx.x * CK_L, len = a.seq_len[b];
-  if (len < a.min_len || t0 >= len) return;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wp = warp & 3, wh = warp >> 2;
-  const int64_t start = a.seq_start[b];
-  const __nv_bfloat16* qg = static_cast<const __nv_bfloat16*>(a.q) + start * a.ldq + static_cast<size_t>(g) * D;
-  const __nv_bfloat16* kg = static_cast<const __nv_bfloat16*>(a.k) + start * a.ldk + static_cast<size_t>(g) * D;
-  for (int idx = tid; idx < CK_L * (D / 8); idx += 256) {
-    const int j = idx / (D / 8), ch = idx % (D / 8);
-    const bool ok = t0 + j < len;
-    const size_t row = ok ? t0 + j : 0;
-    cp_async_16(reinterpret_cast<unsigned char*>(q_s) + tile_off(j, ch, RB), qg + row * a.ldq + ch * 8, ok);
-    cp_async_16(reinterpret_cast<unsigned char*>(k_s) + tile_off(j, ch, RB), kg + row * a.ldk + ch * 8, ok);
+__device__ __forceinline__ void delta_prepare(const ScanArgs& a, const __nv_bfloat16* q_s, const __nv_bfloat16* k_s, const float* cp, int t0, int len,
+                                              DeltaWork& w, DeltaPrep& p) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wp = warp & 3, wh = warp >> 2, g4 = lane >> 2, c2 = 2 * (lane & 3);
+  if (tid == 0) w.wild = 0;
+  float ecum[2], wl[2];
+  if (warp == 0) {                                         // lane l: tokens 2 l, 2 l + 1
+    float l[2] = {0.f, 0.f}, b[2] = {0.f, 0.f};
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int t = t0 + 2 * lane + e;
+      if (t < len) { b[e] = cp[static_cast<size_t>(t) * a.H * 3 + 1]; l[e] = cp[static_cast<size_t>(t) * a.H * 3 + 2]; }
+    }
+    const bool fine = fabsf(l[0]) < 1e30f && fabsf(l[1]) < 1e30f && fabsf(b[0]) < 1e6f && fabsf(b[1]) < 1e6f;
+    l[0] = cut_log(l[0]); l[1] = cut_log(l[1]);
+    double c1 = static_cast<double>(l[0]) + l[1], x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      x = __shfl_up_sync(0xffffffffu, c1, o);
+      if (lane >= o) c1 += x;
+    }
+    double c0 = __shfl_up_sync(0xffffffffu, c1, 1);
+    c0 = (lane == 0 ? 0.0 : c0) + l[0];
+    const double ce = __shfl_sync(0xffffffffu, c1, 31);
+    w.cum[2 * lane] = c0; w.cum[2 * lane + 1] = c1;
+    w.beta[2 * lane] = b[0]; w.beta[2 * lane + 1] = b[1];
+    ecum[0] = exp_sum(c0); ecum[1] = exp_sum(c1);
+    wl[0] = exp_sum(ce - c0); wl[1] = exp_sum(ce - c1);
+    if (!fine) w.wild = 1;                                 // behind lane 0's zero: the shuffles lie between
   }
-  cp_async_commit();
-  cp_async_wait<0>();
-  __syncthreads();
-  float* at = a.scores + (static_cast<int64_t>(chunks_before(a.seq_len, b, lane) + t0 / CK_L) * a.G + g) * CK_DOTS;
   uint32_t m = 0;
-  const float n = delta_row_norm<D>(k_s, q_s, tid, a.qscale, m);
-  if ((tid & 1) == 0) at[CK_DOTS_NORMS + (tid >> 1)] = n;  // keys, then queries
+  const float nrm = delta_row_norm<D>(k_s, q_s, tid, a.qscale, m);
+  if ((tid & 1) == 0) (tid < 2 * CK_L ? w.kn[tid >> 1] : w.qn[(tid >> 1) - CK_L]) = nrm;
   const int wild = __syncthreads_or((m & 0xffffu) >= CK_BIG_IN || (m >> 16) >= CK_BIG_IN);
-  if (tid == 0) at[CK_DOTS_NORMS + 2 * CK_L] = wild ? 1.f : 0.f;
-  float4* out = reinterpret_cast<float4*>(at) + warp * 6 * 32 + lane;
+  // ---- decays between the chunk's tokens: rows x and 63 - x together have as many for every x
+  {
+    const int x = tid >> 3, sub = tid & 7;
+#pragma unroll 2
+    for (int n = 0; n < 2; ++n) {
+      const int i = n ? CK_L - 1 - x : x;
+      const double ci = w.cum[i];
+      for (int j = sub; j <= i; j += 8) w.E[i * CK_FS + j] = exp_sum(ci - w.cum[j]);
+    }
+  }
+  if (warp == 0) {
 #pragma unroll
-  for (int x = 0; x < 3; ++x) {
-    if (x == 2 && (wp & 1)) break;
+    for (int e = 0; e < 2; ++e) {
+      const int i = 2 * lane + e;
+      p.ecum[i] = ecum[e]; p.beta[i] = w.beta[i];
+      p.ek[i] = ecum[e] * w.kn[i]; p.eq[i] = ecum[e] * w.qn[i]; p.wk[i] = wl[e] * w.kn[i];
+      p.kn[i] = w.kn[i]; p.qn[i] = w.qn[i];
+    }
+  }
+  if (tid == 0) { p.wild = wild || w.wild ? 1.f : 0.f; p.pad[0] = p.pad[1] = p.pad[2] = 0.f; }
+  __syncthreads();
+  // ---- dot products of the keys (wh 0) or the queries (wh 1) with the keys up to the diagonal, in 16 x 16 blocks
+  const uint32_t k_u = smem_u32(k_s), x_u = wh ? smem_u32(q_s) : k_u;
+#pragma unroll
+  for (int nb = 0; nb < 3; ++nb) {
+    if (nb == 2 && (wp & 1)) break;
     int rblk, cblk;
-    delta_block(wp, x, rblk, cblk);
+    delta_block(wp, nb, rblk, cblk);
     float sc[2][4];
-    delta_block_dots<D>(smem_u32(wh ? q_s : k_s), smem_u32(k_s), rblk, cblk, lane, sc);
+    delta_block_dots<D>(x_u, k_u, rblk, cblk, lane, sc);
+    uint32_t part[3][4];
 #pragma unroll
-    for (int w = 0; w < 2; ++w) out[(x * 2 + w) * 32] = make_float4(sc[w][0], sc[w][1], sc[w][2], sc[w][3]);
+    for (int half = 0; half < 2; ++half) {
+      const int i = rblk * 16 + g4 + 8 * half;
+      const float fi = wh ? w.qn[i] : w.beta[i] * w.kn[i];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int j = cblk * 16 + c * 8 + c2;
+        const float2 e2 = *reinterpret_cast<const float2*>(w.E + i * CK_FS + j), k2 = *reinterpret_cast<const float2*>(w.kn + j);
+        const bool in0 = wh ? j <= i : j < i, in1 = wh ? j + 1 <= i : j + 1 < i;
+        const float x = in0 ? sc[c][2 * half] * (e2.x * (fi * k2.x)) : 0.f, y = in1 ? sc[c][2 * half + 1] * (e2.y * (fi * k2.y)) : 0.f;
+        if (wh) split3(x, y, part[0][2 * half + c], part[1][2 * half + c], part[2][2 * half + c]);
+        else *reinterpret_cast<float2*>(w.A + i * CK_FS + j) = make_float2(x, y);
+      }
+    }
+    if (wh) {
+#pragma unroll
+      for (int e = 0; e < 3; ++e) p.m[rblk * (rblk + 1) / 2 + cblk][e][lane] = make_uint4(part[e][0], part[e][1], part[e][2], part[e][3]);
+    }
+  }
+  __syncthreads();
+  // ---- N of the four 16 x 16 blocks on the diagonal: four lanes per column
+  {
+    const int sub = lane & 3, top = (warp >> 1) * 16, col = warp * 8 + g4;
+    const float* A = w.A + top * CK_FS + top;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int m0 = 0; m0 < 4; ++m0) {
+      const float* d = A + 4 * m0 * CK_FS + 4 * m0;        // the 4 x 4 block on the diagonal
+      const float d10 = d[CK_FS], d20 = d[2 * CK_FS], d21 = d[2 * CK_FS + 1], d30 = d[3 * CK_FS], d31 = d[3 * CK_FS + 1], d32 = d[3 * CK_FS + 2];
+      float as[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) as[e] = __shfl_sync(0xffffffffu, acc[m0], (lane & ~3) + e);
+      const int at = col - top - 4 * m0;                   // the unit vector's one
+      const float n0 = as[0], u0 = (at == 0 ? 1.f : 0.f) - n0;
+      const float n1 = fmaf(d10, u0, as[1]), u1 = (at == 1 ? 1.f : 0.f) - n1;
+      const float n2 = fmaf(d21, u1, fmaf(d20, u0, as[2])), u2 = (at == 2 ? 1.f : 0.f) - n2;
+      const float n3 = fmaf(d32, u2, fmaf(d31, u1, fmaf(d30, u0, as[3]))), u3 = (at == 3 ? 1.f : 0.f) - n3;
+      w.E[(top + 4 * m0 + sub) * CK_FS + col] = sub == 0 ? n0 : sub == 1 ? n1 : sub == 2 ? n2 : n3;
+#pragma unroll
+      for (int x = m0 + 1; x < 4; ++x) {
+        const float4 y = *reinterpret_cast<const float4*>(A + (4 * x + sub) * CK_FS + 4 * m0);
+        acc[x] = fmaf(y.w, u3, fmaf(y.z, u2, fmaf(y.y, u1, fmaf(y.x, u0, acc[x]))));
+      }
+    }
+  }
+  __syncthreads();
+  // ---- the blocks below, a diagonal of them at a time: X_ij = A_ij (1 - N_jj) - sum_(j < k < i) A_ik N_kj (kept in the mirrored block), N_ij = X_ij - N_ii X_ij
+  {
+    const int row = tid >> 4, col = tid & 15;
+    auto product = [&](const float* x, const float* y) -> float {      // row of x times column of y
+      float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+      for (int t = 0; t < 16; t += 4) {
+        const float4 a4 = *reinterpret_cast<const float4*>(x + row * CK_FS + t);
+        s0 = fmaf(a4.x, y[t * CK_FS + col], s0);
+        s1 = fmaf(a4.y, y[(t + 1) * CK_FS + col], s1);
+        s0 = fmaf(a4.z, y[(t + 2) * CK_FS + col], s0);
+        s1 = fmaf(a4.w, y[(t + 3) * CK_FS + col], s1);
+      }
+      return s0 + s1;
+    };
+    auto block = [](float* x, int i, int j) { return x + 16 * i * CK_FS + 16 * j; };
+#pragma unroll
+    for (int d = 1; d < 4; ++d) {
+#pragma unroll
+      for (int i = d; i < 4; ++i) {                        // unrolled: a diagonal's products overlap
+        const int j = i - d;
+        float s = product(block(w.A, i, j), block(w.E, j, j));
+#pragma unroll
+        for (int k = j + 1; k < i; ++k) s += product(block(w.A, i, k), block(w.E, k, j));
+        block(w.E, j, i)[row * CK_FS + col] = block(w.A, i, j)[row * CK_FS + col] - s;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int i = d; i < 4; ++i) {
+        const int j = i - d;
+        block(w.E, i, j)[row * CK_FS + col] = block(w.E, j, i)[row * CK_FS + col] - product(block(w.E, i, i), block(w.E, j, i));
+      }
+      __syncthreads();
+    }
+  }
+  for (int blk = warp; blk < 10; blk += 8) {
+    const int ib = blk >= 6 ? 3 : blk >= 3 ? 2 : blk >= 1 ? 1 : 0, jb = blk - ib * (ib + 1) / 2;
+    uint32_t part[3][4];
+#pragma unroll
+    for (int half = 0; half < 2; ++half)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int i = ib * 16 + half * 8 + g4, j = jb * 16 + c * 8 + c2;
+        const float x = j < i ? w.E[i * CK_FS + j] : 0.f, y = j + 1 < i ? w.E[i * CK_FS + j + 1] : 0.f;
+        split3(x, y, part[0][2 * half + c], part[1][2 * half + c], part[2][2 * half + c]);
+      }
+#pragma unroll
+    for (int e = 0; e < 3; ++e) p.n[blk][e][lane] = make_uint4(part[e][0], part[e][1], part[e][2], part[e][3]);
   }
 }
 
-// AHEAD: delta_dots_kernel has run
+template <int D> struct DeltaAheadTiles {
+  __nv_bfloat16 q[CK_L * D], k[CK_L * D];
+  DeltaWork work;
+};
+template <int D>
+__global__ void __launch_bounds__(CK_DELTA_THREADS, 3)
+delta_prepare_kernel(const ScanArgs a) {
+  constexpr int RB = D * 2;
+  extern __shared__ __align__(128) unsigned char ck_smem[];
+  DeltaAheadTiles<D>& sm = *reinterpret_cast<DeltaAheadTiles<D>*>(ck_smem);
+  const int b = blockIdx.z, h = blockIdx.y, t0 = blockIdx.x * CK_L, len = a.seq_len[b];
+  if (len < a.min_len || t0 >= len) return;
+  const int tid = threadIdx.x, g = h / (a.H / a.G);
+  const int64_t start = a.seq_start[b];
+  const __nv_bfloat16* qg = static_cast<const __nv_bfloat16*>(a.q) + start * a.ldq + static_cast<size_t>(g) * D;
+  const __nv_bfloat16* kg = static_cast<const __nv_bfloat16*>(a.k) + start * a.ldk + static_cast<size_t>(g) * D;
+  for (int idx = tid; idx < CK_L * (D / 8); idx += CK_DELTA_THREADS) {
+    const int j = idx / (D / 8), ch = idx % (D / 8);
+    const bool ok = t0 + j < len;
+    const size_t row = ok ? t0 + j : 0;
+    cp_async_16(reinterpret_cast<unsigned char*>(sm.q) + tile_off(j, ch, RB), qg + row * a.ldq + ch * 8, ok);
+    cp_async_16(reinterpret_cast<unsigned char*>(sm.k) + tile_off(j, ch, RB), kg + row * a.ldk + ch * 8, ok);
+  }
+  cp_async_commit();
+  const int64_t number = static_cast<int64_t>(chunks_before(a.seq_len, b, tid & 31) + t0 / CK_L) * a.H + h;
+  cp_async_wait<0>();
+  __syncthreads();
+  delta_prepare<D>(a, sm.q, sm.k, a.coef + (start * a.H + h) * 3, t0, len, sm.work, reinterpret_cast<DeltaPrep*>(a.scores)[number]);
+}
+
+template <int D, bool AHEAD> struct DeltaTiles {
+  __nv_bfloat16 q[2][CK_L * D], k[2][CK_L * D], v[2][CK_L * CK_P];
+  DeltaPrep prep[AHEAD ? 2 : 1];
+  float4 part[8][8][32];                    // [warp][8 tokens]: S^T k over the warp's channels; u of its blocks lies over it
+  float4 other[8][4][32];                   // [warp]: S^T q of the partner's blocks
+  union {
+    float red[2][2][2][CK_P];               // token by token: [parity][k or q][half][value column]
+    typename std::conditional<AHEAD, char, DeltaWork>::type work;
+  };
+};
+
+__device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+
+// c -= x n (SUBTRACT) or c += x n over the blocks jb <= ib of row block ib: x in three parts per column block, n the fragments of a row of blocks
+template <bool SUBTRACT>
+__device__ __forceinline__ void delta_row_product(float c[2][4], const uint32_t x[4][3][4], const uint4 (*n)[3][32], int ib, int lane) {
+  float small[2][4], mid[2][4], big[2][4];
+#pragma unroll
+  for (int w = 0; w < 2; ++w)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) small[w][e] = mid[w][e] = big[w][e] = 0.f;
+#pragma unroll
+  for (int jb = 0; jb < 4; ++jb) {
+    if (jb <= ib) {
+      const uint4 (*f)[32] = n[ib * (ib + 1) / 2 + jb];
+      const uint4 b0 = f[0][lane], b1 = f[1][lane], b2 = f[2][lane];
+#pragma unroll
+      for (int w = 0; w < 2; ++w) {
+        const uint32_t h0 = w ? b0.z : b0.x, h1 = w ? b0.w : b0.y, m0 = w ? b1.z : b1.x, m1 = w ? b1.w : b1.y, l0 = w ? b2.z : b2.x, l1 = w ? b2.w : b2.y;
+        mma_bf16_16816(small[w], x[jb][2], h0, h1);
+        mma_bf16_16816(mid[w], x[jb][1], h0, h1);
+        mma_add_rest(big[w], x[jb][0], h0, h1);
+        mma_bf16_16816(small[w], x[jb][0], l0, l1);
+        mma_bf16_16816(mid[w], x[jb][0], m0, m1);
+        mma_bf16_16816(small[w], x[jb][1], m0, m1);
+      }
+    }
+  }
+#pragma unroll
+  for (int w = 0; w < 2; ++w)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float t = (small[w][e] + mid[w][e]) + big[w][e];
+      c[w][e] = SUBTRACT ? c[w][e] - t : c[w][e] + t;
+    }
+}
+
+// AHEAD: delta_prepare_kernel has run
 template <int D, bool AHEAD>
-__global__ void __launch_bounds__(256, 1)
+__global__ void __launch_bounds__(CK_DELTA_THREADS, 1)
 delta_chunk_kernel(const ScanArgs a) {
-  using Sm = DeltaTiles<D>;
-  constexpr int RB = D * 2, VB = CK_P * 2, MB = CK_L * 2, FS = Sm::FS, THREADS = 256, CH = D / 2, NT = CH / 8;
+  using Sm = DeltaTiles<D, AHEAD>;
+  constexpr int RB = D * 2, VB = CK_P * 2, THREADS = CK_DELTA_THREADS, CH = D / 2, NT = CH / 8;
   extern __shared__ __align__(128) unsigned char ck_smem[];
   Sm& sm = *reinterpret_cast<Sm*>(ck_smem);
   const int b = blockIdx.z, h = blockIdx.y, p0 = blockIdx.x * CK_P;
@@ -621,6 +841,8 @@ delta_chunk_kernel(const ScanArgs a) {
   const float* cp = a.coef + (start * H + h) * 3;
   float* Sg = a.state + (static_cast<size_t>(a.seq_slot[b]) * H + h) * D * dv + p0;
   float* og = a.out + start * H * dv + static_cast<size_t>(h) * dv + p0;
+  const DeltaPrep* pg = nullptr;                           // the sequence's first chunk; one chunk is H of them
+  if constexpr (AHEAD) pg = reinterpret_cast<const DeltaPrep*>(a.scores) + static_cast<int64_t>(chunks_before(a.seq_len, b, lane)) * H + h;
   auto load_chunk = [&](int t0, int s) {
     for (int idx = tid; idx < CK_L * (D / 8); idx += THREADS) {
       const int j = idx / (D / 8), ch = idx % (D / 8);
@@ -634,11 +856,13 @@ delta_chunk_kernel(const ScanArgs a) {
       const bool ok = t0 + j < len;
       cp_async_16(reinterpret_cast<unsigned char*>(sm.v[s]) + tile_off(j, ch, VB), vg + (ok ? t0 + j : 0) * a.ldv + ch * 8, ok);
     }
+    if constexpr (AHEAD) {
+      const uint4* src = reinterpret_cast<const uint4*>(pg + static_cast<int64_t>(t0 / CK_L) * H);
+      for (int i = tid; i < CK_DELTA_PREP / 4; i += THREADS) cp_async_16(reinterpret_cast<uint4*>(&sm.prep[s]) + i, src + i, true);
+    }
   };
   load_chunk(0, 0);
   cp_async_commit();
-  int chunk0 = 0;                                          // number of the sequence's first chunk
-  if constexpr (AHEAD) chunk0 = chunks_before(a.seq_len, b, lane);
   const int pr = wp * 16 + g4, n0 = wh * CH;               // S^T fragments: value columns pr (+ 8), key channels n0 + nt * 8 + c2 (+ 1)
   float S[NT][4];
   const bool carried = a.seq_pos0[b] > 0;
@@ -646,92 +870,39 @@ delta_chunk_kernel(const ScanArgs a) {
   for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
     for (int e = 0; e < 4; ++e) S[nt][e] = carried ? Sg[static_cast<size_t>(n0 + nt * 8 + c2 + (e & 1)) * dv + pr + 8 * (e >> 1)] : 0.f;
-  // scalars of a chunk (warp 1: lane l holds tokens 2 l, 2 l + 1), fetched two chunks ahead and summed one ahead
-  float cl[2], cb_[2];
-  auto fetch_coef = [&](int t0) {
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int t = t0 + 2 * lane + e;
-      cl[e] = cb_[e] = 0.f;
-      if (t < len) { cb_[e] = cp[static_cast<size_t>(t) * H * 3 + 1]; cl[e] = cp[static_cast<size_t>(t) * H * 3 + 2]; }
-    }
-  };
-  auto sum_coef = [&](int s) {
-    const bool fine = fabsf(cl[0]) < 1e30f && fabsf(cl[1]) < 1e30f && fabsf(cb_[0]) < 1e6f && fabsf(cb_[1]) < 1e6f;
-    cl[0] = cut_log(cl[0]); cl[1] = cut_log(cl[1]);
-    double c1 = static_cast<double>(cl[0]) + cl[1], x;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      x = __shfl_up_sync(0xffffffffu, c1, o);
-      if (lane >= o) c1 += x;
-    }
-    double c0 = __shfl_up_sync(0xffffffffu, c1, 1);
-    c0 = (lane == 0 ? 0.0 : c0) + cl[0];
-    const double ce = __shfl_sync(0xffffffffu, c1, 31);
-    sm.cum[s][2 * lane] = c0; sm.cum[s][2 * lane + 1] = c1;
-    sm.ecum[s][2 * lane] = exp_sum(c0); sm.ecum[s][2 * lane + 1] = exp_sum(c1);
-    sm.beta[s][2 * lane] = cb_[0]; sm.beta[s][2 * lane + 1] = cb_[1];
-    sm.wl[s][2 * lane] = exp_sum(ce - c0); sm.wl[s][2 * lane + 1] = exp_sum(ce - c1);
-    const bool all = __all_sync(0xffffffffu, fine);
-    if (lane == 0) sm.wild[s] = !all;
-  };
-  if (warp == 1) {
-    fetch_coef(0);
-    sum_coef(0);
-    fetch_coef(CK_L);
-  }
-  const uint32_t m_u = smem_u32(sm.m);
   const int rb = (lane >> 4) * 8 + (lane & 7), cb = (lane >> 3) & 1;
   const int rt = ((lane >> 3) & 1) * 8 + (lane & 7), ct = lane >> 4;
   for (int t0 = 0, s = 0; t0 < len; t0 += CK_L, s ^= 1) {
     const int L = min(CK_L, len - t0);
     cp_async_wait<0>();
-    __syncthreads();                                       // the chunk has landed; the previous one is consumed
-    // ---- norms of k and q rows (two threads a row) and the range of everything that will be split
+    // ---- the range of what this thread has copied and of its part of the state
     bool wild = false;
-    float4 ahead[AHEAD ? 3 : 1][2];
     {
       uint32_t m = 0;
-      if constexpr (AHEAD) {
-        const float* at = a.scores + (static_cast<int64_t>(chunk0 + t0 / CK_L) * a.G + g) * CK_DOTS;
-        const float4* sc = reinterpret_cast<const float4*>(at) + warp * 6 * 32 + lane;
-#pragma unroll
-        for (int n = 0; n < 3; ++n)
-#pragma unroll
-          for (int w = 0; w < 2; ++w) ahead[n][w] = n == 2 && (wp & 1) ? make_float4(0.f, 0.f, 0.f, 0.f) : sc[(n * 2 + w) * 32];
-        if (tid < CK_L) sm.kn[tid] = at[CK_DOTS_NORMS + tid];
-        else if (tid < 2 * CK_L) sm.qn[tid - CK_L] = at[CK_DOTS_NORMS + tid];
-        wild = at[CK_DOTS_NORMS + 2 * CK_L] != 0.f;
-      } else {
-        const float n = delta_row_norm<D>(sm.k[s], sm.q[s], tid, a.qscale, m);
-        if ((tid & 1) == 0) (tid < 2 * CK_L ? sm.kn[tid >> 1] : sm.qn[(tid >> 1) - CK_L]) = n;
+      for (int idx = tid; idx < CK_L * (CK_P / 8); idx += THREADS) {
+        const uint4 x = *reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned char*>(sm.v[s]) + tile_off(idx / (CK_P / 8), idx % (CK_P / 8), VB));
+        m = mag2(mag2(mag2(mag2(m, x.x), x.y), x.z), x.w);
       }
-      const uint4* v4 = reinterpret_cast<const uint4*>(sm.v[s]);
-      for (int i = tid; i < CK_L * CK_P / 8; i += THREADS) { const uint4 x = v4[i]; m = mag2(mag2(mag2(mag2(m, x.x), x.y), x.z), x.w); }
-      wild = wild || (m & 0xffffu) >= CK_BIG_IN || (m >> 16) >= CK_BIG_IN;
+      wild = (m & 0xffffu) >= CK_BIG_IN || (m >> 16) >= CK_BIG_IN;
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
         for (int e = 0; e < 4; ++e) wild = wild || !(fabsf(S[nt][e]) < CK_BIG_STATE);
     }
-    // ---- decays between the chunk's tokens: rows x and 63 - x together have as many for every x
-    {
-      const int x = tid >> 3, sub = tid & 7;
-#pragma unroll 2
-      for (int n = 0; n < 2; ++n) {
-        const int i = n ? CK_L - 1 - x : x;
-        const double ci = sm.cum[s][i];
-        for (int j = sub; j <= i; j += 8) sm.E[i * FS + j] = exp_sum(ci - sm.cum[s][j]);
-      }
-      wild = wild || sm.wild[s];
+    wild = __syncthreads_or(wild);                         // the chunk has landed; the previous one is consumed
+    if constexpr (!AHEAD) {
+      delta_prepare<D>(a, sm.q[s], sm.k[s], cp, t0, len, sm.work, sm.prep[0]);
+      __syncthreads();
     }
+    const DeltaPrep& pre = sm.prep[AHEAD ? s : 0];
+    wild = wild || pre.wild != 0.f;
     if (t0 + CK_L < len) load_chunk(t0 + CK_L, s ^ 1);
     cp_async_commit();
-    if (__syncthreads_or(wild)) {
+    if (wild) {
       // ---- token by token: the same sums, every product in float
       for (int i = 0; i < L; ++i) {
         const float* c = cp + static_cast<size_t>(t0 + i) * H * 3;
-        const float c0 = c[0], c1 = c[1], kn = sm.kn[i];
+        const float c0 = c[0], c1 = c[1], kn = pre.kn[i];
         float (*red)[2][CK_P] = sm.red[i & 1];
         float x0 = 0.f, x1 = 0.f;
 #pragma unroll
@@ -762,209 +933,148 @@ delta_chunk_kernel(const ScanArgs a) {
         for (int x = 1; x < 4; x <<= 1) { x0 += __shfl_xor_sync(0xffffffffu, x0, x); x1 += __shfl_xor_sync(0xffffffffu, x1, x); }
         if ((lane & 3) == 0) { red[1][wh][pr] = x0; red[1][wh][pr + 8] = x1; }
         __syncthreads();
-        if (tid < CK_P) og[static_cast<size_t>(t0 + i) * H * dv + tid] = (red[1][0][tid] + red[1][1][tid]) * sm.qn[i];
-      }
-      if (warp == 1) {
-        sum_coef(s ^ 1);
-        fetch_coef(t0 + 2 * CK_L);
+        if (tid < CK_P) og[static_cast<size_t>(t0 + i) * H * dv + tid] = (red[1][0][tid] + red[1][1][tid]) * pre.qn[i];
       }
       continue;
     }
-    const uint32_t q_u = smem_u32(sm.q[s]), k_u = smem_u32(sm.k[s]);
-    // ---- dot products of the keys (wh 0) or the queries (wh 1) with the keys up to the diagonal, in 16 x 16 blocks: rows and first
-    // column block of this warp's two or three
-    if (warp == 1) {
-      sum_coef(s ^ 1);                                     // warps 1, 3, 5, 7 have two blocks
-      fetch_coef(t0 + 2 * CK_L);
-    }
-    {
-      const uint32_t x_u = wh ? q_u : k_u;
-#pragma unroll
-      for (int n = 0; n < 3; ++n) {
-        if (n == 2 && (wp & 1)) break;
-        int rblk, cblk;
-        delta_block(wp, n, rblk, cblk);
-        float sc[2][4];
-        if constexpr (AHEAD) {
-#pragma unroll
-          for (int w = 0; w < 2; ++w) { sc[w][0] = ahead[n][w].x; sc[w][1] = ahead[n][w].y; sc[w][2] = ahead[n][w].z; sc[w][3] = ahead[n][w].w; }
-        } else {
-          delta_block_dots<D>(x_u, k_u, rblk, cblk, lane, sc);
-        }
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          const int i = rblk * 16 + g4 + 8 * half;
-          const float fi = wh ? sm.qn[i] : sm.beta[s][i] * sm.kn[i];
-#pragma unroll
-          for (int w = 0; w < 2; ++w) {
-            const int j = cblk * 16 + w * 8 + c2;
-            const float2 e2 = *reinterpret_cast<const float2*>(sm.E + i * FS + j), k2 = *reinterpret_cast<const float2*>(sm.kn + j);
-            const bool in0 = wh ? j <= i : j < i, in1 = wh ? j + 1 <= i : j + 1 < i;
-            const float x = in0 ? sc[w][2 * half] * (e2.x * (fi * k2.x)) : 0.f, y = in1 ? sc[w][2 * half + 1] * (e2.y * (fi * k2.y)) : 0.f;
-            if (wh) {
-              uint32_t hi, mid, lo;
-              split3(x, y, hi, mid, lo);
-              const uint32_t off = (tile_off(i, cblk * 2 + w, MB) + c2 * 2) / 4;
-              reinterpret_cast<uint32_t*>(sm.m[0])[off] = hi;
-              reinterpret_cast<uint32_t*>(sm.m[1])[off] = mid;
-              reinterpret_cast<uint32_t*>(sm.m[2])[off] = lo;
-            } else {
-              *reinterpret_cast<float2*>(sm.A + i * FS + j) = make_float2(x, y);
-            }
-          }
-        }
-      }
-    }
-    // ---- S^T k and S^T q over this half of the channels
+    const uint32_t q_u = smem_u32(sm.q[s]), k_u = smem_u32(sm.k[s]), v_u = smem_u32(sm.v[s]);
+    const bool front = carried || t0 > 0;
+    // ---- S^T k, then S^T q over this half of the channels, the small parts first
     float oq[8][4];
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
       for (int e = 0; e < 4; ++e) oq[nt][e] = 0.f;
-    const bool front = carried || t0 > 0;
-    {
+    if (front) {
+      uint32_t part[3][CH / 16][4];
+#pragma unroll
+      for (int ks = 0; ks < CH / 16; ++ks)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          split3(S[2 * ks + (e >> 1)][2 * (e & 1)], S[2 * ks + (e >> 1)][2 * (e & 1) + 1], part[0][ks][e], part[1][ks][e], part[2][ks][e]);
+      auto against = [&](uint32_t x_u, float c[8][4]) {
+#pragma unroll
+        for (int pass = 0; pass < 2; ++pass)
+#pragma unroll
+          for (int ks = 0; ks < CH / 16; ++ks)
+#pragma unroll
+            for (int np = 0; np < 4; ++np)
+              if (np * 16 < L) {
+                uint32_t bf[4];
+                ldsm4(bf, x_u + tile_off(np * 16 + rb, n0 / 8 + ks * 2 + cb, RB));
+                if (pass == 0) {
+                  mma_bf16_16816(c[2 * np], part[2][ks], bf[0], bf[1]);
+                  mma_bf16_16816(c[2 * np + 1], part[2][ks], bf[2], bf[3]);
+                  mma_bf16_16816(c[2 * np], part[1][ks], bf[0], bf[1]);
+                  mma_bf16_16816(c[2 * np + 1], part[1][ks], bf[2], bf[3]);
+                } else {
+                  mma_add(c[2 * np], part[0][ks], bf[0], bf[1]);
+                  mma_add(c[2 * np + 1], part[0][ks], bf[2], bf[3]);
+                }
+              }
+      };
       float ok[8][4];
 #pragma unroll
       for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
         for (int e = 0; e < 4; ++e) ok[nt][e] = 0.f;
-      if (front) {
+      against(k_u, ok);
 #pragma unroll
-        for (int pass = 0; pass < 2; ++pass)               // the small parts first
+      for (int nt = 0; nt < 8; ++nt) sm.part[warp][nt][lane] = make_float4(ok[nt][0], ok[nt][1], ok[nt][2], ok[nt][3]);
+      against(q_u, oq);
+    } else {
 #pragma unroll
-          for (int ks = 0; ks < CH / 16; ++ks) {
-            uint32_t hi[4], mid[4], lo[4];
+      for (int nt = 0; nt < 8; ++nt) sm.part[warp][nt][lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
 #pragma unroll
-            for (int e = 0; e < 4; ++e) split3(S[2 * ks + (e >> 1)][2 * (e & 1)], S[2 * ks + (e >> 1)][2 * (e & 1) + 1], hi[e], mid[e], lo[e]);
+    for (int x = 0; x < 4; ++x) {                          // the partner's token blocks
+      const float* y = wh ? oq[x < 2 ? x : 4 + x] : oq[2 + x];
+      sm.other[warp][x][lane] = make_float4(y[0], y[1], y[2], y[3]);
+    }
+    pair_sync(1 + wp);
+    // ---- what the chunk has to write before its tokens see one another
+    float r[8][4];
+    {
+      uint32_t vf[4][4];
 #pragma unroll
-            for (int np = 0; np < 4; ++np) {
-              if (np * 16 < L) {
-                uint32_t bk[4], bq[4];
-                ldsm4(bk, k_u + tile_off(np * 16 + rb, n0 / 8 + ks * 2 + cb, RB));
-                ldsm4(bq, q_u + tile_off(np * 16 + rb, n0 / 8 + ks * 2 + cb, RB));
-                if (pass == 0) {
-                  mma_bf16_16816(ok[2 * np], lo, bk[0], bk[1]);
-                  mma_bf16_16816(ok[2 * np + 1], lo, bk[2], bk[3]);
-                  mma_bf16_16816(oq[2 * np], lo, bq[0], bq[1]);
-                  mma_bf16_16816(oq[2 * np + 1], lo, bq[2], bq[3]);
-                  mma_bf16_16816(ok[2 * np], mid, bk[0], bk[1]);
-                  mma_bf16_16816(ok[2 * np + 1], mid, bk[2], bk[3]);
-                  mma_bf16_16816(oq[2 * np], mid, bq[0], bq[1]);
-                  mma_bf16_16816(oq[2 * np + 1], mid, bq[2], bq[3]);
-                } else {
-                  mma_add(ok[2 * np], hi, bk[0], bk[1]);
-                  mma_add(ok[2 * np + 1], hi, bk[2], bk[3]);
-                  mma_add(oq[2 * np], hi, bq[0], bq[1]);
-                  mma_add(oq[2 * np + 1], hi, bq[2], bq[3]);
-                }
-              }
-            }
-          }
-      }
+      for (int js = 0; js < 4; ++js) ldsm4t(vf[js], v_u + tile_off(js * 16 + rb, wp * 2 + cb, VB));
 #pragma unroll
       for (int nt = 0; nt < 8; ++nt) {
-        *reinterpret_cast<float2*>(sm.f[wh] + pr * FS + nt * 8 + c2) = make_float2(ok[nt][0], ok[nt][1]);
-        *reinterpret_cast<float2*>(sm.f[wh] + (pr + 8) * FS + nt * 8 + c2) = make_float2(ok[nt][2], ok[nt][3]);
+        const float4 x = sm.part[wp][nt][lane], y = sm.part[wp + 4][nt][lane];
+        const float2 be = *reinterpret_cast<const float2*>(pre.beta + nt * 8 + c2), ek = *reinterpret_cast<const float2*>(pre.ek + nt * 8 + c2);
+        const uint32_t v0 = vf[nt >> 1][2 * (nt & 1)], v1 = vf[nt >> 1][2 * (nt & 1) + 1];
+        r[nt][0] = be.x * (bf16lo(v0) - ek.x * (x.x + y.x)); r[nt][1] = be.y * (bf16hi(v0) - ek.y * (x.y + y.y));
+        r[nt][2] = be.x * (bf16lo(v1) - ek.x * (x.z + y.z)); r[nt][3] = be.y * (bf16hi(v1) - ek.y * (x.w + y.w));
       }
     }
-    __syncthreads();
-    // ---- the solve: four lanes per value column
-    {
-      const int col = warp * 8 + (lane >> 2), sub = lane & 3;
-      float r[CK_L / 4], acc[CK_L / 4];
-#pragma unroll
-      for (int m = 0; m < CK_L / 4; ++m) {
-        acc[m] = 0.f;
-        const int i = 4 * m + sub;
-        const float v = to_f(sm.v[s][tile_off(i, col >> 3, VB) / 2 + (col & 7)]);
-        r[m] = sm.beta[s][i] * (v - sm.ecum[s][i] * sm.kn[i] * (sm.f[0][col * FS + i] + sm.f[1][col * FS + i]));   // 0 behind the portion's end
-      }
-#pragma unroll
-      for (int m0 = 0; m0 < CK_L / 4; ++m0) {
-        const float* d = sm.A + 4 * m0 * FS + 4 * m0;      // the 4 x 4 block on the diagonal
-        const float d10 = d[FS], d20 = d[2 * FS], d21 = d[2 * FS + 1], d30 = d[3 * FS], d31 = d[3 * FS + 1], d32 = d[3 * FS + 2];
-        float rr[4], as[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          rr[e] = __shfl_sync(0xffffffffu, r[m0], (lane & ~3) + e);
-          as[e] = __shfl_sync(0xffffffffu, acc[m0], (lane & ~3) + e);
-        }
-        const float u0 = rr[0] - as[0];
-        const float u1 = rr[1] - fmaf(d10, u0, as[1]);
-        const float u2 = rr[2] - fmaf(d21, u1, fmaf(d20, u0, as[2]));
-        const float u3 = rr[3] - fmaf(d32, u2, fmaf(d31, u1, fmaf(d30, u0, as[3])));
-        r[m0] = sub == 0 ? u0 : sub == 1 ? u1 : sub == 2 ? u2 : u3;
-#pragma unroll
-        for (int m = m0 + 1; m < CK_L / 4; ++m) {
-          const float4 x = *reinterpret_cast<const float4*>(sm.A + (4 * m + sub) * FS + 4 * m0);
-          acc[m] = fmaf(x.w, u3, fmaf(x.z, u2, fmaf(x.y, u1, fmaf(x.x, u0, acc[m]))));
-        }
-      }
-#pragma unroll
-      for (int m = 0; m < CK_L / 4; ++m) sm.f[0][col * FS + 4 * m + sub] = r[m];
-    }
-    __syncthreads();
-    // ---- the solution's part of the outputs (token blocks 0, 3 or 1, 2), beside this half's S^T q
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-      const int i = nt * 8 + c2;
-      const float e0 = sm.ecum[s][i] * sm.qn[i], e1 = sm.ecum[s][i + 1] * sm.qn[i + 1];
-      oq[nt][0] *= e0; oq[nt][1] *= e1; oq[nt][2] *= e0; oq[nt][3] *= e1;
-    }
-#pragma unroll
-    for (int jj = 0; jj < 2; ++jj) {
-      const int js = wh ? 1 + jj : 3 * jj;
-      if (js * 16 < L) {
-        uint32_t uf[3][4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 x = *reinterpret_cast<const float2*>(sm.f[0] + (pr + 8 * (e & 1)) * FS + js * 16 + (e >> 1) * 8 + c2);
-          split3(x.x, x.y, uf[0][e], uf[1][e], uf[2][e]);
-        }
-#pragma unroll
-        for (int np = 0; np < 4; ++np) {
-          if (np >= js && np * 16 < L) {
-            uint32_t b0[4], b1[4], b2[4];
-            const uint32_t off = tile_off(np * 16 + rb, js * 2 + cb, MB);
-            ldsm4(b0, m_u + off);
-            ldsm4(b1, m_u + CK_L * MB + off);
-            ldsm4(b2, m_u + 2 * CK_L * MB + off);
-#pragma unroll
-            for (int w = 0; w < 2; ++w) {
-              float t[4] = {0.f, 0.f, 0.f, 0.f};
-              mma_bf16_16816(t, uf[2], b0[2 * w], b0[2 * w + 1]);
-              mma_bf16_16816(t, uf[0], b2[2 * w], b2[2 * w + 1]);
-              mma_bf16_16816(t, uf[1], b1[2 * w], b1[2 * w + 1]);
-              mma_bf16_16816(t, uf[1], b0[2 * w], b0[2 * w + 1]);
-              mma_bf16_16816(t, uf[0], b1[2 * w], b1[2 * w + 1]);
-              mma_add_rest(t, uf[0], b0[2 * w], b0[2 * w + 1]);
-#pragma unroll
-              for (int e = 0; e < 4; ++e) oq[2 * np + w][e] += t[e];
-            }
-          }
-        }
-      }
-    }
-    // ---- the halves exchange: wh 0 finishes tokens 0 .. 31, wh 1 the others
-#pragma unroll
-    for (int x = 0; x < 4; ++x) {
-      const float* y0 = wh ? oq[x] : oq[4 + x];
-      const int i = (wh ? x : 4 + x) * 8 + c2;
-      *reinterpret_cast<float2*>(sm.f[1] + pr * FS + i) = make_float2(y0[0], y0[1]);
-      *reinterpret_cast<float2*>(sm.f[1] + (pr + 8) * FS + i) = make_float2(y0[2], y0[3]);
-    }
-    // ---- the state behind the chunk, this half of the channels
-    {
-      uint32_t af[4][3][4];
+    // ---- u = r - N r, this warp's two token blocks
+    uint32_t xf[4][3][4];
+    auto split_all = [&]() {
 #pragma unroll
       for (int js = 0; js < 4; ++js)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int j = js * 16 + (e >> 1) * 8 + c2;
-          const float2 x = *reinterpret_cast<const float2*>(sm.f[0] + (pr + 8 * (e & 1)) * FS + j);
-          split3(x.x * (sm.wl[s][j] * sm.kn[j]), x.y * (sm.wl[s][j + 1] * sm.kn[j + 1]), af[js][0][e], af[js][1][e], af[js][2][e]);
+        for (int e = 0; e < 4; ++e)
+          split3(r[2 * js + (e >> 1)][2 * (e & 1)], r[2 * js + (e >> 1)][2 * (e & 1) + 1], xf[js][0][e], xf[js][1][e], xf[js][2][e]);
+    };
+    split_all();
+    if (wh == 0) {
+      delta_row_product<true>(r + 0, xf, pre.n, 0, lane);
+      if (48 < L) delta_row_product<true>(r + 6, xf, pre.n, 3, lane);
+    } else {
+      if (16 < L) delta_row_product<true>(r + 2, xf, pre.n, 1, lane);
+      if (32 < L) delta_row_product<true>(r + 4, xf, pre.n, 2, lane);
+    }
+    pair_sync(1 + wp);                                     // both have read the sums that u takes the place of
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const float* y = wh ? r[2 + x] : r[x < 2 ? x : 4 + x];
+      sm.part[warp][x][lane] = make_float4(y[0], y[1], y[2], y[3]);
+    }
+    pair_sync(1 + wp);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const float4 y = sm.part[warp ^ 4][x][lane];
+      float* z = wh ? r[x < 2 ? x : 4 + x] : r[2 + x];
+      z[0] = y.x; z[1] = y.y; z[2] = y.z; z[3] = y.w;
+    }
+    split_all();
+    // ---- the outputs of this warp's blocks
+    {
+      auto finish = [&](int ib, float* const c0, float* const c1) {
+        float c[2][4];
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+          const float* y = w ? c1 : c0;
+          const float4 x = sm.other[warp ^ 4][(wh ? (ib - 1) : (ib ? 1 : 0)) * 2 + w][lane];
+          const float2 eq = *reinterpret_cast<const float2*>(pre.eq + ib * 16 + w * 8 + c2);
+          c[w][0] = (y[0] + x.x) * eq.x; c[w][1] = (y[1] + x.y) * eq.y; c[w][2] = (y[2] + x.z) * eq.x; c[w][3] = (y[3] + x.w) * eq.y;
         }
-      const float gl = sm.ecum[s][CK_L - 1];
+        delta_row_product<false>(c, xf, pre.m, ib, lane);
+#pragma unroll
+        for (int w = 0; w < 2; ++w)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int i = ib * 16 + w * 8 + c2 + (e & 1), p = pr + 8 * (e >> 1);
+            if (i < L) og[static_cast<size_t>(t0 + i) * H * dv + p] = c[w][e];
+          }
+      };
+      if (wh == 0) {
+        finish(0, oq[0], oq[1]);
+        if (48 < L) finish(3, oq[6], oq[7]);
+      } else {
+        if (16 < L) finish(1, oq[2], oq[3]);
+        if (32 < L) finish(2, oq[4], oq[5]);
+      }
+    }
+    // ---- the state behind the chunk, this half of the channels: what the chunk adds is summed by itself, then S <- e^(c_L) S + sum
+    {
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt) {
+        const float2 wk = *reinterpret_cast<const float2*>(pre.wk + nt * 8 + c2);
+        r[nt][0] *= wk.x; r[nt][1] *= wk.y; r[nt][2] *= wk.x; r[nt][3] *= wk.y;
+      }
+      split_all();
+      const float gl = pre.ecum[CK_L - 1];
 #pragma unroll
       for (int np = 0; np < CH / 16; ++np) {
         float t[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
@@ -978,11 +1088,11 @@ delta_chunk_kernel(const ScanArgs a) {
           for (int js = 0; js < 4; ++js)
             if (js * 16 < L) {
               if (part > 0) {
-                mma_bf16_16816(t[0], af[js][part], bf[js][0], bf[js][1]);
-                mma_bf16_16816(t[1], af[js][part], bf[js][2], bf[js][3]);
+                mma_bf16_16816(t[0], xf[js][part], bf[js][0], bf[js][1]);
+                mma_bf16_16816(t[1], xf[js][part], bf[js][2], bf[js][3]);
               } else {
-                mma_add(t[0], af[js][part], bf[js][0], bf[js][1]);
-                mma_add(t[1], af[js][part], bf[js][2], bf[js][3]);
+                mma_add(t[0], xf[js][part], bf[js][0], bf[js][1]);
+                mma_add(t[1], xf[js][part], bf[js][2], bf[js][3]);
               }
             }
 #pragma unroll
@@ -990,16 +1100,6 @@ delta_chunk_kernel(const ScanArgs a) {
           S[2 * np][e] = fmaf(gl, S[2 * np][e], t[0][e]);
           S[2 * np + 1][e] = fmaf(gl, S[2 * np + 1][e], t[1][e]);
         }
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int x = 0; x < 4; ++x) {
-      const float* y0 = wh ? oq[4 + x] : oq[x];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int i = (wh ? 4 + x : x) * 8 + c2 + (e & 1), p = pr + 8 * (e >> 1);
-        if (i < L) og[static_cast<size_t>(t0 + i) * H * dv + p] = y0[e] + sm.f[1][p * FS + i];
       }
     }
   }
@@ -1058,18 +1158,21 @@ int launch_linear_chunk(const char* what, const ScanArgs& a, int n_seqs, int lon
   return a.d == 64 ? go_linear<64, true>(what, a, n_seqs, longest, chunks, st) : go_linear<128, true>(what, a, n_seqs, longest, chunks, st);
 }
 
-int64_t delta_dots_floats(int n_tokens, int n_seqs, int G) { return (static_cast<int64_t>(n_tokens) / CK_L + n_seqs + 1) * G * CK_DOTS; }
+int64_t delta_prep_floats(int n_tokens, int n_seqs, int H) { return (static_cast<int64_t>(n_tokens) / CK_L + n_seqs + 1) * H * CK_DELTA_PREP; }
 
 template <int D, bool AHEAD>
 static int go_delta(const char* what, const ScanArgs& a, int n_seqs, int longest, cudaStream_t st) {
-  constexpr int smem = static_cast<int>(sizeof(DeltaTiles<D>));
-  const cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel<D, AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  constexpr int smem = static_cast<int>(sizeof(DeltaTiles<D, AHEAD>));
+  cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel<D, AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return cuda_fail(e, what);
   if constexpr (AHEAD) {
-    delta_dots_kernel<D><<<dim3((longest + CK_L - 1) / CK_L, a.G, n_seqs), 256, 0, st>>>(a);
+    constexpr int ahead = static_cast<int>(sizeof(DeltaAheadTiles<D>));
+    e = cudaFuncSetAttribute(delta_prepare_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, ahead);
+    if (e != cudaSuccess) return cuda_fail(e, what);
+    delta_prepare_kernel<D><<<dim3((longest + CK_L - 1) / CK_L, a.H, n_seqs), CK_DELTA_THREADS, ahead, st>>>(a);
     B2_CHECK_LAUNCH(what);
   }
-  delta_chunk_kernel<D, AHEAD><<<dim3(a.dv / CK_P, a.H, n_seqs), 256, smem, st>>>(a);
+  delta_chunk_kernel<D, AHEAD><<<dim3(a.dv / CK_P, a.H, n_seqs), CK_DELTA_THREADS, smem, st>>>(a);
   B2_CHECK_LAUNCH(what);
   return B2TTS_OK;
 }

@@ -23,7 +23,7 @@ struct ScanArgs {
   const int32_t* seq_start; const int32_t* seq_pos0; const int32_t* seq_len; const int32_t* seq_slot;
   int H, G, d, dv;
   float qscale;
-  float* scores = nullptr;                // what the chunks' queries and keys alone say, formed ahead (chunk_scores_floats(), delta_dots_floats()), or null
+  float* scores = nullptr;                // what chunks say without the state, formed ahead (chunk_scores_floats(), delta_prep_floats()), or null
   int divide;                             // linear: out = S^T q * qscale / coef[2] instead of S^T q * qscale
 };
 
@@ -35,7 +35,7 @@ int delta_walk_len(const ScanArgs& a, int n_seqs);
 int launch_linear_chunk(const char* what, const ScanArgs& a, int n_seqs, int longest, int64_t chunks, cudaStream_t st);
 int64_t chunk_scores_floats(int n_tokens, int n_seqs, int G);
 int launch_delta_chunk(const char* what, const ScanArgs& a, int n_seqs, int longest, cudaStream_t st);
-int64_t delta_dots_floats(int n_tokens, int n_seqs, int G);
+int64_t delta_prep_floats(int n_tokens, int n_seqs, int H);
 
 }  // namespace row
 }  // namespace b2
