@@ -420,6 +420,20 @@ B2TTS_API int    b2tts_decoder_stack_decode(const void* x, int64_t x_row_stride,
                                             const int32_t* context_lens, int page_size, float scale,
                                             void* workspace, size_t workspace_bytes, void* stream);
 
+/* A decode step of a whole stack (every layer and the final norm) for 1 .. 8 rows in one persistent launch; out = normalised rows.  Packed weights, caches and
+ * rounding as b2tts_decoder_stack_decode; positions [m], or [3][m] with row stride pos_row_stride where modality [128] picks the row per rotary channel.
+ * The results are those of the separate launches (b2tts_rmsnorm, b2tts_gemm_bf16, b2tts_fused_decode_attn with max_context_len), to the bit.
+ * _supported(): whether there is a kernel for these widths and rows.  workspace: _workspace_bytes() bytes, 256-byte aligned, ZEROED once; launches that
+ * share one must not overlap.  Cooperative launch: all multiprocessors are taken.  A wait that runs out is an error of a later call (b2tts_grouped_gemm_check()). */
+B2TTS_API int b2tts_decode_rows_supported(int m, int hidden, int q_size, int kv_size, int intermediate);
+B2TTS_API size_t b2tts_decode_rows_workspace_bytes(int hidden, int q_size, int kv_size, int intermediate);
+B2TTS_API int b2tts_decode_rows(const void* x, int64_t x_row_stride, void* out, int64_t out_row_stride, const b2tts_stack_layer* layers,
+                                int num_layers, const void* final_norm_weight, int m, int hidden, int num_heads, int num_kv_heads, int head_dim,
+                                int intermediate, float eps, int rounding, const int64_t* positions, int64_t pos_row_stride, const float* inv_freq,
+                                const int32_t* modality, float attention_scaling, const int32_t* slot_mapping, const int32_t* block_table,
+                                int bt_stride, const int32_t* context_lens, int page_size, int max_context_len, float scale, void* workspace,
+                                size_t workspace_bytes, void* stream);
+
 /* ---- token-id decoder models with a 32-bit residual stream -------------------------------------
  * (no counterpart in the reference, whose models take embeddings and keep a bf16 residual)
  * `dtype` selects the activation / cache / table type of the void* tensors: bf16 for serving, float for the

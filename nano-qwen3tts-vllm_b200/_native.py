@@ -78,6 +78,9 @@ def _load():
         "b2tts_gemm_chain": (I, [P, I, I, F, I, P, Z, I, P]),
         "b2tts_prompt_assemble": (I, [P, L, I, P, L, I, P, P, P, L, I, I, P]),
         "b2tts_float_to_pcm16": (I, [P, P, L, F, P]),
+        "b2tts_decode_rows_supported": (I, [I, I, I, I, I]),
+        "b2tts_decode_rows_workspace_bytes": (Z, [I, I, I, I]),
+        "b2tts_decode_rows": (I, [P, L, P, L, P, I, P, I, I, I, I, I, I, F, I, P, L, P, P, F, P, P, I, P, I, I, F, P, Z, P]),
         "b2tts_decoder_stack_plan": (I, [I, I, I, I, P, P]),
         "b2tts_decoder_stack_workspace_bytes": (Z, [I, I, I, I]),
         "b2tts_decoder_stack_decode": (I, [P, L, P, L, P, I, P, I, I, I, I, I, I, F, I, P, P, F, P, P, I, P, I, F, P, Z, P]),
@@ -725,6 +728,46 @@ def stack_layer_array(layers: list[dict]):
         for name, _ in StackLayer._fields_:
             setattr(a, name, d[name].data_ptr())
     return arr
+
+
+DECODE_ROWS_MAX_LAYERS = 40
+
+
+def decode_rows_supported(m: int, hidden: int, q_size: int, kv_size: int, intermediate: int) -> bool:
+    """Whether ``decode_rows`` has a kernel for these widths and rows."""
+    return bool(_load().b2tts_decode_rows_supported(int(m), int(hidden), int(q_size), int(kv_size), int(intermediate)))
+
+
+def decode_rows_workspace(hidden: int, q_size: int, kv_size: int, intermediate: int, device) -> torch.Tensor | None:
+    """Zero-filled, 256-byte aligned workspace of ``decode_rows`` (None: no kernel for these widths)."""
+    n = int(_load().b2tts_decode_rows_workspace_bytes(int(hidden), int(q_size), int(kv_size), int(intermediate)))
+    if n == 0:
+        return None
+    buf = torch.zeros(n + 256, dtype=torch.uint8, device=device)
+    off = (-buf.data_ptr()) % 256
+    return buf[off:off + n]
+
+
+def decode_rows(x, layer_array, num_layers, final_norm_weight, positions, inv_freq, slot_mapping, block_table, context_lens, *, num_heads,
+                num_kv_heads, head_dim, intermediate, page_size, max_context_len, eps, scale, workspace, modality=None, attention_scaling=1.0,
+                rounding=ROUND_EAGER):
+    """One decode step of a whole decoder stack for a few rows in one persistent launch (``b2tts_decode_rows``): x [m, hidden] -> normalised
+    hidden states [m, hidden].  ``layer_array``: ``stack_layer_array`` of the layers; positions [m], or [3, m] with ``modality`` [128]."""
+    _cuda(x, BF16, "x"); _cuda(positions, I64, "positions"); _cuda(inv_freq, F32, "inv_freq")
+    _cuda(slot_mapping, I32, "slot_mapping"); _cuda(block_table, I32, "block_table"); _cuda(context_lens, I32, "context_lens")
+    m, hidden = x.shape
+    if x.stride(1) != 1 or x.stride(0) % 2 or x.data_ptr() % 4:
+        x = x.contiguous()
+    if positions.stride(-1) != 1:
+        positions = positions.contiguous()
+    out = torch.empty(m, hidden, dtype=BF16, device=x.device)
+    _check(_load().b2tts_decode_rows(
+        x.data_ptr(), x.stride(0), out.data_ptr(), out.stride(0), ctypes.byref(layer_array), num_layers, final_norm_weight.data_ptr(), m, hidden,
+        num_heads, num_kv_heads, head_dim, intermediate, float(eps), int(rounding), positions.data_ptr(),
+        positions.stride(0) if positions.dim() > 1 else 0, inv_freq.data_ptr(), _ptr(modality), float(attention_scaling),
+        slot_mapping.data_ptr(), block_table.data_ptr(), block_table.stride(0), context_lens.data_ptr(), page_size, max_context_len, float(scale),
+        workspace.data_ptr(), workspace.numel(), _stream()), "decode_rows")
+    return out
 
 
 # ------------------------------------------------------------------------------------------ f3: prompt assembly

@@ -71,7 +71,7 @@ int wait_check(int kind, const char* what) {
   const int* words = __atomic_load_n(&g_words, __ATOMIC_ACQUIRE);
   if (words == nullptr || !wait_moved(words, kind, &g_told[kind])) return B2TTS_OK;
   set_error("%s: a wait inside an earlier %s ran out, its results are not valid", what,
-            kind == WAITS_GROUPED ? "grouped product" : "attention over prompt portions");
+            kind == WAITS_GROUPED ? "grouped product" : kind == WAITS_PORTIONS ? "attention over prompt portions" : "decode step");
   return B2TTS_ECUDA;
 }
 

@@ -18,12 +18,11 @@
 //     ticket) folds them in split order - deterministic - and resets the ticket for the next launch.
 #include <stdlib.h>
 
-#include "common.cuh"
+#include "fused_attn.cuh"
 
 namespace b2 {
 
 constexpr int FA_HD = 128;
-constexpr int FA_TILE = 8;
 constexpr int FA_NSTAGE = 3;
 // The per-row split-KV tickets live in a FIXED span at the start of the workspace, whatever the batch size of the
 // launch: one workspace serves every batch size / graph of a runner, and the partial accumulators of one launch
@@ -54,15 +53,6 @@ struct FusedAttnParams {
   float scale_log2;
 };
 
-__device__ __forceinline__ float fa_exp2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ void fa_unpack8(const uint4& r, float* f) {
-  f[0] = bf16lo(r.x); f[1] = bf16hi(r.x); f[2] = bf16lo(r.y); f[3] = bf16hi(r.y);
-  f[4] = bf16lo(r.z); f[5] = bf16hi(r.z); f[6] = bf16lo(r.w); f[7] = bf16hi(r.w);
-}
 __device__ __forceinline__ uint4 fa_pack8(const float* f) {
   uint4 r;
   r.x = pack_bf16(f[0], f[1]); r.y = pack_bf16(f[2], f[3]); r.z = pack_bf16(f[4], f[5]); r.w = pack_bf16(f[6], f[7]);
@@ -715,7 +705,7 @@ static size_t fa_smem_bytes(int kv_heads, int num_heads) {
 }
 
 // split-KV factor: one wave of 2 CTAs per SM, at least 8 tiles (64 tokens) of table capacity per split
-static int fa_choose_nsplit(int rows, int max_ctx) {
+int fa_choose_nsplit(int rows, int max_ctx) {
   if (const char* e = getenv("B2TTS_FA_NSPLIT")) {             // experiments only
     const int v = atoi(e);
     if (v >= 1 && v <= 32) return v;

@@ -573,6 +573,8 @@ static int choose_splits(int n_tiles, int kblocks, int mpad) {
   return best;
 }
 
+int gemm_splits(int n, int k, int m) { return choose_splits(n / G_BN, k / G_BK, (m + 15) / 16 * 16); }
+
 template <int NCH, bool EXT>
 static int launch_gemm(const GemmParams& p, const CUtensorMap& tmap, cudaStream_t st, int pdl) {
   static bool configured = false;

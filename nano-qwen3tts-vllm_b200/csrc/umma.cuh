@@ -204,4 +204,7 @@ int make_x_tensor_map(CUtensorMap* tm, const void* x, int64_t row_stride, int m,
 // The same for a bf16 tensor of rank 2 or 3: extents innermost first, strides of the outer ones in elements, the box's inner extent 64.
 int make_tensor_map(CUtensorMap* tm, const void* x, int rank, const int64_t* dims, const int64_t* strides, const int* box, const char* what);
 
+// Slices into which a projection of up to 64 rows cuts K where the caller leaves that to the kernel (gemm.cu).
+int gemm_splits(int n, int k, int m);
+
 }  // namespace b2

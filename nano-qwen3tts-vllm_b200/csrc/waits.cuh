@@ -5,7 +5,7 @@
 
 namespace b2 {
 
-enum { WAITS_GROUPED = 0, WAITS_PORTIONS = 1, WAITS_KINDS = 2 };
+enum { WAITS_GROUPED = 0, WAITS_PORTIONS = 1, WAITS_ROWS = 2, WAITS_KINDS = 3 };
 constexpr int WAIT_DEVICES = 64;                   // as many as sm_count() knows; later ones share the last word
 
 // Words lie [device][kind]: every device counts for itself, so two of them must not store to the same word (the second one's first

@@ -216,6 +216,9 @@ class ModelRunner:
                 module.workspace = self.attn_workspace
                 module.fused_workspace = self.fused_attn_workspace
                 layer_id += 1
+        for module in self.model.modules():
+            if hasattr(module, "bind_decode_rows"):
+                module.bind_decode_rows()
 
     # ------------------------------------------------------------------ batch layout
     def prepare_prefill(self, seqs: list[Sequence]):

@@ -50,6 +50,9 @@ FUSED_NORM_MIN_ROWS = int(os.environ.get("B2TTS_FUSED_NORM_MIN_ROWS", "9"))
 # bit-identical to the separate launches, but measured at 260 us per 5-layer pass against their 246 us at 64 rows
 # (every hand-over between phases costs a gpu-scope release + an L2 poll, ~2.5 us, 7 per layer)
 DATAFLOW_STACK = os.environ.get("B2TTS_DATAFLOW_STACK", "0") != "0"
+# decode steps of up to so many rows (fewer where csrc/decode_rows.cu says so) as ONE persistent launch of the whole stack, where a runner has given it a workspace:
+# the same bits as the separate launches
+DECODE_ROWS_MAX = 8
 
 
 class Qwen3TTSAttention(nn.Module):
@@ -297,6 +300,39 @@ class DecoderStack(nn.Module):
             intermediate=c.intermediate_size, eps=c.rms_norm_eps, scale=self.layers[0].self_attn.scaling, workspace=ws,
             attention_scaling=rope.attention_scaling, rounding=self.rounding, layer_array=arr)
 
+    def bind_decode_rows(self) -> None:
+        """Room for the persistent decode kernel, given by the runner that owns the KV cache: steps of one runner run one after another."""
+        c, rope = self.config, self.layers[0].self_attn.rotary_emb
+        widths = (c.hidden_size, c.num_attention_heads * c.head_dim, c.num_key_value_heads * c.head_dim, c.intermediate_size)
+        page = self.layers[0].self_attn.attn.k_cache.shape[1]
+        self._rows_most = max([m for m in range(1, DECODE_ROWS_MAX + 1) if nat.decode_rows_supported(m, *widths)], default=0)
+        if len(self.layers) > nat.DECODE_ROWS_MAX_LAYERS or c.head_dim != 128 or rope.inv_freq.numel() != 64 or page & (page - 1):
+            self._rows_most = 0
+        self._rows_ws = nat.decode_rows_workspace(*widths, self.norm.weight.device) if self._rows_most else None
+
+    def _takes_rows(self, x: torch.Tensor) -> bool:
+        ctx = get_context()
+        return (getattr(self, "_rows_ws", None) is not None and not ctx.is_prefill and ctx.block_tables is not None and x.dim() == 2
+                and 1 <= x.shape[0] <= min(self._rows_most, DECODE_ROWS_MAX) and x.dtype == torch.bfloat16)
+
+    def _run_rows(self, x: torch.Tensor, positions: torch.Tensor) -> torch.Tensor:
+        c, ctx, a0 = self.config, get_context(), self.layers[0].self_attn
+        layers = []
+        for layer in self.layers:
+            a, m = layer.self_attn, layer.mlp
+            layers.append(dict(
+                qkv_w=packed_weight(a.qkv_proj.weight), o_w=packed_weight(a.o_proj.weight),
+                gate_up_w=packed_weight(m.gate_up_proj.weight, nat.PACK_GATE_UP), down_w=packed_weight(m.down_proj.weight),
+                input_norm_w=layer.input_layernorm.weight, post_norm_w=layer.post_attention_layernorm.weight,
+                q_norm_w=a.q_norm.weight, k_norm_w=a.k_norm.weight, k_cache=a.attn.k_cache, v_cache=a.attn.v_cache))
+        rope = a0.rotary_emb
+        return nat.decode_rows(
+            x, nat.stack_layer_array(layers), len(layers), self.norm.weight, positions, rope.inv_freq, ctx.slot_mapping, ctx.block_tables,
+            ctx.context_lens, num_heads=c.num_attention_heads, num_kv_heads=c.num_key_value_heads, head_dim=c.head_dim,
+            intermediate=c.intermediate_size, page_size=a0.attn.k_cache.shape[1],
+            max_context_len=ctx.max_context_len or ctx.block_tables.shape[1] * a0.attn.k_cache.shape[1], eps=c.rms_norm_eps, scale=a0.scaling, workspace=self._rows_ws,
+            modality=rope.modality if positions.dim() > 1 else None, attention_scaling=rope.attention_scaling, rounding=self.rounding)
+
     def _run_layers_native(self, input_embeds, positions, input_ssq, tail_weight):
         residual, ssq = input_embeds, input_ssq
         nl = len(self.layers)
@@ -311,7 +347,7 @@ class DecoderStack(nn.Module):
         it), or None when this batch does not take the fused-epilogue path (the caller then uses ``run_layers``)."""
         ctx = get_context()
         m = input_embeds.shape[0]
-        if (DATAFLOW_STACK or GEMM_CHAIN or FINAL_NORM_UNFUSED or input_embeds.dim() != 2 or not max(1, FUSED_NORM_MIN_ROWS) <= m <= FUSED_NORM_MAX_ROWS
+        if (self._takes_rows(input_embeds) or DATAFLOW_STACK or GEMM_CHAIN or FINAL_NORM_UNFUSED or input_embeds.dim() != 2 or not max(1, FUSED_NORM_MIN_ROWS) <= m <= FUSED_NORM_MAX_ROWS
                 or m > GEMM_NATIVE_MAX_M or not self._native_gemm_shapes()):
             return None
         residual, ssq = self._run_layers_native(input_embeds, positions, input_ssq, tail_weight)
@@ -325,6 +361,8 @@ class DecoderStack(nn.Module):
                 and 1 <= input_embeds.shape[0] <= nat.DECODER_STACK_MAX_M and input_embeds.dim() == 2
                 and self.layers[0].self_attn.attn.k_cache.numel() > 0 and self.dataflow_plan() is not None):
             return self.run_layers_dataflow(input_embeds, positions)
+        if self._takes_rows(input_embeds):
+            return self._run_rows(input_embeds, positions)
         if GEMM_CHAIN and 1 <= input_embeds.shape[0] <= nat.GEMM_CHAIN_MAX_M and self._chain_supported():
             return self.run_layers_chained(input_embeds, positions, input_ssq)
         if 1 <= input_embeds.shape[0] <= GEMM_NATIVE_MAX_M and self._native_gemm_shapes():
