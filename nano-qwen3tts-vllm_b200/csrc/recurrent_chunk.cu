@@ -18,10 +18,16 @@
 // Numbers that the split could not represent (not finite, or so large that a product might overflow) send their chunk through a
 // token-by-token walk over the same registers, so that an infinity reaches the outputs it reaches there and no others.
 //
-// Bound: the chain of chunks (about 500 m16n8k16 per warp and chunk, each waiting for its fragments).  Scores of queries and keys do not
+// Bound: the chain of chunks, 22500 cycles each with two CTAs a multiprocessor: 9500 S^T q and the weights, 5200 the update (its 256 m16n8k16 a warp are 4100 of
+// them), 4100 the chunk's own tokens and the outputs, 2100 until the chunk has landed and is known to be in range.  Scores of queries and keys do not
 // depend on the state and are the same for all heads of a group, so a kernel in front forms them once (chunk_scores_kernel) where at least four
-// heads share them.  4 sequences x 2048 tokens, 64 heads of 64 values x 128 channels: 561 us with the scores in the chain, 492 + 5 ahead of it,
-// token by token 3371 us; one sequence of 300 tokens 79 / 186 us.  Short portions stay with that kernel, see linear_walk_len().
+// heads share them; rows up to the diagonal are uneven, so that the weights are shared out by tiles of 8 x 8 (the last warp had four times the
+// exponentials of the first and the others waited: 28000 cycles), each small and large part of the state is multiplied beside one reading of the queries, decays are
+// differences of pairs of floats (conversions from double were half of them), and skipped values come from the registers that hold them.
+// 4 sequences x 2048 tokens, 64 heads of 64 values x 128 channels: 504 -> 452 us, 64 channels and 32 heads 316 -> 237; one sequence of 300 tokens 70 -> 61,
+// 64 of 64 tokens 255 -> 239.  Scores that are asked for only during S^T q made it 465, two readings of the queries 527.
+// Errors against 64 bits over 512 tokens, 24 inputs of three sizes, outputs / state: 128 channels 8.46e-8 / 7.64e-8 -> 8.43e-8 / 7.64e-8, 64 channels 8.10e-8 /
+// 7.83e-8 -> 8.02e-8 / 7.83e-8.  Short portions stay with the token-by-token kernel, see linear_walk_len().
 #include <type_traits>
 
 #include "scan.cuh"
@@ -67,7 +73,7 @@ __device__ __forceinline__ void halves(uint32_t x, uint32_t& head, uint32_t& tai
 template <int D> struct ChunkTiles {
   __nv_bfloat16 q[2][CK_L * D], k[2][CK_L * D], v[2][CK_L * CK_P];
   __nv_bfloat16 m[3][CK_L * CK_L];          // the chunk's weights [i][j] in three parts
-  double cum[2][CK_L];                      // sums of the log decays
+  float2 cum[2][CK_L];                      // sums of the log decays: a float and what it leaves
   float ecum[2][CK_L], w[2][CK_L], wl[2][CK_L];   // e^(c_i); write scales; e^(c_L - c_j) w_j
   int wild[2];                              // a scalar of the chunk is out of the split's range
 };
@@ -76,6 +82,13 @@ template <int D> struct ChunkTiles {
 __device__ __forceinline__ float exp_sum(double x) {
   const float hi = static_cast<float>(x), e = expf(hi);
   return fmaf(e, static_cast<float>(x - hi), e);
+}
+
+// e^(a - b) of two such sums in pairs of floats: the difference of the first floats with its rounding error, which joins the differences of the second ones (48
+// bits; conversions between float and double cost eight times an addition), then the exponential of the nearest float and what that leaves
+__device__ __forceinline__ float exp_between(float2 a, float2 b) {
+  const float d = a.x - b.x, t = d - a.x, rest = ((a.x - (d - t)) - (b.x + t)) + (a.y - b.y), x = d + rest, e = expf(x);
+  return fmaf(e, rest - (x - d), e);
 }
 
 // A log decay as it enters the sums.  e^l is 0 in float below -104; taken as it comes, a very large l would leave the running sum of
@@ -102,7 +115,8 @@ __device__ __forceinline__ void chunk_scalars(ChunkTiles<D>& sm, int s, const fl
   double c0 = __shfl_up_sync(0xffffffffu, c1, 1);
   c0 = (lane == 0 ? 0.0 : c0) + l[0];
   const double cl = __shfl_sync(0xffffffffu, c1, 31);
-  sm.cum[s][2 * lane] = c0; sm.cum[s][2 * lane + 1] = c1;
+  const float h0 = static_cast<float>(c0), h1 = static_cast<float>(c1);
+  sm.cum[s][2 * lane] = make_float2(h0, static_cast<float>(c0 - h0)); sm.cum[s][2 * lane + 1] = make_float2(h1, static_cast<float>(c1 - h1));
   sm.ecum[s][2 * lane] = exp_sum(c0); sm.ecum[s][2 * lane + 1] = exp_sum(c1);
   sm.w[s][2 * lane] = w[0]; sm.w[s][2 * lane + 1] = w[1];
   sm.wl[s][2 * lane] = exp_sum(cl - c0) * w[0]; sm.wl[s][2 * lane + 1] = exp_sum(cl - c1) * w[1];
@@ -199,6 +213,12 @@ chunk_scores_kernel(const ScanArgs a, int64_t chunks) {
     if (nt <= 2 * warp + 1) out[nt * 32] = make_float4(sc[nt][0], sc[nt][1], sc[nt][2], sc[nt][3]);
 }
 
+// The 36 tiles of 8 x 8 up to the diagonal of a chunk, counted row by row: row of tiles * 8 + column
+__device__ __forceinline__ int ck_tile(int n) {
+  const int row = (n >= 1) + (n >= 3) + (n >= 6) + (n >= 10) + (n >= 15) + (n >= 21) + (n >= 28);
+  return row * 8 + n - row * (row + 1) / 2;
+}
+
 // AHEAD: chunk_scores_kernel has run
 template <int D, bool AHEAD>
 __global__ void __launch_bounds__(CK_THREADS, 2)
@@ -234,10 +254,14 @@ linear_chunk_kernel(const ScanArgs a, int64_t chunks) {
       cp_async_16(reinterpret_cast<unsigned char*>(sm.v[s]) + tile_off(j, ch, VB), vg + (ok ? t0 + j : 0) * a.ldv + ch * 8, ok);
     }
   };
+  for (int i = tid; i < 3 * CK_L * CK_L / 8; i += CK_THREADS) reinterpret_cast<uint4*>(sm.m[0])[i] = make_uint4(0, 0, 0, 0);      // above the diagonal it stays so
   load_chunk(0, 0);
   cp_async_commit();
-  int chunk0 = 0;                                          // number of the sequence's first chunk
-  if constexpr (AHEAD) chunk0 = chunks_before(a.seq_len, b, lane);
+  int chunk0 = 0, out_of_range = 0;                        // number of the sequence's first chunk; the next chunk's word behind the scores
+  if constexpr (AHEAD) {
+    chunk0 = chunks_before(a.seq_len, b, lane);
+    out_of_range = reinterpret_cast<const int*>(a.scores + chunks * a.G * CK_SCORES)[static_cast<int64_t>(chunk0) * a.G + g];
+  }
   if (warp == 3) chunk_scalars<D>(sm, 0, cp, H, 0, len, lane);
   // S^T fragments: value columns pr (+ 8), key channels nt * 8 + c2 (+ 1)
   const int pr = warp * 16 + g4;
@@ -255,17 +279,22 @@ linear_chunk_kernel(const ScanArgs a, int64_t chunks) {
     cp_async_wait<0>();
     // ---- this thread's share of the tiles and of the state within the range of the split?
     bool wild = false;
-    float4 ahead[AHEAD ? 8 : 1];
+    float2 ahead[AHEAD ? 9 : 1];
     {
       __syncthreads();                                                              // the chunk has landed; the previous one is consumed
       uint32_t m = 0;
       const uint4* t4;
       if constexpr (AHEAD) {
+        // asked for here, used behind S^T q; whether something is out of range was asked for a chunk ago
         const int64_t number = static_cast<int64_t>(chunk0 + t0 / CK_L) * a.G + g;
-        wild = reinterpret_cast<const int*>(a.scores + chunks * a.G * CK_SCORES)[number] != 0;
-        const float4* sc = reinterpret_cast<const float4*>(a.scores + number * CK_SCORES) + warp * 8 * 32 + lane;
+        const float2* sc = reinterpret_cast<const float2*>(a.scores + number * CK_SCORES);
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt) ahead[nt] = nt <= 2 * warp + 1 ? sc[nt * 32] : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int x = 0; x < 9; ++x) {
+          const int tile = ck_tile(warp + 4 * x), oct = tile >> 3;
+          ahead[x] = sc[((((oct >> 1) * 8 + (tile & 7)) * 32) + lane) * 2 + (oct & 1)];
+        }
+        wild = out_of_range != 0;
+        if (t0 + CK_L < len) out_of_range = reinterpret_cast<const int*>(a.scores + chunks * a.G * CK_SCORES)[number + a.G];
       } else {
         t4 = reinterpret_cast<const uint4*>(sm.q[s]);
         for (int i = tid; i < CK_L * D / 8; i += CK_THREADS) { const uint4 x = t4[i]; m = mag2(mag2(mag2(mag2(m, x.x), x.y), x.z), x.w); }
@@ -311,36 +340,7 @@ linear_chunk_kernel(const ScanArgs a, int64_t chunks) {
       continue;
     }
     const uint32_t q_u = smem_u32(sm.q[s]), k_u = smem_u32(sm.k[s]), v_u = smem_u32(sm.v[s]);
-    // ---- weights of rows 16 warp .. + 15: scores against the keys up to the diagonal, decay and write scale, in three parts
-    if (warp * 16 < L) {
-      float sc[8][4];
-      if constexpr (AHEAD) {
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) { sc[nt][0] = ahead[nt].x; sc[nt][1] = ahead[nt].y; sc[nt][2] = ahead[nt].z; sc[nt][3] = ahead[nt].w; }
-      } else {
-        chunk_row_scores<D>(q_u, k_u, warp, lane, sc);
-      }
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int i = warp * 16 + g4 + 8 * half;
-        const double ci = sm.cum[s][i];
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-          if (nt <= 2 * warp + 1) {
-            const int j = nt * 8 + c2;
-            const float x = j <= i ? sc[nt][2 * half] * (exp_sum(ci - sm.cum[s][j]) * sm.w[s][j]) : 0.f;
-            const float y = j + 1 <= i ? sc[nt][2 * half + 1] * (exp_sum(ci - sm.cum[s][j + 1]) * sm.w[s][j + 1]) : 0.f;
-            uint32_t hi, mid, lo;
-            split3(x, y, hi, mid, lo);
-            const uint32_t off = (tile_off(i, nt, MB) + c2 * 2) / 4;
-            reinterpret_cast<uint32_t*>(sm.m[0])[off] = hi;
-            reinterpret_cast<uint32_t*>(sm.m[1])[off] = mid;
-            reinterpret_cast<uint32_t*>(sm.m[2])[off] = lo;
-          }
-        }
-      }
-    }
-    // ---- S^T q: this warp's 16 value columns x the chunk's tokens; the small parts first, so that they are added to small sums
+    // ---- S^T q: this warp's 16 value columns x the chunk's tokens; the small parts by themselves, then the large ones with their sum
     float o[8][4];
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt)
@@ -348,6 +348,11 @@ linear_chunk_kernel(const ScanArgs a, int64_t chunks) {
       for (int e = 0; e < 4; ++e) o[nt][e] = 0.f;
     const bool front = carried || t0 > 0;
     if (front) {
+      float large[8][4];
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) large[nt][e] = 0.f;
 #pragma unroll
       for (int ks = 0; ks < D / 16; ++ks) {
         uint32_t hi[4], mid[4], lo[4];
@@ -360,26 +365,46 @@ linear_chunk_kernel(const ScanArgs a, int64_t chunks) {
             ldsm4(bf, q_u + tile_off(np * 16 + rb, ks * 2 + cb, RB));
             mma_bf16_16816(o[2 * np], lo, bf[0], bf[1]);
             mma_bf16_16816(o[2 * np + 1], lo, bf[2], bf[3]);
+            mma_add(large[2 * np], hi, bf[0], bf[1]);
+            mma_add(large[2 * np + 1], hi, bf[2], bf[3]);
             mma_bf16_16816(o[2 * np], mid, bf[0], bf[1]);
             mma_bf16_16816(o[2 * np + 1], mid, bf[2], bf[3]);
           }
         }
       }
 #pragma unroll
-      for (int ks = 0; ks < D / 16; ++ks) {
-        uint32_t hi[4];
+      for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) hi[e] = pack_bf16(S[2 * ks + (e >> 1)][2 * (e & 1)], S[2 * ks + (e >> 1)][2 * (e & 1) + 1]);
+        for (int e = 0; e < 4; ++e) o[nt][e] += large[nt][e];
+    }
+    // ---- the chunk's weights: scores up to the diagonal, decay and write scale, in three parts
+    auto weigh = [&](int i, int nt, float s0, float s1) {                           // row i, columns 8 nt + c2 (+ 1)
+      const int j = nt * 8 + c2;
+      const float2 ci = sm.cum[s][i], wj = *reinterpret_cast<const float2*>(sm.w[s] + j);
+      const float4 cj = *reinterpret_cast<const float4*>(sm.cum[s] + j);
+      const float x = j <= i ? s0 * (exp_between(ci, make_float2(cj.x, cj.y)) * wj.x) : 0.f;
+      const float y = j + 1 <= i ? s1 * (exp_between(ci, make_float2(cj.z, cj.w)) * wj.y) : 0.f;
+      uint32_t hi, mid, lo;
+      split3(x, y, hi, mid, lo);
+      const uint32_t off = (tile_off(i, nt, MB) + c2 * 2) / 4;
+      reinterpret_cast<uint32_t*>(sm.m[0])[off] = hi;
+      reinterpret_cast<uint32_t*>(sm.m[1])[off] = mid;
+      reinterpret_cast<uint32_t*>(sm.m[2])[off] = lo;
+    };
+    if constexpr (AHEAD) {
 #pragma unroll
-        for (int np = 0; np < 4; ++np) {
-          if (np * 16 < L) {
-            uint32_t bf[4];
-            ldsm4(bf, q_u + tile_off(np * 16 + rb, ks * 2 + cb, RB));
-            mma_add(o[2 * np], hi, bf[0], bf[1]);
-            mma_add(o[2 * np + 1], hi, bf[2], bf[3]);
-          }
-        }
+      for (int x = 0; x < 9; ++x) {                                                 // nine of the 36 tiles of 8 x 8 each: rows up to the diagonal are uneven
+        const int tile = ck_tile(warp + 4 * x), oct = tile >> 3;
+        if (oct * 8 < L) weigh(oct * 8 + g4, tile & 7, ahead[x].x, ahead[x].y);
       }
+    } else if (warp * 16 < L) {
+      float sc[8][4];
+      chunk_row_scores<D>(q_u, k_u, warp, lane, sc);
+#pragma unroll
+      for (int half = 0; half < 2; ++half)
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt)
+          if (nt <= 2 * warp + half) weigh(warp * 16 + g4 + 8 * half, nt, sc[nt][2 * half], sc[nt][2 * half + 1]);
     }
     __syncthreads();                                                                // the weights are in shared memory
     if (warp == 3 && t0 + CK_L < len) chunk_scalars<D>(sm, s ^ 1, cp, H, t0 + CK_L, len, lane);
@@ -412,16 +437,17 @@ linear_chunk_kernel(const ScanArgs a, int64_t chunks) {
             }
           }
 #pragma unroll
-      for (int nt = 0; nt < 8; ++nt)
+      for (int nt = 0; nt < 8; ++nt) {
+        const float2 ec = *reinterpret_cast<const float2*>(sm.ecum[s] + nt * 8 + c2);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const int i = nt * 8 + c2 + (e & 1), p = pr + 8 * (e >> 1);
-          if (i < L) {
-            float x = (front ? fmaf(sm.ecum[s][i], o[nt][e], oi[nt][e]) : oi[nt][e]) * a.qscale;
-            if (a.skip != nullptr) x += skip * to_f(sm.v[s][tile_off(i, p >> 3, VB) / 2 + (p & 7)]);
-            og[static_cast<size_t>(t0 + i) * H * dv + p] = x;
-          }
+          const int i = nt * 8 + c2 + (e & 1);
+          const uint32_t vw = vf[nt >> 1][2 * (nt & 1) + (e >> 1)];                 // v lies in the lanes as the sums do
+          float x = (front ? fmaf(e & 1 ? ec.y : ec.x, o[nt][e], oi[nt][e]) : oi[nt][e]) * a.qscale;
+          if (a.skip != nullptr) x += skip * (e & 1 ? bf16hi(vw) : bf16lo(vw));
+          if (i < L) og[static_cast<size_t>(t0 + i) * H * dv + pr + 8 * (e >> 1)] = x;
         }
+      }
     }
     // ---- the state behind the chunk: what the chunk adds is summed by itself, then S <- e^(c_L) S + sum with one rounding
     uint32_t af[4][4][4];
