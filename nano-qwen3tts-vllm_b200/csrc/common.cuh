@@ -61,6 +61,49 @@ __device__ __forceinline__ void stg_na_v4(void* p, uint4 v) {        // streamin
                :: "l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
+// ---------------------------------------------------------------- pairs of floats (two of them an instruction, each with its own rounding)
+__device__ __forceinline__ uint64_t f2_pack(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void f2_unpack(uint64_t x, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x)); }
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// four neighbouring values as they lie in memory, and as two pairs of floats
+template <typename T> struct Quad;
+template <> struct Quad<float> {
+  using Raw = uint4;
+  static __device__ __forceinline__ Raw zero() { return make_uint4(0u, 0u, 0u, 0u); }
+  static __device__ __forceinline__ Raw load(const float* p) { return ldg_v4(p); }
+  static __device__ __forceinline__ void pairs(const Raw& r, uint64_t* f) {
+    f[0] = f2_pack(__uint_as_float(r.x), __uint_as_float(r.y));
+    f[1] = f2_pack(__uint_as_float(r.z), __uint_as_float(r.w));
+  }
+};
+template <> struct Quad<__nv_bfloat16> {
+  using Raw = uint2;
+  static __device__ __forceinline__ Raw zero() { return make_uint2(0u, 0u); }
+  static __device__ __forceinline__ Raw load(const __nv_bfloat16* p) { return ldg_v2(p); }
+  static __device__ __forceinline__ void pairs(const Raw& r, uint64_t* f) {
+    f[0] = f2_pack(bf16lo(r.x), bf16hi(r.x));
+    f[1] = f2_pack(bf16lo(r.y), bf16hi(r.y));
+  }
+};
+
 // ---------------------------------------------------------------- programmatic dependent launch
 // Every kernel of this library may be launched with programmatic stream serialization: it must
 // execute pdl_wait() before it reads anything a previous kernel wrote or writes anything a previous

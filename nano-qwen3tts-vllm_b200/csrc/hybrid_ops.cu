@@ -681,86 +681,79 @@ short_conv_act_kernel(const T* __restrict__ u, int64_t ldu, const float* __restr
   out[t * ldo + c] = from_f<T>(acc);
 }
 
-// The same convolution for TAPS known at compile time: a thread owns VEC = 16 / sizeof(T) consecutive channels and walks
-// CONV_RUN consecutive tokens of one sequence with its filters and the last TAPS - 1 rows in registers, so every row is
-// read once, as one 16-byte vector (channels, c_off and the row strides multiples of VEC; u, state, out 16-byte aligned).
+// The same convolution for TAPS known at compile time: a thread owns four consecutive channels and walks CONV_RUN consecutive tokens of one
+// sequence with its filters in registers, so that every row is read once (channels and row strides multiples of 16 bytes; u, state, out 16-byte
+// aligned).
+// What bounds it is the instructions of its elements (25 of them, 17 for the activation) while enough warps are there to hide the rows' way: every row
+// of the run is asked for before the first is used and kept as it lies in memory, products are formed two at a time.
+// 4 x 2048 tokens of 4352 channels with the state's advance: 60 -> 47 us (eight channels a thread, 127 registers and half of the issue slots empty, before), 300 tokens
+// 8.7 -> 7.3; runs of 4 tokens 52 and 7.0, of 16 47 and 7.9.
 constexpr int CONV_RUN = 8;
 
-template <typename T> struct RowVec {
-  static constexpr int VEC = 16 / static_cast<int>(sizeof(T));
-  static __device__ __forceinline__ void load(const T* p, float* f) { unpack(ldg_v4(p), f); }
-  static __device__ __forceinline__ void unpack(const uint4& raw, float* f) {
-    if constexpr (VEC == 8) {
-      f[0] = bf16lo(raw.x); f[1] = bf16hi(raw.x); f[2] = bf16lo(raw.y); f[3] = bf16hi(raw.y);
-      f[4] = bf16lo(raw.z); f[5] = bf16hi(raw.z); f[6] = bf16lo(raw.w); f[7] = bf16hi(raw.w);
-    } else {
-      f[0] = __uint_as_float(raw.x); f[1] = __uint_as_float(raw.y); f[2] = __uint_as_float(raw.z); f[3] = __uint_as_float(raw.w);
-    }
-  }
-  static __device__ __forceinline__ void store(T* p, const float* f) {
-    if constexpr (VEC == 8) stg_v4(p, make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7])));
-    else stg_v4(p, make_uint4(__float_as_uint(f[0]), __float_as_uint(f[1]), __float_as_uint(f[2]), __float_as_uint(f[3])));
-  }
-};
-
-// What bounds it is the rows' traffic once they are in flight early enough: every row of the run is asked for before the first is
-// used (the loads sat behind the previous token's activation before, one 16-byte load in flight a thread), and a thread's filters are
-// contiguous and come as 16-byte vectors (as scalars a warp's load touched 32 lines).  8192 tokens of 4352 channels: 129 -> 78 us, with the
-// approximate quotient of the activation 58.
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(128)
 short_conv_act_run_kernel(const T* __restrict__ u, int64_t ldu, const float* __restrict__ w, const float* __restrict__ bias,
                           const T* __restrict__ state, const int32_t* __restrict__ seq_start, const int32_t* __restrict__ seq_pos0,
                           const int32_t* __restrict__ seq_len, const int32_t* __restrict__ seq_slot, T* __restrict__ out,
                           int64_t ldo, int C, int act) {
-  using V = RowVec<T>;
-  constexpr int VEC = V::VEC, R = TAPS - 1;
-  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * VEC;
+  using Q = Quad<T>;
+  constexpr int R = TAPS - 1;
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
   const int b = blockIdx.z, t0 = blockIdx.x * CONV_RUN;
-  const int len = seq_len[b];
+  const int len = seq_len[b], pos0 = seq_pos0[b], start = seq_start[b], slot = seq_slot[b];
   if (c >= C || t0 >= len) return;
-  const int pos0 = seq_pos0[b], start = seq_start[b], cnt = min(CONV_RUN, len - t0);
+  const int cnt = min(CONV_RUN, len - t0);
   const T* rows = u + static_cast<int64_t>(start + t0) * ldu + c;
-  uint4 raw[CONV_RUN];
+  typename Q::Raw raw[CONV_RUN + R];                       // raw[j]: the row of token t0 - R + j
 #pragma unroll
-  for (int i = 0; i < CONV_RUN; ++i) raw[i] = i < cnt ? ldg_v4(rows + i * ldu) : make_uint4(0, 0, 0, 0);
-  const T* st = state + static_cast<size_t>(seq_slot[b]) * R * C;
-  float wt[VEC * TAPS], bs[VEC], win[TAPS][VEC];           // win[j]: the row TAPS - 1 - j tokens back
-  if ((reinterpret_cast<uintptr_t>(w) & 15) == 0) {        // c is a multiple of four
-#pragma unroll
-    for (int i = 0; i < VEC * TAPS; i += 4)
-      *reinterpret_cast<float4*>(wt + i) = __ldg(reinterpret_cast<const float4*>(w + static_cast<size_t>(c) * TAPS + i));
-  } else {
-#pragma unroll
-    for (int i = 0; i < VEC * TAPS; ++i) wt[i] = w[static_cast<size_t>(c) * TAPS + i];
-  }
-#pragma unroll
-  for (int e = 0; e < VEC; ++e) bs[e] = bias != nullptr ? bias[c + e] : 0.f;
+  for (int i = 0; i < CONV_RUN; ++i) raw[R + i] = i < cnt ? Q::load(rows + i * ldu) : Q::zero();
 #pragma unroll
   for (int j = 0; j < R; ++j) {                            // the rows before the run's first token
     const int pj = pos0 + t0 - R + j;
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) win[j][e] = 0.f;
-    if (pj >= pos0) V::load(u + static_cast<int64_t>(start + pj - pos0) * ldu + c, win[j]);
-    else if (pj >= 0) V::load(st + static_cast<size_t>(pj - (pos0 - R)) * C + c, win[j]);
+    raw[j] = Q::zero();
+    if (pj >= pos0) raw[j] = Q::load(rows - static_cast<int64_t>(R - j) * ldu);
+    else if (pj >= 0) raw[j] = Q::load(state + (static_cast<size_t>(slot) * R + (pj - (pos0 - R))) * C + c);
   }
+  float flat[4 * TAPS], bs[4];                             // the filters of four channels lie one behind another
+  const float* wc = w + static_cast<size_t>(c) * TAPS;
+  if ((reinterpret_cast<uintptr_t>(w) & 15) == 0) {
+#pragma unroll
+    for (int i = 0; i < 4 * TAPS; i += 4) *reinterpret_cast<float4*>(flat + i) = __ldg(reinterpret_cast<const float4*>(wc + i));
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4 * TAPS; ++i) flat[i] = wc[i];
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) bs[e] = bias != nullptr ? bias[c + e] : 0.f;
+  uint64_t wt[TAPS][2], first[2] = {f2_pack(bs[0], bs[1]), f2_pack(bs[2], bs[3])}, win[TAPS][2];
+#pragma unroll
+  for (int j = 0; j < TAPS; ++j)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) wt[j][h] = f2_pack(flat[2 * h * TAPS + j], flat[(2 * h + 1) * TAPS + j]);
+#pragma unroll
+  for (int j = 0; j < R; ++j) Q::pairs(raw[j], win[j]);
+  T* o = out + static_cast<int64_t>(start + t0) * ldo + c;
 #pragma unroll
   for (int i = 0; i < CONV_RUN; ++i) {
     if (i >= cnt) break;
-    V::unpack(raw[i], win[R]);
-    float acc[VEC];
+    Q::pairs(raw[R + i], win[R]);
+    float acc[4];
 #pragma unroll
-    for (int e = 0; e < VEC; ++e) {
-      float a = bs[e];
+    for (int h = 0; h < 2; ++h) {
+      uint64_t a = first[h];
 #pragma unroll
-      for (int j = 0; j < TAPS; ++j) a += wt[e * TAPS + j] * win[j][e];
-      acc[e] = act == 1 ? silu_for<T>(a) : a;
+      for (int j = 0; j < TAPS; ++j) a = f2_fma(wt[j][h], win[j][h], a);
+      f2_unpack(a, acc[2 * h], acc[2 * h + 1]);
     }
-    V::store(out + static_cast<int64_t>(start + t0 + i) * ldo + c, acc);
+    if (act == 1) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[e] = silu_for<T>(acc[e]);
+    }
+    store4<T>(o + i * ldo, make_float4(acc[0], acc[1], acc[2], acc[3]));
 #pragma unroll
     for (int j = 0; j < R; ++j)
 #pragma unroll
-      for (int e = 0; e < VEC; ++e) win[j][e] = win[j + 1][e];
+      for (int h = 0; h < 2; ++h) win[j][h] = win[j + 1][h];
   }
 }
 
@@ -854,7 +847,7 @@ gated_group_norm_vec4_kernel(const float* __restrict__ y, const T* __restrict__ 
   };
   // a group of up to GN_KEEP vectors per thread stays in registers between the sum of squares and the scaled write; all of them are
   // asked for before the first gate is formed (8192 rows of 4096: 89 -> 71 us, with the
-  // approximate quotient of the gates 59; behind each other's gates the loads came one at a time)
+  // approximate reciprocal of the gates 55; behind each other's gates the loads came one at a time)
   constexpr int GN_KEEP = 4;
   const bool keep = gs <= 4 * GN_KEEP * static_cast<int>(blockDim.x);
   float4 kv[GN_KEEP], kg[GN_KEEP];
@@ -1090,8 +1083,8 @@ static void launch_conv_act(cudaStream_t st, const void* u, int64_t ldu, int c_o
   const bool vec = taps >= 2 && taps <= 4 && max_new > 0 && C % VEC == 0 && ldu % VEC == 0 && ldo % VEC == 0 && aligned16(uu) &&
                    aligned16(out) && aligned16(state) && n_seqs <= 65535;
   if (vec) {
-    const int threads = std::min(128, (C / VEC + 31) / 32 * 32);
-    const dim3 grid((max_new + CONV_RUN - 1) / CONV_RUN, (C / VEC + threads - 1) / threads, n_seqs);
+    const int threads = std::min(128, (C / 4 + 31) / 32 * 32);
+    const dim3 grid((max_new + CONV_RUN - 1) / CONV_RUN, (C / 4 + threads - 1) / threads, n_seqs);
 #define CONV_RUN_GO(TP) short_conv_act_run_kernel<T, TP><<<grid, threads, 0, st>>>(uu, ldu, w, bias, static_cast<const T*>(state), seq_start, \
         seq_pos0, seq_len, seq_slot, static_cast<T*>(out), ldo, C, act)
     if (taps == 4) CONV_RUN_GO(4);

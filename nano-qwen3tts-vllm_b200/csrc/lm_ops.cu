@@ -303,6 +303,10 @@ constexpr int CONV4_TOKENS = 8;            // consecutive rows of a prompt step 
 
 // One warp per (block of TOK rows, head slice): TOK = CONV4_TOKENS, or 1 for steps of few rows, which then spread over more
 // warps.  The lane keeps the taps of its four channels in registers.
+// Bound: instructions and the way of a warp's rows (bookkeeping, then its projections), not the rows' bytes.  A block's rows stay as they lie in memory until they are
+// used, products are formed two at a time, and the norms of four rows share one tree of shuffles and one root, in the order of warp_sum().
+// 16 + 8 + 8 heads of 128, 4 taps, us before / now: 4 x 2048 tokens 103 / 57 (64 coordinates turned 157 / 96), 4856 ragged 53 / 38 (79 / 57), 300 11.4 / 9.9;
+// blocks of 4 rows 64, 41, 8.1, of 16 58, 49, 15.4.
 template <typename T, int TAPS, int NCH, bool ROT, int TOK>
 __global__ void __launch_bounds__(CONV_WARPS * 32)
 conv_headnorm_kvwrite_vec4_kernel(const T* __restrict__ u, int64_t u_stride, const float* __restrict__ conv_w,
@@ -325,6 +329,14 @@ conv_headnorm_kvwrite_vec4_kernel(const T* __restrict__ u, int64_t u_stride, con
   else if (hs < H + G) { kind = 1; head = hs - H; width = d; c0 = H * d + head * d; }
   else { kind = 2; head = hs - H - G; width = dv; c0 = H * d + G * d + head * dv; }
   constexpr int R = TAPS - 1;
+  // the rows' bookkeeping (two dependent loads each) is fetched by one lane per row, all rows at once
+  int m_slot = -1, m_p = 0, m_pos0 = 0, m_start = 0, m_sslot = 0;
+  if (lane < TOK && n0 + lane < n_tokens) {
+    m_slot = slot_mapping[n0 + lane];
+    const int b = tok_seq[n0 + lane];
+    m_p = positions[n0 + lane];
+    if (m_slot >= 0) { m_pos0 = seq_pos0[b]; m_start = seq_start[b]; m_sslot = seq_slot[b]; }
+  }
   float w[NCH][4][TAPS];
   float g4[NCH][4];
 #pragma unroll
@@ -354,16 +366,6 @@ conv_headnorm_kvwrite_vec4_kernel(const T* __restrict__ u, int64_t u_stride, con
       }
     }
   }
-  // the rows' bookkeeping (three dependent loads each) is fetched by one lane per row, all rows at once
-  int m_slot = -1, m_p = 0, m_pos0 = 0, m_start = 0, m_sslot = 0;
-  if (lane < TOK && n0 + lane < n_tokens) {
-    m_slot = slot_mapping[n0 + lane];
-    if (m_slot >= 0) {
-      const int b = tok_seq[n0 + lane];
-      m_p = positions[n0 + lane];
-      m_pos0 = seq_pos0[b]; m_start = seq_start[b]; m_sslot = seq_slot[b];
-    }
-  }
   // the lane's cosines and sines for row n (ROT; rot_dims / 2 is a multiple of four: partners are whole quads)
   struct Turn { float cs[ROT ? NCH : 1][4], sn[ROT ? NCH : 1][4]; };
   auto turn_of = [&](int n) {
@@ -384,8 +386,9 @@ conv_headnorm_kvwrite_vec4_kernel(const T* __restrict__ u, int64_t u_stride, con
     }
     return t;
   };
-  // rotation and norm of a head (see ConvHeadOps), then the row's destination
-  auto finish = [&](float (&y)[NCH][4], int n, int slot, const Turn& turn) {
+  // rounding and rotation of a head (see ConvHeadOps); returns the lane's part of the sum of squares
+  const bool normed = kind != 2 || (ops.flags & CONV_UNIT_V);
+  auto turned = [&](float (&y)[NCH][4], const Turn& turn) {
     if (kind != 2 && (ops.flags & CONV_ROUND)) {
 #pragma unroll
       for (int i = 0; i < NCH; ++i)
@@ -417,14 +420,19 @@ conv_headnorm_kvwrite_vec4_kernel(const T* __restrict__ u, int64_t u_stride, con
           for (int e = 0; e < 4; ++e) y[i][e] = r[i][e];
       }
     }
-    if (kind != 2 || (ops.flags & CONV_UNIT_V)) {
-      float ssq = 0.f;
+    float ssq = 0.f;
+    if (normed) {
 #pragma unroll
       for (int i = 0; i < NCH; ++i)
 #pragma unroll
         for (int e = 0; e < 4; ++e) ssq += y[i][e] * y[i][e];
-      ssq = warp_sum(ssq);
-      const float inv = 1.0f / sqrtf(ssq / static_cast<float>(width) + eps);
+    }
+    return ssq;
+  };
+  auto inv_of = [&](float sum) { return 1.0f / sqrtf(sum / static_cast<float>(width) + eps); };
+  // the norm's scaling, then the row's destination
+  auto put = [&](float (&y)[NCH][4], int n, int slot, float inv) {
+    if (normed) {
 #pragma unroll
       for (int i = 0; i < NCH; ++i)
 #pragma unroll
@@ -445,36 +453,74 @@ conv_headnorm_kvwrite_vec4_kernel(const T* __restrict__ u, int64_t u_stride, con
   const bool mine = lane >= TOK || (m_slot >= 0 && m_start == start0 && m_p == p0 + lane);
   if (__all_sync(0xffffffffu, mine)) {
     const int pos0 = __shfl_sync(0xffffffffu, m_pos0, 0), sslot = __shfl_sync(0xffffffffu, m_sslot, 0);
-    float uv[TOK + R][NCH][4];
+    typename Quad<T>::Raw raw[TOK + R][NCH];
 #pragma unroll
     for (int k = 0; k < TOK + R; ++k) {
       const int pk = p0 - R + k;
 #pragma unroll
       for (int i = 0; i < NCH; ++i) {
         const int cc = (lane + 32 * i) * 4;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) uv[k][i][e] = 0.f;             // before the sequence's start
+        raw[k][i] = Quad<T>::zero();                               // before the sequence's start
         if (cc < width) {
-          if (pk >= pos0) Vec4<T>::load(u + static_cast<int64_t>(start0 + pk - pos0) * u_stride + c0 + cc, uv[k][i]);
-          else if (pk >= 0) Vec4<T>::load(state + (static_cast<size_t>(sslot) * R + (pk - (pos0 - R))) * C + c0 + cc, uv[k][i]);
+          if (pk >= pos0) raw[k][i] = Quad<T>::load(u + static_cast<int64_t>(start0 + pk - pos0) * u_stride + c0 + cc);
+          else if (pk >= 0) raw[k][i] = Quad<T>::load(state + (static_cast<size_t>(sslot) * R + (pk - (pos0 - R))) * C + c0 + cc);
         }
       }
     }
+    uint64_t wp[TAPS][NCH][2], win[TAPS][NCH][2];
+#pragma unroll
+    for (int i = 0; i < NCH; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) wp[j][i][h] = f2_pack(w[i][2 * h][j], w[i][2 * h + 1][j]);
+#pragma unroll
+    for (int k = 0; k < R; ++k)
+#pragma unroll
+      for (int i = 0; i < NCH; ++i) Quad<T>::pairs(raw[k][i], win[k][i]);
     Turn ahead = turn_of(n0);                // a row ahead of its use
+    constexpr int B = TOK < 4 ? TOK : 4;     // rows whose norms are formed together
 #pragma unroll
-    for (int t = 0; t < TOK; ++t) {
-      const Turn turn = ahead;
-      if (t + 1 < TOK) ahead = turn_of(n0 + t + 1);
-      float y[NCH][4];
+    for (int t0 = 0; t0 < TOK; t0 += B) {
+      float y[B][NCH][4], ssq[B];
 #pragma unroll
-      for (int i = 0; i < NCH; ++i)
+      for (int t = 0; t < B; ++t) {
+        const Turn turn = ahead;
+        if (t0 + t + 1 < TOK) ahead = turn_of(n0 + t0 + t + 1);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          y[i][e] = 0.f;
+        for (int i = 0; i < NCH; ++i) {
+          Quad<T>::pairs(raw[t0 + t + R][i], win[R][i]);
 #pragma unroll
-          for (int j = 0; j < TAPS; ++j) y[i][e] = fmaf(w[i][e][j], uv[t + j][i][e], y[i][e]);
+          for (int h = 0; h < 2; ++h) {
+            uint64_t a = 0;
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j) a = f2_fma(wp[j][i][h], win[j][i][h], a);
+            f2_unpack(a, y[t][i][2 * h], y[t][i][2 * h + 1]);
+#pragma unroll
+            for (int j = 0; j < R; ++j) win[j][i][h] = win[j + 1][i][h];
+          }
         }
-      finish(y, n0 + t, __shfl_sync(0xffffffffu, m_slot, t), turn);
+        ssq[t] = turned(y[t], turn);
+      }
+      float inv[B];
+      if constexpr (B == 1) {
+        inv[0] = inv_of(warp_sum(ssq[0]));
+      } else {
+        // the tree of warp_sum() for four sums at once: halves of the lanes keep two rows, then one, and one root serves four rows
+        const bool hi = lane & 16, odd = lane & 8;
+        float a = hi ? ssq[2] : ssq[0], b = hi ? ssq[3] : ssq[1];
+        a += __shfl_xor_sync(0xffffffffu, hi ? ssq[0] : ssq[2], 16);
+        b += __shfl_xor_sync(0xffffffffu, hi ? ssq[1] : ssq[3], 16);
+        float v = odd ? b : a;
+        v += __shfl_xor_sync(0xffffffffu, odd ? a : b, 8);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        v = inv_of(v);
+#pragma unroll
+        for (int t = 0; t < B; ++t) inv[t] = __shfl_sync(0xffffffffu, v, (t >> 1) * 16 + (t & 1) * 8);
+      }
+#pragma unroll
+      for (int t = 0; t < B; ++t) put(y[t], n0 + t0 + t, __shfl_sync(0xffffffffu, m_slot, t0 + t), inv[t]);
     }
     return;
   }
@@ -512,7 +558,8 @@ conv_headnorm_kvwrite_vec4_kernel(const T* __restrict__ u, int64_t u_stride, con
         }
       }
     }
-    finish(y, n, slot, turn_of(n));
+    const float ssq = turned(y, turn_of(n));
+    put(y, n, slot, normed ? inv_of(warp_sum(ssq)) : 1.f);
   }
 }
 

@@ -67,28 +67,6 @@ __device__ __forceinline__ void po_umma_ts(uint32_t d, uint32_t a, uint32_t b_lo
       "}"
       :: "r"(d), "r"(a), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(UMMA_DESC_HI_SW128) : "memory");
 }
-// pairs of floats
-__device__ __forceinline__ uint64_t po_pair(float a, float b) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void po_split(uint64_t x, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x)); }
-__device__ __forceinline__ uint64_t po_fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t po_add2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ uint64_t po_mul2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 // 32 columns of 16 lanes for lanes 0 .. 15 of the warp and 32 columns of the same lanes, SPLIT columns further, for the others
 template <int SPLIT>
 __device__ __forceinline__ void po_ld32(uint32_t taddr, uint32_t* r) {
@@ -631,7 +609,7 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
           first = false;
         }
         // ---- weights, their bf16 parts in place of the scores, and the sum of those: pairs' remainders in sb, minus the rounded weights in sa
-        const uint64_t f2 = po_pair(f, f), m2 = po_pair(-m, -m);
+        const uint64_t f2 = f2_pack(f, f), m2 = f2_pack(-m, -m);
         uint64_t sa = 0, sb = 0;
 #pragma unroll 1
         for (int part = 0; part < HK; part += 32) {
@@ -659,27 +637,27 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
               w0 = po_sigmoid(__uint_as_float(vv[0])); w1 = po_sigmoid(__uint_as_float(vv[1]));
               w2 = po_sigmoid(__uint_as_float(vv[2])); w3 = po_sigmoid(__uint_as_float(vv[3]));
             } else {
-              po_split(po_fma2(po_pair(__uint_as_float(vv[0]), __uint_as_float(vv[1])), f2, m2), w0, w1);
-              po_split(po_fma2(po_pair(__uint_as_float(vv[2]), __uint_as_float(vv[3])), f2, m2), w2, w3);
+              f2_unpack(f2_fma(f2_pack(__uint_as_float(vv[0]), __uint_as_float(vv[1])), f2, m2), w0, w1);
+              f2_unpack(f2_fma(f2_pack(__uint_as_float(vv[2]), __uint_as_float(vv[3])), f2, m2), w2, w3);
               w0 = po_ex2(w0); w1 = po_ex2(w1); w2 = po_ex2(w2); w3 = po_ex2(w3);
             }
-            const uint64_t wa = po_pair(w0, w1), wb = po_pair(w2, w3);
+            const uint64_t wa = f2_pack(w0, w1), wb = f2_pack(w2, w3);
             const uint32_t p0 = pack_bf16(w0, w1), p1 = pack_bf16(w2, w3);
             if constexpr (MODE != PO_ROUNDED) {
               const uint32_t n0 = p0 ^ 0x80008000u, n1 = p1 ^ 0x80008000u;
-              const uint64_t h0 = po_pair(bf16lo(n0), bf16hi(n0)), h1 = po_pair(bf16lo(n1), bf16hi(n1));
-              po_split(po_add2(wa, h0), r0, r1);
-              po_split(po_add2(wb, h1), r2, r3);
+              const uint64_t h0 = f2_pack(bf16lo(n0), bf16hi(n0)), h1 = f2_pack(bf16lo(n1), bf16hi(n1));
+              f2_unpack(f2_add(wa, h0), r0, r1);
+              f2_unpack(f2_add(wb, h1), r2, r3);
               const uint32_t q0 = pack_bf16(r0, r1), q1 = pack_bf16(r2, r3);
               if constexpr (!SIG) {
-                sa = po_add2(po_add2(sa, h0), h1);
-                sb = po_add2(po_add2(sb, po_pair(bf16lo(q0), bf16hi(q0))), po_pair(bf16lo(q1), bf16hi(q1)));
+                sa = f2_add(f2_add(sa, h0), h1);
+                sb = f2_add(f2_add(sb, f2_pack(bf16lo(q0), bf16hi(q0))), f2_pack(bf16lo(q1), bf16hi(q1)));
               }
               rest[c / 2] = q0;
               rest[c / 2 + 1] = q1;
             } else {
-              sa = po_add2(sa, po_pair(bf16lo(p0), bf16hi(p0)));
-              sb = po_add2(sb, po_pair(bf16lo(p1), bf16hi(p1)));
+              sa = f2_add(sa, f2_pack(bf16lo(p0), bf16hi(p0)));
+              sb = f2_add(sb, f2_pack(bf16lo(p1), bf16hi(p1)));
             }
             hi[c / 2] = p0;
             hi[c / 2 + 1] = p1;
@@ -688,7 +666,7 @@ portion_attn_kernel(const PortionArgs a, const PortionPlan p, const __grid_const
           if constexpr (MODE != PO_ROUNDED) po_st16<HK>(tm_s + part + 16, rest);
         }
         float s0, s1;
-        po_split(po_add2(MODE == PO_PAIRS ? sa ^ 0x8000000080000000ull : sa, sb), s0, s1);
+        f2_unpack(f2_add(MODE == PO_PAIRS ? sa ^ 0x8000000080000000ull : sa, sb), s0, s1);
         l += s0 + s1;
         po_st_wait();
         tc_fence_before();
