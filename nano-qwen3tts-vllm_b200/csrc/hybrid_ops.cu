@@ -491,6 +491,25 @@ __device__ __forceinline__ void load8_f(const float* p, float* f) {
   f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
 }
 
+// From a head's sums of squares of two tokens to the reciprocals of its roots (1 where !normed).  The first exchange leaves each half of the head's lanes with one
+// of the tokens: one tree and one root for both, in the order of a tree for each.
+template <int LPH>
+__device__ __forceinline__ void both_inverses(float (&inv)[2], int lane, bool normed, float eps) {
+  const bool second = lane & (LPH / 2);
+  float v = second ? inv[1] : inv[0];
+  v += __shfl_xor_sync(0xffffffffu, second ? inv[0] : inv[1], LPH / 2);
+#pragma unroll
+  for (int o = LPH / 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  v = normed ? 1.0f / sqrtf(v / static_cast<float>(LPH * 8) + eps) : 1.f;
+  inv[0] = __shfl_sync(0xffffffffu, v, lane & ~(LPH / 2));
+  inv[1] = __shfl_sync(0xffffffffu, v, lane | (LPH / 2));
+}
+__device__ __forceinline__ void turn_pair(float& a, float& b, float co, float si) {
+  const float first = a;
+  a = first * co - b * si;
+  b = b * co + first * si;
+}
+
 template <int TOK, int LPH>
 __global__ void __launch_bounds__(ROW_THREADS)
 prep_vec8_kernel(const PrepArgs p) {
@@ -502,7 +521,9 @@ prep_vec8_kernel(const PrepArgs p) {
 #pragma unroll
   for (int t = 0; t < TOK; ++t) slot[t] = t0 + t < p.n_tokens ? p.slot_mapping[t0 + t] : -1;      // -1: padding row, or behind the last token
   const int q8 = nq / 8, k8 = p.k_cache != nullptr ? nk / 8 : 0, v8 = p.v_cache != nullptr ? nv / 8 : 0, items = q8 + k8 + v8;
-  const int lane = tid & 31;                              // LPH = d / 8 lanes have a head
+  const int lane = tid & 31;                              // LPH lanes have a head
+  constexpr int DIM = LPH * 8;
+  static_assert(TOK <= 2, "one exchange shares out the tokens");
   uint4 x[TOK], ahead[TOK];                               // a thread's pieces, and those of its next turn
   auto load = [&](int i) {
     const bool is_q = i < q8, is_k = !is_q && i < q8 + k8;
@@ -510,7 +531,7 @@ prep_vec8_kernel(const PrepArgs p) {
 #pragma unroll
     for (int t = 0; t < TOK; ++t) {
       ahead[t] = make_uint4(0u, 0u, 0u, 0u);
-      if (i < items && slot[t] >= 0) ahead[t] = ldg_v4(p.u + static_cast<int64_t>(t0 + t) * p.ldu + off + c);
+      if (i < items && t0 + t < p.n_tokens) ahead[t] = ldg_v4(p.u + static_cast<int64_t>(t0 + t) * p.ldu + off + c);   // a padding row too: its slot is not waited for
     }
   };
   load(tid);
@@ -558,27 +579,38 @@ prep_vec8_kernel(const PrepArgs p) {
     float b[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, w[8] = {1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f};
     if (live && bias != nullptr) load8_f(bias + c, b);
     const bool qk = live && (is_q || is_k);
-    const int ci = qk ? c % p.d : p.d;                    // the piece's first coordinate in its head
+    const int ci = qk ? c & (DIM - 1) : DIM;              // the piece's first coordinate in its head
     if (qk && p.norm != 0) load8_f((is_q ? p.q_norm_w : p.k_norm_w) + (p.norm == 2 ? ci : c), w);
     const bool turned = qk && ci < p.rot_dims;
+    uint64_t y[TOK][4];
+#pragma unroll
+    for (int t = 0; t < TOK; ++t) {
+      const uint32_t word[4] = {x[t].x, x[t].y, x[t].z, x[t].w};
+#pragma unroll
+      for (int h = 0; h < 4; ++h) y[t][h] = f2_add(f2_pack(bf16lo(word[h]), bf16hi(word[h])), f2_pack(b[2 * h], b[2 * h + 1]));
+    }
     float inv[TOK];
 #pragma unroll
     for (int t = 0; t < TOK; ++t) inv[t] = 1.f;
     if (p.norm == 2) {
 #pragma unroll
       for (int t = 0; t < TOK; ++t) {
-        float f[8];
-        unpack8(x[t], f);
         inv[t] = 0.f;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) { const float v = f[e] + b[e]; inv[t] += v * v; }
+        for (int h = 0; h < 4; ++h) {
+          float lo, hi;
+          f2_unpack(y[t][h], lo, hi);
+          inv[t] += lo * lo;
+          inv[t] += hi * hi;
+        }
       }
+      if constexpr (TOK == 2) {
+        both_inverses<LPH>(inv, lane, qk, p.eps);
+      } else {
 #pragma unroll
-      for (int o = LPH / 2; o > 0; o >>= 1)
-#pragma unroll
-        for (int t = 0; t < TOK; ++t) inv[t] += __shfl_xor_sync(0xffffffffu, inv[t], o);
-#pragma unroll
-      for (int t = 0; t < TOK; ++t) inv[t] = qk ? 1.0f / sqrtf(inv[t] / static_cast<float>(p.d) + p.eps) : 1.f;
+        for (int o = LPH / 2; o > 0; o >>= 1) inv[0] += __shfl_xor_sync(0xffffffffu, inv[0], o);
+        inv[0] = qk ? 1.0f / sqrtf(inv[0] / static_cast<float>(DIM) + p.eps) : 1.f;
+      }
     } else if (p.norm == 1 && qk) {
 #pragma unroll
       for (int t = 0; t < TOK; ++t) inv[t] = inv_s[is_k][t];
@@ -586,17 +618,16 @@ prep_vec8_kernel(const PrepArgs p) {
 #pragma unroll
     for (int t = 0; t < TOK; ++t) {
       float f[8];
-      unpack8(x[t], f);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) f[e] = (f[e] + b[e]) * inv[t] * w[e];
+      for (int h = 0; h < 4; ++h)
+        f2_unpack(f2_mul(f2_mul(y[t][h], f2_pack(inv[t], inv[t])), f2_pack(w[2 * h], w[2 * h + 1])), f[2 * h], f[2 * h + 1]);
       if (p.rot_dims > 0 && p.interleaved) {
         if (turned) {
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             const float4 cs = reinterpret_cast<const float4*>(turn + t * half + ci / 2)[e];
-            const float a0 = f[4 * e], a1 = f[4 * e + 2];
-            f[4 * e] = a0 * cs.x - f[4 * e + 1] * cs.y;     f[4 * e + 1] = f[4 * e + 1] * cs.x + a0 * cs.y;
-            f[4 * e + 2] = a1 * cs.z - f[4 * e + 3] * cs.w; f[4 * e + 3] = f[4 * e + 3] * cs.z + a1 * cs.w;
+            turn_pair(f[4 * e], f[4 * e + 1], cs.x, cs.y);
+            turn_pair(f[4 * e + 2], f[4 * e + 3], cs.z, cs.w);
           }
         }
       } else if (p.rot_dims > 0) {
@@ -620,6 +651,126 @@ prep_vec8_kernel(const PrepArgs p) {
   }
 }
 
+// The same for many tokens where heads are normed one by one or not at all (one pass over a row): a thread keeps its piece of the row - bias, norm weights, source and
+// destination - and walks WALK consecutive tokens two at a time, with the pieces of the next four on their way and the angles of all WALK in shared memory.  Above,
+// every two tokens paid for their own indexes, weights, angles and barrier.
+// Bound: HBM where nothing is turned, the turns' instructions beside it else.  16 + 8 + 8 heads of 128, 8192 / 4856 ragged tokens in us, above / this one: plain
+// 31.5 / 24.5 and 18.0 / 11.4, 64 coordinates turned by frequencies 37.4 / 28.2 and 20.8 / 14.5, head norms 37.4 / 25.5 and 22.1 / 13.8, head norms and a table
+// 45.1 / 31.4 and 26.0 / 17.5 (pairs), 57.8 / 38.0 and 34.3 / 22.0 (halves).  Angles read from the table by every thread 52 us, cosines beside sines in shared memory 32
+// and 51; WALK of 4 30.8 and 18.5, of 16 31.2 and 19.4; two pieces on their way 32.2 and 19.3.  Fewer than 8 tokens a multiprocessor stay above, a token a CTA.
+constexpr int WALK = 8, AHEAD = 4;
+
+template <int LPH, bool PAIRS>
+__global__ void __launch_bounds__(ROW_THREADS, 3)
+prep_walk_kernel(const PrepArgs p) {
+  extern __shared__ __align__(16) float turns[];          // [WALK][rot_dims]: the tokens' rows of the table, cosines and then sines
+  constexpr int DIM = LPH * 8;
+  const int nq = p.H * p.d, nk = p.G * p.d, nv = p.Gv * p.dv, half = p.rot_dims / 2;
+  const int q8 = nq / 8, k8 = p.k_cache != nullptr ? nk / 8 : 0, v8 = p.v_cache != nullptr ? nv / 8 : 0, items = q8 + k8 + v8;
+  const int i = blockIdx.y * ROW_THREADS + threadIdx.x, lane = threadIdx.x & 31;
+  const bool live = i < items, is_q = i < q8, is_k = !is_q && i < q8 + k8, qk = live && (is_q || is_k);
+  const int c = live ? (is_q ? i : is_k ? i - q8 : i - q8 - k8) * 8 : 0;
+  const __nv_bfloat16* src = p.u + (is_q ? p.q_off : is_k || p.v_off < 0 ? p.k_off : p.v_off) + c;
+  __nv_bfloat16* dst = (is_q ? p.q_out : is_k ? p.k_cache : p.v_cache) + c;
+  const int64_t dst_row = is_q ? nq : is_k ? nk : nv;
+  const int t0 = blockIdx.x * WALK, cnt = min(WALK, p.n_tokens - t0);
+  uint4 x[WALK];
+  int slot[WALK];                                         // -1: padding row, or behind the last token
+  auto load = [&](int t) {
+    x[t] = make_uint4(0u, 0u, 0u, 0u);
+    slot[t] = -1;
+    if (live && t < cnt) {
+      x[t] = ldg_v4(src + static_cast<int64_t>(t0 + t) * p.ldu);
+      slot[t] = p.slot_mapping[t0 + t];
+    }
+  };
+#pragma unroll
+  for (int t = 0; t < AHEAD; ++t) load(t);
+  if (p.rot != nullptr) {
+    for (int a = threadIdx.x * 4; a < cnt * p.rot_dims; a += ROW_THREADS * 4)
+      *reinterpret_cast<float4*>(turns + a) = *reinterpret_cast<const float4*>(p.rot + static_cast<int64_t>(t0) * p.rot_dims + a);
+  } else {
+    for (int a = threadIdx.x; a < cnt * half; a += ROW_THREADS) {
+      const int t = a / half, k = a - t * half;
+      float* row = turns + t * p.rot_dims;
+      sincosf(static_cast<float>(p.positions[t0 + t]) * p.freq[k], row + half + k, row + k);
+    }
+  }
+  const float* bias = is_q ? p.q_bias : is_k || p.v_off < 0 ? p.k_bias : p.v_bias;
+  float b[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, w[8] = {1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f};
+  if (live && bias != nullptr) load8_f(bias + c, b);
+  const int ci = qk ? c & (DIM - 1) : DIM;                // the piece's first coordinate in its head
+  if (qk && p.norm != 0) load8_f((is_q ? p.q_norm_w : p.k_norm_w) + ci, w);
+  const bool turned = qk && ci < p.rot_dims, second = !PAIRS && ci >= half;
+  const int angle = PAIRS ? ci / 2 : second ? ci - half : ci;      // the first angle of the piece
+  if (p.rot_dims > 0) __syncthreads();
+  if ((i & ~31) >= items) return;                         // a warp stays together for the shuffles
+  const int from = !turned ? lane : second ? lane - half / 8 : lane + half / 8;
+#pragma unroll
+  for (int t = 0; t < WALK; t += 2) {
+    if (t >= cnt) break;
+#pragma unroll
+    for (int k = AHEAD; k < AHEAD + 2; ++k) if (t + k < WALK) load(t + k);
+    uint64_t y[2][4];
+    float inv[2] = {1.f, 1.f};
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const uint32_t word[4] = {x[t + k].x, x[t + k].y, x[t + k].z, x[t + k].w};
+#pragma unroll
+      for (int h = 0; h < 4; ++h) y[k][h] = f2_add(f2_pack(bf16lo(word[h]), bf16hi(word[h])), f2_pack(b[2 * h], b[2 * h + 1]));
+    }
+    if (p.norm == 2) {
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        inv[k] = 0.f;
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          float lo, hi;
+          f2_unpack(y[k][h], lo, hi);
+          inv[k] += lo * lo;
+          inv[k] += hi * hi;
+        }
+      }
+      both_inverses<LPH>(inv, lane, qk, p.eps);
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int row = t0 + t + k;
+      float f[8];
+#pragma unroll
+      for (int h = 0; h < 4; ++h)
+        f2_unpack(f2_mul(f2_mul(y[k][h], f2_pack(inv[k], inv[k])), f2_pack(w[2 * h], w[2 * h + 1])), f[2 * h], f[2 * h + 1]);
+      if (p.rot_dims > 0) {
+        const float* cs = turns + (t + k) * p.rot_dims + angle;
+        if constexpr (PAIRS) {
+          if (turned) {
+            const float4 co = *reinterpret_cast<const float4*>(cs), si = *reinterpret_cast<const float4*>(cs + half);
+            turn_pair(f[0], f[1], co.x, si.x);
+            turn_pair(f[2], f[3], co.y, si.y);
+            turn_pair(f[4], f[5], co.z, si.z);
+            turn_pair(f[6], f[7], co.w, si.w);
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; e += 4) {
+            float co[4] = {1.f, 1.f, 1.f, 1.f}, si[4] = {0.f, 0.f, 0.f, 0.f}, other[4];
+#pragma unroll
+            for (int m = 0; m < 4; ++m) other[m] = __shfl_sync(0xffffffffu, f[e + m], from);
+            if (turned) {
+              load4_f<float>(cs + e, co);
+              load4_f<float>(cs + half + e, si);
+#pragma unroll
+              for (int m = 0; m < 4; ++m) f[e + m] = f[e + m] * co[m] + (second ? other[m] : -other[m]) * si[m];
+            }
+          }
+        }
+      }
+      if (slot[t + k] >= 0)
+        stg_v4(dst + (is_q ? row : slot[t + k]) * dst_row, make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7])));
+    }
+  }
+}
+
 // Whole 16-byte pieces everywhere, and a head's lanes a power of two, so that heads never straddle warps; the kernels above take the rest.
 static bool prep_vec8_applies(const PrepArgs& p) {
   const int lanes = p.d / 8;
@@ -634,6 +785,13 @@ static bool prep_vec8_applies(const PrepArgs& p) {
 template <int LPH>
 static void go_prep_vec8(const PrepArgs& p, cudaStream_t st) {
   const size_t turn = static_cast<size_t>(p.rot_dims / 2) * sizeof(float2);
+  if (p.n_tokens >= 8 * sm_count() && p.norm != 1 && aligned16(p.rot)) {
+    const int items = (p.H * p.d + (p.k_cache != nullptr ? p.G * p.d : 0) + (p.v_cache != nullptr ? p.Gv * p.dv : 0)) / 8;
+    const dim3 grid((p.n_tokens + WALK - 1) / WALK, (items + ROW_THREADS - 1) / ROW_THREADS);
+    if (p.interleaved) prep_walk_kernel<LPH, true><<<grid, ROW_THREADS, WALK * turn, st>>>(p);
+    else prep_walk_kernel<LPH, false><<<grid, ROW_THREADS, WALK * turn, st>>>(p);
+    return;
+  }
   if (p.n_tokens >= 8 * sm_count()) prep_vec8_kernel<2, LPH><<<(p.n_tokens + 1) / 2, ROW_THREADS, 2 * turn, st>>>(p);
   else prep_vec8_kernel<1, LPH><<<p.n_tokens, ROW_THREADS, turn, st>>>(p);
 }
