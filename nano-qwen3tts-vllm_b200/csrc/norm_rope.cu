@@ -22,10 +22,34 @@ __device__ __forceinline__ float rstd_of(float sumsq, int cols, float eps) {
   return EAGER ? 1.0f / sqrtf(var) : rsqrtf(var);
 }
 
-template <bool EAGER>
-__device__ __forceinline__ float norm_out(float x, float rstd, float w) {
-  return EAGER ? rbf(rbf(x * rstd) * w) : (x * rstd) * w;   // caller rounds once more (no-op for EAGER)
+// Two bf16 at once.  A product or sum of two bf16 that is rounded once is what float arithmetic and a conversion give: the float product is exact, and a float
+// sum of two bf16 is inexact only far from the middle of two bf16.  Conversions were what bounded head norms (turning 24 heads of 5627 tokens 36 -> 30 us) and
+// cost row norms a tenth (8192 rows of 2048 20.6 -> 17.9).
+__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
 }
+__device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+template <bool EAGER>
+__device__ __forceinline__ uint32_t norm_pair(float a, float b, float rstd, uint32_t w) {
+  if (EAGER) return mul_bf16x2(pack_bf16(a * rstd, b * rstd), w);
+  return pack_bf16(a * rstd * bf16lo(w), b * rstd * bf16hi(w));
+}
+template <bool EAGER>
+__device__ __forceinline__ uint32_t norm_pair(uint32_t x, float rstd, uint32_t w) { return norm_pair<EAGER>(bf16lo(x), bf16hi(x), rstd, w); }
+template <bool EAGER>
+__device__ __forceinline__ uint4 norm_eight(const float* f, float rstd, uint4 w) {
+  return make_uint4(norm_pair<EAGER>(f[0], f[1], rstd, w.x), norm_pair<EAGER>(f[2], f[3], rstd, w.y), norm_pair<EAGER>(f[4], f[5], rstd, w.z),
+                    norm_pair<EAGER>(f[6], f[7], rstd, w.w));
+}
+// (x1, x2) turned: rotate_half pairs the first half with minus the second
+__device__ __forceinline__ uint32_t turn_first(uint32_t x1, uint32_t x2, uint32_t c, uint32_t s) { return add_bf16x2(mul_bf16x2(x1, c), mul_bf16x2(x2 ^ 0x80008000u, s)); }
+__device__ __forceinline__ uint32_t turn_second(uint32_t x1, uint32_t x2, uint32_t c, uint32_t s) { return add_bf16x2(mul_bf16x2(x2, c), mul_bf16x2(x1, s)); }
 
 __device__ __forceinline__ float block_sum(float v, float* red) {
   v = warp_sum(v);
@@ -85,16 +109,7 @@ rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_stride, const __nv
   for (int i = 0; i < RMS_MAXV; ++i) {
     const int v = threadIdx.x + i * RMS_THREADS;
     if (v < nvec) {
-      uint4 wr = ldg_v4(w + 8 * v);
-      float o[8];
-      o[0] = norm_out<EAGER>(f[i][0], rstd, bf16lo(wr.x)); o[1] = norm_out<EAGER>(f[i][1], rstd, bf16hi(wr.x));
-      o[2] = norm_out<EAGER>(f[i][2], rstd, bf16lo(wr.y)); o[3] = norm_out<EAGER>(f[i][3], rstd, bf16hi(wr.y));
-      o[4] = norm_out<EAGER>(f[i][4], rstd, bf16lo(wr.z)); o[5] = norm_out<EAGER>(f[i][5], rstd, bf16hi(wr.z));
-      o[6] = norm_out<EAGER>(f[i][6], rstd, bf16lo(wr.w)); o[7] = norm_out<EAGER>(f[i][7], rstd, bf16hi(wr.w));
-      uint4 ov;
-      ov.x = pack_bf16(o[0], o[1]); ov.y = pack_bf16(o[2], o[3]);
-      ov.z = pack_bf16(o[4], o[5]); ov.w = pack_bf16(o[6], o[7]);
-      stg_v4(y + (int64_t)row * cols + 8 * v, ov);
+      stg_v4(y + (int64_t)row * cols + 8 * v, norm_eight<EAGER>(f[i], rstd, ldg_v4(w + 8 * v)));
     }
   }
 }
@@ -120,13 +135,7 @@ rmsnorm_narrow_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_stride, con
   }
   const float rstd = rstd_of<EAGER>(warp_sum(ss), cols, eps);
   if (lane < nvec) {
-    uint4 wr = ldg_v4(w + 8 * lane);
-    uint4 ov;
-    ov.x = pack_bf16(norm_out<EAGER>(f[0], rstd, bf16lo(wr.x)), norm_out<EAGER>(f[1], rstd, bf16hi(wr.x)));
-    ov.y = pack_bf16(norm_out<EAGER>(f[2], rstd, bf16lo(wr.y)), norm_out<EAGER>(f[3], rstd, bf16hi(wr.y)));
-    ov.z = pack_bf16(norm_out<EAGER>(f[4], rstd, bf16lo(wr.z)), norm_out<EAGER>(f[5], rstd, bf16hi(wr.z)));
-    ov.w = pack_bf16(norm_out<EAGER>(f[6], rstd, bf16lo(wr.w)), norm_out<EAGER>(f[7], rstd, bf16hi(wr.w)));
-    stg_v4(y + (int64_t)row * cols + 8 * lane, ov);
+    stg_v4(y + (int64_t)row * cols + 8 * lane, norm_eight<EAGER>(f, rstd, ldg_v4(w + 8 * lane)));
   }
 }
 
@@ -134,8 +143,7 @@ rmsnorm_narrow_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_stride, con
 // Fused q/k head-norm + RoPE + KV write.  One CTA per token, 8 warps; a warp owns one head at a
 // time (lane l holds dims {2l, 2l+1, 64+2l, 64+2l+1} -> two fully coalesced 128-byte accesses) and walks heads
 // warp, warp+8, ...  Cosines and sines are formed once a token, by 128 threads, while the rows of a warp's first four heads
-// and of the values are on their way.  Bound: HBM; 5627 tokens of 16 + 8 + 8 heads: 42 -> 37 us (14 at the copy rate; every warp
-// formed all of them for itself before, in front of its loads).
+// and of the values are on their way.  For steps of few tokens, see the kernel behind it.
 struct QkRopeParams {
   const __nv_bfloat16 *q, *k, *v;
   int64_t q_stride, k_stride, v_stride;
@@ -182,20 +190,17 @@ qknorm_rope_kvwrite_kernel(const QkRopeParams p) {
   if (put_v && threadIdx.x < (kv_dim >> 3)) v0 = ldg_nc_v4(p.v + (int64_t)tok * p.v_stride + 8 * threadIdx.x);
   // cos/sin of columns f (turns[0]) and 64 + f (turns[1]): fp32 angle, fp32 cos/sin, bf16 result.  Both share frequency f but - in the
   // sectioned M-RoPE branch (rotary_embedding.py:73-80) - not necessarily the position row.
-  __shared__ float2 turns[2][HD / 2];
+  __shared__ __align__(4) __nv_bfloat16 turns[2][2][HD / 2];          // [column half][cosine, sine]
   if (threadIdx.x < HD) {
     const int f = threadIdx.x & 63;
     const int m = p.modality ? __ldg(p.modality + threadIdx.x) : 0;
     const float ang = (float)__ldg(p.positions + (int64_t)m * p.pos_row_stride + tok) * __ldg(p.inv_freq + f);
-    turns[threadIdx.x >> 6][f] = make_float2(rbf(cosf(ang) * p.attention_scaling), rbf(sinf(ang) * p.attention_scaling));
+    turns[threadIdx.x >> 6][0][f] = __float2bfloat16_rn(cosf(ang) * p.attention_scaling);
+    turns[threadIdx.x >> 6][1][f] = __float2bfloat16_rn(sinf(ang) * p.attention_scaling);
   }
   __syncthreads();
-  float c1[2], s1[2], c2[2], s2[2];
-#pragma unroll
-  for (int e = 0; e < 2; ++e) {
-    const float2 a = turns[0][2 * lane + e], b = turns[1][2 * lane + e];
-    c1[e] = a.x; s1[e] = a.y; c2[e] = b.x; s2[e] = b.y;
-  }
+  const auto pair_of = [&](int half, int part) { return *reinterpret_cast<const uint32_t*>(&turns[half][part][2 * lane]); };
+  const uint32_t c1 = pair_of(0, 0), s1 = pair_of(0, 1), c2 = pair_of(1, 0), s2 = pair_of(1, 1);
 
   for (int h0 = warp; h0 < total; h0 += 8 * AHEAD) {
     if (h0 != warp) fetch(h0);
@@ -206,24 +211,15 @@ qknorm_rope_kvwrite_kernel(const QkRopeParams p) {
       const bool is_k = hh >= p.num_heads;
       const int h = is_k ? hh - p.num_heads : hh;
       const __nv_bfloat16* w = is_k ? p.k_w : p.q_w;
-      float x1[2] = {bf16lo(r1[i]), bf16hi(r1[i])};
-      float x2[2] = {bf16lo(r2[i]), bf16hi(r2[i])};
+      uint32_t x1 = r1[i], x2 = r2[i];
       if (w) {
-        float ss = x1[0] * x1[0];
-        ss = fmaf(x1[1], x1[1], ss); ss = fmaf(x2[0], x2[0], ss); ss = fmaf(x2[1], x2[1], ss);
+        float ss = bf16lo(x1) * bf16lo(x1);
+        ss = fmaf(bf16hi(x1), bf16hi(x1), ss); ss = fmaf(bf16lo(x2), bf16lo(x2), ss); ss = fmaf(bf16hi(x2), bf16hi(x2), ss);
         const float rstd = rstd_of<EAGER>(warp_sum(ss), HD, p.eps);
-        const uint32_t w1 = *reinterpret_cast<const uint32_t*>(w + 2 * lane);
-        const uint32_t w2 = *reinterpret_cast<const uint32_t*>(w + 64 + 2 * lane);
-        x1[0] = rbf(norm_out<EAGER>(x1[0], rstd, bf16lo(w1))); x1[1] = rbf(norm_out<EAGER>(x1[1], rstd, bf16hi(w1)));
-        x2[0] = rbf(norm_out<EAGER>(x2[0], rstd, bf16lo(w2))); x2[1] = rbf(norm_out<EAGER>(x2[1], rstd, bf16hi(w2)));
+        x1 = norm_pair<EAGER>(x1, rstd, *reinterpret_cast<const uint32_t*>(w + 2 * lane));
+        x2 = norm_pair<EAGER>(x2, rstd, *reinterpret_cast<const uint32_t*>(w + 64 + 2 * lane));
       }
-      float o1[2], o2[2];
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        o1[e] = rbf(x1[e] * c1[e]) + rbf(-x2[e] * s1[e]);   // rotate_half: first half pairs with -x2
-        o2[e] = rbf(x2[e] * c2[e]) + rbf(x1[e] * s2[e]);
-      }
-      const uint32_t y1 = pack_bf16(o1[0], o1[1]), y2 = pack_bf16(o2[0], o2[1]);
+      const uint32_t y1 = turn_first(x1, x2, c1, s1), y2 = turn_second(x1, x2, c2, s2);
       __nv_bfloat16* dst = nullptr;
       if (is_k) {
         if (p.k_out) dst = p.k_out + (int64_t)tok * kv_dim + h * HD;
@@ -246,6 +242,119 @@ qknorm_rope_kvwrite_kernel(const QkRopeParams p) {
     __nv_bfloat16* vd = p.v_cache + (int64_t)slot * kv_dim;
     if (threadIdx.x < (kv_dim >> 3)) stg_v4(vd + 8 * threadIdx.x, v0);
     for (int i = threadIdx.x + blockDim.x; i < (kv_dim >> 3); i += blockDim.x) stg_v4(vd + 8 * i, ldg_nc_v4(vs + 8 * i));
+  }
+}
+
+// The same for many tokens: a thread keeps coordinates 4m .. 4m + 3 and 64 + 4m .. of one head (a turn's partners; sixteen threads have a head) over QK_WALK
+// consecutive tokens, with its norm weights in registers and the pieces of the next four tokens on their way; the angles of all QK_WALK tokens are formed first, in
+// shared memory.  Two tokens share one tree of shuffles and one root, summed in the order of the kernel above: results are the same bits.
+// Bound: HBM (14 us at the copy rate without k_out) and instructions.  Tokens of 16 + 8 + 8 heads with k_out in us, above with float arithmetic and a conversion for
+// every rounding / above / this one: 5627 35.9 / 29.9 / 23.9, 1184 10.2 / 7.9 / 6.5; 3000 of 32 + 4 + 4 28.0 / 20.9 / 15.7; 1189 of 3 + 1 + 1 5.8 / 5.3 / 4.5.
+// Runs of 8 tokens 24.7, 7.0, 16.4, 5.7, of 16 25.0, 9.8, 18.9, 9.5.  Few tokens stay above: 300 of 4 + 2 + 2 heads 3.5, here 4.0.
+constexpr int QK_WALK = 4, QK_AHEAD = 2;
+
+template <bool EAGER>
+__global__ void __launch_bounds__(256, 4)
+qknorm_rope_walk_kernel(const QkRopeParams p, int n_tokens) {
+  constexpr int HD = 128;
+  __shared__ __align__(16) __nv_bfloat16 turns[QK_WALK][4][HD / 2];  // cosines and sines of the first columns, then (sectioned positions) of the others
+  const int t0 = blockIdx.x * QK_WALK, cnt = min(QK_WALK, n_tokens - t0), lane = threadIdx.x & 31;
+  const bool put_v = p.slot_mapping != nullptr && p.v != nullptr;
+  const int heads = p.num_heads + p.num_kv_heads * (put_v ? 2 : 1), kv_dim = p.num_kv_heads * HD;
+  const int i = blockIdx.y * 256 + threadIdx.x, head = i >> 4, col = (i & 15) * 4;
+  const bool live = head < heads, is_q = head < p.num_heads, is_k = !is_q && head < p.num_heads + p.num_kv_heads;
+  const int h = is_q ? head : is_k ? head - p.num_heads : head - p.num_heads - p.num_kv_heads;
+  const __nv_bfloat16* src = (is_q ? p.q : is_k ? p.k : p.v) + h * HD + col;
+  const int64_t stride = is_q ? p.q_stride : is_k ? p.k_stride : p.v_stride;
+  uint2 x1[QK_WALK], x2[QK_WALK];
+  int slot[QK_WALK];
+  auto load = [&](int t) {
+    x1[t] = x2[t] = make_uint2(0u, 0u);
+    slot[t] = -1;
+    if (live && t < cnt) {
+      x1[t] = ldg_v2(src + (t0 + t) * stride);
+      x2[t] = ldg_v2(src + (t0 + t) * stride + HD / 2);
+      if (!is_q && p.slot_mapping != nullptr) slot[t] = __ldg(p.slot_mapping + t0 + t);
+    }
+  };
+#pragma unroll
+  for (int t = 0; t < QK_AHEAD; ++t) load(t);
+  const int planes = p.modality != nullptr ? 2 : 1;
+  for (int a = threadIdx.x; a < cnt * planes * (HD / 2); a += 256) {
+    const int f = a & 63, t = (a >> 6) / planes, half = (a >> 6) - t * planes;
+    const int m = planes == 2 ? __ldg(p.modality + half * 64 + f) : 0;
+    const float ang = (float)__ldg(p.positions + (int64_t)m * p.pos_row_stride + t0 + t) * __ldg(p.inv_freq + f);
+    turns[t][2 * half][f] = __float2bfloat16_rn(cosf(ang) * p.attention_scaling);
+    turns[t][2 * half + 1][f] = __float2bfloat16_rn(sinf(ang) * p.attention_scaling);
+  }
+  const __nv_bfloat16* w = is_q ? p.q_w : is_k ? p.k_w : nullptr;
+  uint32_t w1[2] = {}, w2[2] = {};
+  if (live && w != nullptr) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      w1[e] = *reinterpret_cast<const uint32_t*>(w + col + 2 * e);
+      w2[e] = *reinterpret_cast<const uint32_t*>(w + HD / 2 + col + 2 * e);
+    }
+  }
+  __syncthreads();
+  if (((i & ~31) >> 4) >= heads) return;                  // a warp stays together for the shuffles
+#pragma unroll
+  for (int t = 0; t < QK_WALK; t += 2) {
+    if (t >= cnt) break;
+#pragma unroll
+    for (int k = QK_AHEAD; k < QK_AHEAD + 2; ++k) if (t + k < QK_WALK) load(t + k);
+    float rstd[2] = {1.f, 1.f};
+    if (p.q_w != nullptr) {
+      float ss[2][2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const uint32_t a = e ? x1[t + k].y : x1[t + k].x, b = e ? x2[t + k].y : x2[t + k].x;
+          float v = bf16lo(a) * bf16lo(a);
+          v = fmaf(bf16hi(a), bf16hi(a), v);
+          v = fmaf(bf16lo(b), bf16lo(b), v);
+          ss[k][e] = fmaf(bf16hi(b), bf16hi(b), v);
+        }
+      // upper eight of the sixteen threads go on with the second sums, every other four with the second token
+      const bool up = lane & 8, second = lane & 4;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const float keep = up ? ss[k][1] : ss[k][0];
+        ss[k][0] = keep + __shfl_xor_sync(0xffffffffu, up ? ss[k][0] : ss[k][1], 8);
+      }
+      float v = second ? ss[1][0] : ss[0][0];
+      v += __shfl_xor_sync(0xffffffffu, second ? ss[0][0] : ss[1][0], 4);
+      v += __shfl_xor_sync(0xffffffffu, v, 2);
+      v += __shfl_xor_sync(0xffffffffu, v, 1);
+      v += __shfl_xor_sync(0xffffffffu, v, 8);
+      v = rstd_of<EAGER>(v, HD, p.eps);
+      rstd[0] = __shfl_sync(0xffffffffu, v, lane & ~4);
+      rstd[1] = __shfl_sync(0xffffffffu, v, lane | 4);
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int tok = t0 + t + k;
+      uint2 y1 = x1[t + k], y2 = x2[t + k];
+      if (is_q || is_k) {
+        if (w != nullptr) {
+          y1 = make_uint2(norm_pair<EAGER>(y1.x, rstd[k], w1[0]), norm_pair<EAGER>(y1.y, rstd[k], w1[1]));
+          y2 = make_uint2(norm_pair<EAGER>(y2.x, rstd[k], w2[0]), norm_pair<EAGER>(y2.y, rstd[k], w2[1]));
+        }
+        const __nv_bfloat16 *first = &turns[t + k][0][col], *other = first + (planes - 1) * HD;
+        const uint2 c1 = ldg_v2(first), s1 = ldg_v2(first + HD / 2), c2 = ldg_v2(other), s2 = ldg_v2(other + HD / 2), a = y1, b = y2;
+        y1 = make_uint2(turn_first(a.x, b.x, c1.x, s1.x), turn_first(a.y, b.y, c1.y, s1.y));
+        y2 = make_uint2(turn_second(a.x, b.x, c2.x, s2.x), turn_second(a.y, b.y, c2.y, s2.y));
+      }
+      if (!live || t + k >= cnt) continue;
+      auto put = [&](__nv_bfloat16* dst) { stg_v2(dst, y1); stg_v2(dst + HD / 2, y2); };
+      if (is_q) {
+        put(p.q_out + ((int64_t)tok * p.num_heads + h) * HD + col);
+      } else {
+        if (is_k && p.k_out) put(p.k_out + (int64_t)tok * kv_dim + h * HD + col);
+        if (slot[t + k] >= 0) put((is_k ? p.k_cache : p.v_cache) + (int64_t)slot[t + k] * kv_dim + h * HD + col);
+      }
+    }
   }
 }
 
@@ -356,7 +465,12 @@ extern "C" int b2tts_qknorm_rope_kvwrite(const void* q, int64_t q_row_stride,
   p.k_cache = static_cast<__nv_bfloat16*>(k_cache); p.v_cache = static_cast<__nv_bfloat16*>(v_cache);
   p.num_heads = num_heads; p.num_kv_heads = num_kv_heads;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (rounding == B2TTS_ROUND_EAGER) qknorm_rope_kvwrite_kernel<true><<<n_tokens, 256, 0, st>>>(p);
+  if (n_tokens >= 8 * sm_count()) {                       // enough runs of tokens for every multiprocessor
+    const int heads = num_heads + num_kv_heads * (slot_mapping && v ? 2 : 1);
+    const dim3 grid((n_tokens + QK_WALK - 1) / QK_WALK, (heads * 16 + 255) / 256);
+    if (rounding == B2TTS_ROUND_EAGER) qknorm_rope_walk_kernel<true><<<grid, 256, 0, st>>>(p, n_tokens);
+    else qknorm_rope_walk_kernel<false><<<grid, 256, 0, st>>>(p, n_tokens);
+  } else if (rounding == B2TTS_ROUND_EAGER) qknorm_rope_kvwrite_kernel<true><<<n_tokens, 256, 0, st>>>(p);
   else qknorm_rope_kvwrite_kernel<false><<<n_tokens, 256, 0, st>>>(p);
   B2_CHECK_LAUNCH(what);
   return B2TTS_OK;
