@@ -196,48 +196,37 @@ fused_decode_attn_kernel(const FusedAttnParams p) {
   // warp+kvh, ...): q heads -> shared memory, and on the writer split k (normed + rotated) and v (raw)
   // -> cache[slot] and shared memory.
   {
-    float c1[2], s1[2], c2[2], s2[2];
+    float cf[2][2], sf[2][2];                             // [column half][dim 2l, 2l + 1]
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const float a1 = (float)(md1[e] == 0 ? pos[0] : md1[e] == 1 ? pos[1] : pos[2]) * frq[e];
-      c1[e] = rbf(cosf(a1) * p.attention_scaling);
-      s1[e] = rbf(sinf(a1) * p.attention_scaling);
+      cf[0][e] = cosf(a1) * p.attention_scaling;
+      sf[0][e] = sinf(a1) * p.attention_scaling;
+      cf[1][e] = cf[0][e];
+      sf[1][e] = sf[0][e];
       if (md2[e] != md1[e]) {
         const float a2 = (float)(md2[e] == 0 ? pos[0] : md2[e] == 1 ? pos[1] : pos[2]) * frq[e];
-        c2[e] = rbf(cosf(a2) * p.attention_scaling);
-        s2[e] = rbf(sinf(a2) * p.attention_scaling);
-      } else {
-        c2[e] = c1[e]; s2[e] = s1[e];
+        cf[1][e] = cosf(a2) * p.attention_scaling;
+        sf[1][e] = sinf(a2) * p.attention_scaling;
       }
     }
+    const uint32_t c1 = pack_bf16(cf[0][0], cf[0][1]), s1 = pack_bf16(sf[0][0], sf[0][1]), c2 = pack_bf16(cf[1][0], cf[1][1]), s2 = pack_bf16(sf[1][0], sf[1][1]);
 #pragma unroll
     for (int i = 0; i < GROUP + 1; ++i) {
       const bool is_k = i == GROUP;
       if (!(i < nh_q || (is_k && writer))) continue;
       const int h = is_k ? warp : warp + i * kvh;
       const bool has_w = is_k ? (p.k_w != nullptr) : (p.q_w != nullptr);
-      float x1[2] = {bf16lo(raw1[i]), bf16hi(raw1[i])};
-      float x2[2] = {bf16lo(raw2[i]), bf16hi(raw2[i])};
+      uint32_t x1 = raw1[i], x2 = raw2[i];
       if (has_w) {
-        float ss = x1[0] * x1[0];
-        ss = fmaf(x1[1], x1[1], ss); ss = fmaf(x2[0], x2[0], ss); ss = fmaf(x2[1], x2[1], ss);
+        float ss = bf16lo(x1) * bf16lo(x1);
+        ss = fmaf(bf16hi(x1), bf16hi(x1), ss); ss = fmaf(bf16lo(x2), bf16lo(x2), ss); ss = fmaf(bf16hi(x2), bf16hi(x2), ss);
         const float var = warp_sum(ss) / (float)FA_HD + p.eps;
         const float rstd = EAGER ? 1.0f / sqrtf(var) : rsqrtf(var);
-        const uint32_t w1 = is_k ? kw1 : qw1, w2 = is_k ? kw2 : qw2;
-        const float wf[4] = {bf16lo(w1), bf16hi(w1), bf16lo(w2), bf16hi(w2)};
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          x1[e] = rbf(EAGER ? rbf(x1[e] * rstd) * wf[e] : (x1[e] * rstd) * wf[e]);
-          x2[e] = rbf(EAGER ? rbf(x2[e] * rstd) * wf[2 + e] : (x2[e] * rstd) * wf[2 + e]);
-        }
+        x1 = norm_pair<EAGER>(x1, rstd, is_k ? kw1 : qw1);
+        x2 = norm_pair<EAGER>(x2, rstd, is_k ? kw2 : qw2);
       }
-      float o1[2], o2[2];
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        o1[e] = rbf(x1[e] * c1[e]) + rbf(-x2[e] * s1[e]);   // rotate_half: first half pairs with -x2
-        o2[e] = rbf(x2[e] * c2[e]) + rbf(x1[e] * s2[e]);
-      }
-      const uint32_t y1 = pack_bf16(o1[0], o1[1]), y2 = pack_bf16(o2[0], o2[1]);
+      const uint32_t y1 = turn_first(x1, x2, c1, s1), y2 = turn_second(x1, x2, c2, s2);
       __nv_bfloat16* dst = is_k ? kn_s + h * FA_HD : q_s + h * FA_HD;
       *reinterpret_cast<uint32_t*>(dst + 2 * lane) = y1;
       *reinterpret_cast<uint32_t*>(dst + 64 + 2 * lane) = y2;
@@ -536,39 +525,28 @@ fused_decode_attn_small_kernel(const FusedAttnParams p, int rows) {
   load_pair(0);
   // ---- prologue: q/k head norm + RoPE of the new token (the body of qknorm_rope_kvwrite_kernel), K / V to the cache
   {
-    float c1[2], s1[2];
+    float cf[2], sf[2];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const float a1 = (float)pos * frq[e];
-      c1[e] = rbf(cosf(a1) * p.attention_scaling);
-      s1[e] = rbf(sinf(a1) * p.attention_scaling);
+      cf[e] = cosf(a1) * p.attention_scaling;
+      sf[e] = sinf(a1) * p.attention_scaling;
     }
+    const uint32_t c1 = pack_bf16(cf[0], cf[1]), s1 = pack_bf16(sf[0], sf[1]);
 #pragma unroll
     for (int i = 0; i < GROUP + 1; ++i) {
       const bool is_k = i == GROUP;
       const bool has_w = is_k ? (p.k_w != nullptr) : (p.q_w != nullptr);
-      float x1[2] = {bf16lo(raw1[i]), bf16hi(raw1[i])};
-      float x2[2] = {bf16lo(raw2[i]), bf16hi(raw2[i])};
+      uint32_t x1 = raw1[i], x2 = raw2[i];
       if (has_w) {
-        float ss = x1[0] * x1[0];
-        ss = fmaf(x1[1], x1[1], ss); ss = fmaf(x2[0], x2[0], ss); ss = fmaf(x2[1], x2[1], ss);
+        float ss = bf16lo(x1) * bf16lo(x1);
+        ss = fmaf(bf16hi(x1), bf16hi(x1), ss); ss = fmaf(bf16lo(x2), bf16lo(x2), ss); ss = fmaf(bf16hi(x2), bf16hi(x2), ss);
         const float var = warp_sum(ss) / (float)FA_HD + p.eps;
         const float rstd = EAGER ? 1.0f / sqrtf(var) : rsqrtf(var);
-        const uint32_t w1 = is_k ? kw1 : qw1, w2 = is_k ? kw2 : qw2;
-        const float wf[4] = {bf16lo(w1), bf16hi(w1), bf16lo(w2), bf16hi(w2)};
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          x1[e] = rbf(EAGER ? rbf(x1[e] * rstd) * wf[e] : (x1[e] * rstd) * wf[e]);
-          x2[e] = rbf(EAGER ? rbf(x2[e] * rstd) * wf[2 + e] : (x2[e] * rstd) * wf[2 + e]);
-        }
+        x1 = norm_pair<EAGER>(x1, rstd, is_k ? kw1 : qw1);
+        x2 = norm_pair<EAGER>(x2, rstd, is_k ? kw2 : qw2);
       }
-      float o1[2], o2[2];
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        o1[e] = rbf(x1[e] * c1[e]) + rbf(-x2[e] * s1[e]);
-        o2[e] = rbf(x2[e] * c1[e]) + rbf(x1[e] * s1[e]);
-      }
-      const uint32_t y1 = pack_bf16(o1[0], o1[1]), y2 = pack_bf16(o2[0], o2[1]);
+      const uint32_t y1 = turn_first(x1, x2, c1, s1), y2 = turn_second(x1, x2, c1, s1);
       __nv_bfloat16* dst = is_k ? kn_s : q_s + i * FA_HD;
       *reinterpret_cast<uint32_t*>(dst + 2 * lane) = y1;
       *reinterpret_cast<uint32_t*>(dst + 64 + 2 * lane) = y2;

@@ -161,7 +161,7 @@ struct DrUnit { int row, head, part, L, s0, s1; };
 // The arithmetic of fused_decode_attn_kernel, a warp a query head of a split; returns whether no wait ran out.  Out of line: the projections' loops keep their
 // registers.
 template <bool EAGER>
-__device__ __forceinline__ bool dr_attend(const DrParams& p, const DrLayer& y, uint32_t e0, const DrUnit& a, __nv_bfloat16* q_s, const float4* trig_s, const int* pages, uint8_t* x_s,
+__device__ __forceinline__ bool dr_attend(const DrParams& p, const DrLayer& y, uint32_t e0, const DrUnit& a, __nv_bfloat16* q_s, const uint4* trig_s, const int* pages, uint8_t* x_s,
                                        bool alive) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ag = lane >> 3, aj = lane & 7;
   const int row = a.row, head = a.head, part = a.part, L = a.L, s0 = a.s0, s1 = a.s1, tiles = (L + FA_TILE - 1) / FA_TILE;
@@ -219,27 +219,18 @@ __device__ __forceinline__ bool dr_attend(const DrParams& p, const DrLayer& y, u
     uint32_t y1 = dr_wait(at, e0 + DR_E_QKV, alive), y2 = dr_wait(at + 32, e0 + DR_E_QKV, alive);
     __syncwarp();
     if (warp < DR_GROUP + 1) {
-      float x1[2] = {bf16lo(y1), bf16hi(y1)}, x2[2] = {bf16lo(y2), bf16hi(y2)};
       if (nw != nullptr) {
-        float ss = x1[0] * x1[0];
-        ss = fmaf(x1[1], x1[1], ss); ss = fmaf(x2[0], x2[0], ss); ss = fmaf(x2[1], x2[1], ss);
+        float ss = bf16lo(y1) * bf16lo(y1);
+        ss = fmaf(bf16hi(y1), bf16hi(y1), ss); ss = fmaf(bf16lo(y2), bf16lo(y2), ss); ss = fmaf(bf16hi(y2), bf16hi(y2), ss);
         const float var = warp_sum(ss) / static_cast<float>(DR_HD) + p.eps;
         const float rstd = EAGER ? 1.0f / sqrtf(var) : rsqrtf(var);
-        const float wf[4] = {bf16lo(w1), bf16hi(w1), bf16lo(w2), bf16hi(w2)};
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          x1[e] = rbf(EAGER ? rbf(x1[e] * rstd) * wf[e] : (x1[e] * rstd) * wf[e]);
-          x2[e] = rbf(EAGER ? rbf(x2[e] * rstd) * wf[2 + e] : (x2[e] * rstd) * wf[2 + e]);
-        }
+        y1 = norm_pair<EAGER>(y1, rstd, w1);
+        y2 = norm_pair<EAGER>(y2, rstd, w2);
       }
-      float r1[2], r2[2];
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const float4 z = trig_s[2 * lane + e];
-        r1[e] = rbf(x1[e] * z.x) + rbf(-x2[e] * z.y);                         // rotate_half: the first half pairs with -x2
-        r2[e] = rbf(x2[e] * z.z) + rbf(x1[e] * z.w);
-      }
-      y1 = pack_bf16(r1[0], r1[1]); y2 = pack_bf16(r2[0], r2[1]);
+      const uint4 z = trig_s[lane];
+      const uint32_t x1 = y1, x2 = y2;
+      y1 = turn_first(x1, x2, z.x, z.y);
+      y2 = turn_second(x1, x2, z.z, z.w);
     }
     uint32_t* to = reinterpret_cast<uint32_t*>(q_s + warp * DR_HD);
     to[lane] = y1; to[32 + lane] = y2;
@@ -374,7 +365,7 @@ template <int H, int I, int ROWS> struct DrShared {
   float red[2][DR_SUMS * 64];                            // of even and odd phases: [tile][slice][row][8 features]
   float ssq[DR_MAX_ROWS][8];
   __nv_bfloat16 q[(DR_GROUP + 2) * DR_HD];               // two query heads, key, value of the new token
-  float4 trig[DR_HD / 2];                                // cos, sin of dim i, cos, sin of dim 64 + i
+  __align__(16) __nv_bfloat16 trig[DR_HD / 4][4][2];     // for dims 2l, 2l + 1: cosines, sines, and those of dims 64 + 2l, 65 + 2l
   int pages[DR_PAGES];                                   // of the unit's row
   uint64_t full[DR_STAGES], empty[DR_STAGES];
   DrPlan plan;
@@ -607,8 +598,11 @@ decode_rows_kernel(const __grid_constant__ DrParams p) {
     const int m1 = p.modality != nullptr ? __ldg(p.modality + tid) : 0, m2 = p.modality != nullptr ? __ldg(p.modality + 64 + tid) : 0;
     const float a1 = static_cast<float>(m1 == 0 ? pos[0] : m1 == 1 ? pos[1] : pos[2]) * f;
     const float a2 = static_cast<float>(m2 == 0 ? pos[0] : m2 == 1 ? pos[1] : pos[2]) * f;
-    sm.trig[tid] = make_float4(rbf(cosf(a1) * p.attention_scaling), rbf(sinf(a1) * p.attention_scaling), rbf(cosf(a2) * p.attention_scaling),
-                               rbf(sinf(a2) * p.attention_scaling));
+    __nv_bfloat16(*to)[2] = sm.trig[tid >> 1];
+    to[0][tid & 1] = __float2bfloat16_rn(cosf(a1) * p.attention_scaling);
+    to[1][tid & 1] = __float2bfloat16_rn(sinf(a1) * p.attention_scaling);
+    to[2][tid & 1] = __float2bfloat16_rn(cosf(a2) * p.attention_scaling);
+    to[3][tid & 1] = __float2bfloat16_rn(sinf(a2) * p.attention_scaling);
   }
   dr_sync();
 
@@ -629,7 +623,7 @@ decode_rows_kernel(const __grid_constant__ DrParams p) {
     uint32_t r = 0;
     if (phase & 1) {
       if (phase == 1) {
-        if (sm.plan.unit.s1 > 0) alive = dr_attend<EAGER>(p, y, e0, sm.plan.unit, sm.q, sm.trig, sm.pages, sm.x, alive);
+        if (sm.plan.unit.s1 > 0) alive = dr_attend<EAGER>(p, y, e0, sm.plan.unit, sm.q, reinterpret_cast<const uint4*>(sm.trig), sm.pages, sm.x, alive);
         dr_sync();                                                                // its splits have been read
         asm volatile("" : "+r"(tid), "+r"(warp), "+r"(lane));
       }

@@ -22,35 +22,11 @@ __device__ __forceinline__ float rstd_of(float sumsq, int cols, float eps) {
   return EAGER ? 1.0f / sqrtf(var) : rsqrtf(var);
 }
 
-// Two bf16 at once.  A product or sum of two bf16 that is rounded once is what float arithmetic and a conversion give: the float product is exact, and a float
-// sum of two bf16 is inexact only far from the middle of two bf16.  Conversions were what bounded head norms (turning 24 heads of 5627 tokens 36 -> 30 us) and
-// cost row norms a tenth (8192 rows of 2048 20.6 -> 17.9).
-__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
-  uint32_t r;
-  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-  return r;
-}
-__device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
-  uint32_t r;
-  asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-  return r;
-}
-template <bool EAGER>
-__device__ __forceinline__ uint32_t norm_pair(float a, float b, float rstd, uint32_t w) {
-  if (EAGER) return mul_bf16x2(pack_bf16(a * rstd, b * rstd), w);
-  return pack_bf16(a * rstd * bf16lo(w), b * rstd * bf16hi(w));
-}
-template <bool EAGER>
-__device__ __forceinline__ uint32_t norm_pair(uint32_t x, float rstd, uint32_t w) { return norm_pair<EAGER>(bf16lo(x), bf16hi(x), rstd, w); }
 template <bool EAGER>
 __device__ __forceinline__ uint4 norm_eight(const float* f, float rstd, uint4 w) {
   return make_uint4(norm_pair<EAGER>(f[0], f[1], rstd, w.x), norm_pair<EAGER>(f[2], f[3], rstd, w.y), norm_pair<EAGER>(f[4], f[5], rstd, w.z),
                     norm_pair<EAGER>(f[6], f[7], rstd, w.w));
 }
-// (x1, x2) turned: rotate_half pairs the first half with minus the second
-__device__ __forceinline__ uint32_t turn_first(uint32_t x1, uint32_t x2, uint32_t c, uint32_t s) { return add_bf16x2(mul_bf16x2(x1, c), mul_bf16x2(x2 ^ 0x80008000u, s)); }
-__device__ __forceinline__ uint32_t turn_second(uint32_t x1, uint32_t x2, uint32_t c, uint32_t s) { return add_bf16x2(mul_bf16x2(x2, c), mul_bf16x2(x1, s)); }
-
 __device__ __forceinline__ float block_sum(float v, float* red) {
   v = warp_sum(v);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = (blockDim.x + 31) >> 5;
