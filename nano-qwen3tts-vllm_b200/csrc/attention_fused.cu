@@ -59,9 +59,13 @@ __device__ __forceinline__ uint4 fa_pack8(const float* f) {
   return r;
 }
 
-template <int GROUP, bool EAGER>
+template <int GROUP, bool EAGER, bool SPLIT>
 __global__ void __launch_bounds__(288, 2)
 fused_decode_attn_kernel(const FusedAttnParams p) {
+  // Two heads a key head without splits: many tiles a CTA, and a turn of the ring without branches (200 rows of 200 tokens 32.5 -> 30.2 us); with splits the longer
+  // code costs more than it gives (64 rows of 40 tokens 8.4, unrolled 10.1), with four heads it spills.
+  constexpr int UNROLL = GROUP == 2 && !SPLIT ? FA_NSTAGE : 1;
+  constexpr bool PACKED = GROUP < 4;                      // pairs of four heads spill: 200 rows of 200 tokens 104 us one by one, 113 packed
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const int kvh = p.num_kv_heads;
   const int kv_dim = kvh * FA_HD;
@@ -244,24 +248,26 @@ fused_decode_attn_kernel(const FusedAttnParams p) {
   asm volatile("bar.sync 1, %0;" :: "r"(kvh * 32) : "memory");      // the consumer warps only
 
   // ---- this warp's q heads from shared memory, pre-scaled for exp2
-  float qv[GROUP][16];
+  uint64_t qv[GROUP][8];
 #pragma unroll
   for (int h = 0; h < GROUP; ++h) {
     const __nv_bfloat16* qp = q_s + (head0 + h) * FA_HD;
-    fa_unpack8(*reinterpret_cast<const uint4*>(qp + 8 * j), qv[h]);
-    fa_unpack8(*reinterpret_cast<const uint4*>(qp + 64 + 8 * j), qv[h] + 8);
+    fa_pairs8(*reinterpret_cast<const uint4*>(qp + 8 * j), qv[h]);
+    fa_pairs8(*reinterpret_cast<const uint4*>(qp + 64 + 8 * j), qv[h] + 4);
 #pragma unroll
-    for (int d = 0; d < 16; ++d) qv[h][d] *= p.scale_log2;
+    for (int d = 0; d < 8; ++d) qv[h][d] = f2_mul(qv[h][d], f2_pack(p.scale_log2, p.scale_log2));
   }
 
-  float m[GROUP], l[GROUP], acc[GROUP][16];
+  float m[GROUP], l[GROUP];
+  uint64_t acc2[GROUP][8];                                // weighted sums of values, in pairs
 #pragma unroll
   for (int h = 0; h < GROUP; ++h) {
     m[h] = -INFINITY; l[h] = 0.f;
 #pragma unroll
-    for (int d = 0; d < 16; ++d) acc[h][d] = 0.f;
+    for (int d = 0; d < 8; ++d) acc2[h][d] = 0;
   }
 
+#pragma unroll UNROLL
   for (int i = 0; i < my_tiles; ++i) {
     const int stage = i % FA_NSTAGE;
     const uint32_t ph = (i / FA_NSTAGE) & 1;
@@ -286,32 +292,40 @@ fused_decode_attn_kernel(const FusedAttnParams p) {
       __syncwarp();
     }
 
+    // Keys of all token slots, their products, then the values on their way while the products are summed over lanes and turned into weights
     float s[FA_TILE / 4][GROUP];
-    int tokc[FA_TILE / 4];
+    uint4 raw[FA_TILE / 4][2];
+    int at[FA_TILE / 4];
 #pragma unroll
     for (int it = 0; it < FA_TILE / 4; ++it) {
       const int tok = it * 4 + g;
-      const bool valid = tok < ntok;
-      tokc[it] = valid ? tok : 0;
-      const __nv_bfloat16* kr = kt + tokc[it] * kv_dim;
-      float kf[16];
-      fa_unpack8(*reinterpret_cast<const uint4*>(kr + 8 * j), kf);
-      fa_unpack8(*reinterpret_cast<const uint4*>(kr + 64 + 8 * j), kf + 8);
-#pragma unroll
-      for (int h = 0; h < GROUP; ++h) {
-        float d0 = 0.f, d1 = 0.f;
-#pragma unroll
-        for (int d = 0; d < 16; d += 2) {
-          d0 = fmaf(qv[h][d], kf[d], d0);
-          d1 = fmaf(qv[h][d + 1], kf[d + 1], d1);
-        }
-        float dot = d0 + d1;
-        dot += __shfl_xor_sync(0xffffffffu, dot, 1);
-        dot += __shfl_xor_sync(0xffffffffu, dot, 2);
-        dot += __shfl_xor_sync(0xffffffffu, dot, 4);
-        s[it][h] = valid ? dot : -INFINITY;
-      }
+      at[it] = (tok < ntok ? tok : 0) * kv_dim + 8 * j;
+      raw[it][0] = *reinterpret_cast<const uint4*>(kt + at[it]);
+      raw[it][1] = *reinterpret_cast<const uint4*>(kt + at[it] + 64);
     }
+#pragma unroll
+    for (int it = 0; it < FA_TILE / 4; ++it) {
+      uint64_t kf[8];
+      fa_pairs8(raw[it][0], kf);
+      fa_pairs8(raw[it][1], kf + 4);
+#pragma unroll
+      for (int h = 0; h < GROUP; ++h) s[it][h] = fa_dot16<PACKED>(qv[h], kf);
+    }
+#pragma unroll
+    for (int it = 0; it < FA_TILE / 4; ++it) {
+      raw[it][0] = *reinterpret_cast<const uint4*>(vt + at[it]);
+      raw[it][1] = *reinterpret_cast<const uint4*>(vt + at[it] + 64);
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+      for (int it = 0; it < FA_TILE / 4; ++it)
+#pragma unroll
+        for (int h = 0; h < GROUP; ++h) s[it][h] += __shfl_xor_sync(0xffffffffu, s[it][h], o);
+#pragma unroll
+    for (int it = 0; it < FA_TILE / 4; ++it)
+#pragma unroll
+      for (int h = 0; h < GROUP; ++h) s[it][h] = it * 4 + g < ntok ? s[it][h] : -INFINITY;
     float alpha[GROUP];
 #pragma unroll
     for (int h = 0; h < GROUP; ++h) {
@@ -331,26 +345,28 @@ fused_decode_attn_kernel(const FusedAttnParams p) {
       }
       l[h] = fmaf(l[h], alpha[h], ps);
 #pragma unroll
-      for (int d = 0; d < 16; ++d) acc[h][d] *= alpha[h];
+      for (int d = 0; d < 8; ++d) acc2[h][d] = fa_mul2<PACKED>(acc2[h][d], f2_pack(alpha[h], alpha[h]));
     }
 #pragma unroll
     for (int it = 0; it < FA_TILE / 4; ++it) {
-      const __nv_bfloat16* vr = vt + tokc[it] * kv_dim;
-      float vf[16];
-      fa_unpack8(*reinterpret_cast<const uint4*>(vr + 8 * j), vf);
-      fa_unpack8(*reinterpret_cast<const uint4*>(vr + 64 + 8 * j), vf + 8);
+      uint64_t vf[8];
+      fa_pairs8(raw[it][0], vf);
+      fa_pairs8(raw[it][1], vf + 4);
 #pragma unroll
       for (int h = 0; h < GROUP; ++h)
 #pragma unroll
-        for (int d = 0; d < 16; ++d) acc[h][d] = fmaf(s[it][h], vf[d], acc[h][d]);
+        for (int d = 0; d < 8; ++d) acc2[h][d] = fa_fma2<PACKED>(f2_pack(s[it][h], s[it][h]), vf[d], acc2[h][d]);
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(empty_bar + stage);
   }
 
   // ---- fold the 4 token slots of the warp
+  float acc[GROUP][16];
 #pragma unroll
   for (int h = 0; h < GROUP; ++h) {
+#pragma unroll
+    for (int d = 0; d < 8; ++d) f2_unpack(acc2[h][d], acc[h][2 * d], acc[h][2 * d + 1]);
     l[h] += __shfl_xor_sync(0xffffffffu, l[h], 8);
     l[h] += __shfl_xor_sync(0xffffffffu, l[h], 16);
 #pragma unroll
@@ -360,7 +376,7 @@ fused_decode_attn_kernel(const FusedAttnParams p) {
     }
   }
 
-  if (p.nsplit == 1) {
+  if constexpr (!SPLIT) {
     if (g == 0) {
 #pragma unroll
       for (int h = 0; h < GROUP; ++h) {
@@ -373,9 +389,7 @@ fused_decode_attn_kernel(const FusedAttnParams p) {
         stg_v4(op + 64 + 8 * j, fa_pack8(o + 8));
       }
     }
-    return;
-  }
-
+  } else {
   // ---- split-KV: partials out, then the last CTA of this sequence folds all of them
   if (g == 0) {
 #pragma unroll
@@ -405,31 +419,53 @@ fused_decode_attn_kernel(const FusedAttnParams p) {
   }
   asm volatile("bar.sync 1, %0;" :: "r"(kvh * 32) : "memory");
   if (!*last_flag) return;
-  // warp w folds heads head0 .. head0+GROUP-1; lane owns 4 consecutive dims
+  // warp w folds heads head0 .. head0+GROUP-1; lane owns 4 consecutive dims.  Lane s asks for split s's maximum and sum (at most 32 splits), and the partials of
+  // four splits of all heads are asked for at once: a split after another was up to three dependent round trips for each: 64 rows of 40
+  // tokens 10.4 -> 8.5 us, of 200 16.1 -> 14.7, 16 rows of 700 22.3 -> 15.9, 4 of 2000 25.7 -> 18.4 (16 query and 8 key heads).
+  float top[GROUP], sum[GROUP];
 #pragma unroll
   for (int h = 0; h < GROUP; ++h) {
-    const int head = head0 + h;
-    const int64_t base = ((int64_t)row * p.nsplit) * p.num_heads + head;
-    float M = -INFINITY;
-    for (int s = 0; s < p.nsplit; ++s) M = fmaxf(M, __ldcg(p.part_ml + (base + (int64_t)s * p.num_heads) * 2));
-    float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
-    float den = 0.f;
-    for (int s = 0; s < p.nsplit; ++s) {
-      const int64_t idx = base + (int64_t)s * p.num_heads;
-      const float ls = __ldcg(p.part_ml + idx * 2 + 1);
-      if (ls > 0.f) {
-        const float w = fa_exp2(__ldcg(p.part_ml + idx * 2) - M);
-        const float4 a = __ldcg(reinterpret_cast<const float4*>(p.part_acc + idx * FA_HD) + lane);
-        num.x = fmaf(w, a.x, num.x); num.y = fmaf(w, a.y, num.y);
-        num.z = fmaf(w, a.z, num.z); num.w = fmaf(w, a.w, num.w);
-        den = fmaf(w, ls, den);
+    const int64_t at = ((int64_t)row * p.nsplit + lane) * p.num_heads + head0 + h;
+    top[h] = lane < p.nsplit ? __ldcg(p.part_ml + at * 2) : -INFINITY;
+    sum[h] = lane < p.nsplit ? __ldcg(p.part_ml + at * 2 + 1) : 0.f;
+  }
+  float4 num[GROUP];
+  float den[GROUP];
+#pragma unroll
+  for (int h = 0; h < GROUP; ++h) { num[h] = make_float4(0.f, 0.f, 0.f, 0.f); den[h] = 0.f; }
+  for (int s0 = 0; s0 < p.nsplit; s0 += 4) {
+    float4 a[4][GROUP];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int h = 0; h < GROUP; ++h) {
+        const int64_t idx = ((int64_t)row * p.nsplit + s0 + u) * p.num_heads + head0 + h;
+        a[u][h] = s0 + u < p.nsplit ? __ldcg(reinterpret_cast<const float4*>(p.part_acc + idx * FA_HD) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
+    if (s0 == 0) {
+#pragma unroll
+      for (int h = 0; h < GROUP; ++h) top[h] = fa_exp2(top[h] - warp_max(top[h]));          // the splits' weights
     }
-    const float inv = den > 0.f ? 1.f / den : 0.f;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int h = 0; h < GROUP; ++h) {
+        const float w = __shfl_sync(0xffffffffu, top[h], (s0 + u) & 31), ls = __shfl_sync(0xffffffffu, sum[h], (s0 + u) & 31);
+        if (s0 + u < p.nsplit && ls > 0.f) {
+          num[h].x = fmaf(w, a[u][h].x, num[h].x); num[h].y = fmaf(w, a[u][h].y, num[h].y);
+          num[h].z = fmaf(w, a[u][h].z, num[h].z); num[h].w = fmaf(w, a[u][h].w, num[h].w);
+          den[h] = fmaf(w, ls, den[h]);
+        }
+      }
+  }
+#pragma unroll
+  for (int h = 0; h < GROUP; ++h) {
+    const float inv = den[h] > 0.f ? 1.f / den[h] : 0.f;
     uint2 o;
-    o.x = pack_bf16(num.x * inv, num.y * inv);
-    o.y = pack_bf16(num.z * inv, num.w * inv);
-    stg_v2(p.out + ((int64_t)row * p.num_heads + head) * FA_HD + 4 * lane, o);
+    o.x = pack_bf16(num[h].x * inv, num[h].y * inv);
+    o.y = pack_bf16(num[h].z * inv, num[h].w * inv);
+    stg_v2(p.out + ((int64_t)row * p.num_heads + head0 + h) * FA_HD + 4 * lane, o);
+  }
   }
 }
 
@@ -562,21 +598,22 @@ fused_decode_attn_small_kernel(const FusedAttnParams p, int rows) {
     }
   }
   __syncwarp();
-  float qv[GROUP][16];
+  uint64_t qv[GROUP][8];
 #pragma unroll
   for (int h = 0; h < GROUP; ++h) {
     const __nv_bfloat16* qp = q_s + h * FA_HD;
-    fa_unpack8(*reinterpret_cast<const uint4*>(qp + 8 * j), qv[h]);
-    fa_unpack8(*reinterpret_cast<const uint4*>(qp + 64 + 8 * j), qv[h] + 8);
+    fa_pairs8(*reinterpret_cast<const uint4*>(qp + 8 * j), qv[h]);
+    fa_pairs8(*reinterpret_cast<const uint4*>(qp + 64 + 8 * j), qv[h] + 4);
 #pragma unroll
-    for (int d = 0; d < 16; ++d) qv[h][d] *= p.scale_log2;
+    for (int d = 0; d < 8; ++d) qv[h][d] = f2_mul(qv[h][d], f2_pack(p.scale_log2, p.scale_log2));
   }
-  float m[GROUP], l[GROUP], acc[GROUP][16];
+  float m[GROUP], l[GROUP];
+  uint64_t acc2[GROUP][8];                                // weighted sums of values, in pairs
 #pragma unroll
   for (int h = 0; h < GROUP; ++h) {
     m[h] = -INFINITY; l[h] = 0.f;
 #pragma unroll
-    for (int d = 0; d < 16; ++d) acc[h][d] = 0.f;
+    for (int d = 0; d < 8; ++d) acc2[h][d] = 0;
   }
   for (int i0 = 0; i0 < n_tiles; i0 += 2) {
 #pragma unroll
@@ -591,23 +628,17 @@ fused_decode_attn_small_kernel(const FusedAttnParams p, int rows) {
         const int tok = it * 4 + g;
         const bool valid = tok < ntok;
         isnew[it] = tok0 + (valid ? tok : 0) == L - 1;
-        float kf[16];
+        uint64_t kf[8];
         if (isnew[it]) {
-          fa_unpack8(*reinterpret_cast<const uint4*>(kn_s + 8 * j), kf);
-          fa_unpack8(*reinterpret_cast<const uint4*>(kn_s + 64 + 8 * j), kf + 8);
+          fa_pairs8(*reinterpret_cast<const uint4*>(kn_s + 8 * j), kf);
+          fa_pairs8(*reinterpret_cast<const uint4*>(kn_s + 64 + 8 * j), kf + 4);
         } else {
-          fa_unpack8(kbuf[u][it][0], kf);
-          fa_unpack8(kbuf[u][it][1], kf + 8);
+          fa_pairs8(kbuf[u][it][0], kf);
+          fa_pairs8(kbuf[u][it][1], kf + 4);
         }
 #pragma unroll
         for (int h = 0; h < GROUP; ++h) {
-          float d0 = 0.f, d1 = 0.f;
-#pragma unroll
-          for (int d = 0; d < 16; d += 2) {
-            d0 = fmaf(qv[h][d], kf[d], d0);
-            d1 = fmaf(qv[h][d + 1], kf[d + 1], d1);
-          }
-          float dot = d0 + d1;
+          float dot = fa_dot16<true>(qv[h], kf);
           dot += __shfl_xor_sync(0xffffffffu, dot, 1);
           dot += __shfl_xor_sync(0xffffffffu, dot, 2);
           dot += __shfl_xor_sync(0xffffffffu, dot, 4);
@@ -633,28 +664,31 @@ fused_decode_attn_small_kernel(const FusedAttnParams p, int rows) {
         }
         l[h] = fmaf(l[h], alpha[h], ps);
 #pragma unroll
-        for (int d = 0; d < 16; ++d) acc[h][d] *= alpha[h];
+        for (int d = 0; d < 8; ++d) acc2[h][d] = f2_mul(acc2[h][d], f2_pack(alpha[h], alpha[h]));
       }
 #pragma unroll
       for (int it = 0; it < FA_TILE / 4; ++it) {
-        float vf[16];
+        uint64_t vf[8];
         if (isnew[it]) {
-          fa_unpack8(*reinterpret_cast<const uint4*>(vn_s + 8 * j), vf);
-          fa_unpack8(*reinterpret_cast<const uint4*>(vn_s + 64 + 8 * j), vf + 8);
+          fa_pairs8(*reinterpret_cast<const uint4*>(vn_s + 8 * j), vf);
+          fa_pairs8(*reinterpret_cast<const uint4*>(vn_s + 64 + 8 * j), vf + 4);
         } else {
-          fa_unpack8(vbuf[u][it][0], vf);
-          fa_unpack8(vbuf[u][it][1], vf + 8);
+          fa_pairs8(vbuf[u][it][0], vf);
+          fa_pairs8(vbuf[u][it][1], vf + 4);
         }
 #pragma unroll
         for (int h = 0; h < GROUP; ++h)
 #pragma unroll
-          for (int d = 0; d < 16; ++d) acc[h][d] = fmaf(s[it][h], vf[d], acc[h][d]);
+          for (int d = 0; d < 8; ++d) acc2[h][d] = f2_fma(f2_pack(s[it][h], s[it][h]), vf[d], acc2[h][d]);
       }
     }
     if (i0 + 2 < n_tiles) load_pair(i0 + 2);
   }
+  float acc[GROUP][16];
 #pragma unroll
   for (int h = 0; h < GROUP; ++h) {
+#pragma unroll
+    for (int d = 0; d < 8; ++d) f2_unpack(acc2[h][d], acc[h][2 * d], acc[h][2 * d + 1]);
     l[h] += __shfl_xor_sync(0xffffffffu, l[h], 8);
     l[h] += __shfl_xor_sync(0xffffffffu, l[h], 16);
 #pragma unroll
@@ -788,9 +822,12 @@ extern "C" int b2tts_fused_decode_attn(const void* q, int64_t q_row_stride, cons
     return B2TTS_OK;
   }
   void (*kern)(const FusedAttnParams) = nullptr;
-  if (group == 1) kern = eager ? fused_decode_attn_kernel<1, true> : fused_decode_attn_kernel<1, false>;
-  else if (group == 2) kern = eager ? fused_decode_attn_kernel<2, true> : fused_decode_attn_kernel<2, false>;
-  else if (group == 4) kern = eager ? fused_decode_attn_kernel<4, true> : fused_decode_attn_kernel<4, false>;
+#define FA_PICK(G) (p.nsplit == 1 ? (eager ? fused_decode_attn_kernel<G, true, false> : fused_decode_attn_kernel<G, false, false>) \
+                                  : (eager ? fused_decode_attn_kernel<G, true, true> : fused_decode_attn_kernel<G, false, true>))
+  if (group == 1) kern = FA_PICK(1);
+  else if (group == 2) kern = FA_PICK(2);
+  else if (group == 4) kern = FA_PICK(4);
+#undef FA_PICK
   B2_REQUIRE(kern, B2TTS_EUNSUPPORTED, "%s: GQA group %d unsupported (1, 2, 4)", what, group);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   if (e != cudaSuccess) return cuda_fail(e, what);
