@@ -1263,10 +1263,11 @@ def _coef(out, heads):
 
 
 # The longest portion from which what chunks say without the state is formed by a launch of its own.  That launch and its scratch cost the host 4 to 8 us; each
-# 64 tokens of the state space's chain give back 1 to 2, those of the delta rule 8, so that there two chunks are enough.  State space, layers of 1, 2, 4 and 8
+# 64 tokens of the state space's chain give back 1 to 2, those of the delta rule 8, so that there four chunks are enough.  State space, layers of 1, 2, 4 and 8
 # portions, in the chain / ahead of it in us: 192 tokens 70 75 87 160 / 75 78 85 149, 256 tokens 85 90 108 200 / 82 88 103 185.  Delta rule, the scan
-# of 1, 4 and 8 portions alone on the GPU: 100 tokens 34 38 70 / 29 31 54 (called one by one, host and all, 37.6 before and 37.7), 200 tokens 64 68 / 45 51.
-SSM_AHEAD_FROM, DELTA_AHEAD_FROM = 256, 65
+# of 1, 4 and 8 portions alone on the GPU: 100 tokens 34 38 70 / 29 31 54, 200 tokens 64 68 / 45 51; layers called one by one, host and all: 130 and 20 tokens
+# 72.9 / 75.5 to 77.0, 70 tokens 68.7 / 71.8 to 74.2, 200 tokens 80.0 / 73.1.
+SSM_AHEAD_FROM, DELTA_AHEAD_FROM = 256, 193
 
 
 def ssm_scan(xbc, dt_in, dt_bias, a_log, d_skip, state, out, lay, heads, groups, vdim, nstate, ahead=None):
