@@ -61,10 +61,20 @@ template <> struct Vec4<__nv_bfloat16> {
   }
   __device__ static void store(__nv_bfloat16* p, const float* f) { *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3])); }
 };
-// The same for a row whose values the block's threads still hold, four adjacent ones at a time (columns (threadIdx.x + it * ROW_THREADS) * 4 ..).
+// The same for a row whose values the block's threads still hold, four adjacent ones at a time (columns (threadIdx.x + it * ROW_THREADS) * 4 ..).  The squares are summed as
+// above - a thread has every ROW_THREADS-th column - so that h has the same bits whichever way a row is read: a root that differs in its last bit turns roundings of h, and
+// the layers behind multiply them.
 constexpr int ROW_KEEP = 4;                // rows of up to 4096
 template <typename T, int KEEP>
-__device__ __forceinline__ void gain_norm_kept(const float (&v)[KEEP][4], T* hr, int cols, float ssq, const float* gain, float eps, float* red) {
+__device__ __forceinline__ void gain_norm_kept(const float (&v)[KEEP][4], T* hr, int cols, const float* gain, float eps, float* red) {
+  __shared__ float4 row_s[KEEP * ROW_THREADS];
+#pragma unroll
+  for (int it = 0; it < KEEP; ++it) row_s[threadIdx.x + it * ROW_THREADS] = make_float4(v[it][0], v[it][1], v[it][2], v[it][3]);
+  __syncthreads();
+  const float* xs = reinterpret_cast<const float*>(row_s) + threadIdx.x;
+  float ssq = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4 * KEEP; ++i) if (static_cast<int>(threadIdx.x) + i * ROW_THREADS < cols) ssq += xs[i * ROW_THREADS] * xs[i * ROW_THREADS];
   const float tot = block_sum(ssq, red);
   const float inv = 1.0f / sqrtf(tot / static_cast<float>(cols) + eps);
   const float g = gain[0];
@@ -110,7 +120,7 @@ embed_pos_norm_vec4_kernel(const int32_t* __restrict__ tokens, const int32_t* __
   const int tok = min(max(tokens[row], 0), vocab - 1), p = min(max(positions[row], 0), max_pos - 1);
   const T *er = embed + static_cast<size_t>(tok) * cols, *pr = pos_table + static_cast<size_t>(p) * cols;
   float* xr = x + static_cast<size_t>(row) * cols;
-  float v[KEEP][4], ssq = 0.f;
+  float v[KEEP][4];
 #pragma unroll
   for (int it = 0; it < KEEP; ++it) {
     const int c = (threadIdx.x + it * ROW_THREADS) * 4;
@@ -120,10 +130,10 @@ embed_pos_norm_vec4_kernel(const int32_t* __restrict__ tokens, const int32_t* __
       Vec4<T>::load(pr + c, q);
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) { v[it][i] = e[i] + q[i]; ssq += v[it][i] * v[it][i]; }
+    for (int i = 0; i < 4; ++i) v[it][i] = e[i] + q[i];
     if (c < cols) Vec4<float>::store(xr + c, v[it]);
   }
-  if (h != nullptr) gain_norm_kept<T, KEEP>(v, h + static_cast<size_t>(row) * cols, cols, ssq, gain, eps, red);
+  if (h != nullptr) gain_norm_kept<T, KEEP>(v, h + static_cast<size_t>(row) * cols, cols, gain, eps, red);
 }
 
 // ------------------------------------------------------------------ residual update (+ next norm)
@@ -155,8 +165,9 @@ residual_norm_kernel(float* __restrict__ x, const T* __restrict__ a, const T* __
 }
 
 // The same for rows of up to 4096 columns, a multiple of four, in 8- and 16-byte pieces: all pieces of a thread are asked for before the first sum, and the new row
-// stays in registers until the norm is known.  Bound: HBM.  bf16 rows of 2048, one column at a time / now in us: 4138 rows 19.1 / 12.9 with a, 77 / 28 with four experts' z,
-// 8192 54 / 37 and 139 / 53, one row 4.3 / 3.0 and 9.4 / 3.4; embeddings of 4138 rows 20.9 / 11.9.  Registers for 4096 columns in every instance: 15.6, 45, 42, 88.
+// stays in registers until the norm is known.  Bound: HBM.  bf16 rows of 2048 that L2 does not hold, one column at a time / now in us: 4138 rows 30.5 / 20.3 with a, 79 / 35
+// with four experts' z, 8192 55 / 38 and 142 / 64, one row 3.4 / 2.2 and 7.7 / 2.8; embeddings of 4138 rows 30.8 / 17.1 (squares summed over a thread's own four columns, without
+// the way through shared memory: 19.9, 34, 37, 64, 2.1, 2.7 and 16.7, at other bits of the root).  Registers for 4096 columns in every instance cost 10 to 60 % more.
 template <typename T, int KEEP>
 __global__ void __launch_bounds__(ROW_THREADS)
 residual_norm_vec4_kernel(float* __restrict__ x, const T* __restrict__ a, const T* __restrict__ b, const T* __restrict__ z,
@@ -165,7 +176,7 @@ residual_norm_vec4_kernel(float* __restrict__ x, const T* __restrict__ a, const 
   __shared__ float red[33];
   const size_t row = blockIdx.x;
   float* xr = x + row * cols;
-  float v[KEEP][4], s[KEEP][4], ssq = 0.f;
+  float v[KEEP][4], s[KEEP][4];
 #pragma unroll
   for (int it = 0; it < KEEP; ++it) {
     const int c = (threadIdx.x + it * ROW_THREADS) * 4;
@@ -202,10 +213,10 @@ residual_norm_vec4_kernel(float* __restrict__ x, const T* __restrict__ a, const 
   for (int it = 0; it < KEEP; ++it) {
     const int c = (threadIdx.x + it * ROW_THREADS) * 4;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) { v[it][i] += mult * s[it][i]; ssq += v[it][i] * v[it][i]; }
+    for (int i = 0; i < 4; ++i) v[it][i] += mult * s[it][i];
     if (c < cols) Vec4<float>::store(xr + c, v[it]);
   }
-  if (h != nullptr) gain_norm_kept<T, KEEP>(v, h + row * cols, cols, ssq, gain, eps, red);
+  if (h != nullptr) gain_norm_kept<T, KEEP>(v, h + row * cols, cols, gain, eps, red);
 }
 
 // out[i] = gain norm of x[rows[i]] (the rows whose logits are wanted)

@@ -38,3 +38,30 @@ def test_against_64_bits(cols, dtype, off):
     x, h = put(torch.zeros(n, cols)), put(torch.zeros(n, cols, dtype=dtype))
     nat.embed_pos_norm(tok.to(DEV), pos.to(DEV), put(z), put(a), x, h, gain.to(DEV), eps)
     check(x, h, z.double()[tok.long()] + a.double()[pos.long()])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("cols", [4, 36, 1020, 1024, 1028, 2048, 2052, 4096])
+def test_the_same_bits_whichever_way_a_row_is_read(cols, dtype):
+    """An address that is no multiple of 16 bytes sends a row to the kernels of one column at a time: sums, squares and roots are those of four at a time."""
+    import nano_qwen3tts_vllm_b200._native as nat
+    g = torch.Generator().manual_seed(cols)
+    n, top, eps, gain = 300, 3, 1e-5, torch.tensor([1.3], device=DEV)
+    x0, zw = torch.randn(n, cols, generator=g), torch.rand(n, top, generator=g).to(DEV)
+    a, b, z = (torch.randn(m, cols, generator=g).to(dtype) for m in (n, n, n * top))
+    tok, pos = (torch.randint(0, n, (n,), generator=g, dtype=torch.int32).to(DEV) for _ in range(2))
+    got = []
+    for off in (0, 1):
+        def put(t):
+            buf = torch.empty(t.numel() + off, dtype=t.dtype, device=DEV)
+            buf[off:] = t.flatten().to(DEV)
+            return buf[off:].view(t.shape)
+        for use in [(1, 1, 1), (1, 0, 0), (0, 0, 1)]:
+            x, h = put(x0), put(torch.zeros(n, cols, dtype=dtype))
+            nat.residual_norm(x, put(a) if use[0] else None, put(b) if use[1] else None, put(z) if use[2] else None, zw if use[2] else None, 0.5, h, gain, eps, dtype)
+            got.append((off, x, h))
+        x, h = put(torch.zeros(n, cols)), put(torch.zeros(n, cols, dtype=dtype))
+        nat.embed_pos_norm(tok, pos, put(a), put(b), x, h, gain, eps)
+        got.append((off, x, h))
+    for (_, x, h), (_, y, k) in zip(got[:4], got[4:]):
+        assert torch.equal(x, y) and torch.equal(h, k)
