@@ -1,32 +1,31 @@
 // elementwise.cu - a6 SiLU / SiLU*mul, a9 row gathers and the frame-loop codebook embedding sum.
 // Streaming 16-byte vector passes; grids are sized to cover the data once (no reuse to tile for).
+#include "piece_walk.cuh"
 #include "row_ops.cuh"
 
 namespace b2 {
 
-// A thread keeps a 16-byte piece of the columns and walks rows gridDim.x apart, two at a time; SiLU by the approximate reciprocal (its argument is between 1 and 2).
-// Bound: HBM and, close behind, the activation's instructions.  5627 rows of 6144: 47.2 -> 34.6 us (31 at the copy rate; an exact
-// quotient for every value and a 64-bit division for every piece before), 8192 of 3072 34.1 -> 25.5.
+// Threads walk the 16-byte pieces of all rows, two of them at a time (piece_walk.cuh).  Bound: HBM and, close behind, the activation's instructions.  A block
+// for a part of a row's pieces had one busy lane in 32 for rows of 8 columns (200000 rows 53.6 us, now 3.8), counted rows near 2^31 in 32 bits and took no more than 65535 blocks of columns.
 template <bool EAGER, bool MUL>
 __global__ void __launch_bounds__(256)
 silu_mul_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ up, int64_t in_stride,
-                __nv_bfloat16* __restrict__ out, int rows, int inter) {
-  const int v = blockIdx.y * blockDim.x + threadIdx.x;
-  if (v >= inter >> 3) return;
-  for (int r = blockIdx.x; r < rows; r += 2 * gridDim.x) {
-    const int both[2] = {r, r + static_cast<int>(gridDim.x)};
+                __nv_bfloat16* __restrict__ out, int rows, int pieces, PieceStep step) {
+  PieceWalk w = piece_at(blockIdx.x * 256 + threadIdx.x, pieces);
+  while (w.row < rows) {
+    const PieceWalk both[2] = {w, piece_next(w, step, pieces)};
     uint4 g[2], u[2];
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
       g[k] = u[k] = make_uint4(0, 0, 0, 0);
-      if (both[k] < rows) {
-        g[k] = ldg_nc_v4(gate + (int64_t)both[k] * in_stride + 8 * v);
-        if (MUL) u[k] = ldg_nc_v4(up + (int64_t)both[k] * in_stride + 8 * v);
+      if (both[k].row < rows) {
+        g[k] = ldg_nc_v4(gate + both[k].row * in_stride + 8 * both[k].piece);
+        if (MUL) u[k] = ldg_nc_v4(up + both[k].row * in_stride + 8 * both[k].piece);
       }
     }
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      if (both[k] >= rows) break;
+      if (both[k].row >= rows) break;
       const uint32_t gw[4] = {g[k].x, g[k].y, g[k].z, g[k].w};
       const uint32_t uw[4] = {u[k].x, u[k].y, u[k].z, u[k].w};
       uint32_t ow[4];
@@ -40,8 +39,9 @@ silu_mul_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __r
         }
         ow[e] = pack_bf16(a, b);
       }
-      stg_v4(out + (int64_t)both[k] * inter + 8 * v, make_uint4(ow[0], ow[1], ow[2], ow[3]));
+      stg_v4(out + 8 * (both[k].row * pieces + both[k].piece), make_uint4(ow[0], ow[1], ow[2], ow[3]));
     }
+    w = piece_next(both[1], step, pieces);
   }
 }
 
@@ -106,16 +106,18 @@ extern "C" int b2tts_silu_and_mul(const void* gate, const void* up, int64_t in_r
   B2_REQUIRE(inter % 8 == 0 && in_row_stride % 8 == 0 && aligned16(gate) && aligned16(up) && aligned16(out),
              B2TTS_EALIGN, "silu_and_mul: inter/stride must be multiples of 8 and pointers 16-byte aligned");
   B2_REQUIRE(rounding == B2TTS_ROUND_EAGER || rounding == B2TTS_ROUND_FUSED, B2TTS_EINVAL, "silu_and_mul: rounding %d", rounding);
-  const int nvec = inter >> 3, threads = nvec < 256 ? (nvec + 31) / 32 * 32 : 256, chunks = (nvec + threads - 1) / threads;
-  const int pairs = rows / 2 + rows % 2, cap = (sm_count() * 16 + chunks - 1) / chunks;
-  const dim3 blocks(pairs < cap ? pairs : cap, chunks);
+  const int pieces = inter >> 3;
+  // one piece a thread up to a wave of threads, pairs of them beyond it
+  const int64_t all = static_cast<int64_t>(rows) * pieces, wave = static_cast<int64_t>(sm_count()) * 2048, turns = all <= wave ? (all + 255) / 256 : (all + 511) / 512;
+  const int cap = sm_count() * 16, blocks = turns < cap ? static_cast<int>(turns) : cap;
+  const PieceStep step = piece_step(blocks * 256u, pieces);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   auto g = static_cast<const __nv_bfloat16*>(gate);
   auto u = static_cast<const __nv_bfloat16*>(up);
   auto o = static_cast<__nv_bfloat16*>(out);
-  if (!up) silu_mul_kernel<true, false><<<blocks, threads, 0, st>>>(g, u, in_row_stride, o, rows, inter);
-  else if (rounding == B2TTS_ROUND_EAGER) silu_mul_kernel<true, true><<<blocks, threads, 0, st>>>(g, u, in_row_stride, o, rows, inter);
-  else silu_mul_kernel<false, true><<<blocks, threads, 0, st>>>(g, u, in_row_stride, o, rows, inter);
+  if (!up) silu_mul_kernel<true, false><<<blocks, 256, 0, st>>>(g, u, in_row_stride, o, rows, pieces, step);
+  else if (rounding == B2TTS_ROUND_EAGER) silu_mul_kernel<true, true><<<blocks, 256, 0, st>>>(g, u, in_row_stride, o, rows, pieces, step);
+  else silu_mul_kernel<false, true><<<blocks, 256, 0, st>>>(g, u, in_row_stride, o, rows, pieces, step);
   B2_CHECK_LAUNCH("silu_and_mul");
   return B2TTS_OK;
 }
