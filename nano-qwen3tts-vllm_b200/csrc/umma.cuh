@@ -132,7 +132,7 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* t
       :: "r"(smem_u32(smem_dst)), "l"(tmap), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2) : "memory");
 }
 
-__device__ __forceinline__ float gsilu_f(float g) { return g / (1.0f + expf(-g)); }   // as elementwise.cu
+__device__ __forceinline__ float gsilu_f(float g) { return g / (1.0f + expf(-g)); }   // silu_mul_kernel has the same bits for every gate of bf16
 // z/2 (1 + tanh(sqrt(2/pi) (z + 0.044715 z^3)))
 __device__ __forceinline__ float gelu_tanh_f(float z) {
   return 0.5f * z * (1.0f + tanhf(0.7978845608f * (z + 0.044715f * z * z * z)));

@@ -1,5 +1,5 @@
 """SiLU and SiLU products over all rows' pieces: rows of one piece, rows that no block fits, calls of one turn, of several and of an odd number of pieces a thread, strided
-rows, against 64 bits."""
+rows, against 64 bits; and every gate that bf16 has."""
 import pytest
 import torch
 
@@ -33,3 +33,27 @@ def test_against_64_bits(inter, rows, mode):
         # float arithmetic in front is a few units of 2^-24
         tol = (2 ** -8 if mode in ("alone", "fused") else 2 ** -7) + 2 ** -15
         assert bool(((got[s].double() - want).abs() <= tol * want.abs() + 1e-38).all())
+
+
+def test_every_gate():
+    """All bf16 values: the quotient g / (1 + e^-g) of floats, rounded once, as the epilogues of the products form it."""
+    import nano_qwen3tts_vllm_b200._native as nat
+    g = torch.arange(65536, dtype=torch.int32, device=DEV).to(torch.int16).view(BF).view(512, 128)
+    one, up = torch.ones_like(g), torch.full_like(g, 1.2421875)
+    f = g.float() / (1 + torch.exp(-g.float()))
+    same = lambda x, y: torch.equal(x.isnan(), y.isnan()) and torch.equal(x[~x.isnan()], y[~y.isnan()])
+    assert same(nat.silu_and_mul(g, None), f.to(BF))
+    assert same(nat.silu_and_mul(g, one), f.to(BF))
+    assert same(nat.silu_and_mul(g, up), f.to(BF) * up)
+    assert same(nat.silu_and_mul(g, up, rounding=nat.ROUND_FUSED), (f * up.float()).to(BF))
+
+
+def test_fused_products_of_every_gate():
+    """With fused rounding the SiLU meets the other factor as a float: factors that leave the rounding of the product to its last bits."""
+    import nano_qwen3tts_vllm_b200._native as nat
+    g = torch.arange(65536, dtype=torch.int32, device=DEV).to(torch.int16).view(BF).view(512, 128)
+    f = g.float() / (1 + torch.exp(-g.float()))
+    for up in (1.0078125, 1.109375, 0.703125, 1.9921875, 3.015625e-3):
+        u = torch.full_like(g, up)
+        got, want = nat.silu_and_mul(g, u, rounding=nat.ROUND_FUSED), (f * u.float()).to(BF)
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got[~got.isnan()], want[~want.isnan()])
