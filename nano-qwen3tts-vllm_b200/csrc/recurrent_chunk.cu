@@ -516,9 +516,10 @@ linear_chunk_kernel(const ScanArgs a, int64_t chunks) {
 // launches 467 -> 366 us, one sequence of 300 tokens 83 -> 66, of 100 tokens 38 -> 38 (GPU 32 -> 29).  Where there is no room for what is formed ahead, the
 // chain forms it at 15500 cycles a chunk: 4 x 2048 tokens 492 -> 530 us, 16 x 40 63 -> 65.
 //
-// Errors against 64 bits over 512 tokens (means of 24 inputs of three sizes, outputs / state, before -> now): 128 channels 1.054e-7 / 9.15e-8 -> 1.052e-7 /
-// 9.19e-8, 64 channels 0.998e-7 / 9.35e-8 -> 0.995e-7 / 9.37e-8, keys that point half the same way 1.166e-7 / 9.18e-8 -> 1.175e-7 / 9.37e-8; token by token
-// 1.14e-7 / 1.05e-7.
+// Errors against 64 bits over 512 tokens (means of 48 inputs of three sizes, outputs / state; a substitution of floats in the chain, the rows of u rounded to floats, now):
+// 128 channels 1.051e-7 / 9.21e-8, 1.049e-7 / 9.23e-8, 1.023e-7 / 8.89e-8; 64 channels 0.998e-7 / 9.21e-8, 0.996e-7 / 9.22e-8, 0.967e-7 / 8.85e-8; keys that point half the
+// same way 1.164e-7 / 9.22e-8, 1.171e-7 / 9.37e-8, 1.136e-7 / 8.90e-8; most of it 1.284e-7 / 9.62e-8, 1.303e-7 / 1.003e-7, 1.257e-7 / 9.34e-8; token by token 1.14e-7 /
+// 1.05e-7.  What is cut off u costs 14 of 369 us (4 ragged sequences, all launches); what the write scales' products cut off would take 3 % of the states' errors for 3 us more.
 // mma_add with what the tensor core cut off its sum (it keeps two bits behind a float's): the same product on top of minus the sum
 __device__ __forceinline__ void mma_add_rest(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
   float t[4] = {0.f, 0.f, 0.f, 0.f};
@@ -802,7 +803,7 @@ delta_prepare_kernel(const ScanArgs a) {
 template <int D, bool AHEAD> struct DeltaTiles {
   __nv_bfloat16 q[2][CK_L * D], k[2][CK_L * D], v[2][CK_L * CK_P];
   DeltaPrep prep[AHEAD ? 2 : 1];
-  float4 part[8][8][32];                    // [warp][8 tokens]: S^T k over the warp's channels; u of its blocks lies over it
+  float4 part[8][8][32];                    // [warp][8 tokens]: S^T k over the warp's channels; u of its blocks and what was cut off it lie over it
   float4 other[8][4][32];                   // [warp]: S^T q of the partner's blocks
   union {
     float red[2][2][2][CK_P];               // token by token: [parity][k or q][half][value column]
@@ -812,10 +813,9 @@ template <int D, bool AHEAD> struct DeltaTiles {
 
 __device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
 
-// c -= x n (SUBTRACT) or c += x n over the blocks jb <= ib of row block ib: x in three parts per column block, n the fragments of a row of blocks
-template <bool SUBTRACT>
-__device__ __forceinline__ void delta_row_product(float c[2][4], const uint32_t x[4][3][4], const uint4 (*n)[3][32], int ib, int lane) {
-  float small[2][4], mid[2][4], big[2][4];
+// t = x n over the blocks jb <= ib of row block ib: x in three parts per column block, n the fragments of a row of blocks; t = small + big
+__device__ __forceinline__ void delta_row_product(float small[2][4], float big[2][4], const uint32_t x[4][3][4], const uint4 (*n)[3][32], int ib, int lane) {
+  float mid[2][4];
 #pragma unroll
   for (int w = 0; w < 2; ++w)
 #pragma unroll
@@ -840,9 +840,35 @@ __device__ __forceinline__ void delta_row_product(float c[2][4], const uint32_t 
 #pragma unroll
   for (int w = 0; w < 2; ++w)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float t = (small[w][e] + mid[w][e]) + big[w][e];
-      c[w][e] = SUBTRACT ? c[w][e] - t : c[w][e] + t;
+    for (int e = 0; e < 4; ++e) small[w][e] += mid[w][e];
+}
+// c += x n
+__device__ __forceinline__ void delta_add_row(float c[2][4], const uint32_t x[4][3][4], const uint4 (*n)[3][32], int ib, int lane) {
+  float small[2][4], big[2][4];
+  delta_row_product(small, big, x, n, ib, lane);
+#pragma unroll
+  for (int w = 0; w < 2; ++w)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) c[w][e] += small[w][e] + big[w][e];
+}
+// c -= x n; rest: what the two roundings of that cut off, which joins the last parts of c where it enters products (bf16 as they are, with bits to spare).  Rounded to
+// floats, each with an error of its own, the rows of u left states up to 4 % further from 64 bits than a substitution, whose rows take up the errors of those in front.
+__device__ __forceinline__ void delta_take_row(float c[2][4], uint32_t rest[2][2], const uint32_t x[4][3][4], const uint4 (*n)[3][32], int ib, int lane) {
+  float small[2][4], big[2][4];
+  delta_row_product(small, big, x, n, ib, lane);
+#pragma unroll
+  for (int w = 0; w < 2; ++w)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float cut[2];
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        float& y = c[w][2 * h + x];
+        const float sm = small[w][2 * h + x], bg = big[w][2 * h + x], t = sm + bg, u = y - t, v = u - y;
+        cut[x] = ((y - (u - v)) - (t + v)) - (sm - (t - bg));
+        y = u;
+      }
+      rest[w][h] = pack_bf16(cut[0], cut[1]);
     }
 }
 
@@ -1019,7 +1045,7 @@ delta_chunk_kernel(const ScanArgs a) {
     }
     pair_sync(1 + wp);
     // ---- what the chunk has to write before its tokens see one another
-    float r[8][4];
+    float r[8][4];                                         // r, then u
     {
       uint32_t vf[4][4];
 #pragma unroll
@@ -1035,20 +1061,24 @@ delta_chunk_kernel(const ScanArgs a) {
     }
     // ---- u = r - N r, this warp's two token blocks
     uint32_t xf[4][3][4];
-    auto split_all = [&]() {
+    auto split_all = [&](auto rest) {
 #pragma unroll
-      for (int js = 0; js < 4; ++js)
+      for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-          split3(r[2 * js + (e >> 1)][2 * (e & 1)], r[2 * js + (e >> 1)][2 * (e & 1) + 1], xf[js][0][e], xf[js][1][e], xf[js][2][e]);
+        for (int h = 0; h < 2; ++h) {
+          const int e = 2 * (nt & 1) + h;
+          split3(r[nt][2 * h], r[nt][2 * h + 1], xf[nt >> 1][0][e], xf[nt >> 1][1][e], xf[nt >> 1][2][e]);
+          rest(nt, h, xf[nt >> 1][2][e]);
+        }
     };
-    split_all();
+    split_all([](int, int, uint32_t&) {});
+    uint32_t rest[4][2] = {};                              // what was cut off u
     if (wh == 0) {
-      delta_row_product<true>(r + 0, xf, pre.n, 0, lane);
-      if (48 < L) delta_row_product<true>(r + 6, xf, pre.n, 3, lane);
+      delta_take_row(r + 0, rest + 0, xf, pre.n, 0, lane);
+      if (48 < L) delta_take_row(r + 6, rest + 2, xf, pre.n, 3, lane);
     } else {
-      if (16 < L) delta_row_product<true>(r + 2, xf, pre.n, 1, lane);
-      if (32 < L) delta_row_product<true>(r + 4, xf, pre.n, 2, lane);
+      if (16 < L) delta_take_row(r + 2, rest + 0, xf, pre.n, 1, lane);
+      if (32 < L) delta_take_row(r + 4, rest + 2, xf, pre.n, 2, lane);
     }
     pair_sync(1 + wp);                                     // both have read the sums that u takes the place of
 #pragma unroll
@@ -1056,6 +1086,9 @@ delta_chunk_kernel(const ScanArgs a) {
       const float* y = wh ? r[2 + x] : r[x < 2 ? x : 4 + x];
       sm.part[warp][x][lane] = make_float4(y[0], y[1], y[2], y[3]);
     }
+    uint4* cut_s = reinterpret_cast<uint4*>(sm.part[warp][4]);
+    cut_s[lane] = make_uint4(rest[0][0], rest[0][1], rest[1][0], rest[1][1]);
+    cut_s[32 + lane] = make_uint4(rest[2][0], rest[2][1], rest[3][0], rest[3][1]);
     pair_sync(1 + wp);
 #pragma unroll
     for (int x = 0; x < 4; ++x) {
@@ -1063,7 +1096,13 @@ delta_chunk_kernel(const ScanArgs a) {
       float* z = wh ? r[x < 2 ? x : 4 + x] : r[2 + x];
       z[0] = y.x; z[1] = y.y; z[2] = y.z; z[3] = y.w;
     }
-    split_all();
+    // what was cut off u for eight tokens (row h of the lane's two), by the warp of the pair that formed it
+    auto cut_off = [&](int nt, int h) {
+      const bool second = nt >= 2 && nt < 6;
+      const int x = second ? nt - 2 : nt < 2 ? nt : nt - 4;
+      return reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint4*>(sm.part[second ? wp + 4 : wp][4]) + (x >> 1) * 32 + lane)[2 * (x & 1) + h];
+    };
+    split_all([&](int nt, int h, uint32_t& lo) { lo = add_bf16x2(lo, cut_off(nt, h)); });
     // ---- the outputs of this warp's blocks
     {
       auto finish = [&](int ib, float* const c0, float* const c1) {
@@ -1075,7 +1114,7 @@ delta_chunk_kernel(const ScanArgs a) {
           const float2 eq = *reinterpret_cast<const float2*>(pre.eq + ib * 16 + w * 8 + c2);
           c[w][0] = (y[0] + x.x) * eq.x; c[w][1] = (y[1] + x.y) * eq.y; c[w][2] = (y[2] + x.z) * eq.x; c[w][3] = (y[3] + x.w) * eq.y;
         }
-        delta_row_product<false>(c, xf, pre.m, ib, lane);
+        delta_add_row(c, xf, pre.m, ib, lane);
 #pragma unroll
         for (int w = 0; w < 2; ++w)
 #pragma unroll
@@ -1094,12 +1133,18 @@ delta_chunk_kernel(const ScanArgs a) {
     }
     // ---- the state behind the chunk, this half of the channels: what the chunk adds is summed by itself, then S <- e^(c_L) S + sum
     {
+      uint32_t off[8][2];
 #pragma unroll
       for (int nt = 0; nt < 8; ++nt) {
         const float2 wk = *reinterpret_cast<const float2*>(pre.wk + nt * 8 + c2);
-        r[nt][0] *= wk.x; r[nt][1] *= wk.y; r[nt][2] *= wk.x; r[nt][3] *= wk.y;
+        const uint32_t w2 = pack_bf16(wk.x, wk.y);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          r[nt][2 * h] *= wk.x; r[nt][2 * h + 1] *= wk.y;
+          off[nt][h] = mul_bf16x2(cut_off(nt, h), w2);
+        }
       }
-      split_all();
+      split_all([&](int nt, int h, uint32_t& lo) { lo = add_bf16x2(lo, off[nt][h]); });
       const float gl = pre.ecum[CK_L - 1];
 #pragma unroll
       for (int np = 0; np < CH / 16; ++np) {
