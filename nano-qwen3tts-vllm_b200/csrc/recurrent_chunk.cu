@@ -520,16 +520,6 @@ linear_chunk_kernel(const ScanArgs a, int64_t chunks) {
 // 128 channels 1.051e-7 / 9.21e-8, 1.049e-7 / 9.23e-8, 1.023e-7 / 8.89e-8; 64 channels 0.998e-7 / 9.21e-8, 0.996e-7 / 9.22e-8, 0.967e-7 / 8.85e-8; keys that point half the
 // same way 1.164e-7 / 9.22e-8, 1.171e-7 / 9.37e-8, 1.136e-7 / 8.90e-8; most of it 1.284e-7 / 9.62e-8, 1.303e-7 / 1.003e-7, 1.257e-7 / 9.34e-8; token by token 1.14e-7 /
 // 1.05e-7.  What is cut off u costs 14 of 369 us (4 ragged sequences, all launches); what the write scales' products cut off would take 3 % of the states' errors for 3 us more.
-// mma_add with what the tensor core cut off its sum (it keeps two bits behind a float's): the same product on top of minus the sum
-__device__ __forceinline__ void mma_add_rest(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
-  float t[4] = {0.f, 0.f, 0.f, 0.f};
-  mma_bf16_16816(t, a, b0, b1);
-  float r[4] = {-t[0], -t[1], -t[2], -t[3]};
-  mma_bf16_16816(r, a, b0, b1);
-#pragma unroll
-  for (int e = 0; e < 4; ++e) c[e] = (c[e] + r[e]) + t[e];
-}
-
 constexpr int CK_FS = CK_L + 4;             // padded float rows: a warp's quads fall into distinct banks
 constexpr int CK_DELTA_THREADS = 256;
 
@@ -546,11 +536,25 @@ static_assert(sizeof(DeltaPrep) % 16 == 0, "copied in 16-byte pieces");
 constexpr int CK_DELTA_PREP = sizeof(DeltaPrep) / 4;
 
 struct DeltaWork {                          // scratch of delta_prepare()
-  float A[CK_L * CK_FS], E[CK_L * CK_FS];   // E: e^(c_i - c_j), j <= i; then N
-  double cum[CK_L];
+  float A[CK_L * CK_FS], E[CK_L * CK_FS];   // A, then N in its blocks on the diagonal; E: e^(c_i - c_j), j <= i, then N below them
+  __align__(16) float2 cum[CK_L];           // sums of the log decays: a float and what it leaves
   float beta[CK_L], kn[CK_L], qn[CK_L];
   int wild;
 };
+
+__device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+
+// Decays and write factors of a chunk, two tokens a lane (zeros behind the portion's end)
+struct DeltaCoef { float l[2], b[2]; };
+__device__ __forceinline__ DeltaCoef delta_coef(const float* cp, int H, int t0, int len, int lane) {
+  DeltaCoef c = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int t = t0 + 2 * lane + e;
+    if (t < len) { c.b[e] = cp[static_cast<size_t>(t) * H * 3 + 1]; c.l[e] = cp[static_cast<size_t>(t) * H * 3 + 2]; }
+  }
+  return c;
+}
 
 // The 16 x 16 blocks of the dot products, rows rblk and columns cblk, that warp (wp, wh) has: three for even wp, two for odd ones
 __device__ __forceinline__ void delta_block(int wp, int n, int& rblk, int& cblk) {
@@ -558,26 +562,38 @@ __device__ __forceinline__ void delta_block(int wp, int n, int& rblk, int& cblk)
   rblk = extra ? 0 : wp == 0 ? 3 : wp == 1 ? 3 : wp == 2 ? 2 : 1;
   cblk = extra ? 0 : (wp == 1 ? 2 : 0) + n;
 }
+// All of them at once: products of one step of 16 channels for every block, so that none waits for another.  Warps that have two form the second one twice: a branch
+// for every step costs more.
 template <int D>
-__device__ __forceinline__ void delta_block_dots(uint32_t x_u, uint32_t k_u, int rblk, int cblk, int lane, float sc[2][4]) {
+__device__ __forceinline__ void delta_block_dots(uint32_t x_u, uint32_t k_u, int wp, int lane, float sc[3][2][4]) {
   constexpr int RB = D * 2;
   const int ra = lane & 15, ca = lane >> 4, rb = (lane >> 4) * 8 + (lane & 7), cb = (lane >> 3) & 1;
+  int rblk[3], cblk[3];
 #pragma unroll
-  for (int w = 0; w < 2; ++w)
+  for (int n = 0; n < 3; ++n) {
+    delta_block(wp, (wp & 1) && n == 2 ? 1 : n, rblk[n], cblk[n]);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) sc[w][e] = 0.f;
-  uint32_t af[D / 16][4], bf[D / 16][4];
+    for (int w = 0; w < 2; ++w)
 #pragma unroll
-  for (int ks = 0; ks < D / 16; ++ks) {
-    ldsm4(af[ks], x_u + tile_off(rblk * 16 + ra, ks * 2 + ca, RB));
-    ldsm4(bf[ks], k_u + tile_off(cblk * 16 + rb, ks * 2 + cb, RB));
+      for (int e = 0; e < 4; ++e) sc[n][w][e] = 0.f;
   }
 #pragma unroll
   for (int ks = 0; ks < D / 16; ++ks) {
-    mma_add(sc[0], af[ks], bf[ks][0], bf[ks][1]);
-    mma_add(sc[1], af[ks], bf[ks][2], bf[ks][3]);
+    uint32_t af[2][4], bf[3][4];
+    ldsm4(af[0], x_u + tile_off(rblk[0] * 16 + ra, ks * 2 + ca, RB));       // the first two have the same rows
+    ldsm4(af[1], x_u + tile_off(rblk[2] * 16 + ra, ks * 2 + ca, RB));
+#pragma unroll
+    for (int n = 0; n < 3; ++n) ldsm4(bf[n], k_u + tile_off(cblk[n] * 16 + rb, ks * 2 + cb, RB));
+#pragma unroll
+    for (int n = 0; n < 3; ++n) {
+      mma_add(sc[n][0], af[n >> 1], bf[n][0], bf[n][1]);
+      mma_add(sc[n][1], af[n >> 1], bf[n][2], bf[n][3]);
+    }
   }
 }
+// The double of a bf16, by its bits (a conversion takes eight times as long as the addition behind it): right for all normal numbers; zero and what is below 2^-126 come out as
+// less than 2^-126.
+__device__ __forceinline__ double bf16_double(uint32_t x) { return __hiloint2double(((x & 0x7fffu) << 13) + (896 << 20), 0); }
 // 1 / |row| (times the scale for queries) of row tid / 2 of the keys, then of the queries, on the even one of two threads; the largest
 // magnitude of what the thread has seen
 template <int D>
@@ -585,42 +601,55 @@ __device__ __forceinline__ float delta_row_norm(const __nv_bfloat16* k, const __
   constexpr int RB = D * 2;
   const int r = tid >> 1;
   const unsigned char* row = reinterpret_cast<const unsigned char*>(r < CK_L ? k : q);
+  auto piece = [&](int c) { return *reinterpret_cast<const uint4*>(row + tile_off(r & (CK_L - 1), c * 2 + (tid & 1), RB)); };
   double part[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
   for (int c = 0; c < D / 16; ++c) {
-    const uint4 x = *reinterpret_cast<const uint4*>(row + tile_off(r & (CK_L - 1), c * 2 + (tid & 1), RB));
+    const uint4 x = piece(c);
     m = mag2(mag2(mag2(mag2(m, x.x), x.y), x.z), x.w);
     const uint32_t w[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const float f0 = bf16lo(w[e]), f1 = bf16hi(w[e]);
-      part[e] += static_cast<double>(f0 * f0);             // exact: 16 significant bits
-      part[e] += static_cast<double>(f1 * f1);
+      const double f0 = bf16_double(w[e]), f1 = bf16_double(w[e] >> 16);
+      part[e] = fma(f0, f0, part[e]);                      // exact squares: 16 significant bits
+      part[e] = fma(f1, f1, part[e]);
     }
   }
   double ss = (part[0] + part[1]) + (part[2] + part[3]);
   ss += __shfl_xor_sync(0xffffffffu, ss, 1);
-  return static_cast<float>((r < CK_L ? 1.0 : static_cast<double>(qscale)) / sqrt(ss + 1e-6));
+  const uint32_t both = __vmaxu2(m, __shfl_xor_sync(0xffffffffu, m, 1));
+  if (max(both & 0xffffu, both >> 16) >= CK_BIG_IN) {      // infinities and what overflows a float's square reach the token-by-token sums as they always did
+    ss = 0.0;
+    for (int c = 0; c < D / 16; ++c) {
+      const uint4 x = piece(c);
+      const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        ss += static_cast<double>(bf16lo(w[e]) * bf16lo(w[e]));
+        ss += static_cast<double>(bf16hi(w[e]) * bf16hi(w[e]));
+      }
+    }
+    ss += __shfl_xor_sync(3u << (tid & 30), ss, 1);
+    return static_cast<float>((r < CK_L ? 1.0 : static_cast<double>(qscale)) / sqrt(ss + 1e-6));
+  }
+  // the root's reciprocal to 2^-43: a float's and one Newton step
+  ss += 1e-6;
+  const double y = rsqrtf(static_cast<float>(ss)), z = fma(0.5 * y, fma(-ss * y, y, 1.0), y);
+  return static_cast<float>(r < CK_L ? z : qscale * z);
 }
 
 // All 256 threads; keys and queries of the chunk that starts at token t0 in shared memory.  Ends without a barrier.
 //
-// N in blocks of 16: those on the diagonal by substitution (column c of (1 + A)^-1 solves the system for the unit vector c; four lanes have a column, four
-// rows at a time are exchanged, solved by all four lanes and subtracted from the rows behind), those below from them by products.  64 rows of substitution in a row
-// took 7500 cycles of a chunk, this 3000.  Sums are formed beside the rows: a row is rounded once at its own size and not up to 64 times.
+// N in blocks of 16: those on the diagonal by substitution (column c of (1 + A)^-1 solves the system for the unit vector c), those below from them by
+// products, 64 threads a block with four neighbouring sums each.  Sums are formed beside the rows: a row is rounded once at its own size and not up to 64 times.
 template <int D>
-__device__ __forceinline__ void delta_prepare(const ScanArgs& a, const __nv_bfloat16* q_s, const __nv_bfloat16* k_s, const float* cp, int t0, int len,
-                                              DeltaWork& w, DeltaPrep& p) {
+__device__ __forceinline__ void delta_prepare(const ScanArgs& a, const __nv_bfloat16* q_s, const __nv_bfloat16* k_s, DeltaCoef coef, int L, DeltaWork& w, DeltaPrep& p) {
+  const int blocks = (L + 15) >> 4;                        // rows of blocks that the portion reaches: nobody asks for those behind them
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wp = warp & 3, wh = warp >> 2, g4 = lane >> 2, c2 = 2 * (lane & 3);
   if (tid == 0) w.wild = 0;
   float ecum[2], wl[2];
   if (warp == 0) {                                         // lane l: tokens 2 l, 2 l + 1
-    float l[2] = {0.f, 0.f}, b[2] = {0.f, 0.f};
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int t = t0 + 2 * lane + e;
-      if (t < len) { b[e] = cp[static_cast<size_t>(t) * a.H * 3 + 1]; l[e] = cp[static_cast<size_t>(t) * a.H * 3 + 2]; }
-    }
+    float *l = coef.l, *b = coef.b;
     const bool fine = fabsf(l[0]) < 1e30f && fabsf(l[1]) < 1e30f && fabsf(b[0]) < 1e6f && fabsf(b[1]) < 1e6f;
     l[0] = cut_log(l[0]); l[1] = cut_log(l[1]);
     double c1 = static_cast<double>(l[0]) + l[1], x;
@@ -632,7 +661,8 @@ __device__ __forceinline__ void delta_prepare(const ScanArgs& a, const __nv_bflo
     double c0 = __shfl_up_sync(0xffffffffu, c1, 1);
     c0 = (lane == 0 ? 0.0 : c0) + l[0];
     const double ce = __shfl_sync(0xffffffffu, c1, 31);
-    w.cum[2 * lane] = c0; w.cum[2 * lane + 1] = c1;
+    const float h0 = static_cast<float>(c0), h1 = static_cast<float>(c1);
+    *reinterpret_cast<float4*>(w.cum + 2 * lane) = make_float4(h0, static_cast<float>(c0 - h0), h1, static_cast<float>(c1 - h1));
     w.beta[2 * lane] = b[0]; w.beta[2 * lane + 1] = b[1];
     ecum[0] = exp_sum(c0); ecum[1] = exp_sum(c1);
     wl[0] = exp_sum(ce - c0); wl[1] = exp_sum(ce - c1);
@@ -642,15 +672,11 @@ __device__ __forceinline__ void delta_prepare(const ScanArgs& a, const __nv_bflo
   const float nrm = delta_row_norm<D>(k_s, q_s, tid, a.qscale, m);
   if ((tid & 1) == 0) (tid < 2 * CK_L ? w.kn[tid >> 1] : w.qn[(tid >> 1) - CK_L]) = nrm;
   const int wild = __syncthreads_or((m & 0xffffu) >= CK_BIG_IN || (m >> 16) >= CK_BIG_IN);
-  // ---- decays between the chunk's tokens: rows x and 63 - x together have as many for every x
-  {
-    const int x = tid >> 3, sub = tid & 7;
-#pragma unroll 2
-    for (int n = 0; n < 2; ++n) {
-      const int i = n ? CK_L - 1 - x : x;
-      const double ci = w.cum[i];
-      for (int j = sub; j <= i; j += 8) w.E[i * CK_FS + j] = exp_sum(ci - w.cum[j]);
-    }
+  // ---- decays between the chunk's tokens: the 36 tiles of 8 x 8 up to the diagonal, nine for each 64 threads, none waiting for another
+#pragma unroll
+  for (int x = 0; x < 9; ++x) {
+    const int tile = ck_tile((tid >> 6) + 4 * x), i = (tile >> 3) * 8 + ((tid >> 3) & 7), j = (tile & 7) * 8 + (tid & 7);
+    if ((tile >> 4) < blocks) w.E[i * CK_FS + j] = exp_between(w.cum[i], w.cum[j]);
   }
   if (warp == 0) {
 #pragma unroll
@@ -665,13 +691,15 @@ __device__ __forceinline__ void delta_prepare(const ScanArgs& a, const __nv_bflo
   __syncthreads();
   // ---- dot products of the keys (wh 0) or the queries (wh 1) with the keys up to the diagonal, in 16 x 16 blocks
   const uint32_t k_u = smem_u32(k_s), x_u = wh ? smem_u32(q_s) : k_u;
+  float dots[3][2][4];
+  if ((wp == 0 ? 0 : wp == 1 ? 3 : wp == 2 ? 2 : 1) < blocks) delta_block_dots<D>(x_u, k_u, wp, lane, dots);
 #pragma unroll
   for (int nb = 0; nb < 3; ++nb) {
     if (nb == 2 && (wp & 1)) break;
     int rblk, cblk;
     delta_block(wp, nb, rblk, cblk);
-    float sc[2][4];
-    delta_block_dots<D>(x_u, k_u, rblk, cblk, lane, sc);
+    if (rblk >= blocks) continue;
+    const float (&sc)[2][4] = dots[nb];
     uint32_t part[3][4];
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
@@ -692,77 +720,79 @@ __device__ __forceinline__ void delta_prepare(const ScanArgs& a, const __nv_bflo
       for (int e = 0; e < 3; ++e) p.m[rblk * (rblk + 1) / 2 + cblk][e][lane] = make_uint4(part[e][0], part[e][1], part[e][2], part[e][3]);
     }
   }
-  __syncthreads();
-  // ---- N of the four 16 x 16 blocks on the diagonal: four lanes per column
-  {
-    const int sub = lane & 3, top = (warp >> 1) * 16, col = warp * 8 + g4;
-    const float* A = w.A + top * CK_FS + top;
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  // ---- N of the 16 x 16 blocks on the diagonal, a warp each, in place of A's; a lane has a column (the upper half of the lanes the same ones)
+  if (wh == 0) {
+    asm volatile("bar.sync 1, 128;" ::: "memory");         // A is there; the other four warps are still at M
+    if (warp < blocks) {
+      float* A = w.A + warp * 16 * (CK_FS + 1);
+      float n[16];
 #pragma unroll
-    for (int m0 = 0; m0 < 4; ++m0) {
-      const float* d = A + 4 * m0 * CK_FS + 4 * m0;        // the 4 x 4 block on the diagonal
-      const float d10 = d[CK_FS], d20 = d[2 * CK_FS], d21 = d[2 * CK_FS + 1], d30 = d[3 * CK_FS], d31 = d[3 * CK_FS + 1], d32 = d[3 * CK_FS + 2];
-      float as[4];
+      for (int i = 0; i < 16; ++i) n[i] = 0.f;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) as[e] = __shfl_sync(0xffffffffu, acc[m0], (lane & ~3) + e);
-      const int at = col - top - 4 * m0;                   // the unit vector's one
-      const float n0 = as[0], u0 = (at == 0 ? 1.f : 0.f) - n0;
-      const float n1 = fmaf(d10, u0, as[1]), u1 = (at == 1 ? 1.f : 0.f) - n1;
-      const float n2 = fmaf(d21, u1, fmaf(d20, u0, as[2])), u2 = (at == 2 ? 1.f : 0.f) - n2;
-      const float n3 = fmaf(d32, u2, fmaf(d31, u1, fmaf(d30, u0, as[3]))), u3 = (at == 3 ? 1.f : 0.f) - n3;
-      w.E[(top + 4 * m0 + sub) * CK_FS + col] = sub == 0 ? n0 : sub == 1 ? n1 : sub == 2 ? n2 : n3;
+      for (int j = 0; j < 16; ++j) {                       // row j is complete: n[j], and u = (the unit vector's entry) - n[j] for the rows behind
+        const float u = (j == (lane & 15) ? 1.f : 0.f) - n[j];
 #pragma unroll
-      for (int x = m0 + 1; x < 4; ++x) {
-        const float4 y = *reinterpret_cast<const float4*>(A + (4 * x + sub) * CK_FS + 4 * m0);
-        acc[x] = fmaf(y.w, u3, fmaf(y.z, u2, fmaf(y.y, u1, fmaf(y.x, u0, acc[x]))));
+        for (int i = j + 1; i < 16; ++i) n[i] = fmaf(A[i * CK_FS + j], u, n[i]);
       }
+      __syncwarp();
+      if (lane < 16)
+#pragma unroll
+        for (int i = 0; i < 16; ++i) A[i * CK_FS + lane] = n[i];
     }
   }
   __syncthreads();
   // ---- the blocks below, a diagonal of them at a time: X_ij = A_ij (1 - N_jj) - sum_(j < k < i) A_ik N_kj (kept in the mirrored block), N_ij = X_ij - N_ii X_ij
   {
-    const int row = tid >> 4, col = tid & 15;
-    auto product = [&](const float* x, const float* y) -> float {      // row of x times column of y
-      float s0 = 0.f, s1 = 0.f;
+    const int grp = tid >> 6, row = (tid >> 2) & 15, col = 4 * (tid & 3);
+    auto product = [&](const float* x, const float* y) -> float4 {     // row of x times four columns of y
+      float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
+      auto add = [](float4& s, float f, const float4& v) { s.x = fmaf(f, v.x, s.x); s.y = fmaf(f, v.y, s.y); s.z = fmaf(f, v.z, s.z); s.w = fmaf(f, v.w, s.w); };
+      auto line = [&](int t) { return *reinterpret_cast<const float4*>(y + t * CK_FS + col); };
 #pragma unroll
       for (int t = 0; t < 16; t += 4) {
         const float4 a4 = *reinterpret_cast<const float4*>(x + row * CK_FS + t);
-        s0 = fmaf(a4.x, y[t * CK_FS + col], s0);
-        s1 = fmaf(a4.y, y[(t + 1) * CK_FS + col], s1);
-        s0 = fmaf(a4.z, y[(t + 2) * CK_FS + col], s0);
-        s1 = fmaf(a4.w, y[(t + 3) * CK_FS + col], s1);
+        add(s0, a4.x, line(t));
+        add(s1, a4.y, line(t + 1));
+        add(s0, a4.z, line(t + 2));
+        add(s1, a4.w, line(t + 3));
       }
-      return s0 + s1;
+      return make_float4(s0.x + s1.x, s0.y + s1.y, s0.z + s1.z, s0.w + s1.w);
     };
     auto block = [](float* x, int i, int j) { return x + 16 * i * CK_FS + 16 * j; };
-#pragma unroll
+    auto at = [&](float* x) -> float4& { return *reinterpret_cast<float4*>(x + row * CK_FS + col); };
+    auto less = [](const float4& x, const float4& y) { return make_float4(x.x - y.x, x.y - y.y, x.z - y.z, x.w - y.w); };
+#pragma unroll 1
     for (int d = 1; d < 4; ++d) {
-#pragma unroll
-      for (int i = d; i < 4; ++i) {                        // unrolled: a diagonal's products overlap
-        const int j = i - d;
-        float s = product(block(w.A, i, j), block(w.E, j, j));
-#pragma unroll
-        for (int k = j + 1; k < i; ++k) s += product(block(w.A, i, k), block(w.E, k, j));
-        block(w.E, j, i)[row * CK_FS + col] = block(w.A, i, j)[row * CK_FS + col] - s;
-      }
-      __syncthreads();
-#pragma unroll
-      for (int i = d; i < 4; ++i) {
-        const int j = i - d;
-        block(w.E, i, j)[row * CK_FS + col] = block(w.E, j, i)[row * CK_FS + col] - product(block(w.E, i, i), block(w.E, j, i));
+      if (d >= blocks) break;
+      const int j = grp, i = grp + d;                      // the group's block of the diagonal
+      if (i < blocks) {
+        float4 s = product(block(w.A, i, j), block(w.A, j, j));
+#pragma unroll 1
+        for (int x = 1; x < d; ++x) {
+          const float4 y = product(block(w.A, i, j + x), block(w.E, j + x, j));
+          s.x += y.x; s.y += y.y; s.z += y.z; s.w += y.w;
+        }
+        const float4 x = less(at(block(w.A, i, j)), s);
+        at(block(w.E, j, i)) = x;
+        if (grp == 0) asm volatile("bar.sync 2, 64;" ::: "memory");      // two warps have a block; numbers as constants, of which a CTA then takes few
+        else if (grp == 1) asm volatile("bar.sync 3, 64;" ::: "memory");
+        else asm volatile("bar.sync 4, 64;" ::: "memory");
+        at(block(w.E, i, j)) = less(x, product(block(w.A, i, i), block(w.E, j, i)));
       }
       __syncthreads();
     }
   }
   for (int blk = warp; blk < 10; blk += 8) {
     const int ib = blk >= 6 ? 3 : blk >= 3 ? 2 : blk >= 1 ? 1 : 0, jb = blk - ib * (ib + 1) / 2;
+    if (ib >= blocks) break;
+    const float* N = ib == jb ? w.A : w.E;
     uint32_t part[3][4];
 #pragma unroll
     for (int half = 0; half < 2; ++half)
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         const int i = ib * 16 + half * 8 + g4, j = jb * 16 + c * 8 + c2;
-        const float x = j < i ? w.E[i * CK_FS + j] : 0.f, y = j + 1 < i ? w.E[i * CK_FS + j + 1] : 0.f;
+        const float x = j < i ? N[i * CK_FS + j] : 0.f, y = j + 1 < i ? N[i * CK_FS + j + 1] : 0.f;
         split3(x, y, part[0][2 * half + c], part[1][2 * half + c], part[2][2 * half + c]);
       }
 #pragma unroll
@@ -794,10 +824,12 @@ delta_prepare_kernel(const ScanArgs a) {
     cp_async_16(reinterpret_cast<unsigned char*>(sm.k) + tile_off(j, ch, RB), kg + row * a.ldk + ch * 8, ok);
   }
   cp_async_commit();
+  DeltaCoef coef = {};
+  if (tid < 32) coef = delta_coef(a.coef + (start * a.H + h) * 3, a.H, t0, len, tid);
   const int64_t number = static_cast<int64_t>(chunks_before(a.seq_len, b, tid & 31) + t0 / CK_L) * a.H + h;
   cp_async_wait<0>();
   __syncthreads();
-  delta_prepare<D>(a, sm.q, sm.k, a.coef + (start * a.H + h) * 3, t0, len, sm.work, reinterpret_cast<DeltaPrep*>(a.scores)[number]);
+  delta_prepare<D>(a, sm.q, sm.k, coef, min(CK_L, len - t0), sm.work, reinterpret_cast<DeltaPrep*>(a.scores)[number]);
 }
 
 template <int D, bool AHEAD> struct DeltaTiles {
@@ -811,8 +843,6 @@ template <int D, bool AHEAD> struct DeltaTiles {
   };
 };
 
-__device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
-
 // t = x n over the blocks jb <= ib of row block ib: x in three parts per column block, n the fragments of a row of blocks; t = small + big
 __device__ __forceinline__ void delta_row_product(float small[2][4], float big[2][4], const uint32_t x[4][3][4], const uint4 (*n)[3][32], int ib, int lane) {
   float mid[2][4];
@@ -825,16 +855,28 @@ __device__ __forceinline__ void delta_row_product(float small[2][4], float big[2
     if (jb <= ib) {
       const uint4 (*f)[32] = n[ib * (ib + 1) / 2 + jb];
       const uint4 b0 = f[0][lane], b1 = f[1][lane], b2 = f[2][lane];
+      // products that add to the same sums lie as far from one another as their order allows.  The large ones by themselves, with what the tensor
+      // core cut off their sum (it keeps two bits behind a float's): the same products on top of minus the sum
+      const auto pair = [&](float c[2][4], int part, const uint4& b) {
+        mma_bf16_16816(c[0], x[jb][part], b.x, b.y);
+        mma_bf16_16816(c[1], x[jb][part], b.z, b.w);
+      };
+      float t[2][4] = {}, r[2][4];
+      pair(t, 0, b0);
+      pair(small, 2, b0);
+      pair(mid, 1, b0);
 #pragma unroll
-      for (int w = 0; w < 2; ++w) {
-        const uint32_t h0 = w ? b0.z : b0.x, h1 = w ? b0.w : b0.y, m0 = w ? b1.z : b1.x, m1 = w ? b1.w : b1.y, l0 = w ? b2.z : b2.x, l1 = w ? b2.w : b2.y;
-        mma_bf16_16816(small[w], x[jb][2], h0, h1);
-        mma_bf16_16816(mid[w], x[jb][1], h0, h1);
-        mma_add_rest(big[w], x[jb][0], h0, h1);
-        mma_bf16_16816(small[w], x[jb][0], l0, l1);
-        mma_bf16_16816(mid[w], x[jb][0], m0, m1);
-        mma_bf16_16816(small[w], x[jb][1], m0, m1);
-      }
+      for (int w = 0; w < 2; ++w)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) r[w][e] = -t[w][e];
+      pair(small, 0, b2);
+      pair(r, 0, b0);
+      pair(mid, 0, b1);
+      pair(small, 1, b1);
+#pragma unroll
+      for (int w = 0; w < 2; ++w)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) big[w][e] = (big[w][e] + r[w][e]) + t[w][e];
     }
   }
 #pragma unroll
@@ -915,6 +957,8 @@ delta_chunk_kernel(const ScanArgs a) {
   };
   load_chunk(0, 0);
   cp_async_commit();
+  DeltaCoef coef = {};                                     // of the next chunk, where the chain prepares it
+  if (!AHEAD && warp == 0) coef = delta_coef(cp, H, 0, len, lane);
   const int pr = wp * 16 + g4, n0 = wh * CH;               // S^T fragments: value columns pr (+ 8), key channels n0 + nt * 8 + c2 (+ 1)
   float S[NT][4];
   const bool carried = a.seq_pos0[b] > 0;
@@ -943,7 +987,8 @@ delta_chunk_kernel(const ScanArgs a) {
     }
     wild = __syncthreads_or(wild);                         // the chunk has landed; the previous one is consumed
     if constexpr (!AHEAD) {
-      delta_prepare<D>(a, sm.q[s], sm.k[s], cp, t0, len, sm.work, sm.prep[0]);
+      delta_prepare<D>(a, sm.q[s], sm.k[s], coef, L, sm.work, sm.prep[0]);
+      if (warp == 0) coef = delta_coef(cp, H, t0 + CK_L, len, lane);
       __syncthreads();
     }
     const DeltaPrep& pre = sm.prep[AHEAD ? s : 0];
@@ -1004,26 +1049,38 @@ delta_chunk_kernel(const ScanArgs a) {
 #pragma unroll
         for (int e = 0; e < 4; ++e)
           split3(S[2 * ks + (e >> 1)][2 * (e & 1)], S[2 * ks + (e >> 1)][2 * (e & 1) + 1], part[0][ks][e], part[1][ks][e], part[2][ks][e]);
+      // sums are added to every eight products, so that none waits for the one in front of it; all 64 tokens, however many there are (zeros behind the last one): code for
+      // fewer of them costs every chunk more, by what has to be fetched, than it saves the last one
       auto against = [&](uint32_t x_u, float c[8][4]) {
+        constexpr int NP = CK_L / 16;
 #pragma unroll
         for (int pass = 0; pass < 2; ++pass)
 #pragma unroll
-          for (int ks = 0; ks < CH / 16; ++ks)
+          for (int ks = 0; ks < CH / 16; ++ks) {
+            uint32_t bf[NP][4];
 #pragma unroll
-            for (int np = 0; np < 4; ++np)
-              if (np * 16 < L) {
-                uint32_t bf[4];
-                ldsm4(bf, x_u + tile_off(np * 16 + rb, n0 / 8 + ks * 2 + cb, RB));
-                if (pass == 0) {
-                  mma_bf16_16816(c[2 * np], part[2][ks], bf[0], bf[1]);
-                  mma_bf16_16816(c[2 * np + 1], part[2][ks], bf[2], bf[3]);
-                  mma_bf16_16816(c[2 * np], part[1][ks], bf[0], bf[1]);
-                  mma_bf16_16816(c[2 * np + 1], part[1][ks], bf[2], bf[3]);
-                } else {
-                  mma_add(c[2 * np], part[0][ks], bf[0], bf[1]);
-                  mma_add(c[2 * np + 1], part[0][ks], bf[2], bf[3]);
+            for (int np = 0; np < NP; ++np) ldsm4(bf[np], x_u + tile_off(np * 16 + rb, n0 / 8 + ks * 2 + cb, RB));
+            if (pass == 0) {
+#pragma unroll
+              for (int y = 2; y > 0; --y)
+#pragma unroll
+                for (int np = 0; np < NP; ++np) {
+                  mma_bf16_16816(c[2 * np], part[y][ks], bf[np][0], bf[np][1]);
+                  mma_bf16_16816(c[2 * np + 1], part[y][ks], bf[np][2], bf[np][3]);
                 }
+            } else {
+              float t[2 * NP][4] = {};
+#pragma unroll
+              for (int np = 0; np < NP; ++np) {
+                mma_bf16_16816(t[2 * np], part[0][ks], bf[np][0], bf[np][1]);
+                mma_bf16_16816(t[2 * np + 1], part[0][ks], bf[np][2], bf[np][3]);
               }
+#pragma unroll
+              for (int x = 0; x < 2 * NP; ++x)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) c[x][e] += t[x][e];
+            }
+          }
       };
       float ok[8][4];
 #pragma unroll
@@ -1146,31 +1203,41 @@ delta_chunk_kernel(const ScanArgs a) {
       }
       split_all([&](int nt, int h, uint32_t& lo) { lo = add_bf16x2(lo, off[nt][h]); });
       const float gl = pre.ecum[CK_L - 1];
+      constexpr int JS = CK_L / 16;
 #pragma unroll
-      for (int np = 0; np < CH / 16; ++np) {
-        float t[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-        uint32_t bf[4][4];
+      for (int np = 0; np < CH / 16; np += 2) {
+        float t[4][4] = {};
+        uint32_t bf[JS][2][4];
 #pragma unroll
-        for (int js = 0; js < 4; ++js)
-          if (js * 16 < L) ldsm4t(bf[js], k_u + tile_off(js * 16 + rt, n0 / 8 + np * 2 + ct, RB));
+        for (int js = 0; js < JS; ++js)
 #pragma unroll
-        for (int part = 2; part >= 0; --part)
+          for (int h = 0; h < 2; ++h) ldsm4t(bf[js][h], k_u + tile_off(js * 16 + rt, n0 / 8 + (np + h) * 2 + ct, RB));
 #pragma unroll
-          for (int js = 0; js < 4; ++js)
-            if (js * 16 < L) {
-              if (part > 0) {
-                mma_bf16_16816(t[0], xf[js][part], bf[js][0], bf[js][1]);
-                mma_bf16_16816(t[1], xf[js][part], bf[js][2], bf[js][3]);
-              } else {
-                mma_add(t[0], xf[js][part], bf[js][0], bf[js][1]);
-                mma_add(t[1], xf[js][part], bf[js][2], bf[js][3]);
-              }
+        for (int part = 2; part > 0; --part)
+#pragma unroll
+          for (int js = 0; js < JS; ++js)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              mma_bf16_16816(t[2 * h], xf[js][part], bf[js][h][0], bf[js][h][1]);
+              mma_bf16_16816(t[2 * h + 1], xf[js][part], bf[js][h][2], bf[js][h][3]);
             }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          S[2 * np][e] = fmaf(gl, S[2 * np][e], t[0][e]);
-          S[2 * np + 1][e] = fmaf(gl, S[2 * np + 1][e], t[1][e]);
+        for (int js = 0; js < JS; ++js) {
+          float y[4][4] = {};
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            mma_bf16_16816(y[2 * h], xf[js][0], bf[js][h][0], bf[js][h][1]);
+            mma_bf16_16816(y[2 * h + 1], xf[js][0], bf[js][h][2], bf[js][h][3]);
+          }
+#pragma unroll
+          for (int x = 0; x < 4; ++x)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) t[x][e] += y[x][e];
         }
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) S[2 * np + x][e] = fmaf(gl, S[2 * np + x][e], t[x][e]);
       }
     }
   }
