@@ -1263,11 +1263,13 @@ def _coef(out, heads):
 
 
 # The longest portion from which what chunks say without the state is formed by a launch of its own.  That launch and its scratch cost the host 4 to 8 us; each
-# 64 tokens of the state space's chain give back 1 to 2, those of the delta rule 8, so that there four chunks are enough.  State space, layers of 1, 2, 4 and 8
-# portions, in the chain / ahead of it in us: 192 tokens 70 75 87 160 / 75 78 85 149, 256 tokens 85 90 108 200 / 82 88 103 185.  Delta rule, the scan
-# of 1, 4 and 8 portions alone on the GPU: 100 tokens 34 38 70 / 29 31 54, 200 tokens 64 68 / 45 51; layers called one by one, host and all: 130 and 20 tokens
-# 72.9 / 75.5 to 77.0, 70 tokens 68.7 / 71.8 to 74.2, 200 tokens 80.0 / 73.1.
+# 64 tokens of the state space's chain give back 1 to 2, those of the delta rule 5 to 10, so that there four chunks are enough, or two where the portions' CTAs
+# are more than the multiprocessors and the host waits for them anyway.  State space, layers of 1, 2, 4 and 8 portions, in the chain / ahead of it in us: 192 tokens
+# 70 75 87 160 / 75 78 85 149, 256 tokens 85 90 108 200 / 82 88 103 185.  Delta rule, 16 heads of 128 x 128, scans alone on the GPU: 1 x 100 tokens 31 / 27, 3 x 100 35 /
+# 30, 5 x 100 64 / 48, 10 x 66 83 / 64; layers of few portions called one by one, host and all: 130 and 20 tokens 72.9 / 75.5 to 77.0, 70 tokens 68.7 / 71.8 to 74.2, 200 tokens
+# 80.0 / 73.1.
 SSM_AHEAD_FROM, DELTA_AHEAD_FROM = 256, 193
+DELTA_SCRATCH_MOST = 1 << 28               # floats (1 GB: 130000 tokens of 16 heads); steps that would need more leave all to the chain
 
 
 def ssm_scan(xbc, dt_in, dt_bias, a_log, d_skip, state, out, lay, heads, groups, vdim, nstate, ahead=None):
@@ -1288,13 +1290,13 @@ def ssm_scan(xbc, dt_in, dt_bias, a_log, d_skip, state, out, lay, heads, groups,
                                         dt, _ptr(scores), 0 if scores is None else scores.numel(), _stream()), "ssm_scan")
 
 
-_delta_chunk_floats = None
+_delta_chunk_floats = _multiprocessors = None
 
 
 def delta_rule_scan(qkv, beta_in, a_in, a_log, dt_bias, state, out, lay, heads, kv_heads, dim, vdim, ahead=None):
     """qkv [n, 2*kv_heads*dim + heads*vdim] (convolved, activated); beta_in, a_in: column slices [n, heads] of one tensor.  ``ahead``: what
     portions' chunks say without the state is formed for all of them at once (None: where that is faster)."""
-    global _delta_chunk_floats
+    global _delta_chunk_floats, _multiprocessors
     dt = _act(qkv, "qkv")
     _cuda(state, F32, "state"); _cuda(out, F32, "out")
     assert beta_in.dtype == qkv.dtype and a_in.dtype == qkv.dtype and beta_in.stride(0) == a_in.stride(0)
@@ -1302,11 +1304,15 @@ def delta_rule_scan(qkv, beta_in, a_in, a_log, dt_bias, state, out, lay, heads, 
     max_new, room, n = getattr(lay, "max_new", 0), 0, lay.n_tokens
     if ahead is None:
         ahead = max_new >= DELTA_AHEAD_FROM
+        if not ahead and max_new > 64:
+            if _multiprocessors is None:
+                _multiprocessors = device_info()["sm_count"]
+            ahead = n // max_new * heads * vdim > 64 * _multiprocessors          # at most so many portions of that length, a CTA for 64 value columns of a head
     if ahead and max_new > 64 and dt == DTYPE_CODE[BF16]:
         if _delta_chunk_floats is None:                                          # of a head and chunk; a call for its number costs as much as a launch
             _delta_chunk_floats = _load().b2tts_delta_rule_scan_ahead_floats(64, 1, 1) // 3
         room = (n // 64 + lay.n_seqs + 1) * heads * _delta_chunk_floats
-        if room > 1 << 28:                                                       # not more than 1 GB of scratch
+        if room > DELTA_SCRATCH_MOST:
             room = 0
     work = torch.empty(room + 3 * out.shape[0] * heads, dtype=F32, device=out.device)        # the chunks, then the scalars, in one piece
     at = work.data_ptr()

@@ -510,11 +510,13 @@ linear_chunk_kernel(const ScanArgs a, int64_t chunks) {
 // Accumulators turn into operands in registers; N and M arrive as the fragments that the lanes need.  Floats enter products as three bf16 parts,
 // two floats as the six part products down to 2^-16.
 //
-// Bound: the chain of chunks, of which a chunk takes about 17000 cycles: its 430 m16n8k16 a warp are 40 % of that, the rest is what they wait for
-// (two warps a scheduler; a CTA has the shared memory to itself).  With the tables and a triangular solve per value column in the chain it was 28000.
-// 4 ragged sequences (4856 tokens, 16 heads of 128 x 128): 302 us a chain and 50 ahead of it, the form before (dot products alone ahead) 444 + 11; all
-// launches 467 -> 366 us, one sequence of 300 tokens 83 -> 66, of 100 tokens 38 -> 38 (GPU 32 -> 29).  Where there is no room for what is formed ahead, the
-// chain forms it at 15500 cycles a chunk: 4 x 2048 tokens 492 -> 530 us, 16 x 40 63 -> 65.
+// Bound: the chain of chunks, of which a chunk takes about 14000 cycles: S^T k 2700, S^T q 1900, r, N and their exchange 4200, outputs 1800, the update 2500.  Two warps
+// a scheduler (a CTA has the shared memory to itself) leave most of that to what products and sums wait for; code is fetched once a chunk, so that shorter
+// code is faster than fewer products.  With the tables and a triangular solve per value column in the chain it was 28000.
+// All launches in us, that form with dot products alone ahead / now: 4 ragged sequences (4856 tokens, 16 heads of 128 x 128) 455 / 302, 4 x 2048 467 / 326, 32 heads of 64 409 / 273
+// and 411 / 314, one sequence of 300 tokens 74 / 51, 8 x 100 62 / 49.  Where there is no room for what is formed ahead, the chain forms it at 13000 cycles a
+// chunk; without room then and now: ragged 490 / 492, 4 x 2048 494 / 497, heads of 64 409 / 401 and 411 / 404, 300 tokens 77 / 75, 130 and 20 tokens 47.1 / 46.8, 16 x 40 63 / 61,
+// 8 x 100 63 / 66.
 //
 // Errors against 64 bits over 512 tokens (means of 48 inputs of three sizes, outputs / state; a substitution of floats in the chain, the rows of u rounded to floats, now):
 // 128 channels 1.051e-7 / 9.21e-8, 1.049e-7 / 9.23e-8, 1.023e-7 / 8.89e-8; 64 channels 0.998e-7 / 9.21e-8, 0.996e-7 / 9.22e-8, 0.967e-7 / 8.85e-8; keys that point half the
