@@ -79,6 +79,7 @@ def _load():
         "b2tts_prompt_assemble": (I, [P, L, I, P, L, I, P, P, P, L, I, I, P]),
         "b2tts_float_to_pcm16": (I, [P, P, L, F, P]),
         "b2tts_decode_rows_supported": (I, [I, I, I, I, I]),
+        "b2tts_decode_rows_taken": (I, [I, I, I, I, I, I]),
         "b2tts_decode_rows_workspace_bytes": (Z, [I, I, I, I]),
         "b2tts_decode_rows": (I, [P, L, P, L, P, I, P, I, I, I, I, I, I, F, I, P, L, P, P, F, P, P, I, P, I, I, F, P, Z, P]),
         "b2tts_decoder_stack_plan": (I, [I, I, I, I, P, P]),
@@ -736,6 +737,11 @@ DECODE_ROWS_MAX_LAYERS = 40
 def decode_rows_supported(m: int, hidden: int, q_size: int, kv_size: int, intermediate: int) -> bool:
     """Whether ``decode_rows`` has a kernel for these widths and rows."""
     return bool(_load().b2tts_decode_rows_supported(int(m), int(hidden), int(q_size), int(kv_size), int(intermediate)))
+
+
+def decode_rows_taken(m: int, max_context_len: int, hidden: int, q_size: int, kv_size: int, intermediate: int) -> bool:
+    """Whether ``decode_rows`` is the faster way for steps of ``m`` rows whose contexts have room for ``max_context_len`` tokens."""
+    return bool(_load().b2tts_decode_rows_taken(int(m), int(max_context_len), int(hidden), int(q_size), int(kv_size), int(intermediate)))
 
 
 def decode_rows_workspace(hidden: int, q_size: int, kv_size: int, intermediate: int, device) -> torch.Tensor | None:

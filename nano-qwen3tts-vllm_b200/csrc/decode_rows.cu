@@ -708,6 +708,12 @@ decode_rows_kernel(const __grid_constant__ DrParams p) {
   }
 }
 
+// CTAs that a unit of attention may take
+static int dr_parts(int m, int nsplit) {
+  const int want = (nsplit + DR_PART_SPLITS - 1) / DR_PART_SPLITS, most = sm_count() / (m * DR_KVH);
+  return want < most ? want : most;
+}
+
 struct DrSizes { size_t qkv, att, res, act, part, total; };
 static DrSizes dr_sizes(int hidden, int inter) {
   DrSizes s{};
@@ -768,6 +774,17 @@ extern "C" int b2tts_decode_rows_supported(int m, int hidden, int q_size, int kv
   const int form = b2::dr_form(hidden, q_size, kv_size, intermediate);
   return form != 0 && m >= 1 && m <= (form == 1 ? 4 : b2::DR_MAX_ROWS);
 }
+extern "C" int b2tts_decode_rows_taken(int m, int max_context_len, int hidden, int q_size, int kv_size, int intermediate) {
+  using namespace b2;
+  // ... and what attention takes grows with the contexts, by one chain of tiles after another where a CTA has more splits than it can walk at once (DR_PART_SPLITS).  So
+  // the tables' room decides: no CTA has a second turn.  28 layers, contexts that fill the tables, separate launches / this in us, the last size that is taken and the first one
+  // that is not: 2048 wide, 3 rows 1536 1435 / 1341, 2048 1475 / 1593; 4 rows 1024 1404 / 1292, 1536 1449 / 1527; 1024 wide, 4 rows 1024 1090 / 882, 1536 1142 / 1111; 6 rows
+  // 768 1085 / 914, 1024 1105 / 1123; 8 rows 512 1064 / 910, 768 1094 / 1115.  Up to 2 rows have the CTAs for any context: 2048 wide 4000 1741 / 1522, 16000 3339 / 2789.
+  // Tables of 16384 with 4 rows behind 16000 tokens 3382 / 4479, 1024 wide with 8 rows 3167 / 7012; the same behind 100 tokens 1278 / 1233 and 1014 / 920.
+  if (max_context_len <= 0 || !b2tts_decode_rows_supported(m, hidden, q_size, kv_size, intermediate)) return 0;
+  const int nsplit = fa_choose_nsplit(m, max_context_len);
+  return nsplit <= DR_PART_SPLITS * dr_parts(m, nsplit);
+}
 extern "C" size_t b2tts_decode_rows_workspace_bytes(int hidden, int q_size, int kv_size, int intermediate) {
   return b2::dr_form(hidden, q_size, kv_size, intermediate) != 0 ? b2::dr_sizes(hidden, intermediate).total : 0;
 }
@@ -822,8 +839,7 @@ extern "C" int b2tts_decode_rows(const void* x, int64_t x_row_stride, void* out,
   p.slot_mapping = slot_mapping; p.block_table = block_table; p.bt_stride = bt_stride; p.context_lens = context_lens;
   while ((1 << p.page_shift) < page_size) ++p.page_shift;
   p.nsplit = fa_choose_nsplit(m, max_context_len);
-  p.max_parts = (p.nsplit + DR_PART_SPLITS - 1) / DR_PART_SPLITS;
-  if (p.max_parts > sm_count() / (m * DR_KVH)) p.max_parts = sm_count() / (m * DR_KVH);
+  p.max_parts = dr_parts(m, p.nsplit);
   uint8_t* w = static_cast<uint8_t*>(workspace);
   auto take = [&w](size_t n) { uint64_t* at = reinterpret_cast<uint64_t*>(w); w += n; return at; };
   p.sync = reinterpret_cast<unsigned*>(take(256));

@@ -218,7 +218,7 @@ class ModelRunner:
                 layer_id += 1
         for module in self.model.modules():
             if hasattr(module, "bind_decode_rows"):
-                module.bind_decode_rows()
+                module.bind_decode_rows(where_faster=True)
 
     # ------------------------------------------------------------------ batch layout
     def prepare_prefill(self, seqs: list[Sequence]):

@@ -300,20 +300,30 @@ class DecoderStack(nn.Module):
             intermediate=c.intermediate_size, eps=c.rms_norm_eps, scale=self.layers[0].self_attn.scaling, workspace=ws,
             attention_scaling=rope.attention_scaling, rounding=self.rounding, layer_array=arr)
 
-    def bind_decode_rows(self) -> None:
-        """Room for the persistent decode kernel, given by the runner that owns the KV cache: steps of one runner run one after another."""
-        c, rope = self.config, self.layers[0].self_attn.rotary_emb
-        widths = (c.hidden_size, c.num_attention_heads * c.head_dim, c.num_key_value_heads * c.head_dim, c.intermediate_size)
+    def bind_decode_rows(self, where_faster: bool = False) -> None:
+        """Room for the persistent decode kernel, given by the runner that owns the KV cache: steps of one runner run one after another.  ``where_faster``: steps whose
+        contexts may be too long for it stay with the separate launches (else all that there is a kernel for take it)."""
+        self._rows_where_faster = where_faster
+        c, rope, widths = self.config, self.layers[0].self_attn.rotary_emb, self._widths()
         page = self.layers[0].self_attn.attn.k_cache.shape[1]
         self._rows_most = max([m for m in range(1, DECODE_ROWS_MAX + 1) if nat.decode_rows_supported(m, *widths)], default=0)
         if len(self.layers) > nat.DECODE_ROWS_MAX_LAYERS or c.head_dim != 128 or rope.inv_freq.numel() != 64 or page & (page - 1):
             self._rows_most = 0
         self._rows_ws = nat.decode_rows_workspace(*widths, self.norm.weight.device) if self._rows_most else None
 
+    def _widths(self) -> tuple[int, int, int, int]:
+        c = self.config
+        return c.hidden_size, c.num_attention_heads * c.head_dim, c.num_key_value_heads * c.head_dim, c.intermediate_size
+
+    def _max_context(self) -> int:
+        ctx = get_context()
+        return ctx.max_context_len or ctx.block_tables.shape[1] * self.layers[0].self_attn.attn.k_cache.shape[1]
+
     def _takes_rows(self, x: torch.Tensor) -> bool:
         ctx = get_context()
         return (getattr(self, "_rows_ws", None) is not None and not ctx.is_prefill and ctx.block_tables is not None and x.dim() == 2
-                and 1 <= x.shape[0] <= min(self._rows_most, DECODE_ROWS_MAX) and x.dtype == torch.bfloat16)
+                and 1 <= x.shape[0] <= min(self._rows_most, DECODE_ROWS_MAX) and x.dtype == torch.bfloat16
+                and (not self._rows_where_faster or nat.decode_rows_taken(x.shape[0], self._max_context(), *self._widths())))
 
     def _run_rows(self, x: torch.Tensor, positions: torch.Tensor) -> torch.Tensor:
         c, ctx, a0 = self.config, get_context(), self.layers[0].self_attn
@@ -330,7 +340,7 @@ class DecoderStack(nn.Module):
             x, nat.stack_layer_array(layers), len(layers), self.norm.weight, positions, rope.inv_freq, ctx.slot_mapping, ctx.block_tables,
             ctx.context_lens, num_heads=c.num_attention_heads, num_kv_heads=c.num_key_value_heads, head_dim=c.head_dim,
             intermediate=c.intermediate_size, page_size=a0.attn.k_cache.shape[1],
-            max_context_len=ctx.max_context_len or ctx.block_tables.shape[1] * a0.attn.k_cache.shape[1], eps=c.rms_norm_eps, scale=a0.scaling, workspace=self._rows_ws,
+            max_context_len=self._max_context(), eps=c.rms_norm_eps, scale=a0.scaling, workspace=self._rows_ws,
             modality=rope.modality if positions.dim() > 1 else None, attention_scaling=rope.attention_scaling, rounding=self.rounding)
 
     def _run_layers_native(self, input_embeds, positions, input_ssq, tail_weight):
