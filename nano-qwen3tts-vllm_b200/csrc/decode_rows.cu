@@ -519,6 +519,7 @@ decode_rows_kernel(const __grid_constant__ DrParams p) {
         if (u < n) put_vec(width, i / per, i % per, x[u]);
       }
     }
+    __syncwarp();                                          // lanes leave the polling one by one, the barrier wants whole warps
     dr_sync();
   };
   // The rows x this warp's tiles (of a slice's, every 8 / slices-th), whose chains of products take turns.  A step's fragments are read while the products of the
