@@ -434,6 +434,16 @@ B2TTS_API int b2tts_decode_rows(const void* x, int64_t x_row_stride, void* out, 
                                 const int32_t* modality, float attention_scaling, const int32_t* slot_mapping, const int32_t* block_table,
                                 int bt_stride, const int32_t* context_lens, int page_size, int max_context_len, float scale, void* workspace,
                                 size_t workspace_bytes, void* stream);
+/* For tests: the same with waits that give up after so many tries (its results are not valid then, the next launch's are), how often a launch's waits ran out
+ * since the library was loaded (expected: 0), and a kernel whose wait runs out. */
+B2TTS_API int b2tts_decode_rows_polls(const void* x, int64_t x_row_stride, void* out, int64_t out_row_stride, const b2tts_stack_layer* layers,
+                                      int num_layers, const void* final_norm_weight, int m, int hidden, int num_heads, int num_kv_heads, int head_dim,
+                                      int intermediate, float eps, int rounding, const int64_t* positions, int64_t pos_row_stride, const float* inv_freq,
+                                      const int32_t* modality, float attention_scaling, const int32_t* slot_mapping, const int32_t* block_table,
+                                      int bt_stride, const int32_t* context_lens, int page_size, int max_context_len, float scale, void* workspace,
+                                      size_t workspace_bytes, int polls, void* stream);
+B2TTS_API int b2tts_decode_rows_timeouts(void);
+B2TTS_API int b2tts_decode_rows_lose_wait(void* stream);
 
 /* ---- token-id decoder models with a 32-bit residual stream -------------------------------------
  * (no counterpart in the reference, whose models take embeddings and keep a bf16 residual)
@@ -520,7 +530,7 @@ B2TTS_API int b2tts_grouped_gemm_silu(const void* a, int64_t lda, const void* w,
                                       const int32_t* sorted_pair, int n_pairs, int experts, int ff, int k, int top, void* stream);
 /* How often a wait inside the grouped tensor-core kernel ran out since the library was loaded (expected: 0).  A launch whose wait runs
  * out leaves no result; the next grouped_gemm* call answers with B2TTS_ECUDA, and so does _check(), once: call it behind a
- * synchronisation (it makes none itself) before results are used; it answers for the waits of portion_attn.cu as well.  _lose_wait()
+ * synchronisation (it makes none itself) before results are used; it answers for the waits of portion_attn.cu and decode_rows.cu as well.  _lose_wait()
  * launches a kernel whose wait runs out, for tests. */
 B2TTS_API int b2tts_grouped_gemm_timeouts(void);
 B2TTS_API int b2tts_grouped_gemm_check(void);

@@ -82,6 +82,9 @@ def _load():
         "b2tts_decode_rows_taken": (I, [I, I, I, I, I, I]),
         "b2tts_decode_rows_workspace_bytes": (Z, [I, I, I, I]),
         "b2tts_decode_rows": (I, [P, L, P, L, P, I, P, I, I, I, I, I, I, F, I, P, L, P, P, F, P, P, I, P, I, I, F, P, Z, P]),
+        "b2tts_decode_rows_polls": (I, [P, L, P, L, P, I, P, I, I, I, I, I, I, F, I, P, L, P, P, F, P, P, I, P, I, I, F, P, Z, I, P]),
+        "b2tts_decode_rows_timeouts": (I, []),
+        "b2tts_decode_rows_lose_wait": (I, [P]),
         "b2tts_decoder_stack_plan": (I, [I, I, I, I, P, P]),
         "b2tts_decoder_stack_workspace_bytes": (Z, [I, I, I, I]),
         "b2tts_decoder_stack_decode": (I, [P, L, P, L, P, I, P, I, I, I, I, I, I, F, I, P, P, F, P, P, I, P, I, F, P, Z, P]),
@@ -756,9 +759,10 @@ def decode_rows_workspace(hidden: int, q_size: int, kv_size: int, intermediate: 
 
 def decode_rows(x, layer_array, num_layers, final_norm_weight, positions, inv_freq, slot_mapping, block_table, context_lens, *, num_heads,
                 num_kv_heads, head_dim, intermediate, page_size, max_context_len, eps, scale, workspace, modality=None, attention_scaling=1.0,
-                rounding=ROUND_EAGER):
+                rounding=ROUND_EAGER, polls=None):
     """One decode step of a whole decoder stack for a few rows in one persistent launch (``b2tts_decode_rows``): x [m, hidden] -> normalised
-    hidden states [m, hidden].  ``layer_array``: ``stack_layer_array`` of the layers; positions [m], or [3, m] with ``modality`` [128]."""
+    hidden states [m, hidden].  ``layer_array``: ``stack_layer_array`` of the layers; positions [m], or [3, m] with ``modality`` [128].
+    ``polls`` (tests): waits give up after so many tries."""
     _cuda(x, BF16, "x"); _cuda(positions, I64, "positions"); _cuda(inv_freq, F32, "inv_freq")
     _cuda(slot_mapping, I32, "slot_mapping"); _cuda(block_table, I32, "block_table"); _cuda(context_lens, I32, "context_lens")
     m, hidden = x.shape
@@ -767,13 +771,18 @@ def decode_rows(x, layer_array, num_layers, final_norm_weight, positions, inv_fr
     if positions.stride(-1) != 1:
         positions = positions.contiguous()
     out = torch.empty(m, hidden, dtype=BF16, device=x.device)
-    _check(_load().b2tts_decode_rows(
+    entry, limit = (_load().b2tts_decode_rows, ()) if polls is None else (_load().b2tts_decode_rows_polls, (int(polls),))
+    _check(entry(
         x.data_ptr(), x.stride(0), out.data_ptr(), out.stride(0), ctypes.byref(layer_array), num_layers, final_norm_weight.data_ptr(), m, hidden,
         num_heads, num_kv_heads, head_dim, intermediate, float(eps), int(rounding), positions.data_ptr(),
         positions.stride(0) if positions.dim() > 1 else 0, inv_freq.data_ptr(), _ptr(modality), float(attention_scaling),
         slot_mapping.data_ptr(), block_table.data_ptr(), block_table.stride(0), context_lens.data_ptr(), page_size, max_context_len, float(scale),
-        workspace.data_ptr(), workspace.numel(), _stream()), "decode_rows")
+        workspace.data_ptr(), workspace.numel(), *limit, _stream()), "decode_rows")
     return out
+
+
+def decode_rows_timeouts() -> int:
+    return int(_load().b2tts_decode_rows_timeouts())
 
 
 # ------------------------------------------------------------------------------------------ f3: prompt assembly

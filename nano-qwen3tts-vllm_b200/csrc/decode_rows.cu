@@ -23,7 +23,8 @@
 // Why no word is overwritten before its readers are done: a phase's outputs are complete only when all its readers have read (each sum needs
 // all slices), and a phase that reads whole rows waits for all outputs of the phase before.  So who writes a buffer again, a layer later,
 // has waited for something that followed the last read of it.  A CTA that has no tile in a phase does not read that phase's input.
-// All waits are bounded; a wait that runs out is counted (waits.cuh), and the launch goes on to its end with what it has.
+// All waits are bounded; a wait that runs out is counted (waits.cuh), and the launch goes on to its end with what it has: who has given up waits for no more words, but
+// reads, writes and meets the others of its CTA as ever, so that other CTAs find their words, every copy its readers and the next launch everything as it should be.
 //
 // Bound: a layer of the talker takes 28 us for one row, 13.9 of them the stream at HBM's rate; hand-overs of 1.2 to 2.5 us, five a layer, are the rest (a word
 // takes about 0.8 us from store to load while L2 feeds the stream), with 2 us of a tile's softmax after another in attention.  28 layers, one row, us: 1241
@@ -41,7 +42,7 @@ namespace b2 {
 constexpr int DR_WARPS = 8, DR_READERS = DR_WARPS * 32, DR_THREADS = DR_READERS + 32;
 constexpr int DR_HD = 128, DR_GROUP = 2, DR_Q = 2048, DR_KV = DR_Q / DR_GROUP, DR_KVH = DR_KV / DR_HD, DR_MAX_LAYERS = 40, DR_MAX_ROWS = 8;
 constexpr int DR_PART_SPLITS = DR_WARPS / DR_GROUP;        // splits of a context that one CTA takes: a warp a query head
-constexpr int DR_POLLS = 1 << 20, DR_PAGES = 64;
+constexpr int DR_POLLS = 1 << 20, DR_PAGES = 64;         // tries for a word; pages of a row that are kept
 constexpr int DR_UNIT = 1024;                      // 8 features x 64 columns, as the packed weights have them
 constexpr int DR_STAGES = 16;                      // stages in flight at most
 constexpr int DR_SUMS = 32;                        // (tile, slice) sums of a CTA's phase
@@ -49,6 +50,11 @@ constexpr int DR_MAX_TILES = 4;                    // tiles of a warp in a phase
 enum { DR_E_QKV = 1, DR_E_ATT = 2, DR_E_RES1 = 3, DR_E_ACT = 4, DR_E_RES2 = 5, DR_E_PART = 6, DR_E_LAYER = 8 };
 
 __device__ int g_rows_timeouts = 0;                // see waits.cuh
+__device__ __forceinline__ void dr_report(int* word) {
+  const int n = atomicAdd(&g_rows_timeouts, 1) + 1;
+  if (word != nullptr) *reinterpret_cast<volatile int*>(word) = n;
+  __threadfence_system();
+}
 
 struct DrLayer {
   const uint8_t *w_qkv, *w_o, *w_gu, *w_down;            // packed weights
@@ -72,6 +78,7 @@ struct DrParams {
   const int32_t* block_table;
   int bt_stride, page_shift;
   const int32_t* context_lens;
+  int polls;                                             // tries after which a wait for a word gives up
   int nsplit, max_parts;                                 // splits of a context; CTAs a unit may take
   unsigned* sync;                                        // [0] the number of the last phase, [1] CTAs that are done
   uint64_t *qkv, *att, *res1, *act, *res2, *part;
@@ -93,17 +100,17 @@ __device__ __forceinline__ void dr_get2(const uint64_t* at, uint64_t& a, uint64_
   asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(at) : "memory");
 }
 // one word, polled
-__device__ __forceinline__ uint32_t dr_wait(const uint64_t* at, uint32_t flag, bool& alive) {
+__device__ __forceinline__ uint32_t dr_wait(const uint64_t* at, uint32_t flag, int polls, bool& alive) {
   uint64_t w = dr_get(at);
   for (int n = 0; static_cast<uint32_t>(w >> 32) != flag && alive; ++n) {
-    if (n >= DR_POLLS) alive = false;
+    if (n >= polls) alive = false;
     w = dr_get(at);
   }
   return static_cast<uint32_t>(w);
 }
 // the first n of N vectors of four words (32-byte aligned), `apart` words from one another: all asked for at once, those that are not there yet again
 template <int N>
-__device__ __forceinline__ void dr_wait_all(const uint64_t* at, int apart, int n, uint32_t flag, uint4 (&x)[N], bool& alive) {
+__device__ __forceinline__ void dr_wait_all(const uint64_t* at, int apart, int n, uint32_t flag, uint4 (&x)[N], int polls, bool& alive) {
   uint32_t todo = (1u << n) - 1;
   for (int tries = 0; todo != 0; ++tries) {
     uint64_t w[N][4];
@@ -123,7 +130,7 @@ __device__ __forceinline__ void dr_wait_all(const uint64_t* at, int apart, int n
           todo &= ~(1u << i);
         }
       }
-    if (tries >= DR_POLLS) alive = false;
+    if (tries >= polls) alive = false;
   }
 }
 
@@ -216,7 +223,7 @@ __device__ __forceinline__ bool dr_attend(const DrParams& p, const DrLayer& y, u
     const __nv_bfloat16* nw = warp < DR_GROUP ? y.qn_w : y.kn_w;
     const uint32_t w1 = nw != nullptr ? __ldg(reinterpret_cast<const unsigned*>(nw + 2 * lane)) : 0u;
     const uint32_t w2 = nw != nullptr ? __ldg(reinterpret_cast<const unsigned*>(nw + 64 + 2 * lane)) : 0u;
-    uint32_t y1 = dr_wait(at, e0 + DR_E_QKV, alive), y2 = dr_wait(at + 32, e0 + DR_E_QKV, alive);
+    uint32_t y1 = dr_wait(at, e0 + DR_E_QKV, p.polls, alive), y2 = dr_wait(at + 32, e0 + DR_E_QKV, p.polls, alive);
     __syncwarp();
     if (warp < DR_GROUP + 1) {
       if (nw != nullptr) {
@@ -324,7 +331,7 @@ __device__ __forceinline__ bool dr_attend(const DrParams& p, const DrLayer& y, u
 #pragma unroll 1
     for (int k = tid; k < DR_GROUP * words; k += DR_READERS) {
       const int h = k >= words ? 1 : 0, at = k - h * words, s = s1 + at / (2 + DR_HD), e = at % (2 + DR_HD);
-      const float z = __uint_as_float(dr_wait(part_w + (h * 32 + s) * (2 + DR_HD) + e, e0 + DR_E_PART, alive));
+      const float z = __uint_as_float(dr_wait(part_w + (h * 32 + s) * (2 + DR_HD) + e, e0 + DR_E_PART, p.polls, alive));
       if (e < 2) reinterpret_cast<float*>(fold_ml + h * 32 + s)[e] = z;
       else fold_av[(h * 32 + s) * DR_HD + e - 2] = z;
     }
@@ -370,7 +377,7 @@ template <int H, int I, int ROWS> struct DrShared {
   uint64_t full[DR_STAGES], empty[DR_STAGES];
   DrPlan plan;
   unsigned base;
-  int lost;                                              // the copying warp gave up
+  int lost;                                              // somebody gave up
 };
 
 // H, I: hidden and inner width; SG, SQ: slices of K of gate_up and of the other projections; ROWS: most rows
@@ -455,7 +462,7 @@ decode_rows_kernel(const __grid_constant__ DrParams p) {
 
   // =========================== the phases
   const uint32_t base = sm.base;
-  bool alive = true;
+  bool alive = true, stream = true;                        // no wait of this lane for words, of this warp for weights ran out
   int stage = 0, head = 0;                                 // the next one of the stream, and where the one before it ends
   // Rows lie in shared memory as they are, vector v (8 columns) of row r at v ^ r in its group of eight: a warp's ldmatrix reads eight rows without conflicts
   auto put_vec = [&](int width, int r, int v, const uint4& x) {
@@ -485,7 +492,7 @@ decode_rows_kernel(const __grid_constant__ DrParams p) {
         if (r < m) x[i] = make_uint4(at[0], at[1], at[2], at[3]);
       }
     } else {
-      dr_wait_all<PASSES>(res + r0 * (H / 2) + 4 * v, RP * (H / 2), r0 < m ? (m - r0 + RP - 1) / RP : 0, flag, x, alive);
+      dr_wait_all<PASSES>(res + r0 * (H / 2) + 4 * v, RP * (H / 2), r0 < m ? (m - r0 + RP - 1) / RP : 0, flag, x, p.polls, alive);
     }
     __syncwarp();
 #pragma unroll
@@ -512,14 +519,14 @@ decode_rows_kernel(const __grid_constant__ DrParams p) {
     for (int i0 = tid; i0 < all; i0 += AT_ONCE * DR_READERS) {
       uint4 x[AT_ONCE] = {};
       const int n = min(AT_ONCE, (all - i0 + DR_READERS - 1) / DR_READERS);
-      dr_wait_all<AT_ONCE>(in + 4 * i0, 4 * DR_READERS, n, flag, x, alive);
+      dr_wait_all<AT_ONCE>(in + 4 * i0, 4 * DR_READERS, n, flag, x, p.polls, alive);
+      __syncwarp();                                        // lanes leave the polling one by one, the barrier behind it wants whole warps
 #pragma unroll
       for (int u = 0; u < AT_ONCE; ++u) {
         const int i = i0 + u * DR_READERS;
         if (u < n) put_vec(width, i / per, i % per, x[u]);
       }
     }
-    __syncwarp();                                          // lanes leave the polling one by one, the barrier wants whole warps
     dr_sync();
   };
   // The rows x this warp's tiles (of a slice's, every 8 / slices-th), whose chains of products take turns.  A step's fragments are read while the products of the
@@ -538,7 +545,8 @@ decode_rows_kernel(const __grid_constant__ DrParams p) {
       const int at = head + size > Sm::UNITS ? 0 : head;
       head = at + size;
       in = at * DR_UNIT;
-      if (alive && !mbar_wait_limit(sm.full + stage % DR_STAGES, (stage / DR_STAGES) & 1)) alive = false;
+      // (alive or not: readers that ran ahead of the copies would free stages that are still to land)
+      if (stream && !mbar_wait_limit(sm.full + stage % DR_STAGES, (stage / DR_STAGES) & 1)) stream = alive = false;
       ++stage;
     };
     auto read = [&](int j, Stage& f) {
@@ -564,7 +572,6 @@ decode_rows_kernel(const __grid_constant__ DrParams p) {
       __syncwarp();
       if (lane == 0) mbar_arrive(sm.empty + number % DR_STAGES);
     };
-    alive = __all_sync(0xffffffffu, alive);                                       // lanes give up one by one, the waits here need all of them
     Stage f0 = {}, f1 = {};                                                       // (what is set under a condition alone counts as live everywhere)
     enter();
     read(0, f0);
@@ -632,7 +639,7 @@ decode_rows_kernel(const __grid_constant__ DrParams p) {
       take_rows(phase == 3 ? I : DR_Q, phase == 3 ? p.act : p.att, e0 + (phase == 3 ? DR_E_ACT : DR_E_ATT));
       if (mine)
         r = i == 1 ? *reinterpret_cast<const uint32_t*>(p.x_in + row * p.x_stride + n)
-                   : dr_wait((phase == 3 ? p.res1 : p.res2) + (row * H + n) / 2, phase == 3 ? e0 + DR_E_RES1 : e0 - DR_E_LAYER + DR_E_RES2, alive);
+                   : dr_wait((phase == 3 ? p.res1 : p.res2) + (row * H + n) / 2, phase == 3 ? e0 + DR_E_RES1 : e0 - DR_E_LAYER + DR_E_RES2, p.polls, alive);
       __syncwarp();
     } else {
       if (tile0 == tile1) continue;
@@ -678,7 +685,7 @@ decode_rows_kernel(const __grid_constant__ DrParams p) {
     uint4 x = make_uint4(0, 0, 0, 0);
     if (tid < VECS) {
       uint4 y[1] = {};
-      dr_wait_all<1>(p.res2 + r * (H / 2) + 4 * tid, 0, 1, last, y, alive);
+      dr_wait_all<1>(p.res2 + r * (H / 2) + 4 * tid, 0, 1, last, y, p.polls, alive);
       x = y[0];
       __syncwarp();
       const float s = warp_sum(squares(x));
@@ -697,9 +704,7 @@ decode_rows_kernel(const __grid_constant__ DrParams p) {
   __syncthreads();                                         // the copying warp too
   if (tid == 0) {
     if (sm.lost) {
-      const int n = atomicAdd(&g_rows_timeouts, 1) + 1;
-      if (p.waits != nullptr) *reinterpret_cast<volatile int*>(p.waits) = n;
-      __threadfence_system();
+      dr_report(p.waits);
     }
     __threadfence();
     if (atomicAdd(p.sync + 1, 1u) == gridDim.x - 1) {
@@ -789,12 +794,12 @@ extern "C" int b2tts_decode_rows_taken(int m, int max_context_len, int hidden, i
 extern "C" size_t b2tts_decode_rows_workspace_bytes(int hidden, int q_size, int kv_size, int intermediate) {
   return b2::dr_form(hidden, q_size, kv_size, intermediate) != 0 ? b2::dr_sizes(hidden, intermediate).total : 0;
 }
-extern "C" int b2tts_decode_rows(const void* x, int64_t x_row_stride, void* out, int64_t out_row_stride, const b2tts_stack_layer* layers, int num_layers,
+extern "C" int b2tts_decode_rows_polls(const void* x, int64_t x_row_stride, void* out, int64_t out_row_stride, const b2tts_stack_layer* layers, int num_layers,
                                  const void* final_norm_weight, int m, int hidden, int num_heads, int num_kv_heads, int head_dim, int intermediate,
                                  float eps, int rounding, const int64_t* positions, int64_t pos_row_stride, const float* inv_freq, const int32_t* modality,
                                  float attention_scaling, const int32_t* slot_mapping, const int32_t* block_table, int bt_stride,
                                  const int32_t* context_lens, int page_size, int max_context_len, float scale, void* workspace, size_t workspace_bytes,
-                                 void* stream) {
+                                 int polls, void* stream) {
   using namespace b2;
   const char* what = "decode_rows";
   if (m == 0) return B2TTS_OK;
@@ -846,6 +851,7 @@ extern "C" int b2tts_decode_rows(const void* x, int64_t x_row_stride, void* out,
   p.sync = reinterpret_cast<unsigned*>(take(256));
   p.qkv = take(z.qkv); p.att = take(z.att); p.res1 = take(z.res); p.res2 = take(z.res); p.act = take(z.act); p.part = take(z.part);
   p.waits = wait_word(WAITS_ROWS);
+  p.polls = polls;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool eager = rounding == B2TTS_ROUND_EAGER;
   // few rows leave the ring more room: instances for 2, 4 and 8
@@ -857,4 +863,34 @@ extern "C" int b2tts_decode_rows(const void* x, int64_t x_row_stride, void* out,
     return eager ? go_rows<1024, 3072, 8, 4, R, true>(p, st) : go_rows<1024, 3072, 8, 4, R, false>(p, st);
   };
   return m <= 2 ? go(std::integral_constant<int, 2>{}) : m <= 4 ? go(std::integral_constant<int, 4>{}) : go(std::integral_constant<int, DR_MAX_ROWS>{});
+}
+extern "C" int b2tts_decode_rows(const void* x, int64_t x_row_stride, void* out, int64_t out_row_stride, const b2tts_stack_layer* layers, int num_layers,
+                                 const void* final_norm_weight, int m, int hidden, int num_heads, int num_kv_heads, int head_dim, int intermediate,
+                                 float eps, int rounding, const int64_t* positions, int64_t pos_row_stride, const float* inv_freq, const int32_t* modality,
+                                 float attention_scaling, const int32_t* slot_mapping, const int32_t* block_table, int bt_stride,
+                                 const int32_t* context_lens, int page_size, int max_context_len, float scale, void* workspace, size_t workspace_bytes,
+                                 void* stream) {
+  return b2tts_decode_rows_polls(x, x_row_stride, out, out_row_stride, layers, num_layers, final_norm_weight, m, hidden, num_heads, num_kv_heads, head_dim, intermediate, eps,
+                                 rounding, positions, pos_row_stride, inv_freq, modality, attention_scaling, slot_mapping, block_table, bt_stride, context_lens, page_size,
+                                 max_context_len, scale, workspace, workspace_bytes, b2::DR_POLLS, stream);
+}
+
+namespace b2 {
+// One wait for a word that nobody writes, with a short limit
+__device__ uint64_t g_rows_unwritten = 0;
+__global__ void rows_lost_wait_kernel(int* word) {
+  bool alive = true;
+  dr_wait(&g_rows_unwritten, 1u, 64, alive);
+  if (!alive && threadIdx.x == 0) dr_report(word);
+}
+}  // namespace b2
+
+extern "C" int b2tts_decode_rows_timeouts(void) { return b2::wait_count(b2::WAITS_ROWS); }
+extern "C" int b2tts_decode_rows_lose_wait(void* stream) {
+  using namespace b2;
+  int* word = wait_word(WAITS_ROWS);
+  B2_REQUIRE(word != nullptr, B2TTS_ECUDA, "decode_rows_lose_wait: no host memory");
+  rows_lost_wait_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(word);
+  B2_CHECK_LAUNCH("decode_rows_lose_wait");
+  return B2TTS_OK;
 }
