@@ -423,10 +423,11 @@ B2TTS_API int    b2tts_decoder_stack_decode(const void* x, int64_t x_row_stride,
 /* A decode step of a whole stack (every layer and the final norm) for 1 .. 8 rows in one persistent launch; out = normalised rows.  Packed weights, caches and
  * rounding as b2tts_decoder_stack_decode; positions [m], or [3][m] with row stride pos_row_stride where modality [128] picks the row per rotary channel.
  * The results are those of the separate launches (b2tts_rmsnorm, b2tts_gemm_bf16, b2tts_fused_decode_attn with max_context_len), to the bit.
- * _supported(): whether there is a kernel for these widths and rows; _taken(): and it is the faster one for contexts of up to max_context_len.  workspace: _workspace_bytes() bytes, 256-byte aligned, ZEROED once; launches that
+ * _supported(): whether there is a kernel for these widths and rows, and the current context has the multiprocessors that it wants (a green context may have
+ * fewer); _taken(): and it is the faster one for contexts of up to max_context_len, on this stream.  workspace: _workspace_bytes() bytes, 256-byte aligned, ZEROED once; launches that
  * share one must not overlap.  Cooperative launch: all multiprocessors are taken.  A wait that runs out is an error of a later call (b2tts_grouped_gemm_check()). */
 B2TTS_API int b2tts_decode_rows_supported(int m, int hidden, int q_size, int kv_size, int intermediate);
-B2TTS_API int b2tts_decode_rows_taken(int m, int max_context_len, int hidden, int q_size, int kv_size, int intermediate);
+B2TTS_API int b2tts_decode_rows_taken(int m, int max_context_len, int hidden, int q_size, int kv_size, int intermediate, void* stream);
 B2TTS_API size_t b2tts_decode_rows_workspace_bytes(int hidden, int q_size, int kv_size, int intermediate);
 B2TTS_API int b2tts_decode_rows(const void* x, int64_t x_row_stride, void* out, int64_t out_row_stride, const b2tts_stack_layer* layers,
                                 int num_layers, const void* final_norm_weight, int m, int hidden, int num_heads, int num_kv_heads, int head_dim,

@@ -79,7 +79,7 @@ def _load():
         "b2tts_prompt_assemble": (I, [P, L, I, P, L, I, P, P, P, L, I, I, P]),
         "b2tts_float_to_pcm16": (I, [P, P, L, F, P]),
         "b2tts_decode_rows_supported": (I, [I, I, I, I, I]),
-        "b2tts_decode_rows_taken": (I, [I, I, I, I, I, I]),
+        "b2tts_decode_rows_taken": (I, [I, I, I, I, I, I, P]),
         "b2tts_decode_rows_workspace_bytes": (Z, [I, I, I, I]),
         "b2tts_decode_rows": (I, [P, L, P, L, P, I, P, I, I, I, I, I, I, F, I, P, L, P, P, F, P, P, I, P, I, I, F, P, Z, P]),
         "b2tts_decode_rows_polls": (I, [P, L, P, L, P, I, P, I, I, I, I, I, I, F, I, P, L, P, P, F, P, P, I, P, I, I, F, P, Z, I, P]),
@@ -743,8 +743,9 @@ def decode_rows_supported(m: int, hidden: int, q_size: int, kv_size: int, interm
 
 
 def decode_rows_taken(m: int, max_context_len: int, hidden: int, q_size: int, kv_size: int, intermediate: int) -> bool:
-    """Whether ``decode_rows`` is the faster way for steps of ``m`` rows whose contexts have room for ``max_context_len`` tokens."""
-    return bool(_load().b2tts_decode_rows_taken(int(m), int(max_context_len), int(hidden), int(q_size), int(kv_size), int(intermediate)))
+    """Whether ``decode_rows`` is the faster way for steps of ``m`` rows whose contexts have room for ``max_context_len`` tokens, and can run on the current stream."""
+    return bool(_load().b2tts_decode_rows_taken(int(m), int(max_context_len), int(hidden), int(q_size), int(kv_size), int(intermediate),
+                                                _stream() if torch.cuda.is_initialized() else None))
 
 
 def decode_rows_workspace(hidden: int, q_size: int, kv_size: int, intermediate: int, device) -> torch.Tensor | None:

@@ -770,26 +770,93 @@ static int go_rows(const DrParams& p, cudaStream_t st) {
   return e != cudaSuccess ? cuda_fail(e, "decode_rows") : B2TTS_OK;
 }
 
+// The multiprocessors that a launch on this stream (null: of the current context) gets: a green context has fewer than the device
+static int dr_multiprocessors(cudaStream_t st) {
+  auto entry = [](const char* name) -> void* {
+    void* at = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint(name, &at, cudaEnableDefault, &found) != cudaSuccess || found != cudaDriverEntryPointSuccess) at = nullptr;
+    cudaGetLastError();
+    return at;
+  };
+  static const auto green_of = reinterpret_cast<decltype(&cuStreamGetGreenCtx)>(entry("cuStreamGetGreenCtx"));
+  static const auto green_has = reinterpret_cast<decltype(&cuGreenCtxGetDevResource)>(entry("cuGreenCtxGetDevResource"));
+  static const auto current = reinterpret_cast<decltype(&cuCtxGetCurrent)>(entry("cuCtxGetCurrent"));
+  static const auto context_has = reinterpret_cast<decltype(&cuCtxGetDevResource)>(entry("cuCtxGetDevResource"));
+  CUdevResource r{};
+  CUgreenCtx green = nullptr;
+  if (st != nullptr && green_of != nullptr && green_has != nullptr && green_of(st, &green) == CUDA_SUCCESS && green != nullptr)
+    return green_has(green, &r, CU_DEV_RESOURCE_TYPE_SM) == CUDA_SUCCESS ? static_cast<int>(r.sm.smCount) : 0;
+  CUcontext c = nullptr;
+  if (current == nullptr || context_has == nullptr || current(&c) != CUDA_SUCCESS || c == nullptr || context_has(c, &r, CU_DEV_RESOURCE_TYPE_SM) != CUDA_SUCCESS) return sm_count();
+  return static_cast<int>(r.sm.smCount);
+}
+
+template <int H, int I, int SQ, int SG, int ROWS>
+static bool dr_one_fits() {
+  constexpr int smem = static_cast<int>(sizeof(DrShared<H, I, ROWS>));
+  int least = 1;
+  auto ask = [&](auto kern) {
+    int n = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, DR_THREADS, smem) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    least = least < n ? least : n;
+  };
+  ask(decode_rows_kernel<H, I, SQ, SG, ROWS, true>);
+  ask(decode_rows_kernel<H, I, SQ, SG, ROWS, false>);
+  return least >= 1;
+}
+// Whether a CTA can be resident on every multiprocessor at once, as the launch wants (without a device: as if so)
+static bool dr_resident(int form, int m, cudaStream_t st) {
+  int dev = 0, cooperative = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  if (cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || cooperative == 0) return false;
+  // Whether one fits a multiprocessor is asked once for each instance (a device that this library runs on is an sm_100a like another)
+  if (form == 1) {
+    static const bool two = dr_one_fits<2048, 6144, 8, 2, 2>(), four = dr_one_fits<2048, 6144, 8, 2, 4>();
+    if (!(m <= 2 ? two : four)) return false;
+  } else {
+    static const bool two = dr_one_fits<1024, 3072, 8, 4, 2>(), four = dr_one_fits<1024, 3072, 8, 4, 4>(), eight = dr_one_fits<1024, 3072, 8, 4, DR_MAX_ROWS>();
+    if (!(m <= 2 ? two : m <= 4 ? four : eight)) return false;
+  }
+  return dr_multiprocessors(st) >= sm_count();
+}
+
 }  // namespace b2
 
-extern "C" int b2tts_decode_rows_supported(int m, int hidden, int q_size, int kv_size, int intermediate) {
+namespace b2 {
+// The kernel for these rows and widths (dr_form), or 0
+static int dr_form_for(int m, int hidden, int q_size, int kv_size, int intermediate) {
   // Every CTA reads all rows of an activation, twice their size with the flags: what hand-overs take grows with the rows, what separate launches take hardly
   // does.  Separate launches / this, us: talker of 28 layers, contexts of 97 and of 400 tokens, 1 row 1241 1386 / 825 955, 2 rows 1268 1430 / 918 1059,
   // 4 rows 1321 1453 / 1047 1183, 5 rows 1343 1450 / 1280 1422, 6 rows 1322 1460 / 1342 1488, 8 rows 1333 1467 / 1410 1684; predictor of 5 layers with its head
   // 1 row 170 / 117, 4 rows 175 / 136, 6 rows 177 / 151, 8 rows 179 / 160.
-  const int form = b2::dr_form(hidden, q_size, kv_size, intermediate);
-  return form != 0 && m >= 1 && m <= (form == 1 ? 4 : b2::DR_MAX_ROWS);
+  const int form = dr_form(hidden, q_size, kv_size, intermediate);
+  return form != 0 && m >= 1 && m <= (form == 1 ? 4 : DR_MAX_ROWS) ? form : 0;
 }
-extern "C" int b2tts_decode_rows_taken(int m, int max_context_len, int hidden, int q_size, int kv_size, int intermediate) {
+}  // namespace b2
+
+extern "C" int b2tts_decode_rows_supported(int m, int hidden, int q_size, int kv_size, int intermediate) {
+  const int form = b2::dr_form_for(m, hidden, q_size, kv_size, intermediate);
+  return form != 0 && b2::dr_resident(form, m, nullptr);
+}
+extern "C" int b2tts_decode_rows_taken(int m, int max_context_len, int hidden, int q_size, int kv_size, int intermediate, void* stream) {
   using namespace b2;
   // ... and what attention takes grows with the contexts, by one chain of tiles after another where a CTA has more splits than it can walk at once (DR_PART_SPLITS).  So
   // the tables' room decides: no CTA has a second turn.  28 layers, contexts that fill the tables, separate launches / this in us, the last size that is taken and the first one
   // that is not: 2048 wide, 3 rows 1536 1435 / 1341, 2048 1475 / 1593; 4 rows 1024 1404 / 1292, 1536 1449 / 1527; 1024 wide, 4 rows 1024 1090 / 882, 1536 1142 / 1111; 6 rows
   // 768 1085 / 914, 1024 1105 / 1123; 8 rows 512 1064 / 910, 768 1094 / 1115.  Up to 2 rows have the CTAs for any context: 2048 wide 4000 1741 / 1522, 16000 3339 / 2789.
   // Tables of 16384 with 4 rows behind 16000 tokens 3382 / 4479, 1024 wide with 8 rows 3167 / 7012; the same behind 100 tokens 1278 / 1233 and 1014 / 920.
-  if (max_context_len <= 0 || !b2tts_decode_rows_supported(m, hidden, q_size, kv_size, intermediate)) return 0;
+  const int form = dr_form_for(m, hidden, q_size, kv_size, intermediate);
+  if (max_context_len <= 0 || form == 0) return 0;
   const int nsplit = fa_choose_nsplit(m, max_context_len);
-  return nsplit <= DR_PART_SPLITS * dr_parts(m, nsplit);
+  return nsplit <= DR_PART_SPLITS * dr_parts(m, nsplit) && dr_resident(form, m, static_cast<cudaStream_t>(stream));
 }
 extern "C" size_t b2tts_decode_rows_workspace_bytes(int hidden, int q_size, int kv_size, int intermediate) {
   return b2::dr_form(hidden, q_size, kv_size, intermediate) != 0 ? b2::dr_sizes(hidden, intermediate).total : 0;
@@ -806,8 +873,8 @@ extern "C" int b2tts_decode_rows_polls(const void* x, int64_t x_row_stride, void
   B2_REQUIRE(layers && num_layers >= 1 && num_layers <= DR_MAX_LAYERS, B2TTS_EUNSUPPORTED, "%s: 1..%d layers", what, DR_MAX_LAYERS);
   B2_REQUIRE(head_dim == DR_HD && num_kv_heads >= 1 && num_heads == DR_GROUP * num_kv_heads, B2TTS_EUNSUPPORTED,
              "%s: head_dim %d / heads %d / kv heads %d unsupported (128, heads = 2 x kv heads)", what, head_dim, num_heads, num_kv_heads);
-  const int Q = num_heads * head_dim, KV = num_kv_heads * head_dim, form = dr_form(hidden, Q, KV, intermediate);
-  B2_REQUIRE(b2tts_decode_rows_supported(m, hidden, Q, KV, intermediate), B2TTS_EUNSUPPORTED, "%s: %d rows of widths %d / %d / %d", what, m, hidden, Q, intermediate);
+  const int Q = num_heads * head_dim, KV = num_kv_heads * head_dim, form = dr_form_for(m, hidden, Q, KV, intermediate);
+  B2_REQUIRE(form != 0, B2TTS_EUNSUPPORTED, "%s: %d rows of widths %d / %d / %d", what, m, hidden, Q, intermediate);
   B2_REQUIRE(x && out && final_norm_weight && positions && inv_freq && slot_mapping && block_table && context_lens && workspace, B2TTS_EINVAL,
              "%s: null pointer", what);
   B2_REQUIRE(rounding == B2TTS_ROUND_EAGER || rounding == B2TTS_ROUND_FUSED, B2TTS_EINVAL, "%s: rounding %d", what, rounding);
