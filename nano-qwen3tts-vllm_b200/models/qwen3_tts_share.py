@@ -51,8 +51,8 @@ FUSED_NORM_MIN_ROWS = int(os.environ.get("B2TTS_FUSED_NORM_MIN_ROWS", "9"))
 # (every hand-over between phases costs a gpu-scope release + an L2 poll, ~2.5 us, 7 per layer)
 DATAFLOW_STACK = os.environ.get("B2TTS_DATAFLOW_STACK", "0") != "0"
 # decode steps of up to so many rows (fewer where csrc/decode_rows.cu says so) as ONE persistent launch of the whole stack, where a runner has given it a workspace:
-# the same bits as the separate launches
-DECODE_ROWS_MAX = 8
+# the same bits as the separate launches.  0: never
+DECODE_ROWS_MAX = int(os.environ.get("B2TTS_DECODE_ROWS_MAX", "8"))
 
 
 class Qwen3TTSAttention(nn.Module):
@@ -320,9 +320,13 @@ class DecoderStack(nn.Module):
         return ctx.max_context_len or ctx.block_tables.shape[1] * self.layers[0].self_attn.attn.k_cache.shape[1]
 
     def _takes_rows(self, x: torch.Tensor) -> bool:
-        ctx = get_context()
-        return (getattr(self, "_rows_ws", None) is not None and not ctx.is_prefill and ctx.block_tables is not None and x.dim() == 2
-                and 1 <= x.shape[0] <= min(self._rows_most, DECODE_ROWS_MAX) and x.dtype == torch.bfloat16
+        """Whether the persistent step takes these rows.  It stands for separate launches with the attention of one launch and norms of their own: the switches that lead
+        to others lead there still."""
+        if getattr(self, "_rows_ws", None) is None or x.dim() != 2 or x.dtype != torch.bfloat16:
+            return False
+        ctx, m = get_context(), x.shape[0]
+        return (not ctx.is_prefill and ctx.block_tables is not None and 1 <= m <= min(self._rows_most, DECODE_ROWS_MAX, GEMM_NATIVE_MAX_M)
+                and FUSED_DECODE_ATTENTION and not GEMM_CHAIN and not FUSED_NORM_MIN_ROWS <= m <= FUSED_NORM_MAX_ROWS
                 and (not self._rows_where_faster or nat.decode_rows_taken(x.shape[0], self._max_context(), *self._widths())))
 
     def _run_rows(self, x: torch.Tensor, positions: torch.Tensor) -> torch.Tensor:
