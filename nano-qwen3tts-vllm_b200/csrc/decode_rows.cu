@@ -22,7 +22,8 @@
 //
 // Why no word is overwritten before its readers are done: a phase's outputs are complete only when all its readers have read (each sum needs
 // all slices), and a phase that reads whole rows waits for all outputs of the phase before.  So who writes a buffer again, a layer later,
-// has waited for something that followed the last read of it.  A CTA that has no tile in a phase does not read that phase's input.
+// has waited for something that followed the last read of it.  A CTA that has no tile in a phase does not read that phase's input; so every CTA has to have tiles of
+// gate_up (dr_form() asks for it): with rows that are all padding nobody waits for qkv, and without gate_up a CTA would wait for nothing between two layers.
 // All waits are bounded; a wait that runs out is counted (waits.cuh), and the launch goes on to its end with what it has: who has given up waits for no more words, but
 // reads, writes and meets the others of its CTA as ever, so that other CTAs find their words, every copy its readers and the next launch everything as it should be.
 //
@@ -743,6 +744,7 @@ static int dr_form(int hidden, int q, int kv, int inter) {
            (tiles + 3) / 4 + 1 <= 32 / s;
   };
   const int width = q + 2 * kv;
+  if ((2 * inter / 8 + dr_group(2 * inter / 8, n) - 1) / dr_group(2 * inter / 8, n) < n) return 0;        // tiles of gate_up for every CTA, see the head of this file
   if (!fits(width, hidden, 8) || !fits(hidden, q, 8) || !fits(hidden, inter, 8)) return 0;
   if (hidden == 2048 && inter == 6144 && fits(2 * inter, hidden, 2)) return 1;
   if (hidden == 1024 && inter == 3072 && fits(2 * inter, hidden, 4)) return 2;
