@@ -48,6 +48,7 @@ constexpr int DR_UNIT = 1024;                      // 8 features x 64 columns, a
 constexpr int DR_STAGES = 16;                      // stages in flight at most
 constexpr int DR_SUMS = 32;                        // (tile, slice) sums of a CTA's phase
 constexpr int DR_MAX_TILES = 4;                    // tiles of a warp in a phase
+constexpr unsigned DR_LAST_BASE = 0xffffffffu - 2 * DR_MAX_LAYERS * 8;      // behind a later one the numbers of a step might pass 2^32
 enum { DR_E_QKV = 1, DR_E_ATT = 2, DR_E_RES1 = 3, DR_E_ACT = 4, DR_E_RES2 = 5, DR_E_PART = 6, DR_E_LAYER = 8 };
 
 __device__ int g_rows_timeouts = 0;                // see waits.cuh
@@ -82,7 +83,7 @@ struct DrParams {
   int polls;                                             // tries after which a wait for a word gives up
   int nsplit, max_parts;                                 // splits of a context; CTAs a unit may take
   unsigned* sync;                                        // [0] the number of the last phase, [1] CTAs that are done
-  uint64_t *qkv, *att, *res1, *act, *res2, *part;
+  uint64_t *qkv, *att, *res1, *act, *res2, *part, *words_end;
   int* waits;                                            // host word of waits that ran out (or null)
   DrLayer layer[DR_MAX_LAYERS];
 };
@@ -708,10 +709,20 @@ decode_rows_kernel(const __grid_constant__ DrParams p) {
       dr_report(p.waits);
     }
     __threadfence();
-    if (atomicAdd(p.sync + 1, 1u) == gridDim.x - 1) {
+    const bool last_out = atomicAdd(p.sync + 1, 1u) == gridDim.x - 1;
+    if (last_out) {
       p.sync[1] = 0;
-      p.sync[0] = base + p.num_layers * DR_E_LAYER;
+      p.sync[0] = base > DR_LAST_BASE ? 0 : base + p.num_layers * DR_E_LAYER;
     }
+    sm.plan.unit.L = last_out;
+    __threadfence();
+  }
+  // Numbers would come again after 2^32 / 8 layers (four hours of steps), and words of rows that were not used meanwhile would be taken for theirs.  Before that the last
+  // CTA writes zeros over all words, 5 MB, and numbers start anew.
+  if (base > DR_LAST_BASE) {
+    dr_sync();
+    if (sm.plan.unit.L)
+      for (uint64_t* at = p.qkv + tid; at < p.words_end; at += DR_READERS) *at = 0;
   }
 }
 
@@ -918,7 +929,7 @@ extern "C" int b2tts_decode_rows_polls(const void* x, int64_t x_row_stride, void
   uint8_t* w = static_cast<uint8_t*>(workspace);
   auto take = [&w](size_t n) { uint64_t* at = reinterpret_cast<uint64_t*>(w); w += n; return at; };
   p.sync = reinterpret_cast<unsigned*>(take(256));
-  p.qkv = take(z.qkv); p.att = take(z.att); p.res1 = take(z.res); p.res2 = take(z.res); p.act = take(z.act); p.part = take(z.part);
+  p.qkv = take(z.qkv); p.att = take(z.att); p.res1 = take(z.res); p.res2 = take(z.res); p.act = take(z.act); p.part = take(z.part); p.words_end = take(0);
   p.waits = wait_word(WAITS_ROWS);
   p.polls = polls;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
