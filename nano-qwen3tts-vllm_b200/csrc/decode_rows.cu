@@ -893,7 +893,8 @@ extern "C" int b2tts_decode_rows_polls(const void* x, int64_t x_row_stride, void
   B2_REQUIRE(rounding == B2TTS_ROUND_EAGER || rounding == B2TTS_ROUND_FUSED, B2TTS_EINVAL, "%s: rounding %d", what, rounding);
   B2_REQUIRE(page_size > 0 && bt_stride > 0 && max_context_len > 0, B2TTS_EINVAL, "%s: page_size=%d bt_stride=%d max_context_len=%d", what, page_size, bt_stride,
              max_context_len);
-  B2_REQUIRE((page_size & (page_size - 1)) == 0, B2TTS_EUNSUPPORTED, "%s: pages of %d tokens (a power of two)", what, page_size);
+  B2_REQUIRE((page_size & (page_size - 1)) == 0 && page_size % FA_TILE == 0, B2TTS_EUNSUPPORTED, "%s: pages of %d tokens (a power of two, %d or more)", what, page_size,
+             FA_TILE);
   auto word = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 3u) == 0; };
   B2_REQUIRE(word(x) && word(out) && word(final_norm_weight) && x_row_stride % 2 == 0 && out_row_stride % 2 == 0 &&
                  (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0, B2TTS_EALIGN, "%s: rows must be 4-byte, the workspace 256-byte aligned", what);

@@ -307,7 +307,7 @@ class DecoderStack(nn.Module):
         c, rope, widths = self.config, self.layers[0].self_attn.rotary_emb, self._widths()
         page = self.layers[0].self_attn.attn.k_cache.shape[1]
         self._rows_most = max([m for m in range(1, DECODE_ROWS_MAX + 1) if nat.decode_rows_supported(m, *widths)], default=0)
-        if len(self.layers) > nat.DECODE_ROWS_MAX_LAYERS or c.head_dim != 128 or rope.inv_freq.numel() != 64 or page & (page - 1):
+        if len(self.layers) > nat.DECODE_ROWS_MAX_LAYERS or c.head_dim != 128 or rope.inv_freq.numel() != 64 or page % 8 or page & (page - 1):
             self._rows_most = 0
         self._rows_ws = nat.decode_rows_workspace(*widths, self.norm.weight.device) if self._rows_most else None
 
