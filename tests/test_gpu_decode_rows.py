@@ -98,7 +98,9 @@ def test_contexts_around_tiles_splits_and_parts(lens):
 
 
 def test_replayed_from_a_graph():
-    """Captured once with one workspace: every replay gives the eager result, and launches of other row counts between them do no harm."""
+    """Captured once with one workspace: every replay gives the eager result, and launches of other row counts between them do no harm.  All of them are the
+    persistent step, with the results of the separate launches."""
+    from nano_qwen3tts_vllm_b200 import _native as nat
     from nano_qwen3tts_vllm_b200.utils.context import reset_context, set_context
     stack = _stack(1024, 3072, 5, False, 0)
     ctx, bt, slots, pos, npages, width = _layout(8, 120, 3)
@@ -108,17 +110,24 @@ def test_replayed_from_a_graph():
     stack.bind_decode_rows()
     x = torch.randn(8, 1024, device="cuda").to(BF16)
 
-    def step(n):
+    def step(n, rows=True):
         set_context(False, slot_mapping=slots[:n], context_lens=ctx[:n], block_tables=bt[:n], max_context_len=width * PAGE)
+        assert stack._takes_rows(x[:n]) == rows
         return stack.run_layers(x[:n], pos[:n])
     try:
+        kept, stack._rows_ws = stack._rows_ws, None
+        for layer in stack.layers:
+            layer.self_attn.attn.fused_workspace = nat.fused_decode_attn_workspace(8, 16, 128, width * PAGE, "cuda")
+        separate = {n: step(n, False).clone() for n in (1, 2, 3, 8)}
+        stack._rows_ws = kept
         eager = step(8).clone()
+        assert torch.equal(eager, separate[8])
         torch.cuda.synchronize()
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
             out = step(8)
         for n in (1, 3, 8, 2):
-            step(n)
+            assert torch.equal(step(n), separate[n])
             graph.replay()
             torch.cuda.synchronize()
             assert torch.equal(out, eager)
