@@ -4,7 +4,7 @@
 // A step of a few rows is a stream of weights (100 MB a layer of the 1.7B talker, 15.4 us at the copy rate) through a chain of dependent phases.  As
 // separate launches the chain costs 44 us a layer: each starts its stream anew and pays drain, boundary and first fetch.  Here one CTA per SM lives for the
 // whole step:
-//   * a warp of its own copies the CTA's weights - tiles of 8 features, slices of K, layer after layer - into a ring of 96 to 160 KB and waits for nobody but its
+//   * a warp of its own copies the CTA's weights - tiles of 8 features, slices of K, layer after layer - into a ring of 144 or 160 KB and waits for nobody but its
 //     readers, so that what a phase needs is in shared memory when its input arrives and HBM stays busy while the phases hand over.  A stage is 64
 //     or 128 columns of every slice; its copies take up to four tiles at once: copies of 1 KB come in at 33 KB/us a multiprocessor, those of 2 KB and more at the
 //     rate of HBM (49);
@@ -13,7 +13,7 @@
 //     the tensor cores' rate does not matter;
 //   * hand-overs carry their own flags: every 8-byte word of an activation is two bf16 and the number of the phase that wrote it.  A reader polls the data
 //     itself: one L2 trip from store to use, no fence, no counter, no grid barrier (2 to 2.5 us a hand-over in decoder_stack.cu).
-// Attention is a phase of its own: a unit (row, key head) per CTA, a warp per query head and split of the context; contexts of more than 8 splits take several
+// Attention is a phase of its own: a unit (row, key head) per CTA, a warp per query head and split of the context; contexts of more than 4 splits take several
 // CTAs, whose partial sums meet in the first one.
 //
 // Every sum is formed in the order of the separate launches, so that a row has the same bits on either path: products by chains of 16-wide MMAs over
@@ -28,8 +28,9 @@
 // reads, writes and meets the others of its CTA as ever, so that other CTAs find their words, every copy its readers and the next launch everything as it should be.
 //
 // Bound: a layer of the talker takes 28 us for one row, 13.9 of them the stream at HBM's rate; hand-overs of 1.2 to 2.5 us, five a layer, are the rest (a word
-// takes about 0.8 us from store to load while L2 feeds the stream), with 2 us of a tile's softmax after another in attention.  28 layers, one row, us: 1241
-// as launches, 931 with slices of 16 warps in copies of 1 KB, 825 so; behind 1300 and 2700 tokens 1588 1767 / 1136 1348, 4 rows 1696 1923 / 1572 1953.
+// takes about 0.8 us from store to load while L2 feeds the stream), with 2 us of a tile's softmax after another in attention.  28 layers of the talker and its head, one row
+// behind 97 tokens: 1251 us as launches, 812 so (slices of 16 warps in copies of 1 KB: 931).  Tables with room for more tokens cut a context into more splits and CTAs, whatever
+// its length: the stack alone, one row behind 100 tokens in tables of 4096 1240 / 1020, behind 2700 1535 / 1250; 4 rows see b2tts_decode_rows_taken().
 // What did not do: cp.async of the warps themselves (25 to 40 cycles a 512-byte instruction, 1610 us), 16 warps with one tile each (four times the
 // instructions a byte), projections of 5 and more rows (every CTA reads every row, with flags).
 #include <type_traits>
@@ -167,8 +168,7 @@ __device__ __forceinline__ void dr_sync() { asm volatile("bar.sync 1, %0;" ::"n"
 // A unit of attention: a row's key head, which of the CTAs that have it this is, the context, and the CTA's splits of it
 struct DrUnit { int row, head, part, L, s0, s1; };
 
-// The arithmetic of fused_decode_attn_kernel, a warp a query head of a split; returns whether no wait ran out.  Out of line: the projections' loops keep their
-// registers.
+// The arithmetic of fused_decode_attn_kernel, a warp a query head of a split; returns whether no wait ran out.
 template <bool EAGER>
 __device__ __forceinline__ bool dr_attend(const DrParams& p, const DrLayer& y, uint32_t e0, const DrUnit& a, __nv_bfloat16* q_s, const uint4* trig_s, const int* pages, uint8_t* x_s,
                                        bool alive) {
@@ -478,7 +478,7 @@ decode_rows_kernel(const __grid_constant__ DrParams p) {
     return s;
   };
   auto rstd_of = [&](float s) -> float { const float var = s / static_cast<float>(H) + p.eps; return EAGER ? 1.0f / sqrtf(var) : rsqrtf(var); };
-  // Normed rows: thread tid has vector tid % VECS of rows tid / VECS, + 512 / VECS, ...  Sums: a thread's eight squares in order, the lanes of a warp, the
+  // Normed rows: thread tid has vector tid % VECS of rows tid / VECS, + 256 / VECS, ...  Sums: a thread's eight squares in order, the lanes of a warp, the
   // warps of a row.
   auto norm_rows = [&](bool first, const uint64_t* res, uint32_t flag, const __nv_bfloat16* w) {
     constexpr int RP = DR_READERS / VECS, PASSES = (ROWS + RP - 1) / RP, RW = VECS / 32;        // rows a pass; warps a row

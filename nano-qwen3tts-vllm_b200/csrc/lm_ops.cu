@@ -75,7 +75,12 @@ __device__ __forceinline__ void gain_norm_kept(const float (&v)[KEEP][4], T* hr,
   float ssq = 0.f;
 #pragma unroll
   for (int i = 0; i < 4 * KEEP; ++i) if (static_cast<int>(threadIdx.x) + i * ROW_THREADS < cols) ssq += xs[i * ROW_THREADS] * xs[i * ROW_THREADS];
-  const float tot = block_sum(ssq, red);
+  // as block_sum(), with the last sum formed by every warp instead of handed out by the first
+  ssq = warp_sum(ssq);
+  const int lane = threadIdx.x & 31;
+  if (lane == 0) red[threadIdx.x >> 5] = ssq;
+  __syncthreads();
+  const float tot = warp_sum(lane < ROW_THREADS / 32 ? red[lane] : 0.f);
   const float inv = 1.0f / sqrtf(tot / static_cast<float>(cols) + eps);
   const float g = gain[0];
 #pragma unroll
