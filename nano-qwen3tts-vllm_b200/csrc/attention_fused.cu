@@ -476,6 +476,8 @@ fused_decode_attn_kernel(const FusedAttnParams p) {
 // rows are read straight from the paged cache, two 8-token tiles per round trip, and the new token never leaves
 // the warp.  Arithmetic, lane mapping and summation order are those of fused_decode_attn_kernel with nsplit == 1
 // (GROUP 2, 1-D RoPE), so outputs and K / V cache bytes are bit-identical.
+// One product after another: pairs gave nothing for a tile or two (201 rows of 17 tokens 10.8 us) and cost a third for more (300 rows of 50 29.6 -> 41.1, 200 of 200 in tables
+// said to have room for 60 63 -> 101).
 constexpr int FS_WARPS = 4;
 constexpr int FS_MAX_CTX = 64;
 
@@ -598,22 +600,21 @@ fused_decode_attn_small_kernel(const FusedAttnParams p, int rows) {
     }
   }
   __syncwarp();
-  uint64_t qv[GROUP][8];
+  float qv[GROUP][16];
 #pragma unroll
   for (int h = 0; h < GROUP; ++h) {
     const __nv_bfloat16* qp = q_s + h * FA_HD;
-    fa_pairs8(*reinterpret_cast<const uint4*>(qp + 8 * j), qv[h]);
-    fa_pairs8(*reinterpret_cast<const uint4*>(qp + 64 + 8 * j), qv[h] + 4);
+    fa_unpack8(*reinterpret_cast<const uint4*>(qp + 8 * j), qv[h]);
+    fa_unpack8(*reinterpret_cast<const uint4*>(qp + 64 + 8 * j), qv[h] + 8);
 #pragma unroll
-    for (int d = 0; d < 8; ++d) qv[h][d] = f2_mul(qv[h][d], f2_pack(p.scale_log2, p.scale_log2));
+    for (int d = 0; d < 16; ++d) qv[h][d] *= p.scale_log2;
   }
-  float m[GROUP], l[GROUP];
-  uint64_t acc2[GROUP][8];                                // weighted sums of values, in pairs
+  float m[GROUP], l[GROUP], acc[GROUP][16];
 #pragma unroll
   for (int h = 0; h < GROUP; ++h) {
     m[h] = -INFINITY; l[h] = 0.f;
 #pragma unroll
-    for (int d = 0; d < 8; ++d) acc2[h][d] = 0;
+    for (int d = 0; d < 16; ++d) acc[h][d] = 0.f;
   }
   for (int i0 = 0; i0 < n_tiles; i0 += 2) {
 #pragma unroll
@@ -628,17 +629,23 @@ fused_decode_attn_small_kernel(const FusedAttnParams p, int rows) {
         const int tok = it * 4 + g;
         const bool valid = tok < ntok;
         isnew[it] = tok0 + (valid ? tok : 0) == L - 1;
-        uint64_t kf[8];
+        float kf[16];
         if (isnew[it]) {
-          fa_pairs8(*reinterpret_cast<const uint4*>(kn_s + 8 * j), kf);
-          fa_pairs8(*reinterpret_cast<const uint4*>(kn_s + 64 + 8 * j), kf + 4);
+          fa_unpack8(*reinterpret_cast<const uint4*>(kn_s + 8 * j), kf);
+          fa_unpack8(*reinterpret_cast<const uint4*>(kn_s + 64 + 8 * j), kf + 8);
         } else {
-          fa_pairs8(kbuf[u][it][0], kf);
-          fa_pairs8(kbuf[u][it][1], kf + 4);
+          fa_unpack8(kbuf[u][it][0], kf);
+          fa_unpack8(kbuf[u][it][1], kf + 8);
         }
 #pragma unroll
         for (int h = 0; h < GROUP; ++h) {
-          float dot = fa_dot16<true>(qv[h], kf);
+          float d0 = 0.f, d1 = 0.f;
+#pragma unroll
+          for (int d = 0; d < 16; d += 2) {
+            d0 = fmaf(qv[h][d], kf[d], d0);
+            d1 = fmaf(qv[h][d + 1], kf[d + 1], d1);
+          }
+          float dot = d0 + d1;
           dot += __shfl_xor_sync(0xffffffffu, dot, 1);
           dot += __shfl_xor_sync(0xffffffffu, dot, 2);
           dot += __shfl_xor_sync(0xffffffffu, dot, 4);
@@ -664,31 +671,28 @@ fused_decode_attn_small_kernel(const FusedAttnParams p, int rows) {
         }
         l[h] = fmaf(l[h], alpha[h], ps);
 #pragma unroll
-        for (int d = 0; d < 8; ++d) acc2[h][d] = f2_mul(acc2[h][d], f2_pack(alpha[h], alpha[h]));
+        for (int d = 0; d < 16; ++d) acc[h][d] *= alpha[h];
       }
 #pragma unroll
       for (int it = 0; it < FA_TILE / 4; ++it) {
-        uint64_t vf[8];
+        float vf[16];
         if (isnew[it]) {
-          fa_pairs8(*reinterpret_cast<const uint4*>(vn_s + 8 * j), vf);
-          fa_pairs8(*reinterpret_cast<const uint4*>(vn_s + 64 + 8 * j), vf + 4);
+          fa_unpack8(*reinterpret_cast<const uint4*>(vn_s + 8 * j), vf);
+          fa_unpack8(*reinterpret_cast<const uint4*>(vn_s + 64 + 8 * j), vf + 8);
         } else {
-          fa_pairs8(vbuf[u][it][0], vf);
-          fa_pairs8(vbuf[u][it][1], vf + 4);
+          fa_unpack8(vbuf[u][it][0], vf);
+          fa_unpack8(vbuf[u][it][1], vf + 8);
         }
 #pragma unroll
         for (int h = 0; h < GROUP; ++h)
 #pragma unroll
-          for (int d = 0; d < 8; ++d) acc2[h][d] = f2_fma(f2_pack(s[it][h], s[it][h]), vf[d], acc2[h][d]);
+          for (int d = 0; d < 16; ++d) acc[h][d] = fmaf(s[it][h], vf[d], acc[h][d]);
       }
     }
     if (i0 + 2 < n_tiles) load_pair(i0 + 2);
   }
-  float acc[GROUP][16];
 #pragma unroll
   for (int h = 0; h < GROUP; ++h) {
-#pragma unroll
-    for (int d = 0; d < 8; ++d) f2_unpack(acc2[h][d], acc[h][2 * d], acc[h][2 * d + 1]);
     l[h] += __shfl_xor_sync(0xffffffffu, l[h], 8);
     l[h] += __shfl_xor_sync(0xffffffffu, l[h], 16);
 #pragma unroll
