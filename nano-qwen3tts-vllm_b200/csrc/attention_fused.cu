@@ -59,13 +59,65 @@ __device__ __forceinline__ uint4 fa_pack8(const float* f) {
   return r;
 }
 
-template <int GROUP, bool EAGER, bool SPLIT>
-__global__ void __launch_bounds__(288, 2)
+// The splits of a sequence in order, by its last CTA to finish.  Not inline: its registers would be taken from the loop over tiles (32 rows of 2000 tokens, two query and two key
+// heads 28.6 us inline, 19.2 so; 8 and 2 heads 41, 33).
+template <int GROUP>
+__device__ __noinline__ void fa_fold(const float* part_ml, const float* part_acc, __nv_bfloat16* out, int nsplit, int num_heads, int row, int head0) {
+  const int lane = threadIdx.x & 31;
+  // warp w folds heads head0 .. head0+GROUP-1; lane owns 4 consecutive dims.  Lane s asks for split s's maximum and sum (at most 32 splits), and the partials of
+  // four splits of all heads are asked for at once: a split after another was up to three dependent round trips for each: 64 rows of 40
+  // tokens 10.4 -> 8.5 us, of 200 16.1 -> 14.7, 16 rows of 700 22.3 -> 15.9, 4 of 2000 25.7 -> 18.4 (16 query and 8 key heads).
+  float top[GROUP], sum[GROUP];
+#pragma unroll
+  for (int h = 0; h < GROUP; ++h) {
+    const int64_t at = ((int64_t)row * nsplit + lane) * num_heads + head0 + h;
+    top[h] = lane < nsplit ? __ldcg(part_ml + at * 2) : -INFINITY;
+    sum[h] = lane < nsplit ? __ldcg(part_ml + at * 2 + 1) : 0.f;
+  }
+  float4 num[GROUP];
+  float den[GROUP];
+#pragma unroll
+  for (int h = 0; h < GROUP; ++h) { num[h] = make_float4(0.f, 0.f, 0.f, 0.f); den[h] = 0.f; }
+  for (int s0 = 0; s0 < nsplit; s0 += 4) {
+    float4 a[4][GROUP];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int h = 0; h < GROUP; ++h) {
+        const int64_t idx = ((int64_t)row * nsplit + s0 + u) * num_heads + head0 + h;
+        a[u][h] = s0 + u < nsplit ? __ldcg(reinterpret_cast<const float4*>(part_acc + idx * FA_HD) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    if (s0 == 0) {
+#pragma unroll
+      for (int h = 0; h < GROUP; ++h) top[h] = fa_exp2(top[h] - warp_max(top[h]));          // the splits' weights
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int h = 0; h < GROUP; ++h) {
+        const float w = __shfl_sync(0xffffffffu, top[h], (s0 + u) & 31), ls = __shfl_sync(0xffffffffu, sum[h], (s0 + u) & 31);
+        if (s0 + u < nsplit && ls > 0.f) {
+          num[h].x = fmaf(w, a[u][h].x, num[h].x); num[h].y = fmaf(w, a[u][h].y, num[h].y);
+          num[h].z = fmaf(w, a[u][h].z, num[h].z); num[h].w = fmaf(w, a[u][h].w, num[h].w);
+          den[h] = fmaf(w, ls, den[h]);
+        }
+      }
+  }
+#pragma unroll
+  for (int h = 0; h < GROUP; ++h) {
+    const float inv = den[h] > 0.f ? 1.f / den[h] : 0.f;
+    uint2 o;
+    o.x = pack_bf16(num[h].x * inv, num[h].y * inv);
+    o.y = pack_bf16(num[h].z * inv, num[h].w * inv);
+    stg_v2(out + ((int64_t)row * num_heads + head0 + h) * FA_HD + 4 * lane, o);
+  }
+}
+
+// HEADS: as many key heads at most, see fa_pick()
+template <int GROUP, bool EAGER, bool SPLIT, int HEADS>
+__global__ void __launch_bounds__(GROUP == 4 ? 32 * (HEADS + 1) : 288, GROUP < 4 || HEADS > 4 ? 2 : HEADS > 2 ? 3 : 4)
 fused_decode_attn_kernel(const FusedAttnParams p) {
-  // Two heads a key head without splits: many tiles a CTA, and a turn of the ring without branches (200 rows of 200 tokens 32.5 -> 30.2 us); with splits the longer
-  // code costs more than it gives (64 rows of 40 tokens 8.4, unrolled 10.1), with four heads it spills.
-  constexpr int UNROLL = GROUP == 2 && !SPLIT ? FA_NSTAGE : 1;
-  constexpr bool PACKED = GROUP < 4;                      // pairs of four heads spill: 200 rows of 200 tokens 104 us one by one, 113 packed
+  constexpr int UNROLL = GROUP == 2 && (!SPLIT || HEADS <= 4) ? FA_NSTAGE : 1;
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const int kvh = p.num_kv_heads;
   const int kv_dim = kvh * FA_HD;
@@ -247,35 +299,15 @@ fused_decode_attn_kernel(const FusedAttnParams p) {
   }
   asm volatile("bar.sync 1, %0;" :: "r"(kvh * 32) : "memory");      // the consumer warps only
 
-  // ---- this warp's q heads from shared memory, pre-scaled for exp2
-  uint64_t qv[GROUP][8];
-#pragma unroll
-  for (int h = 0; h < GROUP; ++h) {
-    const __nv_bfloat16* qp = q_s + (head0 + h) * FA_HD;
-    fa_pairs8(*reinterpret_cast<const uint4*>(qp + 8 * j), qv[h]);
-    fa_pairs8(*reinterpret_cast<const uint4*>(qp + 64 + 8 * j), qv[h] + 4);
-#pragma unroll
-    for (int d = 0; d < 8; ++d) qv[h][d] = f2_mul(qv[h][d], f2_pack(p.scale_log2, p.scale_log2));
-  }
-
-  float m[GROUP], l[GROUP];
-  uint64_t acc2[GROUP][8];                                // weighted sums of values, in pairs
-#pragma unroll
-  for (int h = 0; h < GROUP; ++h) {
-    m[h] = -INFINITY; l[h] = 0.f;
-#pragma unroll
-    for (int d = 0; d < 8; ++d) acc2[h][d] = 0;
-  }
-
-#pragma unroll UNROLL
-  for (int i = 0; i < my_tiles; ++i) {
+  // a tile in its stage, with the new token in its place: tokens, keys and values of this warp's key head
+  auto enter = [&](int i, __nv_bfloat16*& kt, __nv_bfloat16*& vt) -> int {
     const int stage = i % FA_NSTAGE;
     const uint32_t ph = (i / FA_NSTAGE) & 1;
     const int tok0 = (t_begin + i) * FA_TILE;
     const int ntok = min(FA_TILE, L - tok0);
     mbar_wait(full_bar + stage, ph);
-    __nv_bfloat16* kt = Ks + stage * stage_elems + warp * FA_HD;
-    __nv_bfloat16* vt = Vs + stage * stage_elems + warp * FA_HD;
+    kt = Ks + stage * stage_elems + warp * FA_HD;
+    vt = Vs + stage * stage_elems + warp * FA_HD;
     if (writer && i == my_tiles - 1) {
       // the bulk copy may have read the new token's row before or after the global store above:
       // replace this head's slice of that row with the register copy
@@ -291,82 +323,195 @@ fused_decode_attn_kernel(const FusedAttnParams p) {
       }
       __syncwarp();
     }
+    return ntok;
+  };
+  auto leave = [&](int i) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(empty_bar + i % FA_NSTAGE);
+  };
 
-    // Keys of all token slots, their products, then the values on their way while the products are summed over lanes and turned into weights
-    float s[FA_TILE / 4][GROUP];
-    uint4 raw[FA_TILE / 4][2];
-    int at[FA_TILE / 4];
+  // ---- this warp's q heads from shared memory, pre-scaled for exp2, against its tiles
+  float m[GROUP], l[GROUP], acc[GROUP][16];
+  if constexpr (GROUP < 4) {
+    uint64_t qv[GROUP][8];
 #pragma unroll
-    for (int it = 0; it < FA_TILE / 4; ++it) {
-      const int tok = it * 4 + g;
-      at[it] = (tok < ntok ? tok : 0) * kv_dim + 8 * j;
-      raw[it][0] = *reinterpret_cast<const uint4*>(kt + at[it]);
-      raw[it][1] = *reinterpret_cast<const uint4*>(kt + at[it] + 64);
+    for (int h = 0; h < GROUP; ++h) {
+      const __nv_bfloat16* qp = q_s + (head0 + h) * FA_HD;
+      fa_pairs8(*reinterpret_cast<const uint4*>(qp + 8 * j), qv[h]);
+      fa_pairs8(*reinterpret_cast<const uint4*>(qp + 64 + 8 * j), qv[h] + 4);
+#pragma unroll
+      for (int d = 0; d < 8; ++d) qv[h][d] = f2_mul(qv[h][d], f2_pack(p.scale_log2, p.scale_log2));
     }
+
+    uint64_t acc2[GROUP][8];                                // weighted sums of values, in pairs
 #pragma unroll
-    for (int it = 0; it < FA_TILE / 4; ++it) {
-      uint64_t kf[8];
-      fa_pairs8(raw[it][0], kf);
-      fa_pairs8(raw[it][1], kf + 4);
+    for (int h = 0; h < GROUP; ++h) {
+      m[h] = -INFINITY; l[h] = 0.f;
 #pragma unroll
-      for (int h = 0; h < GROUP; ++h) s[it][h] = fa_dot16<PACKED>(qv[h], kf);
+      for (int d = 0; d < 8; ++d) acc2[h][d] = 0;
     }
+
+#pragma unroll UNROLL
+    for (int i = 0; i < my_tiles; ++i) {
+      __nv_bfloat16 *kt, *vt;
+      const int ntok = enter(i, kt, vt);
+      // Keys of all token slots, their products, then the values on their way while the products are summed over lanes and turned into weights
+      float s[FA_TILE / 4][GROUP];
+      uint4 raw[FA_TILE / 4][2];
+      int at[FA_TILE / 4];
 #pragma unroll
-    for (int it = 0; it < FA_TILE / 4; ++it) {
-      raw[it][0] = *reinterpret_cast<const uint4*>(vt + at[it]);
-      raw[it][1] = *reinterpret_cast<const uint4*>(vt + at[it] + 64);
-    }
+      for (int it = 0; it < FA_TILE / 4; ++it) {
+        const int tok = it * 4 + g;
+        at[it] = (tok < ntok ? tok : 0) * kv_dim + 8 * j;
+        raw[it][0] = *reinterpret_cast<const uint4*>(kt + at[it]);
+        raw[it][1] = *reinterpret_cast<const uint4*>(kt + at[it] + 64);
+      }
 #pragma unroll
-    for (int o = 1; o < 8; o <<= 1)
+      for (int it = 0; it < FA_TILE / 4; ++it) {
+        uint64_t kf[8];
+        fa_pairs8(raw[it][0], kf);
+        fa_pairs8(raw[it][1], kf + 4);
+#pragma unroll
+        for (int h = 0; h < GROUP; ++h) s[it][h] = fa_dot16(qv[h], kf);
+      }
+#pragma unroll
+      for (int it = 0; it < FA_TILE / 4; ++it) {
+        raw[it][0] = *reinterpret_cast<const uint4*>(vt + at[it]);
+        raw[it][1] = *reinterpret_cast<const uint4*>(vt + at[it] + 64);
+      }
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+        for (int it = 0; it < FA_TILE / 4; ++it)
+#pragma unroll
+          for (int h = 0; h < GROUP; ++h) s[it][h] += __shfl_xor_sync(0xffffffffu, s[it][h], o);
 #pragma unroll
       for (int it = 0; it < FA_TILE / 4; ++it)
 #pragma unroll
-        for (int h = 0; h < GROUP; ++h) s[it][h] += __shfl_xor_sync(0xffffffffu, s[it][h], o);
+        for (int h = 0; h < GROUP; ++h) s[it][h] = it * 4 + g < ntok ? s[it][h] : -INFINITY;
+      float alpha[GROUP];
 #pragma unroll
-    for (int it = 0; it < FA_TILE / 4; ++it)
+      for (int h = 0; h < GROUP; ++h) {
+        float mt = s[0][h];
 #pragma unroll
-      for (int h = 0; h < GROUP; ++h) s[it][h] = it * 4 + g < ntok ? s[it][h] : -INFINITY;
-    float alpha[GROUP];
+        for (int it = 1; it < FA_TILE / 4; ++it) mt = fmaxf(mt, s[it][h]);
+        mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, 8));
+        mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, 16));
+        const float mn = fmaxf(m[h], mt);
+        alpha[h] = fa_exp2(m[h] - mn);
+        m[h] = mn;
+        float ps = 0.f;
 #pragma unroll
-    for (int h = 0; h < GROUP; ++h) {
-      float mt = s[0][h];
+        for (int it = 0; it < FA_TILE / 4; ++it) {
+          s[it][h] = fa_exp2(s[it][h] - mn);
+          ps += s[it][h];
+        }
+        l[h] = fmaf(l[h], alpha[h], ps);
 #pragma unroll
-      for (int it = 1; it < FA_TILE / 4; ++it) mt = fmaxf(mt, s[it][h]);
-      mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, 8));
-      mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, 16));
-      const float mn = fmaxf(m[h], mt);
-      alpha[h] = fa_exp2(m[h] - mn);
-      m[h] = mn;
-      float ps = 0.f;
+        for (int d = 0; d < 8; ++d) acc2[h][d] = f2_mul(acc2[h][d], f2_pack(alpha[h], alpha[h]));
+      }
 #pragma unroll
       for (int it = 0; it < FA_TILE / 4; ++it) {
-        s[it][h] = fa_exp2(s[it][h] - mn);
-        ps += s[it][h];
+        uint64_t vf[8];
+        fa_pairs8(raw[it][0], vf);
+        fa_pairs8(raw[it][1], vf + 4);
+#pragma unroll
+        for (int h = 0; h < GROUP; ++h)
+#pragma unroll
+          for (int d = 0; d < 8; ++d) acc2[h][d] = f2_fma(f2_pack(s[it][h], s[it][h]), vf[d], acc2[h][d]);
       }
-      l[h] = fmaf(l[h], alpha[h], ps);
-#pragma unroll
-      for (int d = 0; d < 8; ++d) acc2[h][d] = fa_mul2<PACKED>(acc2[h][d], f2_pack(alpha[h], alpha[h]));
+      leave(i);
     }
 #pragma unroll
-    for (int it = 0; it < FA_TILE / 4; ++it) {
-      uint64_t vf[8];
-      fa_pairs8(raw[it][0], vf);
-      fa_pairs8(raw[it][1], vf + 4);
+    for (int h = 0; h < GROUP; ++h)
 #pragma unroll
-      for (int h = 0; h < GROUP; ++h)
+      for (int d = 0; d < 8; ++d) f2_unpack(acc2[h][d], acc[h][2 * d], acc[h][2 * d + 1]);
+  } else {
+    float qv[GROUP][16];
 #pragma unroll
-        for (int d = 0; d < 8; ++d) acc2[h][d] = fa_fma2<PACKED>(f2_pack(s[it][h], s[it][h]), vf[d], acc2[h][d]);
+    for (int h = 0; h < GROUP; ++h) {
+      const __nv_bfloat16* qp = q_s + (head0 + h) * FA_HD;
+      fa_unpack8(*reinterpret_cast<const uint4*>(qp + 8 * j), qv[h]);
+      fa_unpack8(*reinterpret_cast<const uint4*>(qp + 64 + 8 * j), qv[h] + 8);
+#pragma unroll
+      for (int d = 0; d < 16; ++d) qv[h][d] *= p.scale_log2;
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(empty_bar + stage);
+
+#pragma unroll
+    for (int h = 0; h < GROUP; ++h) {
+      m[h] = -INFINITY; l[h] = 0.f;
+#pragma unroll
+      for (int d = 0; d < 16; ++d) acc[h][d] = 0.f;
+    }
+
+    for (int i = 0; i < my_tiles; ++i) {
+      __nv_bfloat16 *kt, *vt;
+      const int ntok = enter(i, kt, vt);
+      float s[FA_TILE / 4][GROUP];
+      int tokc[FA_TILE / 4];
+#pragma unroll
+      for (int it = 0; it < FA_TILE / 4; ++it) {
+        const int tok = it * 4 + g;
+        const bool valid = tok < ntok;
+        tokc[it] = valid ? tok : 0;
+        const __nv_bfloat16* kr = kt + tokc[it] * kv_dim;
+        float kf[16];
+        fa_unpack8(*reinterpret_cast<const uint4*>(kr + 8 * j), kf);
+        fa_unpack8(*reinterpret_cast<const uint4*>(kr + 64 + 8 * j), kf + 8);
+#pragma unroll
+        for (int h = 0; h < GROUP; ++h) {
+          float d0 = 0.f, d1 = 0.f;
+#pragma unroll
+          for (int d = 0; d < 16; d += 2) {
+            d0 = fmaf(qv[h][d], kf[d], d0);
+            d1 = fmaf(qv[h][d + 1], kf[d + 1], d1);
+          }
+          float dot = d0 + d1;
+          dot += __shfl_xor_sync(0xffffffffu, dot, 1);
+          dot += __shfl_xor_sync(0xffffffffu, dot, 2);
+          dot += __shfl_xor_sync(0xffffffffu, dot, 4);
+          s[it][h] = valid ? dot : -INFINITY;
+        }
+      }
+      float alpha[GROUP];
+#pragma unroll
+      for (int h = 0; h < GROUP; ++h) {
+        float mt = s[0][h];
+#pragma unroll
+        for (int it = 1; it < FA_TILE / 4; ++it) mt = fmaxf(mt, s[it][h]);
+        mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, 8));
+        mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, 16));
+        const float mn = fmaxf(m[h], mt);
+        alpha[h] = fa_exp2(m[h] - mn);
+        m[h] = mn;
+        float ps = 0.f;
+#pragma unroll
+        for (int it = 0; it < FA_TILE / 4; ++it) {
+          s[it][h] = fa_exp2(s[it][h] - mn);
+          ps += s[it][h];
+        }
+        l[h] = fmaf(l[h], alpha[h], ps);
+#pragma unroll
+        for (int d = 0; d < 16; ++d) acc[h][d] *= alpha[h];
+      }
+#pragma unroll
+      for (int it = 0; it < FA_TILE / 4; ++it) {
+        const __nv_bfloat16* vr = vt + tokc[it] * kv_dim;
+        float vf[16];
+        fa_unpack8(*reinterpret_cast<const uint4*>(vr + 8 * j), vf);
+        fa_unpack8(*reinterpret_cast<const uint4*>(vr + 64 + 8 * j), vf + 8);
+#pragma unroll
+        for (int h = 0; h < GROUP; ++h)
+#pragma unroll
+          for (int d = 0; d < 16; ++d) acc[h][d] = fmaf(s[it][h], vf[d], acc[h][d]);
+      }
+      leave(i);
+    }
   }
 
   // ---- fold the 4 token slots of the warp
-  float acc[GROUP][16];
 #pragma unroll
   for (int h = 0; h < GROUP; ++h) {
-#pragma unroll
-    for (int d = 0; d < 8; ++d) f2_unpack(acc2[h][d], acc[h][2 * d], acc[h][2 * d + 1]);
     l[h] += __shfl_xor_sync(0xffffffffu, l[h], 8);
     l[h] += __shfl_xor_sync(0xffffffffu, l[h], 16);
 #pragma unroll
@@ -419,53 +564,7 @@ fused_decode_attn_kernel(const FusedAttnParams p) {
   }
   asm volatile("bar.sync 1, %0;" :: "r"(kvh * 32) : "memory");
   if (!*last_flag) return;
-  // warp w folds heads head0 .. head0+GROUP-1; lane owns 4 consecutive dims.  Lane s asks for split s's maximum and sum (at most 32 splits), and the partials of
-  // four splits of all heads are asked for at once: a split after another was up to three dependent round trips for each: 64 rows of 40
-  // tokens 10.4 -> 8.5 us, of 200 16.1 -> 14.7, 16 rows of 700 22.3 -> 15.9, 4 of 2000 25.7 -> 18.4 (16 query and 8 key heads).
-  float top[GROUP], sum[GROUP];
-#pragma unroll
-  for (int h = 0; h < GROUP; ++h) {
-    const int64_t at = ((int64_t)row * p.nsplit + lane) * p.num_heads + head0 + h;
-    top[h] = lane < p.nsplit ? __ldcg(p.part_ml + at * 2) : -INFINITY;
-    sum[h] = lane < p.nsplit ? __ldcg(p.part_ml + at * 2 + 1) : 0.f;
-  }
-  float4 num[GROUP];
-  float den[GROUP];
-#pragma unroll
-  for (int h = 0; h < GROUP; ++h) { num[h] = make_float4(0.f, 0.f, 0.f, 0.f); den[h] = 0.f; }
-  for (int s0 = 0; s0 < p.nsplit; s0 += 4) {
-    float4 a[4][GROUP];
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int h = 0; h < GROUP; ++h) {
-        const int64_t idx = ((int64_t)row * p.nsplit + s0 + u) * p.num_heads + head0 + h;
-        a[u][h] = s0 + u < p.nsplit ? __ldcg(reinterpret_cast<const float4*>(p.part_acc + idx * FA_HD) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    if (s0 == 0) {
-#pragma unroll
-      for (int h = 0; h < GROUP; ++h) top[h] = fa_exp2(top[h] - warp_max(top[h]));          // the splits' weights
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int h = 0; h < GROUP; ++h) {
-        const float w = __shfl_sync(0xffffffffu, top[h], (s0 + u) & 31), ls = __shfl_sync(0xffffffffu, sum[h], (s0 + u) & 31);
-        if (s0 + u < p.nsplit && ls > 0.f) {
-          num[h].x = fmaf(w, a[u][h].x, num[h].x); num[h].y = fmaf(w, a[u][h].y, num[h].y);
-          num[h].z = fmaf(w, a[u][h].z, num[h].z); num[h].w = fmaf(w, a[u][h].w, num[h].w);
-          den[h] = fmaf(w, ls, den[h]);
-        }
-      }
-  }
-#pragma unroll
-  for (int h = 0; h < GROUP; ++h) {
-    const float inv = den[h] > 0.f ? 1.f / den[h] : 0.f;
-    uint2 o;
-    o.x = pack_bf16(num[h].x * inv, num[h].y * inv);
-    o.y = pack_bf16(num[h].z * inv, num[h].w * inv);
-    stg_v2(p.out + ((int64_t)row * p.num_heads + head0 + h) * FA_HD + 4 * lane, o);
-  }
+  fa_fold<GROUP>(p.part_ml, p.part_acc, p.out, p.nsplit, p.num_heads, row, head0);
   }
 }
 
@@ -715,6 +814,21 @@ fused_decode_attn_small_kernel(const FusedAttnParams p, int rows) {
   }
 }
 
+// One and two query heads a key head: two products an instruction, keys and values of a tile asked for together.  A turn of the ring without branches (unrolled) where there
+// are many tiles a CTA: without splits (200 rows of 200 tokens, 16 and 8 heads, 32.5 -> 30.2 us), and with few key heads, whose CTAs wait for each tile (32 rows of 2000 tokens, 4
+// and 2 heads 31 -> 22, 8 and 4 35 -> 30; 28 and 34 before pairs); else the longer code costs more than it gives (64 rows of 40 tokens, 16 and 8 heads 8.8, unrolled 10.1).
+// Four query heads a key head: products one by one (pairs spill: 113 us for 200 rows of 200 tokens and 32 heads, 106 so), and as many registers as the CTAs of few key heads
+// leave: 300 rows of 1000 tokens, 8 and 2 heads 162 us, with 96 registers 245 (285 with pairs' order of loads, 233 before pairs), 16 and 4 245 (447); 32 and 8 heads have no more: 765 (743).
+static void (*fa_pick(int group, bool split, int kv_heads, bool eager))(const FusedAttnParams) {
+#define FA_ONE(G, K) (split ? (eager ? fused_decode_attn_kernel<G, true, true, K> : fused_decode_attn_kernel<G, false, true, K>) \
+                            : (eager ? fused_decode_attn_kernel<G, true, false, K> : fused_decode_attn_kernel<G, false, false, K>))
+  if (group == 1) return FA_ONE(1, 8);
+  if (group == 2) return kv_heads <= 4 ? FA_ONE(2, 4) : FA_ONE(2, 8);
+  if (group == 4) return kv_heads <= 2 ? FA_ONE(4, 2) : kv_heads <= 4 ? FA_ONE(4, 4) : FA_ONE(4, 8);
+#undef FA_ONE
+  return nullptr;
+}
+
 static size_t fa_smem_bytes(int kv_heads, int num_heads) {
   return (size_t)2 * FA_NSTAGE * FA_TILE * kv_heads * FA_HD * 2 + 2 * FA_NSTAGE * sizeof(uint64_t) + 16 +
          (size_t)(num_heads + 2 * kv_heads) * FA_HD * 2;
@@ -825,13 +939,7 @@ extern "C" int b2tts_fused_decode_attn(const void* q, int64_t q_row_stride, cons
     if (e != cudaSuccess) return cuda_fail(e, what);
     return B2TTS_OK;
   }
-  void (*kern)(const FusedAttnParams) = nullptr;
-#define FA_PICK(G) (p.nsplit == 1 ? (eager ? fused_decode_attn_kernel<G, true, false> : fused_decode_attn_kernel<G, false, false>) \
-                                  : (eager ? fused_decode_attn_kernel<G, true, true> : fused_decode_attn_kernel<G, false, true>))
-  if (group == 1) kern = FA_PICK(1);
-  else if (group == 2) kern = FA_PICK(2);
-  else if (group == 4) kern = FA_PICK(4);
-#undef FA_PICK
+  void (*kern)(const FusedAttnParams) = fa_pick(group, p.nsplit > 1, num_kv_heads, eager);
   B2_REQUIRE(kern, B2TTS_EUNSUPPORTED, "%s: GQA group %d unsupported (1, 2, 4)", what, group);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   if (e != cudaSuccess) return cuda_fail(e, what);

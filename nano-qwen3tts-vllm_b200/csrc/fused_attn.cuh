@@ -17,34 +17,15 @@ __device__ __forceinline__ void fa_unpack8(const uint4& r, float* f) {
   f[0] = bf16lo(r.x); f[1] = bf16hi(r.x); f[2] = bf16lo(r.y); f[3] = bf16hi(r.y);
   f[4] = bf16lo(r.z); f[5] = bf16hi(r.z); f[6] = bf16lo(r.w); f[7] = bf16hi(r.w);
 }
-// The same as pairs (2i, 2i + 1), products of pairs, and sixteen products with sums over the even and over the odd ones.  PACKED: two to an instruction; otherwise one by
-// one, where registers are too few for aligned pairs.
+// The same as pairs (2i, 2i + 1), and sixteen products with sums over the even and over the odd ones
 __device__ __forceinline__ void fa_pairs8(const uint4& r, uint64_t* f) {
   f[0] = f2_pack(bf16lo(r.x), bf16hi(r.x)); f[1] = f2_pack(bf16lo(r.y), bf16hi(r.y));
   f[2] = f2_pack(bf16lo(r.z), bf16hi(r.z)); f[3] = f2_pack(bf16lo(r.w), bf16hi(r.w));
 }
-template <bool PACKED>
-__device__ __forceinline__ uint64_t fa_mul2(uint64_t a, uint64_t b) {
-  if constexpr (PACKED) return f2_mul(a, b);
-  float x[2], y[2];
-  f2_unpack(a, x[0], x[1]);
-  f2_unpack(b, y[0], y[1]);
-  return f2_pack(x[0] * y[0], x[1] * y[1]);
-}
-template <bool PACKED>
-__device__ __forceinline__ uint64_t fa_fma2(uint64_t a, uint64_t b, uint64_t c) {
-  if constexpr (PACKED) return f2_fma(a, b, c);
-  float x[2], y[2], z[2];
-  f2_unpack(a, x[0], x[1]);
-  f2_unpack(b, y[0], y[1]);
-  f2_unpack(c, z[0], z[1]);
-  return f2_pack(fmaf(x[0], y[0], z[0]), fmaf(x[1], y[1], z[1]));
-}
-template <bool PACKED>
 __device__ __forceinline__ float fa_dot16(const uint64_t* q, const uint64_t* k) {
   uint64_t d = 0;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) d = fa_fma2<PACKED>(q[i], k[i], d);
+  for (int i = 0; i < 8; ++i) d = f2_fma(q[i], k[i], d);
   float even, odd;
   f2_unpack(d, even, odd);
   return even + odd;
