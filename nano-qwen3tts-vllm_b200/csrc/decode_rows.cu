@@ -805,22 +805,21 @@ static int dr_multiprocessors(cudaStream_t st) {
   return static_cast<int>(r.sm.smCount);
 }
 
+// Whether a CTA fits a multiprocessor: asked once for each number of rows (a device that this library runs on is an sm_100a like another), and only for those that
+// steps have, since asking loads the kernel
 template <int H, int I, int SQ, int SG, int ROWS>
 static bool dr_one_fits() {
-  constexpr int smem = static_cast<int>(sizeof(DrShared<H, I, ROWS>));
-  int least = 1;
-  auto ask = [&](auto kern) {
+  static const bool fits = [] {
+    constexpr int smem = static_cast<int>(sizeof(DrShared<H, I, ROWS>));
+    auto kern = decode_rows_kernel<H, I, SQ, SG, ROWS, true>;             // the other rounding has the same registers and shared memory
     int n = 0;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, DR_THREADS, smem) != cudaSuccess) {
-      cudaGetLastError();
-      n = 0;
-    }
-    least = least < n ? least : n;
-  };
-  ask(decode_rows_kernel<H, I, SQ, SG, ROWS, true>);
-  ask(decode_rows_kernel<H, I, SQ, SG, ROWS, false>);
-  return least >= 1;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, DR_THREADS, smem) == cudaSuccess)
+      return n >= 1;
+    cudaGetLastError();
+    return false;
+  }();
+  return fits;
 }
 // Whether a CTA can be resident on every multiprocessor at once, as the launch wants (without a device: as if so)
 static bool dr_resident(int form, int m, cudaStream_t st) {
@@ -830,15 +829,9 @@ static bool dr_resident(int form, int m, cudaStream_t st) {
     return true;
   }
   if (cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || cooperative == 0) return false;
-  // Whether one fits a multiprocessor is asked once for each instance (a device that this library runs on is an sm_100a like another)
-  if (form == 1) {
-    static const bool two = dr_one_fits<2048, 6144, 8, 2, 2>(), four = dr_one_fits<2048, 6144, 8, 2, 4>();
-    if (!(m <= 2 ? two : four)) return false;
-  } else {
-    static const bool two = dr_one_fits<1024, 3072, 8, 4, 2>(), four = dr_one_fits<1024, 3072, 8, 4, 4>(), eight = dr_one_fits<1024, 3072, 8, 4, DR_MAX_ROWS>();
-    if (!(m <= 2 ? two : m <= 4 ? four : eight)) return false;
-  }
-  return dr_multiprocessors(st) >= sm_count();
+  const bool fits = form == 1 ? (m <= 2 ? dr_one_fits<2048, 6144, 8, 2, 2>() : dr_one_fits<2048, 6144, 8, 2, 4>())
+                              : m <= 2 ? dr_one_fits<1024, 3072, 8, 4, 2>() : m <= 4 ? dr_one_fits<1024, 3072, 8, 4, 4>() : dr_one_fits<1024, 3072, 8, 4, DR_MAX_ROWS>();
+  return fits && dr_multiprocessors(st) >= sm_count();
 }
 
 }  // namespace b2

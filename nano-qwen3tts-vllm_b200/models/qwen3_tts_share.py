@@ -306,10 +306,12 @@ class DecoderStack(nn.Module):
         self._rows_where_faster = where_faster
         c, rope, widths = self.config, self.layers[0].self_attn.rotary_emb, self._widths()
         page = self.layers[0].self_attn.attn.k_cache.shape[1]
-        self._rows_most = max([m for m in range(1, DECODE_ROWS_MAX + 1) if nat.decode_rows_supported(m, *widths)], default=0)
-        if len(self.layers) > nat.DECODE_ROWS_MAX_LAYERS or c.head_dim != 128 or rope.inv_freq.numel() != 64 or page % 8 or page & (page - 1):
-            self._rows_most = 0
-        self._rows_ws = nat.decode_rows_workspace(*widths, self.norm.weight.device) if self._rows_most else None
+        self._rows_most, self._rows_ws = 0, None
+        if len(self.layers) <= nat.DECODE_ROWS_MAX_LAYERS and c.head_dim == 128 and rope.inv_freq.numel() == 64 and page % 8 == 0 and page & (page - 1) == 0:
+            self._rows_ws = nat.decode_rows_workspace(*widths, self.norm.weight.device)       # None: no kernel for these widths
+        if self._rows_ws is not None:
+            # a runner's steps are asked about one by one (which loads the kernels of those that it has)
+            self._rows_most = DECODE_ROWS_MAX if where_faster else max([m for m in range(1, DECODE_ROWS_MAX + 1) if nat.decode_rows_supported(m, *widths)], default=0)
 
     def _widths(self) -> tuple[int, int, int, int]:
         c = self.config
