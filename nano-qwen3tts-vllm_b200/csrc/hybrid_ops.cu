@@ -638,7 +638,8 @@ prep_vec8_kernel(const PrepArgs p) {
           const float other = __shfl_sync(0xffffffffu, f[e], from);
           if (turned) {
             const float2 cs = turn[t * half + (second ? ci - half : ci) + e];
-            f[e] = second ? f[e] * cs.x + other * cs.y : f[e] * cs.x - other * cs.y;
+            const float x1 = second ? other : f[e], x2 = second ? f[e] * cs.x : -(other * cs.y);
+            f[e] = fmaf(x1, second ? cs.y : cs.x, x2);   // the product of the head's first half joins the sum unrounded
           }
         }
       }
@@ -656,7 +657,8 @@ prep_vec8_kernel(const PrepArgs p) {
 // every two tokens paid for their own indexes, weights, angles and barrier.
 // Bound: HBM where nothing is turned, the turns' instructions beside it else.  16 + 8 + 8 heads of 128, 8192 / 4856 ragged tokens in us, above / this one: plain
 // 31.5 / 24.5 and 18.0 / 11.4, 64 coordinates turned by frequencies 37.4 / 28.2 and 20.8 / 14.5, head norms 37.4 / 25.5 and 22.1 / 13.8, head norms and a table
-// 45.1 / 31.4 and 26.0 / 17.5 (pairs), 57.8 / 38.0 and 34.3 / 22.0 (halves).  Angles read from the table by every thread 52 us, cosines beside sines in shared memory 32
+// 45.1 / 31.4 and 26.0 / 17.5 (pairs), 57.8 / 39.0 and 34.3 / 22.3 (halves; 38.0 and 22.0 where each coordinate's own
+// product joins the sum unrounded, which gives other bits than above).  Angles read from the table by every thread 52 us, cosines beside sines in shared memory 32
 // and 51; WALK of 4 30.8 and 18.5, of 16 31.2 and 19.4; two pieces on their way 32.2 and 19.3.  Fewer than 8 tokens a multiprocessor stay above, a token a CTA.
 constexpr int WALK = 8, AHEAD = 4;
 
@@ -753,14 +755,17 @@ prep_walk_kernel(const PrepArgs p) {
         } else {
 #pragma unroll
           for (int e = 0; e < 8; e += 4) {
-            float co[4] = {1.f, 1.f, 1.f, 1.f}, si[4] = {0.f, 0.f, 0.f, 0.f}, other[4];
+            float a1[4] = {1.f, 1.f, 1.f, 1.f}, a2[4] = {0.f, 0.f, 0.f, 0.f}, other[4];
 #pragma unroll
             for (int m = 0; m < 4; ++m) other[m] = __shfl_sync(0xffffffffu, f[e + m], from);
             if (turned) {
-              load4_f<float>(cs + e, co);
-              load4_f<float>(cs + half + e, si);
+              load4_f<float>(cs + (second ? half : 0) + e, a1);
+              load4_f<float>(cs + (second ? 0 : half) + e, a2);
 #pragma unroll
-              for (int m = 0; m < 4; ++m) f[e + m] = f[e + m] * co[m] + (second ? other[m] : -other[m]) * si[m];
+              for (int m = 0; m < 4; ++m) {              // as above, with the cosines and sines of a second half changed over
+                const float x1 = second ? other[m] : f[e + m], x2 = (second ? f[e + m] : -other[m]) * a2[m];
+                f[e + m] = fmaf(x1, a1[m], x2);
+              }
             }
           }
         }
